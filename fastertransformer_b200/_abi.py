@@ -25,6 +25,14 @@ class SamplingParams(C.Structure):
     ]
 
 
+class StopParams(C.Structure):
+    """ftb200_stop_params."""
+    _fields_ = [
+        ("stop_words", C.c_void_p), ("stop_words_len", C.c_int), ("sequence_limit_length", C.c_void_p),
+        ("arrived_dev", C.c_void_p), ("result_host", C.c_void_p), ("sequence", C.c_uint32),
+    ]
+
+
 class BeamHyps(C.Structure):
     """ftb200_beam_hyps."""
     _fields_ = [

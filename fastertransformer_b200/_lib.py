@@ -12,7 +12,7 @@ class FtbError(RuntimeError):
         self.status = status
 
 
-from ._abi import BeamHyps, BeamParams, GatherTreeParams, SamplingParams  # noqa: E402,F401
+from ._abi import BeamHyps, BeamParams, GatherTreeParams, SamplingParams, StopParams  # noqa: E402,F401
 
 
 def _load():
@@ -32,6 +32,7 @@ def _load():
         C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     l.ftb200_sampling_workspace_bytes.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_size_t)]
     l.ftb200_decode_step_sampling.argtypes = [C.POINTER(SamplingParams)]
+    l.ftb200_decode_step.argtypes = [C.POINTER(SamplingParams), C.POINTER(StopParams), C.c_int, C.POINTER(C.c_int)]
     l.ftb200_decode_step_sampling_static.argtypes = [C.POINTER(SamplingParams)]
     l.ftb200_static_scratch_bytes.restype = C.c_size_t
     l.ftb200_set_row_trace.argtypes = [C.c_void_p]

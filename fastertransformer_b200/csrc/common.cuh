@@ -94,6 +94,32 @@ __device__ __forceinline__ uint2 ld_nc_v2(const void* p)
 // ld.shared / st.shared instead of generic accesses (every pointer of the kernel's shared-memory map qualifies).
 #define FTB_ASSUME_SHARED(p) __builtin_assume(__isShared(p))
 
+// ---- word lists -----------------------------------------------------------------------------------
+// A word list is [2, L]: row 0 the concatenated token ids, row 1 the exclusive end offset of each word,
+// padded with -1.  Returns true when word `i` matches the tail of the sequence ending at position
+// `last` (inclusive) of column `col`, following parent_ids for beams.
+// kernels/ban_bad_words.cu:49-75 (n_match = size-1, last = step-1) and
+// kernels/stop_criteria_kernels.cu:53-75 (n_match = size, last = step).
+__device__ __forceinline__ bool tail_matches(const int* ids, const int* parents, const int* words, int item_start,
+                                             int n_match, int first_pos, size_t row_stride, size_t col_base,
+                                             int beam_idx, int beam_width)
+{
+    int parent = beam_idx;
+    for (int t = n_match - 1; t >= 0; --t) {
+        const size_t at = (size_t)(first_pos + t) * row_stride + col_base + parent;
+        if (ids[at] != words[item_start + t]) {
+            return false;
+        }
+        if (beam_width > 1) {
+            parent = parents[at];
+            if (parent < 0 || parent >= beam_width) {
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
 // ---- in-place ascending sort of u64 keys by a cooperating thread group ---------------------------
 // Bitonic network in its "all ascending" form (first sub-step of every merge compares mirrored
 // positions), which tolerates any n: positions >= n behave as +infinity and are never touched.

@@ -4,33 +4,9 @@
 
 #include "common.cuh"
 #include "ftb200.h"
+#include "split_args.cuh"
 
 namespace ftb200 {
-
-// A word list is [2, L]: row 0 the concatenated token ids, row 1 the exclusive end offset of each word,
-// padded with -1.  Returns true when word `i` matches the tail of the sequence ending at position
-// `last` (inclusive) of column `col`, following parent_ids for beams.
-// kernels/ban_bad_words.cu:49-75 (n_match = size-1, last = step-1) and
-// kernels/stop_criteria_kernels.cu:53-75 (n_match = size, last = step).
-__device__ __forceinline__ bool tail_matches(const int* ids, const int* parents, const int* words, int item_start,
-                                             int n_match, int first_pos, size_t row_stride, size_t col_base,
-                                             int beam_idx, int beam_width)
-{
-    int parent = beam_idx;
-    for (int t = n_match - 1; t >= 0; --t) {
-        const size_t at = (size_t)(first_pos + t) * row_stride + col_base + parent;
-        if (ids[at] != words[item_start + t]) {
-            return false;
-        }
-        if (beam_width > 1) {
-            parent = parents[at];
-            if (parent < 0 || parent >= beam_width) {
-                return false;
-            }
-        }
-    }
-    return true;
-}
 
 template<typename T>
 __global__ void ban_bad_words_kernel(T* logits, const int* output_ids, const int* parent_ids, int batch_size,
@@ -63,7 +39,8 @@ __global__ void ban_bad_words_kernel(T* logits, const int* output_ids, const int
 // One CTA: stop words for the local rows, then the length limit and the finished count for the batch.
 __global__ void stop_criteria_kernel(const int* output_ids, const int* parent_ids, const int* stop_words, int L,
                                      uint8_t* finished, const uint32_t* limit, int id_offset, int local_batch,
-                                     int batch_size, int beam_width, int step, int* count_out, int* count_host)
+                                     int batch_size, int beam_width, int step, int* count_out, int* count_host,
+                                     u64* result, u32 sequence)
 {
     __shared__ int s_count;
     if (threadIdx.x == 0) {
@@ -104,12 +81,32 @@ __global__ void stop_criteria_kernel(const int* output_ids, const int* parent_id
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            *count_out = s_count;
+            if (count_out != nullptr) {
+                *count_out = s_count;
+            }
+            if (result != nullptr) {
+                __threadfence_system();
+                *(volatile u64*)result = ((u64)sequence << 32) | (u32)s_count;
+            }
             if (count_host != nullptr) {
                 *count_host = s_count;  // pinned host memory, written from here: no copy has to follow the kernel
             }
         }
     }
+}
+
+// The criteria of a sampling step as a kernel of their own, for steps whose sampling kernel does not apply them.
+int stop_criteria_launch(const ftb200_sampling_params* p, const StopArgs& T, cudaStream_t st)
+{
+    if (T.stop_words == nullptr && T.limit == nullptr) {
+        return FTB200_OK;
+    }
+    stop_criteria_kernel<<<1, 1024, 0, st>>>(p->output_ids, nullptr, T.stop_words, T.stop_words_len, T.finished, T.limit,
+                                             p->ite * p->local_batch_size, p->local_batch_size, p->batch_size, 1, p->step,
+                                             nullptr, nullptr, T.result, T.sequence);
+    FTB_CUDA_CHECK(cudaGetLastError());
+    note_launch(1);
+    return FTB200_OK;
 }
 
 }  // namespace ftb200
@@ -181,7 +178,8 @@ extern "C" int ftb200_stop_criteria(const int* output_ids, const int* parent_ids
     }
     stop_criteria_kernel<<<1, 1024, 0, st>>>(output_ids, parent_ids, stop_words_len > 0 ? stop_words : nullptr,
                                              stop_words_len, finished, sequence_limit_length, id_offset,
-                                             local_batch_size, batch_size, beam_width, step, finished_count_dev, direct);
+                                             local_batch_size, batch_size, beam_width, step, finished_count_dev, direct,
+                                             nullptr, 0);
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);
     if (sequence_limit_length != nullptr && direct == nullptr) {

@@ -1,8 +1,10 @@
 // extern "C" entry of the fused decode-sampling step: argument checks, shared-memory plan, launch.
 #include <atomic>
+#include <chrono>
 #include <mutex>
 
 #include "sampling_params.cuh"
+#include "split_args.cuh"
 
 namespace ftb200 {
 
@@ -32,6 +34,11 @@ extern template int fast_sampling_occupancy<FTB200_F16, true>(size_t, int*);
 extern template int fast_sampling_occupancy<FTB200_BF16, true>(size_t, int*);
 extern template int fast_sampling_launch<FTB200_F16, true>(const KParams&, int, size_t, cudaStream_t);
 extern template int fast_sampling_launch<FTB200_BF16, true>(const KParams&, int, size_t, cudaStream_t);
+template<int DT>
+int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_general, cudaStream_t st);
+extern template int split_sampling_launch<FTB200_F32>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
+extern template int split_sampling_launch<FTB200_F16>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
+extern template int split_sampling_launch<FTB200_BF16>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
 size_t fast_smem_for(int hash_slots, int vocab_padded, bool topp);
 int    fast_max_history();
 int    fast_max_words();
@@ -79,6 +86,49 @@ static size_t redo_list_bytes(int local_batch)
 }
 
 static int g_fast_path = 1;  // see ftb200_set_single_pass
+
+// Whether the split kernel (a row over a cluster of CTAs) serves a call, and in which form.  `single_pass`: the
+// single-pass kernels could serve it too.  The lines come from timing both at 32000 .. 256000 columns and 1 .. 1024
+// rows: the split form ends a row in 6 us (arg-max) to 40 us (wide nucleus) however slow the row is for one CTA, but
+// costs 2 to 4 times the SM time, so it loses once the single-pass kernels have the chip full.  With both kinds of rows
+// in a call those wait longest for their slowest rows (1024 x 32000: 191 us split, 216 us single-pass; 128 x 128256:
+// 113 / 120; 256 x 128256: 207 / 134); nucleus rows alone pack better (256 x 51200: 100 / 71, 64 x 51200: 51 / 72);
+// rows of a small k are nearly as quick in one CTA.
+static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool single_pass, size_t smem_general,
+                         SplitArgs* A, bool* whole)
+{
+    const int rows = p->local_batch_size, vocab = p->vocab_size, sms = sm_count();
+    if (vocab < 1024) {
+        return false;  // (the denominator's chains are then not 1024)
+    }
+    if (single_pass) {
+        const double work = (double)rows * vocab;
+        const bool   topk = K.topk_states != nullptr, topp = K.topp_states != nullptr;
+        const double most = topk && topp ? 16.5e6 : (topp ? (rows <= 96 ? 9e6 : 0.0) : (K.max_top_k > 256 ? 4.2e6 : 2.1e6));
+        if (work > most) {
+            return false;
+        }
+    }
+    // CTAs per row: eight while they are all resident (and for rows so long that a slice would not leave room for
+    // three CTAs on an SM), four or two when there are more rows or the rows are short: a CTA's fixed costs then weigh
+    // more than its columns (1024 x 32000 fp32, k = 50: 445 us with eight, 184 us with two).
+    int lgn = rows * 8 <= 2 * sms || vocab > 65536 ? 3 : (rows * 4 <= 2 * sms || vocab > 40960 ? 2 : 1);
+    for (; lgn <= 3; ++lgn) {
+        A->slice = ((vocab + 1023) / 1024) << (10 - lgn);
+        A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
+        if (split_smem_bytes(A->slice) <= kSpMaxSmem) {
+            break;
+        }
+    }
+    if (lgn > 3) {
+        return false;
+    }
+    A->lgn            = lgn;
+    const size_t smem = split_smem_bytes(A->slice) > smem_general ? split_smem_bytes(A->slice) : smem_general;
+    const int    fit  = smem <= 105 * 1024 ? 2 : 1;
+    *whole            = lgn >= 2 && (rows << lgn) <= fit * sms;
+    return true;
+}
 
 // Second stream of the single-pass step (one per device, made on first use) with the two events of its fork and join.
 struct SideStream {
@@ -268,6 +318,7 @@ static int plan_sampling(const ftb200_sampling_params* p, KParams& K, size_t& sm
     K.redo_count     = nullptr;
     K.redo_rows      = nullptr;
     K.row_count_dev  = nullptr;
+    K.row_flags      = nullptr;
     K.scratch        = (u64*)((char*)p->workspace + 256 + redo_list_bytes(p->local_batch_size));
     K.scratch_stride = scratch_stride_for(p->vocab_size_padded);
     return FTB200_OK;
@@ -282,7 +333,9 @@ extern "C" int ftb200_set_row_trace(uint64_t* device_buf)
 // One fused step.  `fork` allows the second stream of the single-pass kernels (made on first use); without it
 // the same kernels run one after the other on the caller's stream and nothing is created.
 namespace ftb200 {
-int decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork);
+int decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop = nullptr,
+                              bool* stop_done = nullptr);
+int stop_criteria_launch(const ftb200_sampling_params* p, const StopArgs& T, cudaStream_t st);
 }
 
 extern "C" int ftb200_decode_step_sampling(const ftb200_sampling_params* p)
@@ -290,7 +343,56 @@ extern "C" int ftb200_decode_step_sampling(const ftb200_sampling_params* p)
     return decode_step_sampling_impl(p, true);
 }
 
-int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork)
+extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_params* s, int timeout_ms, int* should_stop)
+{
+    if (s == nullptr || should_stop == nullptr || p == nullptr || p->finished == nullptr
+        || (s->sequence_limit_length != nullptr && (s->result_host == nullptr || s->arrived_dev == nullptr))) {
+        set_error("ftb200_decode_step: invalid argument");
+        return FTB200_INVALID_ARG;
+    }
+    StopArgs T{};
+    T.stop_words     = s->stop_words_len > 0 ? s->stop_words : nullptr;
+    T.stop_words_len = s->stop_words_len;
+    T.limit          = s->sequence_limit_length;
+    T.finished       = p->finished - (size_t)p->ite * p->local_batch_size;
+    T.arrived        = s->arrived_dev;
+    T.result         = (u64*)s->result_host;
+    T.sequence       = ++s->sequence;
+    bool done        = false;
+    int  rc          = decode_step_sampling_impl(p, true, &T, &done);
+    if (rc == FTB200_OK && !done) {
+        rc = stop_criteria_launch(p, T, (cudaStream_t)p->stream);
+    }
+    *should_stop = 0;
+    if (rc != FTB200_OK || T.limit == nullptr) {
+        return rc;
+    }
+    // The last kernel of the step stores (sequence, count) into the page-locked word: no query of the stream, whose
+    // answer comes several microseconds after the kernel's end.
+    const volatile u64* w  = T.result;
+    const auto          t0 = std::chrono::steady_clock::now();
+    for (u32 spin = 1;; ++spin) {
+        const u64 v = *w;
+        if ((u32)(v >> 32) == T.sequence) {
+            *should_stop = (u32)v == (u32)p->batch_size ? 1 : 0;
+            return FTB200_OK;
+        }
+        if ((spin & 1023u) == 0) {
+            const cudaError_t e = cudaStreamQuery((cudaStream_t)p->stream);
+            if (e != cudaSuccess && e != cudaErrorNotReady) {
+                set_error(std::string("ftb200_decode_step: ") + cudaGetErrorString(e));
+                return FTB200_CUDA_ERROR;
+            }
+            const auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0);
+            if (timeout_ms >= 0 && ms.count() > timeout_ms) {
+                set_error("ftb200_decode_step: the step did not end within the deadline");
+                return FTB200_TIMEOUT;
+            }
+        }
+    }
+}
+
+int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop, bool* stop_done)
 {
     reset_launch_count();
     KParams K;
@@ -304,14 +406,38 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
         return FTB200_OK;
     }
     cudaStream_t st = (cudaStream_t)p->stream;
-    FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
     // 16-bit logits without a bias, log-probs or timeline: the single-pass kernel serves the rows first and
     // leaves a list of the rows it does not cover; decode_sampling_kernel then works that list off.
     const bool single_pass = g_fast_path && p->dtype != FTB200_F32 && K.bias == nullptr && K.cum_log_probs == nullptr
                              && K.out_log_probs == nullptr && p->vocab_size_padded <= (1 << 20)
                              && p->vocab_size >= 16384 + 16 && (K.apply_rep ? p->step : 0) <= fast_max_history()
                              && (K.bad_words != nullptr ? K.bad_words_len : 0) <= fast_max_words();
-    if (single_pass) {
+    SplitArgs A{};
+    bool      whole = false;
+    if (g_fast_path && choose_split(p, K, single_pass, smem, &A, &whole)) {
+        A.redo_flags = whole ? nullptr : (int*)((char*)p->workspace + 256);
+        if (whole && stop != nullptr) {
+            A.stop     = *stop;
+            *stop_done = true;
+        }
+        switch (p->dtype) {
+            case FTB200_F32: rc = split_sampling_launch<FTB200_F32>(K, A, smem, st); break;
+            case FTB200_F16: rc = split_sampling_launch<FTB200_F16>(K, A, smem, st); break;
+            default: rc = split_sampling_launch<FTB200_BF16>(K, A, smem, st); break;
+        }
+        if (rc != FTB200_OK) {
+            return rc;
+        }
+        note_launch(1);
+        if (whole) {
+            return FTB200_OK;
+        }
+        K.row_flags = A.redo_flags;
+    }
+    if (K.row_flags == nullptr) {
+        FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
+    }
+    if (single_pass && K.row_flags == nullptr) {
         const size_t fsmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, false);
         const size_t psmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, true);
         const bool   f16   = p->dtype == FTB200_F16;

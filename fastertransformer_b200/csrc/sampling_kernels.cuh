@@ -1060,6 +1060,37 @@ static __device__ __noinline__ int resolve_topk_class(u64* cls, int m, int want,
     if (m == 1) {
         return (int)(cls[0] & 0xffffffffu);
     }
+    if (m <= 32) {
+        // a class that fits a warp: both orders by counting, one shuffle per member
+        if (tid < 32) {
+            const bool in   = tid < m;
+            const u32  col  = in ? (u32)(cls[tid] & 0xffffffffu) : 0u;
+            const u32  lane = (col / bs1) & 7u;
+            const u64  key1 = in ? ((u64)lane << 56) | ((u64)(bs1 - 1 - (int)(col % bs1)) << 40) | col : ~0ull;
+            u32        r = lane_base[lane];
+            for (int j = 0; j < m; ++j) {
+                const u64 o = __shfl_sync(0xffffffffu, key1, j);
+                r += ((u32)(o >> 56) == lane && o < key1) ? 1u : 0u;
+            }
+            u64 key2 = ~0ull;
+            if (in && r < (u32)k) {
+                const u32 i2 = lane * k + r;
+                key2         = ((u64)(bs2 - 1 - (i2 % bs2)) << 48) | ((u64)i2 << 32) | col;
+            }
+            int at = 0;
+            for (int j = 0; j < m; ++j) {
+                const u64 o = __shfl_sync(0xffffffffu, key2, j);
+                at += (o < key2 || (o == key2 && j < tid)) ? 1 : 0;
+            }
+            if (in && at == (want < m ? want : m - 1)) {
+                s_ans = key2 == ~0ull ? -1 : (int)col;
+            }
+        }
+        __syncthreads();
+        const int r = s_ans;
+        __syncthreads();
+        return r;
+    }
     if (tid < 8) {
         s_lane_cnt[tid] = 0;
     }
@@ -1395,8 +1426,10 @@ __device__ __forceinline__ void write_lengths(const KParams& P, const RowOut& O,
 
 // The draw of topk_stage2_sampling (sampling_topk_kernels.cu:255-311) over `sorted` (value descending),
 // then the tie-order resolution.  use_exp: values are logits (exp taken here) or probabilities.
-static __device__ __noinline__ void topk_finish(const KParams& P, const Smem& S, const RowOut& O, u64* sorted, int n, int k, float u,
-                            float top_p, bool use_exp, bool want_lp)
+// open_end: the lowest value class of `sorted` may have members that were not collected.  The sum and the walk do not
+// depend on which of them are missing; a draw that lands in that class does: false then, and nothing is written.
+static __device__ __noinline__ bool topk_finish(const KParams& P, const Smem& S, const RowOut& O, u64* sorted, int n, int k, float u,
+                            float top_p, bool use_exp, bool want_lp, bool open_end = false)
 {
     __shared__ int   s_pick, s_lo, s_hi;
     __shared__ float s_e, s_sum;
@@ -1517,10 +1550,14 @@ static __device__ __noinline__ void topk_finish(const KParams& P, const Smem& S,
             write_lengths(P, O, 0);
         }
         __syncthreads();
-        return;
+        return true;
     }
     // extent of the value class of the picked entry
     const u32 kv = (u32)(sorted[pick] >> 32);
+    if (open_end && kv == (u32)(sorted[n - 1] >> 32)) {
+        __syncthreads();
+        return false;
+    }
     for (int i = tid; i < n; i += kThreads) {
         if ((u32)(sorted[i] >> 32) == kv) {
             atomicMin(&s_lo, i);
@@ -1576,6 +1613,7 @@ static __device__ __noinline__ void topk_finish(const KParams& P, const Smem& S,
         write_lengths(P, O, col);
     }
     __syncthreads();
+    return true;
 }
 
 // ---- top-k, k == 1, no log-probs: a single arg-max with the reference's tie order ------------------
@@ -2497,6 +2535,56 @@ constexpr int kMaxRuns  = 4096;  // runs held in shared memory
 constexpr int kMaxSpecs = 1024;  // special / edge columns above the cut
 constexpr int kMaxAbove = 256;   // ordinary columns above a class window that does not reach the row maximum
 
+// J-th smallest column of the n > J distinct columns in cls: they are counted per block of columns (reversed, so that
+// the walk from the top runs over ascending columns), the block holding rank J is found, and only the few members of
+// that block are ranked against each other.
+static __device__ __noinline__ int select_jth_column(const u32* cls, int n, int J, u32* hist, int vocab_padded)
+{
+    __shared__ u32 s_blk[512];
+    __shared__ u32 s_nblk;
+    __shared__ int s_col;
+    const int      tid   = threadIdx.x;
+    int            shift = 0;
+    while (((vocab_padded - 1) >> shift) >= kNB) {
+        ++shift;
+    }
+    for (int i = tid; i < kNB; i += kThreads) {
+        hist[i] = 0;
+    }
+    if (tid == 0) {
+        s_nblk = 0;
+        s_col  = 0;
+    }
+    __syncthreads();
+    for (int a = tid; a < n; a += kThreads) {
+        smem_add(&hist[kNB - 1 - (int)(cls[a] >> shift)], 1u);
+    }
+    __syncthreads();
+    u32       before = 0;
+    const int bsel   = find_count_from_top(hist, (u32)(J + 1), &before);
+    for (int a = tid; a < n; a += kThreads) {
+        const int b = kNB - 1 - (int)(cls[a] >> shift);
+        if (b == bsel) {
+            s_blk[atomicAdd(&s_nblk, 1u)] = cls[a];
+        }
+    }
+    __syncthreads();
+    const int m  = (int)s_nblk;
+    const int jj = J - (int)before;
+    for (int a = tid; a < m; a += kThreads) {
+        const u32 ca = s_blk[a];
+        int       rk = 0;
+        for (int b = 0; b < m; ++b) {
+            rk += s_blk[b] < ca ? 1 : 0;
+        }
+        if (rk == jj) {
+            s_col = (int)ca;
+        }
+    }
+    __syncthreads();
+    return s_col;
+}
+
 template<int DT>
 __device__ __noinline__ int row_topp_classes(const KParams& P, const Smem& S, const RowCtx& C, const RowOut& O,
                                              float maxv, float denom, float rand_num, float cut0, u32 kmax16,
@@ -3069,52 +3157,9 @@ __device__ __noinline__ int row_topp_classes(const KParams& P, const Smem& S, co
     if (ncls > 2 * kMaxRuns || J >= ncls) {
         { if (O.trace != nullptr && threadIdx.x == 0) { O.trace[4 + 25] = 10; } return 0; }
     }
-    // J-th smallest column of the class: members are counted per block of columns (reversed, so that the
-    // walk from the top runs over ascending columns), the block holding rank J is found, and only the few
-    // members of that block are ranked against each other.
-    {
-        __shared__ u32 s_blk[512];
-        __shared__ u32 s_nblk;
-        int            shift = 0;
-        while (((P.vocab_padded - 1) >> shift) >= kNB) {
-            ++shift;
-        }
-        for (int i = tid; i < kNB; i += kThreads) {
-            S.hist[i] = 0;
-        }
-        if (tid == 0) {
-            s_nblk = 0;
-        }
-        __syncthreads();
-        for (int a = tid; a < ncls; a += kThreads) {
-            smem_add(&S.hist[kNB - 1 - (int)(cls[a] >> shift)], 1u);
-        }
-        __syncthreads();
-        u32       before = 0;
-        const int bsel   = find_count_from_top(S.hist, (u32)(J + 1), &before);
-        for (int a = tid; a < ncls; a += kThreads) {
-            const int b = kNB - 1 - (int)(cls[a] >> shift);
-            if (b == bsel) {
-                s_blk[atomicAdd(&s_nblk, 1u)] = cls[a];
-            }
-        }
-        __syncthreads();
-        const int m  = (int)s_nblk;
-        const int jj = J - (int)before;
-        for (int a = tid; a < m; a += kThreads) {
-            const u32 ca = s_blk[a];
-            int       rk = 0;
-            for (int b = 0; b < m; ++b) {
-                rk += s_blk[b] < ca ? 1 : 0;
-            }
-            if (rk == jj) {
-                s_sel = (int)ca;
-            }
-        }
-    }
-    __syncthreads();
+    const int id_class = select_jth_column(cls, ncls, J, S.hist, P.vocab_padded);
     if (tid == 0) {
-        const int id = s_sel;
+        const int id = id_class;
         *O.id_out    = id;
         if (want_lp) {
             const float lprob = logf(p_sel);
@@ -3787,6 +3832,46 @@ __device__ __noinline__ void row_vp_stats(const KParams& P, const Smem& S, const
     __syncthreads();
 }
 
+// A finished row of the top-p layer (one thread): one-hot, probability 1/(1+1e-6) on the end id
+// (sampling_topp_kernels.cu:1309-1341).
+template<int DT>
+__device__ __forceinline__ void finished_topp_row(const KParams& P, const RowOut& O, float u, bool want_lp)
+{
+    const int   r     = O.r;
+    const float top_p = P.topp_ps[r];
+    const float p0    = round_to_T<DT>(1.0f / (1.0f + 1e-6f));
+    *O.id_out         = O.end_id;
+    if (p0 >= top_p || u * top_p <= p0) {
+        if (want_lp) {
+            float lprob = logf(p0);
+            if (P.cum_log_probs != nullptr) {
+                P.cum_log_probs[r] += lprob;
+            }
+            if (P.out_log_probs != nullptr) {
+                P.out_log_probs[r] = lprob;
+            }
+        }
+        if (P.seq_len != nullptr && P.finished != nullptr) {
+            P.finished[r] = 1;
+        }
+    }
+}
+
+// Top-p decay / reset of one row (one thread; sampling_topp_kernels.cu:1381-1408), applied to every row of the call.
+__device__ __forceinline__ void topp_decay_row(const KParams& P, int r, int id)
+{
+    if (P.topp_states != nullptr && P.topp_decay != nullptr) {
+        float p = P.topp_ps[r];
+        if (id == P.topp_reset[r]) {
+            p = P.topp_initial[r];
+        }
+        else {
+            p = fmaxf(p * P.topp_decay[r], P.topp_min[r]);
+        }
+        P.topp_ps[r] = p;
+    }
+}
+
 template<int DT>
 __device__ void process_row(const KParams& P, const Smem& S, int r, u64* gscratch, u64* trace)
 {
@@ -3857,26 +3942,8 @@ __device__ void process_row(const KParams& P, const Smem& S, int r, u64* gscratc
         __syncthreads();
         const float u = s_u;
         if (mode == 2 && fin) {
-            // one-hot row: probability 1/(1+1e-6) on the end id (sampling_topp_kernels.cu:1309-1341)
             if (tid == 0) {
-                const float top_p = P.topp_ps[r];
-                const float p0    = DT == FTB200_F16 ? __half2float(__float2half_rn(1.0f / (1.0f + 1e-6f))) :
-                                                       1.0f / (1.0f + 1e-6f);
-                *O.id_out         = O.end_id;
-                if (p0 >= top_p || u * top_p <= p0) {
-                    if (want_lp) {
-                        float lprob = logf(p0);
-                        if (P.cum_log_probs != nullptr) {
-                            P.cum_log_probs[r] += lprob;
-                        }
-                        if (P.out_log_probs != nullptr) {
-                            P.out_log_probs[r] = lprob;
-                        }
-                    }
-                    if (P.seq_len != nullptr && P.finished != nullptr) {
-                        P.finished[r] = 1;
-                    }
-                }
+                finished_topp_row<DT>(P, O, u, want_lp);
             }
         }
         else {
@@ -3902,18 +3969,23 @@ __device__ void process_row(const KParams& P, const Smem& S, int r, u64* gscratc
         }
     }
     __syncthreads();
-    // top-p decay / reset (sampling_topp_kernels.cu:1381-1408), applied to every row of the call
-    if (P.topp_states != nullptr && P.topp_decay != nullptr && tid == 0) {
-        const int id = *O.id_out;
-        float     p  = P.topp_ps[r];
-        if (id == P.topp_reset[r]) {
-            p = P.topp_initial[r];
-        }
-        else {
-            p = fmaxf(p * P.topp_decay[r], P.topp_min[r]);
-        }
-        P.topp_ps[r] = p;
+    if (tid == 0) {
+        topp_decay_row(P, r, *O.id_out);
     }
+}
+
+// Shared-memory map of the general row code (the size is computed by the entry point).
+__device__ __forceinline__ void map_general_smem(const KParams& P, Smem& S, unsigned char* smem)
+{
+    S.cand  = (u64*)smem;
+    S.hist  = (u32*)(S.cand + kCap);
+    S.val2  = (float*)(S.hist + kNB);
+    S.flags = (u32*)(S.val2 + 1024);
+    S.hash  = S.flags + P.flag_words;
+    S.spre  = (float*)(S.hash + P.hash_slots);
+    S.sfin  = S.spre + P.hash_slots;
+    S.nhit  = (u32*)(S.sfin + P.hash_slots);
+    S.hitq  = (unsigned short*)(S.nhit + 4);
 }
 
 template<int DT>
@@ -3924,26 +3996,28 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
     __shared__ Smem                               s_S;
     Smem&                                         S = s_S;
     if (threadIdx.x == 0) {
-        S.cand  = (u64*)smem_raw;
-        S.hist  = (u32*)(S.cand + kCap);
-        S.val2  = (float*)(S.hist + kNB);
-        S.flags = (u32*)(S.val2 + 1024);
-        S.hash  = S.flags + P.flag_words;
-        S.spre  = (float*)(S.hash + P.hash_slots);
-        S.sfin  = S.spre + P.hash_slots;
-        S.nhit  = (u32*)(S.sfin + P.hash_slots);
-        S.hitq  = (unsigned short*)(S.nhit + 4);
+        map_general_smem(P, S, smem_raw);
     }
     u64* gscratch = P.scratch + (size_t)blockIdx.x * P.scratch_stride;
     // rows to serve: the whole local batch, or the list the single-pass kernel left behind
     const int n_rows = P.row_count_dev != nullptr ? (int)*P.row_count_dev : P.local_batch;
-    for (;;) {
+    for (int next = blockIdx.x;; next += gridDim.x) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            s_row = (int)atomicAdd(P.ticket, 1u);
+        int t;
+        if (P.row_flags != nullptr) {
+            // the rows the split kernel left (normally none): no ticket, every CTA looks through its share
+            t = next;
+            if (t < n_rows && P.row_flags[P.row_order != nullptr ? P.row_order[t] : t] == 0) {
+                continue;
+            }
         }
-        __syncthreads();
-        const int t = s_row;
+        else {
+            if (threadIdx.x == 0) {
+                s_row = (int)atomicAdd(P.ticket, 1u);
+            }
+            __syncthreads();
+            t = s_row;
+        }
         if (t >= n_rows) {
             break;
         }

@@ -60,6 +60,9 @@ struct KParams {
     u32*       redo_count;
     int*       redo_rows;
     const u32* row_count_dev;
+    // Rows the split kernel leaves: decode_sampling_kernel launched with row_flags != null serves the rows r with
+    // row_flags[r] != 0.
+    const int* row_flags;
     u64*     trace;           // optional per-row timeline: {row, CTA, start ns, end ns} per ticket, else null
     u64*     scratch;         // per-CTA candidate overflow area
     size_t   scratch_stride;  // u64 entries per CTA

@@ -1,0 +1,38 @@
+// Launch arguments of the split decode-sampling kernel (split_sampling.cuh), shared with the entry point.
+#pragma once
+#include "sampling_params.cuh"
+
+namespace ftb200 {
+
+constexpr int kSpBins     = 2048;
+constexpr int kSpAreaCap  = 5120;                   // fp32 keys a CTA can receive of a nucleus
+constexpr int kSpCandCap  = kSpAreaCap / 2;         // 64-bit candidates the leader can receive
+constexpr int kSpSub      = kSpAreaCap / 2;         // sub-buckets of the nucleus sort: four keys each and room between bins
+constexpr int kSpMaxN     = 8;                       // portable cluster size
+constexpr size_t kSpMaxSmem = 216 * 1024;
+constexpr int kSpMinSlice = (kNB * 4 + 1024 * 4) / 4;  // the draw's histogram and values lie over the slice
+
+// Stop criteria of the step, for the launch forms that finish everything themselves.
+struct StopArgs {
+    const int*      stop_words;      // [local_batch, 2, stop_words_len] or null
+    int             stop_words_len;
+    const uint32_t* limit;           // [batch_size] or null: then nothing is counted
+    uint8_t*        finished;        // [batch_size], the whole batch
+    u32*            arrived;         // one word, zero between calls
+    u64*            result;          // page-locked host word: sequence << 32 | finished rows
+    u32             sequence;
+};
+
+struct SplitArgs {
+    int  lgn;         // log2 of the CTAs per row
+    int  slice;       // floats of the slice area
+    int* redo_flags;  // [local_batch]: 1 when the row is left to decode_sampling_kernel (null: the kernel serves it itself)
+    StopArgs stop;    // (only where redo_flags is null)
+};
+
+__host__ __device__ inline size_t split_smem_bytes(int slice)
+{
+    return (size_t)slice * 4 + (size_t)kSpAreaCap * 4 + (size_t)kSpBins * 8 + (size_t)kSpSub * 2;
+}
+
+}  // namespace ftb200

@@ -1,0 +1,1606 @@
+// Decode-sampling step with a row split over a cluster of CTAs (sm_100a thread-block clusters, distributed shared
+// memory).  One cluster serves one row: CTA c of n owns the columns whose number modulo 1024 lies in
+// [c * 1024 / n, (c + 1) * 1024 / n), keeps their final values (temperature, bias, penalties and bans applied) in its
+// shared memory as fp32, and every later step - maximum, ordered soft-max denominator, histogram, selection, nucleus
+// sort - reads shared memory only: the row is read from HBM once, whatever the logits type and options are.
+//
+// Why this split: the reference's soft-max denominator is a sum over 1024 strided chains (column modulo 1024, added
+// chunk after chunk), so a CTA that owns whole chains can add them in the reference's order without talking to the
+// others, and the special columns (history, bans) are scattered evenly.  What is exchanged per row is small: a bit per
+// special column, one maximum and 1024 / 32 / n partial sums per CTA, a 2048-bin histogram, the candidates.
+//
+// What bounds it: latency.  A row takes six to ten cluster barriers (0.5 us each) and about six sweeps over its shared
+// memory; a CTA-per-row kernel walks eight times as many columns with the same 256 threads.  Measured on B200, one row
+// alone on its SMs: arg-max of 32000 columns 5 us, k = 50 of 50257 fp32 17 us, a nucleus of 50257 fp32 22 us (the general
+// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 10 us (k = 1) to 70 us (25000-column nucleus).  Batch
+// of 64 x 50257 fp32 top-p: 1186 -> 61 us a step; 48 x 51200 half with bias and log-probs: 920 -> 103 us.
+//
+// The results are those of sampling_kernels.cuh, bit for bit; rows that do not fit the fixed tables here (a nucleus
+// above the collection areas, thousands of equal values around the k-th) go to the general row code.
+#pragma once
+#include "sampling_kernels.cuh"
+#include "split_args.cuh"
+
+namespace ftb200 {
+
+// ---- distributed shared memory ----------------------------------------------------------------------------------
+__device__ __forceinline__ u32 cluster_rank()
+{
+    u32 r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ u32 cluster_addr(u32 smem, u32 rank)
+{
+    u32 a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    cluster_arrive();
+    cluster_wait();
+}
+__device__ __forceinline__ void dst_u32(u32 a, u32 v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void dst_u64(u32 a, u64 v)
+{
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ u32 dld_u32(u32 a)
+{
+    u32 v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ u32 datom_add(u32 a, u32 v)
+{
+    u32 o;
+    asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory");
+    return o;
+}
+__device__ __forceinline__ void dred_or(u32 a, u32 v)
+{
+    asm volatile("red.shared::cluster.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void dred_min(u32 a, u32 v)
+{
+    asm volatile("red.shared::cluster.min.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void dred_max(u32 a, u32 v)
+{
+    asm volatile("red.shared::cluster.max.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ u32 smem_addr(const void* p)
+{
+    return (u32)__cvta_generic_to_shared(p);
+}
+
+// ---- bins -------------------------------------------------------------------------------------------------------
+// Distance d below the row maximum -> position on the scale of bins: 128 bins a logit for the first 8 (where nearly
+// every selection ends), 32 up to 24, 8 beyond.  The least of three lines: monotone, no branch, and a distance that is
+// not a number lands on the last bin.
+__device__ __forceinline__ float sp_pos(float d)
+{
+    return fminf(fminf(fminf(d * 128.0f, d * 32.0f + 768.0f), d * 8.0f + 1344.0f), (float)(kSpBins - 1));
+}
+__device__ __forceinline__ int sp_bin(float d)
+{
+    return (int)sp_pos(d);
+}
+__device__ __forceinline__ float sp_edge(int b)  // near edge of bin b = far edge of bin b - 1
+{
+    return fmaxf(fmaxf((float)b * (1.0f / 128.0f), ((float)b - 768.0f) * (1.0f / 32.0f)), ((float)b - 1344.0f) * 0.125f);
+}
+// a value that every column of bins 0 .. b reaches (the exact test is the bin's)
+__device__ __forceinline__ float sp_floor_value(float maxv, int b)
+{
+    return b + 1 < kSpBins ? maxv - sp_edge(b + 1) * 1.0001f - 1e-6f * fabsf(maxv) - 1e-6f : -INFINITY;
+}
+
+// Exclusive block-wide prefix of one value per thread; *total receives the sum.
+static __device__ u32 block_excl_u32(u32 v, u32* total)
+{
+    __shared__ u32 s_w[kWarps];
+    const int      lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    u32            incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const u32 t = __shfl_up_sync(0xffffffffu, incl, off);
+        incl += lane >= off ? t : 0u;
+    }
+    __syncthreads();  // (the previous call's sums have been read)
+    if (lane == 31) {
+        s_w[wid] = incl;
+    }
+    __syncthreads();
+    u32 base = 0, tot = 0;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+        const u32 w = s_w[i];
+        base += i < wid ? w : 0u;
+        tot += w;
+    }
+    *total = tot;
+    return base + incl - v;
+}
+
+// Shared-memory map of a CTA, as 32-bit addresses and pointers.
+struct SpMap {
+    float* y;       // [slice] final values of this CTA's columns; local index = (column / 1024) * vt + column % vt
+    u32*   area;    // [kSpAreaCap] nucleus keys received (all CTAs) or 64-bit candidates (leader)
+    u32*   merged;  // [kSpBins] counts of the whole row, then their exclusive prefix
+    u32*   sub;     // [kSpSub / 2] pairs of 16-bit sub-bucket counters
+    u32*   hist;    // [kSpBins] counts of this CTA's columns, then cursors
+};
+
+struct SpShared {
+    float wsum[32];        // warp sums of the soft-max denominator, written by all CTAs
+    u32   max_key[kSpMaxN];
+    u32   area_n;          // entries received
+    u32   first_max;       // smallest column that holds the maximum
+    u32   best_tie;        // largest tie key of the columns that hold the maximum
+    u32   n_cls;           // columns of the crossing class
+    u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
+    u32   p_sel, j_sel;    // crossing: probability (bits), rank inside its class
+    u32   bad_order;
+    float agg[(kSpMaxN * kSpAreaCap) / 256];
+};
+
+// Loads this CTA's columns of row r and stores their values after temperature and bias.
+template<int DT>
+__device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, const char* rowp, float* y, int rank, int lgvt,
+                                              int nchunk)
+{
+    constexpr int ES = DT == FTB200_F32 ? 4 : 2, EPV = 16 / ES, LGE = DT == FTB200_F32 ? 2 : 3;
+    const int     tid = threadIdx.x, vt = 1 << lgvt, col0 = rank << lgvt, vocab = P.vocab;
+    if (((size_t)rowp & 15) == 0 && lgvt >= LGE) {
+        // a chunk of 1024 columns starts on a 16-byte boundary: whole vectors, four in flight per thread
+        constexpr int U   = 4;
+        const int     lgv = lgvt - LGE, nv = nchunk << lgv;
+        for (int i0 = tid; i0 < nv; i0 += kThreads * U) {
+            uint4 q[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * kThreads, v = ((i >> lgv) << 10) + col0 + ((i & ((1 << lgv) - 1)) << LGE);
+                if (i < nv && v + EPV <= vocab) {
+                    q[u] = ld_nc_v4(rowp + (size_t)v * ES);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * kThreads, v = ((i >> lgv) << 10) + col0 + ((i & ((1 << lgv) - 1)) << LGE);
+                if (i >= nv) {
+                    continue;
+                }
+                float f[EPV];
+                if (v + EPV <= vocab) {
+#pragma unroll
+                    for (int e = 0; e < EPV; ++e) {
+                        f[e] = temp_value<DT>(X, raw_bits<DT>(q[u], e), v + e);
+                    }
+                }
+                else {
+#pragma unroll
+                    for (int e = 0; e < EPV; ++e) {
+                        f[e] = -INFINITY;
+                        if (v + e < vocab) {
+                            const u32 bits = DT == FTB200_F32 ? __ldg((const u32*)rowp + v + e) :
+                                                                (u32)__ldg((const unsigned short*)rowp + v + e);
+                            f[e]           = temp_value<DT>(X, bits, v + e);
+                        }
+                    }
+                }
+                float4* dst = (float4*)(y + ((size_t)i << LGE));
+#pragma unroll
+                for (int e = 0; e < EPV; e += 4) {
+                    dst[e / 4] = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+                }
+            }
+        }
+    }
+    else {
+        // a row that starts between two 16-byte boundaries: one column per load, eight in flight
+        constexpr int U  = 8;
+        const int     ny = nchunk << lgvt;
+        for (int i0 = tid; i0 < ny; i0 += kThreads * U) {
+            u32 q[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
+                q[u]        = 0;
+                if (i < ny && v < vocab) {
+                    q[u] = DT == FTB200_F32 ? __ldg((const u32*)rowp + v) : (u32)__ldg((const unsigned short*)rowp + v);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
+                if (i < ny) {
+                    y[i] = v < vocab ? temp_value<DT>(X, q[u], v) : -INFINITY;
+                }
+            }
+        }
+    }
+}
+
+// History ids of the row that this CTA looks after, kHistRegs per thread: loaded before the row itself so that they are
+// there when the bit maps are ready.  (-1: a padding position or none.)
+constexpr int kHistRegs = 2;
+__device__ __forceinline__ int sp_history_id(const KParams& P, size_t col, int input_len, int t)
+{
+    // sampling_penalty_kernels.cu:385-410
+    return (t < P.step && !(t >= input_len && t < P.max_input_len)) ? P.output_ids[(size_t)t * P.batch_size + col] : -1;
+}
+
+// Marks the special columns of the row in the bit maps of the CTAs that own them: history ids (map 0) and banned words /
+// the masked end token (map 1).  The CTAs of the cluster share the work.
+template<int LGN>
+__device__ __noinline__ void sp_mark_specials(const KParams& P, int r, u32 bits_addr, int words, int rank, int id0, int id1)
+{
+    constexpr int n = 1 << LGN, lgvt = 10 - LGN;
+    const int     tid = threadIdx.x;
+    const size_t  col = (size_t)P.ite * P.local_batch + r;
+    auto          mark = [&](int v, int map) {
+        if (v < 0 || v >= P.vocab) {
+            return;
+        }
+        const int local = ((v >> 10) << lgvt) | (v & ((1 << lgvt) - 1));
+        dred_or(cluster_addr(bits_addr + 4u * (u32)(map * words + (local >> 5)), (u32)((v & 1023) >> lgvt)), 1u << (local & 31));
+    };
+    if (P.apply_rep) {
+        const int input_len = P.input_lengths != nullptr ? P.input_lengths[r] : P.max_input_len;
+        mark(id0, 0);
+        mark(id1, 0);
+        for (int t = (kHistRegs * n + rank) * kThreads + tid; t < P.step; t += n * kThreads) {
+            mark(sp_history_id(P, col, input_len, t), 0);
+        }
+    }
+    if (P.bad_words != nullptr) {
+        // a word bans its last token when the tokens before it match the tail of the sequence (ban_bad_words.cu:35-85)
+        const int  L     = P.bad_words_len;
+        const int* wbase = P.bad_words_shared ? P.bad_words : P.bad_words + (size_t)r * 2 * L;
+        for (int i = rank * kThreads + tid; i < L; i += n * kThreads) {
+            const int end = wbase[L + i];
+            if (end < 0) {
+                continue;
+            }
+            const int start = i > 0 ? wbase[L + i - 1] : 0, size = end - start;
+            const int tok   = wbase[end - 1];
+            bool      ban   = size == 1;
+            if (size > 1 && P.step >= size - 1) {
+                ban = true;
+                for (int j = size - 2; j >= 0 && ban; --j) {
+                    ban = P.output_ids[(size_t)(P.step - (size - 1) + j) * P.batch_size + col] == wbase[start + j];
+                }
+            }
+            if (ban && tok > 0) {
+                mark(tok, 1);
+            }
+        }
+    }
+    if (P.apply_minlen && rank == 0 && tid == 0 && P.seq_len[r] + 1 - P.max_input_len < P.min_lengths[r]) {
+        mark(P.end_ids[r], 1);  // sampling_penalty_kernels.cu:493-499
+    }
+}
+
+template<int DT>
+__device__ __forceinline__ float sp_prob(float y, float maxv, float denom)
+{
+    return round_to_T<DT>(round_to_T<DT>(__expf(y - maxv)) / denom);
+}
+
+// Ordered pieces of the soft-max denominator: this CTA's virtual threads (columns modulo 1024) add their exponentials
+// in chunk order, the butterfly over 32 of them follows, and the warp sums go to every CTA of the cluster.
+template<int DT, int LGN>
+__device__ __noinline__ void sp_chain_sums(const float* y, int nchunk, float maxv, u32 wsum_addr, int rank)
+{
+    constexpr int n = 1 << LGN, lgvt = 10 - LGN;
+    FTB_ASSUME_SHARED(y);
+    const int tid = threadIdx.x, vt = 1 << lgvt;
+    for (int t = tid; t < vt; t += kThreads) {
+        float a = 0.0f;
+        int   m = 0;
+        for (; m + 8 <= nchunk; m += 8) {
+            float e[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                e[i] = round_to_T<DT>(__expf(y[((m + i) << lgvt) + t] - maxv));
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                a += e[i];
+            }
+        }
+        for (; m < nchunk; ++m) {
+            a += round_to_T<DT>(__expf(y[(m << lgvt) + t] - maxv));
+        }
+        // (vt is a multiple of 32: whole warps take part)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a = a + __shfl_xor_sync(0xffffffffu, a, o);
+        }
+        if ((tid & 31) == 0) {
+            const u32 w = (u32)(((rank << lgvt) + t) >> 5);
+#pragma unroll
+            for (int q = 0; q < n; ++q) {
+                dst_u32(cluster_addr(wsum_addr + 4u * w, (u32)q), __float_as_uint(a));
+            }
+        }
+    }
+}
+
+// Per-thread walk over the CTA's values: f(local index, value) for every column that can be selected and is not below
+// thr.  Four vectors of four are in flight per thread; one compare rules a vector out.
+template<class F>
+__device__ __forceinline__ void sp_sweep(const float* y, int ny, float neg_max, float thr, F&& f)
+{
+    FTB_ASSUME_SHARED(y);
+    constexpr int U = 4;
+    for (int i0 = 4 * (int)threadIdx.x; i0 < ny; i0 += 4 * kThreads * U) {
+        float4 v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int i = i0 + q * 4 * kThreads;
+            v[q]        = i < ny ? *(const float4*)(y + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const float m = fmaxf(fmaxf(v[q].x, v[q].y), fmaxf(v[q].z, v[q].w));
+            if (m >= thr && m > neg_max) {
+                const int i = i0 + q * 4 * kThreads;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float x = e == 0 ? v[q].x : (e == 1 ? v[q].y : (e == 2 ? v[q].z : v[q].w));
+                    if (x >= thr && x > neg_max) {
+                        f(i + e, x);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Counts of the CTA's selectable columns per bin.
+static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float neg_max, float maxv, u32 hist)
+{
+    FTB_ASSUME_SHARED(y);
+    constexpr int U = 4;
+    for (int i0 = 4 * (int)threadIdx.x; i0 < ny; i0 += 4 * kThreads * U) {
+        float4 v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int i = i0 + q * 4 * kThreads;
+            v[q]        = i < ny ? *(const float4*)(y + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float x = e == 0 ? v[q].x : (e == 1 ? v[q].y : (e == 2 ? v[q].z : v[q].w));
+                const u32   a = hist + 4u * (u32)sp_bin(maxv - x);
+                if (x > neg_max) {
+                    reds_add(a, 1u);
+                }
+            }
+        }
+    }
+}
+
+// One nucleus owner's keys (fp32 values, any order) into descending order; n <= kSpAreaCap - 64.  `excl` holds the first
+// position of every bin in the row's order, `place` is scratch for one word per bin.  A key's place inside its bin is
+// guessed from its position between the bin's edges, so that a sub-bucket of four places receives four keys on average
+// whatever the distribution is; a bin of eight keys or more shares no sub-bucket with its neighbours (two runs of equal
+// 16-bit values in one sub-bucket would take quadratic time).  Sub-buckets that come out unsorted are finished by one
+// thread each.  Returns false when a long sub-bucket would have to be ordered.
+static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* place, u32 start, int n, float maxv)
+{
+    constexpr int PER = kSpAreaCap / kThreads;    // keys per thread: 20
+    constexpr int BPT = kSpBins / kThreads;       // bins per thread: 8
+    constexpr int WPT = kSpSub / 2 / kThreads;    // words of two 16-bit sub-bucket counters per thread: 5
+    FTB_ASSUME_SHARED(a);
+    FTB_ASSUME_SHARED(sub);
+    FTB_ASSUME_SHARED(excl);
+    FTB_ASSUME_SHARED(place);
+    const int tid = threadIdx.x;
+    for (int i = tid; i < kSpSub / 2; i += kThreads) {
+        sub[i] = 0;
+    }
+    {
+        // sub-buckets a bin takes: its keys one after the other with padding around a large bin
+        u32 c[BPT], mine = 0, tot;
+#pragma unroll
+        for (int i = 0; i < BPT; ++i) {
+            const int b  = tid * BPT + i;
+            const u32 e0 = excl[b], e1 = b + 1 < kSpBins ? excl[b + 1] : start + (u32)n;
+            c[i]         = (e0 >= start && e0 < start + (u32)n) ? e1 - e0 : 0u;
+            c[i] += c[i] >= 8u ? 8u : 0u;
+            mine += c[i];
+        }
+        u32 run = block_excl_u32(mine, &tot);
+#pragma unroll
+        for (int i = 0; i < BPT; ++i) {
+            place[tid * BPT + i] = run + (c[i] >= 16u ? 4u : 0u);
+            run += c[i];
+        }
+    }
+    __syncthreads();
+    // The keys arrive bin by bin: the 32 lanes of a warp take theirs from 32 places far apart, or they would all count
+    // in the same sub-bucket.
+    const int seg = ((n + 31) / 32) | 1;
+    float     v[PER];
+    u32       at[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int q = i * kThreads + tid, p = (q >> 5) < seg ? (q & 31) * seg + (q >> 5) : n;
+        at[i]       = 0xffffffffu;
+        v[i]        = 0.0f;
+        if (i * kThreads < 32 * seg && p < n) {
+            v[i]          = a[p];
+            const float t = sp_pos(maxv - v[i]);
+            const int   b = (int)t;
+            const u32   c = (b + 1 < kSpBins ? excl[b + 1] : start + (u32)n) - excl[b];
+            u32         o = (u32)((t - (float)b) * (float)c);
+            o             = c > 0 && o >= c ? c - 1u : o;
+            u32 s         = (place[b] + o) >> 2;
+            s             = s < (u32)kSpSub ? s : (u32)kSpSub - 1u;
+            const u32 old = atomicAdd(&sub[s >> 1], 1u << (16 * (s & 1u)));
+            at[i]         = (s << 16) | ((old >> (16 * (s & 1u))) & 0xffffu);
+        }
+    }
+    __syncthreads();
+    {
+        u32 c[WPT], mine = 0, tot;
+#pragma unroll
+        for (int i = 0; i < WPT; ++i) {
+            c[i] = sub[tid * WPT + i];
+            mine += (c[i] & 0xffffu) + (c[i] >> 16);
+        }
+        u32 run = block_excl_u32(mine, &tot);
+#pragma unroll
+        for (int i = 0; i < WPT; ++i) {
+            sub[tid * WPT + i] = run | ((run + (c[i] & 0xffffu)) << 16);
+            run += (c[i] & 0xffffu) + (c[i] >> 16);
+        }
+    }
+    __syncthreads();
+    auto first_of = [&](int s) { return s < kSpSub ? (int)((sub[s >> 1] >> (16 * (s & 1))) & 0xffffu) : n; };
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        if (i * kThreads < 32 * seg && at[i] != 0xffffffffu) {
+            a[first_of((int)(at[i] >> 16)) + (int)(at[i] & 0xffffu)] = v[i];
+        }
+    }
+    __syncthreads();
+    // a sub-bucket of equal values (16-bit logits have many) is in order already; the others are short.  Where two
+    // neighbours stand the wrong way round is noted first, so that a long run of equal values is not walked.
+    __shared__ u32 s_wrong[kSpAreaCap / 32];
+    __shared__ u32 s_long[64], s_nlong;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int p = i * kThreads + tid;
+        if (i * kThreads < n) {
+            const u32 m = __ballot_sync(0xffffffffu, p + 1 < n && a[p] < a[p + 1]);
+            if ((tid & 31) == 0) {
+                s_wrong[p >> 5] = m;
+            }
+        }
+    }
+    if (tid == 0) {
+        s_nlong = 0;
+    }
+    __syncthreads();
+    bool ok = true;
+    for (int s = tid; s < kSpSub; s += kThreads) {
+        const int lo = first_of(s), hi = first_of(s + 1);
+        if (hi - lo < 2) {
+            continue;
+        }
+        // bits lo .. hi - 2
+        const int w0 = lo >> 5, w1 = (hi - 2) >> 5;
+        bool      wrong = false;
+        for (int w = w0; w <= w1; ++w) {
+            u32 m = s_wrong[w];
+            m &= w == w0 ? 0xffffffffu << (lo & 31) : 0xffffffffu;
+            m &= w == w1 ? 0xffffffffu >> (31 - ((hi - 2) & 31)) : 0xffffffffu;
+            wrong |= m != 0;
+        }
+        if (!wrong) {
+            continue;
+        }
+        if (hi - lo > 12) {
+            const u32 slot = atomicAdd(&s_nlong, 1u);
+            if (slot < 64u && hi - lo <= 512) {
+                s_long[slot] = (u32)s;
+            }
+            else {
+                ok = false;
+            }
+            continue;
+        }
+        for (int i = lo + 1; i < hi; ++i) {
+            const float x = a[i];
+            int         j = i - 1;
+            while (j >= lo && a[j] < x) {
+                a[j + 1] = a[j];
+                --j;
+            }
+            a[j + 1] = x;
+        }
+    }
+    ok = __syncthreads_and(ok) != 0;
+    // A long sub-bucket holds few distinct values (a run of equal ones with a penalised column's beside it): a warp takes
+    // the largest value left, writes it as often as it occurs, and goes on.
+    const int lane = tid & 31;
+    for (u32 w = (u32)(tid >> 5); ok && w < s_nlong; w += kWarps) {
+        const int lo = first_of((int)s_long[w]), m = first_of((int)s_long[w] + 1) - lo;
+        u32       k[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            k[i] = i * 32 + lane < m ? fkey(a[lo + i * 32 + lane]) : 0u;
+        }
+        __syncwarp();
+        u32 below = 0xffffffffu;
+        for (int at_pos = 0; at_pos < m;) {
+            u32 top = 0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                top = k[i] < below && k[i] > top ? k[i] : top;
+            }
+            top     = __reduce_max_sync(0xffffffffu, top);
+            u32 cnt = 0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                cnt += k[i] == top ? 1u : 0u;
+            }
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            if (cnt == 0) {
+                break;
+            }
+            for (int i = lane; i < (int)cnt; i += 32) {
+                a[lo + at_pos + i] = fkey_inv(top);
+            }
+            at_pos += (int)cnt;
+            below = top;
+        }
+    }
+    __syncthreads();
+    return ok;
+}
+
+// First bin whose inclusive count reaches `want` (kSpBins - 1 when the total stays below) with, for half, a
+// probability at its far edge that cannot round to the one at `p_floor`.
+template<bool MIND_P>
+static __device__ int sp_bin_reaching(const u32* excl, u32 total, u32 want, float p_below, float inv_denom)
+{
+    __shared__ int s_b;
+    constexpr int  PER = kSpBins / kThreads;
+    const int      tid = threadIdx.x;
+    FTB_ASSUME_SHARED(excl);
+    __syncthreads();
+    if (tid == 0) {
+        s_b = kSpBins - 1;
+    }
+    __syncthreads();
+    int found = kSpBins;
+    for (int i = PER - 1; i >= 0; --i) {
+        const int b    = tid * PER + i;
+        const u32 incl = b + 1 < kSpBins ? excl[b + 1] : total;
+        bool      ok   = incl >= want;
+        if (MIND_P) {
+            ok = ok && __expf(-sp_edge(b)) * inv_denom <= p_below;
+        }
+        found = ok ? b : found;
+    }
+    if (found < kSpBins) {
+        atomicMin(&s_b, found);
+    }
+    __syncthreads();
+    return s_b;
+}
+
+// The nucleus scan of the reference (topp_sampling: cub::BlockScan<float, 256> in raking order, 256 sorted
+// probabilities per chunk, sampling_topp_kernels.cu:877-1004) over keys that lie in the areas of `owners` CTAs.
+struct SpKeys {
+    u32 area;            // 32-bit address of the area in this CTA
+    int owners;
+    u32 start[kSpMaxN + 1];  // first position of every owner, then the total
+};
+__device__ __forceinline__ float sp_key_at(const SpKeys& K, u32 pos)
+{
+    int o = 0;
+    while (o + 1 < K.owners && pos >= K.start[o + 1]) {
+        ++o;
+    }
+    return __uint_as_float(dld_u32(cluster_addr(K.area + 4u * (pos - K.start[o]), (u32)o)));
+}
+__device__ __forceinline__ void sp_load8(const SpKeys& K, u32 c, int lane, float* x)
+{
+    const u32 total = K.start[K.owners], p0 = c * 256u + (u32)lane * 8u;
+    int       o = 0;
+    while (o + 1 < K.owners && p0 >= K.start[o + 1]) {
+        ++o;
+    }
+    if (p0 + 8u <= K.start[o + 1]) {
+        const u32 base = cluster_addr(K.area + 4u * (p0 - K.start[o]), (u32)o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            x[i] = __uint_as_float(dld_u32(base + 4u * (u32)i));
+        }
+    }
+    else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            x[i] = p0 + (u32)i < total ? sp_key_at(K, p0 + (u32)i) : 0.0f;
+        }
+    }
+}
+// inclusive sum of the lane's eight values and the Kogge-Stone scan of the lane totals
+__device__ __forceinline__ float sp_rake(const float* x, int lane)
+{
+    float up = x[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        up = up + x[i];
+    }
+    float inc = up;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) {
+            inc = inc + t;
+        }
+    }
+    return inc;
+}
+
+// Warp 0 of the leader: running prefix over the chunk aggregates, the crossing inside its chunk, the crossing's
+// probability and its rank among the equal ones.  Returns the verdict (see SpShared).
+static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float* agg, float rand_num, bool complete, u32* p_out,
+                                                    u32* j_out)
+{
+    FTB_ASSUME_SHARED(agg);
+    const int lane = threadIdx.x & 31;
+    const u32 N    = K.start[K.owners];
+    const int nch  = (int)((N + 255u) / 256u);
+    // chunk by chunk, as the reference's prefix functor accumulates; stopped a little early (inside a chunk the partial
+    // sums differ from prefix + aggregate in the last bits only)
+    const float stop = rand_num * (1.0f - 1e-4f);
+    float       R    = 0.0f;
+    int         c1   = nch;
+    for (int c = 0; c < nch; ++c) {
+        const float R2 = R + agg[c];
+        if (R2 >= stop) {
+            c1 = c;
+            break;
+        }
+        R = R2;
+    }
+    int sel = -1;
+    for (int c = c1; c < nch; ++c) {
+        float x[8];
+        sp_load8(K, (u32)c, lane, x);
+        const float inc = sp_rake(x, lane);
+        const float ag  = __shfl_sync(0xffffffffu, inc, 31);
+        const float ex  = __shfl_up_sync(0xffffffffu, inc, 1);
+        float       o   = lane == 0 ? R : R + ex;
+        u32         cnt = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            o = o + x[i];
+            cnt += rand_num <= o ? 1u : 0u;
+        }
+        // a warp of the reference covers 4 of these lanes (32 consecutive probabilities)
+        u32 c4 = cnt;
+        c4 += __shfl_xor_sync(0xffffffffu, c4, 1);
+        c4 += __shfl_xor_sync(0xffffffffu, c4, 2);
+        const u32 any = __ballot_sync(0xffffffffu, c4 > 0);
+        if (any) {
+            const int g  = (__ffs(any) - 1) >> 2;
+            const u32 pc = __shfl_sync(0xffffffffu, c4, g * 4);
+            sel          = c * 256 + g * 32 + (32 - (int)pc);
+            if (!complete && (u32)(c * 256 + g * 32 + 31) >= N) {
+                return 2;  // the 32 probabilities of that warp are not all known
+            }
+            break;
+        }
+        R = R + ag;
+    }
+    if (sel < 0 || (u32)sel >= N) {
+        if (!complete || N == 0) {
+            return 2;
+        }
+        // the cumulative sum never reached the draw: the reference leaves the best token in place
+        *p_out = __float_as_uint(sp_key_at(K, 0));
+        *j_out = 0;
+        return 1;
+    }
+    const float p = sp_key_at(K, (u32)sel);
+    if (!complete && p == sp_key_at(K, N - 1)) {
+        return 2;  // the lowest class may have members that were not collected
+    }
+    // first position with this probability: 32 probes at a time
+    u32 lo = 0, hi = (u32)sel;  // the answer lies in [lo, hi]
+    while (lo < hi) {
+        const u32 span = hi - lo, step = (span + 31u) / 32u;
+        const u32 q    = lo + (u32)lane * step;
+        const bool eq  = q >= hi || sp_key_at(K, q) == p;
+        const u32 m    = __ballot_sync(0xffffffffu, eq);
+        const int f    = m != 0 ? __ffs(m) - 1 : 32;
+        const u32 nhi  = lo + (u32)f * step;
+        const u32 nlo  = f == 0 ? lo : lo + (u32)(f - 1) * step + 1u;
+        hi             = nhi < hi ? nhi : hi;
+        lo             = nlo < hi ? nlo : hi;
+    }
+    *p_out = __float_as_uint(p);
+    *j_out = (u32)sel - lo;
+    return 0;
+}
+
+// The leader's candidates (~key << 32 | column) into order.  The bins of the row are already counted: an entry goes to
+// its bin's range of the sorted list, and its place inside the range is the number of smaller entries there, a handful
+// unless many columns are equal.  Three barriers, where a sorting network takes tens.  `bin_of` gives an entry's bin.
+// Returns the sorted list (the second half of the candidate area); `excl` is used up.
+template<class B>
+static __device__ __forceinline__ u64* sp_bucket_sort(u64* cand, u32* excl, int n, u64* tmp, u64* dst, B&& bin_of)
+{
+    FTB_ASSUME_SHARED(cand);
+    FTB_ASSUME_SHARED(tmp);
+    FTB_ASSUME_SHARED(dst);
+    const int tid = threadIdx.x;
+    if (n <= 128) {
+        for (int i = tid; i < n; i += kThreads) {
+            const u64 e  = cand[i];
+            int       rk = 0;
+#pragma unroll 8
+            for (int j = 0; j < n; ++j) {
+                rk += cand[j] < e ? 1 : 0;
+            }
+            dst[rk] = e;
+        }
+        __syncthreads();
+        return dst;
+    }
+    for (int i = tid; i < n; i += kThreads) {
+        const u64 e                            = cand[i];
+        tmp[atomicAdd(&excl[bin_of(e)], 1u)] = e;  // the cursor of bin b ends at the start of bin b + 1
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += kThreads) {
+        const u64 e  = tmp[i];
+        const int b  = bin_of(e);
+        const int lo = b > 0 ? (int)excl[b - 1] : 0, hi = (int)excl[b];
+        int       rk = lo;
+#pragma unroll 4
+        for (int j = lo; j < hi; ++j) {
+            rk += tmp[j] < e ? 1 : 0;
+        }
+        dst[rk] = e;
+    }
+    __syncthreads();
+    return dst;
+}
+
+// Note of why a row is left to decode_sampling_kernel (word 25 of its trace record).
+__device__ __forceinline__ bool sp_leave(const RowOut& O, int why)
+{
+    if (O.trace != nullptr && threadIdx.x == 0) {
+        O.trace[4 + 25] = (u64)why;
+    }
+    return false;
+}
+
+// Result of a top-p row (one thread).
+template<int DT>
+__device__ __forceinline__ void sp_write_topp(const KParams& P, const RowOut& O, int id, float prob, bool drawn, bool want_lp)
+{
+    *O.id_out = id;
+    if (drawn) {
+        if (want_lp) {
+            const float lprob = logf(prob);
+            if (P.cum_log_probs != nullptr) {
+                P.cum_log_probs[O.r] += lprob;
+            }
+            if (P.out_log_probs != nullptr) {
+                P.out_log_probs[O.r] = lprob;
+            }
+        }
+        write_lengths(P, O, id);
+    }
+}
+
+// One row on the cluster.  Every branch that skips a cluster barrier depends on values that all CTAs hold alike.
+// Returns (leader only) whether the row is decided.
+template<int DT, int LGN>
+__device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, const SpMap& M, SpShared& X, const RowOut& O, int mode,
+                                       bool want_lp)
+{
+    __shared__ float s_u, s_denom;
+    __shared__ u32   s_start[kSpMaxN + 1], s_base[kSpMaxN + 1], s_rbase[kSpMaxN];
+    __shared__ u32   s_base1, s_cutbin;
+    const int        tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    constexpr int    n = 1 << LGN, lgvt = 10 - LGN;
+    const int        rank = (int)cluster_rank(), r = O.r;
+    const int        nchunk = (P.vocab + 1023) >> 10, ny = nchunk << lgvt;
+    float* const     y = M.y;
+    const bool       specials = P.apply_rep || P.bad_words != nullptr || P.apply_minlen;
+    const bool       softmax  = mode == 2 || want_lp;
+    const float      neg_max  = DT == FTB200_F16 ? -65504.0f : -FLT_MAX;
+    FTB_ASSUME_SHARED(y);
+
+    // ---- set-up: counters, the row's slice, special columns ----
+    const int words = ny >> 5;
+    u32*      bits  = M.area;  // [2][words] bit maps of the special columns
+    for (int i = tid; i < kSpBins; i += kThreads) {
+        M.hist[i] = 0;
+    }
+    if (specials) {
+        for (int i = tid; i < 2 * words; i += kThreads) {
+            bits[i] = 0;
+        }
+    }
+    if (tid == 0) {
+        X.area_n    = 0;
+        X.first_max = 0xffffffffu;
+        X.best_tie  = 0;
+        X.n_cls     = 0;
+        X.bad_order = 0;
+        curandState_t st = (mode == 1 ? P.topk_states : P.topp_states)[r];
+        s_u              = curand_uniform(&st);
+    }
+    __syncthreads();
+    cluster_arrive();  // this CTA's counters may be written by the others
+    Xf X0;
+    X0.bias       = P.bias;
+    X0.apply_temp = P.apply_temp;
+    X0.inv_t      = P.apply_temp ? 1.0f / (P.temperature[r] + 1e-6f) : 1.0f;
+    X0.inv_t_h    = __float2half_rn(X0.inv_t);
+    X0.theta      = P.apply_rep ? P.rep_penalty[r] : 1.0f;
+    X0.apply_rep = P.apply_rep, X0.penalty_type = P.penalty_type;
+    X0.vocab     = P.vocab;
+    const char* rowp = (const char*)P.logits + (size_t)r * P.vocab_padded * (DT == FTB200_F32 ? 4 : 2);
+    int         hist0 = -1, hist1 = -1;
+    if (P.apply_rep) {
+        const size_t col       = (size_t)P.ite * P.local_batch + r;
+        const int    input_len = P.input_lengths != nullptr ? P.input_lengths[r] : P.max_input_len;
+        hist0                  = sp_history_id(P, col, input_len, rank * kThreads + tid);
+        hist1                  = sp_history_id(P, col, input_len, (n + rank) * kThreads + tid);
+    }
+    sp_load_slice<DT>(P, X0, rowp, y, rank, lgvt, nchunk);
+    trace_mark(O.trace, 0);
+    cluster_wait();
+    if (specials) {
+        sp_mark_specials<LGN>(P, r, smem_addr(bits), words, rank, hist0, hist1);
+        cluster_sync();
+        for (int w = tid; w < words; w += kThreads) {
+            const u32 dead = bits[words + w];
+            u32       any  = bits[w] | dead;
+            while (any != 0) {
+                const int b = __ffs(any) - 1;
+                any &= any - 1;
+                const int i = w * 32 + b;
+                y[i]        = special_value<DT>(X0, y[i], (dead >> b) & 1u ? kFlagDead : kFlagHist);
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- row maximum ----
+    trace_mark(O.trace, 1);
+    float best = -INFINITY;
+    for (int i = 4 * tid; i < ny; i += 4 * kThreads) {
+        const float4 v = *(const float4*)(y + i);
+        best           = fmaxf(best, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+    }
+    {
+        const u32 k = (u32)block_max_u64((u64)(best > neg_max ? fkey(best) : 0u));
+        if (tid < n) {
+            dst_u32(cluster_addr(smem_addr(&X.max_key[rank]), (u32)tid), k);
+        }
+    }
+    cluster_sync();
+    u32 kmax = 0;
+    for (int q = 0; q < n; ++q) {
+        kmax = X.max_key[q] > kmax ? X.max_key[q] : kmax;
+    }
+    trace_mark(O.trace, 2);
+    const float u = s_u;
+    if (kmax == 0) {
+        // nothing can be selected: token 0
+        if (rank == 0 && tid == 0) {
+            *O.id_out = 0;
+            write_lengths(P, O, 0);
+        }
+        return true;
+    }
+    const float maxv = fkey_inv(kmax);
+    if (!(maxv < INFINITY)) {
+        return sp_leave(O, 1);
+    }
+
+    if (mode == 1 && !want_lp && P.topk_ks[r] <= 1u) {
+        // ---- arg-max: value, then the reference's tie order (CTA lane and thread descending, column ascending) ----
+        const u32 bs1 = P.max_top_k <= 16 ? 128 : 256;
+        const int sh1 = bs1 == 128 ? 7 : 8;
+        u32       tie = 0;
+        sp_sweep(y, ny, neg_max, maxv, [&](int i, float x) {
+            if (fkey(x) != kmax) {
+                return;  // (a zero of the other sign)
+            }
+            const u32 v = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
+            const u32 c = (((v >> sh1) & 7u) << 29) | ((v & (bs1 - 1)) << 21) | (0x1fffffu - v);
+            tie         = c > tie ? c : tie;
+        });
+        if (tie != 0) {
+            dred_max(cluster_addr(smem_addr(&X.best_tie), 0), tie);
+        }
+        cluster_sync();
+        if (rank == 0 && tid == 0) {
+            const int id = (int)(0x1fffffu - (X.best_tie & 0x1fffffu));
+            *O.id_out    = id;
+            write_lengths(P, O, id);
+        }
+        return true;
+    }
+
+    // ---- counts per bin; for a soft-max row the ordered denominator ----
+    sp_count_bins(y, ny, neg_max, maxv, smem_addr(M.hist));
+    trace_mark(O.trace, 3);
+    if (softmax) {
+        sp_chain_sums<DT, LGN>(y, nchunk, maxv, smem_addr(X.wsum), rank);
+    }
+    trace_mark(O.trace, 4);
+    cluster_sync();
+    trace_mark(O.trace, 16);
+    {
+        // this CTA adds its share of the bins over the cluster and hands the sums to everybody
+        constexpr int share = kSpBins >> LGN;
+        for (int i = tid; i < share; i += kThreads) {
+            const int b = rank * share + i;
+            const u32 a = smem_addr(&M.hist[b]), m = smem_addr(&M.merged[b]);
+            u32       part[n], sum = 0;
+#pragma unroll
+            for (int q = 0; q < n; ++q) {
+                part[q] = dld_u32(cluster_addr(a, (u32)q));
+            }
+#pragma unroll
+            for (int q = 0; q < n; ++q) {
+                sum += part[q];
+            }
+#pragma unroll
+            for (int q = 0; q < n; ++q) {
+                dst_u32(cluster_addr(m, (u32)q), sum);
+            }
+        }
+        if (softmax && wid == 0) {
+            float v = X.wsum[lane];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                v = v + __shfl_xor_sync(0xffffffffu, v, o);
+            }
+            if (lane == 0) {
+                s_denom = v + 1e-6f;
+            }
+        }
+    }
+    cluster_sync();
+    const float denom = softmax ? s_denom : 1.0f;
+    trace_mark(O.trace, 5);
+    if (softmax && !(denom > 0.0f && denom < INFINITY)) {
+        return sp_leave(O, 2);
+    }
+    constexpr int PER = kSpBins / kThreads;
+    u32           total;
+    float         mass = 0.0f;  // lower bound of this thread's bins' probability (top-p rows)
+    {
+        u32 c[PER], mine = 0;
+        const float scale = 0.99f / denom;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int b = tid * PER + i;
+            c[i]        = M.merged[b];
+            mine += c[i];
+            if (mode == 2 && c[i] != 0 && b + 1 < kSpBins) {
+                mass += (float)c[i] * __expf(-sp_edge(b + 1)) * scale;
+            }
+        }
+        u32 run = block_excl_u32(mine, &total);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            M.merged[tid * PER + i] = run;
+            run += c[i];
+        }
+    }
+    __syncthreads();
+    u32* const excl = M.merged;
+
+    trace_mark(O.trace, 6);
+    // ---- how far down the selection can reach: every column of bins 0 .. b_thr takes part ----
+    int         k = 1, b_thr;
+    float       rand_num = 0.0f;
+    if (mode == 1) {
+        k     = (int)P.topk_ks[r];
+        k     = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
+        b_thr = sp_bin_reaching<false>(excl, total, (u32)k, 0.0f, 0.0f);
+        if (want_lp) {
+            // equal probabilities may lie in different bins: a few more columns, so that the k-th is not in the last class
+            const u32 incl = b_thr + 1 < kSpBins ? excl[b_thr + 1] : total;
+            b_thr          = sp_bin_reaching<false>(excl, total, incl + 32u, 0.0f, 0.0f);
+        }
+    }
+    else {
+    const float top_p = P.topp_ps[r];
+    const float p_max = round_to_T<DT>(round_to_T<DT>(1.0f) / denom);
+    if (p_max >= top_p) {
+        // arg-max shortcut of topp_beam_topk_kernel (sampling_topp_kernels.cu:801-860): first column of the maximum
+        u32 col = 0xffffffffu;
+        sp_sweep(y, ny, neg_max, maxv, [&](int i, float v) {
+            if (v == maxv) {
+                const u32 c = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
+                col         = c < col ? c : col;
+            }
+        });
+        if (col != 0xffffffffu) {
+            dred_min(cluster_addr(smem_addr(&X.first_max), 0), col);
+        }
+        cluster_sync();
+        if (rank == 0 && tid == 0) {
+            sp_write_topp<DT>(P, O, (int)X.first_max, p_max, true, want_lp);
+        }
+        return true;
+    }
+    rand_num = u * top_p;
+    {
+        // first bin down to which the lower bound of the mass covers the draw
+        __shared__ float s_mw[kWarps];
+        float            incl = mass;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, incl, off);
+            incl += lane >= off ? t : 0.0f;
+        }
+        if (lane == 31) {
+            s_mw[wid] = incl;
+        }
+        if (tid == 0) {
+            s_cutbin = kSpBins - 1;
+        }
+        __syncthreads();
+        float base = 0.0f;
+        for (int i = 0; i < wid; ++i) {
+            base += s_mw[i];
+        }
+        if (base + incl >= rand_num) {
+            // (the bin inside the thread's eight is not looked for: the last of them is taken)
+            atomicMin(&s_cutbin, (u32)(tid * PER + PER - 1));
+        }
+        __syncthreads();
+        const int b_star = (int)s_cutbin;
+        // at least 64 columns more: the scan reads 32 entries past the crossing, and the crossing must not fall into
+        // the lowest collected class; half-precision probabilities are equal over several bins
+        const u32   have = b_star + 1 < kSpBins ? excl[b_star + 1] : total;
+        const float p_at = __expf(-sp_edge(b_star + 1)) / denom;
+        b_thr = sp_bin_reaching<DT == FTB200_F16>(excl, total, have + 64u, p_at * (1.0f - 1.0f / 512.0f) - 1.3e-7f, 1.0f / denom);
+    }
+    }
+    const bool complete = b_thr == kSpBins - 1;
+    const u32  N        = complete ? total : excl[b_thr + 1];
+    trace_mark(O.trace, 9);
+
+    if (N <= (u32)kSpCandCap) {
+        // ---- few candidates: the leader gets them all and finishes the row alone ----
+        // (a thread meets few candidates: the first four are remembered, more make it walk again)
+        u32         mine = 0, tot;
+        u64         keep0 = 0, keep1 = 0, keep2 = 0, keep3 = 0;
+        const float thr  = sp_floor_value(maxv, b_thr);
+        auto        entry = [&](int i, float v) {
+            const u32 col = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
+            return ((u64)(~fkey(v)) << 32) | col;
+        };
+        sp_sweep(y, ny, neg_max, thr, [&](int i, float v) {
+            if (sp_bin(maxv - v) <= b_thr) {
+                keep3 = keep2, keep2 = keep1, keep1 = keep0;
+                keep0 = entry(i, v);
+                ++mine;
+            }
+        });
+        u32 at = block_excl_u32(mine, &tot);
+        if (tid == 0) {
+            s_base1 = tot != 0 ? datom_add(cluster_addr(smem_addr(&X.area_n), 0), tot) : 0u;
+        }
+        __syncthreads();
+        if (mine != 0) {
+            const u32 dst = cluster_addr(smem_addr(M.area), 0) + 8u * (at + s_base1);
+            if (mine <= 4) {
+                dst_u64(dst, keep0);
+                if (mine > 1) {
+                    dst_u64(dst + 8, keep1);
+                }
+                if (mine > 2) {
+                    dst_u64(dst + 16, keep2);
+                }
+                if (mine > 3) {
+                    dst_u64(dst + 24, keep3);
+                }
+            }
+            else {
+                u32 w = 0;
+                sp_sweep(y, ny, neg_max, thr, [&](int i, float v) {
+                    if (sp_bin(maxv - v) <= b_thr) {
+                        dst_u64(dst + 8u * w, entry(i, v));
+                        ++w;
+                    }
+                });
+            }
+        }
+        cluster_sync();
+        trace_mark(O.trace, 7);
+        if (rank != 0) {
+            return true;
+        }
+        // (the leader's slice has been read for the last time: it is the sort's and the draw's scratch)
+        const int n_cand = (int)N;
+        auto      key_of = [&](u64 e) { return fkey_inv(~(u32)(e >> 32)); };
+        u64*      sorted = (u64*)M.area;
+        sorted = sp_bucket_sort(sorted, excl, n_cand, (u64*)M.y, n_cand <= 128 ? sorted + 1024 : sorted,
+                                [&](u64 e) { return sp_bin(maxv - key_of(e)); });
+        trace_mark(O.trace, 8);
+        Smem S;
+        S.cand = (u64*)M.area;
+        S.hist = (u32*)M.y;
+        S.val2 = (float*)(M.y + kNB);
+        if (!softmax) {
+            return topk_finish(P, S, O, sorted, n_cand, k, u, P.topk_ps[r], true, false);
+        }
+        // values -> probabilities; their order has to be that of the values
+        float* const pr  = (float*)M.merged;
+        bool         bad = false;
+        for (int i = tid; i < n_cand; i += kThreads) {
+            const u64   e = sorted[i];
+            const float q = sp_prob<DT>(key_of(e), maxv, denom);
+            pr[i]         = q;
+            sorted[i]     = ((u64)(~fkey(q)) << 32) | (u32)e;
+        }
+        __syncthreads();
+        for (int i = tid; i + 1 < n_cand; i += kThreads) {
+            bad |= pr[i] < pr[i + 1];
+        }
+        if (__syncthreads_or(bad)) {
+            return sp_leave(O, 3);
+        }
+        if (mode == 1) {
+            return topk_finish(P, S, O, sorted, n_cand, k, u, P.topk_ps[r], false, true, !complete);
+        }
+        __shared__ SpKeys s_K1;
+        __shared__ u32    s_res[3];
+        if (tid == 0) {
+            s_K1.area   = smem_addr(pr);
+            s_K1.owners = 1;
+        }
+        if (tid <= kSpMaxN) {
+            s_K1.start[tid] = tid == 0 ? 0u : N;
+        }
+        __syncthreads();
+        for (int c = wid; c * 256 < n_cand; c += kWarps) {
+            float x[8];
+            sp_load8(s_K1, (u32)c, lane, x);
+            const float inc = sp_rake(x, lane);
+            if (lane == 31) {
+                X.agg[c] = inc;
+            }
+        }
+        __syncthreads();
+        if (wid == 0) {
+            u32       p = 0, j = 0;
+            const u32 v = sp_find_crossing(s_K1, X.agg, rand_num, complete, &p, &j);
+            if (lane == 0) {
+                s_res[0] = v, s_res[1] = p, s_res[2] = j;
+            }
+        }
+        __syncthreads();
+        trace_mark(O.trace, 14);
+        if (s_res[0] == 2) {
+            return sp_leave(O, 4);
+        }
+        // equal probabilities stand in column order in the reference's stable sort
+        const float p_sel = __uint_as_float(s_res[1]);
+        const u32   key   = ~fkey(p_sel);
+        for (int i = tid; i < n_cand; i += kThreads) {
+            const u64 e = sorted[i];
+            if ((u32)(e >> 32) != key) {
+                continue;
+            }
+            u32 rk = 0;
+            int j  = i;
+            while (j > 0 && (u32)(sorted[j - 1] >> 32) == key) {
+                --j;
+                rk += sorted[j] < e ? 1u : 0u;
+            }
+            for (j = i + 1; j < n_cand && (u32)(sorted[j] >> 32) == key; ++j) {
+                rk += sorted[j] < e ? 1u : 0u;
+            }
+            if (rk == s_res[2]) {
+                sp_write_topp<DT>(P, O, (int)(u32)e, p_sel, s_res[0] == 0, want_lp);
+            }
+        }
+        return true;
+    }
+    if (mode == 1) {
+        return sp_leave(O, 5);
+    }
+
+    // ---- a large nucleus: sorted by several CTAs ----
+    int owners = (int)((N + 1023u) / 1024u);
+    owners     = owners < 1 ? 1 : (owners > n ? n : owners);
+    auto owner_of = [&](u32 e) { return (int)(((u64)e * (u32)owners) / N); };
+    {
+        // this CTA's counts become cursors into its own list, ordered by bin
+        u32 c[PER], mine = 0, ltot;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            c[i] = M.hist[tid * PER + i];
+            mine += c[i];
+        }
+        u32 run = block_excl_u32(mine, &ltot);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            M.hist[tid * PER + i] = run;
+            run += c[i];
+        }
+        __syncthreads();
+        if (tid <= kSpMaxN) {
+            s_start[tid] = tid == 0 ? 0u : N;
+            s_base[tid]  = tid == 0 ? 0u : (complete ? ltot : M.hist[b_thr + 1]);
+        }
+        __syncthreads();
+        for (int b = tid + 1; b <= b_thr; b += kThreads) {
+            // the first bin of an owner: where its keys start in the whole row's order and in this CTA's list
+            const int o = owner_of(excl[b]), before = owner_of(excl[b - 1]);
+            for (int q = before + 1; q <= o && q <= kSpMaxN; ++q) {
+                s_start[q] = excl[b];
+                s_base[q]  = M.hist[b];
+            }
+        }
+        __syncthreads();
+    }
+    __shared__ SpKeys s_K;
+    const SpKeys&     K = s_K;
+    if (tid == 0) {
+        s_K.area   = smem_addr(M.area);
+        s_K.owners = owners;
+    }
+    if (tid <= kSpMaxN) {
+        s_K.start[tid] = s_start[tid];
+    }
+    const bool fits = N > 0 && __syncthreads_and(tid >= kSpMaxN || s_start[tid + 1] - s_start[tid] <= (u32)kSpAreaCap - 64u);
+    if (!fits) {
+        return sp_leave(O, 4);
+    }
+    trace_mark(O.trace, 10);
+    // a range of every owner's area for this CTA's keys, then the keys (values: ordered like the probabilities)
+    if (tid < owners) {
+        const u32 cnt = s_base[tid + 1] - s_base[tid];
+        s_rbase[tid]  = cnt != 0 ? datom_add(cluster_addr(smem_addr(&X.area_n), (u32)tid), cnt) : 0u;
+    }
+    __syncthreads();
+    u32 first[n];  // first position of every owner after the leader
+#pragma unroll
+    for (int q = 1; q < n; ++q) {
+        first[q] = q < owners ? s_start[q] : 0xffffffffu;
+    }
+    sp_sweep(y, ny, neg_max, sp_floor_value(maxv, b_thr), [&](int, float v) {
+        const int b = sp_bin(maxv - v);
+        if (b <= b_thr) {
+            const u32 pos = atomicAdd(&M.hist[b], 1u), e = excl[b];
+            int       o = 0;
+#pragma unroll
+            for (int q = 1; q < n; ++q) {
+                o += e >= first[q] ? 1 : 0;
+            }
+            dst_u32(cluster_addr(K.area + 4u * (s_rbase[o] + pos - s_base[o]), (u32)o), __float_as_uint(v));
+        }
+    });
+    cluster_sync();
+    trace_mark(O.trace, 11);
+    if (rank < owners) {
+        float* const a   = (float*)M.area;
+        const int    cnt = (int)(s_start[rank + 1] - s_start[rank]);
+        bool         bad = !sp_sort_area(a, M.sub, excl, M.hist, s_start[rank], cnt, maxv);
+        for (int i = tid; i < cnt; i += kThreads) {
+            a[i] = sp_prob<DT>(a[i], maxv, denom);
+        }
+        __syncthreads();
+        // the exponential has to be monotone over the keys for their order to be the sorted order
+        for (int i = tid; i + 1 < cnt; i += kThreads) {
+            bad |= a[i] < a[i + 1];
+        }
+        if (__syncthreads_or(bad) && tid == 0) {
+            dst_u32(cluster_addr(smem_addr(&X.bad_order), 0), 1u);
+        }
+    }
+    if (owners > 1) {
+        cluster_sync();
+        if (rank > 0 && rank < owners && tid == 0 && s_start[rank + 1] > s_start[rank]
+            && sp_key_at(K, K.start[rank] - 1u) < ((const float*)M.area)[0]) {
+            dst_u32(cluster_addr(smem_addr(&X.bad_order), 0), 1u);
+        }
+    }
+    trace_mark(O.trace, 12);
+    if (rank < owners) {
+        // aggregates of the chunks that start in this owner's range
+        const u32 c0 = (s_start[rank] + 255u) >> 8, c1 = (s_start[rank + 1] + 255u) >> 8;
+        for (u32 c = c0 + (u32)wid; c < c1; c += kWarps) {
+            float x[8];
+            sp_load8(K, c, lane, x);
+            const float inc = sp_rake(x, lane);
+            if (lane == 31) {
+                dst_u32(cluster_addr(smem_addr(&X.agg[c]), 0), __float_as_uint(inc));
+            }
+        }
+    }
+    if (owners > 1) {
+        cluster_sync();
+    }
+    else {
+        __syncthreads();
+    }
+    trace_mark(O.trace, 13);
+    if (rank == 0 && wid == 0) {
+        u32 p = 0, j = 0, verdict = 2;
+        if (!X.bad_order) {
+            verdict = sp_find_crossing(K, X.agg, rand_num, complete, &p, &j);
+        }
+        if (lane < n) {
+            const u32 q = (u32)lane;
+            dst_u32(cluster_addr(smem_addr(&X.verdict), q), verdict);
+            dst_u32(cluster_addr(smem_addr(&X.p_sel), q), p);
+            dst_u32(cluster_addr(smem_addr(&X.j_sel), q), j);
+        }
+    }
+    cluster_sync();
+    const u32 verdict = X.verdict;
+    trace_mark(O.trace, 14);
+    if (verdict == 2) {
+        return sp_leave(O, 5);
+    }
+    // ---- columns whose probability is that of the crossing; the one of its rank is the id ----
+    const float p_sel = __uint_as_float(X.p_sel);
+    // (no column outside [y_lo, y_hi] has that probability: rounding of the exponential, the quotient and the logarithm,
+    // in half also of the two stored results, are allowed for)
+    const float slack = DT == FTB200_F16 ? 1.0f / 256.0f : 1e-4f, tiny = DT == FTB200_F16 ? 1.3e-7f * (1.0f + denom) : 0.0f;
+    const float e_sel = p_sel * denom, e_lo = e_sel * (1.0f - slack) - tiny, pad = 1e-4f + 2e-6f * fabsf(maxv);
+    const float y_lo  = e_lo > 1e-37f ? maxv + __logf(e_lo) * 1.00001f - pad : -INFINITY;
+    const float y_hi  = maxv + __logf(fmaxf(e_sel * (1.0f + slack) + tiny, 1e-37f)) * 0.99999f + pad;
+    sp_sweep(y, ny, neg_max, y_lo, [&](int i, float v) {
+        if (v <= y_hi && sp_prob<DT>(v, maxv, denom) == p_sel) {
+            const u32 pos = datom_add(cluster_addr(smem_addr(&X.n_cls), 0), 1u);
+            if (pos < (u32)kSpAreaCap) {
+                dst_u32(cluster_addr(K.area + 4u * pos, 0), (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1))));
+            }
+        }
+    });
+    cluster_sync();
+    if (rank != 0) {
+        return true;
+    }
+    const u32 n_cls = X.n_cls, j_sel = X.j_sel;
+    trace_mark(O.trace, 15);
+    if (n_cls > (u32)kSpAreaCap || j_sel >= n_cls) {
+        return sp_leave(O, 6);
+    }
+    const int id = n_cls == 1 ? (int)M.area[0] : select_jth_column(M.area, (int)n_cls, (int)j_sel, (u32*)M.y, P.vocab_padded);
+    if (tid == 0) {
+        sp_write_topp<DT>(P, O, id, p_sel, verdict == 0, want_lp);
+    }
+    return true;
+}
+
+// The step's stop criteria (stop words of row r, then - by the last row of the call - the length limit and the count of
+// finished rows over the batch), by the CTA that finished row r.  Same results as stop_criteria_kernel.
+static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const StopArgs& T, int r)
+{
+    __shared__ u32 s_last, s_sum;
+    const int      tid = threadIdx.x;
+    const size_t   row = (size_t)P.ite * P.local_batch + r;
+    __syncthreads();
+    if (T.stop_words != nullptr) {
+        const int* base = T.stop_words + (size_t)r * 2 * T.stop_words_len;
+        const int* offs = base + T.stop_words_len;
+        for (int i = tid; i < T.stop_words_len; i += kThreads) {
+            if (offs[i] < 0) {
+                continue;
+            }
+            const int start = i > 0 ? offs[i - 1] : 0, size = offs[i] - start;
+            if (P.step + 1 >= size
+                && tail_matches(P.output_ids, nullptr, base, start, size, P.step - (size - 1), (size_t)P.batch_size, row, 0, 1)) {
+                T.finished[row] = 1;
+            }
+        }
+        __syncthreads();
+    }
+    if (T.limit == nullptr) {
+        return;
+    }
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicAdd(T.arrived, 1u) == (u32)P.local_batch - 1u ? 1u : 0u;
+        s_sum  = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last == 0) {
+        return;
+    }
+    u32 mine = 0;
+    for (int i = tid; i < P.batch_size; i += kThreads) {
+        const uint8_t f = (uint8_t)(__ldcg(T.finished + i) | ((u32)P.step >= T.limit[i] ? 1 : 0));
+        T.finished[i]   = f;
+        mine += f ? 1u : 0u;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((tid & 31) == 0) {
+        atomicAdd(&s_sum, mine);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        *T.arrived = 0;
+        __threadfence_system();
+        *(volatile u64*)T.result = ((u64)T.sequence << 32) | s_sum;
+    }
+}
+
+// A row that the tables of the split form cannot hold, by the leader CTA alone.
+template<int DT>
+static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, unsigned char* smem, u64* rec)
+{
+    __shared__ Smem s_S;
+    Smem&           S = s_S;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        map_general_smem(P, S, smem);
+    }
+    __syncthreads();
+    process_row<DT>(P, S, r, P.scratch + (size_t)r * P.scratch_stride, rec);
+}
+
+// WHOLE: the kernel finishes every row itself (rows its tables cannot hold go through the general row code in the
+// leader CTA) and, when asked to, the step's stop criteria: one launch per decode step.  Taken while all rows are
+// resident at once; with more rows the general code's shared memory would cost residency, and the rows it is needed
+// for are left to decode_sampling_kernel.
+template<int DT, int LGN, bool WHOLE>
+__global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
+                                                                     const __grid_constant__ SplitArgs A)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ SpShared                           s_X;
+    __shared__ RowOut                             s_O;
+    SpMap                                         M;
+    M.y      = (float*)smem_raw;
+    M.area   = (u32*)(M.y + A.slice);
+    M.merged = M.area + kSpAreaCap;
+    M.sub    = M.merged + kSpBins;
+    M.hist   = M.sub + kSpSub / 2;
+    const int  tid = threadIdx.x, rank = (int)cluster_rank();
+    const bool want_lp = P.cum_log_probs != nullptr || P.out_log_probs != nullptr;
+    for (int t = (int)blockIdx.x >> LGN; t < P.local_batch; t += (int)gridDim.x >> LGN) {
+        const int r    = P.row_order != nullptr ? P.row_order[t] : t;
+        int       mode = 0;
+        if (P.topk_states != nullptr && !(P.topk_skip != nullptr && P.topk_skip[r])) {
+            mode = 1;
+        }
+        else if (P.topp_states != nullptr && !(P.topp_skip != nullptr && P.topp_skip[r])) {
+            mode = 2;
+        }
+        const bool fin = P.finished != nullptr ? P.finished[r] != 0 : false;
+        __syncthreads();  // (the previous row's record has been read)
+        if (tid == 0) {
+            s_O.r      = r;
+            s_O.end_id = P.end_ids[r];
+            s_O.id_out = P.output_ids + (size_t)P.step * P.batch_size + (size_t)P.ite * P.local_batch + r;
+            s_O.trace  = rank == 0 && P.trace != nullptr ? P.trace + (size_t)t * kTraceWords : nullptr;
+            if (s_O.trace != nullptr) {
+                s_O.trace[0] = (u64)r, s_O.trace[1] = (u64)blockIdx.x, s_O.trace[2] = global_timer_ns();
+            }
+        }
+        __syncthreads();
+        bool decided = true;
+        if (mode != 0 && !fin) {
+            decided = sp_row<DT, LGN>(P, A, M, s_X, s_O, mode, want_lp);
+            __syncthreads();
+        }
+        if (rank == 0 && tid == 0) {
+            if (decided) {
+                if (mode == 1 && fin) {
+                    *s_O.id_out = s_O.end_id;  // no draw, length unchanged (sampling_topk_kernels.cu:249-252)
+                }
+                else if (mode != 0) {
+                    const float u = draw_uniform(mode == 1 ? P.topk_states : P.topp_states, r);
+                    if (fin) {
+                        finished_topp_row<DT>(P, s_O, u, want_lp);
+                    }
+                }
+                topp_decay_row(P, r, *s_O.id_out);
+            }
+            if (!WHOLE) {
+                A.redo_flags[r] = decided ? 0 : 1;
+            }
+            if (s_O.trace != nullptr) {
+                s_O.trace[3] = global_timer_ns();
+            }
+        }
+        if (WHOLE && rank == 0) {
+            if (!decided) {
+                sp_whole_row<DT>(P, r, smem_raw, nullptr);
+            }
+            if (A.stop.stop_words != nullptr || A.stop.limit != nullptr) {
+                sp_stop_criteria(P, A.stop, r);
+            }
+        }
+    }
+    cluster_sync();  // no CTA leaves while another may still reach into its shared memory
+}
+
+template<int DT, int LGN, bool WHOLE>
+int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, cudaStream_t st)
+{
+    constexpr int     kMaxDev = 64;
+    static std::mutex mu;
+    static bool       opted_in[kMaxDev];
+    int               dev = 0;
+    FTB_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDev) {
+        set_error("ftb200_decode_step_sampling: device ordinal out of range");
+        return FTB200_UNSUPPORTED;
+    }
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!opted_in[dev]) {
+            FTB_CUDA_CHECK(cudaFuncSetAttribute(split_sampling_kernel<DT, LGN, WHOLE>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpMaxSmem));
+            opted_in[dev] = true;
+        }
+    }
+    cudaLaunchConfig_t  cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id               = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << LGN;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim              = dim3((unsigned)K.local_batch << LGN);
+    cfg.blockDim             = dim3(kThreads);
+    cfg.dynamicSmemBytes     = smem;
+    cfg.stream               = st;
+    cfg.attrs                = attr;
+    cfg.numAttrs             = 1;
+    FTB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_sampling_kernel<DT, LGN, WHOLE>, K, A));
+    return FTB200_OK;
+}
+
+// smem_general: shared memory of the general row code, for the form that keeps every row.
+template<int DT>
+int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_general, cudaStream_t st)
+{
+    const size_t smem = split_smem_bytes(A.slice);
+    if (A.redo_flags == nullptr) {
+        const size_t both = smem > smem_general ? smem : smem_general;
+        return A.lgn == 2 ? split_sampling_launch_n<DT, 2, true>(K, A, both, st) :
+                            split_sampling_launch_n<DT, 3, true>(K, A, both, st);
+    }
+    switch (A.lgn) {
+        case 1: return split_sampling_launch_n<DT, 1, false>(K, A, smem, st);
+        case 2: return split_sampling_launch_n<DT, 2, false>(K, A, smem, st);
+        default: return split_sampling_launch_n<DT, 3, false>(K, A, smem, st);
+    }
+}
+
+}  // namespace ftb200

@@ -10,10 +10,14 @@ import ctypes as C
 import numpy as np
 import torch
 
-from ._lib import BeamHyps, BeamParams, SamplingParams, check, lib
+from ._lib import BeamHyps, BeamParams, SamplingParams, StopParams, check, lib
 
 _DT = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 CURAND_STATE_BYTES = 48  # sizeof(curandState_t), XORWOW
+
+
+# the current stream's handle without a Stream object per call, where this torch has it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _ptr(t):
@@ -41,6 +45,7 @@ class DynamicDecodeLayer:
         self.dtype = dtype
         self.device = torch.device(device)
         self.stream = stream
+        self._device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self._workspace = None
         self._beam_ws = None
         self._gate = {}
@@ -48,12 +53,19 @@ class DynamicDecodeLayer:
         self.kernel_events = []
         self._count_dev = None
         self._count_host = None
+        self._stop = None
         self.launches = 0
 
     # ---- helpers -------------------------------------------------------------------------------
     def _stream_ptr(self):
-        s = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
-        return C.c_void_p(s.cuda_stream)
+        return C.c_void_p(self._raw_stream())
+
+    def _raw_stream(self):
+        if self.stream is not None:
+            return self.stream.cuda_stream
+        if _raw_stream is not None:
+            return _raw_stream(self._device_index)
+        return torch.cuda.current_stream(self.device).cuda_stream
 
     @staticmethod
     def _arg(args, key):
@@ -174,9 +186,10 @@ class DynamicDecodeLayer:
     # ---- forward (DynamicDecodeLayer.cc:191-474, sampling branch) ---------------------------------
     def forward(self, outputs, inputs):
         logits = inputs["logits"]
-        if logits.dim() == 3 and logits.shape[1] > 1:
+        shape = logits.shape
+        if len(shape) == 3 and shape[1] > 1:
             return self._forward_beam(outputs, inputs)
-        B = logits.shape[0]
+        B = shape[0]
         step = int(inputs["step"])
         ite = int(inputs.get("ite", 0))
         lbs = int(inputs.get("local_batch_size", B))
@@ -194,11 +207,35 @@ class DynamicDecodeLayer:
                 .to(self.device),
             }
         self._g = g
-        self._stream = self._stream_ptr()  # one look-up per call, used by the sampling and the criteria launch
-        topk_on, topp_on = g["topk_on"], g["topp_on"]
-        if topk_on or topp_on:
-            self._sample(outputs, inputs, logits, B, step, ite, lbs, mil, lo, hi, topk_on, topp_on)
-        return self._stop_criteria(outputs, inputs, B, step, lbs, lo)
+        self._stream = self._raw_stream()  # one look-up per call, used by the sampling and the criteria launch
+        if not (g["topk_on"] or g["topp_on"]):
+            return self._stop_criteria(outputs, inputs, B, step, lbs, lo)
+        P = self._fill(outputs, inputs, logits, B, step, ite, lbs, mil, lo)
+        sw = inputs.get("stop_words_list")
+        lim = inputs.get("sequence_limit_length")
+        if (sw is None and lim is None) or self.time_kernels or P.finished is None:
+            self._sample(P)
+            return self._stop_criteria(outputs, inputs, B, step, lbs, lo)
+        # sampling, stop criteria and the wait for should_stop in one call
+        S = self._stop
+        if S is None:
+            self._arrived = torch.zeros(1, dtype=torch.int32, device=self.device)
+            self._result = torch.zeros(1, dtype=torch.int64).pin_memory()
+            S = self._stop = StopParams()
+            S.arrived_dev, S.result_host = self._arrived.data_ptr(), self._result.data_ptr()
+            self._stop_ref, self._should_stop = C.byref(S), C.c_int(0)
+            self._should_stop_ref = C.byref(self._should_stop)
+        if sw is None:
+            S.stop_words, S.stop_words_len = None, 0
+        else:
+            L = sw.shape[-1]
+            S.stop_words, S.stop_words_len = sw.data_ptr() + lo * 2 * L * 4, L
+        S.sequence_limit_length = None if lim is None else lim.data_ptr()
+        rc = lib.ftb200_decode_step(g["params_ref"], self._stop_ref, 10000, self._should_stop_ref)
+        if rc:
+            check(rc)
+        self.launches += lib.ftb200_last_launch_count()
+        return bool(self._should_stop.value)
 
     # ---- beam search branch (DynamicDecodeLayer.cc:286-386 -> OnlineBeamSearchLayer::forward) -------
     def _forward_beam(self, outputs, inputs):
@@ -208,7 +245,8 @@ class DynamicDecodeLayer:
         ite = int(inputs.get("ite", 0))
         lbs = int(inputs.get("local_batch_size", B))
         mil = int(inputs["max_input_length"])
-        st = self._stream = self._stream_ptr()
+        self._stream = self._raw_stream()
+        st = C.c_void_p(self._stream)
         es = logits.element_size()
         out_ids = outputs["output_ids"]
         L = out_ids.shape[0]
@@ -296,7 +334,7 @@ class DynamicDecodeLayer:
             self._count_dev = torch.zeros(1, dtype=torch.int32, device=self.device)
             self._count_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         L = 0 if sw is None else sw.shape[-1]
-        st = getattr(self, "_stream", None) or self._stream_ptr()
+        st = C.c_void_p(self._stream)
         check(lib.ftb200_stop_criteria(
             _ptr(outputs["output_ids"]), _ptr(outputs.get("parent_ids")),
             None if sw is None else C.c_void_p(sw.data_ptr() + lo * 2 * L * 4), L, _ptr(outputs["finished"]),
@@ -309,14 +347,15 @@ class DynamicDecodeLayer:
         check(lib.ftb200_wait_should_stop(C.c_void_p(self._count_host.data_ptr()), B, beam, st, 10000, C.byref(stop)))
         return bool(stop.value)
 
-    def _sample(self, outputs, inputs, logits, B, step, ite, lbs, mil, lo, hi, topk_on, topp_on):
+    def _fill(self, outputs, inputs, logits, B, step, ite, lbs, mil, lo):
+        """The argument block of a slice.  It is kept between steps: what setup() fixed (the layer's own buffers, the
+        launch order, the slice) is written once, the caller's pointers when one of them changes, the step's own
+        values every time."""
         Vp = self.vocab_size_padded
-        es = logits.element_size()
-
-        # The argument block of a slice is kept between steps: what setup() fixed (the layer's own buffers, the
-        # launch order, the slice) is written once, the step's own values every time.
-        P = self._g.get("params")
-        if P is None or self._g["params_key"] != (B, lbs, ite, topk_on, topp_on):
+        g = self._g
+        P = g.get("params")
+        if P is None or g["params_key"] != (B, lbs, ite):
+            topk_on, topp_on = g["topk_on"], g["topp_on"]
             P = SamplingParams()
             P.batch_size, P.local_batch_size, P.ite = B, lbs, ite
             P.vocab_size, P.vocab_size_padded = self.vocab_size, Vp
@@ -338,50 +377,53 @@ class DynamicDecodeLayer:
                 P.topp_decay = self.topp.decay.data_ptr() + lo * 4
                 P.topp_min = self.topp.min.data_ptr() + lo * 4
                 P.topp_reset_ids = self.topp.reset.data_ptr() + lo * 4
-            P.row_order = self._g["order"].data_ptr()
-            self._g["params"], self._g["params_key"] = P, (B, lbs, ite, topk_on, topp_on)
-        P.dtype = _DT[logits.dtype]
-        P.step, P.max_input_length = step, mil
-        P.logits = logits.data_ptr() + lo * Vp * es
-        bias = inputs.get("embedding_bias")
-        P.embedding_bias = None if bias is None else bias.data_ptr()
-        P.end_ids = inputs["end_id"].data_ptr() + lo * 4
-        il = inputs.get("input_lengths")
-        P.input_lengths = None if il is None else il.data_ptr() + lo * 4
-        P.output_ids = outputs["output_ids"].data_ptr()
-        bw = inputs.get("bad_words_list")
-        if bw is not None:
-            shared = bw.dim() == 2 or bw.shape[0] == 1
-            L = bw.shape[-1]
-            P.bad_words = bw.data_ptr() if shared else bw.data_ptr() + lo * 2 * L * 4
-            P.bad_words_len, P.bad_words_shared = L, int(shared)
-        else:
-            P.bad_words, P.bad_words_len, P.bad_words_shared = None, 0, 0
-        # host-side gating of the penalty kernels (BaseSamplingLayer.cc:302-349)
-        P.apply_temperature = int(bias is not None or self._g["temp"])
-        P.apply_repetition = int(step > 1 and self.penalty_type != 2 and self._g["pen"])
-        P.apply_min_length = int(self._g["minlen"] > step - mil)
-
-        def sl(key, width):
-            t = outputs.get(key)
-            return None if t is None else t.data_ptr() + lo * width
-
-        P.sequence_length = sl("sequence_length", 4)
-        P.finished = sl("finished", 1)
-        P.cum_log_probs = sl("cum_log_probs", 4)
-        olp = outputs.get("output_log_probs")
-        # [request_output_len, batch] sliced at (step - max_input_length) (DynamicDecodeLayer.cc:427-435)
-        P.output_log_probs = None if olp is None else olp.data_ptr() + ((step - mil) * B + lo) * 4
-
-        if self._workspace is None or self._ws_key != (P.dtype, lbs, Vp):
-            need = C.c_size_t(0)
-            check(lib.ftb200_sampling_workspace_bytes(P.dtype, lbs, Vp, C.byref(need)))
-            if self._workspace is None or self._workspace.numel() < need.value:
-                self._workspace = torch.empty(need.value, dtype=torch.uint8, device=self.device)
-            self._ws_key = (P.dtype, lbs, Vp)
+            P.row_order = g["order"].data_ptr()
+            g["params"], g["params_key"], g["params_ref"], g["ptrs"] = P, (B, lbs, ite), C.byref(P), None
+        P.step = step
+        P.logits = logits.data_ptr() + lo * Vp * logits.element_size()
+        bias, il, bw = inputs.get("embedding_bias"), inputs.get("input_lengths"), inputs.get("bad_words_list")
+        seq, fin = outputs.get("sequence_length"), outputs.get("finished")
+        cum, olp = outputs.get("cum_log_probs"), outputs.get("output_log_probs")
+        ptrs = (logits.dtype, mil, inputs["end_id"].data_ptr(), outputs["output_ids"].data_ptr(), self._stream,
+                None if bias is None else bias.data_ptr(), None if il is None else il.data_ptr(),
+                None if bw is None else (bw.data_ptr(), bw.shape), None if seq is None else seq.data_ptr(),
+                None if fin is None else fin.data_ptr(), None if cum is None else cum.data_ptr())
+        if ptrs != g["ptrs"]:
+            P.dtype = _DT[logits.dtype]
+            P.max_input_length = mil
+            P.embedding_bias = None if bias is None else bias.data_ptr()
+            P.end_ids = inputs["end_id"].data_ptr() + lo * 4
+            P.input_lengths = None if il is None else il.data_ptr() + lo * 4
+            P.output_ids = outputs["output_ids"].data_ptr()
+            if bw is not None:
+                shared = bw.dim() == 2 or bw.shape[0] == 1
+                L = bw.shape[-1]
+                P.bad_words = bw.data_ptr() if shared else bw.data_ptr() + lo * 2 * L * 4
+                P.bad_words_len, P.bad_words_shared = L, int(shared)
+            else:
+                P.bad_words, P.bad_words_len, P.bad_words_shared = None, 0, 0
+            P.apply_temperature = int(bias is not None or g["temp"])
+            P.sequence_length = None if seq is None else seq.data_ptr() + lo * 4
+            P.finished = None if fin is None else fin.data_ptr() + lo
+            P.cum_log_probs = None if cum is None else cum.data_ptr() + lo * 4
+            if self._workspace is None or self._ws_key != (P.dtype, lbs, Vp):
+                need = C.c_size_t(0)
+                check(lib.ftb200_sampling_workspace_bytes(P.dtype, lbs, Vp, C.byref(need)))
+                if self._workspace is None or self._workspace.numel() < need.value:
+                    self._workspace = torch.empty(need.value, dtype=torch.uint8, device=self.device)
+                self._ws_key = (P.dtype, lbs, Vp)
+            P.stream = self._stream
+            g["ptrs"] = ptrs
         P.workspace = self._workspace.data_ptr()
         P.workspace_bytes = self._workspace.numel()
-        P.stream = self._stream.value
+        # host-side gating of the penalty kernels (BaseSamplingLayer.cc:302-349)
+        P.apply_repetition = int(step > 1 and self.penalty_type != 2 and g["pen"])
+        P.apply_min_length = int(g["minlen"] > step - mil)
+        # [request_output_len, batch] sliced at (step - max_input_length) (DynamicDecodeLayer.cc:427-435)
+        P.output_log_probs = None if olp is None else olp.data_ptr() + ((step - mil) * B + lo) * 4
+        return P
+
+    def _sample(self, P):
         if self.time_kernels:
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
@@ -389,5 +431,5 @@ class DynamicDecodeLayer:
             e1.record()
             self.kernel_events.append((e0, e1))
         else:
-            check(lib.ftb200_decode_step_sampling(C.byref(P)))
+            check(lib.ftb200_decode_step_sampling(self._g["params_ref"]))
         self.launches += lib.ftb200_last_launch_count()

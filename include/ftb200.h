@@ -175,19 +175,21 @@ int ftb200_last_launch_count(void);
 /* Diagnostic, no counterpart in the reference: when `device_buf` is not null every later
  * ftb200_decode_step_sampling call writes records of 32 uint64 each, {row, CTA, start, end, 28 phase marks}
  * with the times in nanoseconds of the GPU's global timer (a mark the row did not pass is left untouched).
- * With R = local_batch_size the record of the single-pass top-k kernel's ticket t lies at device_buf[32 t..],
- * the general kernel's at device_buf[32 (R + t)..] and the single-pass top-p kernel's at
+ * With R = local_batch_size the record of the single-pass top-k kernel's ticket t lies at device_buf[32 t..] (the split
+ * kernel's row t likewise), the general kernel's at device_buf[32 (R + t)..] and the single-pass top-p kernel's at
  * device_buf[32 (2 R + t)..]: the buffer must hold 3 * 256 bytes per row of the call.  Pass null to switch the
  * trace off (the default). */
 int ftb200_set_row_trace(uint64_t* device_buf);
 
-/* Diagnostic, no counterpart in the reference.  ftb200_decode_step_sampling serves 16-bit logits of at least
- * 16400 columns (no embedding bias, no log-probabilities) in up to three launches: a single-pass kernel for the
- * top-p rows and one for the top-k rows side by side (one read of each row for a top-k row, several rows in
- * flight per SM), then the general kernel on the rows those two leave behind; ftb200_vocab_parallel_local does
- * the same with the top-k rows' kernel in its record form.  ftb200_set_single_pass(0) sends every row to the
- * general kernel (the results are the same either way; tests compare the two); 1 (the default) restores the
- * single-pass kernels.  Process-wide. */
+/* Diagnostic, no counterpart in the reference.  ftb200_decode_step_sampling serves a call by one of three routes.
+ * Small batches, and all calls with fp32 logits, an embedding bias or log-probabilities, take the split kernel: a row
+ * over a cluster of two to eight CTAs.  Larger batches of 16-bit logits of at least 16400 columns take up to three
+ * launches: a single-pass kernel for the top-p rows and one for the top-k rows side by side (one read of each row for
+ * a top-k row, several rows in flight per SM), then the general kernel on the rows those two leave behind;
+ * ftb200_vocab_parallel_local does the same with the top-k rows' kernel in its record form.  The general kernel alone
+ * serves what neither can (under 1024 columns, above 352256).  ftb200_set_single_pass(0) sends every row to the
+ * general kernel (the results are the same either way; tests compare them); 1 (the default) restores the others.
+ * Process-wide. */
 int ftb200_set_single_pass(int on);
 
 /* ------------------------------------------------------------------------------------------
@@ -219,6 +221,29 @@ int ftb200_stop_criteria(const int* output_ids, const int* parent_ids, const int
  * that) and reports *should_stop = (finished_count_host[0] == batch_size*beam_width). */
 int ftb200_wait_should_stop(const int* finished_count_host, int batch_size, int beam_width, void* stream,
                             int timeout_ms, int* should_stop);
+
+/* ------------------------------------------------------------------------------------------
+ * A whole step of the sampling path in one call: ftb200_decode_step_sampling, then the stop criteria above for
+ * beam width 1, then - when a length limit is given - the wait for "is the whole batch done".  Small batches take a
+ * single kernel launch for all of it; the count reaches the host through a word in page-locked memory that the
+ * step's last kernel stores, so the wait ends with that kernel.  p->finished is required.
+ *   stop_words, sequence_limit_length   as in ftb200_stop_criteria (device; null: not wanted)
+ *   arrived_dev   one 32-bit device word, zero before the first call; every call leaves it zero
+ *   result_host   one 64-bit word of page-locked host memory the device can reach (cudaHostAlloc, cudaHostRegister)
+ *   sequence      counts the calls on this block (in/out); the word holds sequence << 32 | finished rows afterwards
+ * A block serves one call at a time.  *should_stop = 1 when all batch_size rows are finished; FTB200_TIMEOUT after
+ * timeout_ms (negative: no deadline).
+ * ------------------------------------------------------------------------------------------ */
+typedef struct ftb200_stop_params {
+    const int*      stop_words;
+    int             stop_words_len;
+    const uint32_t* sequence_limit_length;
+    uint32_t*       arrived_dev;
+    uint64_t*       result_host;
+    uint32_t        sequence;
+} ftb200_stop_params;
+
+int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_params* s, int timeout_ms, int* should_stop);
 
 /* ------------------------------------------------------------------------------------------
  * The fused decode-sampling step without a caller-provided workspace.

@@ -1,0 +1,71 @@
+"""The split decode-sampling kernel (a row over a cluster of CTAs) against the general kernel, which the other tests pin
+to the CPU restatement and the reference: everything a step writes has to be the same, bit for bit.  The sizes are the
+edges of its split: chunks of 1024 columns, two / four / eight CTAs per row, rows that start between two 16-byte
+boundaries, the largest slice, one row, and batches either side of "all rows resident"."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
+
+
+def run(general, dtype, V, Vp, B, ties, log_probs, device):
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    rng = np.random.default_rng(V + B)
+    g = torch.Generator(device=device)
+    g.manual_seed(V * 7 + B)
+    step, mil = 40, 32
+    ids = torch.randint(1, V, (step + 4, B), generator=g, device=device, dtype=torch.int32)
+    st = {"output_ids": ids, "finished": torch.zeros(B, dtype=torch.bool, device=device),
+          "sequence_length": torch.full((B,), step, dtype=torch.int32, device=device)}
+    st["finished"][B // 2:B // 2 + 1] = B > 2
+    if log_probs:
+        st["cum_log_probs"] = torch.zeros(B, device=device)
+        st["output_log_probs"] = torch.zeros(step + 4 - mil, B, device=device)
+    args = {"runtime_top_k": rng.choice(np.asarray([0, 1, 7, 1024], np.uint32), size=B),
+            "runtime_top_p": rng.choice(np.asarray([0.3, 0.9, 0.99], np.float32), size=B),
+            "temperature": rng.choice(np.asarray([0.7, 1.0], np.float32), size=B),
+            "repetition_penalty": rng.choice(np.asarray([0.8, 1.2], np.float32), size=B),
+            "min_length": rng.choice(np.asarray([0, 30], np.int32), size=B),
+            "random_seed": np.arange(B).astype(np.uint64)}
+    words = torch.from_numpy(np.tile(np.asarray([[[3, 5, 6, 9], [1, 3, 4, -1]]], np.int32), (B, 1, 1))).to(device)
+    lim = torch.full((B,), step + 2, dtype=torch.int32, device=device)
+    layer = DynamicDecodeLayer(V, Vp, dtype, device)
+    layer.setup(B, 1, args)
+    lib.ftb200_set_single_pass(0 if general else 1)
+    stops = []
+    try:
+        for s in range(3):
+            x = torch.randn(B, Vp, generator=g, device=device) * 2.5
+            x[::2, rng.integers(0, V, 3)] += 9.0
+            if ties:
+                x = (x * 4).round() / 4
+            x[1::5, ::2] = -float("inf")
+            stop = layer.forward(st, {"logits": x.to(dtype), "step": step + s, "max_input_length": mil, "ite": 0,
+                                      "local_batch_size": B, "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=device),
+                                      "input_lengths": torch.full((B,), mil - 3, dtype=torch.int32, device=device),
+                                      "bad_words_list": words, "stop_words_list": words, "sequence_limit_length": lim})
+            stops.append(bool(stop))
+        torch.cuda.synchronize()
+    finally:
+        lib.ftb200_set_single_pass(1)
+    out = {k: v.cpu().numpy() for k, v in st.items()}
+    out["curand"] = np.concatenate([layer.topk.curand.cpu().numpy(), layer.topp.curand.cpu().numpy()])
+    out["stops"] = np.asarray(stops)
+    return out
+
+
+@pytest.mark.parametrize("dtype,V,Vp,B,ties,log_probs", [
+    (F32, 1024, 1024, 1, False, False), (F32, 1025, 1032, 5, True, True), (F16, 2047, 2047, 3, False, True),
+    (BF16, 40960, 40960, 37, True, False), (F16, 40961, 40963, 38, False, False), (F32, 16384, 16384, 74, False, True),
+    (F32, 16385, 16388, 75, True, False), (BF16, 32000, 32000, 150, False, False), (BF16, 65537, 65543, 20, True, False),
+    (F32, 128256, 128256, 9, False, False), (F32, 128256, 128256, 40, True, True), (BF16, 128257, 128257, 4, False, True),
+    (F32, 350208, 350208, 3, False, False), (F32, 352257, 352260, 2, False, False)])
+def test_split_kernel_equals_general_kernel(dtype, V, Vp, B, ties, log_probs, cuda_device):
+    want = run(True, dtype, V, Vp, B, ties, log_probs, cuda_device)
+    got = run(False, dtype, V, Vp, B, ties, log_probs, cuda_device)
+    for k, v in want.items():
+        np.testing.assert_array_equal(got[k], v, err_msg=k)
+    assert want["stops"].tolist() == [False, False, True]
