@@ -9,6 +9,8 @@
 // tile in shared memory, and the CTA writes results back with coalesced stores.
 #include <limits.h>
 
+#include <mutex>
+
 #include "common.cuh"
 #include "ftb200.h"
 
@@ -192,6 +194,284 @@ __global__ void __launch_bounds__(kDkThreads) gather_tree_kernel(GatherTree p)
     }
 }
 
+// ---- parent chains in parallel ----------------------------------------------------------------------------
+// A level's parents map a beam to a beam, and maps compose: the levels are cut into segments, every segment finds
+// where each of its K possible entries comes out (all segments at once), a short walk over the segments gives every
+// beam its entry, and the segments are walked again, now writing.  Three walks of about sqrt(levels) dependent
+// shared-memory reads instead of one of `levels` (2048 levels x 4 beams: 5 us, against 60).
+// `par` [levels][K + 1]: byte offset (2 x beam) of each beam's parent within its row; the last entry of a row stands for
+// "no parent" and leads to itself, so that a step of a walk is one add and one shared-memory read.  `sel` [levels][K]
+// receives the beam that beam j's chain passes at each level below its start (K: none); `start` / `from`: the level
+// above which beam j's chain begins and its beam there (K: none).
+struct Chains {
+    u32 par, sel, comp, entry;  // 32-bit shared-memory addresses; comp, entry: [segments][K + 1], [segments][K]
+    u32 start, from;            // [K] ints
+    int K, levels, seglen, segments;
+};
+constexpr int kChainThreads  = 1024;
+constexpr int kChainSegments = 64;
+
+__device__ __forceinline__ u32 lds_u16(u32 a)
+{
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_u16(u32 a, u32 v)
+{
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+}
+
+__device__ __forceinline__ void walk_chains(const Chains& c)
+{
+    const int tid = threadIdx.x, K = c.K, W = K + 1;
+    const u32 row = 2u * (u32)W;
+    for (int e = tid; e < c.segments * W; e += kChainThreads) {
+        const int seg = e / W, lo = seg * c.seglen, hi = min(lo + c.seglen, c.levels);
+        u32       cur = 2u * (u32)(e % W), at = c.par + (u32)hi * row;
+        for (int i = lo; i < hi; ++i) {
+            at -= row;
+            cur = lds_u16(at + cur);
+        }
+        sts_u16(c.comp + 2u * (u32)e, cur);
+    }
+    __syncthreads();
+    for (int j = tid; j < K; j += kChainThreads) {
+        const int top = (int)lds_u32(c.start + 4u * (u32)j);
+        u32       cur = 2u * lds_u32(c.from + 4u * (u32)j);
+        int       seg = top > 0 ? (top - 1) / c.seglen : -1;
+        if (seg >= 0) {
+            sts_u16(c.entry + 2u * (u32)(seg * K + j), cur);
+            const int lo = seg * c.seglen;  // the chain starts inside this segment
+            for (int level = top - 1; level >= lo; --level) {
+                cur = lds_u16(c.par + (u32)level * row + cur);
+            }
+            for (--seg; seg >= 0; --seg) {
+                sts_u16(c.entry + 2u * (u32)(seg * K + j), cur);
+                cur = lds_u16(c.comp + (u32)seg * row + cur);
+            }
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < c.segments * K; e += kChainThreads) {
+        const int seg = e / K, j = e % K, lo = seg * c.seglen, top = (int)lds_u32(c.start + 4u * (u32)j);
+        const int hi  = min(min(lo + c.seglen, c.levels), top);
+        if (lo < hi) {
+            u32 cur = lds_u16(c.entry + 2u * (u32)e), at = c.par + (u32)hi * row, out = c.sel + 2u * (u32)(hi * K + j);
+            for (int i = lo; i < hi; ++i) {
+                at -= row;
+                out -= 2u * (u32)K;
+                sts_u16(out, cur >> 1);
+                cur = lds_u16(at + cur);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+__host__ __device__ inline int chain_segments(int levels, int K)
+{
+    int s = 1;
+    while (s * s < levels && s < kChainSegments && (s + 1) * (K + 1) <= kChainThreads) {
+        ++s;
+    }
+    return s;
+}
+inline size_t chain_smem_bytes(int levels, int K)
+{
+    return (size_t)levels * (2 * K + 1) * 2 + (size_t)chain_segments(levels, K) * (2 * K + 1) * 2 + 64;
+}
+// Tables of an entry behind each other in dynamic shared memory.
+__device__ __forceinline__ Chains map_chains(void* smem, int levels, int K, const int* start, const int* from)
+{
+    Chains c;
+    c.K = K, c.levels = levels;
+    c.segments = chain_segments(levels, K);
+    c.seglen   = levels > 0 ? (levels + c.segments - 1) / c.segments : 1;
+    c.par      = (u32)__cvta_generic_to_shared(smem);
+    c.sel      = c.par + 2u * (u32)(levels * (K + 1));
+    c.comp     = c.sel + 2u * (u32)(levels * K);
+    c.entry    = c.comp + 2u * (u32)(c.segments * (K + 1));
+    c.start    = (u32)__cvta_generic_to_shared(start);
+    c.from     = (u32)__cvta_generic_to_shared(from);
+    return c;
+}
+constexpr size_t kChainMaxSmem = 200 * 1024;
+
+// The tree with the whole parent table of an entry in shared memory.  Bound by latency: 8 levels of ids and parents in
+// flight per thread, then the chains, then one pass that writes and one that cuts and transposes.
+// 64 entries x 4 beams x 2048 levels: 245 us with one thread per chain, 17 us this way.
+__global__ void __launch_bounds__(kChainThreads) gather_tree_chains_kernel(GatherTree p)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int     s_start[kMaxBeams], s_from[kMaxBeams], s_first[kMaxBeams];
+    __shared__ uint8_t s_bad[kMaxBeams];
+    __shared__ int     s_maxlen, s_uneven;
+
+    const int    b = blockIdx.x, K = p.beam_width, tid = threadIdx.x;
+    const size_t BK = (size_t)p.batch_size * K, col0 = (size_t)b * K;
+    const int    max_input_length = p.input_lengths == nullptr ? 0 : p.max_input_length;
+    const int    prompt_len = p.prefix_lengths == nullptr ? 0 : p.prefix_lengths[b];
+    const int    virt = p.virtual_lengths == nullptr ? 0 : p.virtual_lengths[b];
+    const int    trimmed = p.max_prefix_length + (p.max_input_length - p.max_input_without_prompt_length);
+    const int    end = p.end_tokens[b];
+    auto         at = [&](int time, int beam) { return BK * (size_t)time + col0 + beam; };
+    auto         in_len = [&](int beam) { return (p.input_lengths == nullptr ? 0 : p.input_lengths[col0 + beam]) - virt; };
+
+    if (tid == 0) {
+        s_maxlen = -1;
+        s_uneven = 0;
+    }
+    __syncthreads();
+    // (one update of the lengths per entry: see gather_tree_kernel)
+    for (int j = tid; j < K; j += kChainThreads) {
+        const int tmp_len                = p.max_sequence_lengths[col0 + j] + p.final_step;
+        p.max_sequence_lengths[col0 + j] = tmp_len - trimmed;
+        if (p.response_input_lengths != nullptr) {
+            p.response_input_lengths[col0 + j] = in_len(j) - prompt_len;
+        }
+        atomicMax(&s_maxlen, tmp_len);
+        if (in_len(j) != in_len(0)) {
+            s_uneven = 1;
+        }
+    }
+    __syncthreads();
+    const int max_len = s_maxlen, top = min(p.max_time, max_len);
+    if (top <= 0) {
+        return;
+    }
+    const int levels = top - 1;  // levels below the beam's own last token
+    auto      skipped = [&](int level, int len) { return level < prompt_len || (level >= len && level < max_input_length); };
+    const Chains c = map_chains(smem, levels, K, s_start, s_from);
+    const u32    row = 2u * (u32)(K + 1);
+    // every thread keeps to one beam (no division in the loops) and takes every step-th level or position of it
+    const int  step = kChainThreads / K, j = tid % K, t0 = tid / K;
+    const bool busy = t0 < step;
+    const int  len = in_len(j), len0 = in_len(0), shift = max_input_length - len + prompt_len;
+    if (busy) {
+#pragma unroll 8
+        for (int level = t0; level < levels; level += step) {
+            int v              = p.parent_ids == nullptr ? 0 : __ldg(p.parent_ids + at(level, j));
+            v                  = (unsigned)v < (unsigned)K ? v : v % K;
+            v                  = s_uneven == 0 && skipped(level, len0) ? j : (v < 0 ? K : v);  // a skipped level passes on
+            sts_u16(c.par + (u32)level * row + 2u * (u32)j, 2u * (u32)v);
+            if (j == 0) {
+                sts_u16(c.par + (u32)level * row + 2u * (u32)K, 2u * (u32)K);
+            }
+        }
+    }
+    for (int k = tid; k < K; k += kChainThreads) {
+        const int v = p.parent_ids == nullptr ? 0 : p.parent_ids[at(top - 1, k)] % K;
+        s_start[k]  = levels;
+        s_from[k]   = v < 0 ? K : v;
+        s_bad[k]    = 0;
+        s_first[k]  = INT_MAX;
+    }
+    __syncthreads();
+    if (s_uneven == 0) {
+        walk_chains(c);
+    }
+    else {
+        // beams of different prompt lengths skip different levels: one chain after the other
+        for (int k = tid; k < K; k += kChainThreads) {
+            const int lk  = in_len(k);
+            int       cur = s_from[k];
+            for (int level = levels - 1; level >= 0; --level) {
+                sts_u16(c.sel + 2u * (u32)(level * K + k), (u32)cur);
+                if (!skipped(level, lk)) {
+                    cur = (int)lds_u16(c.par + (u32)level * row + 2u * (u32)cur) / 2;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    // Position t of the beam: end tokens after the sequence, else the token of the level that lands there (levels of the
+    // prompt first, then the generated ones, then the beam's own last token), else what the caller left.  Where a chain
+    // broke off everything below is the end token, and the cut after the first end token is left out.
+    const int     first_t = max_input_length == 0 ? 1 : max_input_length;
+    const int     fill = max(0, max_len - shift), fill_end = p.max_time - p.max_prefix_length;
+    const int     out_len = p.max_time - trimmed;
+    constexpr int U = 8, R = 2;  // positions in flight, batches of them kept in registers
+    int           v[R][U];
+    auto          batch = [&](int t1, int* w) {
+        bool put[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = t1 + u * step;
+            put[u]      = false;
+            if (t < p.max_time) {
+                const int la = t + prompt_len, lb = t + shift;
+                int       level = lb < levels && lb >= max_input_length && lb >= prompt_len ? lb : -1;
+                level           = la < levels && la < max_input_length && la < len ? la : level;
+                const int from  = level >= 0 ? (int)lds_u16(c.sel + 2u * (u32)(level * K + j)) : j;
+                level           = level < 0 && t == top - 1 - shift ? top - 1 : level;
+                put[u]          = true;
+                if ((t >= fill && t < fill_end) || (level >= 0 && from == K)) {
+                    w[u] = end;
+                    if (level >= 0 && from == K) {
+                        s_bad[j] = 1;
+                    }
+                }
+                else if (level >= 0) {
+                    w[u] = __ldg(p.step_ids + at(level, from));
+                }
+                else {
+                    put[u] = false;
+                    w[u]   = p.beams[at(t, j)];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = t1 + u * step;
+            if (put[u]) {
+                p.beams[at(t, j)] = w[u];
+            }
+            if (t < p.max_time && t >= first_t && t < top && w[u] == end) {
+                atomicMin(&s_first[j], t);
+            }
+        }
+    };
+    if (busy) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            batch(t0 + r * U * step, v[r]);
+        }
+        for (int t1 = t0 + R * U * step; t1 < p.max_time; t1 += U * step) {
+            int w[U];
+            batch(t1, w);
+        }
+    }
+    __syncthreads();
+    // nothing but end tokens after the first one, and the transposed copy (each thread meets what it wrote itself)
+    if (busy) {
+        const int cut_from = s_bad[j] || s_first[j] == INT_MAX ? INT_MAX : s_first[j];
+        int*      out = p.output_ids == nullptr ? nullptr : p.output_ids + (col0 + j) * (size_t)out_len;
+        auto      finish = [&](int t, int w) {
+            const bool cut = t > cut_from && t < top;
+            if (cut) {
+                p.beams[at(t, j)] = end;
+            }
+            if (out != nullptr && t < out_len) {
+                out[t] = cut ? end : w;
+            }
+        };
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int t = t0 + (r * U + u) * step;
+                if (t < p.max_time) {
+                    finish(t, v[r][u]);
+                }
+            }
+        }
+        for (int t = t0 + R * U * step; t < p.max_time; t += step) {
+            finish(t, p.beams[at(t, j)]);
+        }
+    }
+}
+
 // ---- finalize ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kDkThreads) finalize_kernel(int* output_ids, int* sequence_lengths,
                                                               float* cum_log_probs, float* output_log_probs,
@@ -225,14 +505,14 @@ __global__ void __launch_bounds__(kDkThreads) finalize_kernel(int* output_ids, i
         }
     }
     __syncthreads();
-    for (int beam = tid; beam < K; beam += kDkThreads) {
+    for (int beam = tid; blockIdx.y == 0 && beam < K; beam += kDkThreads) {
         const size_t src = (size_t)b * 2 * K + s_rank[beam];
         sequence_lengths[(size_t)b * K + beam] = topk_sequence_lengths[src];
         if (cum_log_probs != nullptr) {
             cum_log_probs[(size_t)b * K + beam] = topk_cum_log_probs[src];
         }
     }
-    for (int beam = 0; beam < K; ++beam) {
+    for (int beam = blockIdx.y; beam < K; beam += gridDim.y) {
         const size_t src = ((size_t)b * 2 * K + s_rank[beam]) * (size_t)(max_seq_len + 1);
         const size_t dst = ((size_t)b * K + beam) * (size_t)max_seq_len;
         const int    len = topk_sequence_lengths[(size_t)b * 2 * K + s_rank[beam]];
@@ -349,6 +629,113 @@ __global__ void __launch_bounds__(kDkThreads) insert_unfinished_path_kernel(Inse
     }
 }
 
+// The archive with the whole parent table of an entry in shared memory (see walk_chains).
+__global__ void __launch_bounds__(kChainThreads) insert_chains_kernel(InsertPath p)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_start[kMaxArchiveBeams], s_from[kMaxArchiveBeams];
+    __shared__ int s_top;
+
+    const int b = blockIdx.x, K = p.beam_width, tid = threadIdx.x;
+    if (p.is_done[b]) {
+        return;
+    }
+    const size_t BK = (size_t)p.batch_size * K, col0 = (size_t)b * K;
+    const int    first_slot = p.num_beams[b];
+    const size_t row = (size_t)p.max_seq_len + 1;
+    const bool   with_lp = p.log_probs_tgt != nullptr && p.log_probs_src != nullptr;
+    if (tid == 0) {
+        s_top = 0;
+    }
+    __syncthreads();
+    for (int beam = tid; beam < K; beam += kChainThreads) {
+        const int    len = p.sequence_lengths_src[col0 + beam];
+        const size_t tgt = (size_t)b * 2 * K + beam + first_slot;
+        const size_t g   = (size_t)len * BK + col0 + beam;
+        p.output_ids_tgt[tgt * row + len] = p.output_ids_src[g];
+        if (with_lp) {
+            p.log_probs_tgt[tgt * row + len] = p.log_probs_src[g];
+        }
+        s_start[beam]               = min(len, p.max_seq_len);
+        s_from[beam]                = min(max(p.parent_ids_src[g], 0), K - 1);  // the reference follows it unchecked
+        p.sequence_lengths_tgt[tgt] = len;
+        const float cum   = p.cum_log_probs[col0 + beam];
+        const int   n_tok = p.finished[col0 + beam] ? len + 1 : len;
+        p.normed_scores[tgt] =
+            (p.length_penalty == 0.0f || n_tok == 1) ? cum : cum / powf((float)n_tok, p.length_penalty);
+        p.cum_log_probs_tgt[tgt] = cum;
+        atomicMax(&s_top, s_start[beam]);
+    }
+    __syncthreads();
+    const int    levels = s_top;
+    const Chains c = map_chains(smem, levels, K, s_start, s_from);
+    const u32    row_bytes = 2u * (u32)(K + 1);
+    const int  step = kChainThreads / K, j = tid % K, t0 = tid / K;  // one beam per thread, every step-th level of it
+    const bool busy = t0 < step;
+    if (busy) {
+#pragma unroll 8
+        for (int level = t0; level < levels; level += step) {
+            const int v = min(max(__ldg(p.parent_ids_src + BK * (size_t)level + col0 + j), 0), K - 1);
+            sts_u16(c.par + (u32)level * row_bytes + 2u * (u32)j, 2u * (u32)v);
+            if (j == 0) {
+                sts_u16(c.par + (u32)level * row_bytes + 2u * (u32)K, 2u * (u32)K);
+            }
+        }
+    }
+    __syncthreads();
+    walk_chains(c);
+    if (busy) {
+        const size_t tgt = ((size_t)b * 2 * K + j + first_slot) * row;
+        const int    n = s_start[j];
+        constexpr int U = 8;
+        for (int l0 = t0; l0 < n; l0 += U * step) {
+            int   id[U];
+            float lp[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int level = l0 + u * step;
+                if (level < n) {
+                    const size_t g = BK * (size_t)level + col0 + lds_u16(c.sel + 2u * (u32)(level * K + j));
+                    id[u]          = __ldg(p.output_ids_src + g);
+                    lp[u]          = with_lp ? __ldg(p.log_probs_src + g) : 0.0f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int level = l0 + u * step;
+                if (level < n) {
+                    p.output_ids_tgt[tgt + level] = id[u];
+                    if (with_lp) {
+                        p.log_probs_tgt[tgt + level] = lp[u];
+                    }
+                }
+            }
+        }
+    }
+    if (tid == 0) {
+        p.num_beams[b] = first_slot + K;
+    }
+}
+
+// Shared memory above 48 KB is opted into once per device and kernel.
+template<class F>
+int chain_opt_in(F kernel, bool* done)
+{
+    static std::mutex           mu;
+    int                         dev = 0;
+    FTB_CUDA_CHECK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 0 || dev >= 64) {
+        set_error("device ordinal out of range");
+        return FTB200_UNSUPPORTED;
+    }
+    if (!done[dev]) {
+        FTB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainMaxSmem));
+        done[dev] = true;
+    }
+    return FTB200_OK;
+}
+
 }  // namespace
 }  // namespace ftb200
 
@@ -419,7 +806,19 @@ extern "C" int ftb200_gather_tree(const ftb200_gather_tree_params* a)
     p.max_input_without_prompt_length = a->max_input_without_prompt_length;
     p.max_prefix_length               = a->max_prefix_soft_prompt_length;
     p.output_ids                      = a->output_ids;
-    gather_tree_kernel<<<a->batch_size, kDkThreads, 0, (cudaStream_t)a->stream>>>(p);
+    // the parent table of an entry in shared memory where it fits (50000 level-beams), else tile by tile
+    const size_t smem = chain_smem_bytes(a->max_time, a->beam_width);
+    if (smem <= kChainMaxSmem) {
+        static bool opted_in[64];
+        const int   rc = chain_opt_in(gather_tree_chains_kernel, opted_in);
+        if (rc != FTB200_OK) {
+            return rc;
+        }
+        gather_tree_chains_kernel<<<a->batch_size, kChainThreads, smem, (cudaStream_t)a->stream>>>(p);
+    }
+    else {
+        gather_tree_kernel<<<a->batch_size, kDkThreads, 0, (cudaStream_t)a->stream>>>(p);
+    }
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);
     return FTB200_OK;
@@ -441,7 +840,8 @@ extern "C" int ftb200_finalize(int* output_ids, int* sequence_lengths, float* cu
         set_error("ftb200_finalize: 2 * beam_width rounded up to a warp must stay below 1024");
         return FTB200_UNSUPPORTED;
     }
-    finalize_kernel<<<batch_size, kDkThreads, 0, (cudaStream_t)stream>>>(
+    // a CTA per beam (each ranks the entry's few scores for itself): the copies of an entry's beams run side by side
+    finalize_kernel<<<dim3(batch_size, beam_width < 64 ? beam_width : 64), kDkThreads, 0, (cudaStream_t)stream>>>(
         output_ids, sequence_lengths, cum_log_probs, output_log_probs, topk_output_ids, topk_sequence_lengths, scores,
         topk_cum_log_probs, topk_log_probs, num_beams, beam_width, max_seq_len);
     FTB_CUDA_CHECK(cudaGetLastError());
@@ -485,7 +885,18 @@ extern "C" int ftb200_insert_unfinished_path(const ftb200_beam_hyps* hyps, const
     p.cum_log_probs        = cum_log_probs;
     p.batch_size           = batch_size;
     p.beam_width           = beam_width;
-    insert_unfinished_path_kernel<<<batch_size, kDkThreads, 0, (cudaStream_t)stream>>>(p);
+    const size_t smem = chain_smem_bytes(max_seq_len, beam_width);
+    if (smem <= kChainMaxSmem) {
+        static bool opted_in[64];
+        const int   rc = chain_opt_in(insert_chains_kernel, opted_in);
+        if (rc != FTB200_OK) {
+            return rc;
+        }
+        insert_chains_kernel<<<batch_size, kChainThreads, smem, (cudaStream_t)stream>>>(p);
+    }
+    else {
+        insert_unfinished_path_kernel<<<batch_size, kDkThreads, 0, (cudaStream_t)stream>>>(p);
+    }
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);
     return FTB200_OK;
