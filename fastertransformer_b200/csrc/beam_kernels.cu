@@ -1,11 +1,14 @@
-// Beam search, one step in one launch (sm_100a).
+// Beam search, one step in two launches (sm_100a).
 //
-// One CTA per (batch entry, beam): penalties on the fly, one read of the row that yields the online
-// soft-max statistics (max, sum of exponentials) and the row's best 2K columns.  The CTA that finishes
-// last for a batch entry merges the K x 2K candidates, applies length penalty and diversity, archives
-// finished hypotheses, picks the K live continuations, updates lengths / finished / parents and
-// rewrites the KV-cache indirection - everything OnlineBeamSearchLayer<T>::forward launches
-// (layers/beam_search_layers/BaseBeamSearchLayer.cu:181-289) in five kernels.
+// beam_rows_kernel, one CTA per (batch entry, beam): penalties on the fly, one read of the row from HBM that yields the
+// online soft-max statistics (max, sum of exponentials), a second one from L1 for the row's best 2K columns.
+// beam_merge_kernel, one CTA per batch entry: merges the K x 2K candidates, applies length penalty and diversity,
+// archives finished hypotheses, picks the K live continuations, updates lengths / finished / parents and rewrites the
+// KV-cache indirection - everything OnlineBeamSearchLayer<T>::forward launches
+// (layers/beam_search_layers/BaseBeamSearchLayer.cu:181-289) in five kernels.  The second kernel starts while the first
+// drains (programmatic dependent launch).  Two kernels and not one with a last-arrival counter: the merge reads flags
+// of other entries as they were before the step, which the first kernel can simply write down.
+#include "chains.cuh"
 #include "common.cuh"
 #include "ftb200.h"
 
@@ -13,6 +16,7 @@ namespace ftb200 {
 
 constexpr int kBeamThreads = 256;
 constexpr int kMaxBeam     = 64;
+constexpr int kMergeRank   = 512;  // candidates of an entry that are ordered by counting
 
 struct BeamK {
     int dtype, batch_size, local_batch, ite, K, vocab, vocab_padded, step, max_input_len, max_seq_len;
@@ -34,11 +38,12 @@ struct BeamK {
     ftb200_beam_hyps hyps;
     int         has_hyps;
     // workspace
-    u32*   arrivals;  // [local_batch]
     int*   cand_id;   // [local_batch, K, 2K]
     float* cand_val;  // [local_batch, K, 2K]  (already rounded to the logits type)
-    const uint8_t* snap_finished;  // finished / sequence_length as they were before this step
-    const int*     snap_seq_len;
+    uint8_t* snap_finished;  // finished / sequence_length as they were before this step
+    int*     snap_seq_len;
+    int      flag_words;   // words of the bit map of penalised columns; 0: none in this call
+    int      chain_levels; // levels of the parent table in shared memory; 0: the chain is followed in global memory
 };
 
 template<int DT>
@@ -50,33 +55,29 @@ __device__ __forceinline__ float beam_round(float x)
 // logits value of column v with bias / temperature / pad mask applied in the logits type
 // (kernels/beam_search_penalty_kernels.cu:24-87); bf16 goes the fp32 way on the up-cast value.
 template<int DT>
-__device__ __forceinline__ float beam_temp(const BeamK& P, u32 bits, int v)
+__device__ __forceinline__ float beam_plain(u32 bits)
+{
+    return DT == FTB200_F16 ? __half2float(__ushort_as_half((unsigned short)bits)) :
+                              (DT == FTB200_F32 ? __uint_as_float(bits) : __uint_as_float(bits << 16));
+}
+template<int DT>
+__device__ __forceinline__ float beam_temp(const BeamK& P, u32 bits, int v, float inv, __half inv_h)
 {
     if (DT == FTB200_F16) {
         __half h = __ushort_as_half((unsigned short)bits);
-        if (P.apply_temp) {
-            if (v >= P.vocab) {
-                return -65504.0f;
-            }
-            if (P.bias != nullptr) {
-                h = __hadd(h, ((const __half*)P.bias)[v]);
-            }
-            h = __hmul(h, __float2half_rn(1.0f / (P.temperature + 1e-6f)));
+        if (P.bias != nullptr && v < P.vocab) {
+            h = __hadd(h, ((const __half*)P.bias)[v]);
         }
-        return __half2float(h);
+        const float y = __half2float(__hmul(h, inv_h));
+        return v < P.vocab ? y : -65504.0f;
     }
-    float x = DT == FTB200_F32 ? __uint_as_float(bits) : __uint_as_float(bits << 16);
-    if (P.apply_temp) {
-        if (v >= P.vocab) {
-            return -FLT_MAX;
-        }
-        float b = 0.0f;
-        if (P.bias != nullptr) {
-            b = DT == FTB200_F32 ? ((const float*)P.bias)[v] : __bfloat162float(((const __nv_bfloat16*)P.bias)[v]);
-        }
-        x = (x + b) * (1.0f / (P.temperature + 1e-6f));
+    const float x = beam_plain<DT>(bits);
+    float       b = 0.0f;
+    if (P.bias != nullptr && v < P.vocab) {
+        b = DT == FTB200_F32 ? ((const float*)P.bias)[v] : __bfloat162float(((const __nv_bfloat16*)P.bias)[v]);
     }
-    return x;
+    const float y = (x + b) * inv;
+    return v < P.vocab ? y : -FLT_MAX;
 }
 
 template<int DT>
@@ -105,16 +106,108 @@ __device__ __forceinline__ u64 order_key(float val, u32 col)
     return ((u64)(~fkey(val)) << 32) | col;
 }
 
-template<int DT>
-__global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_constant__ BeamK P)
+constexpr int kBeamTile    = 4096;  // columns of a tile: sixteen per thread
+constexpr int kBeamStages  = 4;     // tiles in the ring
+constexpr int kBeamCollect = 2048;  // columns at or above the row's bound that are sorted in shared memory
+
+// Marks the tokens of row bb's ancestry (the ids that the repetition / presence penalty applies to,
+// beam_search_penalty_kernels.cu:89-152) in the bit map.  The chain runs through every level's parents: it is cut into
+// segments whose maps compose (see chains.cuh), so that a long history costs a few walks of a segment's length.
+static __device__ __noinline__ void mark_ancestry(const BeamK& P, int bb, u32* bits, unsigned char* tables)
+{
+    const int    tid = threadIdx.x, K = P.K, b = bb / K, V = P.vocab_padded;
+    const int    bbsize = P.batch_size * K, top = P.step - 1;
+    const int    input_len = P.input_lengths != nullptr ? P.input_lengths[bb] : P.max_input_len;
+    const int*   ids = P.output_ids + (size_t)b * K;
+    const int*   par = P.parent_ids + (size_t)P.ite * K * P.local_batch + (size_t)b * K;
+    auto         mark = [&](int id) {
+        if (id >= 0 && id < V) {
+            smem_or(&bits[id >> 5], 1u << (id & 31));
+        }
+    };
+    auto skipped = [&](int level) { return level >= input_len && level < P.max_input_len; };
+    if (tid == 0) {
+        mark(P.output_ids[(size_t)top * bbsize + (size_t)P.ite * P.local_batch * K + bb]);
+    }
+    if (P.chain_levels == 0) {
+        if (tid == 0) {
+            int beam = bb % K;
+            for (int i = top - 1; i >= 0; --i) {
+                if (!skipped(i)) {
+                    beam = par[(size_t)i * bbsize + beam];
+                    mark(ids[(size_t)i * bbsize + beam]);
+                }
+            }
+        }
+        return;
+    }
+    const int levels = top, W = K + 1;
+    const u32 row = 2u * (u32)W, t_par = (u32)__cvta_generic_to_shared(tables), t_sel = t_par + (u32)levels * row;
+    int       segments = kBeamThreads / W;
+    segments           = segments < 1 ? 1 : (segments > 32 ? 32 : segments);
+    const int seglen   = (levels + segments - 1) / segments;
+    const u32 t_comp   = t_sel + 2u * (u32)levels;
+    __shared__ u32 s_entry[32];
+    for (int e = tid; e < levels * K; e += kBeamThreads) {
+        const int level = e / K, k = e - level * K;
+        int       v = skipped(level) ? k : __ldg(par + (size_t)level * bbsize + k);  // a skipped level passes the chain on
+        v           = v < 0 || v >= K ? k : v;
+        sts_u16(t_par + (u32)level * row + 2u * (u32)k, 2u * (u32)v);
+    }
+    __syncthreads();
+    for (int e = tid; e < segments * K; e += kBeamThreads) {
+        const int seg = e / K, lo = min(seg * seglen, levels), hi = min(lo + seglen, levels);
+        u32       cur = 2u * (u32)(e % K), at = t_par + (u32)hi * row;
+        for (int i = lo; i < hi; ++i) {
+            at -= row;
+            cur = lds_u16(at + cur);
+        }
+        sts_u16(t_comp + (u32)seg * row + 2u * (u32)(e % K), cur);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        u32 cur = 2u * (u32)(bb % K);
+        for (int seg = segments - 1; seg >= 0; --seg) {
+            s_entry[seg] = cur;
+            cur          = lds_u16(t_comp + (u32)seg * row + cur);
+        }
+    }
+    __syncthreads();
+    if (tid < segments) {
+        const int lo = min(tid * seglen, levels), hi = min(lo + seglen, levels);
+        u32       cur = s_entry[tid], at = t_par + (u32)hi * row;
+        for (int i = hi - 1; i >= lo; --i) {
+            at -= row;
+            cur = lds_u16(at + cur);  // the parent at this level is the beam whose token counts
+            sts_u16(t_sel + 2u * (u32)i, cur);
+        }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int level = tid; level < levels; level += kBeamThreads) {
+        if (!skipped(level)) {
+            mark(__ldg(ids + (size_t)level * bbsize + lds_u16(t_sel + 2u * (u32)level) / 2u));
+        }
+    }
+}
+
+// TEMP: temperature, bias or a padded vocabulary; PEN: penalised columns.  A branch per column costs as much as the
+// column's arithmetic, so the variants are compiled apart.  Bound by latency and issue (24 instructions a column, a
+// running maximum and a sum as chains): one row of 32000 half columns 12 us, 256 of them 16 us; with a list search per
+// column, sixteen sorted lists and a pass per winner of a wide beam it was 80 us and up.
+template<int DT, bool TEMP, bool PEN>
+__global__ void __launch_bounds__(kBeamThreads, 3) beam_rows_kernel(const __grid_constant__ BeamK P)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // layout: u64 sortbuf[max(kBeamThreads * 8, K * 2K)] | int spec_id[step] | float spec_val[step]
-    u64*             sortbuf = (u64*)smem_raw;
-    __shared__ MD    s_md[kBeamThreads / 32];
-    __shared__ int   s_nspec, s_last;
-    __shared__ float s_old_cum[kMaxBeam];
-    __shared__ int   s_newseq[kMaxBeam];
+    // layout: ring of row tiles | u64 collected[kBeamCollect] | u32 bits[flag_words] | chain tables
+    const u32      ring = (u32)__cvta_generic_to_shared(smem_raw);
+    u64*           col  = (u64*)(smem_raw + (size_t)kBeamStages * kBeamTile * (DT == FTB200_F32 ? 4 : 2));
+    u32*           bits = (u32*)(col + kBeamCollect);
+    __shared__ MD  s_md[kBeamThreads / 32];
+    __shared__ __align__(16) u32 s_key[kBeamThreads];
+    __shared__ u32 s_n, s_bound;
+    FTB_ASSUME_SHARED(col);
+    FTB_ASSUME_SHARED(bits);
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int bb  = blockIdx.x;  // local batch-beam row
@@ -123,99 +216,239 @@ __global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_co
     const size_t ES  = DT == FTB200_F32 ? 4 : 2;
     const char*  row = (const char*)P.logits + (size_t)bb * V * ES;
     const float  MAXT = DT == FTB200_F16 ? 65504.0f : FLT_MAX;
-    const int    sort_cap = kBeamThreads * 8 > K * twoK ? kBeamThreads * 8 : K * twoK;
-    int*         spec_id  = (int*)(sortbuf + sort_cap);
-    float*       spec_val = (float*)(spec_id + (P.step > 0 ? P.step : 1));
 
     const bool fin    = P.finished[bb] != 0;
     const int  end_id = P.end_ids[b];
-
-    // ---- columns with a value of their own: repetition / presence penalty along the beam's ancestry
-    //      (beam_search_penalty_kernels.cu:89-152: one thread walks parent_ids) and the min-length mask
+    const float cum   = P.cum_log_probs[bb];
     if (tid == 0) {
-        int n = 0;
-        if (!fin && P.penalty_type != FTB200_PENALTY_NONE && P.step > 0
-            && P.rep_penalty != (P.penalty_type == FTB200_PENALTY_MULTIPLICATIVE ? 1.0f : 0.0f)) {
-            const int    bbsize    = P.batch_size * K;
-            const int    input_len = P.input_lengths != nullptr ? P.input_lengths[bb] : P.max_input_len;
-            const int*   cur       = P.output_ids + (size_t)(P.step - 1) * bbsize + (size_t)P.ite * P.local_batch * K;
-            const int*   parents   = P.parent_ids + (size_t)P.ite * K * P.local_batch;
-            const float  pen       = beam_round<DT>(P.rep_penalty);
-            auto         add       = [&](int id) {
-                if (id < 0 || id >= V) {
-                    return;
-                }
-                const float x = beam_temp<DT>(P, beam_load<DT>(row, id), id);
-                float       y;
+        P.snap_finished[bb] = fin ? 1 : 0;
+        P.snap_seq_len[bb]  = P.seq_len[bb];
+        s_n                 = 0;
+    }
+    int*   my_id  = P.cand_id + (size_t)bb * twoK;
+    float* my_val = P.cand_val + (size_t)bb * twoK;
+    if (fin) {
+        // every column but the end token is -MAX: the end token first, then the smallest columns (:410-432)
+        const bool  has   = end_id >= 0 && end_id < V;
+        const float m     = has ? MAXT : -MAXT;
+        const float log_d = logf(has ? 1.0f : (float)V);
+        for (int n = tid; n < twoK; n += kBeamThreads) {
+            const int   v = has ? (n == 0 ? end_id : (n - 1 < end_id ? n - 1 : n)) : n;
+            const float u = has && n == 0 ? MAXT : -MAXT;
+            my_id[n]      = v < V ? bb * V + v : -1;
+            my_val[n]     = beam_round<DT>(u - m - log_d + cum);
+        }
+        return;
+    }
+
+    // ---- columns with a value of their own: repetition / presence penalty along the beam's ancestry, min-length mask
+    if (PEN) {
+        for (int i = tid; i < P.flag_words; i += kBeamThreads) {
+            bits[i] = 0;
+        }
+        __syncthreads();
+        mark_ancestry(P, bb, bits, (unsigned char*)(bits + P.flag_words));
+        __syncthreads();
+    }
+    const bool   minlen = (P.step - P.max_input_len < P.min_length) && (P.seq_len[bb] + 1 - P.max_input_len < P.min_length);
+    const int    masked = minlen ? end_id : -1;
+    const float  pen    = beam_round<DT>(P.rep_penalty);
+    const float  inv    = 1.0f / (P.temperature + 1e-6f);
+    const __half inv_h  = __float2half_rn(inv);
+    // value of column v as the reference's stage-1 kernel sees it (:410-432)
+    auto value_of = [&](int v, u32 raw) -> float {
+        float y = TEMP ? beam_temp<DT>(P, raw, v, inv, inv_h) : beam_plain<DT>(raw);
+        if (PEN) {
+            const u32 w = bits[v >> 5];  // one word for the 32 columns of a warp
+            if ((w >> (v & 31)) & 1u) {
                 if (P.penalty_type == FTB200_PENALTY_ADDITIVE) {
-                    y = beam_round<DT>(x - pen);
+                    y = beam_round<DT>(y - pen);
                 }
                 else {
-                    y = beam_round<DT>(x > 0.0f ? x / pen : x * pen);
+                    y = beam_round<DT>(y > 0.0f ? y / pen : y * pen);
                 }
-                spec_id[n]  = id;
-                spec_val[n] = y;
-                ++n;
-            };
-            add(cur[bb]);
-            int parent_beam = bb % K;
-            for (int i = P.step - 2; i >= 0; --i) {
-                if (i >= input_len && i < P.max_input_len) {
-                    continue;
-                }
-                parent_beam = parents[(size_t)i * bbsize + b * K + parent_beam];
-                add(P.output_ids[(size_t)i * bbsize + b * K + parent_beam]);
             }
         }
-        s_nspec = n;
-    }
-    __syncthreads();
-    const int  nspec  = s_nspec;
-    const bool minlen = !fin && (P.step - P.max_input_len < P.min_length)
-                        && (P.seq_len[bb] + 1 - P.max_input_len < P.min_length);
-
-    // value of column v as the reference's stage-1 kernel sees it (:410-432)
-    auto value_of = [&](int v, u32 bits) -> float {
-        if (fin) {
-            return v == end_id ? MAXT : -MAXT;
-        }
-        if (minlen && v == end_id) {
-            return -MAXT;
-        }
-        float y = beam_temp<DT>(P, bits, v);
-        for (int i = 0; i < nspec; ++i) {  // later entries of the walk are older; the first match wins
-            if (spec_id[i] == v) {
-                y = spec_val[i];
-                break;
-            }
-        }
-        return y;
+        return v == masked ? -MAXT : y;
     };
 
-    // ---- one pass: online soft-max statistics and this thread's best columns
-    constexpr int LN = 8;  // per-thread list length; rows needing more than 8 winners take extra passes
-    u64           best[LN];
+    // ---- one pass: soft-max statistics and the candidates ----
+    // Thread t takes columns t, t + 256, ... one after the other (an online maximum and sum; the order is kept, so that
+    // scores rounded to half do not depend on the launch); only the maximum and the sum themselves are chains.  The
+    // threads' maxima over the first tile give a bound that every one of the row's best 2K reaches: later columns at or above it are kept, a few times 2K V / 4096.
+    constexpr int U = 16;
+    MD            md{-MAXT, 0.0f};
+    float         bound = -INFINITY;
+    auto          add = [&](float y) {
+        // md_merge(md, {y, 1}) in fewer instructions: |difference| serves both orders
+        const float t = md.m - y, e = __expf(-fabsf(t));
+        const bool  keep = t > 0.0f;
+        md.d             = fmaf(md.d, keep ? 1.0f : e, keep ? e : 1.0f);
+        md.m             = fmaxf(md.m, y);
+    };
+    auto push = [&](int v, float y) {
+        const u32 at = atomicAdd(&s_n, 1u);
+        if (at < (u32)kBeamCollect) {
+            col[at] = order_key(y, (u32)v);
+        }
+    };
+    // The 2K-th largest of the threads' maxima: a value that at least 2K columns seen so far reach (CTA-wide).  Narrow
+    // beams: every warp takes out its 2K largest, warp 0 goes through those; wide ones: every thread counts.
+    auto thread_bound = [&]() {
+        u32 mine = fkey(md.m);
+        if (twoK <= 16) {
+            for (int r = 0; r < twoK; ++r) {
+                const u32 top     = __reduce_max_sync(0xffffffffu, mine);
+                const u32 holders = __ballot_sync(0xffffffffu, mine == top);
+                mine              = lane == __ffs(holders) - 1 ? 0u : mine;
+                if (lane == 0) {
+                    s_key[wid * twoK + r] = top;
+                }
+            }
+            __syncthreads();
+            if (wid == 0) {
+                u32 k[4];
 #pragma unroll
-    for (int i = 0; i < LN; ++i) {
-        best[i] = ~0ull;
-    }
-    MD md{-MAXT, 0.0f};
-    for (int v = tid; v < V; v += kBeamThreads) {
-        const float y = value_of(v, fin ? 0u : beam_load<DT>(row, v));
-        md            = md_merge(md, MD{y, 1.0f});
-        const u64 kk  = order_key(y, (u32)v);
-        if (kk < best[LN - 1]) {
-            best[LN - 1] = kk;
+                for (int i = 0; i < 4; ++i) {
+                    const int at = i * 32 + lane;
+                    k[i]         = at < twoK * (kBeamThreads / 32) ? s_key[at] : 0u;
+                }
+                u32 top = 0;
+                for (int r = 0; r < twoK; ++r) {
+                    const u32 best = max(max(k[0], k[1]), max(k[2], k[3]));
+                    top            = __reduce_max_sync(0xffffffffu, best);
+                    const u32 holders = __ballot_sync(0xffffffffu, best == top);
+                    if (lane == __ffs(holders) - 1) {
+                        bool gone = false;  // one of them, once
 #pragma unroll
-            for (int i = LN - 1; i > 0; --i) {
-                if (best[i] < best[i - 1]) {
-                    u64 t       = best[i];
-                    best[i]     = best[i - 1];
-                    best[i - 1] = t;
+                        for (int i = 0; i < 4; ++i) {
+                            const bool hit = (k[i] == top) & !gone;
+                            gone |= hit;
+                            k[i] = hit ? 0u : k[i];
+                        }
+                    }
+                }
+                if (lane == 0) {
+                    s_bound = top;
                 }
             }
         }
+        else {
+            s_key[tid] = mine;
+            __syncthreads();
+            int rk = 0;
+#pragma unroll 8
+            for (int i = 0; i < kBeamThreads; i += 4) {
+                // larger, or equal and of an earlier thread (short-circuit forms of this compile to branches: 12 us, not 2)
+                const uint4 o = *(const uint4*)(s_key + i);
+                rk += o.x >= mine + (i + 0 >= tid ? 1u : 0u) ? 1 : 0;
+                rk += o.y >= mine + (i + 1 >= tid ? 1u : 0u) ? 1 : 0;
+                rk += o.z >= mine + (i + 2 >= tid ? 1u : 0u) ? 1 : 0;
+                rk += o.w >= mine + (i + 3 >= tid ? 1u : 0u) ? 1 : 0;
+            }
+            if (rk == twoK - 1) {
+                s_bound = mine;
+            }
+        }
+        __syncthreads();
+        return fkey_inv(s_bound);
+    };
+    // The row comes through a ring of tiles in shared memory, three tiles ahead (16-byte asynchronous copies; the few
+    // columns before the first and after the last 16-byte boundary go through registers).
+    const int sh   = (int)(((size_t)row & 15) / ES);  // the row's first column inside its 16 bytes
+    auto      fill = [&](int k) {
+        constexpr int EPC = 16 / (DT == FTB200_F32 ? 4 : 2);
+        for (int c = tid; c < kBeamTile / EPC; c += kBeamThreads) {
+            const int v    = k * kBeamTile + c * EPC - sh;
+            const u32 slot = ring + (u32)((k % kBeamStages) * kBeamTile + c * EPC) * (u32)ES;
+            if (v >= 0 && v + EPC <= V) {
+                cp_async16(slot, row + (ptrdiff_t)v * (ptrdiff_t)ES);
+            }
+            else {
+#pragma unroll
+                for (int e = 0; e < EPC; ++e) {
+                    if (v + e >= 0 && v + e < V) {
+                        if (DT == FTB200_F32) {
+                            sts_u32(slot + 4u * (u32)e, beam_load<DT>(row, v + e));
+                        }
+                        else {
+                            sts_u16(slot + 2u * (u32)e, beam_load<DT>(row, v + e));
+                        }
+                    }
+                }
+            }
+        }
+    };
+    constexpr u32 kRing = kBeamStages * kBeamTile;
+    auto staged = [&](u32 at) { return DT == FTB200_F32 ? lds_u32(at) : lds_u16(at); };
+    // (no branch per column: a mask of the sixteen, and the rare column that is kept is read again)
+    auto keep_above = [&](const float* y, int v0, auto&& again) {
+        u32 hits = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            hits |= (y[u] >= bound ? 1u : 0u) << u;
+        }
+        while (hits != 0) {
+            const int v = v0 + (__ffs(hits) - 1) * kBeamThreads;
+            hits &= hits - 1;
+            push(v, value_of(v, again(v)));
+        }
+    };
+    float     y[U];
+    const int v_whole = V / kBeamTile * kBeamTile, tiles = (V + sh + kBeamTile - 1) / kBeamTile;
+    for (int k = 0; k < kBeamStages - 1; ++k) {
+        if (k < tiles) {
+            fill(k);
+        }
+        cp_async_commit();
     }
+    for (int k = 0; k * kBeamTile < V; ++k) {
+        cp_async_wait<kBeamStages - 3>();  // tile k + 1 has arrived too: a row that starts off a 16-byte boundary reaches into it
+        __syncthreads();                   // for every thread; and tile k - 1 has been used up
+        if (k + kBeamStages - 1 < tiles) {
+            fill(k + kBeamStages - 1);
+        }
+        cp_async_commit();
+        const int v0 = k * kBeamTile + tid;
+        const u32 at = (u32)(v0 + sh) % kRing;
+        if (v0 - tid < v_whole) {
+            u32 raw[U];
+            if (sh == 0) {
+                const u32 a0 = ring + at * (u32)ES;  // the tile does not wrap: one address for all sixteen
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    raw[u] = staged(a0 + (u32)(u * kBeamThreads) * (u32)ES);
+                }
+            }
+            else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    raw[u] = staged(ring + (at + (u32)(u * kBeamThreads)) % kRing * (u32)ES);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                y[u] = value_of(v0 + u * kBeamThreads, raw[u]);
+                add(y[u]);
+            }
+        }
+        else {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int v = v0 + u * kBeamThreads;
+                y[u]        = __int_as_float(0x7fc00000);  // not a number: below every bound
+                if (v < V) {
+                    y[u] = value_of(v, staged(ring + (at + (u32)(u * kBeamThreads)) % kRing * (u32)ES));
+                    add(y[u]);
+                }
+            }
+        }
+        if (k == 0) {
+            bound = thread_bound();
+        }
+        keep_above(y, v0, [&](int v) { return staged(ring + (u32)(v + sh) % kRing * (u32)ES); });
+    }
+    bound = thread_bound();  // (also a barrier: everything has been collected)
     for (int off = 16; off > 0; off >>= 1) {
         MD o;
         o.m = __shfl_down_sync(0xffffffffu, md.m, off);
@@ -225,78 +458,113 @@ __global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_co
     if (lane == 0) {
         s_md[wid] = md;
     }
+    const int n_all = (int)s_n;
     __syncthreads();
     md = s_md[0];
     for (int i = 1; i < kBeamThreads / 32; ++i) {
         md = md_merge(md, s_md[i]);
     }
     const float log_d = logf(md.d);
-    const float cum   = P.cum_log_probs[bb];
-
-    int*   my_id  = P.cand_id + (size_t)bb * twoK;
-    float* my_val = P.cand_val + (size_t)bb * twoK;
-    if (twoK <= LN) {
+    auto        score = [&](u64 e) { return beam_round<DT>(fkey_inv(~(u32)(e >> 32)) - md.m - log_d + cum); };
+    // the bound of the whole row leaves a few more than 2K of them
+    if (tid == 0) {
+        s_n = 0;
+    }
+    __syncthreads();
+    u64 kept[kBeamCollect / kBeamThreads];
+    if (n_all <= kBeamCollect) {
 #pragma unroll
-        for (int i = 0; i < LN; ++i) {
-            sortbuf[tid * LN + i] = best[i];
+        for (int i = 0; i < kBeamCollect / kBeamThreads; ++i) {
+            const int at = i * kBeamThreads + tid;
+            kept[i]      = at < n_all ? col[at] : ~0ull;
         }
         __syncthreads();
-        group_sort_u64(sortbuf, kBeamThreads * LN, tid, kBeamThreads, CtaSync());
-        __syncthreads();
-        if (tid < twoK) {
-            const u64   e   = sortbuf[tid];
-            const float u   = fkey_inv(~(u32)(e >> 32));
-            const int   col = (int)(e & 0xffffffffu);
-            my_id[tid]      = e == ~0ull ? -1 : bb * V + col;
-            my_val[tid]     = beam_round<DT>(u - md.m - log_d + cum);
+#pragma unroll
+        for (int i = 0; i < kBeamCollect / kBeamThreads; ++i) {
+            if ((kept[i] != ~0ull) & ((u32)(~(u32)(kept[i] >> 32)) >= s_bound)) {
+                col[atomicAdd(&s_n, 1u)] = kept[i];
+            }
         }
     }
     else {
-        // wide beams: extract the winners one by one, each pass over the row (it sits in L2 by now)
-        __shared__ u64 s_prev;
-        if (tid == 0) {
-            s_prev = 0;
-        }
-        __syncthreads();
-        for (int n = 0; n < twoK; ++n) {
-            const u64 prev = s_prev;
-            u64       mine = ~0ull;
-            for (int v = tid; v < V; v += kBeamThreads) {
-                const u64 kk = order_key(value_of(v, fin ? 0u : beam_load<DT>(row, v)), (u32)v);
-                if ((n == 0 || kk > prev) && kk < mine) {
-                    mine = kk;
-                }
+        // a wide beam over a long row: the columns at or above the final bound, in a second pass
+        for (int v0 = tid; v0 < V; v0 += kBeamThreads * U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int v = v0 + u * kBeamThreads;
+                y[u]        = v < V ? value_of(v, beam_load<DT>(row, v)) : __int_as_float(0x7fc00000);
             }
-            sortbuf[tid] = mine;
-            __syncthreads();
-            for (int s = kBeamThreads / 2; s > 0; s >>= 1) {
-                if (tid < s && sortbuf[tid + s] < sortbuf[tid]) {
-                    sortbuf[tid] = sortbuf[tid + s];
-                }
-                __syncthreads();
-            }
-            if (tid == 0) {
-                const u64 e = sortbuf[0];
-                s_prev      = e;
-                my_id[n]    = e == ~0ull ? -1 : bb * V + (int)(e & 0xffffffffu);
-                my_val[n]   = beam_round<DT>(fkey_inv(~(u32)(e >> 32)) - md.m - log_d + cum);
-            }
-            __syncthreads();
+            keep_above(y, v0, [&](int v) { return beam_load<DT>(row, v); });
         }
     }
-
-    // ---- the last CTA of this batch entry merges
-    __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        s_last = atomicAdd(&P.arrivals[b], 1u) == (u32)(K - 1);
-    }
-    __syncthreads();
-    if (!s_last) {
+    const int n = (int)s_n;
+    if (n <= kBeamCollect && n >= (twoK < V ? twoK : V)) {
+        for (int i = tid; i < n; i += kBeamThreads) {
+            const u64 e  = col[i];
+            int       rk = 0;
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) {
+                rk += col[j] < e ? 1 : 0;
+            }
+            if (rk < twoK) {
+                my_id[rk]  = bb * V + (int)(e & 0xffffffffu);
+                my_val[rk] = score(e);
+            }
+        }
+        for (int i = n + tid; i < twoK; i += kBeamThreads) {
+            my_id[i]  = -1;
+            my_val[i] = score(~0ull);
+        }
         return;
     }
-    __threadfence();
+    // thousands of equal values at the bound, or columns that are not above -MAX: the winners one by one, each in a pass
+    // over the row
+    __syncthreads();
+    __shared__ u64 s_prev;
+    if (tid == 0) {
+        s_prev = 0;
+    }
+    __syncthreads();
+    for (int w = 0; w < twoK; ++w) {
+        const u64 prev = s_prev;
+        u64       mine = ~0ull;
+        for (int v = tid; v < V; v += kBeamThreads) {
+            const u64 kk = order_key(value_of(v, beam_load<DT>(row, v)), (u32)v);
+            if ((w == 0 || kk > prev) && kk < mine) {
+                mine = kk;
+            }
+        }
+        col[tid] = mine;
+        __syncthreads();
+        for (int s = kBeamThreads / 2; s > 0; s >>= 1) {
+            if (tid < s && col[tid + s] < col[tid]) {
+                col[tid] = col[tid + s];
+            }
+            __syncthreads();
+        }
+        if (tid == 0) {
+            const u64 e = col[0];
+            s_prev      = e;
+            my_id[w]    = e == ~0ull ? -1 : bb * V + (int)(e & 0xffffffffu);
+            my_val[w]   = score(e);
+        }
+        __syncthreads();
+    }
+}
 
+template<int DT>
+__global__ void __launch_bounds__(kBeamThreads) beam_merge_kernel(const __grid_constant__ BeamK P)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u64*             sortbuf = (u64*)smem_raw;  // [2 * ncand] below kMergeRank candidates, else [ncand]
+    constexpr int    kTop    = 128;
+    __shared__ float s_old_cum[kMaxBeam], s_y[kTop];
+    __shared__ int   s_newseq[kMaxBeam], s_word[kTop];
+    const int        tid = threadIdx.x, b = blockIdx.x, K = P.K, twoK = 2 * K, V = P.vocab_padded;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the rows' kernel has ended and its results are visible
+
+    const int    end_id  = P.end_ids[b];
     const int    ncand   = K * twoK;
     const int*   x       = P.cand_id + (size_t)b * ncand;
     const float* y       = P.cand_val + (size_t)b * ncand;
@@ -343,20 +611,52 @@ __global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_co
             sortbuf[i] = x[i] < 0 ? ~0ull : order_key(e, (u32)i);
         }
         __syncthreads();
-        group_sort_u64(sortbuf, ncand, tid, kBeamThreads, CtaSync());
+        if (ncand <= kMergeRank) {
+            // a few hundred: by counting the smaller ones (missing ones in the order they stand)
+            for (int i = tid; i < ncand; i += kBeamThreads) {
+                const u64 e  = sortbuf[i];
+                int       rk = 0;
+#pragma unroll 4
+                for (int j = 0; j < ncand; ++j) {
+                    rk += (int)(sortbuf[j] < e) | ((int)(sortbuf[j] == e) & (int)(j < i));
+                }
+                sortbuf[ncand + rk] = e;
+            }
+            __syncthreads();
+            sortbuf += ncand;
+        }
+        else {
+            group_sort_u64(sortbuf, ncand, tid, kBeamThreads, CtaSync());
+            __syncthreads();
+        }
+        const int top_n = ncand < 2 * 4 ? ncand : (twoK <= 8 ? 8 : (twoK <= 16 ? 16 : (twoK <= 32 ? 32 : (twoK <= 64 ? 64 : 128))));
+        // what the choice reads, fetched together
+        for (int i = tid; i < top_n && i < ncand; i += kBeamThreads) {
+            const u64 e = sortbuf[i];
+            s_word[i]   = e == ~0ull ? -1 : x[(u32)e];
+            s_y[i]      = e == ~0ull ? 0.0f : y[(u32)e];
+        }
         __syncthreads();
-        if (tid == 0) {
-            const int top_n = ncand < 2 * 4 ? ncand : (twoK <= 8 ? 8 : (twoK <= 16 ? 16 : (twoK <= 32 ? 32 : (twoK <= 64 ? 64 : 128))));
+        if (!P.has_hyps) {
+            // no archive: the K best go on
+            if (tid < K && tid < top_n && tid < ncand && s_word[tid] >= 0) {
+                z[tid] = s_word[tid];
+                if (olp != nullptr) {
+                    olp[b * K + tid] = s_y[tid] - s_old_cum[(s_word[tid] / V) % K];
+                }
+                v_cum[tid] = s_y[tid];
+            }
+        }
+        else if (tid == 0) {
             int       selected = 0;
             for (int i = 0; i < top_n && i < ncand; ++i) {
                 const u64 e = sortbuf[i];
                 if (e == ~0ull) {
                     break;
                 }
-                const int   ci           = (int)(e & 0xffffffffu);
                 const float normed_score = fkey_inv(~(u32)(e >> 32));
-                const int   word         = x[ci];
-                if (P.has_hyps && word % V == end_id) {
+                const int   word         = s_word[i];
+                if (word % V == end_id) {
                     if (i < K) {
                         const int num_beam = P.hyps.num_beams[gbi];
                         int       beam_idx = num_beam;
@@ -388,7 +688,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_co
                         const size_t tgt = ((size_t)gbi * twoK + beam_idx) * P.max_seq_len;
                         P.hyps.output_ids_tgt[tgt + P.step] = end_id;
                         if (P.hyps.log_probs != nullptr) {
-                            P.hyps.log_probs[tgt + P.step] = y[ci] - s_old_cum[(word / V) % K];
+                            P.hyps.log_probs[tgt + P.step] = s_y[i] - s_old_cum[(word / V) % K];
                         }
                         int prev_id = (word / V) % K;
                         for (int j = P.step - 1; j >= 0; j--) {
@@ -404,29 +704,27 @@ __global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_co
                         P.hyps.normed_scores[tb]          = normed_score;
                         P.hyps.min_normed_scores[gbi]     = fminf(P.hyps.min_normed_scores[gbi], normed_score);
                         P.hyps.num_beams[gbi]++;
-                        P.hyps.cum_log_probs[tb]          = y[ci];
+                        P.hyps.cum_log_probs[tb]          = s_y[i];
                     }
                 }
-                else if ((P.has_hyps && i < twoK) || (!P.has_hyps && i < K)) {
+                else if (i < twoK) {
                     z[selected] = word;
                     if (olp != nullptr) {
-                        olp[b * K + selected] = y[ci] - s_old_cum[(word / V) % K];
+                        olp[b * K + selected] = s_y[i] - s_old_cum[(word / V) % K];
                     }
-                    v_cum[selected] = y[ci];
+                    v_cum[selected] = s_y[i];
                     selected++;
                 }
                 if (selected >= K) {
                     break;
                 }
             }
-            if (P.has_hyps) {
-                // the reference indexes by the local batch index here (:254-261)
-                if (P.hyps.num_beams[b] < K) {
-                    P.hyps.is_done[b] = 0;
-                }
-                else if (P.hyps.early_stopping) {
-                    P.hyps.is_done[b] = 1;
-                }
+            // the reference indexes by the local batch index here (:254-261)
+            if (P.hyps.num_beams[b] < K) {
+                P.hyps.is_done[b] = 0;
+            }
+            else if (P.hyps.early_stopping) {
+                P.hyps.is_done[b] = 1;
             }
         }
         __syncthreads();
@@ -470,6 +768,49 @@ __global__ void __launch_bounds__(kBeamThreads) beam_step_kernel(const __grid_co
             P.tgt_indir[base + (size_t)k * L + tc] = t == P.step ? k : P.src_indir[base + (size_t)src_beam * L + tc];
         }
     }
+}
+
+constexpr size_t kBeamMaxSmem = 200 * 1024;
+
+template<int DT, bool TEMP, bool PEN>
+static int beam_rows_launch(const BeamK& K, size_t smem, cudaStream_t st)
+{
+    static bool opted[64];
+    const int   rc = chain_opt_in(beam_rows_kernel<DT, TEMP, PEN>, opted);
+    if (rc != FTB200_OK) {
+        return rc;
+    }
+    beam_rows_kernel<DT, TEMP, PEN><<<K.local_batch * K.K, kBeamThreads, smem, st>>>(K);
+    FTB_CUDA_CHECK(cudaGetLastError());
+    return FTB200_OK;
+}
+
+template<int DT>
+static int beam_launch(const BeamK& K, size_t smem, cudaStream_t st)
+{
+    static bool merge_opted[64];
+    int         rc = chain_opt_in(beam_merge_kernel<DT>, merge_opted);
+    if (rc == FTB200_OK) {
+        rc = K.apply_temp ? (K.flag_words > 0 ? beam_rows_launch<DT, true, true>(K, smem, st) : beam_rows_launch<DT, true, false>(K, smem, st)) :
+                            (K.flag_words > 0 ? beam_rows_launch<DT, false, true>(K, smem, st) : beam_rows_launch<DT, false, false>(K, smem, st));
+    }
+    if (rc != FTB200_OK) {
+        return rc;
+    }
+    const int             ncand = K.K * 2 * K.K;
+    cudaLaunchConfig_t    cfg{};
+    cudaLaunchAttribute   attr[1];
+    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim          = dim3((unsigned)K.local_batch);
+    cfg.blockDim         = dim3(kBeamThreads);
+    cfg.dynamicSmemBytes = (size_t)ncand * (ncand <= kMergeRank ? 16 : 8);
+    cfg.stream           = st;
+    cfg.attrs            = attr;
+    cfg.numAttrs         = 1;
+    FTB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, beam_merge_kernel<DT>, K));
+    note_launch(2);
+    return FTB200_OK;
 }
 
 }  // namespace ftb200
@@ -531,43 +872,34 @@ extern "C" int ftb200_beam_search_step(const ftb200_beam_params* p)
     if (p->beam_hyps != nullptr) {
         K.hyps = *p->beam_hyps;
     }
-    char* ws   = (char*)p->workspace;
-    K.arrivals = (u32*)ws;
+    // (the first 256 + 4 * local_batch_size bytes of the workspace are not used any more)
+    char*        ws   = (char*)p->workspace;
     const size_t rows = (size_t)p->local_batch_size * p->beam_width;
-    K.cand_id  = (int*)(ws + (((size_t)p->local_batch_size * 4 + 255) / 256) * 256 + 256);
-    K.cand_val = (float*)(K.cand_id + rows * 2 * p->beam_width);
-    uint8_t* snap_fin = (uint8_t*)(K.cand_val + rows * 2 * p->beam_width);
-    int*     snap_seq = (int*)(snap_fin + ((rows + 255) / 256) * 256);
-    K.snap_finished   = snap_fin;
-    K.snap_seq_len    = snap_seq;
+    K.cand_id         = (int*)(ws + (((size_t)p->local_batch_size * 4 + 255) / 256) * 256 + 256);
+    K.cand_val        = (float*)(K.cand_id + rows * 2 * p->beam_width);
+    K.snap_finished   = (uint8_t*)(K.cand_val + rows * 2 * p->beam_width);
+    K.snap_seq_len    = (int*)(K.snap_finished + ((rows + 255) / 256) * 256);
 
-    cudaStream_t st = (cudaStream_t)p->stream;
-    FTB_CUDA_CHECK(cudaMemsetAsync(K.arrivals, 0, (size_t)p->local_batch_size * 4, st));
-    // the merge of one batch entry reads finished / sequence_length of OTHER entries (the reference indexes
-    // them by the batch index); give it the values from before any entry of this step was updated
-    FTB_CUDA_CHECK(cudaMemcpyAsync(snap_fin, p->finished, rows, cudaMemcpyDeviceToDevice, st));
-    FTB_CUDA_CHECK(cudaMemcpyAsync(snap_seq, p->sequence_length, rows * 4, cudaMemcpyDeviceToDevice, st));
-    const int    twoK     = 2 * p->beam_width;
-    const size_t sort_cap = (size_t)(kBeamThreads * 8 > p->beam_width * twoK ? kBeamThreads * 8 : p->beam_width * twoK);
-    const size_t smem     = sort_cap * 8 + (size_t)(p->step > 0 ? p->step : 1) * 8 + 16;
-    if (smem > 200 * 1024) {
-        set_error("ftb200_beam_search_step: step too large for the shared-memory token list");
+    const bool penalise = p->penalty_type != FTB200_PENALTY_NONE && p->step > 0
+                          && p->repetition_penalty != (p->penalty_type == FTB200_PENALTY_MULTIPLICATIVE ? 1.0f : 0.0f);
+    K.flag_words        = penalise ? ((p->vocab_size_padded + 31) / 32 + 3) / 4 * 4 : 0;
+    size_t smem         = (size_t)kBeamStages * kBeamTile * (p->dtype == FTB200_F32 ? 4 : 2) + (size_t)kBeamCollect * 8 + (size_t)K.flag_words * 4;
+    if (smem > kBeamMaxSmem) {
+        set_error("ftb200_beam_search_step: vocabulary too large for the bit map of penalised columns");
         return FTB200_UNSUPPORTED;
     }
-    const int grid = p->local_batch_size * p->beam_width;
-#define FTB_LAUNCH_BEAM(DT)                                                                                            \
-    do {                                                                                                               \
-        FTB_CUDA_CHECK(cudaFuncSetAttribute(beam_step_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
-                                            200 * 1024));                                                              \
-        beam_step_kernel<DT><<<grid, kBeamThreads, smem, st>>>(K);                                                     \
-    } while (0)
-    switch (p->dtype) {
-        case FTB200_F32: FTB_LAUNCH_BEAM(FTB200_F32); break;
-        case FTB200_F16: FTB_LAUNCH_BEAM(FTB200_F16); break;
-        default: FTB_LAUNCH_BEAM(FTB200_BF16); break;
+    // the parents of all levels in shared memory where they fit
+    K.chain_levels = 0;
+    if (penalise && p->step > 1) {
+        const size_t table = (size_t)(p->step - 1) * (p->beam_width + 2) * 2 + 32 * (size_t)(p->beam_width + 1) * 2 + 16;
+        if (smem + table <= kBeamMaxSmem) {
+            K.chain_levels = p->step - 1;
+            smem += table;
+        }
     }
-#undef FTB_LAUNCH_BEAM
-    FTB_CUDA_CHECK(cudaGetLastError());
-    note_launch(1);
-    return FTB200_OK;
+    switch (p->dtype) {
+        case FTB200_F32: return beam_launch<FTB200_F32>(K, smem, (cudaStream_t)p->stream);
+        case FTB200_F16: return beam_launch<FTB200_F16>(K, smem, (cudaStream_t)p->stream);
+        default: return beam_launch<FTB200_BF16>(K, smem, (cudaStream_t)p->stream);
+    }
 }

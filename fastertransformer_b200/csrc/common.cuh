@@ -90,6 +90,25 @@ __device__ __forceinline__ uint2 ld_nc_v2(const void* p)
     return r;
 }
 
+// 16-byte asynchronous copy global -> shared (both 16-byte aligned), past L1.
+__device__ __forceinline__ void cp_async16(u32 smem, const void* g)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template<int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void sts_u32(u32 a, u32 v)
+{
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
 // Tells the compiler that a pointer loaded from a structure points into shared memory, so that it emits
 // ld.shared / st.shared instead of generic accesses (every pointer of the kernel's shared-memory map qualifies).
 #define FTB_ASSUME_SHARED(p) __builtin_assume(__isShared(p))

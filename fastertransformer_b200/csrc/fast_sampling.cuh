@@ -74,10 +74,6 @@ __device__ __forceinline__ void cp_async4(u32 saddr, const void* g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(g) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit()
-{
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -444,10 +440,6 @@ constexpr int kFPreWords = 48;
 enum { kPreStateK = 0, kPreStateP = 12, kPreSkipK = 24, kPreSkipP, kPreFin, kPreEnd, kPreK, kPrePk, kPrePp, kPreTemp,
        kPreRep };
 
-__device__ __forceinline__ void cp_async16(u32 saddr, const void* g)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr), "l"(g) : "memory");
-}
 
 // Arguments of row nr on their way into pre[] (thread 0 only).
 static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
@@ -621,11 +613,6 @@ __device__ __forceinline__ uint2 lds_v2(u32 addr)
 __device__ __forceinline__ void cp_async8(u32 saddr, const void* g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(saddr), "l"(g) : "memory");
-}
-template<int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ u32 atoms_add(u32 addr, u32 v)
 {

@@ -24,6 +24,21 @@ def _ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+def _addr(t):
+    return None if t is None else t.data_ptr()
+
+
+_HYPS = [f for f, _ in BeamHyps._fields_[:-1]]
+_BEAM_SCALARS = ("temperature", "repetition_penalty", "presence_penalty", "min_length", "beam_search_diversity_rate",
+                 "len_penalty")
+
+
+def _scalar(inputs, name):
+    """First value of a host argument, None where it is absent."""
+    v = inputs.get(name)
+    return None if v is None else (v.flat[0] if isinstance(v, np.ndarray) else np.atleast_1d(np.asarray(v)).reshape(-1)[0]).item()
+
+
 class _SamplingLayerState:
     """Buffers one reference sampling layer keeps (BaseSamplingLayer.cc:29-53, TopK/TopP allocateBuffer)."""
 
@@ -48,6 +63,7 @@ class DynamicDecodeLayer:
         self._device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self._workspace = None
         self._beam_ws = None
+        self._beam_key = self._beam_blocks = None
         self._gate = {}
         self.time_kernels = False   # when set, CUDA events bracket each fused launch (kernel_events)
         self.kernel_events = []
@@ -263,34 +279,58 @@ class DynamicDecodeLayer:
                 ite * lbs, Vp, step, st))
             self.launches += 1
 
-        def scalar(key, default):
-            v = inputs.get(key)
-            return default if v is None else np.atleast_1d(np.asarray(v)).reshape(-1)[0]
-
         sub = 1 if self.has_diff_runtime_args else lbs
         n_sub = lbs // sub
+        hyps = outputs.get("beam_hyps")
+        bias, il, olp = inputs.get("embedding_bias"), inputs.get("input_lengths"), outputs.get("output_log_probs")
+        src, tgt = inputs.get("src_cache_indirection"), outputs.get("tgt_cache_indirection")
+        # The argument blocks of a call (one per sub-batch) are kept between steps and filled again when one of the
+        # caller's pointers or scalars changes; the step's own values are written every time.
+        key = (logits.dtype, B, K, Vp, L, mil, ite, lbs, sub, self._stream, out_ids.data_ptr(), outputs["parent_ids"].data_ptr(),
+               outputs["finished"].data_ptr(), outputs["sequence_length"].data_ptr(), outputs["cum_log_probs"].data_ptr(),
+               inputs["end_id"].data_ptr(), _addr(bias), _addr(il), _addr(olp),
+               None if hyps is None else tuple((f, _addr(hyps.get(f))) for f in _HYPS) + (int(hyps.get("early_stopping", True)),),
+               tuple(_scalar(inputs, k) for k in _BEAM_SCALARS))
+        if key != self._beam_key:
+            self._beam_blocks = self._fill_beam(outputs, inputs, key, B, K, Vp, L, mil, ite, lbs, sub, n_sub, es)
+            self._beam_key = key
+        for P, ref, row0 in self._beam_blocks:
+            P.step = step
+            P.logits = logits.data_ptr() + row0 * Vp * es
+            P.src_cache_indirection = None if src is None else src.data_ptr()
+            P.tgt_cache_indirection = None if tgt is None else tgt.data_ptr()
+            rc = lib.ftb200_beam_search_step(ref)
+            if rc:
+                check(rc)
+            self.launches += lib.ftb200_last_launch_count()
+        return self._stop_criteria(outputs, inputs, B, step, lbs, ite * lbs, beam=K)
+
+    def _fill_beam(self, outputs, inputs, key, B, K, Vp, L, mil, ite, lbs, sub, n_sub, es):
         need = C.c_size_t(0)
         check(lib.ftb200_beam_workspace_bytes(sub, K, C.byref(need)))
         if self._beam_ws is None or self._beam_ws.numel() < need.value:
             self._beam_ws = torch.empty(need.value, dtype=torch.uint8, device=self.device)
-        hyps = outputs.get("beam_hyps")
+        if "repetition_penalty" in inputs and "presence_penalty" in inputs:
+            raise RuntimeError("[FT][ERROR] Found ambiguous parameters repetition_penalty and "
+                               "presence_penalty which are mutually exclusive.")
+
+        def scalar(name, default):
+            v = _scalar(inputs, name)
+            return default if v is None else v
+
+        blocks = []
         for d_ite in range(ite * n_sub, (ite + 1) * n_sub):
             row0 = d_ite * sub * K          # first batch-beam row of this sub-batch
             P = BeamParams()
-            P.dtype = _DT[logits.dtype]
+            P.dtype = _DT[inputs["logits"].dtype]
             P.batch_size, P.local_batch_size, P.ite, P.beam_width = B, sub, d_ite, K
             P.vocab_size, P.vocab_size_padded = self.vocab_size, Vp
-            P.step, P.max_input_length, P.max_seq_len = step, mil, L
-            P.logits = logits.data_ptr() + row0 * Vp * es
-            bias = inputs.get("embedding_bias")
-            P.embedding_bias = None if bias is None else bias.data_ptr()
+            P.max_input_length, P.max_seq_len = mil, L
+            P.embedding_bias = _addr(inputs.get("embedding_bias"))
             P.end_ids = inputs["end_id"].data_ptr() + d_ite * sub * 4
             il = inputs.get("input_lengths")
             P.input_lengths = None if il is None else il.data_ptr() + row0 * 4
             P.temperature = float(scalar("temperature", 1.0))
-            if "repetition_penalty" in inputs and "presence_penalty" in inputs:
-                raise RuntimeError("[FT][ERROR] Found ambiguous parameters repetition_penalty and "
-                                   "presence_penalty which are mutually exclusive.")
             if inputs.get("repetition_penalty") is not None:
                 P.penalty_type, P.repetition_penalty = 1, float(scalar("repetition_penalty", 1.0))
             elif inputs.get("presence_penalty") is not None:
@@ -300,29 +340,24 @@ class DynamicDecodeLayer:
             P.min_length = int(scalar("min_length", 0))
             P.diversity_rate = float(scalar("beam_search_diversity_rate", 0.0))
             P.length_penalty = float(scalar("len_penalty", 0.0))
-            P.output_ids = out_ids.data_ptr()
+            P.output_ids = outputs["output_ids"].data_ptr()
             P.parent_ids = outputs["parent_ids"].data_ptr()
             P.finished = outputs["finished"].data_ptr() + row0
             P.sequence_length = outputs["sequence_length"].data_ptr() + row0 * 4
             P.cum_log_probs = outputs["cum_log_probs"].data_ptr() + row0 * 4
-            olp = outputs.get("output_log_probs")
-            P.output_log_probs = None if olp is None else olp.data_ptr()
-            src, tgt = inputs.get("src_cache_indirection"), outputs.get("tgt_cache_indirection")
-            P.src_cache_indirection = None if src is None else src.data_ptr()
-            P.tgt_cache_indirection = None if tgt is None else tgt.data_ptr()
+            P.output_log_probs = _addr(outputs.get("output_log_probs"))
+            hyps = outputs.get("beam_hyps")
             if hyps is not None:
                 H = BeamHyps()
-                for f, _ in BeamHyps._fields_[:-1]:
-                    t = hyps.get(f)
-                    setattr(H, f, None if t is None else t.data_ptr())
+                for f in _HYPS:
+                    setattr(H, f, _addr(hyps.get(f)))
                 H.early_stopping = int(hyps.get("early_stopping", True))
                 P.beam_hyps = C.pointer(H)
             P.workspace = self._beam_ws.data_ptr()
             P.workspace_bytes = self._beam_ws.numel()
-            P.stream = st.value
-            check(lib.ftb200_beam_search_step(C.byref(P)))
-            self.launches += 1
-        return self._stop_criteria(outputs, inputs, B, step, lbs, ite * lbs, beam=K)
+            P.stream = self._stream
+            blocks.append((P, C.byref(P), row0))
+        return blocks
 
     def _stop_criteria(self, outputs, inputs, B, step, lbs, lo, beam=1):
         """Stop words, length limit and should_stop (DynamicDecodeLayer.cc:447-473)."""

@@ -273,7 +273,7 @@ size_t ftb200_static_scratch_bytes(void);
 int    ftb200_decode_step_sampling_static(const ftb200_sampling_params* p);
 
 /* ------------------------------------------------------------------------------------------
- * Beam search, one step (beam_width > 1), one launch.
+ * Beam search, one step (beam_width > 1), two launches (the rows, then the merge of each entry).
  *
  * Replaces what OnlineBeamSearchLayer<T>::forward launches
  * (layers/beam_search_layers/BaseBeamSearchLayer.cu:181-289, OnlineBeamSearchLayer.cu:88-175):
