@@ -157,6 +157,18 @@ struct SpShared {
     float agg[(kSpMaxN * kSpAreaCap) / 256];
 };
 
+// Bias of a 32-bit word of logits in the logits type's arithmetic (half: two rounded sums; fp32: one).  bf16 sums stay
+// fp32 in the reference's order of operations and do not fit the word: they are added per column.
+template<int DT>
+__device__ __forceinline__ u32 sp_add_bias(u32 x, u32 b)
+{
+    if (DT == FTB200_F16) {
+        const __half2 r = __hadd2(*reinterpret_cast<const __half2*>(&x), *reinterpret_cast<const __half2*>(&b));
+        return *reinterpret_cast<const u32*>(&r);
+    }
+    return __float_as_uint(__uint_as_float(x) + __uint_as_float(b));
+}
+
 // Loads this CTA's columns of row r and stores their values after temperature and bias.
 template<int DT>
 __device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, const char* rowp, float* y, int rank, int lgvt,
@@ -168,6 +180,9 @@ __device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, con
         // a chunk of 1024 columns starts on a 16-byte boundary: whole vectors, four in flight per thread
         constexpr int U   = 4;
         const int     lgv = lgvt - LGE, nv = nchunk << lgv;
+        const bool    bias = X.apply_temp && X.bias != nullptr, bias_vec = DT != FTB200_BF16 && bias && ((size_t)X.bias & 15) == 0;
+        Xf            T    = X;  // (a bias that comes by the vector is added here)
+        T.bias             = bias_vec ? nullptr : X.bias;
         for (int i0 = tid; i0 < nv; i0 += kThreads * U) {
             uint4 q[U];
 #pragma unroll
@@ -185,9 +200,14 @@ __device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, con
                 }
                 float f[EPV];
                 if (v + EPV <= vocab) {
+                    if (bias_vec) {
+                        const uint4 b = ld_nc_v4((const char*)X.bias + (size_t)v * ES);
+                        q[u]          = make_uint4(sp_add_bias<DT>(q[u].x, b.x), sp_add_bias<DT>(q[u].y, b.y),
+                                                   sp_add_bias<DT>(q[u].z, b.z), sp_add_bias<DT>(q[u].w, b.w));
+                    }
 #pragma unroll
                     for (int e = 0; e < EPV; ++e) {
-                        f[e] = temp_value<DT>(X, raw_bits<DT>(q[u], e), v + e);
+                        f[e] = temp_value<DT>(T, raw_bits<DT>(q[u], e), v + e);
                     }
                 }
                 else {
@@ -340,39 +360,36 @@ __device__ __noinline__ void sp_chain_sums(const float* y, int nchunk, float max
     }
 }
 
-// Per-thread walk over the CTA's values: f(local index, value) for every column that can be selected and is not below
-// thr.  Four vectors of four are in flight per thread; one compare rules a vector out.
+// Per-thread walk over the CTA's values: f(local index, value) for every column not below thr, which has to lie above the
+// values that cannot be selected.  Sixteen values a round become a mask without a branch; f stands in the loop over its
+// bits once (inlined per value it was several times the instruction cache, and a branch per value cost more than the
+// compare).
 template<class F>
-__device__ __forceinline__ void sp_sweep(const float* y, int ny, float neg_max, float thr, F&& f)
+__device__ __forceinline__ void sp_sweep(const float* y, int ny, float thr, F&& f)
 {
     FTB_ASSUME_SHARED(y);
     constexpr int U = 4;
     for (int i0 = 4 * (int)threadIdx.x; i0 < ny; i0 += 4 * kThreads * U) {
-        float4 v[U];
+        u32 hits = 0;
 #pragma unroll
         for (int q = 0; q < U; ++q) {
-            const int i = i0 + q * 4 * kThreads;
-            v[q]        = i < ny ? *(const float4*)(y + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            const int    i = i0 + q * 4 * kThreads;
+            const float4 v = i < ny ? *(const float4*)(y + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            hits |= (v.x >= thr ? 1u : 0u) << (4 * q);
+            hits |= (v.y >= thr ? 2u : 0u) << (4 * q);
+            hits |= (v.z >= thr ? 4u : 0u) << (4 * q);
+            hits |= (v.w >= thr ? 8u : 0u) << (4 * q);
         }
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-            const float m = fmaxf(fmaxf(v[q].x, v[q].y), fmaxf(v[q].z, v[q].w));
-            if (m >= thr && m > neg_max) {
-                const int i = i0 + q * 4 * kThreads;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float x = e == 0 ? v[q].x : (e == 1 ? v[q].y : (e == 2 ? v[q].z : v[q].w));
-                    if (x >= thr && x > neg_max) {
-                        f(i + e, x);
-                    }
-                }
-            }
+        while (hits != 0) {
+            const int e = __ffs(hits) - 1, i = i0 + (e >> 2) * 4 * kThreads + (e & 3);
+            hits &= hits - 1;
+            f(i, y[i]);
         }
     }
 }
 
 // Counts of the CTA's selectable columns per bin.
-static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float neg_max, float maxv, u32 hist)
+static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float lowest, float maxv, u32 hist)
 {
     FTB_ASSUME_SHARED(y);
     constexpr int U = 4;
@@ -388,10 +405,9 @@ static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float 
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float x = e == 0 ? v[q].x : (e == 1 ? v[q].y : (e == 2 ? v[q].z : v[q].w));
-                const u32   a = hist + 4u * (u32)sp_bin(maxv - x);
-                if (x > neg_max) {
-                    reds_add(a, 1u);
-                }
+                asm volatile("{\n .reg .pred p;\n setp.ge.f32 p, %0, %1;\n @p red.shared.add.u32 [%2], 1;\n}" ::"f"(x), "f"(lowest),
+                             "r"(hist + 4u * (u32)sp_bin(maxv - x))
+                             : "memory");
             }
         }
     }
@@ -836,6 +852,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     const bool       specials = P.apply_rep || P.bad_words != nullptr || P.apply_minlen;
     const bool       softmax  = mode == 2 || want_lp;
     const float      neg_max  = DT == FTB200_F16 ? -65504.0f : -FLT_MAX;
+    const float      lowest   = __uint_as_float(__float_as_uint(neg_max) - 1u);  // smallest value above neg_max
     FTB_ASSUME_SHARED(y);
 
     // ---- set-up: counters, the row's slice, special columns ----
@@ -933,7 +950,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
         const u32 bs1 = P.max_top_k <= 16 ? 128 : 256;
         const int sh1 = bs1 == 128 ? 7 : 8;
         u32       tie = 0;
-        sp_sweep(y, ny, neg_max, maxv, [&](int i, float x) {
+        sp_sweep(y, ny, maxv, [&](int i, float x) {
             if (fkey(x) != kmax) {
                 return;  // (a zero of the other sign)
             }
@@ -954,7 +971,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     }
 
     // ---- counts per bin; for a soft-max row the ordered denominator ----
-    sp_count_bins(y, ny, neg_max, maxv, smem_addr(M.hist));
+    sp_count_bins(y, ny, lowest, maxv, smem_addr(M.hist));
     trace_mark(O.trace, 3);
     if (softmax) {
         sp_chain_sums<DT, LGN>(y, nchunk, maxv, smem_addr(X.wsum), rank);
@@ -1044,7 +1061,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     if (p_max >= top_p) {
         // arg-max shortcut of topp_beam_topk_kernel (sampling_topp_kernels.cu:801-860): first column of the maximum
         u32 col = 0xffffffffu;
-        sp_sweep(y, ny, neg_max, maxv, [&](int i, float v) {
+        sp_sweep(y, ny, maxv, [&](int i, float v) {
             if (v == maxv) {
                 const u32 c = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
                 col         = c < col ? c : col;
@@ -1102,12 +1119,12 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
         // (a thread meets few candidates: the first four are remembered, more make it walk again)
         u32         mine = 0, tot;
         u64         keep0 = 0, keep1 = 0, keep2 = 0, keep3 = 0;
-        const float thr  = sp_floor_value(maxv, b_thr);
+        const float thr  = fmaxf(sp_floor_value(maxv, b_thr), lowest);
         auto        entry = [&](int i, float v) {
             const u32 col = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
             return ((u64)(~fkey(v)) << 32) | col;
         };
-        sp_sweep(y, ny, neg_max, thr, [&](int i, float v) {
+        sp_sweep(y, ny, thr, [&](int i, float v) {
             if (sp_bin(maxv - v) <= b_thr) {
                 keep3 = keep2, keep2 = keep1, keep1 = keep0;
                 keep0 = entry(i, v);
@@ -1135,7 +1152,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
             }
             else {
                 u32 w = 0;
-                sp_sweep(y, ny, neg_max, thr, [&](int i, float v) {
+                sp_sweep(y, ny, thr, [&](int i, float v) {
                     if (sp_bin(maxv - v) <= b_thr) {
                         dst_u64(dst + 8u * w, entry(i, v));
                         ++w;
@@ -1298,7 +1315,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     for (int q = 1; q < n; ++q) {
         first[q] = q < owners ? s_start[q] : 0xffffffffu;
     }
-    sp_sweep(y, ny, neg_max, sp_floor_value(maxv, b_thr), [&](int, float v) {
+    sp_sweep(y, ny, fmaxf(sp_floor_value(maxv, b_thr), lowest), [&](int, float v) {
         const int b = sp_bin(maxv - v);
         if (b <= b_thr) {
             const u32 pos = atomicAdd(&M.hist[b], 1u), e = excl[b];
@@ -1381,7 +1398,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     const float e_sel = p_sel * denom, e_lo = e_sel * (1.0f - slack) - tiny, pad = 1e-4f + 2e-6f * fabsf(maxv);
     const float y_lo  = e_lo > 1e-37f ? maxv + __logf(e_lo) * 1.00001f - pad : -INFINITY;
     const float y_hi  = maxv + __logf(fmaxf(e_sel * (1.0f + slack) + tiny, 1e-37f)) * 0.99999f + pad;
-    sp_sweep(y, ny, neg_max, y_lo, [&](int i, float v) {
+    sp_sweep(y, ny, fmaxf(y_lo, lowest), [&](int i, float v) {
         if (v <= y_hi && sp_prob<DT>(v, maxv, denom) == p_sel) {
             const u32 pos = datom_add(cluster_addr(smem_addr(&X.n_cls), 0), 1u);
             if (pos < (u32)kSpAreaCap) {
