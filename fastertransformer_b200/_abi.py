@@ -25,6 +25,18 @@ class SamplingParams(C.Structure):
     ]
 
 
+class SetupParams(C.Structure):
+    """ftb200_setup_params."""
+    _fields_ = [
+        ("batch", C.c_int), ("topk_states", C.c_void_p), ("topp_states", C.c_void_p), ("seed", C.c_ulonglong),
+        ("seeds", C.c_void_p), ("topk_top_k", C.c_uint32), ("topp_top_k", C.c_uint32), ("top_ks_size", C.c_int),
+        ("top_ps_size", C.c_int), ("top_p", C.c_float), ("topk_ks", C.c_void_p), ("topk_ps", C.c_void_p),
+        ("topk_skip", C.c_void_p), ("topp_ks", C.c_void_p), ("topp_ps", C.c_void_p), ("topp_skip", C.c_void_p),
+        ("topp_initial", C.c_void_p), ("topp_decay", C.c_void_p), ("top_p_decay", C.c_void_p), ("topp_min", C.c_void_p),
+        ("top_p_min", C.c_void_p), ("topp_reset_ids", C.c_void_p), ("top_p_reset_ids", C.c_void_p), ("stream", C.c_void_p),
+    ]
+
+
 class StopParams(C.Structure):
     """ftb200_stop_params."""
     _fields_ = [

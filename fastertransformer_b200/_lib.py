@@ -12,7 +12,7 @@ class FtbError(RuntimeError):
         self.status = status
 
 
-from ._abi import BeamHyps, BeamParams, GatherTreeParams, SamplingParams, StopParams  # noqa: E402,F401
+from ._abi import BeamHyps, BeamParams, GatherTreeParams, SamplingParams, SetupParams, StopParams  # noqa: E402,F401
 
 
 def _load():
@@ -30,6 +30,7 @@ def _load():
     l.ftb200_setup_topp_runtime_args.argtypes = [
         C.c_int, C.c_uint32, C.c_void_p, C.c_int, C.c_float, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p,
         C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    l.ftb200_setup_sampling.argtypes = [C.POINTER(SetupParams)]
     l.ftb200_sampling_workspace_bytes.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_size_t)]
     l.ftb200_decode_step_sampling.argtypes = [C.POINTER(SamplingParams)]
     l.ftb200_decode_step.argtypes = [C.POINTER(SamplingParams), C.POINTER(StopParams), C.c_int, C.POINTER(C.c_int)]

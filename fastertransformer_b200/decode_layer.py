@@ -10,7 +10,7 @@ import ctypes as C
 import numpy as np
 import torch
 
-from ._lib import BeamHyps, BeamParams, SamplingParams, StopParams, check, lib
+from ._lib import BeamHyps, BeamParams, SamplingParams, SetupParams, StopParams, check, lib
 
 _DT = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 CURAND_STATE_BYTES = 48  # sizeof(curandState_t), XORWOW
@@ -40,15 +40,36 @@ def _scalar(inputs, name):
 
 
 class _SamplingLayerState:
-    """Buffers one reference sampling layer keeps (BaseSamplingLayer.cc:29-53, TopK/TopP allocateBuffer)."""
+    """Buffers one reference sampling layer keeps (BaseSamplingLayer.cc:29-53, TopK/TopP allocateBuffer): device tensors
+    curand, top_ks (uint32 payload), top_ps, skip, and skip_host."""
+    active = False
 
-    def __init__(self, batch, device):
-        self.curand = torch.zeros(batch * CURAND_STATE_BYTES, dtype=torch.uint8, device=device)
-        self.top_ks = torch.zeros(batch, dtype=torch.int32, device=device)  # uint32 payload
-        self.top_ps = torch.zeros(batch, dtype=torch.float32, device=device)
-        self.skip = torch.zeros(batch, dtype=torch.uint8, device=device)
-        self.skip_host = np.ones(batch, dtype=bool)
-        self.active = False
+
+class _Pack:
+    """Host arrays and device-only buffers of a set-up, laid out behind each other in one device allocation; the host
+    part travels in one copy from page-locked memory."""
+
+    def __init__(self):
+        self.parts, self.size = [], 0
+
+    def add(self, owner, name, dtype, count, host=None):
+        size = dtype.itemsize * count
+        self.parts.append((owner, name, dtype, self.size, size, host))
+        self.size += (size + 63) // 64 * 64
+
+    def place(self, device):
+        """Sets the attributes `name` of the owners to tensors; host parts have to be added first."""
+        upload = max([at + size for _, _, _, at, size, host in self.parts if host is not None], default=0)
+        dev = torch.empty(self.size, dtype=torch.uint8, device=device)
+        if upload:
+            staged = torch.empty(upload, dtype=torch.uint8, pin_memory=True)
+            bytes_ = staged.numpy()
+            for _, _, _, at, size, host in self.parts:
+                if host is not None:
+                    bytes_[at:at + size] = host.view(np.uint8)
+            dev[:upload].copy_(staged, non_blocking=True)
+        for owner, name, dtype, at, size, _ in self.parts:
+            setattr(owner, name, dev[at:at + size].view(dtype))
 
 
 class DynamicDecodeLayer:
@@ -134,70 +155,75 @@ class DynamicDecodeLayer:
         self.penalty_default = default_pen
         self.penalty_host = self._broadcast(pen, B, np.float32, default_pen)
         self.min_length_host = self._broadcast(self._arg(a, "min_length"), B, np.int32, 0)
-        self.temperature = torch.from_numpy(self.temperature_host).to(dev)
-        self.penalty = torch.from_numpy(self.penalty_host).to(dev)
-        self.min_length = torch.from_numpy(self.min_length_host).to(dev)
-
-        self.topk = _SamplingLayerState(B, dev)
-        self.topp = _SamplingLayerState(B, dev)
-        for layer in (self.topk, self.topp):
-            if seeds is None:
-                check(lib.ftb200_curand_init(_ptr(layer.curand), B, 0, None, st))
-            elif seeds.size == 1:
-                check(lib.ftb200_curand_init(_ptr(layer.curand), B, int(seeds[0]), None, st))
-            else:
-                if seeds.size != B:
-                    raise RuntimeError("[FT][ERROR] random_seeds must be of shape [1] or [batch_size]")
-                sd = torch.from_numpy(seeds.astype(np.uint64).view(np.int64)).to(dev)
-                check(lib.ftb200_curand_init(_ptr(layer.curand), B, 0, _ptr(sd), st))
-                torch.cuda.current_stream(dev).synchronize()
-
-        # TopKSamplingLayer::setup (TopKSamplingLayer.cu:134-186)
+        # TopKSamplingLayer::setup (TopKSamplingLayer.cu:134-186), TopPSamplingLayer::setup (TopPSamplingLayer.cu:184-253):
+        # the kernel writes the normalised arguments on the device; what the host side needs of them follows from the
+        # same rules here, so nothing is read back.
         k_arr = top_k.astype(np.uint32) if top_k is not None else np.zeros(1, np.uint32)
-        k_scalar = int(k_arr.max())
-        p_scalar = float(top_p[0]) if top_p is not None else 0.0
-        if k_arr.size > 1:
-            self.topk.top_ks.copy_(torch.from_numpy(k_arr.view(np.int32)))
-        if top_p is not None and top_p.size > 1:
-            self.topk.top_ps.copy_(torch.from_numpy(top_p.astype(np.float32)))
-        check(lib.ftb200_setup_topk_runtime_args(B, k_scalar, _ptr(self.topk.top_ks), int(k_arr.size), p_scalar,
-                                                 _ptr(self.topk.top_ps), 0 if top_p is None else int(top_p.size),
-                                                 _ptr(self.topk.skip), st))
-        self.topk.skip_host = self.topk.skip.cpu().numpy().astype(bool)
-        self.max_top_k = int(self.topk.top_ks.cpu().numpy().view(np.uint32).max())
-        self.topk.active = True
-
-        # TopPSamplingLayer::setup (TopPSamplingLayer.cu:184-253)
-        if top_p is None:
-            self.topp.skip_host[:] = True
-            self.topp.active = False
+        p_arr = None if top_p is None else top_p.astype(np.float32)
+        for v in (k_arr, p_arr):
+            if v is not None and v.size not in (1, B):
+                raise RuntimeError("[FT][ERROR] runtime_top_k and runtime_top_p must be of shape [1] or [batch_size]")
+        if seeds is not None and seeds.size not in (1, B):
+            raise RuntimeError("[FT][ERROR] random_seeds must be of shape [1] or [batch_size]")
+        zero = np.float32(0.0)
+        k_all = np.broadcast_to(k_arr if k_arr.size > 1 else k_arr.max(), (B,))
+        p_all = np.broadcast_to(zero if p_arr is None else (p_arr if p_arr.size > 1 else p_arr[0]), (B,))
+        k_topk = np.where((k_all == 0) & (p_all == zero), np.uint32(1), k_all)
+        self.topk, self.topp = _SamplingLayerState(), _SamplingLayerState()
+        self.topk.skip_host, self.topk.active = k_topk == 0, True
+        self.max_top_k = int(np.minimum(k_topk, 1024).max())
+        cost = 1.0 + np.minimum(k_topk, 1024) / 128.0
+        if p_arr is None:
+            self.topp.skip_host = np.ones(B, dtype=bool)
         else:
-            self.topp.initial = torch.zeros(B, dtype=torch.float32, device=dev)
-            self.topp.decay = torch.zeros(B, dtype=torch.float32, device=dev)
-            self.topp.min = torch.zeros(B, dtype=torch.float32, device=dev)
-            self.topp.reset = torch.zeros(B, dtype=torch.int32, device=dev)
-            if k_arr.size > 1:
-                self.topp.top_ks.copy_(torch.from_numpy(k_arr.view(np.int32)))
-            if top_p.size > 1:
-                self.topp.top_ps.copy_(torch.from_numpy(top_p.astype(np.float32)))
-            check(lib.ftb200_setup_topp_runtime_args(
-                B, int(k_arr[0]), _ptr(self.topp.top_ks), int(k_arr.size), p_scalar, _ptr(self.topp.top_ps),
-                int(top_p.size), _ptr(self.topp.skip), _ptr(self.topp.initial), _ptr(self.topp.decay),
-                _ptr(a.get("top_p_decay")), _ptr(self.topp.min), _ptr(a.get("top_p_min")), _ptr(self.topp.reset),
-                _ptr(a.get("top_p_reset_ids")), st))
-            self.topp.skip_host = self.topp.skip.cpu().numpy().astype(bool)
+            k_first = np.broadcast_to(k_arr if k_arr.size > 1 else k_arr[0], (B,))
+            self.topp.skip_host = (k_first > 0) | (p_all == zero)
             self.topp.active = True
-        self._row_cost = self._estimate_row_cost()
+            cost = np.where(self.topk.skip_host, 10.0 + 8.0 * np.clip(p_all, 0.0, 1.0), cost)
+        # Relative cost of a row, for the launch order: top-p rows cost most, then top-k by k.
+        self._row_cost = cost
+        order = np.argsort(-cost, kind="stable").astype(np.int32)
 
-    def _estimate_row_cost(self):
-        """Relative cost of a row for the launch order: top-p rows cost most (three reads of the row and a
-        sort of the nucleus), then top-k by k."""
-        k = self.topk.top_ks.cpu().numpy().view(np.uint32).astype(np.float64)
-        cost = 1.0 + k / 128.0
+        pack = _Pack()
+        per_row_seeds = seeds is not None and seeds.size > 1
+        if per_row_seeds:
+            pack.add(self, "_seeds", torch.int64, B, seeds.astype(np.uint64))
+        pack.add(self, "temperature", torch.float32, B, self.temperature_host)
+        pack.add(self, "penalty", torch.float32, B, self.penalty_host)
+        pack.add(self, "min_length", torch.int32, B, self.min_length_host)
+        pack.add(self, "_order", torch.int32, B, order)
+        for layer in (self.topk, self.topp):
+            pack.add(layer, "top_ks", torch.int32, B, k_arr if k_arr.size > 1 else None)
+            pack.add(layer, "top_ps", torch.float32, B, p_arr if p_arr is not None and p_arr.size > 1 else None)
+        for layer in (self.topk, self.topp):
+            pack.add(layer, "skip", torch.uint8, B)
+            pack.add(layer, "curand", torch.uint8, B * CURAND_STATE_BYTES)
         if self.topp.active:
-            p = self.topp.top_ps.cpu().numpy().astype(np.float64)
-            cost = np.where(self.topk.skip_host, 10.0 + 8.0 * p, cost)
-        return cost
+            for name, dtype in (("initial", torch.float32), ("decay", torch.float32), ("min", torch.float32),
+                                ("reset", torch.int32)):
+                pack.add(self.topp, name, dtype, B)
+        with torch.cuda.stream(self.stream):  # (None: the current one)
+            pack.place(dev)
+        tk, tp = self.topk, self.topp
+        S = SetupParams()
+        S.batch = B
+        S.topk_states, S.topp_states = tk.curand.data_ptr(), tp.curand.data_ptr()
+        if per_row_seeds:
+            S.seeds = self._seeds.data_ptr()
+        elif seeds is not None:
+            S.seed = int(seeds[0])
+        S.topk_top_k, S.topp_top_k = int(k_arr.max()), int(k_arr[0])
+        S.top_ks_size, S.top_ps_size = int(k_arr.size), 0 if p_arr is None else int(p_arr.size)
+        S.top_p = 0.0 if p_arr is None else float(p_arr[0])
+        S.topk_ks, S.topk_ps, S.topk_skip = tk.top_ks.data_ptr(), tk.top_ps.data_ptr(), tk.skip.data_ptr()
+        if tp.active:
+            S.topp_ks, S.topp_ps, S.topp_skip = tp.top_ks.data_ptr(), tp.top_ps.data_ptr(), tp.skip.data_ptr()
+            S.topp_initial, S.topp_decay = tp.initial.data_ptr(), tp.decay.data_ptr()
+            S.topp_min, S.topp_reset_ids = tp.min.data_ptr(), tp.reset.data_ptr()
+            S.top_p_decay, S.top_p_min = _addr(a.get("top_p_decay")), _addr(a.get("top_p_min"))
+            S.top_p_reset_ids = _addr(a.get("top_p_reset_ids"))
+        S.stream = st.value
+        check(lib.ftb200_setup_sampling(C.byref(S)))
 
     # ---- forward (DynamicDecodeLayer.cc:191-474, sampling branch) ---------------------------------
     def forward(self, outputs, inputs):
@@ -219,8 +245,8 @@ class DynamicDecodeLayer:
                 "temp": bool((self.temperature_host[lo:hi] != 1.0).any()),
                 "pen": bool((self.penalty_host[lo:hi] != self.penalty_default).any()),
                 "minlen": int(self.min_length_host[lo:hi].max()),
-                "order": torch.from_numpy(np.argsort(-self._row_cost[lo:hi], kind="stable").astype(np.int32))
-                .to(self.device),
+                "order": self._order if lo == 0 and hi == self.batch_size else
+                torch.from_numpy(np.argsort(-self._row_cost[lo:hi], kind="stable").astype(np.int32)).to(self.device),
             }
         self._g = g
         self._stream = self._raw_stream()  # one look-up per call, used by the sampling and the criteria launch

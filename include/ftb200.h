@@ -76,6 +76,36 @@ int ftb200_setup_topp_runtime_args(int batch, uint32_t top_k, uint32_t* top_ks, 
                                    const float* top_p_min, int32_t* top_p_reset_ids_buf,
                                    const uint32_t* top_p_reset_ids, void* stream);
 
+/* The set-up of both layers in one launch: what ftb200_curand_init does for each layer's states and the two functions
+ * above for their arguments (same meaning; topk_top_k is the largest and topp_top_k the first of the caller's values,
+ * TopKSamplingLayer.cu:160-170, TopPSamplingLayer.cu:215-224).  topp_ps == null: no top-p layer; its states are
+ * initialised all the same. */
+typedef struct ftb200_setup_params {
+    int                       batch;
+    void*                     topk_states;
+    void*                     topp_states;
+    unsigned long long        seed;
+    const unsigned long long* seeds; /* device [batch] or null */
+    uint32_t                  topk_top_k, topp_top_k;
+    int                       top_ks_size, top_ps_size;
+    float                     top_p;
+    uint32_t*                 topk_ks;
+    float*                    topk_ps;
+    uint8_t*                  topk_skip;
+    uint32_t*                 topp_ks;
+    float*                    topp_ps;
+    uint8_t*                  topp_skip;
+    float*                    topp_initial;
+    float*                    topp_decay;
+    const float*              top_p_decay;
+    float*                    topp_min;
+    const float*              top_p_min;
+    int32_t*                  topp_reset_ids;
+    const uint32_t*           top_p_reset_ids;
+    void*                     stream;
+} ftb200_setup_params;
+int ftb200_setup_sampling(const ftb200_setup_params* p);
+
 /* ------------------------------------------------------------------------------------------
  * One fused decode-sampling step.
  *
