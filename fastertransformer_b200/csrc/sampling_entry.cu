@@ -116,17 +116,31 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     for (; lgn <= 3; ++lgn) {
         A->slice = ((vocab + 1023) / 1024) << (10 - lgn);
         A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
-        if (split_smem_bytes(A->slice) <= kSpMaxSmem) {
+        if (split_smem_bytes(A->slice, kSpAreaMin) <= kSpMaxSmem) {
             break;
         }
     }
     if (lgn > 3) {
         return false;
     }
-    A->lgn            = lgn;
-    const size_t smem = split_smem_bytes(A->slice) > smem_general ? split_smem_bytes(A->slice) : smem_general;
-    const int    fit  = smem <= 105 * 1024 ? 2 : 1;
-    *whole            = lgn >= 2 && (rows << lgn) <= fit * sms;
+    A->lgn = lgn;
+    // The form that keeps every row is taken while its CTAs are resident at once, two on an SM where shared memory
+    // allows.  The collection areas: a wide nucleus of a flat row takes half of the columns, so up to 5/8 of a slice is
+    // provided for as far as that residency holds (a row beyond it costs a millisecond in the general code).
+    constexpr size_t whole_two_per_sm = 103 * 1024, two_per_sm = 107 * 1024 + 512, three_per_sm = 69 * 1024;
+    const auto       area_within = [&](size_t budget, int most) {
+        int area = (A->slice * 5 / 8 + 1023) / 1024 * 1024;
+        area     = area > most ? most : (area < kSpAreaMin ? kSpAreaMin : area);
+        while (area > kSpAreaMin && split_smem_bytes(A->slice, area) > budget) {
+            area -= 1024;
+        }
+        return area;
+    };
+    const size_t least = split_smem_bytes(A->slice, kSpAreaMin);
+    const int    ctas  = rows << lgn;
+    *whole             = lgn >= 2 && (ctas <= sms || (ctas <= 2 * sms && least <= whole_two_per_sm && smem_general <= whole_two_per_sm));
+    A->area            = *whole ? area_within(ctas <= sms ? kSpMaxSmem : whole_two_per_sm, kSpAreaMax) :
+                                  area_within(least <= three_per_sm ? three_per_sm : (least <= two_per_sm ? two_per_sm : kSpMaxSmem), kSpAreaMid);
     return true;
 }
 

@@ -5,9 +5,10 @@
 namespace ftb200 {
 
 constexpr int kSpBins     = 2048;
-constexpr int kSpAreaCap  = 5120;                   // fp32 keys a CTA can receive of a nucleus
-constexpr int kSpCandCap  = kSpAreaCap / 2;         // 64-bit candidates the leader can receive
-constexpr int kSpSub      = kSpAreaCap / 2;         // sub-buckets of the nucleus sort: four keys each and room between bins
+constexpr int kSpAreaMin  = 5120;                   // fp32 keys a CTA can receive of a nucleus: least,
+constexpr int kSpAreaMid  = 6144;                   // most where the kernel keeps to 80 registers,
+constexpr int kSpAreaMax  = 10240;                  // and most where it has 128 (multiples of 1024; the launch chooses)
+constexpr int kSpCandCap  = kSpAreaMin / 2;         // 64-bit candidates the leader can receive
 constexpr int kSpMaxN     = 8;                       // portable cluster size
 constexpr size_t kSpMaxSmem = 216 * 1024;
 constexpr int kSpMinSlice = (kNB * 4 + 1024 * 4) / 4;  // the draw's histogram and values lie over the slice
@@ -26,13 +27,14 @@ struct StopArgs {
 struct SplitArgs {
     int  lgn;         // log2 of the CTAs per row
     int  slice;       // floats of the slice area
+    int  area;        // keys of the collection area
     int* redo_flags;  // [local_batch]: 1 when the row is left to decode_sampling_kernel (null: the kernel serves it itself)
     StopArgs stop;    // (only where redo_flags is null)
 };
 
-__host__ __device__ inline size_t split_smem_bytes(int slice)
+__host__ __device__ inline size_t split_smem_bytes(int slice, int area)
 {
-    return (size_t)slice * 4 + (size_t)kSpAreaCap * 4 + (size_t)kSpBins * 8 + (size_t)kSpSub * 2;
+    return (size_t)slice * 4 + (size_t)area * 5 + (size_t)kSpBins * 8;  // (five: a key, and two 16-bit sub-buckets for four)
 }
 
 }  // namespace ftb200

@@ -138,10 +138,11 @@ static __device__ u32 block_excl_u32(u32 v, u32* total)
 // Shared-memory map of a CTA, as 32-bit addresses and pointers.
 struct SpMap {
     float* y;       // [slice] final values of this CTA's columns; local index = (column / 1024) * vt + column % vt
-    u32*   area;    // [kSpAreaCap] nucleus keys received (all CTAs) or 64-bit candidates (leader)
+    u32*   area;    // [area_cap] nucleus keys received (all CTAs) or 64-bit candidates (leader)
     u32*   merged;  // [kSpBins] counts of the whole row, then their exclusive prefix
-    u32*   sub;     // [kSpSub / 2] pairs of 16-bit sub-bucket counters
+    u32*   sub;     // [area_cap / 4] pairs of 16-bit sub-bucket counters
     u32*   hist;    // [kSpBins] counts of this CTA's columns, then cursors
+    int    area_cap;
 };
 
 struct SpShared {
@@ -154,7 +155,7 @@ struct SpShared {
     u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
     u32   p_sel, j_sel;    // crossing: probability (bits), rank inside its class
     u32   bad_order;
-    float agg[(kSpMaxN * kSpAreaCap) / 256];
+    float agg[(kSpMaxN * kSpAreaMax) / 256];
 };
 
 // Bias of a 32-bit word of logits in the logits type's arithmetic (half: two rounded sums; fp32: one).  bf16 sums stay
@@ -413,23 +414,25 @@ static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float 
     }
 }
 
-// One nucleus owner's keys (fp32 values, any order) into descending order; n <= kSpAreaCap - 64.  `excl` holds the first
-// position of every bin in the row's order, `place` is scratch for one word per bin.  A key's place inside its bin is
+// One nucleus owner's keys (fp32 values, any order) into descending order; n <= cap - 64, cap a multiple of 1024 and at
+// most PER keys for every thread.  `excl` holds the first position of every bin in the row's order, `place` is scratch for one word per bin.  A key's place inside its bin is
 // guessed from its position between the bin's edges, so that a sub-bucket of four places receives four keys on average
 // whatever the distribution is; a bin of eight keys or more shares no sub-bucket with its neighbours (two runs of equal
 // 16-bit values in one sub-bucket would take quadratic time).  Sub-buckets that come out unsorted are finished by one
 // thread each.  Returns false when a long sub-bucket would have to be ordered.
-static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* place, u32 start, int n, float maxv)
+template<int PER>
+static __device__ __forceinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* place, u32 start, int n, float maxv,
+                                                    int cap)
 {
-    constexpr int PER = kSpAreaCap / kThreads;    // keys per thread: 20
     constexpr int BPT = kSpBins / kThreads;       // bins per thread: 8
-    constexpr int WPT = kSpSub / 2 / kThreads;    // words of two 16-bit sub-bucket counters per thread: 5
+    constexpr int WMX = PER / 4;                  // words of two 16-bit sub-bucket counters per thread, at most
+    const int     nsub = cap / 2, wpt = cap / 4 / kThreads;
     FTB_ASSUME_SHARED(a);
     FTB_ASSUME_SHARED(sub);
     FTB_ASSUME_SHARED(excl);
     FTB_ASSUME_SHARED(place);
     const int tid = threadIdx.x;
-    for (int i = tid; i < kSpSub / 2; i += kThreads) {
+    for (int i = tid; i < nsub / 2; i += kThreads) {
         sub[i] = 0;
     }
     {
@@ -469,38 +472,41 @@ static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* 
             u32         o = (u32)((t - (float)b) * (float)c);
             o             = c > 0 && o >= c ? c - 1u : o;
             u32 s         = (place[b] + o) >> 2;
-            s             = s < (u32)kSpSub ? s : (u32)kSpSub - 1u;
+            s             = s < (u32)nsub ? s : (u32)nsub - 1u;
             const u32 old = atomicAdd(&sub[s >> 1], 1u << (16 * (s & 1u)));
             at[i]         = (s << 16) | ((old >> (16 * (s & 1u))) & 0xffffu);
         }
     }
     __syncthreads();
     {
-        u32 c[WPT], mine = 0, tot;
+        u32 c[WMX], mine = 0, tot;
 #pragma unroll
-        for (int i = 0; i < WPT; ++i) {
-            c[i] = sub[tid * WPT + i];
+        for (int i = 0; i < WMX; ++i) {
+            c[i] = i < wpt ? sub[tid * wpt + i] : 0u;
             mine += (c[i] & 0xffffu) + (c[i] >> 16);
         }
         u32 run = block_excl_u32(mine, &tot);
 #pragma unroll
-        for (int i = 0; i < WPT; ++i) {
-            sub[tid * WPT + i] = run | ((run + (c[i] & 0xffffu)) << 16);
+        for (int i = 0; i < WMX; ++i) {
+            if (i < wpt) {
+                sub[tid * wpt + i] = run | ((run + (c[i] & 0xffffu)) << 16);
+            }
             run += (c[i] & 0xffffu) + (c[i] >> 16);
         }
     }
     __syncthreads();
-    auto first_of = [&](int s) { return s < kSpSub ? (int)((sub[s >> 1] >> (16 * (s & 1))) & 0xffffu) : n; };
+    auto first_of = [&](int s) { return s < nsub ? (int)((sub[s >> 1] >> (16 * (s & 1))) & 0xffffu) : n; };
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         if (i * kThreads < 32 * seg && at[i] != 0xffffffffu) {
-            a[first_of((int)(at[i] >> 16)) + (int)(at[i] & 0xffffu)] = v[i];
+            const int to         = first_of((int)(at[i] >> 16)) + (int)(at[i] & 0xffffu);
+            a[to < cap ? to : 0] = v[i];
         }
     }
     __syncthreads();
     // a sub-bucket of equal values (16-bit logits have many) is in order already; the others are short.  Where two
     // neighbours stand the wrong way round is noted first, so that a long run of equal values is not walked.
-    __shared__ u32 s_wrong[kSpAreaCap / 32];
+    __shared__ u32 s_wrong[PER * kThreads / 32];
     __shared__ u32 s_long[64], s_nlong;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
@@ -517,7 +523,7 @@ static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* 
     }
     __syncthreads();
     bool ok = true;
-    for (int s = tid; s < kSpSub; s += kThreads) {
+    for (int s = tid; s < nsub; s += kThreads) {
         const int lo = first_of(s), hi = first_of(s + 1);
         if (hi - lo < 2) {
             continue;
@@ -837,7 +843,7 @@ __device__ __forceinline__ void sp_write_topp(const KParams& P, const RowOut& O,
 
 // One row on the cluster.  Every branch that skips a cluster barrier depends on values that all CTAs hold alike.
 // Returns (leader only) whether the row is decided.
-template<int DT, int LGN>
+template<int DT, int LGN, bool WHOLE>
 __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, const SpMap& M, SpShared& X, const RowOut& O, int mode,
                                        bool want_lp)
 {
@@ -1299,9 +1305,9 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     if (tid <= kSpMaxN) {
         s_K.start[tid] = s_start[tid];
     }
-    const bool fits = N > 0 && __syncthreads_and(tid >= kSpMaxN || s_start[tid + 1] - s_start[tid] <= (u32)kSpAreaCap - 64u);
+    const bool fits = N > 0 && __syncthreads_and(tid >= kSpMaxN || s_start[tid + 1] - s_start[tid] <= (u32)M.area_cap - 64u);
     if (!fits) {
-        return sp_leave(O, 4);
+        return sp_leave(O, 6);
     }
     trace_mark(O.trace, 10);
     // a range of every owner's area for this CTA's keys, then the keys (values: ordered like the probabilities)
@@ -1332,7 +1338,8 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     if (rank < owners) {
         float* const a   = (float*)M.area;
         const int    cnt = (int)(s_start[rank + 1] - s_start[rank]);
-        bool         bad = !sp_sort_area(a, M.sub, excl, M.hist, s_start[rank], cnt, maxv);
+        bool         bad = !sp_sort_area<(WHOLE ? kSpAreaMax : kSpAreaMid) / kThreads>(a, M.sub, excl, M.hist, s_start[rank], cnt, maxv,
+                                                                                       M.area_cap);
         for (int i = tid; i < cnt; i += kThreads) {
             a[i] = sp_prob<DT>(a[i], maxv, denom);
         }
@@ -1388,7 +1395,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     const u32 verdict = X.verdict;
     trace_mark(O.trace, 14);
     if (verdict == 2) {
-        return sp_leave(O, 5);
+        return sp_leave(O, 7);
     }
     // ---- columns whose probability is that of the crossing; the one of its rank is the id ----
     const float p_sel = __uint_as_float(X.p_sel);
@@ -1401,7 +1408,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     sp_sweep(y, ny, fmaxf(y_lo, lowest), [&](int i, float v) {
         if (v <= y_hi && sp_prob<DT>(v, maxv, denom) == p_sel) {
             const u32 pos = datom_add(cluster_addr(smem_addr(&X.n_cls), 0), 1u);
-            if (pos < (u32)kSpAreaCap) {
+            if (pos < (u32)M.area_cap) {
                 dst_u32(cluster_addr(K.area + 4u * pos, 0), (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1))));
             }
         }
@@ -1412,8 +1419,8 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     }
     const u32 n_cls = X.n_cls, j_sel = X.j_sel;
     trace_mark(O.trace, 15);
-    if (n_cls > (u32)kSpAreaCap || j_sel >= n_cls) {
-        return sp_leave(O, 6);
+    if (n_cls > (u32)M.area_cap || j_sel >= n_cls) {
+        return sp_leave(O, 8);
     }
     const int id = n_cls == 1 ? (int)M.area[0] : select_jth_column(M.area, (int)n_cls, (int)j_sel, (u32*)M.y, P.vocab_padded);
     if (tid == 0) {
@@ -1504,9 +1511,10 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
     SpMap                                         M;
     M.y      = (float*)smem_raw;
     M.area   = (u32*)(M.y + A.slice);
-    M.merged = M.area + kSpAreaCap;
-    M.sub    = M.merged + kSpBins;
-    M.hist   = M.sub + kSpSub / 2;
+    M.area_cap = A.area;
+    M.merged   = M.area + A.area;
+    M.sub      = M.merged + kSpBins;
+    M.hist     = M.sub + A.area / 4;
     const int  tid = threadIdx.x, rank = (int)cluster_rank();
     const bool want_lp = P.cum_log_probs != nullptr || P.out_log_probs != nullptr;
     for (int t = (int)blockIdx.x >> LGN; t < P.local_batch; t += (int)gridDim.x >> LGN) {
@@ -1532,7 +1540,7 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
         __syncthreads();
         bool decided = true;
         if (mode != 0 && !fin) {
-            decided = sp_row<DT, LGN>(P, A, M, s_X, s_O, mode, want_lp);
+            decided = sp_row<DT, LGN, WHOLE>(P, A, M, s_X, s_O, mode, want_lp);
             __syncthreads();
         }
         if (rank == 0 && tid == 0) {
@@ -1607,7 +1615,7 @@ int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, c
 template<int DT>
 int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_general, cudaStream_t st)
 {
-    const size_t smem = split_smem_bytes(A.slice);
+    const size_t smem = split_smem_bytes(A.slice, A.area);
     if (A.redo_flags == nullptr) {
         const size_t both = smem > smem_general ? smem : smem_general;
         return A.lgn == 2 ? split_sampling_launch_n<DT, 2, true>(K, A, both, st) :
