@@ -5,6 +5,7 @@
 
 #include "sampling_params.cuh"
 #include "split_args.cuh"
+#include "vp_args.cuh"
 
 namespace ftb200 {
 
@@ -42,6 +43,10 @@ extern template int split_sampling_launch<FTB200_BF16>(const KParams&, const Spl
 size_t fast_smem_for(int hash_slots, int vocab_padded, bool topp);
 int    fast_max_history();
 int    fast_max_words();
+template<int DT>
+int vp_select_launch(const KParams& K, const VpArgs& V, size_t smem, int sms, cudaStream_t st);
+extern template int vp_select_launch<FTB200_F16>(const KParams&, const VpArgs&, size_t, int, cudaStream_t);
+extern template int vp_select_launch<FTB200_BF16>(const KParams&, const VpArgs&, size_t, int, cudaStream_t);
 template<int DT>
 int vp_merge_launch(const KParams& K, const u64* gathered, int nranks, int* overflow, int grid, cudaStream_t st);
 extern template int vp_merge_launch<FTB200_F32>(const KParams&, const u64*, int, int*, int, cudaStream_t);
@@ -539,18 +544,44 @@ extern "C" int ftb200_set_single_pass(int on)
 }
 
 // ---- vocabulary-parallel sampling (the logits of a row are split over several GPUs by column) ------
-extern "C" int ftb200_vocab_parallel_local(const ftb200_sampling_params* p, int vocab_offset, int cap,
-                                           uint64_t* records)
+// Records of the shards [0, n) that this device holds: `p` describes them together (vocab_size columns from token id
+// `offset` on, vocab_size_padded columns per shard in memory), `logits` is a host array.  Returns false when the
+// select kernel does not serve the call: fp32 logits, a bias, a row that does not fit into shared memory, top-p rows
+// (statistics form) on more than one shard, which need the general kernel's row list per shard.
+static bool plan_vp_select(const ftb200_sampling_params* p, const KParams& K, const void* const* logits, int n, int offset,
+                           int cap, u64* records, VpArgs* V, size_t* smem)
 {
-    reset_launch_count();
-    if (records == nullptr || cap < 1 || cap > kCap || vocab_offset < 0) {
-        set_error("ftb200_vocab_parallel_local: invalid argument");
-        return FTB200_INVALID_ARG;
+    if (!g_fast_path || p->dtype == FTB200_F32 || K.bias != nullptr || K.topk_states == nullptr || n > kVpMaxShards
+        || (K.topp_states != nullptr && n > 1)) {
+        return false;
     }
-    if (p != nullptr && (p->cum_log_probs != nullptr || p->output_log_probs != nullptr)) {
-        set_error("ftb200_vocab_parallel_local: log-probs are not available with a sharded vocabulary");
-        return FTB200_UNSUPPORTED;
+    vp_select_plan(*V, p->vocab_size_padded, cap, K.max_top_k, K.apply_rep ? p->step : 0, smem);
+    if (*smem > (size_t)kVpMaxSmem) {
+        return false;
     }
+    for (int i = 0; i < n; ++i) {
+        if (((size_t)logits[i] & 1) != 0) {
+            return false;
+        }
+        V->logits[i] = logits[i];
+    }
+    V->out = records, V->n_shards = n, V->vocab = p->vocab_size, V->offset = offset;
+    return true;
+}
+
+static int launch_vp_select(const KParams& K, const VpArgs& V, size_t smem, cudaStream_t st)
+{
+    const int rc = K.dtype == FTB200_F16 ? vp_select_launch<FTB200_F16>(K, V, smem, sm_count(), st) :
+                                           vp_select_launch<FTB200_BF16>(K, V, smem, sm_count(), st);
+    if (rc == FTB200_OK) {
+        note_launch(1);
+    }
+    return rc;
+}
+
+// The local pass of one shard; the caller has reset the launch count.
+static int vp_local(const ftb200_sampling_params* p, int vocab_offset, int cap, uint64_t* records)
+{
     KParams K;
     size_t  smem = 0;
     int     grid = 0;
@@ -565,11 +596,29 @@ extern "C" int ftb200_vocab_parallel_local(const ftb200_sampling_params* p, int 
     K.vp_cap       = cap;
     K.vocab_offset = vocab_offset;
     cudaStream_t st = (cudaStream_t)p->stream;
+    VpArgs       V;
+    size_t       vsmem  = 0;
+    const bool   select = plan_vp_select(p, K, &p->logits, 1, vocab_offset, cap, K.vp_out, &V, &vsmem);
+    if (select && K.topp_states == nullptr) {
+        return launch_vp_select(K, V, vsmem, st);
+    }
     FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
-    // 16-bit shards of at least 16 k columns: the single-pass kernel in its record form serves the top-k rows and
-    // leaves a list of the others (top-p rows of the statistics form, rows it cannot decide) to the kernel below
-    const bool single_pass = g_fast_path && p->dtype != FTB200_F32 && K.bias == nullptr && p->vocab_size_padded <= (1 << 20)
-                             && p->vocab_size >= 16384 + 16 && (K.apply_rep ? p->step : 0) <= fast_max_history()
+    if (select) {
+        KParams F    = K;
+        F.redo_count = K.ticket + 1;
+        F.redo_rows  = (int*)((char*)p->workspace + 256);
+        rc           = launch_vp_select(F, V, vsmem, st);
+        if (rc != FTB200_OK) {
+            return rc;
+        }
+        K.ticket        = K.ticket + 2;
+        K.row_order     = F.redo_rows;
+        K.row_count_dev = F.redo_count;
+    }
+    // wider 16-bit shards: the single-pass kernel in its record form serves the top-k rows and leaves a list of the
+    // others (top-p rows of the statistics form, rows it cannot decide) to the kernel below
+    const bool single_pass = !select && g_fast_path && p->dtype != FTB200_F32 && K.bias == nullptr
+                             && p->vocab_size_padded <= (1 << 20) && p->vocab_size >= 16384 + 16 && (K.apply_rep ? p->step : 0) <= fast_max_history()
                              && (K.bad_words != nullptr ? K.bad_words_len : 0) <= fast_max_words();
     if (single_pass) {
         const size_t fsmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, false);
@@ -608,6 +657,72 @@ extern "C" int ftb200_vocab_parallel_local(const ftb200_sampling_params* p, int 
     return rc;
 }
 
+static int vp_check(const ftb200_sampling_params* p, int vocab_offset, int cap, const void* records)
+{
+    if (records == nullptr || cap < 1 || cap > kCap || vocab_offset < 0) {
+        set_error("ftb200_vocab_parallel_local: invalid argument");
+        return FTB200_INVALID_ARG;
+    }
+    if (p != nullptr && (p->cum_log_probs != nullptr || p->output_log_probs != nullptr)) {
+        set_error("ftb200_vocab_parallel_local: log-probs are not available with a sharded vocabulary");
+        return FTB200_UNSUPPORTED;
+    }
+    return FTB200_OK;
+}
+
+extern "C" int ftb200_vocab_parallel_local(const ftb200_sampling_params* p, int vocab_offset, int cap,
+                                           uint64_t* records)
+{
+    reset_launch_count();
+    const int rc = vp_check(p, vocab_offset, cap, records);
+    return rc != FTB200_OK ? rc : vp_local(p, vocab_offset, cap, records);
+}
+
+extern "C" int ftb200_vocab_parallel_shards(const ftb200_sampling_params* p, const void* const* logits, int n_shards,
+                                            int shard_size, int cap, uint64_t* records)
+{
+    reset_launch_count();
+    int rc = vp_check(p, 0, cap, records);
+    if (rc == FTB200_OK && (p == nullptr || logits == nullptr || n_shards < 1 || shard_size < 1)) {
+        set_error("ftb200_vocab_parallel_shards: invalid argument");
+        rc = FTB200_INVALID_ARG;
+    }
+    if (rc != FTB200_OK) {
+        return rc;
+    }
+    // the argument block of a shard: its columns in memory, and of the vocabulary what lies in it
+    ftb200_sampling_params q = *p;
+    q.logits                 = logits[0];
+    q.vocab_size_padded      = shard_size;
+    const auto columns       = [&](int i) {
+        const long long left = (long long)p->vocab_size - (long long)i * shard_size;
+        return (int)(left < 1 ? 1 : (left < shard_size ? left : shard_size));
+    };
+    q.vocab_size = columns(0);
+    KParams K;
+    size_t  smem = 0, vsmem = 0;
+    int     grid = 0;
+    rc           = plan_sampling(&q, K, smem, grid, true);
+    if (rc != FTB200_OK) {
+        return rc;
+    }
+    if (p->local_batch_size == 0) {
+        return FTB200_OK;
+    }
+    VpArgs V;
+    K.vp_out = (u64*)records, K.vp_cap = cap;
+    if (plan_vp_select(&q, K, logits, n_shards, 0, cap, K.vp_out, &V, &vsmem)) {
+        V.vocab = p->vocab_size;
+        return launch_vp_select(K, V, vsmem, (cudaStream_t)p->stream);
+    }
+    for (int i = 0; i < n_shards && rc == FTB200_OK; ++i) {
+        q.logits     = logits[i];
+        q.vocab_size = columns(i);
+        rc           = vp_local(&q, i * shard_size, cap, records + (size_t)i * p->local_batch_size * (cap + 2));
+    }
+    return rc;
+}
+
 extern "C" int ftb200_vocab_parallel_merge(const ftb200_sampling_params* p, const uint64_t* gathered, int n_ranks,
                                            int cap, int* overflow_count)
 {
@@ -628,7 +743,7 @@ extern "C" int ftb200_vocab_parallel_merge(const ftb200_sampling_params* p, cons
     }
     K.vp_cap        = cap;
     cudaStream_t st = (cudaStream_t)p->stream;
-    grid            = sm_count() * 3 < p->local_batch_size ? sm_count() * 3 : p->local_batch_size;  // (3 CTAs of 52 KB per SM)
+    grid            = sm_count() * 4 < p->local_batch_size ? sm_count() * 4 : p->local_batch_size;
     switch (p->dtype) {
         case FTB200_F32: rc = vp_merge_launch<FTB200_F32>(K, (const u64*)gathered, n_ranks, overflow_count, grid, st); break;
         case FTB200_F16: rc = vp_merge_launch<FTB200_F16>(K, (const u64*)gathered, n_ranks, overflow_count, grid, st); break;

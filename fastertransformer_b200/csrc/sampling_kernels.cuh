@@ -16,6 +16,7 @@
 #pragma once
 #include <curand_kernel.h>
 
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -4280,20 +4281,20 @@ __device__ __noinline__ void vp_merge_topp_row(const KParams& P, const Smem& S, 
 // passes emitted ([rank][row][1 + cap]: count, then (~key(value) << 32 | global column) entries).  The
 // union is sorted and handed to the same draw and tie-order code as the single-GPU path, so every rank
 // arrives at the id the reference would sample from the full row.
+// `area`: entries of the candidate area; without top-p rows it is what the records can hold (at least 1024), so that four
+// CTAs share an SM: the steps of a row are short and wait for one another.
 template<int DT>
-__global__ void __launch_bounds__(kThreads, 3)
-vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nranks, int* overflow)
+__global__ void __launch_bounds__(kThreads, 4)
+vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nranks, int* overflow, int area)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float                              s_u;
-    __shared__ u32                                s_n;
+    __shared__ u32                                s_n, s_bound, s_bad, s_short;
     __shared__ curandState_t                      s_before_k;  // generator of a top-k row before its draw
-    constexpr int                                 kMergeRanks = 64;
-    __shared__ u32                                s_off[kMergeRanks + 1];  // start of every rank's record in the union
     Smem                                          S;
     S.cand  = (u64*)smem_raw;
-    S.hist  = (u32*)(S.cand + kCap);
-    S.val2  = (float*)(S.hist + kNB);
+    S.val2  = (float*)(S.cand + area);
+    S.hist  = (u32*)(S.val2 + 1024);
     S.flags = nullptr, S.hash = nullptr, S.spre = nullptr, S.sfin = nullptr, S.hitq = nullptr, S.nhit = nullptr;
     const int tid = threadIdx.x;
     for (int r = blockIdx.x; r < P.local_batch; r += gridDim.x) {
@@ -4320,39 +4321,62 @@ vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nran
             }
             continue;
         }
-        if (tid == 0) {
+        int k = (int)P.topk_ks[r];
+        k     = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
+        const float top_p = P.topk_ps[r];
+        if (tid == kThreads - 1) {
             s_before_k = P.topk_states[r];
             s_u        = draw_uniform(P.topk_states, r);
-            s_n        = 0;
+        }
+        if (tid == 0) {
+            s_n = 0, s_bound = 0, s_bad = 0, s_short = 0;
         }
         __syncthreads();
-        bool bad = false;
-        for (int q = 0; q < nranks; ++q) {
+        // Every record is sorted.  With at least ceil(k / ranks) entries in each, the largest of the entries at that
+        // place bounds the k-th of the union, and what lies above its value is left where it is: of 8 x 64 entries
+        // about 90 come in, and a warp takes a record, so all records are read at once.
+        const int at_least = (k + nranks - 1) / nranks;
+        for (int q = tid; q < nranks; q += kThreads) {
             const u64* rec = gathered + ((size_t)q * P.local_batch + r) * (P.vp_cap + 2);
             const u64  c   = rec[0];
+            const u64  e   = at_least <= P.vp_cap ? rec[at_least] : 0;
             if (c == ~0ull) {
-                bad = true;
-                continue;
+                s_bad = 1;
             }
-            const u32 base = s_n;
-            __syncthreads();
-            if (base + (u32)c > (u32)kCap) {
-                bad = true;
+            else if (c < (u64)at_least) {
+                s_short = 1;
             }
             else {
-                for (u32 i = tid; i < (u32)c; i += kThreads) {
-                    S.cand[base + i] = rec[1 + i];
-                }
-                if (tid == 0) {
-                    if (q < kMergeRanks) {
-                        s_off[q] = base, s_off[q + 1] = base + (u32)c;
+                atomicMax(&s_bound, (u32)(e >> 32));
+            }
+        }
+        __syncthreads();
+        const u32 bound = s_short ? 0xffffffffu : s_bound;
+        if (!s_bad) {
+            for (int q = tid >> 5; q < nranks; q += kWarps) {
+                const u64* rec = gathered + ((size_t)q * P.local_batch + r) * (P.vp_cap + 2);
+                const int  c   = (int)rec[0];
+                for (int i0 = 0; i0 < c; i0 += 32) {
+                    const int i  = i0 + (tid & 31);
+                    const u64 e  = i < c ? rec[1 + i] : ~0ull;
+                    const u32 in = __ballot_sync(0xffffffffu, i < c && (u32)(e >> 32) <= bound);
+                    if (in == 0) {
+                        break;  // (sorted: nothing further on either)
                     }
-                    s_n = base + (u32)c;
+                    u32 at = 0;
+                    if ((tid & 31) == 0) {
+                        at = atomicAdd(&s_n, (u32)__popc(in));
+                    }
+                    at = __shfl_sync(0xffffffffu, at, 0) + __popc(in & ((1u << (tid & 31)) - 1u));
+                    if (((in >> (tid & 31)) & 1u) && at < (u32)area) {
+                        S.cand[at] = e;
+                    }
                 }
             }
-            __syncthreads();
         }
-        if (bad) {
+        __syncthreads();
+        const int n = (int)s_n;
+        if (s_bad || n > area) {
             if (tid == 0) {
                 atomicAdd(overflow, 1);
                 *O.id_out        = -1;
@@ -4360,58 +4384,54 @@ vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nran
             }
             continue;
         }
-        const int n      = (int)s_n;
-        u64*      sorted = S.cand;
-        if (nranks <= kMergeRanks && n <= kCap / 2) {
-            // every rank's record is sorted already: the place of an entry in the union is its index in its own
-            // record plus the number of smaller entries in each of the others (a binary search each; the entries are
-            // distinct).  No sorting network, two barriers.
-            u64* const dst = S.cand + kCap / 2;
-            for (int a = tid; a < n; a += kThreads) {
-                int q = 0;
-                while (q + 1 < nranks && (u32)a >= s_off[q + 1]) {
-                    ++q;
+        u64* sorted = S.cand;
+        if (n <= 2 * kThreads) {
+            // few entries: the place of each is the number of smaller ones (they are distinct)
+            sorted       = S.cand + 2 * kThreads;
+            const u64 e0 = tid < n ? S.cand[tid] : ~0ull, e1 = tid + kThreads < n ? S.cand[tid + kThreads] : ~0ull;
+            int       c0 = 0, c1 = 0;
+            if ((tid & ~31) < n) {
+                for (int b = 0; b < n; ++b) {
+                    const u64 x = S.cand[b];
+                    c0 += x < e0 ? 1 : 0;
+                    c1 += x < e1 ? 1 : 0;
                 }
-                const u64 e    = S.cand[a];
-                int       rank = a - (int)s_off[q];
-                for (int o = 0; o < nranks; ++o) {
-                    if (o == q) {
-                        continue;
-                    }
-                    int lo = (int)s_off[o], hi = (int)s_off[o + 1];  // first entry of record o that is not below e
-                    const int lo0 = lo;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (S.cand[mid] < e) {
-                            lo = mid + 1;
-                        }
-                        else {
-                            hi = mid;
-                        }
-                    }
-                    rank += lo - lo0;
-                }
-                dst[rank] = e;
+            }
+            if (tid < n) {
+                sorted[c0] = e0;
+            }
+            if (tid + kThreads < n) {
+                sorted[c1] = e1;
             }
             __syncthreads();
-            sorted = dst;
         }
         else {
             group_sort_u64(S.cand, n, tid, kThreads, CtaSync());
             __syncthreads();
         }
-        int k = (int)P.topk_ks[r];
-        k     = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
-        topk_finish(P, S, O, sorted, n, k, s_u, P.topk_ps[r], true, false);
+        topk_finish(P, S, O, sorted, n, k, s_u, top_p, true, false);
     }
 }
 
 template<int DT>
 int vp_merge_launch(const KParams& K, const u64* gathered, int nranks, int* overflow, int grid, cudaStream_t st)
 {
-    const size_t smem = (size_t)kCap * 8 + (size_t)kNB * 4 + 1024 * 4;
-    FTB_CUDA_CHECK(cudaFuncSetAttribute(vp_merge_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    vp_merge_kernel<DT><<<grid, kThreads, smem, st>>>(K, gathered, nranks, overflow);
+    const bool   topp = K.topp_states != nullptr;
+    const size_t most = (size_t)nranks * K.vp_cap;
+    const int    area = topp || most >= (size_t)kCap ? kCap : (most < 4 * kThreads ? 4 * kThreads : ((int)most + 1) & ~1);
+    const size_t smem = (size_t)area * 8 + (size_t)(topp ? kNB : 1024) * 4 + 1024 * 4;
+    constexpr int kMostSmem = kCap * 8 + kNB * 4 + 1024 * 4;
+    constexpr int            kMaxDev = 64;
+    static std::atomic<bool> ready[kMaxDev];  // the opt-in to the shared-memory size, once per device
+    int                      dev = 0;
+    FTB_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDev || !ready[dev].load(std::memory_order_acquire)) {
+        FTB_CUDA_CHECK(cudaFuncSetAttribute(vp_merge_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
+        if (dev >= 0 && dev < kMaxDev) {
+            ready[dev].store(true, std::memory_order_release);
+        }
+    }
+    vp_merge_kernel<DT><<<grid, kThreads, smem, st>>>(K, gathered, nranks, overflow, area);
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
 }

@@ -167,11 +167,14 @@ class VocabParallelSampler(DynamicDecodeLayer):
     def forward_shards(self, outputs, inputs, shards):
         """All shards on this device (no communication): the arithmetic of forward_rank on every rank."""
         if not self._all_top_p:
-            rec, gathered = self._buffers(shards[0].shape[0])
-            for i, sh in enumerate(shards):
-                self.local_pass(outputs, inputs, sh, i, rec)
-                gathered[i].copy_(rec)
-            self.merge(outputs, inputs, gathered, shards[0])
+            P = self._params(outputs, inputs, shards[0], self.vocab_size, self.shard_size * self.n_shards, self._record_halves)
+            gathered = self._buffers(shards[0].shape[0])[1]
+            ptrs = (C.c_void_p * len(shards))(*[sh.data_ptr() for sh in shards])
+            check(lib.ftb200_vocab_parallel_shards(C.byref(P), ptrs, len(shards), self.shard_size, self.cap, gathered.data_ptr()))
+            self.launches += lib.ftb200_last_launch_count()
+            check(lib.ftb200_vocab_parallel_merge(C.byref(P), gathered.data_ptr(), self.n_shards, self.cap,
+                                                  self._overflow.data_ptr()))
+            self.launches += 1
         if self._topp_rows is not None:
             self._sample_top_p_rows(outputs, inputs, torch.stack([sh.index_select(0, self._topp_rows) for sh in shards]))
             return

@@ -398,6 +398,12 @@ int ftb200_beam_search_step(const ftb200_beam_params* p);
  * the single-GPU path makes.
  * ------------------------------------------------------------------------------------------ */
 int ftb200_vocab_parallel_local(const ftb200_sampling_params* p, int vocab_offset, int cap, uint64_t* records);
+/* Step 1 for several shards on this device at once (logits: host array of n_shards device pointers, each
+ * [local_batch, shard_size]; p->vocab_size counts the columns of all of them, p->logits and
+ * p->vocab_size_padded are not looked at): records [n_shards][local_batch][2 + cap], as the all-gather of one
+ * record block per rank lays them out. */
+int ftb200_vocab_parallel_shards(const ftb200_sampling_params* p, const void* const* logits, int n_shards,
+                                 int shard_size, int cap, uint64_t* records);
 int ftb200_vocab_parallel_merge(const ftb200_sampling_params* p, const uint64_t* gathered, int n_ranks, int cap,
                                 int* overflow_count);
 
