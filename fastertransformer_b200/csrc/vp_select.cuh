@@ -1,29 +1,58 @@
 // Local pass of the vocabulary-parallel step for 16-bit logits: the exchange records of all shards a device holds, in
 // one launch.
 //
-// A CTA takes one row of one shard at a time.  The row (up to 200 KB) goes into shared memory by 16-byte asynchronous
-// copies, every thread fetching the vectors that it alone will look at, so a copy is waited for by its own thread and the
-// next row is on its way as soon as the thread has read its vectors for the last time.  With the row at hand no sample
-// and no estimate is needed:
+// A CTA takes one row of one shard at a time.  The row (up to 200 KB) goes into shared memory by bulk copies that one
+// thread issues, and the next row is on its way as soon as the candidates of this one have been collected.  With the row
+// at hand no sample and no estimate is needed:
 //   1. every thread keeps the largest value of each of eight groups of its columns.  The k-th largest of all those maxima
 //      (one per thread while k is small, the finer groups above that) is a threshold that at least k columns reach, and
 //      hardly more: 74 of 32000 for k = 64, 300 for k = 256;
-//   2. the columns at or above it are collected, and placed by counting how many of them come before each (a few
-//      hundred broadcast reads, no sorting network and none of its barriers);
+//   2. the columns at or above it are collected from the groups that reach it, and placed by counting how many of them
+//      come before each (a few hundred broadcast reads, no sorting network and none of its barriers);
 //   3. columns that a penalty or a ban touches are taken out of the copy first (an atomic OR makes them NaN, which no
 //      comparison lets through, and returns the raw value to exactly one thread) and are collected with their final values.
 // A row whose candidates do not fit (thousands of equal values), with fewer than k values to choose from, or with a
 // temperature that turns the order round, gets its threshold by bisection over the final values, counting in the copy:
 // rare, and still this kernel.
 //
-// Bound by HBM in principle (2 bytes a column), by the latency of the steps behind the copy in practice; three CTAs with
-// a row of 32000 columns each share an SM.  2048 rows of 8 x 32000 bf16, k = 64: 8 x 96 us with a sample, a streaming
-// pass and a sorting network in a launch per shard.
+// Bound by the latency of the steps behind the copy: 5.9 us a row (copy and maxima 1.7, threshold 0.9, candidates 1.6,
+// placing and record 1.4) with three CTAs on an SM, which is 4.0 TB/s.  2048 rows of 8 x 32000 bf16, k = 64: 265 us; 8 x 100
+// with a sample, a streaming pass and a sorting network in a launch per shard; 370 with 16-byte asynchronous copies by
+// all threads (a thread's 16 copies take 2 us to issue).
 #pragma once
 #include "fast_sampling.cuh"
 #include "vp_args.cuh"
 
 namespace ftb200 {
+
+// ---- bulk copies and the barriers that count their bytes ----
+__device__ __forceinline__ void bar_init(u32 bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// `bytes` (a multiple of 16, or none) from global to shared memory; both on 16-byte boundaries
+__device__ __forceinline__ void bulk_copy(u32 dst, const void* src, u32 bytes, u32 bar)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    if (bytes != 0) {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                     "l"(src), "r"(bytes), "r"(bar)
+                     : "memory");
+    }
+}
+// false when the copy did not come in (a limit on the wait, nothing else ends it)
+__device__ __forceinline__ bool bar_wait(u32 bar, u32 parity)
+{
+    u32 done = 0;
+    for (int i = 0; i < (1 << 20) && done == 0; ++i) {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+    }
+    return done != 0;
+}
 
 template<int DT, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 1)
@@ -31,7 +60,8 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned short s_max[NT], s_hot[NT * 4];
-    __shared__ u32            s_n, s_nspec, s_nhot, s_thr, s_kv, s_m, s_cnt[3];
+    __shared__ u32            s_n, s_nspec, s_nhot, s_thr, s_kv, s_m, s_cnt[3], s_lost, s_args[5];
+    __shared__ u64            s_bar[4];
     constexpr u32             kDead2 = DT == FTB200_F16 ? 0xfc00fc00u : 0xff80ff80u;  // two columns of -infinity
     uint4* const              row    = (uint4*)smem_raw;
     u64* const                cand   = (u64*)(smem_raw + V.row_bytes);
@@ -48,24 +78,44 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
         float       inv_t;
         bool        live, topp;
     };
-    auto task_at = [&](int t) {
+    // A row's arguments are sent for (asynchronous copies of the words that hold them, by one thread) at the start of the
+    // row before it, and looked at when that one has been collected.
+    enum { kSkipK, kSkipP, kFin, kK, kTemp };
+    auto send_args = [&](int t) {
+        if (tid == 32 && t < tasks) {
+            const int r    = t % rows;
+            auto      word = [&](int slot, const void* p) {
+                if (p != nullptr) {
+                    cp_async4((u32)__cvta_generic_to_shared(&s_args[slot]), (const void*)((size_t)p & ~(size_t)3));
+                }
+            };
+            word(kSkipK, P.topk_skip != nullptr ? P.topk_skip + r : nullptr);
+            word(kSkipP, P.topp_skip != nullptr ? P.topp_skip + r : nullptr);
+            word(kFin, P.finished != nullptr ? P.finished + r : nullptr);
+            word(kK, P.topk_ks + r);
+            word(kTemp, temp ? P.temperature + r : nullptr);
+            cp_async_commit();
+        }
+    };
+    auto args_here = [&]() {  // before the barrier that publishes them
+        if (tid == 32) {
+            cp_async_wait_all();
+        }
+    };
+    auto task_of = [&](int t) {
         Task T;
-        T.live = false, T.topp = false, T.k = 1, T.inv_t = 1.0f, T.nv = 0, T.mis = 0, T.vocab = 0, T.base = nullptr;
-        T.sh = t / rows;
-        T.r  = t - T.sh * rows;
-        if (t >= tasks) {
-            return T;
-        }
-        // (all of a row's arguments are sent for at once, a row ahead of their use)
-        const u32 skip_k = P.topk_skip != nullptr ? P.topk_skip[T.r] : 0u, fin = P.finished != nullptr ? P.finished[T.r] : 0u;
-        const u32 skip_p = P.topp_states == nullptr ? 1u : (P.topp_skip != nullptr ? P.topp_skip[T.r] : 0u);
-        T.live           = (skip_k | fin) == 0;
-        T.topp           = (skip_k != 0) & ((fin | skip_p) == 0);
-        int k              = (int)P.topk_ks[T.r];
-        T.k                = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
-        if (temp) {
-            T.inv_t = 1.0f / (P.temperature[T.r] + 1e-6f);
-        }
+        auto byte_of = [&](int slot, const uint8_t* p, u32 none) {
+            return p != nullptr ? (s_args[slot] >> (8 * ((size_t)(p + T.r) & 3))) & 0xffu : none;
+        };
+        T.sh            = t < tasks ? t / rows : 0;
+        T.r             = t - T.sh * rows;
+        const u32 skip_k = byte_of(kSkipK, P.topk_skip, 0u), fin = byte_of(kFin, P.finished, 0u);
+        const u32 skip_p = P.topp_states == nullptr ? 1u : byte_of(kSkipP, P.topp_skip, 0u);
+        T.live           = (t < tasks) & ((skip_k | fin) == 0);
+        T.topp           = (t < tasks) & (skip_k != 0) & ((fin | skip_p) == 0);
+        const int k      = (int)s_args[kK];
+        T.k              = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
+        T.inv_t          = temp ? 1.0f / (__uint_as_float(s_args[kTemp]) + 1e-6f) : 1.0f;
         const int left  = V.vocab - T.sh * P.vocab_padded;
         T.vocab         = left < P.vocab_padded ? left : P.vocab_padded;
         T.vocab         = T.vocab < 1 ? 1 : T.vocab;
@@ -76,31 +126,47 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
         T.nv            = (T.mis + T.vocab + 7) / 8;
         return T;
     };
-    // the row's vectors in four parts (of whole fours of vectors per thread: vector i belongs to group i % 4), so that the first ones can be looked at while the last are on their way
-    const u32 row_s = (u32)__cvta_generic_to_shared(row);
+    // the row's vectors in four parts (of whole fours of vectors per thread: vector i of a thread belongs to group i % 4),
+    // so that the first ones can be looked at while the last are on their way
+    const u32 row_s = (u32)__cvta_generic_to_shared(row), bar_s = (u32)__cvta_generic_to_shared(s_bar);
     auto      send  = [&](const Task& T) {
-        const int ni = (T.nv + NT - 1) / NT, q = (ni + 15) / 16 * 4;
-        for (int g = 0; g < 4; ++g) {
-            for (int i = g * q; i < (g + 1) * q && i < ni; ++i) {
-                const int j = i * NT + tid;
-                if (j < T.nv) {
-                    cp_async16(row_s + 16u * (u32)j, T.base + 16 * (size_t)j);
-                }
+        if (tid == 0) {
+            const int per = ((T.nv + NT - 1) / NT + 15) / 16 * 4 * NT;
+            for (int g = 0; g < 4; ++g) {
+                const int left = T.nv - g * per, n = left < 0 ? 0 : (left < per ? left : per);
+                bulk_copy(row_s + 16u * (u32)(g * per), T.base + 16 * (size_t)(g * per), 16u * (u32)n, bar_s + 8u * (u32)g);
             }
-            cp_async_commit();
         }
     };
-    Task cur = task_at((int)blockIdx.x);
+    send_args((int)blockIdx.x);
+    args_here();
+    if (tid == 0) {
+        s_n = 0, s_nspec = 0, s_nhot = 0, s_m = 0, s_lost = 0;
+        for (int g = 0; g < 4; ++g) {
+            bar_init(bar_s + 8u * (u32)g);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    Task cur = task_of((int)blockIdx.x);
     if (cur.live) {
         send(cur);
     }
-    if (tid == 0) {
-        s_n = 0, s_nspec = 0, s_nhot = 0, s_m = 0;
-    }
-    __syncthreads();
+    __syncthreads();  // (the arguments are looked at by all threads before the next ones take their place)
+    u32  parity = 0;  // of the row at hand, on all four barriers
+    auto wait   = [&](int g) {
+        if (!bar_wait(bar_s + 8u * (u32)g, parity)) {
+            s_lost = 1;  // (the row is reported as undecided)
+        }
+    };
     for (int t = blockIdx.x; t < tasks; t += gridDim.x) {
         const Task T   = cur;
-        cur            = task_at(t + gridDim.x);
+        u64* const rec = P.trace != nullptr ? P.trace + (size_t)(t % rows) * kTraceWords : nullptr;
+        if (rec != nullptr && tid == 0) {
+            rec[0] = (u64)T.r, rec[1] = (u64)blockIdx.x, rec[2] = global_timer_ns();
+        }
+        send_args(t + (int)gridDim.x);
         u64* const out = V.out + (size_t)t * (P.vp_cap + 2);
         if (!T.live) {
             // nothing to send, or a top-p row: the general kernel's (statistics form)
@@ -112,14 +178,14 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                     out[0] = 0;
                 }
             }
+            args_here();
+            __syncthreads();
+            cur = task_of(t + (int)gridDim.x);
             if (cur.live) {
                 send(cur);
             }
+            __syncthreads();
             continue;
-        }
-        u64* const rec = P.trace != nullptr ? P.trace + (size_t)(t % rows) * kTraceWords : nullptr;
-        if (rec != nullptr && tid == 0) {
-            rec[0] = (u64)T.r, rec[1] = (u64)blockIdx.x, rec[2] = global_timer_ns();
         }
         const __half inv_t_h = __float2half_rn(T.inv_t);
         const int    id0     = V.offset + T.sh * P.vocab_padded;  // token id of the shard's first column
@@ -138,7 +204,9 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
         };
         const bool own_edge = (tid == 0 && T.mis != 0) || ((T.mis + T.vocab) % 8 != 0 && (T.nv - 1) % NT == tid);
         if (special_launch) {
-            cp_async_wait<0>();
+            for (int g = 0; g < 4; ++g) {
+                wait(g);
+            }
             if (own_edge) {
                 for (int j = tid; j < T.nv; j += NT) {
                     if (j == 0 || j == T.nv - 1) {
@@ -235,14 +303,11 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                     }
                 }
             };
-            cp_async_wait<3>();
-            part(0);
-            cp_async_wait<2>();
-            part(1);
-            cp_async_wait<1>();
-            part(2);
-            cp_async_wait<0>();
-            part(3);
+            for (int g = 0; g < 4; ++g) {
+                wait(g);
+                part(g);
+            }
+            parity ^= 1u;
         }
         if (rec != nullptr) {
             trace_mark(rec, 1);
@@ -342,19 +407,9 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                 }
             }
         };
-        // the columns `pm` of vector j, `c` of them; all lanes of a warp take part
+        // the columns `pm` of vector j, `c` of them
         auto put = [&](const uint4& v, int j, u32 pm, u32 c) {
-            u32 incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const u32 x = __shfl_up_sync(0xffffffffu, incl, o);
-                incl += lane >= o ? x : 0u;
-            }
-            u32 pos = 0;
-            if (lane == 31 && incl != 0) {
-                pos = atomicAdd(&s_n, incl);
-            }
-            pos = __shfl_sync(0xffffffffu, pos, 31) + incl - c;
+            u32 pos = c != 0 ? atomicAdd(&s_n, c) : 0u;
             while (pm != 0) {
                 const int e = __ffs(pm) - 1;
                 pm &= pm - 1;
@@ -390,6 +445,7 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                 }
             }
             __syncthreads();
+            trace_mark(rec, 5);
             const u32 thr2  = key16_inv(thr) * 0x10001u;
             const int gs    = (ni + 3) / 4, items = (int)s_nhot * gs;
             for (int x0 = tid & ~31; x0 < items; x0 += NT) {
@@ -411,8 +467,11 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                 put(v, j, pm, c);
             }
             take_specials(fkey(value_of(thr)));
+            args_here();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (what was written into the copy, before the next one)
             __syncthreads();
             by_hand = s_n > (u32)V.cand_cap;
+            trace_mark(rec, 6);
         }
         if (by_hand) {
             // rare: the k-th largest final value itself, by bisection over the ordered 32-bit keys
@@ -474,9 +533,12 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                 put(j < T.nv ? row[j] : make_uint4(0, 0, 0, 0), j, pm, c);
             }
             take_specials(lo);
+            args_here();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncthreads();
         }
         const int n = (int)s_n;
+        cur = task_of(t + (int)gridDim.x);
         if (cur.live) {
             send(cur);  // (no thread looks at this row's copy again)
         }
@@ -509,17 +571,26 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
             const u64 e0 = tid < n ? cand[tid] : ~0ull, e1 = tid + NT < n ? cand[tid + NT] : ~0ull;
             int       c0 = 0, c1 = 0;
             if ((tid & ~31) < n) {
-                for (int b = 0; b + 1 < n; b += 2) {
-                    const ulonglong2 x = *(const ulonglong2*)(cand + b);
-                    c0 += (x.x < e0 ? 1 : 0) + (x.y < e0 ? 1 : 0);
-                    if (n > NT) {
-                        c1 += (x.x < e1 ? 1 : 0) + (x.y < e1 ? 1 : 0);
+                auto before = [&](auto two) {
+#pragma unroll 4
+                    for (int b = 0; b + 1 < n; b += 2) {
+                        const ulonglong2 x = *(const ulonglong2*)(cand + b);
+                        c0 += (x.x < e0 ? 1 : 0) + (x.y < e0 ? 1 : 0);
+                        if (two) {
+                            c1 += (x.x < e1 ? 1 : 0) + (x.y < e1 ? 1 : 0);
+                        }
                     }
+                    if (n & 1) {
+                        const u64 x = cand[n - 1];
+                        c0 += x < e0 ? 1 : 0;
+                        c1 += x < e1 ? 1 : 0;
+                    }
+                };
+                if (n > NT) {
+                    before(std::true_type());
                 }
-                if (n & 1) {
-                    const u64 x = cand[n - 1];
-                    c0 += x < e0 ? 1 : 0;
-                    c1 += x < e1 ? 1 : 0;
+                else {
+                    before(std::false_type());
                 }
                 if (tid < n && c0 == k_eff - 1) {
                     s_kv = (u32)(e0 >> 32);
@@ -548,9 +619,10 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
             }
         }
         __syncthreads();
+        trace_mark(rec, 7);
         if (tid == 0) {
             const u32 m = s_m;
-            out[0]      = m > (u32)P.vp_cap ? ~0ull : (u64)m;
+            out[0]      = m > (u32)P.vp_cap || s_lost ? ~0ull : (u64)m;
             s_n = 0, s_nspec = 0, s_nhot = 0, s_m = 0;
             if (rec != nullptr) {
                 rec[3] = global_timer_ns();
@@ -558,7 +630,6 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
         }
         __syncthreads();
     }
-    cp_async_wait<0>();
 }
 
 template<int DT>

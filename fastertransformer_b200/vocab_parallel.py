@@ -50,6 +50,7 @@ class VocabParallelSampler(DynamicDecodeLayer):
         self._full_rows = None   # [batch, vocab_padded] scratch; only the top-p rows are ever written or read
         self.resolved_rows = 0
         self._seen_overflow = 0
+        self._need = {}          # workspace bytes by (dtype, rows, columns)
         self._records = None
         self._gathered = None
         self._overflow = torch.zeros(1, dtype=torch.int32, device=self.device)
@@ -57,10 +58,15 @@ class VocabParallelSampler(DynamicDecodeLayer):
     def setup(self, batch_size, beam_width, runtime_args):
         super().setup(batch_size, beam_width, runtime_args)
         self._topp_rows = None
+        self._topp_on = self.topp.active and not bool(self.topp.skip_host.all())
         if self.exact_top_p and self._has_topp():
             rows = (~self.topp.skip_host).nonzero()[0]
             self._topp_rows = torch.from_numpy(rows.astype("int64")).to(self.device)
         self._all_top_p = self._topp_rows is not None and bool(self.topk.skip_host.all())
+        # what every step asks of the arguments
+        self._temp_on = int(bool((self.temperature_host != 1.0).any()))
+        self._pen_on = self.penalty_type != 2 and bool((self.penalty_host != self.penalty_default).any())
+        self._most_min_length = int(self.min_length_host.max())
 
     def _params(self, outputs, inputs, logits, vocab, vocab_padded, halves="both"):
         B = logits.shape[0]
@@ -80,13 +86,12 @@ class VocabParallelSampler(DynamicDecodeLayer):
             P.bad_words, P.bad_words_len = bw.data_ptr(), bw.shape[-1]
             P.bad_words_shared = int(bw.dim() == 2 or bw.shape[0] == 1)
         P.temperature = self.temperature.data_ptr()
-        P.apply_temperature = int(bool((self.temperature_host != 1.0).any()))
+        P.apply_temperature = self._temp_on
         P.repetition_penalty = self.penalty.data_ptr()
         P.penalty_type = self.penalty_type
-        P.apply_repetition = int(step > 1 and self.penalty_type != 2
-                                 and bool((self.penalty_host != self.penalty_default).any()))
+        P.apply_repetition = int(step > 1 and self._pen_on)
         P.min_lengths = self.min_length.data_ptr()
-        P.apply_min_length = int(bool((self.min_length_host > step - mil).any()))
+        P.apply_min_length = int(self._most_min_length > step - mil)
         if halves != "top_p":
             P.topk_states = self.topk.curand.data_ptr()
             P.topk_ks, P.topk_ps = self.topk.top_ks.data_ptr(), self.topk.top_ps.data_ptr()
@@ -99,16 +104,19 @@ class VocabParallelSampler(DynamicDecodeLayer):
         for key, width in (("sequence_length", 4), ("finished", 1)):
             t = outputs.get(key)
             setattr(P, key, None if t is None else t.data_ptr())
-        need = C.c_size_t(0)
-        check(lib.ftb200_sampling_workspace_bytes(P.dtype, B, vocab_padded, C.byref(need)))
-        if self._workspace is None or self._workspace.numel() < need.value:
-            self._workspace = torch.empty(need.value, dtype=torch.uint8, device=self.device)
+        need = self._need.get((P.dtype, B, vocab_padded))
+        if need is None:
+            n = C.c_size_t(0)
+            check(lib.ftb200_sampling_workspace_bytes(P.dtype, B, vocab_padded, C.byref(n)))
+            need = self._need[P.dtype, B, vocab_padded] = n.value
+        if self._workspace is None or self._workspace.numel() < need:
+            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
         P.workspace, P.workspace_bytes = self._workspace.data_ptr(), self._workspace.numel()
-        P.stream = self._stream_ptr().value
+        P.stream = self._raw_stream()
         return P
 
     def _has_topp(self):
-        return self.topp.active and not bool(self.topp.skip_host.all())
+        return self._topp_on
 
     @property
     def _record_halves(self):
