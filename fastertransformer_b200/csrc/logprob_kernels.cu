@@ -13,7 +13,11 @@ namespace ftb200 {
 
 namespace {
 
+// 16-bit rows want every warp that fits (the exponentials alone take 137 of 188 us): 4 CTAs of 256 threads 254 us, 6 CTAs 243,
+// 8 CTAs 222; 8 loads in flight instead of 4 change nothing there.
 constexpr int   kLpThreads = 256;
+constexpr int   kLpCtas    = 8;   // per SM
+constexpr int   kLpLoads   = 4;   // 16-byte loads in flight per thread
 constexpr float kLog2e     = 1.4426950408889634f;
 
 template<typename T>
@@ -21,6 +25,10 @@ struct LpType;
 template<>
 struct LpType<float> {
     static constexpr int   kPerVec = 4;
+    __device__ static float maximum(const uint4&, const float* x)
+    {
+        return fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+    }
     static constexpr float kLowest = -FLT_MAX;
     __device__ static float get(const float* p) { return *p; }
     __device__ static void  unpack(const uint4& v, float* x)
@@ -34,6 +42,12 @@ struct LpType<float> {
 template<>
 struct LpType<__half> {
     static constexpr int   kPerVec = 8;
+    __device__ static float maximum(const uint4& v, const float*)
+    {
+        const __half2* h = reinterpret_cast<const __half2*>(&v);
+        const float2   m = __half22float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+        return fmaxf(m.x, m.y);
+    }
     static constexpr float kLowest = -65504.0f;  // the reference starts the maximum at -HALF_FLT_MAX (:58-59)
     __device__ static float get(const __half* p) { return __half2float(*p); }
     __device__ static void  unpack(const uint4& v, float* x)
@@ -50,6 +64,12 @@ struct LpType<__half> {
 template<>
 struct LpType<__nv_bfloat16> {
     static constexpr int   kPerVec = 8;
+    __device__ static float maximum(const uint4& v, const float*)
+    {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+        const float2          m = __bfloat1622float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+        return fmaxf(m.x, m.y);
+    }
     static constexpr float kLowest = -FLT_MAX;
     __device__ static float get(const __nv_bfloat16* p) { return __bfloat162float(*p); }
     __device__ static void  unpack(const uint4& v, float* x)
@@ -97,11 +117,7 @@ __device__ __forceinline__ void add_vec(MaxSum& a, const uint4& v)
     constexpr int N = LpType<T>::kPerVec;
     float         x[N];
     LpType<T>::unpack(v, x);
-    float vm = x[0];
-#pragma unroll
-    for (int i = 1; i < N; ++i) {
-        vm = fmaxf(vm, x[i]);
-    }
+    const float vm = LpType<T>::maximum(v, x);
     if (vm > a.m) {
         a.s *= fast_exp(a.m - vm);
         a.m = vm;
@@ -115,8 +131,15 @@ __device__ __forceinline__ void add_vec(MaxSum& a, const uint4& v)
 }
 
 // One CTA per (step, sequence) row at a time.  Rows past a sequence's length are skipped without a read.
+//
+// The counted rows are dealt out evenly: every CTA adds up the sequences' counts and takes each gridDim-th of the counted
+// rows.  With the rows of the whole [step, sequence] array dealt out instead, the skipped ones included, 1184 CTAs and 32
+// sequences gave a CTA the same sequence every time (512 x 32 x 50257 half, lengths spread over 256 .. 512: 14 rows for
+// some, 7 for others, and the 10.4 of the average took as long as 14: 254 us, now 222).  A batch of more sequences than the
+// table holds keeps that deal; no sequence is a large part of it.
+constexpr int kLpMaxSeq = 1024;
 template<typename T>
-__global__ void __launch_bounds__(kLpThreads) context_log_probs_kernel(float* log_probs, const T* logits,
+__global__ void __launch_bounds__(kLpThreads, kLpCtas) context_log_probs_kernel(float* log_probs, const T* logits,
                                                                         const int* ids, const int* lengths,
                                                                         int max_len, int batch, int vocab,
                                                                         size_t vocab_padded, int batch_first,
@@ -126,10 +149,57 @@ __global__ void __launch_bounds__(kLpThreads) context_log_probs_kernel(float* lo
     __shared__ MaxSum s_part[kLpThreads / 32];
     const int         tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int         steps = max_len - 1;
+    __shared__ int    s_end[kLpMaxSeq];  // counted rows of the sequences up to and with this one
+    const bool        dealt = batch <= kLpMaxSeq && rows <= 0x7fffffff;
+    if (dealt) {
+        constexpr int  PER = kLpMaxSeq / kLpThreads;
+        __shared__ int s_warp[kLpThreads / 32];
+        int            c[PER], sum = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int b = tid * PER + i;
+            sum += b < batch ? max(0, min(lengths[b] - 1, steps)) : 0;
+            c[i] = sum;
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            incl += lane >= o ? x : 0;
+        }
+        if (lane == 31) {
+            s_warp[wid] = incl;
+        }
+        __syncthreads();
+        int before = incl - sum;
+        for (int w = 0; w < wid; ++w) {
+            before += s_warp[w];
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            s_end[tid * PER + i] = before + c[i];
+        }
+        __syncthreads();
+        rows = s_end[kLpMaxSeq - 1];
+    }
 
     for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
         int step, b;
-        if (batch_first) {
+        if (dealt) {
+            int lo = 0, hi = batch - 1;  // the first sequence that ends after row r
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (s_end[mid] > r) {
+                    hi = mid;
+                }
+                else {
+                    lo = mid + 1;
+                }
+            }
+            b    = lo;
+            step = (int)(r - (lo > 0 ? s_end[lo - 1] : 0));
+        }
+        else if (batch_first) {
             b    = (int)(r / steps);
             step = (int)(r % steps);
         }
@@ -153,15 +223,16 @@ __global__ void __launch_bounds__(kLpThreads) context_log_probs_kernel(float* lo
         }
         const uint4* vp = reinterpret_cast<const uint4*>(row + head);
         int          i  = tid;
-        for (; i + 3 * kLpThreads < nvec; i += 4 * kLpThreads) {
-            const uint4 v0 = ld_nc_v4(vp + i);
-            const uint4 v1 = ld_nc_v4(vp + i + kLpThreads);
-            const uint4 v2 = ld_nc_v4(vp + i + 2 * kLpThreads);
-            const uint4 v3 = ld_nc_v4(vp + i + 3 * kLpThreads);
-            add_vec<T>(acc, v0);
-            add_vec<T>(acc, v1);
-            add_vec<T>(acc, v2);
-            add_vec<T>(acc, v3);
+        for (; i + (kLpLoads - 1) * kLpThreads < nvec; i += kLpLoads * kLpThreads) {
+            uint4 v[kLpLoads];
+#pragma unroll
+            for (int u = 0; u < kLpLoads; ++u) {
+                v[u] = ld_nc_v4(vp + i + u * kLpThreads);
+            }
+#pragma unroll
+            for (int u = 0; u < kLpLoads; ++u) {
+                add_vec<T>(acc, v[u]);
+            }
         }
         for (; i < nvec; i += kLpThreads) {
             add_vec<T>(acc, ld_nc_v4(vp + i));
@@ -240,7 +311,7 @@ int launch_log_probs(float* cum, const void* logits, const int* ids, const int* 
     FTB_CUDA_CHECK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
     const long long rows = (long long)(max_len - 1) * (long long)batch;
     if (rows > 0) {
-        const int grid = (int)std::min<long long>(rows, (long long)n_sm * 8);
+        const int grid = (int)std::min<long long>(rows, (long long)n_sm * kLpCtas);
         context_log_probs_kernel<T><<<grid, kLpThreads, 0, st>>>(log_probs, (const T*)logits, ids, lengths,
                                                                  (int)max_len, (int)batch, (int)vocab,
                                                                  vocab_padded, batch_first, rows);

@@ -149,3 +149,24 @@ def test_single_position_sequences_score_nothing():
     n = torch.ones(5, dtype=torch.int32, device="cuda")
     cum = log_prob_from_logits(x, ids, n)
     assert cum.shape == (5,) and bool((cum == 0).all())
+
+
+@pytest.mark.parametrize("batch", [1, 31, 256, 1024, 1025])
+@pytest.mark.parametrize("bf", [False, True], ids=["step_major", "batch_first"])
+def test_ragged_lengths_of_many_sequences(batch, bf):
+    """The counted rows are dealt out from a table of the sequences' counts (up to 1024 of them): lengths from 0 to the
+    longest, a run of empty sequences in front and at the end, against the restatement."""
+    rng = np.random.default_rng(batch)
+    max_len, vocab = 9, 515
+    lengths = rng.integers(0, max_len + 1, batch).astype(np.int32)
+    lengths[: batch // 4] = 1
+    lengths[batch - batch // 8:] = 0
+    lengths[batch // 2] = max_len
+    shape = (batch, max_len) if bf else (max_len, batch)
+    logits = (rng.standard_normal(shape + (vocab,)) * 2).astype(np.float32)
+    ids = rng.integers(0, vocab, shape).astype(np.int32)
+    cum, lp = run_ours(torch.from_numpy(logits).cuda(), torch.from_numpy(ids).cuda(), torch.from_numpy(lengths).cuda(), vocab, bf)
+    want_cum, want_lp = oracle_log_prob_from_logits(logits, ids, lengths, vocab, bf)
+    live = valid_mask(lengths, max_len, bf)
+    assert np.abs(lp - np.asarray(want_lp).ravel()[: lp.size])[live].max() < TOL
+    assert np.abs(cum - want_cum).max() < TOL * max_len
