@@ -1040,23 +1040,43 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         spec[i]     = ((u64)(~fkey(prob_of(fkey_inv(~(u32)(e >> 32))))) << 32) | (e & 0xffffffffu);
     }
     __syncthreads();
-    group_sort_u64<CtaSync, true>(spec, n_sp, tid, kThreads, CtaSync());
+    if (n_sp <= kThreads) {
+        // (distinct words: the place of each is the number of smaller ones; no network and none of its barriers)
+        const u64 mine = tid < n_sp ? spec[tid] : ~0ull;
+        int       at   = 0;
+        if ((tid & ~31) < n_sp) {
+#pragma unroll 4
+            for (int b = 0; b < n_sp; ++b) {
+                at += spec[b] < mine ? 1 : 0;
+            }
+        }
+        __syncthreads();
+        if (tid < n_sp) {
+            spec[at] = mine;
+        }
+    }
+    else {
+        group_sort_u64<CtaSync, true>(spec, n_sp, tid, kThreads, CtaSync());
+    }
     __syncthreads();
     u32* const run_pr = S.emask;            // [kFPRuns] probability of the run (float bits), descending
     u32* const run_st = run_pr + kFPRuns;   // [kFPRuns] length, then first position of the run
     FTB_ASSUME_SHARED(run_pr);
     FTB_ASSUME_SHARED(run_st);
-    constexpr int PER = 16;
     for (int i = tid; i < kFPRuns; i += kThreads) {
         run_st[i] = 0u;  // a position no pattern takes keeps length 0 and goes to a listed column
     }
     __syncthreads();
-    int nA;
+    // A thread takes `per` neighbouring patterns: what the window needs, not the most it can need, so that all threads
+    // work.  1500 patterns are 6 to a thread; with 16 to a thread only 94 threads had any.  Counts are read again where
+    // they are used (one small loop body instead of 16 copies of it).  Row of 51200, phase: 8.6 -> 5 us.
+    const int per = (npat + kThreads - 1) / kThreads;
+    int       nA;
     {
-        u32 cnt[PER], mine = 0;
-        for (int i = 0; i < PER; ++i) {
-            cnt[i] = count_of(tid * PER + i);
-            mine += cnt[i] != 0 ? 1u : 0u;
+        u32 mine = 0;
+#pragma unroll 4
+        for (int i = 0; i < per; ++i) {
+            mine += count_of(tid * per + i) != 0 ? 1u : 0u;
         }
         u32 incl = mine;
         for (int off = 1; off < 32; off <<= 1) {
@@ -1081,22 +1101,31 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
             return false;
         }
         u32 at = base + incl - mine;
-        for (int i = 0; i < PER; ++i) {
-            if (cnt[i] != 0) {
-                const float pr = prob_of(value_of(ktop - (u32)(tid * PER + i)));
+        int lo = -1;  // listed columns with a strictly larger probability (of neighbours in order: it only grows)
+#pragma unroll 1
+        for (int i = 0; i < per; ++i) {
+            const u32 c = count_of(tid * per + i);
+            if (c != 0) {
+                const float pr = prob_of(value_of(ktop - (u32)(tid * per + i)));
                 const u32   kp = ~fkey(pr);  // ascending in this key = descending probability
-                int         lo = 0, hi = n_sp;  // listed columns with a strictly larger probability
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if ((u32)(spec[mid] >> 32) < kp) {
-                        lo = mid + 1;
-                    }
-                    else {
-                        hi = mid;
+                if (lo < 0) {
+                    int hi = n_sp;
+                    lo     = 0;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if ((u32)(spec[mid] >> 32) < kp) {
+                            lo = mid + 1;
+                        }
+                        else {
+                            hi = mid;
+                        }
                     }
                 }
+                while (lo < n_sp && (u32)(spec[lo] >> 32) < kp) {
+                    ++lo;
+                }
                 run_pr[at + lo] = __float_as_uint(pr);
-                run_st[at + lo] = cnt[i];
+                run_st[at + lo] = c;
                 ++at;
             }
         }
@@ -1104,12 +1133,12 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     __syncthreads();
     // both lists keep their order in the merged sequence: the listed columns fill the positions the patterns left
     // free, in order
-    const int M = nA + n_sp;
+    const int M = nA + n_sp, rpt = (M + kThreads - 1) / kThreads;  // (<= kFPRuns / kThreads = 14)
     {
-        constexpr int RPT = kFPRuns / kThreads;
-        u32           freem = 0, mine = 0;
-        for (int i = 0; i < RPT; ++i) {
-            const int q = tid * RPT + i;
+        u32 freem = 0, mine = 0;
+#pragma unroll 4
+        for (int i = 0; i < rpt; ++i) {
+            const int q = tid * rpt + i;
             if (q < M && run_st[q] == 0u) {
                 freem |= 1u << i;
                 ++mine;
@@ -1131,13 +1160,12 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         for (int i = 0; i < wid; ++i) {
             j += s_wsum[i];
         }
-        for (int i = 0; i < RPT; ++i) {
-            if ((freem >> i) & 1u) {
-                const int q = tid * RPT + i;
-                run_pr[q]   = __float_as_uint(fkey_inv(~(u32)(spec[j] >> 32)));
-                run_st[q]   = 1u;
-                ++j;
-            }
+        while (freem != 0) {
+            const int q = tid * rpt + __ffs(freem) - 1;
+            freem &= freem - 1;
+            run_pr[q] = __float_as_uint(fkey_inv(~(u32)(spec[j] >> 32)));
+            run_st[q] = 1u;
+            ++j;
         }
     }
     __syncthreads();
@@ -1154,12 +1182,11 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     // exclusive scan of the run lengths -> first position of each run
     u32 N;
     {
-        constexpr int RPT = kFPRuns / kThreads;
-        u32           c[RPT], mine = 0;
-        for (int i = 0; i < RPT; ++i) {
-            const int q = tid * RPT + i;
-            c[i]        = q < M ? run_st[q] : 0u;
-            mine += c[i];
+        u32 mine = 0;
+#pragma unroll 4
+        for (int i = 0; i < rpt; ++i) {
+            const int q = tid * rpt + i;
+            mine += q < M ? run_st[q] : 0u;
         }
         u32 incl = mine;
         for (int off = 1; off < 32; off <<= 1) {
@@ -1182,11 +1209,12 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
         N      = tot;
         u32 at = base + incl - mine;
-        for (int i = 0; i < RPT; ++i) {
-            const int q = tid * RPT + i;
+        for (int i = 0; i < rpt; ++i) {
+            const int q = tid * rpt + i;
             if (q < M) {
-                run_st[q] = at;
-                at += c[i];
+                const u32 c = run_st[q];
+                run_st[q]   = at;
+                at += c;
             }
         }
     }
@@ -1377,13 +1405,11 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     __syncthreads();
     // bit patterns that map to this probability (one pattern past the counted range is looked at too: a class
     // that reaches down to the cut may go on below it)
-    for (int i = 0; i < PER + 1; ++i) {
-        const int u = tid * (PER + 1) + i;
-        if (u <= npat && ktop >= (u32)u) {
-            if (fkey(prob_of(value_of(ktop - (u32)u))) == k_sel) {
-                atomicMin(&s_imin, u);
-                atomicMax(&s_imax, u);
-            }
+#pragma unroll 2
+    for (int u = tid; u <= npat && u <= (int)ktop; u += kThreads) {
+        if (fkey(prob_of(value_of(ktop - (u32)u))) == k_sel) {
+            atomicMin(&s_imin, u);
+            atomicMax(&s_imax, u);
         }
     }
     __syncthreads();
