@@ -149,6 +149,19 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     return true;
 }
 
+// Slices and areas of the split kernel's second launch, over flagged rows: eight CTAs a row.
+static bool wide_areas(int vocab, SplitArgs* A)
+{
+    A->lgn   = 3;
+    A->slice = ((vocab + 1023) / 1024) << 7;
+    A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
+    A->area  = kSpAreaMax;
+    while (A->area > kSpAreaMin && split_smem_bytes(A->slice, A->area) > kSpMaxSmem) {
+        A->area -= 1024;
+    }
+    return split_smem_bytes(A->slice, A->area) <= kSpMaxSmem;
+}
+
 // Second stream of the single-pass step (one per device, made on first use) with the two events of its fork and join.
 struct SideStream {
     cudaStream_t stream = nullptr;
@@ -439,17 +452,33 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
             A.stop     = *stop;
             *stop_done = true;
         }
-        switch (p->dtype) {
-            case FTB200_F32: rc = split_sampling_launch<FTB200_F32>(K, A, smem, st); break;
-            case FTB200_F16: rc = split_sampling_launch<FTB200_F16>(K, A, smem, st); break;
-            default: rc = split_sampling_launch<FTB200_BF16>(K, A, smem, st); break;
-        }
+        const auto launch = [&](const SplitArgs& args) {
+            switch (p->dtype) {
+                case FTB200_F32: return split_sampling_launch<FTB200_F32>(K, args, smem, st);
+                case FTB200_F16: return split_sampling_launch<FTB200_F16>(K, args, smem, st);
+                default: return split_sampling_launch<FTB200_BF16>(K, args, smem, st);
+            }
+        };
+        rc = launch(A);
         if (rc != FTB200_OK) {
             return rc;
         }
         note_launch(1);
         if (whole) {
             return FTB200_OK;
+        }
+        // Areas below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row) leave the flat
+        // rows' wide nuclei: those go over eight CTAs with areas as large as shared memory allows.  Where these are below half
+        // a slice too (above 163000 columns) the general kernel's many CTAs serve the several rows left sooner.
+        SplitArgs B = A;
+        if (wide_areas(p->vocab_size, &B) && smem <= kSpMaxSmem && K.topp_states != nullptr && A.area < A.slice / 2
+            && B.area >= B.slice / 2) {
+            B.clusters = sm_count() / kSpMaxN < p->local_batch_size ? sm_count() / kSpMaxN : p->local_batch_size;
+            rc         = launch(B);
+            if (rc == FTB200_OK) {
+                note_launch(1);
+            }
+            return rc;
         }
         K.row_flags = A.redo_flags;
     }

@@ -30,6 +30,7 @@ struct SplitArgs {
     int  area;        // keys of the collection area
     int* redo_flags;  // [local_batch]: 1 when the row is left to decode_sampling_kernel (null: the kernel serves it itself)
     StopArgs stop;    // (only where redo_flags is null)
+    int  clusters;    // 0: one per row; else so many, which look for rows with redo_flags set and serve those
 };
 
 __host__ __device__ inline size_t split_smem_bytes(int slice, int area)

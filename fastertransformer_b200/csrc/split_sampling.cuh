@@ -1485,7 +1485,7 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
 
 // A row that the tables of the split form cannot hold, by the leader CTA alone.
 template<int DT>
-static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, unsigned char* smem, u64* rec)
+static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, int area, unsigned char* smem, u64* rec)
 {
     __shared__ Smem s_S;
     Smem&           S = s_S;
@@ -1494,13 +1494,15 @@ static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, unsign
         map_general_smem(P, S, smem);
     }
     __syncthreads();
-    process_row<DT>(P, S, r, P.scratch + (size_t)r * P.scratch_stride, rec);
+    process_row<DT>(P, S, r, P.scratch + (size_t)area * P.scratch_stride, rec);
 }
 
 // WHOLE: the kernel finishes every row itself (rows its tables cannot hold go through the general row code in the
 // leader CTA) and, when asked to, the step's stop criteria: one launch per decode step.  Taken while all rows are
 // resident at once; with more rows the general code's shared memory would cost residency, and the rows it is needed
-// for are left to decode_sampling_kernel.
+// for are left to a second launch: decode_sampling_kernel, or - where the areas of the first launch are small - a few
+// clusters of this form with all the shared memory there is (A.clusters), because a nucleus of half of 127000 columns takes
+// 0.2 ms here and 5 to 9 ms in the general code (800 such rows, 42 of them flagged: 10.7 -> 1.9 ms for most steps).
 template<int DT, int LGN, bool WHOLE>
 __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
                                                                      const __grid_constant__ SplitArgs A)
@@ -1517,7 +1519,36 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
     M.hist     = M.sub + A.area / 4;
     const int  tid = threadIdx.x, rank = (int)cluster_rank();
     const bool want_lp = P.cum_log_probs != nullptr || P.out_log_probs != nullptr;
-    for (int t = (int)blockIdx.x >> LGN; t < P.local_batch; t += (int)gridDim.x >> LGN) {
+    const int  first = (int)blockIdx.x >> LGN, step = (int)gridDim.x >> LGN;
+    const bool again = WHOLE && A.redo_flags != nullptr;
+    __shared__ u32 s_flagged[kWarps];
+    int            base = -kThreads, w = kWarps;  // of the flagged rows: place in the search for the next one
+    u32            word = 0;
+    for (int t = first; t < P.local_batch; t += step) {
+        if (again) {
+            // (every thread looks at one of the cluster's next 256 rows)
+            while (word == 0 && (w + 1 < kWarps || first + step * (base + kThreads) < P.local_batch)) {
+                if (++w < kWarps) {
+                    word = s_flagged[w];
+                    continue;
+                }
+                base += kThreads;
+                w              = -1;
+                const int  at  = first + step * (base + tid);
+                const bool set = at < P.local_batch && A.redo_flags[P.row_order != nullptr ? P.row_order[at] : at] != 0;
+                const u32  b   = __ballot_sync(0xffffffffu, set);
+                __syncthreads();
+                if ((tid & 31) == 0) {
+                    s_flagged[tid >> 5] = b;
+                }
+                __syncthreads();
+            }
+            if (word == 0) {
+                break;
+            }
+            t = first + step * (base + w * 32 + __ffs(word) - 1);
+            word &= word - 1;
+        }
         const int r    = P.row_order != nullptr ? P.row_order[t] : t;
         int       mode = 0;
         if (P.topk_states != nullptr && !(P.topk_skip != nullptr && P.topk_skip[r])) {
@@ -1565,11 +1596,14 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
         }
         if (WHOLE && rank == 0) {
             if (!decided) {
-                sp_whole_row<DT>(P, r, smem_raw, nullptr);
+                sp_whole_row<DT>(P, r, again ? first : r, smem_raw, nullptr);
             }
             if (A.stop.stop_words != nullptr || A.stop.limit != nullptr) {
                 sp_stop_criteria(P, A.stop, r);
             }
+        }
+        if (again) {
+            cluster_sync();  // (the next row starts with nobody inside this one)
         }
     }
     cluster_sync();  // no CTA leaves while another may still reach into its shared memory
@@ -1601,7 +1635,7 @@ int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, c
     attr[0].val.clusterDim.x = 1u << LGN;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim              = dim3((unsigned)K.local_batch << LGN);
+    cfg.gridDim              = dim3((unsigned)(A.clusters > 0 ? A.clusters : K.local_batch) << LGN);
     cfg.blockDim             = dim3(kThreads);
     cfg.dynamicSmemBytes     = smem;
     cfg.stream               = st;
@@ -1616,8 +1650,11 @@ template<int DT>
 int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_general, cudaStream_t st)
 {
     const size_t smem = split_smem_bytes(A.slice, A.area);
+    const size_t both = smem > smem_general ? smem : smem_general;
+    if (A.clusters > 0) {
+        return split_sampling_launch_n<DT, 3, true>(K, A, both, st);
+    }
     if (A.redo_flags == nullptr) {
-        const size_t both = smem > smem_general ? smem : smem_general;
         return A.lgn == 2 ? split_sampling_launch_n<DT, 2, true>(K, A, both, st) :
                             split_sampling_launch_n<DT, 3, true>(K, A, both, st);
     }

@@ -69,3 +69,32 @@ def test_split_kernel_equals_general_kernel(dtype, V, Vp, B, ties, log_probs, cu
     for k, v in want.items():
         np.testing.assert_array_equal(got[k], v, err_msg=k)
     assert want["stops"].tolist() == [False, False, True]
+
+
+@pytest.mark.parametrize("dtype,V,B", [(BF16, 110003, 44), (F32, 60000, 80), (F16, 36000, 150)])
+def test_wide_nuclei_of_many_rows(dtype, V, B, cuda_device):
+    """Flat rows whose nucleus does not fit the first launch's areas, several to a cluster of the second one."""
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    got = []
+    for general in (1, 0):
+        g = torch.Generator(device=cuda_device)
+        g.manual_seed(V)
+        layer = DynamicDecodeLayer(V, V, dtype, cuda_device)
+        layer.setup(B, 1, {"runtime_top_p": np.asarray([0.98], np.float32), "temperature": np.asarray([1.1], np.float32),
+                           "random_seed": np.arange(B).astype(np.uint64)})
+        st = {"output_ids": torch.ones(12, B, dtype=torch.int32, device=cuda_device),
+              "finished": torch.arange(B, device=cuda_device) % 9 == 4,
+              "sequence_length": torch.full((B,), 8, dtype=torch.int32, device=cuda_device),
+              "cum_log_probs": torch.zeros(B, device=cuda_device), "output_log_probs": torch.zeros(8, B, device=cuda_device)}
+        lib.ftb200_set_single_pass(1 - general)
+        try:
+            for s in range(2):
+                x = torch.randn(B, V, generator=g, device=cuda_device) * 0.8
+                layer.forward(st, {"logits": x.to(dtype), "step": 8 + s, "max_input_length": 8, "ite": 0, "local_batch_size": B,
+                                   "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)})
+            torch.cuda.synchronize()
+        finally:
+            lib.ftb200_set_single_pass(1)
+        got.append({k: v.cpu().numpy() for k, v in st.items()} | {"curand": layer.topp.curand.cpu().numpy()})
+    for k, v in got[0].items():
+        np.testing.assert_array_equal(got[1][k], v, err_msg=k)
