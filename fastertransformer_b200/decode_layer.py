@@ -70,6 +70,7 @@ class _Pack:
             dev[:upload].copy_(staged, non_blocking=True)
         for owner, name, dtype, at, size, _ in self.parts:
             setattr(owner, name, dev[at:at + size].view(dtype))
+        return dev
 
 
 class DynamicDecodeLayer:
@@ -82,8 +83,8 @@ class DynamicDecodeLayer:
         self.device = torch.device(device)
         self.stream = stream
         self._device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
-        self._workspace = None
-        self._beam_ws = None
+        self._setup_mem = self._workspace = self._beam_ws = self._arrived = None
+        self._home = None           # stream all of the layer's device memory was allocated on, see _allocated()
         self._beam_key = self._beam_blocks = None
         self._gate = {}
         self.time_kernels = False   # when set, CUDA events bracket each fused launch (kernel_events)
@@ -103,6 +104,33 @@ class DynamicDecodeLayer:
         if _raw_stream is not None:
             return _raw_stream(self._device_index)
         return torch.cuda.current_stream(self.device).cuda_stream
+
+    # Device memory of the layer, by attribute.  The caching allocator hands a freed block out again on the stream it was
+    # allocated on, without a look at the others: a call on another stream has to be noted on each of them.
+    _MEMORY = ("_setup_mem", "_workspace", "_beam_ws", "_arrived", "_count_dev")
+
+    def _allocated(self, make):
+        """What `make` allocates, on the layer's own stream if it has one, else on the current one."""
+        if self.device.type != "cuda":
+            return make()
+        with torch.cuda.stream(self.stream):  # (None: the current one)
+            t = make()
+        on = self._raw_stream()
+        # (several streams: none of them is the home of all)
+        self._home = on if self._home is None or self._home == on else -1
+        return t
+
+    def _enter(self):
+        """Looks up the stream of a call, and keeps the layer's memory from being handed out before its work is done."""
+        self._stream = self._raw_stream()
+        if self._stream != self._home and self._home is not None:
+            here = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
+            for t in self._memory():
+                t.record_stream(here)
+
+    def _memory(self):
+        mem = [getattr(self, name) for name in self._MEMORY] + [g["order"] for g in self._gate.values()]
+        return [t for t in mem if t is not None]
 
     @staticmethod
     def _arg(args, key):
@@ -202,8 +230,7 @@ class DynamicDecodeLayer:
             for name, dtype in (("initial", torch.float32), ("decay", torch.float32), ("min", torch.float32),
                                 ("reset", torch.int32)):
                 pack.add(self.topp, name, dtype, B)
-        with torch.cuda.stream(self.stream):  # (None: the current one)
-            pack.place(dev)
+        self._setup_mem = self._allocated(lambda: pack.place(dev))
         tk, tp = self.topk, self.topp
         S = SetupParams()
         S.batch = B
@@ -224,6 +251,9 @@ class DynamicDecodeLayer:
             S.top_p_reset_ids = _addr(a.get("top_p_reset_ids"))
         S.stream = st.value
         check(lib.ftb200_setup_sampling(C.byref(S)))
+        # The arguments, the launch order and the generators are there when this returns: steps may follow on any stream,
+        # from any thread, under capture.  (An event would do for the first of these only; a request waits 10 us here once.)
+        (self.stream if self.stream is not None else torch.cuda.current_stream(dev)).synchronize()
 
     # ---- forward (DynamicDecodeLayer.cc:191-474, sampling branch) ---------------------------------
     def forward(self, outputs, inputs):
@@ -245,11 +275,11 @@ class DynamicDecodeLayer:
                 "temp": bool((self.temperature_host[lo:hi] != 1.0).any()),
                 "pen": bool((self.penalty_host[lo:hi] != self.penalty_default).any()),
                 "minlen": int(self.min_length_host[lo:hi].max()),
-                "order": self._order if lo == 0 and hi == self.batch_size else
-                torch.from_numpy(np.argsort(-self._row_cost[lo:hi], kind="stable").astype(np.int32)).to(self.device),
+                "order": self._order if lo == 0 and hi == self.batch_size else self._allocated(
+                    lambda: torch.from_numpy(np.argsort(-self._row_cost[lo:hi], kind="stable").astype(np.int32)).to(self.device)),
             }
         self._g = g
-        self._stream = self._raw_stream()  # one look-up per call, used by the sampling and the criteria launch
+        self._enter()  # one look-up of the stream per call, used by the sampling and the criteria launch
         if not (g["topk_on"] or g["topp_on"]):
             return self._stop_criteria(outputs, inputs, B, step, lbs, lo)
         P = self._fill(outputs, inputs, logits, B, step, ite, lbs, mil, lo)
@@ -261,7 +291,7 @@ class DynamicDecodeLayer:
         # sampling, stop criteria and the wait for should_stop in one call
         S = self._stop
         if S is None:
-            self._arrived = torch.zeros(1, dtype=torch.int32, device=self.device)
+            self._arrived = self._allocated(lambda: torch.zeros(1, dtype=torch.int32, device=self.device))
             self._result = torch.zeros(1, dtype=torch.int64).pin_memory()
             S = self._stop = StopParams()
             S.arrived_dev, S.result_host = self._arrived.data_ptr(), self._result.data_ptr()
@@ -287,7 +317,7 @@ class DynamicDecodeLayer:
         ite = int(inputs.get("ite", 0))
         lbs = int(inputs.get("local_batch_size", B))
         mil = int(inputs["max_input_length"])
-        self._stream = self._raw_stream()
+        self._enter()
         st = C.c_void_p(self._stream)
         es = logits.element_size()
         out_ids = outputs["output_ids"]
@@ -335,7 +365,7 @@ class DynamicDecodeLayer:
         need = C.c_size_t(0)
         check(lib.ftb200_beam_workspace_bytes(sub, K, C.byref(need)))
         if self._beam_ws is None or self._beam_ws.numel() < need.value:
-            self._beam_ws = torch.empty(need.value, dtype=torch.uint8, device=self.device)
+            self._beam_ws = self._allocated(lambda: torch.empty(need.value, dtype=torch.uint8, device=self.device))
         if "repetition_penalty" in inputs and "presence_penalty" in inputs:
             raise RuntimeError("[FT][ERROR] Found ambiguous parameters repetition_penalty and "
                                "presence_penalty which are mutually exclusive.")
@@ -392,7 +422,7 @@ class DynamicDecodeLayer:
         if sw is None and lim is None:
             return False
         if self._count_dev is None:
-            self._count_dev = torch.zeros(1, dtype=torch.int32, device=self.device)
+            self._count_dev = self._allocated(lambda: torch.zeros(1, dtype=torch.int32, device=self.device))
             self._count_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         L = 0 if sw is None else sw.shape[-1]
         st = C.c_void_p(self._stream)
@@ -471,7 +501,7 @@ class DynamicDecodeLayer:
                 need = C.c_size_t(0)
                 check(lib.ftb200_sampling_workspace_bytes(P.dtype, lbs, Vp, C.byref(need)))
                 if self._workspace is None or self._workspace.numel() < need.value:
-                    self._workspace = torch.empty(need.value, dtype=torch.uint8, device=self.device)
+                    self._workspace = self._allocated(lambda: torch.empty(need.value, dtype=torch.uint8, device=self.device))
                 self._ws_key = (P.dtype, lbs, Vp)
             P.stream = self._stream
             g["ptrs"] = ptrs
