@@ -113,20 +113,21 @@ class DynamicDecodeLayer:
         """What `make` allocates, on the layer's own stream if it has one, else on the current one."""
         if self.device.type != "cuda":
             return make()
-        with torch.cuda.stream(self.stream):  # (None: the current one)
+        if self.stream is None:
             t = make()
+        else:
+            with torch.cuda.stream(self.stream):
+                t = make()
         on = self._raw_stream()
         # (several streams: none of them is the home of all)
         self._home = on if self._home is None or self._home == on else -1
         return t
 
-    def _enter(self):
-        """Looks up the stream of a call, and keeps the layer's memory from being handed out before its work is done."""
-        self._stream = self._raw_stream()
-        if self._stream != self._home and self._home is not None:
-            here = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
-            for t in self._memory():
-                t.record_stream(here)
+    def _away(self):
+        """Before a call on another stream than the one all of the layer's memory was allocated on."""
+        here = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
+        for t in self._memory():
+            t.record_stream(here)
 
     def _memory(self):
         mem = [getattr(self, name) for name in self._MEMORY] + [g["order"] for g in self._gate.values()]
@@ -279,7 +280,9 @@ class DynamicDecodeLayer:
                     lambda: torch.from_numpy(np.argsort(-self._row_cost[lo:hi], kind="stable").astype(np.int32)).to(self.device)),
             }
         self._g = g
-        self._enter()  # one look-up of the stream per call, used by the sampling and the criteria launch
+        self._stream = self._raw_stream()  # one look-up per call, used by the sampling and the criteria launch
+        if self._stream != self._home:
+            self._away()
         if not (g["topk_on"] or g["topp_on"]):
             return self._stop_criteria(outputs, inputs, B, step, lbs, lo)
         P = self._fill(outputs, inputs, logits, B, step, ite, lbs, mil, lo)
@@ -317,7 +320,9 @@ class DynamicDecodeLayer:
         ite = int(inputs.get("ite", 0))
         lbs = int(inputs.get("local_batch_size", B))
         mil = int(inputs["max_input_length"])
-        self._enter()
+        self._stream = self._raw_stream()
+        if self._stream != self._home:
+            self._away()
         st = C.c_void_p(self._stream)
         es = logits.element_size()
         out_ids = outputs["output_ids"]

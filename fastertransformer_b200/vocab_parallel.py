@@ -115,8 +115,9 @@ class VocabParallelSampler(DynamicDecodeLayer):
         if self._workspace is None or self._workspace.numel() < need:
             self._workspace = self._allocated(lambda: torch.empty(need, dtype=torch.uint8, device=self.device))
         P.workspace, P.workspace_bytes = self._workspace.data_ptr(), self._workspace.numel()
-        self._enter()
-        P.stream = self._stream
+        P.stream = stream = self._raw_stream()
+        if stream != self._home:
+            self._away()
         return P
 
     def _has_topp(self):
