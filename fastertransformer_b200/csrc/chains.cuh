@@ -30,10 +30,6 @@ __device__ __forceinline__ u32 lds_u16(u32 a)
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
     return v;
 }
-__device__ __forceinline__ void sts_u16(u32 a, u32 v)
-{
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
-}
 
 __device__ __forceinline__ void walk_chains(const Chains& c)
 {

@@ -108,6 +108,10 @@ __device__ __forceinline__ void sts_u32(u32 a, u32 v)
 {
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
+__device__ __forceinline__ void sts_u16(u32 a, u32 v)
+{
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+}
 
 // Tells the compiler that a pointer loaded from a structure points into shared memory, so that it emits
 // ld.shared / st.shared instead of generic accesses (every pointer of the kernel's shared-memory map qualifies).

@@ -20,6 +20,7 @@
 // left untouched (its generator state included) and goes to the list.
 #pragma once
 #include "sampling_kernels.cuh"
+#include "spans.cuh"
 
 namespace ftb200 {
 
@@ -73,6 +74,17 @@ __host__ __device__ inline size_t fast_smem_bytes(int hash_slots, int vocab_padd
 __device__ __forceinline__ void cp_async4(u32 saddr, const void* g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(g) : "memory");
+}
+// The aligned word around byte `at` of an array of n bytes, its bytes outside of the array as zeros.
+__device__ __forceinline__ void cp_async_byte(u32 saddr, const uint8_t* array, int n, int at)
+{
+    const WordSpan W = word_span((size_t)array, n, at);
+    if (W.bytes != 0) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(saddr), "l"(array + W.from), "r"(W.bytes) : "memory");
+    }
+    else {
+        sts_u32(saddr, (u32)array[at] << (8 * (at - W.from)));
+    }
 }
 __device__ __forceinline__ void cp_async_wait_all()
 {
@@ -445,9 +457,8 @@ enum { kPreStateK = 0, kPreStateP = 12, kPreSkipK = 24, kPreSkipP, kPreFin, kPre
 static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
 {
     const u32 base = (u32)__cvta_generic_to_shared(pre);
-    auto word = [&](int slot, const void* p) {
-        cp_async4(base + 4u * (u32)slot, (const void*)((size_t)p & ~(size_t)3));
-    };
+    auto word = [&](int slot, const void* p) { cp_async4(base + 4u * (u32)slot, p); };
+    auto byte = [&](int slot, const uint8_t* p) { cp_async_byte(base + 4u * (u32)slot, p, P.local_batch, nr); };
     if (P.topk_states != nullptr) {
         const char* st = (const char*)(P.topk_states + nr);
         cp_async16(base + 4u * kPreStateK, st);
@@ -456,7 +467,7 @@ static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
         word(kPreK, P.topk_ks + nr);
         word(kPrePk, P.topk_ps + nr);
         if (P.topk_skip != nullptr) {
-            word(kPreSkipK, P.topk_skip + nr);
+            byte(kPreSkipK, P.topk_skip);
         }
     }
     if (P.topp_states != nullptr) {
@@ -466,11 +477,11 @@ static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
         cp_async16(base + 4u * kPreStateP + 32u, st + 32);
         word(kPrePp, P.topp_ps + nr);
         if (P.topp_skip != nullptr) {
-            word(kPreSkipP, P.topp_skip + nr);
+            byte(kPreSkipP, P.topp_skip);
         }
     }
     if (P.finished != nullptr) {
-        word(kPreFin, P.finished + nr);
+        byte(kPreFin, P.finished);
     }
     word(kPreEnd, P.end_ids + nr);
     if (P.apply_temp) {

@@ -84,16 +84,20 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
     auto send_args = [&](int t) {
         if (tid == 32 && t < tasks) {
             const int r    = t % rows;
-            auto      word = [&](int slot, const void* p) {
+            const u32 args = (u32)__cvta_generic_to_shared(s_args);
+            auto      word = [&](int slot, const void* p) { cp_async4(args + 4u * (u32)slot, p); };
+            auto      byte = [&](int slot, const uint8_t* p) {
                 if (p != nullptr) {
-                    cp_async4((u32)__cvta_generic_to_shared(&s_args[slot]), (const void*)((size_t)p & ~(size_t)3));
+                    cp_async_byte(args + 4u * (u32)slot, p, rows, r);
                 }
             };
-            word(kSkipK, P.topk_skip != nullptr ? P.topk_skip + r : nullptr);
-            word(kSkipP, P.topp_skip != nullptr ? P.topp_skip + r : nullptr);
-            word(kFin, P.finished != nullptr ? P.finished + r : nullptr);
+            byte(kSkipK, P.topk_skip);
+            byte(kSkipP, P.topp_skip);
+            byte(kFin, P.finished);
             word(kK, P.topk_ks + r);
-            word(kTemp, temp ? P.temperature + r : nullptr);
+            if (temp) {
+                word(kTemp, P.temperature + r);
+            }
             cp_async_commit();
         }
     };
@@ -119,22 +123,24 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
         const int left  = V.vocab - T.sh * P.vocab_padded;
         T.vocab         = left < P.vocab_padded ? left : P.vocab_padded;
         T.vocab         = T.vocab < 1 ? 1 : T.vocab;
-        const char* p   = (const char*)V.logits[T.sh] + (size_t)T.r * P.vocab_padded * 2;
-        const int   off = (int)((size_t)p & 15);
-        T.base          = p - off;
-        T.mis           = off / 2;
-        T.nv            = (T.mis + T.vocab + 7) / 8;
+        const RowSpan S = row_span((size_t)V.logits[T.sh] + (size_t)T.r * P.vocab_padded * 2, T.vocab);
+        T.base          = (const char*)S.base;
+        T.mis           = S.mis;
+        T.nv            = S.nv;
         return T;
     };
     // the row's vectors in four parts (of whole fours of vectors per thread: vector i of a thread belongs to group i % 4),
     // so that the first ones can be looked at while the last are on their way
     const u32 row_s = (u32)__cvta_generic_to_shared(row), bar_s = (u32)__cvta_generic_to_shared(s_bar);
-    auto      send  = [&](const Task& T) {
+    auto      inside = [&](const Task& T) { return whole_vectors(rows, P.vocab_padded, T.r, T.mis, T.nv); };
+    auto      send   = [&](const Task& T) {
         if (tid == 0) {
-            const int per = ((T.nv + NT - 1) / NT + 15) / 16 * 4 * NT;
+            const VecRange W   = inside(T);
+            const int      per = ((T.nv + NT - 1) / NT + 15) / 16 * 4 * NT;
             for (int g = 0; g < 4; ++g) {
-                const int left = T.nv - g * per, n = left < 0 ? 0 : (left < per ? left : per);
-                bulk_copy(row_s + 16u * (u32)(g * per), T.base + 16 * (size_t)(g * per), 16u * (u32)n, bar_s + 8u * (u32)g);
+                const int skip = g == 0 ? W.first : 0, left = W.last - g * per, n = left < 0 ? 0 : (left < per ? left : per);
+                bulk_copy(row_s + 16u * (u32)(g * per + skip), T.base + 16 * (size_t)(g * per + skip), 16u * (u32)(n - skip),
+                          bar_s + 8u * (u32)g);
             }
         }
     };
@@ -189,8 +195,16 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
         }
         const __half inv_t_h = __float2half_rn(T.inv_t);
         const int    id0     = V.offset + T.sh * P.vocab_padded;  // token id of the shard's first column
-        // columns of the first and the last vector that are not the row's
+        // columns of the first and the last vector that are not the row's, and those of a vector that was not copied
         auto edge = [&](int j, uint4& v) {
+            const VecRange W0 = inside(T);
+            if (j < W0.first || j >= W0.last) {
+#pragma unroll 1
+                for (int c = max(j * 8 - T.mis, 0); c < min(j * 8 + 8 - T.mis, T.vocab); ++c) {
+                    sts_u16(row_s + 2u * (u32)(T.mis + c), (u32)__ldg((const unsigned short*)T.base + T.mis + c));
+                }
+                v = row[j];
+            }
             u32 w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
@@ -295,8 +309,8 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                         const int j = (i + u) * NT + tid;
                         if (i + u < i1 && j < T.nv) {
                             uint4 v = row[j];
-                            if (own_edge && (j == 0 || j == T.nv - 1)) {
-                                edge(j, v);
+                            if (own_edge && !special_launch && (j == 0 || j == T.nv - 1)) {
+                                edge(j, v);  // (done above, and columns taken out since, where there are special ones)
                             }
                             mx[u] = max2<DT>(mx[u], max2<DT>(max2<DT>(v.x, v.y), max2<DT>(v.z, v.w)));
                         }

@@ -65,3 +65,50 @@ def test_records_of_all_shards(dtype, n_shards, shard, k, form, cuda_device):
         for key in ("output_ids", "finished", "sequence_length"):
             assert torch.equal(a[key], b[key]), (s, key)
         assert torch.equal(full.topk.curand, vp.topk.curand)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("penalised", [False, True])
+@pytest.mark.parametrize("off,shard", [(1, 1237), (3, 40), (5, 2051), (7, 9001), (4, 60004)])
+def test_shards_off_a_vector_boundary(dtype, penalised, off, shard, cuda_device):
+    """Shards inside larger buffers, between two 16-byte boundaries: the first columns of the first row and the last ones
+    of the last row do not travel with the whole vectors.  They hold the row's largest values, some of them penalised, and
+    what lies around a shard would win if it were looked at."""
+    from fastertransformer_b200 import DynamicDecodeLayer, VocabParallelSampler
+    B, n, k, mil = 3, 2, 6, 6
+    V = n * shard
+    args = {"runtime_top_k": np.asarray([k], np.uint32), "random_seed": np.arange(B).astype(np.uint64)}
+    if penalised:
+        args["repetition_penalty"] = np.asarray([1.5], np.float32)
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(off * 100 + shard)
+    x = torch.randn(B, V, generator=g, device=cuda_device)
+    for i in range(n):
+        x[0, i * shard:i * shard + 8] += 9.0 + torch.arange(8, device=cuda_device)
+        x[-1, (i + 1) * shard - 8:(i + 1) * shard] += 9.0 + torch.arange(8, device=cuda_device)
+    x = x.to(dtype)
+    ids = torch.zeros(mil + 1, B, dtype=torch.int32, device=cuda_device)
+    ids[:mil] = torch.tensor([[0, 0, V - 1], [2, 5, V - 2], [shard, 9, shard - 1], [shard + 1, 3, shard - 3], [7, 7, V - 8], [1, 1, 1]],
+                             device=cuda_device)
+    words = torch.tensor([[4, V - 4], [1, 2]], dtype=torch.int32, device=cuda_device)
+    shards = []
+    for i in range(n):
+        buf = torch.full((off + B * shard + 8,), 1000.0, dtype=dtype, device=cuda_device)
+        shards.append(buf[off:off + B * shard].view(B, shard))
+        shards[-1].copy_(x[:, i * shard:(i + 1) * shard])
+    got = []
+    for layer in (DynamicDecodeLayer(V, V, dtype, cuda_device), VocabParallelSampler(V, shard, n, dtype, cuda_device)):
+        layer.setup(B, 1, args)
+        st = {"output_ids": ids.clone(), "finished": torch.zeros(B + 2, dtype=torch.bool, device=cuda_device)[1:B + 1],
+              "sequence_length": torch.full((B,), mil, dtype=torch.int32, device=cuda_device)}
+        inp = {"step": mil, "max_input_length": mil, "end_id": torch.full((B,), V // 2, dtype=torch.int32, device=cuda_device)}
+        if penalised:
+            inp["bad_words_list"] = words
+        if isinstance(layer, VocabParallelSampler):
+            layer.forward_shards(st, inp, shards)
+        else:
+            layer.forward(st, dict(inp, logits=x))
+        torch.cuda.synchronize()
+        got.append((st["output_ids"].cpu(), st["finished"].cpu(), st["sequence_length"].cpu(), layer.topk.curand.cpu()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
