@@ -40,6 +40,11 @@ int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_gene
 extern template int split_sampling_launch<FTB200_F32>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
 extern template int split_sampling_launch<FTB200_F16>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
 extern template int split_sampling_launch<FTB200_BF16>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
+template<int DT>
+int split_resident(int lgn, bool whole, size_t smem);
+extern template int split_resident<FTB200_F32>(int, bool, size_t);
+extern template int split_resident<FTB200_F16>(int, bool, size_t);
+extern template int split_resident<FTB200_BF16>(int, bool, size_t);
 size_t fast_smem_for(int hash_slots, int vocab_padded, bool topp);
 int    fast_max_history();
 int    fast_max_words();
@@ -92,13 +97,31 @@ static size_t redo_list_bytes(int local_batch)
 
 static int g_fast_path = 1;  // see ftb200_set_single_pass
 
+// Clusters of the split kernel that are resident at once.  A cluster stays inside a group of SMs, and the groups' sizes are
+// no multiples of eight: with one, two, three CTAs on an SM 15, 33 and 48 clusters of eight fit, not 18, 37 and 55.
+static int resident_clusters(int dtype, int lgn, bool whole, size_t smem)
+{
+    switch (dtype) {
+        case FTB200_F32: return split_resident<FTB200_F32>(lgn, whole, smem);
+        case FTB200_F16: return split_resident<FTB200_F16>(lgn, whole, smem);
+        default: return split_resident<FTB200_BF16>(lgn, whole, smem);
+    }
+}
+
+constexpr size_t kWholeTwoPerSm = 103 * 1024, kTwoPerSm = 107 * 1024 + 512, kThreePerSm = 69 * 1024;
+
 // Whether the split kernel (a row over a cluster of CTAs) serves a call, and in which form.  `single_pass`: the
-// single-pass kernels could serve it too.  The lines come from timing both at 32000 .. 256000 columns and 1 .. 1024
-// rows: the split form ends a row in 6 us (arg-max) to 40 us (wide nucleus) however slow the row is for one CTA, but
-// costs 2 to 4 times the SM time, so it loses once the single-pass kernels have the chip full.  With both kinds of rows
-// in a call those wait longest for their slowest rows (1024 x 32000: 191 us split, 216 us single-pass; 128 x 128256:
-// 113 / 120; 256 x 128256: 207 / 134); nucleus rows alone pack better (256 x 51200: 100 / 71, 64 x 51200: 51 / 72);
-// rows of a small k are nearly as quick in one CTA.
+// single-pass kernels could serve it too.  The lines come from timing both at 17000 .. 250000 columns and 6 .. 1024
+// rows (us a step, split / single-pass): the split form ends a row in 6 us (arg-max) to 40 us (wide nucleus) however slow
+// the row is for one CTA, but costs 2 to 4 times the SM time, so it loses once the single-pass kernels have the chip full.
+// With both kinds of rows in a call those wait longest for their slowest rows: 128 x 128256 107 / 117, 160 x 128256 129 / 130,
+// 256 x 128256 196 / 134, 96 x 250000 177 / 173 (at few columns the split form still wins above the line: 700 x 32000
+// 128 / 178, 512 x 51200 174 / 199, 700 x 51200 228 / 210).  Rows of a small k are nearly as quick in one CTA: k = 50 64 x
+// 32000 30 / 32, 128 x 32000 35 / 32; k = 1024 128 x 32000 48 / 76, 32 x 128256 48 / 74, 64 x 128256 79 / 78.
+// Nucleus rows alone: with two CTAs a row all clusters have to be resident (148 x 17000 38 / 52, 148 x 32000 46 / 60, 192 x
+// 32000 71 / 64), with four a third more may wait (64 x 51200 51 / 68, 80 x 51200 66 / 69, 96 x 41000 75 / 77, 112 x 51200
+// 75 / 71), with eight, whose rows take one CTA longest, two rounds of them and more above 110000 columns (64 x 80000 81 / 80,
+// 80 x 80000 100 / 83, 80 x 100000 123 / 111; 64 x 128256 99 / 113, 80 x 128256 117 / 114).
 static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool single_pass, size_t smem_general,
                          SplitArgs* A, bool* whole)
 {
@@ -106,18 +129,16 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     if (vocab < 1024) {
         return false;  // (the denominator's chains are then not 1024)
     }
-    if (single_pass) {
-        const double work = (double)rows * vocab;
-        const bool   topk = K.topk_states != nullptr, topp = K.topp_states != nullptr;
-        const double most = topk && topp ? 16.5e6 : (topp ? (rows <= 96 ? 9e6 : 0.0) : (K.max_top_k > 256 ? 4.2e6 : 2.1e6));
-        if (work > most) {
-            return false;
-        }
+    const bool topk = K.topk_states != nullptr, topp = K.topp_states != nullptr, mixed = topk && topp;
+    if (single_pass && (double)rows * vocab > (mixed ? 16.5e6 : (topp ? 9e6 : (K.max_top_k > 256 ? 4.2e6 : 2.1e6)))) {
+        return false;
     }
     // CTAs per row: eight while they are all resident (and for rows so long that a slice would not leave room for
     // three CTAs on an SM), four or two when there are more rows or the rows are short: a CTA's fixed costs then weigh
-    // more than its columns (1024 x 32000 fp32, k = 50: 445 us with eight, 184 us with two).
-    int lgn = rows * 8 <= 2 * sms || vocab > 65536 ? 3 : (rows * 4 <= 2 * sms || vocab > 40960 ? 2 : 1);
+    // more than its columns (1024 x 32000 fp32, k = 50: 445 us with eight, 184 us with two).  With both kinds of rows the
+    // costliest are started first and a last few that wait for a place are short: there the SMs are counted alone.
+    const auto most_rows = [&](int lg) { return mixed ? 2 * sms >> lg : resident_clusters(p->dtype, lg, false, kTwoPerSm); };
+    int        lgn       = vocab > 65536 || rows <= most_rows(3) ? 3 : (vocab > 40960 || rows <= most_rows(2) ? 2 : 1);
     for (; lgn <= 3; ++lgn) {
         A->slice = ((vocab + 1023) / 1024) << (10 - lgn);
         A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
@@ -128,12 +149,20 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     if (lgn > 3) {
         return false;
     }
-    A->lgn = lgn;
-    // The form that keeps every row is taken while its CTAs are resident at once, two on an SM where shared memory
-    // allows.  The collection areas: a wide nucleus of a flat row takes half of the columns, so up to 5/8 of a slice is
-    // provided for as far as that residency holds (a row beyond it costs a millisecond in the general code).
-    constexpr size_t whole_two_per_sm = 103 * 1024, two_per_sm = 107 * 1024 + 512, three_per_sm = 69 * 1024;
-    const auto       area_within = [&](size_t budget, int most) {
+    A->lgn             = lgn;
+    const size_t least = split_smem_bytes(A->slice, kSpAreaMin);
+    if (single_pass && topp && !topk) {
+        const int at_once = resident_clusters(p->dtype, lgn, false, lgn == 1 ? least : kTwoPerSm);
+        const int most    = lgn == 1 ? at_once : (lgn == 2 ? at_once * 4 / 3 : (int)(2.0 * at_once * (vocab > 110000 ? vocab / 110000.0 : 1.0)));
+        if (rows > most) {
+            return false;
+        }
+    }
+    // The form that keeps every row is taken while its clusters are resident at once, with two CTAs on an SM where shared
+    // memory allows (16 x 128256 bf16, one CTA on an SM: k = 50 60 us a step, 46 in the other form; 14 rows 39 / 45).  The
+    // collection areas: a wide nucleus of a flat row takes half of the columns, so up to 5/8 of a slice is
+    // provided for as far as that residency holds (a row beyond it costs milliseconds in the general code).
+    const auto area_within = [&](size_t budget, int most) {
         int area = (A->slice * 5 / 8 + 1023) / 1024 * 1024;
         area     = area > most ? most : (area < kSpAreaMin ? kSpAreaMin : area);
         while (area > kSpAreaMin && split_smem_bytes(A->slice, area) > budget) {
@@ -141,11 +170,16 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
         }
         return area;
     };
-    const size_t least = split_smem_bytes(A->slice, kSpAreaMin);
-    const int    ctas  = rows << lgn;
-    *whole             = lgn >= 2 && (ctas <= sms || (ctas <= 2 * sms && least <= whole_two_per_sm && smem_general <= whole_two_per_sm));
-    A->area            = *whole ? area_within(ctas <= sms ? kSpMaxSmem : whole_two_per_sm, kSpAreaMax) :
-                                  area_within(least <= three_per_sm ? three_per_sm : (least <= two_per_sm ? two_per_sm : kSpMaxSmem), kSpAreaMid);
+    const int  ctas  = rows << lgn;
+    const auto keeps = [&](int per_sm, size_t budget) {
+        A->area           = area_within(budget, kSpAreaMax);
+        const size_t smem = split_smem_bytes(A->slice, A->area);
+        return mixed ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, smem > smem_general ? smem : smem_general);
+    };
+    *whole = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kWholeTwoPerSm && smem_general <= kWholeTwoPerSm && keeps(2, kWholeTwoPerSm)));
+    if (!*whole) {
+        A->area = area_within(least <= kThreePerSm ? kThreePerSm : (least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem), kSpAreaMid);
+    }
     return true;
 }
 

@@ -3,4 +3,5 @@
 
 namespace ftb200 {
 template int split_sampling_launch<FTB200_F32>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
+template int split_resident<FTB200_F32>(int, bool, size_t);
 }  // namespace ftb200

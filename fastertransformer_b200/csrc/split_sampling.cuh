@@ -1502,7 +1502,11 @@ static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, int ar
 // resident at once; with more rows the general code's shared memory would cost residency, and the rows it is needed
 // for are left to a second launch: decode_sampling_kernel, or - where the areas of the first launch are small - a few
 // clusters of this form with all the shared memory there is (A.clusters), because a nucleus of half of 127000 columns takes
-// 0.2 ms here and 5 to 9 ms in the general code (800 such rows, 42 of them flagged: 10.7 -> 1.9 ms for most steps).
+// 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of 127000 columns, under half of
+// 200000 ones) still ends in the general code, so a batch of flat rows takes what its widest nucleus takes.  Mean and slowest
+// of 30 steps of fresh normal logits, 800 x 126959 bf16 with log-probabilities: 1.2 / 1.2 ms (sigma 2.5, p 0.95), 2.3 / 2.7
+// (sigma 2, p 0.95, temperature 1.2), 27 / 43 (sigma 1.5, p 0.95, temperature 1.2); 60 x 200000 fp32: 0.9 / 1.8, 9.4 / 10.2 and
+// 13.6 / 15.1 ms.
 template<int DT, int LGN, bool WHOLE>
 __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
                                                                      const __grid_constant__ SplitArgs A)
@@ -1610,39 +1614,94 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
 }
 
 template<int DT, int LGN, bool WHOLE>
-int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, cudaStream_t st)
+int split_opt_in(int* device)
 {
     constexpr int     kMaxDev = 64;
     static std::mutex mu;
     static bool       opted_in[kMaxDev];
-    int               dev = 0;
-    FTB_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev) {
+    FTB_CUDA_CHECK(cudaGetDevice(device));
+    if (*device < 0 || *device >= kMaxDev) {
         set_error("ftb200_decode_step_sampling: device ordinal out of range");
         return FTB200_UNSUPPORTED;
     }
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!opted_in[dev]) {
-            FTB_CUDA_CHECK(cudaFuncSetAttribute(split_sampling_kernel<DT, LGN, WHOLE>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpMaxSmem));
-            opted_in[dev] = true;
-        }
+    std::lock_guard<std::mutex> lock(mu);
+    if (!opted_in[*device]) {
+        FTB_CUDA_CHECK(cudaFuncSetAttribute(split_sampling_kernel<DT, LGN, WHOLE>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpMaxSmem));
+        opted_in[*device] = true;
     }
-    cudaLaunchConfig_t  cfg{};
-    cudaLaunchAttribute attr[1];
+    return FTB200_OK;
+}
+
+static inline void split_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int lgn, int clusters, size_t smem,
+                                       cudaStream_t st)
+{
     attr[0].id               = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1u << LGN;
+    attr[0].val.clusterDim.x = 1u << lgn;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim              = dim3((unsigned)(A.clusters > 0 ? A.clusters : K.local_batch) << LGN);
+    cfg.gridDim              = dim3((unsigned)clusters << lgn);
     cfg.blockDim             = dim3(kThreads);
     cfg.dynamicSmemBytes     = smem;
     cfg.stream               = st;
     cfg.attrs                = attr;
     cfg.numAttrs             = 1;
+}
+
+template<int DT, int LGN, bool WHOLE>
+int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, cudaStream_t st)
+{
+    int       dev = 0;
+    const int rc  = split_opt_in<DT, LGN, WHOLE>(&dev);
+    if (rc != FTB200_OK) {
+        return rc;
+    }
+    cudaLaunchConfig_t  cfg{};
+    cudaLaunchAttribute attr[1];
+    split_launch_config(cfg, attr, LGN, A.clusters > 0 ? A.clusters : K.local_batch, smem, st);
     FTB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_sampling_kernel<DT, LGN, WHOLE>, K, A));
     return FTB200_OK;
+}
+
+template<int DT, int LGN, bool WHOLE>
+int split_resident_n(size_t smem)
+{
+    // asked once per device and kilobyte of shared memory (what a call needs moves in steps of the vocabulary)
+    constexpr int             kMost = (int)(kSpMaxSmem / 1024) + 1, kMaxDev = 64;
+    static std::atomic<short> known[kMaxDev][kMost];  // clusters + 1; 0: not asked yet
+    const int                 kb  = (int)((smem + 1023) / 1024);
+    int                       dev = 0;
+    if (kb >= kMost || cudaGetDevice(&dev) != cudaSuccess) {
+        return 0;
+    }
+    const bool keep = dev >= 0 && dev < kMaxDev;
+    short      v    = keep ? known[dev][kb].load(std::memory_order_relaxed) : 0;
+    if (v == 0) {
+        cudaLaunchConfig_t  cfg{};
+        cudaLaunchAttribute attr[1];
+        int                 n = 0;
+        split_launch_config(cfg, attr, LGN, 1, (size_t)kb * 1024, nullptr);
+        if (split_opt_in<DT, LGN, WHOLE>(&dev) != FTB200_OK
+            || cudaOccupancyMaxActiveClusters(&n, split_sampling_kernel<DT, LGN, WHOLE>, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return 0;
+        }
+        v = (short)(n + 1);
+        if (keep) {
+            known[dev][kb].store(v, std::memory_order_relaxed);
+        }
+    }
+    return v - 1;
+}
+
+// Clusters of 2^lgn CTAs with `smem` bytes of shared memory each that the current device holds at once.
+template<int DT>
+int split_resident(int lgn, bool whole, size_t smem)
+{
+    if (whole) {
+        return lgn == 2 ? split_resident_n<DT, 2, true>(smem) : split_resident_n<DT, 3, true>(smem);
+    }
+    return lgn == 1 ? split_resident_n<DT, 1, false>(smem) : (lgn == 2 ? split_resident_n<DT, 2, false>(smem) : split_resident_n<DT, 3, false>(smem));
 }
 
 // smem_general: shared memory of the general row code, for the form that keeps every row.

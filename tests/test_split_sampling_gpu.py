@@ -98,3 +98,48 @@ def test_wide_nuclei_of_many_rows(dtype, V, B, cuda_device):
         got.append({k: v.cpu().numpy() for k, v in st.items()} | {"curand": layer.topp.curand.cpu().numpy()})
     for k, v in got[0].items():
         np.testing.assert_array_equal(got[1][k], v, err_msg=k)
+
+
+def one_kind(general, kind, dtype, V, B, device):
+    """Two steps of a call with top-k rows or top-p rows alone; what they wrote and the launches they took."""
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    g = torch.Generator(device=device)
+    g.manual_seed(V + 3 * B)
+    args = {"random_seed": np.arange(B).astype(np.uint64), "repetition_penalty": np.asarray([1.1], np.float32)}
+    if kind == "topk":
+        args["runtime_top_k"] = np.asarray([40], np.uint32)
+    else:
+        args["runtime_top_p"] = np.asarray([0.9], np.float32)
+    layer = DynamicDecodeLayer(V, V, dtype, device)
+    layer.setup(B, 1, args)
+    st = {"output_ids": torch.randint(1, V, (20, B), generator=g, device=device, dtype=torch.int32),
+          "finished": torch.arange(B, device=device) % 7 == 5,
+          "sequence_length": torch.full((B,), 16, dtype=torch.int32, device=device)}
+    lib.ftb200_set_single_pass(0 if general else 1)
+    try:
+        for s in range(2):
+            x = (torch.randn(B, V, generator=g, device=device) * 2.5).to(dtype)
+            layer.forward(st, {"logits": x, "step": 16 + s, "max_input_length": 8,
+                               "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=device),
+                               "sequence_limit_length": torch.full((B,), 99, dtype=torch.int32, device=device)})
+        torch.cuda.synchronize()
+    finally:
+        lib.ftb200_set_single_pass(1)
+    out = {k: v.cpu().numpy() for k, v in st.items()}
+    out["curand"] = np.concatenate([layer.topk.curand.cpu().numpy(), layer.topp.curand.cpu().numpy()])
+    return out, layer.launches // 2
+
+
+@pytest.mark.parametrize("kind,dtype,V,B", [
+    ("topk", BF16, 128256, 14), ("topk", BF16, 128256, 18), ("topk", F32, 128256, 18), ("topk", F32, 32000, 33),
+    ("topk", F32, 32000, 37), ("topk", F32, 32000, 71), ("topk", F32, 32000, 74), ("topp", F32, 45000, 74), ("topp", F16, 17000, 148),
+    ("topp", F16, 17000, 149), ("topp", BF16, 32000, 120), ("topp", F16, 41000, 94), ("topp", F16, 41000, 95),
+    ("topp", BF16, 80000, 66), ("topp", BF16, 80000, 67)])
+def test_calls_of_one_kind_around_the_resident_clusters(kind, dtype, V, B, cuda_device):
+    """Sizes either side of the lines of the dispatch that follow from how many clusters are resident at once."""
+    want, _ = one_kind(True, kind, dtype, V, B, cuda_device)
+    got, launches = one_kind(False, kind, dtype, V, B, cuda_device)
+    for k, v in want.items():
+        np.testing.assert_array_equal(got[k], v, err_msg=k)
+    if kind == "topk" and V == 128256 and B == 18 and torch.cuda.get_device_properties(0).multi_processor_count <= 148:
+        assert launches > 1  # eighteen clusters of eight CTAs are not resident with one CTA on an SM
