@@ -775,11 +775,8 @@ constexpr size_t kBeamMaxSmem = 200 * 1024;
 template<int DT, bool TEMP, bool PEN>
 static int beam_rows_launch(const BeamK& K, size_t smem, cudaStream_t st)
 {
-    static bool opted[64];
-    const int   rc = chain_opt_in(beam_rows_kernel<DT, TEMP, PEN>, opted);
-    if (rc != FTB200_OK) {
-        return rc;
-    }
+    static std::atomic<bool> opted[kDevicesKnown];
+    FTB_CUDA_CHECK(opt_in_smem(beam_rows_kernel<DT, TEMP, PEN>, kBeamMaxSmem, opted));
     beam_rows_kernel<DT, TEMP, PEN><<<K.local_batch * K.K, kBeamThreads, smem, st>>>(K);
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
@@ -788,12 +785,10 @@ static int beam_rows_launch(const BeamK& K, size_t smem, cudaStream_t st)
 template<int DT>
 static int beam_launch(const BeamK& K, size_t smem, cudaStream_t st)
 {
-    static bool merge_opted[64];
-    int         rc = chain_opt_in(beam_merge_kernel<DT>, merge_opted);
-    if (rc == FTB200_OK) {
-        rc = K.apply_temp ? (K.flag_words > 0 ? beam_rows_launch<DT, true, true>(K, smem, st) : beam_rows_launch<DT, true, false>(K, smem, st)) :
-                            (K.flag_words > 0 ? beam_rows_launch<DT, false, true>(K, smem, st) : beam_rows_launch<DT, false, false>(K, smem, st));
-    }
+    static std::atomic<bool> merge_opted[kDevicesKnown];
+    FTB_CUDA_CHECK(opt_in_smem(beam_merge_kernel<DT>, kBeamMaxSmem, merge_opted));
+    const int rc = K.apply_temp ? (K.flag_words > 0 ? beam_rows_launch<DT, true, true>(K, smem, st) : beam_rows_launch<DT, true, false>(K, smem, st)) :
+                                  (K.flag_words > 0 ? beam_rows_launch<DT, false, true>(K, smem, st) : beam_rows_launch<DT, false, false>(K, smem, st));
     if (rc != FTB200_OK) {
         return rc;
     }

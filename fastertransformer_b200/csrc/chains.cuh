@@ -1,8 +1,7 @@
 // Chains of beam parents followed in parallel, shared by the gather tree, the archive and the beam step's penalties.
 #pragma once
-#include <mutex>
-
 #include "common.cuh"
+#include "device_once.cuh"
 #include "ftb200.h"
 
 namespace ftb200 {
@@ -106,24 +105,5 @@ __device__ __forceinline__ Chains map_chains(void* smem, int levels, int K, cons
     return c;
 }
 constexpr size_t kChainMaxSmem = 200 * 1024;
-
-// Shared memory above 48 KB is opted into once per device and kernel.
-template<class F>
-int chain_opt_in(F kernel, bool* done)
-{
-    static std::mutex           mu;
-    int                         dev = 0;
-    FTB_CUDA_CHECK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 0 || dev >= 64) {
-        set_error("device ordinal out of range");
-        return FTB200_UNSUPPORTED;
-    }
-    if (!done[dev]) {
-        FTB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainMaxSmem));
-        done[dev] = true;
-    }
-    return FTB200_OK;
-}
 
 }  // namespace ftb200

@@ -687,11 +687,8 @@ extern "C" int ftb200_gather_tree(const ftb200_gather_tree_params* a)
     // the parent table of an entry in shared memory where it fits (50000 level-beams), else tile by tile
     const size_t smem = chain_smem_bytes(a->max_time, a->beam_width);
     if (smem <= kChainMaxSmem) {
-        static bool opted_in[64];
-        const int   rc = chain_opt_in(gather_tree_chains_kernel, opted_in);
-        if (rc != FTB200_OK) {
-            return rc;
-        }
+        static std::atomic<bool> opted_in[kDevicesKnown];
+        FTB_CUDA_CHECK(opt_in_smem(gather_tree_chains_kernel, kChainMaxSmem, opted_in));
         gather_tree_chains_kernel<<<a->batch_size, kChainThreads, smem, (cudaStream_t)a->stream>>>(p);
     }
     else {
@@ -765,11 +762,8 @@ extern "C" int ftb200_insert_unfinished_path(const ftb200_beam_hyps* hyps, const
     p.beam_width           = beam_width;
     const size_t smem = chain_smem_bytes(max_seq_len, beam_width);
     if (smem <= kChainMaxSmem) {
-        static bool opted_in[64];
-        const int   rc = chain_opt_in(insert_chains_kernel, opted_in);
-        if (rc != FTB200_OK) {
-            return rc;
-        }
+        static std::atomic<bool> opted_in[kDevicesKnown];
+        FTB_CUDA_CHECK(opt_in_smem(insert_chains_kernel, kChainMaxSmem, opted_in));
         insert_chains_kernel<<<batch_size, kChainThreads, smem, (cudaStream_t)stream>>>(p);
     }
     else {

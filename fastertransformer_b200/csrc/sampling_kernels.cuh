@@ -20,6 +20,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "device_once.cuh"
 #include "sampling_params.cuh"
 
 namespace ftb200 {
@@ -4421,16 +4422,8 @@ int vp_merge_launch(const KParams& K, const u64* gathered, int nranks, int* over
     const int    area = topp || most >= (size_t)kCap ? kCap : (most < 4 * kThreads ? 4 * kThreads : ((int)most + 1) & ~1);
     const size_t smem = (size_t)area * 8 + (size_t)(topp ? kNB : 1024) * 4 + 1024 * 4;
     constexpr int kMostSmem = kCap * 8 + kNB * 4 + 1024 * 4;
-    constexpr int            kMaxDev = 64;
-    static std::atomic<bool> ready[kMaxDev];  // the opt-in to the shared-memory size, once per device
-    int                      dev = 0;
-    FTB_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev || !ready[dev].load(std::memory_order_acquire)) {
-        FTB_CUDA_CHECK(cudaFuncSetAttribute(vp_merge_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
-        if (dev >= 0 && dev < kMaxDev) {
-            ready[dev].store(true, std::memory_order_release);
-        }
-    }
+    static std::atomic<bool> ready[kDevicesKnown];
+    FTB_CUDA_CHECK(opt_in_smem(vp_merge_kernel<DT>, kMostSmem, ready));
     vp_merge_kernel<DT><<<grid, kThreads, smem, st>>>(K, gathered, nranks, overflow, area);
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;

@@ -1502,8 +1502,8 @@ static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, int ar
 // resident at once; with more rows the general code's shared memory would cost residency, and the rows it is needed
 // for are left to a second launch: decode_sampling_kernel, or - where the areas of the first launch are small - a few
 // clusters of this form with all the shared memory there is (A.clusters), because a nucleus of half of 127000 columns takes
-// 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of 127000 columns, under half of
-// 200000 ones) still ends in the general code, so a batch of flat rows takes what its widest nucleus takes.  Mean and slowest
+// 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of 127000 columns; above 163000
+// columns there is no such launch, 49000 columns end it) still ends in the general code, so a batch of flat rows takes what its widest nucleus takes.  Mean and slowest
 // of 30 steps of fresh normal logits, 800 x 126959 bf16 with log-probabilities: 1.2 / 1.2 ms (sigma 2.5, p 0.95), 2.3 / 2.7
 // (sigma 2, p 0.95, temperature 1.2), 27 / 43 (sigma 1.5, p 0.95, temperature 1.2); 60 x 200000 fp32: 0.9 / 1.8, 9.4 / 10.2 and
 // 13.6 / 15.1 ms.
@@ -1614,23 +1614,10 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
 }
 
 template<int DT, int LGN, bool WHOLE>
-int split_opt_in(int* device)
+cudaError_t split_opt_in()
 {
-    constexpr int     kMaxDev = 64;
-    static std::mutex mu;
-    static bool       opted_in[kMaxDev];
-    FTB_CUDA_CHECK(cudaGetDevice(device));
-    if (*device < 0 || *device >= kMaxDev) {
-        set_error("ftb200_decode_step_sampling: device ordinal out of range");
-        return FTB200_UNSUPPORTED;
-    }
-    std::lock_guard<std::mutex> lock(mu);
-    if (!opted_in[*device]) {
-        FTB_CUDA_CHECK(cudaFuncSetAttribute(split_sampling_kernel<DT, LGN, WHOLE>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpMaxSmem));
-        opted_in[*device] = true;
-    }
-    return FTB200_OK;
+    static std::atomic<bool> opted_in[kDevicesKnown];
+    return opt_in_smem(split_sampling_kernel<DT, LGN, WHOLE>, kSpMaxSmem, opted_in);
 }
 
 static inline void split_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int lgn, int clusters, size_t smem,
@@ -1651,11 +1638,7 @@ static inline void split_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttrib
 template<int DT, int LGN, bool WHOLE>
 int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, cudaStream_t st)
 {
-    int       dev = 0;
-    const int rc  = split_opt_in<DT, LGN, WHOLE>(&dev);
-    if (rc != FTB200_OK) {
-        return rc;
-    }
+    FTB_CUDA_CHECK((split_opt_in<DT, LGN, WHOLE>()));
     cudaLaunchConfig_t  cfg{};
     cudaLaunchAttribute attr[1];
     split_launch_config(cfg, attr, LGN, A.clusters > 0 ? A.clusters : K.local_batch, smem, st);
@@ -1667,21 +1650,21 @@ template<int DT, int LGN, bool WHOLE>
 int split_resident_n(size_t smem)
 {
     // asked once per device and kilobyte of shared memory (what a call needs moves in steps of the vocabulary)
-    constexpr int             kMost = (int)(kSpMaxSmem / 1024) + 1, kMaxDev = 64;
-    static std::atomic<short> known[kMaxDev][kMost];  // clusters + 1; 0: not asked yet
+    constexpr int             kMost = (int)(kSpMaxSmem / 1024) + 1;
+    static std::atomic<short> known[kDevicesKnown][kMost];  // clusters + 1; 0: not asked yet
     const int                 kb  = (int)((smem + 1023) / 1024);
     int                       dev = 0;
     if (kb >= kMost || cudaGetDevice(&dev) != cudaSuccess) {
         return 0;
     }
-    const bool keep = dev >= 0 && dev < kMaxDev;
+    const bool keep = dev >= 0 && dev < kDevicesKnown;
     short      v    = keep ? known[dev][kb].load(std::memory_order_relaxed) : 0;
     if (v == 0) {
         cudaLaunchConfig_t  cfg{};
         cudaLaunchAttribute attr[1];
         int                 n = 0;
         split_launch_config(cfg, attr, LGN, 1, (size_t)kb * 1024, nullptr);
-        if (split_opt_in<DT, LGN, WHOLE>(&dev) != FTB200_OK
+        if (split_opt_in<DT, LGN, WHOLE>() != cudaSuccess
             || cudaOccupancyMaxActiveClusters(&n, split_sampling_kernel<DT, LGN, WHOLE>, &cfg) != cudaSuccess) {
             (void)cudaGetLastError();
             return 0;

@@ -653,23 +653,9 @@ int vp_select_launch(const KParams& K, const VpArgs& V, size_t smem, int sms, cu
     // that leaves room for one CTA only gets 512 threads.
     int per_sm = (int)((228 * 1024) / (smem + 3 * 1024 + 768));
     per_sm     = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
-    constexpr int     kMaxDev = 64;
-    static std::mutex mu;
-    static bool       ready[kMaxDev];
-    int               dev = 0;
-    FTB_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev) {
-        set_error("ftb200_vocab_parallel_local: device ordinal out of range");
-        return FTB200_UNSUPPORTED;
-    }
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!ready[dev]) {
-            FTB_CUDA_CHECK(cudaFuncSetAttribute(vp_select_kernel<DT, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVpMaxSmem));
-            FTB_CUDA_CHECK(cudaFuncSetAttribute(vp_select_kernel<DT, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVpMaxSmem));
-            ready[dev] = true;
-        }
-    }
+    static std::atomic<bool> ready_256[kDevicesKnown], ready_512[kDevicesKnown];
+    FTB_CUDA_CHECK(per_sm == 1 ? opt_in_smem(vp_select_kernel<DT, 512>, kVpMaxSmem, ready_512) :
+                                 opt_in_smem(vp_select_kernel<DT, 256>, kVpMaxSmem, ready_256));
     const long long tasks = (long long)K.local_batch * V.n_shards;
     int             grid  = sms * per_sm;
     grid                  = grid < tasks ? grid : (int)tasks;
