@@ -43,6 +43,8 @@ struct BeamK {
     uint8_t* snap_finished;  // finished / sequence_length as they were before this step
     int*     snap_seq_len;
     int      flag_words;   // words of the bit map of penalised columns; 0: none in this call
+    int      listed;       // 0: a bit per column; else the map is a filter over column numbers modulo its (power of two)
+                           // size, and so many ids can stand in the list that decides
     int      chain_levels; // levels of the parent table in shared memory; 0: the chain is followed in global memory
 };
 
@@ -113,6 +115,10 @@ constexpr int kBeamCollect = 2048;  // columns at or above the row's bound that 
 // Marks the tokens of row bb's ancestry (the ids that the repetition / presence penalty applies to,
 // beam_search_penalty_kernels.cu:89-152) in the bit map.  The chain runs through every level's parents: it is cut into
 // segments whose maps compose (see chains.cuh), so that a long history costs a few walks of a segment's length.
+__host__ __device__ inline int list_words(int listed)
+{
+    return listed != 0 ? (listed + 4) / 4 * 4 : 0;  // (its length stands in front)
+}
 static __device__ __noinline__ void mark_ancestry(const BeamK& P, int bb, u32* bits, unsigned char* tables)
 {
     const int    tid = threadIdx.x, K = P.K, b = bb / K, V = P.vocab_padded;
@@ -120,9 +126,14 @@ static __device__ __noinline__ void mark_ancestry(const BeamK& P, int bb, u32* b
     const int    input_len = P.input_lengths != nullptr ? P.input_lengths[bb] : P.max_input_len;
     const int*   ids = P.output_ids + (size_t)b * K;
     const int*   par = P.parent_ids + (size_t)P.ite * K * P.local_batch + (size_t)b * K;
+    u32* const   list = bits + P.flag_words;
     auto         mark = [&](int id) {
         if (id >= 0 && id < V) {
-            smem_or(&bits[id >> 5], 1u << (id & 31));
+            const int at = P.listed != 0 ? id & (32 * P.flag_words - 1) : id;
+            smem_or(&bits[at >> 5], 1u << (at & 31));
+            if (P.listed != 0) {
+                list[1 + atomicAdd(&list[0], 1u)] = (u32)id;  // (one entry a level at most)
+            }
         }
     };
     auto skipped = [&](int level) { return level >= input_len && level < P.max_input_len; };
@@ -191,15 +202,16 @@ static __device__ __noinline__ void mark_ancestry(const BeamK& P, int bb, u32* b
     }
 }
 
-// TEMP: temperature, bias or a padded vocabulary; PEN: penalised columns.  A branch per column costs as much as the
+// TEMP: temperature, bias or a padded vocabulary; PEN: penalised columns (1: a bit map of them; 2: of more columns than
+// shared memory has bits for, about a million: a filter and a list of the ids).  A branch per column costs as much as the
 // column's arithmetic, so the variants are compiled apart.  Bound by latency and issue (24 instructions a column, a
 // running maximum and a sum as chains): one row of 32000 half columns 12 us, 256 of them 16 us; with a list search per
 // column, sixteen sorted lists and a pass per winner of a wide beam it was 80 us and up.
-template<int DT, bool TEMP, bool PEN>
+template<int DT, bool TEMP, int PEN>
 __global__ void __launch_bounds__(kBeamThreads, 3) beam_rows_kernel(const __grid_constant__ BeamK P)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // layout: ring of row tiles | u64 collected[kBeamCollect] | u32 bits[flag_words] | chain tables
+    // layout: ring of row tiles | u64 collected[kBeamCollect] | u32 bits[flag_words] | u32 list[list_words(listed)] | chain tables
     const u32      ring = (u32)__cvta_generic_to_shared(smem_raw);
     u64*           col  = (u64*)(smem_raw + (size_t)kBeamStages * kBeamTile * (DT == FTB200_F32 ? 4 : 2));
     u32*           bits = (u32*)(col + kBeamCollect);
@@ -243,13 +255,23 @@ __global__ void __launch_bounds__(kBeamThreads, 3) beam_rows_kernel(const __grid
 
     // ---- columns with a value of their own: repetition / presence penalty along the beam's ancestry, min-length mask
     if (PEN) {
-        for (int i = tid; i < P.flag_words; i += kBeamThreads) {
-            bits[i] = 0;
+        for (int i = tid; i < P.flag_words + (PEN == 2 ? 1 : 0); i += kBeamThreads) {
+            bits[i] = 0;  // (and the length of the list)
         }
         __syncthreads();
-        mark_ancestry(P, bb, bits, (unsigned char*)(bits + P.flag_words));
+        mark_ancestry(P, bb, bits, (unsigned char*)(bits + P.flag_words + list_words(P.listed)));
         __syncthreads();
     }
+    // rare: a column whose bit of the filter is set
+    auto in_list = [&](int v) {
+        const u32* list = bits + P.flag_words;
+        const int  n    = (int)list[0];
+        bool       hit  = false;
+        for (int i = 1; i <= n && !hit; ++i) {
+            hit = list[i] == (u32)v;
+        }
+        return hit;
+    };
     const bool   minlen = (P.step - P.max_input_len < P.min_length) && (P.seq_len[bb] + 1 - P.max_input_len < P.min_length);
     const int    masked = minlen ? end_id : -1;
     const float  pen    = beam_round<DT>(P.rep_penalty);
@@ -259,8 +281,9 @@ __global__ void __launch_bounds__(kBeamThreads, 3) beam_rows_kernel(const __grid
     auto value_of = [&](int v, u32 raw) -> float {
         float y = TEMP ? beam_temp<DT>(P, raw, v, inv, inv_h) : beam_plain<DT>(raw);
         if (PEN) {
-            const u32 w = bits[v >> 5];  // one word for the 32 columns of a warp
-            if ((w >> (v & 31)) & 1u) {
+            // one word for the 32 columns of a warp
+            const u32 w = bits[PEN == 2 ? (v >> 5) & (P.flag_words - 1) : v >> 5];
+            if (((w >> (v & 31)) & 1u) && (PEN != 2 || in_list(v))) {
                 if (P.penalty_type == FTB200_PENALTY_ADDITIVE) {
                     y = beam_round<DT>(y - pen);
                 }
@@ -772,7 +795,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_merge_kernel(const __grid_c
 
 constexpr size_t kBeamMaxSmem = 200 * 1024;
 
-template<int DT, bool TEMP, bool PEN>
+template<int DT, bool TEMP, int PEN>
 static int beam_rows_launch(const BeamK& K, size_t smem, cudaStream_t st)
 {
     static std::atomic<bool> opted[kDevicesKnown];
@@ -787,8 +810,16 @@ static int beam_launch(const BeamK& K, size_t smem, cudaStream_t st)
 {
     static std::atomic<bool> merge_opted[kDevicesKnown];
     FTB_CUDA_CHECK(opt_in_smem(beam_merge_kernel<DT>, kBeamMaxSmem, merge_opted));
-    const int rc = K.apply_temp ? (K.flag_words > 0 ? beam_rows_launch<DT, true, true>(K, smem, st) : beam_rows_launch<DT, true, false>(K, smem, st)) :
-                                  (K.flag_words > 0 ? beam_rows_launch<DT, false, true>(K, smem, st) : beam_rows_launch<DT, false, false>(K, smem, st));
+    const int pen = K.flag_words == 0 ? 0 : (K.listed == 0 ? 1 : 2);
+    int       rc;
+    if (K.apply_temp) {
+        rc = pen == 0 ? beam_rows_launch<DT, true, 0>(K, smem, st) :
+                        (pen == 1 ? beam_rows_launch<DT, true, 1>(K, smem, st) : beam_rows_launch<DT, true, 2>(K, smem, st));
+    }
+    else {
+        rc = pen == 0 ? beam_rows_launch<DT, false, 0>(K, smem, st) :
+                        (pen == 1 ? beam_rows_launch<DT, false, 1>(K, smem, st) : beam_rows_launch<DT, false, 2>(K, smem, st));
+    }
     if (rc != FTB200_OK) {
         return rc;
     }
@@ -877,10 +908,20 @@ extern "C" int ftb200_beam_search_step(const ftb200_beam_params* p)
 
     const bool penalise = p->penalty_type != FTB200_PENALTY_NONE && p->step > 0
                           && p->repetition_penalty != (p->penalty_type == FTB200_PENALTY_MULTIPLICATIVE ? 1.0f : 0.0f);
+    const size_t base   = (size_t)kBeamStages * kBeamTile * (p->dtype == FTB200_F32 ? 4 : 2) + (size_t)kBeamCollect * 8;
     K.flag_words        = penalise ? ((p->vocab_size_padded + 31) / 32 + 3) / 4 * 4 : 0;
-    size_t smem         = (size_t)kBeamStages * kBeamTile * (p->dtype == FTB200_F32 ? 4 : 2) + (size_t)kBeamCollect * 8 + (size_t)K.flag_words * 4;
+    K.listed            = 0;
+    if (base + (size_t)K.flag_words * 4 > kBeamMaxSmem) {
+        // more columns than there is room for bits: the ids of the ancestry in a list, and as large a filter as that leaves
+        K.listed     = p->step;
+        K.flag_words = 16384;
+        while (K.flag_words > 4096 && base + (size_t)(K.flag_words + list_words(K.listed)) * 4 > kBeamMaxSmem) {
+            K.flag_words /= 2;
+        }
+    }
+    size_t smem = base + (size_t)(K.flag_words + list_words(K.listed)) * 4;
     if (smem > kBeamMaxSmem) {
-        set_error("ftb200_beam_search_step: vocabulary too large for the bit map of penalised columns");
+        set_error("ftb200_beam_search_step: step too large for the list of penalised columns");
         return FTB200_UNSUPPORTED;
     }
     // the parents of all levels in shared memory where they fit

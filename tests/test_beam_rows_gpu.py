@@ -64,10 +64,51 @@ def test_beam_step_against_torch(dtype, B, K, V, step, penalty, ended, cuda_devi
     got = st["cum_log_probs"].view(B, K).cpu().numpy()
     np.testing.assert_allclose(got, scores, rtol=2e-5, atol=2e-5)
     ids, par = st["output_ids"][step].cpu().numpy(), st["parent_ids"][step].cpu().numpy()
-    if dtype == torch.float32 or penalty == 1.0:
-        near = np.abs(np.diff(scores, axis=1)).min(initial=1.0) < 1e-4  # two candidates too close to tell apart here
-        if not near:
-            np.testing.assert_array_equal(par * V + ids, words)
+    near = np.abs(np.diff(scores, axis=1)).min(initial=1.0) < 1e-4  # two candidates too close to tell apart here
+    if not near:
+        np.testing.assert_array_equal(par * V + ids, words)
     # every chosen continuation has the score that is reported for it
     for b in range(B):
         assert len({(int(p), int(i)) for p, i in zip(par[b], ids[b])}) == K
+
+
+def hot_columns(V, K, B, step, seed):
+    """Logits whose largest columns are few and far apart in any type, prompt and parents, with penalised columns among
+    the largest and beside them in the same word of a bit map, and one a power of two away."""
+    rng = np.random.default_rng(seed)
+    x = np.round(rng.uniform(-6.0, -2.0, size=(B, K, V)) * 8) / 8
+    ids, parents = rng.integers(3, V, size=(step + 1, B, K)), rng.integers(0, K, size=(step + 1, B, K))
+    m = step // K  # levels of each beam's columns; every beam's ancestry goes through all of them
+    for b in range(B):
+        level = rng.permutation(step)
+        for k in range(K):
+            cols = rng.choice(np.arange(40, V - 40), size=6 * K, replace=False)  # the largest first
+            x[b, k, cols] = 1.0 + np.arange(6 * K)[::-1] / (4.0 if K < 8 else 16.0)
+            near = np.stack([cols[:2 * K:2], cols[1:2 * K:2] ^ 1, (cols[2 * K:3 * K] + (1 << 19)) % V], 1).reshape(-1)[:m]
+            ids[level[k * m:k * m + near.size], b] = near[:, None]
+    return x, ids.astype(np.int32), parents.astype(np.int32)
+
+
+@pytest.mark.parametrize("dtype,V,B,K,step,seed", [
+    (torch.float32, 4097, 3, 4, 40, 1), (torch.bfloat16, 4097, 3, 4, 40, 1), (torch.bfloat16, 33001, 2, 9, 130, 1),
+    # the last vocabulary that has a bit for every column, and ones with a filter and a list
+    (torch.float32, 983040, 1, 2, 30, 1), (torch.float32, 983041, 1, 2, 30, 1), (torch.float32, 1200003, 2, 3, 600, 1),
+    (torch.bfloat16, 1245184, 1, 2, 30, 1), (torch.bfloat16, 1245192, 1, 4, 300, 2)])
+def test_penalised_columns_of_a_beam(dtype, V, B, K, step, seed, cuda_device):
+    from fastertransformer_b200 import DynamicDecodeLayer
+    x, ids, parents = hot_columns(V, K, B, step, seed)
+    cum = -5.0 - np.random.default_rng(seed).uniform(0, 1, size=B * K).astype(np.float32)
+    words, scores = expected(torch.from_numpy(x.copy()), cum, K, ids, parents, step, 1.25, np.zeros(B * K, bool), 2)
+    assert np.abs(np.diff(scores, axis=1)).min() > 1e-3  # (nothing that rounding could turn round)
+    ints = dict(dtype=torch.int32, device=cuda_device)
+    st = {"output_ids": torch.from_numpy(ids).to(cuda_device), "parent_ids": torch.from_numpy(parents).to(cuda_device),
+          "finished": torch.zeros(B * K, dtype=torch.bool, device=cuda_device), "sequence_length": torch.full((B * K,), step, **ints),
+          "cum_log_probs": torch.from_numpy(cum).to(cuda_device)}
+    args = {"repetition_penalty": np.asarray([1.25], np.float32)}
+    layer = DynamicDecodeLayer(V, V, dtype, cuda_device)
+    layer.setup(B, K, args)
+    layer.forward(st, dict(args, logits=torch.from_numpy(x).to(device=cuda_device, dtype=dtype), step=step, max_input_length=1, ite=0,
+                           local_batch_size=B, end_id=torch.full((B,), 2, **ints), input_lengths=torch.full((B, K), 1, **ints)))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(st["parent_ids"][step].cpu().numpy() * V + st["output_ids"][step].cpu().numpy(), words)
+    np.testing.assert_allclose(st["cum_log_probs"].view(B, K).cpu().numpy(), scores, rtol=2e-5, atol=2e-5)
