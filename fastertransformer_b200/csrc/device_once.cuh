@@ -28,4 +28,19 @@ inline cudaError_t opt_in_smem(F kernel, size_t bytes, std::atomic<bool> (&done)
     return f;
 }
 
+// The same for a kernel whose need moves with the call: the attribute is only ever raised, because another thread may stand
+// between its look at the occupancy and its launch.  `highest` belongs to the kernel and the current device; under a lock.
+template<class F>
+inline cudaError_t raise_smem(F kernel, size_t bytes, size_t& highest)
+{
+    if (bytes <= highest) {
+        return cudaSuccess;
+    }
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) {
+        highest = bytes;
+    }
+    return e;
+}
+
 }  // namespace ftb200

@@ -2337,23 +2337,21 @@ template<int DT, bool TOPP, int VP = 0>
 int fast_sampling_occupancy(size_t smem, int* per_sm)
 {
     // per device: the opt-in to the shared-memory size (a per-device attribute of the kernel) and the answer
-    constexpr int     kMaxDev = 64;
     static std::mutex mu;
-    static size_t     set_smem[kMaxDev];
-    static int        val[kMaxDev];
+    static size_t     highest[kDevicesKnown], asked[kDevicesKnown];
+    static int        val[kDevicesKnown];
     int               dev = 0;
     FTB_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev) {
+    if (dev < 0 || dev >= kDevicesKnown) {
         set_error("ftb200_decode_step_sampling: device ordinal out of range");
         return FTB200_UNSUPPORTED;
     }
     std::lock_guard<std::mutex> lock(mu);
-    if (set_smem[dev] != smem) {
-        FTB_CUDA_CHECK(cudaFuncSetAttribute(fast_sampling_kernel<DT, TOPP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
+    if (asked[dev] != smem) {
+        FTB_CUDA_CHECK(raise_smem(fast_sampling_kernel<DT, TOPP, VP>, smem, highest[dev]));
         FTB_CUDA_CHECK(
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&val[dev], fast_sampling_kernel<DT, TOPP, VP>, kThreads, smem));
-        set_smem[dev] = smem;
+        asked[dev] = smem;
     }
     *per_sm = val[dev];
     return FTB200_OK;

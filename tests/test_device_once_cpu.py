@@ -1,5 +1,6 @@
 """The opt-in to large shared memory (csrc/device_once.cuh) against a fake of the two runtime calls: once per device and
-kernel, again after a failure, and on every call - not refused - for device ordinals beyond the table."""
+kernel, again after a failure, and on every call - not refused - for device ordinals beyond the table.  A limit that
+follows the calls is only ever raised: a thread that has looked at the occupancy still has its launch before it."""
 import os
 import subprocess
 
@@ -30,6 +31,14 @@ int main()
     if (sets(63, 0, 1) || sets(63, 0, 0)) return 2;
     if (sets(64, 0, 1) || sets(64, 0, 1)) return 3; // beyond the table: every time
     if (sets(7, 2, 1) || sets(7, 0, 1) || sets(7, 0, 0)) return 4;  // a failure is reported and not remembered
+    // a larger need raises the limit, a smaller one after it does not lower it, a failure is not remembered
+    size_t highest = 0;
+    auto   raise   = [&](size_t bytes, int fail, int want) {
+        g_fail = fail, g_sets = 0;
+        return ftb200::raise_smem(kernel, bytes, highest) == fail && g_sets == want ? 0 : 1;
+    };
+    if (raise(60000, 0, 1) || raise(68000, 0, 1) || raise(60000, 0, 0) || raise(68000, 0, 0)) return 5;
+    if (raise(90000, 1, 1) || raise(80000, 0, 1) || raise(90000, 0, 1) || highest != 90000) return 6;
     return 0;
 }
 """

@@ -11,10 +11,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _decode(seed, device, stream, steps, out, key):
+def _decode(seed, device, stream, steps, out, key, batch=48, vocab=32768):
     from fastertransformer_b200 import DynamicDecodeLayer
     from fastertransformer_b200.workloads import make_workload
-    w = make_workload("c3", batch=48, steps=steps, vocab=32768, seed=seed)
+    w = make_workload("c3", batch=batch, steps=steps, vocab=vocab, seed=seed)
     with torch.cuda.stream(stream):
         layer = DynamicDecodeLayer(w.vocab, w.vocab_padded, w.dtype, device)
         layer.stream = stream
@@ -42,4 +42,22 @@ def test_two_threads_one_device(cuda_device):
         t.join(timeout=300)
     assert set(together) == {0, 1}
     for i in (0, 1):
+        assert np.array_equal(alone[i], together[i]), "thread %d differs from its run alone" % i
+
+
+def test_two_threads_with_different_vocabularies(cuda_device):
+    """Batches of the single-pass kernels (more columns than the split kernel takes) whose needs of shared memory differ: a
+    launch of one thread must not find the limit that the other one's smaller call set."""
+    steps, shapes = 12, {0: (600, 32768), 1: (300, 100352)}
+    alone, together = {}, {}
+    for i, (batch, vocab) in shapes.items():
+        _decode(21 + i, cuda_device, torch.cuda.Stream(device=cuda_device), steps, alone, i, batch, vocab)
+    threads = [threading.Thread(target=_decode, args=(21 + i, cuda_device, torch.cuda.Stream(device=cuda_device), steps, together,
+                                                      i, batch, vocab)) for i, (batch, vocab) in shapes.items()]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=300)
+    assert set(together) == {0, 1}
+    for i in shapes:
         assert np.array_equal(alone[i], together[i]), "thread %d differs from its run alone" % i
