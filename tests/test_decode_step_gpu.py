@@ -1,0 +1,135 @@
+"""ftb200_decode_step, the whole step in one call, where its parts can come apart: a batch in slices under a length limit (the
+criteria count the whole batch, a slice's kernel serves its own rows), in each of the forms a step can take - the kernel
+that does the criteria itself, the split kernel with a second launch, the single-pass kernels - and a deadline that runs
+out while the stream is held by a sleeping host function (nothing on the GPU waits)."""
+import ctypes as C
+import time
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
+MIL = 8
+
+
+def build(dtype, V, B, device, stop_words, limits):
+    rng = np.random.default_rng(V + B)
+    from fastertransformer_b200 import DynamicDecodeLayer
+    layer = DynamicDecodeLayer(V, V, dtype, device)
+    layer.setup(B, 1, {"runtime_top_k": rng.choice(np.asarray([0, 1, 30], np.uint32), size=B),
+                       "runtime_top_p": np.asarray([0.8], np.float32), "random_seed": np.arange(B).astype(np.uint64)})
+    st = {"output_ids": torch.ones(MIL + 8, B, dtype=torch.int32, device=device),
+          "finished": torch.zeros(B, dtype=torch.bool, device=device),
+          "sequence_length": torch.full((B,), MIL, dtype=torch.int32, device=device)}
+    inputs = {"max_input_length": MIL, "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=device),
+              "sequence_limit_length": torch.from_numpy(limits).to(device)}
+    if stop_words:
+        # [1] for every third row (its history), [0] - a token nobody draws here - for the others
+        words = np.zeros((B, 2, 1), np.int32)
+        words[::3, 0], words[:, 1] = 5, 1
+        inputs["stop_words_list"] = torch.from_numpy(words).to(device)
+    return layer, st, inputs
+
+
+def logits(dtype, V, B, step, device):
+    g = torch.Generator(device=device)
+    g.manual_seed(step)
+    x = torch.randn(B, V, generator=g, device=device) * 2
+    x[:, 5] += 14.0 * (torch.arange(B, device=device) % 2 == step % 2)  # a row draws token 5 in every other step
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("stop_words", [False, True])
+@pytest.mark.parametrize("dtype,V,B,slices", [(F32, 5003, 12, 3), (F16, 32000, 15, 5), (F32, 32000, 300, 3), (BF16, 32768, 1040, 2),
+                                              (F32, 600, 9, 3)])
+def test_slices_under_a_length_limit(dtype, V, B, slices, stop_words, cuda_device):
+    limits = (MIL + 1 + np.arange(B) % 4).astype(np.int32)  # the last rows end in the fifth step
+    limits[0] = MIL + 4
+    n = B // slices
+    got = []
+    for whole_step in (True, False):
+        layer, st, inputs = build(dtype, V, B, cuda_device, stop_words, limits)
+        layer.time_kernels = not whole_step  # (then sampling, criteria and wait are calls of their own)
+        stops = []
+        for s in range(5):
+            x = logits(dtype, V, B, MIL + s, cuda_device)
+            for i in range(slices):
+                stop = layer.forward(st, dict(inputs, logits=x, step=MIL + s, ite=i, local_batch_size=n))
+                # what the host was told is what the flags say
+                assert stop == bool(st["finished"].all()), (whole_step, s, i)
+                stops.append(stop)
+        got.append({k: v.cpu() for k, v in st.items()} | {"stops": torch.tensor(stops), "curand": layer.topk.curand.cpu()})
+    for k in got[0]:
+        assert torch.equal(got[0][k], got[1][k]), k
+    assert got[0]["stops"].tolist()[:slices] == [False] * slices and got[0]["stops"][-1]
+
+
+@pytest.mark.parametrize("dtype,V,B", [(F32, 5003, 6), (F32, 32000, 300), (BF16, 32768, 520)])
+def test_deadline_runs_out(dtype, V, B, cuda_device):
+    from fastertransformer_b200 import lib
+    rt = C.CDLL("libcudart.so.12")
+    HOSTFN = C.CFUNCTYPE(None, C.c_void_p)
+    hold = HOSTFN(lambda _: time.sleep(0.3))
+    rt.cudaLaunchHostFunc.argtypes = [C.c_void_p, HOSTFN, C.c_void_p]
+    limits = np.full(B, MIL + 3, np.int32)
+    xs = [logits(dtype, V, B, MIL + s, cuda_device) for s in range(4)]
+    got = []
+    for late in (False, True):
+        layer, st, inputs = build(dtype, V, B, cuda_device, False, limits)
+        stream = torch.cuda.Stream(device=cuda_device)
+        stops = []
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            for s in range(4):
+                if late and s == 1:
+                    # the block of the step before, moved on by hand, for a deadline of its own
+                    P, stop = layer._gate[0, B]["params"], C.c_int(-7)
+                    P.step, P.logits = MIL + s, xs[s].data_ptr()
+                    assert rt.cudaLaunchHostFunc(C.c_void_p(stream.cuda_stream), hold, None) == 0
+                    assert lib.ftb200_decode_step(layer._gate[0, B]["params_ref"], layer._stop_ref, 20, C.byref(stop)) == 6
+                    assert stop.value == 0 and b"deadline" in lib.ftb200_last_error_string()
+                    stream.synchronize()  # the step itself was launched and ends
+                    stops.append(bool(st["finished"].all()))
+                    continue
+                stops.append(layer.forward(st, dict(inputs, logits=xs[s], step=MIL + s)))
+        torch.cuda.synchronize()
+        assert stops == [False, False, False, True]
+        got.append({k: v.cpu() for k, v in st.items()} | {"curand": layer.topk.curand.cpu()})
+    for k in got[0]:
+        assert torch.equal(got[0][k], got[1][k]), k
+
+
+@pytest.mark.parametrize("dtype,kind,V,B", [(F16, "topp", 41000, 37), (BF16, "topk", 128256, 18), (F32, "topk", 32000, 74),
+                                            (F16, "topp", 32000, 120)])
+def test_step_under_capture(dtype, kind, V, B, cuda_device):
+    """A step whose size the library has not met before, recorded in a graph: the dispatch asks for occupancies then."""
+    from fastertransformer_b200 import DynamicDecodeLayer
+
+    def run(columns, capture):
+        layer = DynamicDecodeLayer(columns, columns, dtype, cuda_device)
+        layer.setup(B, 1, {"runtime_top_k": np.asarray([40], np.uint32)} if kind == "topk" else
+                    {"runtime_top_p": np.asarray([0.9], np.float32)})
+        st = {"output_ids": torch.ones(MIL + 2, B, dtype=torch.int32, device=cuda_device),
+              "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+              "sequence_length": torch.full((B,), MIL, dtype=torch.int32, device=cuda_device)}
+        inputs = {"max_input_length": MIL, "step": MIL, "logits": logits(dtype, columns, B, 3, cuda_device),
+                  "end_id": torch.full((B,), columns - 1, dtype=torch.int32, device=cuda_device)}
+        torch.cuda.synchronize()
+        if capture:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                layer.forward(st, inputs)
+            assert int(st["output_ids"][MIL, 0]) == 1  # (recorded, not run)
+            graph.replay()
+        else:
+            layer.forward(st, inputs)
+        torch.cuda.synchronize()
+        return st["output_ids"][MIL].cpu(), layer.topk.curand.cpu(), layer.topp.curand.cpu()
+
+    run(V + 1024, False)  # (the kernels are loaded; the size of the recorded step is a new one)
+    recorded, direct = run(V, True), run(V, False)
+    for a, b in zip(recorded, direct):
+        assert torch.equal(a, b)
