@@ -4,6 +4,7 @@
 #include <mutex>
 
 #include "sampling_params.cuh"
+#include "spans.cuh"
 #include "split_args.cuh"
 #include "vp_args.cuh"
 
@@ -138,7 +139,8 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     // more than its columns (1024 x 32000 fp32, k = 50: 445 us with eight, 184 us with two).  With both kinds of rows the
     // costliest are started first and a last few that wait for a place are short: there the SMs are counted alone.
     const auto most_rows = [&](int lg) { return mixed ? 2 * sms >> lg : resident_clusters(p->dtype, lg, false, kTwoPerSm); };
-    int        lgn       = vocab > 65536 || rows <= most_rows(3) ? 3 : (vocab > 40960 || rows <= most_rows(2) ? 2 : 1);
+    const bool few       = rows * 16 <= sms;  // (no group of SMs is so small: resident, without a question)
+    int        lgn       = vocab > 65536 || few || rows <= most_rows(3) ? 3 : (vocab > 40960 || rows <= most_rows(2) ? 2 : 1);
     for (; lgn <= 3; ++lgn) {
         A->slice = ((vocab + 1023) / 1024) << (10 - lgn);
         A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
@@ -174,7 +176,7 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     const auto keeps = [&](int per_sm, size_t budget) {
         A->area           = area_within(budget, kSpAreaMax);
         const size_t smem = split_smem_bytes(A->slice, A->area);
-        return mixed ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, smem > smem_general ? smem : smem_general);
+        return mixed || few ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, smem > smem_general ? smem : smem_general);
     };
     *whole = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kWholeTwoPerSm && smem_general <= kWholeTwoPerSm && keeps(2, kWholeTwoPerSm)));
     if (!*whole) {
@@ -332,6 +334,7 @@ static int plan_sampling(const ftb200_sampling_params* p, KParams& K, size_t& sm
     K.finished         = p->finished;
     K.cum_log_probs    = p->cum_log_probs;
     K.out_log_probs    = p->output_log_probs;
+    K.whole_words      = whole_words(p->local_batch_size, (size_t)p->topk_skip, (size_t)p->topp_skip, (size_t)p->finished);
     K.row_order        = p->row_order;
     K.trace            = g_row_trace;
 

@@ -67,6 +67,7 @@ struct KParams {
     u64*     scratch;         // per-CTA candidate overflow area
     size_t   scratch_stride;  // u64 entries per CTA
     int      hash_slots, hash_shift, flag_words;
+    int      whole_words;     // the words around the rows' skip and finished flags may be read whole (see spans.cuh)
 };
 
 }  // namespace ftb200

@@ -88,7 +88,7 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
             auto      word = [&](int slot, const void* p) { cp_async4(args + 4u * (u32)slot, p); };
             auto      byte = [&](int slot, const uint8_t* p) {
                 if (p != nullptr) {
-                    cp_async_byte(args + 4u * (u32)slot, p, rows, r);
+                    cp_async_byte(args + 4u * (u32)slot, p, r, P.whole_words != 0);
                 }
             };
             byte(kSkipK, P.topk_skip);

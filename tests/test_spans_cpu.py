@@ -40,12 +40,13 @@ int main()
     }
     for (size_t a = 0x2000; a < 0x2004; ++a) {
         for (int n = 1; n < 20; ++n) {
+            bool inside = true;
             for (int at = 0; at < n; ++at) {
-                const WordSpan W = word_span(a, n, at);
-                if ((a + W.from) % 4 != 0 || W.from > at || W.from + 4 <= at) return 8;
-                if (W.bytes == 0 ? W.from >= 0 : W.from < 0 || W.from + W.bytes > n || W.from + W.bytes <= at) return 9;
-                ++checked;
+                const size_t word = (a + at) & ~(size_t)3;
+                inside            = inside && word >= a && word + 4 <= a + n;
             }
+            if (whole_words(n, a, 0, 0) != inside || whole_words(n, 0, a, 0) != inside || whole_words(n, 0, 0x3000, a) != inside) return 8;
+            ++checked;
         }
     }
     std::printf("%ld\n", checked);
@@ -58,4 +59,4 @@ def test_copies_stay_inside_their_arrays(tmp_path):
     src, exe = tmp_path / "spans.cc", tmp_path / "spans"
     src.write_text(MAIN)
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "fastertransformer_b200", "csrc"), str(src), "-o", str(exe)])
-    assert int(subprocess.check_output([str(exe)])) > 3000
+    assert int(subprocess.check_output([str(exe)])) > 1500
