@@ -12,7 +12,20 @@ import torch
 
 from ._lib import BeamHyps, BeamParams, SamplingParams, SetupParams, StopParams, check, lib
 
+# Page-locked words that a step which missed its deadline has still to write, with an event behind that step: the host
+# allocator would hand them out again when their layer goes.
+_LATE = []
+
+
+def _keep_until_done(word, stream):
+    """Holds on to `word` until what is on `stream` now has run."""
+    done = torch.cuda.Event()
+    done.record(stream)
+    _LATE[:] = [(w, e) for w, e in _LATE if not e.query()] + [(word, done)]
+
+
 _DT = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
+TIMEOUT = 6  # FTB200_TIMEOUT
 CURAND_STATE_BYTES = 48  # sizeof(curandState_t), XORWOW
 
 
@@ -89,6 +102,7 @@ class DynamicDecodeLayer:
         self._gate = {}
         self.time_kernels = False   # when set, CUDA events bracket each fused launch (kernel_events)
         self.kernel_events = []
+        self.deadline_ms = 10000    # of the wait for should_stop
         self._count_dev = None
         self._count_host = None
         self._stop = None
@@ -104,6 +118,9 @@ class DynamicDecodeLayer:
         if _raw_stream is not None:
             return _raw_stream(self._device_index)
         return torch.cuda.current_stream(self.device).cuda_stream
+
+    def _run_stream(self):
+        return self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
 
     # Device memory of the layer, by attribute.  The caching allocator hands a freed block out again on the stream it was
     # allocated on, without a look at the others: a call on another stream has to be noted on each of them.
@@ -125,7 +142,7 @@ class DynamicDecodeLayer:
 
     def _away(self):
         """Before a call on another stream than the one all of the layer's memory was allocated on."""
-        here = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
+        here = self._run_stream()
         for t in self._memory():
             t.record_stream(here)
 
@@ -254,7 +271,7 @@ class DynamicDecodeLayer:
         check(lib.ftb200_setup_sampling(C.byref(S)))
         # The arguments, the launch order and the generators are there when this returns: steps may follow on any stream,
         # from any thread, under capture.  (An event would do for the first of these only; a request waits 10 us here once.)
-        (self.stream if self.stream is not None else torch.cuda.current_stream(dev)).synchronize()
+        self._run_stream().synchronize()
 
     # ---- forward (DynamicDecodeLayer.cc:191-474, sampling branch) ---------------------------------
     def forward(self, outputs, inputs):
@@ -306,8 +323,10 @@ class DynamicDecodeLayer:
             L = sw.shape[-1]
             S.stop_words, S.stop_words_len = sw.data_ptr() + lo * 2 * L * 4, L
         S.sequence_limit_length = None if lim is None else lim.data_ptr()
-        rc = lib.ftb200_decode_step(g["params_ref"], self._stop_ref, 10000, self._should_stop_ref)
+        rc = lib.ftb200_decode_step(g["params_ref"], self._stop_ref, self.deadline_ms, self._should_stop_ref)
         if rc:
+            if rc == TIMEOUT:
+                _keep_until_done(self._result, self._run_stream())
             check(rc)
         self.launches += lib.ftb200_last_launch_count()
         return bool(self._should_stop.value)
@@ -440,7 +459,11 @@ class DynamicDecodeLayer:
         if lim is None:
             return False
         stop = C.c_int(0)
-        check(lib.ftb200_wait_should_stop(C.c_void_p(self._count_host.data_ptr()), B, beam, st, 10000, C.byref(stop)))
+        rc = lib.ftb200_wait_should_stop(C.c_void_p(self._count_host.data_ptr()), B, beam, st, self.deadline_ms, C.byref(stop))
+        if rc:
+            if rc == TIMEOUT:
+                _keep_until_done(self._count_host, self._run_stream())
+            check(rc)
         return bool(stop.value)
 
     def _fill(self, outputs, inputs, logits, B, step, ite, lbs, mil, lo):

@@ -3,6 +3,7 @@ criteria count the whole batch, a slice's kernel serves its own rows), in each o
 that does the criteria itself, the split kernel with a second launch, the single-pass kernels - and a deadline that runs
 out while the stream is held by a sleeping host function (nothing on the GPU waits)."""
 import ctypes as C
+import gc
 import time
 
 import numpy as np
@@ -100,6 +101,35 @@ def test_deadline_runs_out(dtype, V, B, cuda_device):
         got.append({k: v.cpu() for k, v in st.items()} | {"curand": layer.topk.curand.cpu()})
     for k in got[0]:
         assert torch.equal(got[0][k], got[1][k]), k
+
+
+@pytest.mark.parametrize("one_call", [True, False])
+def test_word_of_a_late_step_is_kept(one_call, cuda_device):
+    """A layer that is dropped after its step missed the deadline: the step still writes its page-locked word, which must
+    not have become somebody else's by then."""
+    from fastertransformer_b200._lib import FtbError
+    rt = C.CDLL("libcudart.so.12")
+    HOSTFN = C.CFUNCTYPE(None, C.c_void_p)
+    hold = HOSTFN(lambda _: time.sleep(0.3))
+    rt.cudaLaunchHostFunc.argtypes = [C.c_void_p, HOSTFN, C.c_void_p]
+    layer, st, inputs = build(F32, 5003, 6, cuda_device, False, np.full(6, MIL + 9, np.int32))
+    layer.time_kernels = not one_call
+    x = logits(F32, 5003, 6, 0, cuda_device)
+    layer.forward(st, dict(inputs, logits=x, step=MIL))
+    layer.deadline_ms = 20
+    word = (layer._result if one_call else layer._count_host).data_ptr()
+    stream = torch.cuda.Stream(device=cuda_device)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        assert rt.cudaLaunchHostFunc(C.c_void_p(stream.cuda_stream), hold, None) == 0
+        with pytest.raises(FtbError, match="deadline"):
+            layer.forward(st, dict(inputs, logits=x, step=MIL + 1))
+        del layer
+        gc.collect()
+        others = [torch.zeros(n, dtype=torch.int64).pin_memory() for n in (1, 1, 1, 1, 8, 64)]
+        assert not stream.query() and word not in [t.data_ptr() for t in others]
+    stream.synchronize()
+    assert all(int(t.abs().sum()) == 0 for t in others)
 
 
 @pytest.mark.parametrize("dtype,kind,V,B", [(F16, "topp", 41000, 37), (BF16, "topk", 128256, 18), (F32, "topk", 32000, 74),
