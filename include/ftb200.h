@@ -79,7 +79,7 @@ int ftb200_setup_topp_runtime_args(int batch, uint32_t top_k, uint32_t* top_ks, 
 /* The set-up of both layers in one launch: what ftb200_curand_init does for each layer's states and the two functions
  * above for their arguments (same meaning; topk_top_k is the largest and topp_top_k the first of the caller's values,
  * TopKSamplingLayer.cu:160-170, TopPSamplingLayer.cu:215-224).  topp_ps == null: no top-p layer; its states are
- * initialised all the same. */
+ * initialised all the same.  Asynchronous on `stream`: a step on another stream has to be ordered after it. */
 typedef struct ftb200_setup_params {
     int                       batch;
     void*                     topk_states;
@@ -262,7 +262,7 @@ int ftb200_wait_should_stop(const int* finished_count_host, int batch_size, int 
  *   result_host   one 64-bit word of page-locked host memory the device can reach (cudaHostAlloc, cudaHostRegister)
  *   sequence      counts the calls on this block (in/out); the word holds sequence << 32 | finished rows afterwards
  * A block serves one call at a time.  *should_stop = 1 when all batch_size rows are finished; FTB200_TIMEOUT after
- * timeout_ms (negative: no deadline).
+ * timeout_ms (negative: no deadline): the step is then still on its way and writes *result_host when it ends.
  * ------------------------------------------------------------------------------------------ */
 typedef struct ftb200_stop_params {
     const int*      stop_words;
@@ -367,6 +367,8 @@ typedef struct ftb200_beam_params {
 } ftb200_beam_params;
 
 int ftb200_beam_workspace_bytes(int local_batch_size, int beam_width, size_t* bytes);
+/* With a penalty on a vocabulary of more than 983040 columns (fp32) or 1245184 (16 bits), step <= 26000; beyond that
+ * FTB200_UNSUPPORTED. */
 int ftb200_beam_search_step(const ftb200_beam_params* p);
 
 /* ------------------------------------------------------------------------------------------
