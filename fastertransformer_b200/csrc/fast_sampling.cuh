@@ -75,18 +75,6 @@ __device__ __forceinline__ void cp_async4(u32 saddr, const void* g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(g) : "memory");
 }
-// The aligned word around byte `at` of an array on its way to `saddr`; `whole`: it may be read whole, else the byte comes by
-// itself, in its place (the arithmetic of a copy of the word's part inside the array, inlined at every stage of a row's
-// header, cost the mixed batch of 1024 x 128256 1 %: 204.4 us a step, this form 202.5).
-__device__ __forceinline__ void cp_async_byte(u32 saddr, const uint8_t* array, int at, bool whole)
-{
-    if (whole) {
-        cp_async4(saddr, (const void*)((size_t)(array + at) & ~(size_t)3));
-    }
-    else {
-        sts_u32(saddr, (u32)array[at] << (8 * ((size_t)(array + at) & 3)));
-    }
-}
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -459,7 +447,6 @@ static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
 {
     const u32 base = (u32)__cvta_generic_to_shared(pre);
     auto word = [&](int slot, const void* p) { cp_async4(base + 4u * (u32)slot, p); };
-    auto byte = [&](int slot, const uint8_t* p) { cp_async_byte(base + 4u * (u32)slot, p, nr, P.whole_words != 0); };
     if (P.topk_states != nullptr) {
         const char* st = (const char*)(P.topk_states + nr);
         cp_async16(base + 4u * kPreStateK, st);
@@ -467,9 +454,6 @@ static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
         cp_async16(base + 4u * kPreStateK + 32u, st + 32);
         word(kPreK, P.topk_ks + nr);
         word(kPrePk, P.topk_ps + nr);
-        if (P.topk_skip != nullptr) {
-            byte(kPreSkipK, P.topk_skip);
-        }
     }
     if (P.topp_states != nullptr) {
         const char* st = (const char*)(P.topp_states + nr);
@@ -477,12 +461,26 @@ static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
         cp_async16(base + 4u * kPreStateP + 16u, st + 16);
         cp_async16(base + 4u * kPreStateP + 32u, st + 32);
         word(kPrePp, P.topp_ps + nr);
-        if (P.topp_skip != nullptr) {
-            byte(kPreSkipP, P.topp_skip);
-        }
     }
-    if (P.finished != nullptr) {
-        byte(kPreFin, P.finished);
+    // The flags are bytes: the words around them where those may be read whole, else the bytes, loaded together and put in
+    // their places.  (A copy of a word's part inside its array, worked out here, where this is inlined at every stage of a
+    // header, cost the mixed batch of 1024 x 128256 1 %: 204.4 us a step, this form 202.5.)
+    const uint8_t *fk = P.topk_states != nullptr ? P.topk_skip : nullptr, *fp = P.topp_states != nullptr ? P.topp_skip : nullptr;
+    if (P.whole_words) {
+        auto around = [&](int slot, const uint8_t* p) {
+            if (p != nullptr) {
+                word(slot, (const void*)((size_t)(p + nr) & ~(size_t)3));
+            }
+        };
+        around(kPreSkipK, fk);
+        around(kPreSkipP, fp);
+        around(kPreFin, P.finished);
+    }
+    else {
+        const u32 a = fk != nullptr ? fk[nr] : 0u, b = fp != nullptr ? fp[nr] : 0u, c = P.finished != nullptr ? P.finished[nr] : 0u;
+        pre[kPreSkipK] = a << (8 * ((size_t)(fk + nr) & 3));
+        pre[kPreSkipP] = b << (8 * ((size_t)(fp + nr) & 3));
+        pre[kPreFin]   = c << (8 * ((size_t)(P.finished + nr) & 3));
     }
     word(kPreEnd, P.end_ids + nr);
     if (P.apply_temp) {

@@ -43,6 +43,19 @@ FTB_HD VecRange whole_vectors(int rows, int stride, int r, int mis, int nv)
     return V;
 }
 
+// The aligned 32-bit word around byte `at` of an array of n bytes: it starts at byte `from`, and `bytes` of it, counted from
+// there, may be read; none where the array starts inside the word (that byte is then loaded by itself).
+struct WordSpan {
+    int from, bytes;
+};
+FTB_HD WordSpan word_span(size_t array, int n, int at)
+{
+    WordSpan W;
+    W.from  = at - (int)((array + (size_t)at) & 3);
+    W.bytes = W.from < 0 ? 0 : (n - W.from < 4 ? n - W.from : 4);
+    return W;
+}
+
 // Whether the aligned 32-bit words around the entries of arrays of n bytes lie inside their arrays (null: no array).
 FTB_HD bool whole_words(int n, size_t a, size_t b, size_t c)
 {

@@ -87,8 +87,18 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
             const u32 args = (u32)__cvta_generic_to_shared(s_args);
             auto      word = [&](int slot, const void* p) { cp_async4(args + 4u * (u32)slot, p); };
             auto      byte = [&](int slot, const uint8_t* p) {
-                if (p != nullptr) {
-                    cp_async_byte(args + 4u * (u32)slot, p, r, P.whole_words != 0);
+                if (p == nullptr) {
+                    return;
+                }
+                // (asynchronous whatever the alignment: a load that is waited for here cost rows of 12000 columns 4 %)
+                const WordSpan W = word_span((size_t)p, rows, r);
+                if (W.bytes != 0) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(args + 4u * (u32)slot), "l"(p + W.from),
+                                 "r"(W.bytes)
+                                 : "memory");
+                }
+                else {
+                    sts_u32(args + 4u * (u32)slot, (u32)p[r] << (8 * (r - W.from)));
                 }
             };
             byte(kSkipK, P.topk_skip);

@@ -44,6 +44,9 @@ int main()
             for (int at = 0; at < n; ++at) {
                 const size_t word = (a + at) & ~(size_t)3;
                 inside            = inside && word >= a && word + 4 <= a + n;
+                const WordSpan W  = word_span(a, n, at);
+                if ((a + W.from) % 4 != 0 || W.from > at || W.from + 4 <= at) return 9;
+                if (W.bytes == 0 ? W.from >= 0 : W.from < 0 || W.from + W.bytes > n || W.from + W.bytes <= at) return 10;
             }
             if (whole_words(n, a, 0, 0) != inside || whole_words(n, 0, a, 0) != inside || whole_words(n, 0, 0x3000, a) != inside) return 8;
             ++checked;
