@@ -1195,7 +1195,7 @@ __device__ __noinline__ void build_row(const KParams& P, const Smem& S, RowCtx& 
     if (has_word && item_end >= 0) {
         const int item_size = item_end - item_start;
         ban                 = item_size == 1;
-        ban_tok             = wbase[item_end - 1];
+        ban_tok             = item_end > 0 ? wbase[item_end - 1] : 0;  // (an empty word stands in front of the list)
         if (item_size > 1 && P.step >= item_size - 1) {
             ban = true;
             if (item_size <= 4) {

@@ -297,7 +297,7 @@ __device__ __noinline__ void sp_mark_specials(const KParams& P, int r, u32 bits_
                 continue;
             }
             const int start = i > 0 ? wbase[L + i - 1] : 0, size = end - start;
-            const int tok   = wbase[end - 1];
+            const int tok   = end > 0 ? wbase[end - 1] : 0;  // (an empty word stands in front of the list)
             bool      ban   = size == 1;
             if (size > 1 && P.step >= size - 1) {
                 ban = true;

@@ -143,3 +143,28 @@ def test_calls_of_one_kind_around_the_resident_clusters(kind, dtype, V, B, cuda_
         np.testing.assert_array_equal(got[k], v, err_msg=k)
     if kind == "topk" and V == 128256 and B == 18 and torch.cuda.get_device_properties(0).multi_processor_count <= 148:
         assert launches > 1  # eighteen clusters of eight CTAs are not resident with one CTA on an SM
+
+
+@pytest.mark.parametrize("general", [True, False])
+def test_empty_word_in_front_of_a_list(general, cuda_device):
+    """A word list whose first word is empty (its end offset is 0): nothing in front of the list is a token of it."""
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    B, V = 5, 6000
+    # tokens 4000 and 4001 in front of the list, 7 and 11 in it
+    buf = torch.tensor([4000, 4001, 7, 11, 0, 0, 0, 1, 2, -1], dtype=torch.int32, device=cuda_device)
+    words = buf[2:].view(2, 4)
+    x = torch.zeros(B, V, device=cuda_device)
+    x[:, 7], x[:, 11], x[:, 4001], x[:, 4000] = 9.0, 8.0, 7.0, 6.0
+    layer = DynamicDecodeLayer(V, V, F32, cuda_device)
+    layer.setup(B, 1, {"runtime_top_k": np.asarray([1], np.uint32)})
+    st = {"output_ids": torch.ones(4, B, dtype=torch.int32, device=cuda_device),
+          "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+          "sequence_length": torch.full((B,), 2, dtype=torch.int32, device=cuda_device)}
+    lib.ftb200_set_single_pass(0 if general else 1)
+    try:
+        layer.forward(st, {"logits": x, "step": 2, "max_input_length": 2, "bad_words_list": words,
+                           "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)})
+        torch.cuda.synchronize()
+    finally:
+        lib.ftb200_set_single_pass(1)
+    assert st["output_ids"][2].tolist() == [4001] * B
