@@ -126,25 +126,27 @@ class DynamicDecodeLayer:
     # allocated on, without a look at the others: a call on another stream has to be noted on each of them.
     _MEMORY = ("_setup_mem", "_workspace", "_beam_ws", "_arrived", "_count_dev")
 
-    def _allocated(self, make):
-        """What `make` allocates, on the layer's own stream if it has one, else on the current one."""
+    def _allocated(self, make, *args, **kw):
+        """What make(...) allocates, on the layer's own stream if it has one, else on the current one."""
         if self.device.type != "cuda":
-            return make()
+            return make(*args, **kw)
         if self.stream is None:
-            t = make()
+            t = make(*args, **kw)
         else:
             with torch.cuda.stream(self.stream):
-                t = make()
+                t = make(*args, **kw)
         on = self._raw_stream()
-        # (several streams: none of them is the home of all)
-        self._home = on if self._home is None or self._home == on else -1
+        if self._home != on:
+            self._home = on if self._home is None else -1  # (several streams: none of them is the home of all)
         return t
 
     def _away(self):
         """Before a call on another stream than the one all of the layer's memory was allocated on."""
-        here = self._run_stream()
-        for t in self._memory():
-            t.record_stream(here)
+        memory = self._memory()
+        if memory:
+            here = self._run_stream()
+            for t in memory:
+                t.record_stream(here)
 
     def _memory(self):
         mem = [getattr(self, name) for name in self._MEMORY] + [g["order"] for g in self._gate.values()]
@@ -248,7 +250,7 @@ class DynamicDecodeLayer:
             for name, dtype in (("initial", torch.float32), ("decay", torch.float32), ("min", torch.float32),
                                 ("reset", torch.int32)):
                 pack.add(self.topp, name, dtype, B)
-        self._setup_mem = self._allocated(lambda: pack.place(dev))
+        self._setup_mem = self._allocated(pack.place, dev)
         tk, tp = self.topk, self.topp
         S = SetupParams()
         S.batch = B
@@ -311,7 +313,7 @@ class DynamicDecodeLayer:
         # sampling, stop criteria and the wait for should_stop in one call
         S = self._stop
         if S is None:
-            self._arrived = self._allocated(lambda: torch.zeros(1, dtype=torch.int32, device=self.device))
+            self._arrived = self._allocated(torch.zeros, 1, dtype=torch.int32, device=self.device)
             self._result = torch.zeros(1, dtype=torch.int64).pin_memory()
             S = self._stop = StopParams()
             S.arrived_dev, S.result_host = self._arrived.data_ptr(), self._result.data_ptr()
@@ -389,7 +391,7 @@ class DynamicDecodeLayer:
         need = C.c_size_t(0)
         check(lib.ftb200_beam_workspace_bytes(sub, K, C.byref(need)))
         if self._beam_ws is None or self._beam_ws.numel() < need.value:
-            self._beam_ws = self._allocated(lambda: torch.empty(need.value, dtype=torch.uint8, device=self.device))
+            self._beam_ws = self._allocated(torch.empty, need.value, dtype=torch.uint8, device=self.device)
         if "repetition_penalty" in inputs and "presence_penalty" in inputs:
             raise RuntimeError("[FT][ERROR] Found ambiguous parameters repetition_penalty and "
                                "presence_penalty which are mutually exclusive.")
@@ -446,7 +448,7 @@ class DynamicDecodeLayer:
         if sw is None and lim is None:
             return False
         if self._count_dev is None:
-            self._count_dev = self._allocated(lambda: torch.zeros(1, dtype=torch.int32, device=self.device))
+            self._count_dev = self._allocated(torch.zeros, 1, dtype=torch.int32, device=self.device)
             self._count_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         L = 0 if sw is None else sw.shape[-1]
         st = C.c_void_p(self._stream)
@@ -529,7 +531,7 @@ class DynamicDecodeLayer:
                 need = C.c_size_t(0)
                 check(lib.ftb200_sampling_workspace_bytes(P.dtype, lbs, Vp, C.byref(need)))
                 if self._workspace is None or self._workspace.numel() < need.value:
-                    self._workspace = self._allocated(lambda: torch.empty(need.value, dtype=torch.uint8, device=self.device))
+                    self._workspace = self._allocated(torch.empty, need.value, dtype=torch.uint8, device=self.device)
                 self._ws_key = (P.dtype, lbs, Vp)
             P.stream = self._stream
             g["ptrs"] = ptrs

@@ -53,7 +53,7 @@ class VocabParallelSampler(DynamicDecodeLayer):
         self._need = {}          # workspace bytes by (dtype, rows, columns)
         self._records = None
         self._gathered = None
-        self._overflow = self._allocated(lambda: torch.zeros(1, dtype=torch.int32, device=self.device))
+        self._overflow = self._allocated(torch.zeros, 1, dtype=torch.int32, device=self.device)
         torch.cuda.current_stream(self.device).synchronize()  # (the count starts at zero for a call on any stream)
 
     _MEMORY = DynamicDecodeLayer._MEMORY + ("_records", "_gathered", "_overflow", "_topp_rows", "_full_rows")
@@ -113,7 +113,7 @@ class VocabParallelSampler(DynamicDecodeLayer):
             check(lib.ftb200_sampling_workspace_bytes(P.dtype, B, vocab_padded, C.byref(n)))
             need = self._need[P.dtype, B, vocab_padded] = n.value
         if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = self._allocated(lambda: torch.empty(need, dtype=torch.uint8, device=self.device))
+            self._workspace = self._allocated(torch.empty, need, dtype=torch.uint8, device=self.device)
         P.workspace, P.workspace_bytes = self._workspace.data_ptr(), self._workspace.numel()
         P.stream = stream = self._raw_stream()
         if stream != self._home:
@@ -152,8 +152,8 @@ class VocabParallelSampler(DynamicDecodeLayer):
     def _buffers(self, B):
         shape = (B, 2 + self.cap)
         if self._records is None or tuple(self._records.shape) != shape:
-            self._records = self._allocated(lambda: torch.zeros(shape, dtype=torch.int64, device=self.device))
-            self._gathered = self._allocated(lambda: torch.zeros((self.n_shards,) + shape, dtype=torch.int64, device=self.device))
+            self._records = self._allocated(torch.zeros, shape, dtype=torch.int64, device=self.device)
+            self._gathered = self._allocated(torch.zeros, (self.n_shards,) + shape, dtype=torch.int64, device=self.device)
         return self._records, self._gathered
 
     def forward_rank(self, outputs, inputs, shard_logits, rank):
@@ -203,7 +203,7 @@ class VocabParallelSampler(DynamicDecodeLayer):
         B = outputs["output_ids"].shape[-1]
         Vp = self.shard_size * self.n_shards
         if self._full_rows is None or tuple(self._full_rows.shape) != (B, Vp) or self._full_rows.dtype != parts.dtype:
-            self._full_rows = self._allocated(lambda: torch.empty(B, Vp, dtype=parts.dtype, device=self.device))
+            self._full_rows = self._allocated(torch.empty, B, Vp, dtype=parts.dtype, device=self.device)
         self._full_rows.view(B, self.n_shards, self.shard_size).index_copy_(0, self._topp_rows, parts.permute(1, 0, 2))
         P = self._params(outputs, inputs, self._full_rows, self.vocab_size, Vp, "top_p")
         check(lib.ftb200_decode_step_sampling(C.byref(P)))
