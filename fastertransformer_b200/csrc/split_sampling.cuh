@@ -12,8 +12,12 @@
 // What bounds it: latency.  A row takes six to ten cluster barriers (0.5 us each) and about six sweeps over its shared
 // memory; a CTA-per-row kernel walks eight times as many columns with the same 256 threads.  Measured on B200, one row
 // alone on its SMs: arg-max of 32000 columns 5 us, k = 50 of 50257 fp32 17 us, a nucleus of 50257 fp32 22 us (the general
-// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 10 us (k = 1) to 70 us (25000-column nucleus).  Batch
-// of 64 x 50257 fp32 top-p: 1186 -> 61 us a step; 48 x 51200 half with bias and log-probs: 920 -> 103 us.
+// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 10 us (k = 1) to 60 us (25000-column nucleus).  Batch
+// of 64 x 50257 fp32 top-p: 52 us a step (61 with the nucleus scattered by list and sorted in one unrolled pass); 48 x 51200
+// half with bias and log-probs: 67 us (83 so); 24 steps of 16 x 128256 bf16: 1707 us (1923 so).
+//
+// Code size matters: a row runs through most of this code once, so a loop that is unrolled for the largest case waits for
+// its instructions in every case.
 //
 // The results are those of sampling_kernels.cuh, bit for bit; rows that do not fit the fixed tables here (a nucleus
 // above the collection areas, thousands of equal values around the k-th) go to the general row code.
@@ -80,6 +84,10 @@ __device__ __forceinline__ void dred_min(u32 a, u32 v)
 __device__ __forceinline__ void dred_max(u32 a, u32 v)
 {
     asm volatile("red.shared::cluster.max.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void dred_add(u32 a, u32 v)
+{
+    asm volatile("red.shared::cluster.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 __device__ __forceinline__ u32 smem_addr(const void* p)
 {
@@ -153,9 +161,10 @@ struct SpShared {
     u32   best_tie;        // largest tie key of the columns that hold the maximum
     u32   n_cls;           // columns of the crossing class
     u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
-    u32   p_sel, j_sel;    // crossing: probability (bits), rank inside its class
+    u32   p_sel, j_sel;    // crossing: probability (bits), position in the sorted order
+    u32   larger;          // columns of a larger probability than the crossing's
     u32   bad_order;
-    float agg[(kSpMaxN * kSpAreaMax) / 256];
+    alignas(16) float agg[(kSpMaxN * kSpAreaMax) / 256];
 };
 
 // Bias of a 32-bit word of logits in the logits type's arithmetic (half: two rounded sums; fp32: one).  bf16 sums stay
@@ -389,6 +398,53 @@ __device__ __forceinline__ void sp_sweep(const float* y, int ny, float thr, F&& 
     }
 }
 
+// The same for the columns with values in [lo, hi]; f returns a number to add.  Returns the thread's sum and its columns above hi.
+template<class F>
+__device__ __forceinline__ u32 sp_sweep_band(const float* y, int ny, float lo, float hi, F&& f)
+{
+    FTB_ASSUME_SHARED(y);
+    constexpr int U = 4;
+    u32           sum = 0;
+    for (int i0 = 4 * (int)threadIdx.x; i0 < ny; i0 += 4 * kThreads * U) {
+        u32 in = 0;
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int    i = i0 + q * 4 * kThreads;
+            const float4 v = i < ny ? *(const float4*)(y + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            const u32    a = (v.x > hi ? 1u : 0u) | (v.y > hi ? 2u : 0u) | (v.z > hi ? 4u : 0u) | (v.w > hi ? 8u : 0u);
+            const u32    b = (v.x >= lo ? 1u : 0u) | (v.y >= lo ? 2u : 0u) | (v.z >= lo ? 4u : 0u) | (v.w >= lo ? 8u : 0u);
+            sum += __popc(a);
+            in |= (b & ~a) << (4 * q);
+        }
+        while (in != 0) {
+            const int e = __ffs(in) - 1, i = i0 + (e >> 2) * 4 * kThreads + (e & 3);
+            in &= in - 1;
+            sum += f(i, y[i]);
+        }
+    }
+    return sum;
+}
+
+// The j-th smallest of n <= 512 columns.
+static __device__ __noinline__ int sp_jth_of_few(const u32* cls, int n, int j)
+{
+    __shared__ u32 s_col;
+    FTB_ASSUME_SHARED(cls);
+    for (int i = threadIdx.x; i < n; i += kThreads) {
+        const u32 c  = cls[i];
+        int       rk = 0;
+#pragma unroll 8
+        for (int q = 0; q < n; ++q) {
+            rk += cls[q] < c ? 1 : 0;
+        }
+        if (rk == j) {
+            s_col = c;
+        }
+    }
+    __syncthreads();
+    return (int)s_col;
+}
+
 // Counts of the CTA's selectable columns per bin.
 static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float lowest, float maxv, u32 hist)
 {
@@ -414,187 +470,275 @@ static __device__ __noinline__ void sp_count_bins(const float* y, int ny, float 
     }
 }
 
-// One nucleus owner's keys (fp32 values, any order) into descending order; n <= cap - 64, cap a multiple of 1024 and at
-// most PER keys for every thread.  `excl` holds the first position of every bin in the row's order, `place` is scratch for one word per bin.  A key's place inside its bin is
-// guessed from its position between the bin's edges, so that a sub-bucket of four places receives four keys on average
-// whatever the distribution is; a bin of eight keys or more shares no sub-bucket with its neighbours (two runs of equal
-// 16-bit values in one sub-bucket would take quadratic time).  Sub-buckets that come out unsorted are finished by one
-// thread each.  Returns false when a long sub-bucket would have to be ordered.
-template<int PER>
-static __device__ __forceinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* place, u32 start, int n, float maxv,
-                                                    int cap)
+// Columns of the nucleus (bins 0 .. b_thr) to their owners: `cursor` [kSpBins] holds, per bin, the cluster address of the next
+// place of this CTA's keys.  No branch: at a tenth and more of the columns nearly every warp has a hit in every value, and
+// four atomics are on their way before the first store waits for its place.
+static __device__ __noinline__ void sp_scatter_keys(const float* y, int ny, float lowest, float maxv, u32 b_thr, u32 cursor)
 {
-    constexpr int BPT = kSpBins / kThreads;       // bins per thread: 8
-    constexpr int WMX = PER / 4;                  // words of two 16-bit sub-bucket counters per thread, at most
-    const int     nsub = cap / 2, wpt = cap / 4 / kThreads;
+    FTB_ASSUME_SHARED(y);
+    constexpr int U = 2;
+    for (int i0 = 4 * (int)threadIdx.x; i0 < ny; i0 += 4 * kThreads * U) {
+        float4 v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int i = i0 + q * 4 * kThreads;
+            v[q]        = i < ny ? *(const float4*)(y + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
+        u32 to[4 * U];
+#pragma unroll
+        for (int e = 0; e < 4 * U; ++e) {
+            const float4& w = v[e >> 2];
+            const float   x = (e & 3) == 0 ? w.x : ((e & 3) == 1 ? w.y : ((e & 3) == 2 ? w.z : w.w));
+            const u32     b = (u32)sp_bin(maxv - x);
+            asm volatile("{\n .reg .pred p;\n setp.le.u32 p, %1, %2;\n setp.ge.and.f32 p, %3, %4, p;\n mov.u32 %0, 0xffffffff;\n"
+                         " @p atom.shared.add.u32 %0, [%5], 4;\n}"
+                         : "=&r"(to[e])
+                         : "r"(b), "r"(b_thr), "f"(x), "f"(lowest), "r"(cursor + 4u * b)
+                         : "memory");
+        }
+#pragma unroll
+        for (int e = 0; e < 4 * U; ++e) {
+            const float4& w = v[e >> 2];
+            const float   x = (e & 3) == 0 ? w.x : ((e & 3) == 1 ? w.y : ((e & 3) == 2 ? w.z : w.w));
+            asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0xffffffff;\n @p st.shared::cluster.f32 [%0], %1;\n}" ::"r"(to[e]),
+                         "f"(x)
+                         : "memory");
+        }
+    }
+}
+
+// One nucleus owner's n keys (fp32 values, bin by bin) into descending order.  `excl` holds the first position of every bin in the
+// row's order, `sub` counters for n / 2 sub-buckets.  A key's place inside its bin is guessed from
+// its position between the bin's edges, so that a sub-bucket of two places receives two keys on average whatever the
+// distribution is; inside it a key's place is the number of larger ones.
+//
+// The keys go to `tmp` by sub-bucket and come back in order: three short loops, because a row passes through this code once and
+// an unrolled form waits for its instructions.  900 keys: 6 us, 4850 keys: 19 us (before, keys held in registers by code
+// unrolled for 10240 of them: 20 to 26 us).  Returns false when a long sub-bucket of many values would have to be ordered.
+constexpr int kSpShort = 24;   // keys of a sub-bucket that every thread orders for itself
+constexpr int kSpLists = 256;  // words for the list of longer ones
+
+// sub-bucket of a key, [0, (n + 1) / 2)
+__device__ __forceinline__ u32 sp_sub_bucket(const u32* excl, float v, float maxv, u32 start, int n)
+{
+    const float t = sp_pos(maxv - v);
+    const int   b = (int)t;
+    const u32   e = excl[b], c = (b + 1 < kSpBins ? excl[b + 1] : start + (u32)n) - e;
+    u32         o = (u32)((t - (float)b) * (float)c);
+    o             = c > 0 && o >= c ? c - 1u : o;
+    const u32 s = (e - start + o) >> 1, last = (u32)(n - 1) >> 1;
+    return s < last ? s : last;
+}
+// the counts of `sub` (two 16-bit ones a word) become first positions
+static __device__ __forceinline__ void sp_sub_prefix(u32* sub, int words)
+{
+    const int wpt = (words + kThreads - 1) / kThreads, w0 = (int)threadIdx.x * wpt, w1 = w0 + wpt < words ? w0 + wpt : words;
+    u32       mine = 0, tot;
+#pragma unroll 1
+    for (int w = w0; w < w1; ++w) {
+        mine += (sub[w] & 0xffffu) + (sub[w] >> 16);
+    }
+    u32 run = block_excl_u32(mine, &tot);
+#pragma unroll 1
+    for (int w = w0; w < w1; ++w) {
+        const u32 c = sub[w];
+        sub[w]      = run | ((run + (c & 0xffffu)) << 16);
+        run += (c & 0xffffu) + (c >> 16);
+    }
+    __syncthreads();
+}
+
+// n <= 25 * kSpLists
+static __device__ __noinline__ bool sp_sort_keys(float* a, float* tmp, u32* sub, const u32* excl, u32* list, u32 start, int n, float maxv)
+{
     FTB_ASSUME_SHARED(a);
+    FTB_ASSUME_SHARED(tmp);
     FTB_ASSUME_SHARED(sub);
     FTB_ASSUME_SHARED(excl);
-    FTB_ASSUME_SHARED(place);
-    const int tid = threadIdx.x;
-    for (int i = tid; i < nsub / 2; i += kThreads) {
+    FTB_ASSUME_SHARED(list);
+    __shared__ u32 s_nlong;
+    const int      tid = threadIdx.x, lane = tid & 31, words = ((n + 1) / 2 + 1) / 2;
+#pragma unroll 1
+    for (int i = tid; i < words; i += kThreads) {
         sub[i] = 0;
-    }
-    {
-        // sub-buckets a bin takes: its keys one after the other with padding around a large bin
-        u32 c[BPT], mine = 0, tot;
-#pragma unroll
-        for (int i = 0; i < BPT; ++i) {
-            const int b  = tid * BPT + i;
-            const u32 e0 = excl[b], e1 = b + 1 < kSpBins ? excl[b + 1] : start + (u32)n;
-            c[i]         = (e0 >= start && e0 < start + (u32)n) ? e1 - e0 : 0u;
-            c[i] += c[i] >= 8u ? 8u : 0u;
-            mine += c[i];
-        }
-        u32 run = block_excl_u32(mine, &tot);
-#pragma unroll
-        for (int i = 0; i < BPT; ++i) {
-            place[tid * BPT + i] = run + (c[i] >= 16u ? 4u : 0u);
-            run += c[i];
-        }
-    }
-    __syncthreads();
-    // The keys arrive bin by bin: the 32 lanes of a warp take theirs from 32 places far apart, or they would all count
-    // in the same sub-bucket.
-    const int seg = ((n + 31) / 32) | 1;
-    float     v[PER];
-    u32       at[PER];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int q = i * kThreads + tid, p = (q >> 5) < seg ? (q & 31) * seg + (q >> 5) : n;
-        at[i]       = 0xffffffffu;
-        v[i]        = 0.0f;
-        if (i * kThreads < 32 * seg && p < n) {
-            v[i]          = a[p];
-            const float t = sp_pos(maxv - v[i]);
-            const int   b = (int)t;
-            const u32   c = (b + 1 < kSpBins ? excl[b + 1] : start + (u32)n) - excl[b];
-            u32         o = (u32)((t - (float)b) * (float)c);
-            o             = c > 0 && o >= c ? c - 1u : o;
-            u32 s         = (place[b] + o) >> 2;
-            s             = s < (u32)nsub ? s : (u32)nsub - 1u;
-            const u32 old = atomicAdd(&sub[s >> 1], 1u << (16 * (s & 1u)));
-            at[i]         = (s << 16) | ((old >> (16 * (s & 1u))) & 0xffffu);
-        }
-    }
-    __syncthreads();
-    {
-        u32 c[WMX], mine = 0, tot;
-#pragma unroll
-        for (int i = 0; i < WMX; ++i) {
-            c[i] = i < wpt ? sub[tid * wpt + i] : 0u;
-            mine += (c[i] & 0xffffu) + (c[i] >> 16);
-        }
-        u32 run = block_excl_u32(mine, &tot);
-#pragma unroll
-        for (int i = 0; i < WMX; ++i) {
-            if (i < wpt) {
-                sub[tid * wpt + i] = run | ((run + (c[i] & 0xffffu)) << 16);
-            }
-            run += (c[i] & 0xffffu) + (c[i] >> 16);
-        }
-    }
-    __syncthreads();
-    auto first_of = [&](int s) { return s < nsub ? (int)((sub[s >> 1] >> (16 * (s & 1))) & 0xffffu) : n; };
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        if (i * kThreads < 32 * seg && at[i] != 0xffffffffu) {
-            const int to         = first_of((int)(at[i] >> 16)) + (int)(at[i] & 0xffffu);
-            a[to < cap ? to : 0] = v[i];
-        }
-    }
-    __syncthreads();
-    // a sub-bucket of equal values (16-bit logits have many) is in order already; the others are short.  Where two
-    // neighbours stand the wrong way round is noted first, so that a long run of equal values is not walked.
-    __shared__ u32 s_wrong[PER * kThreads / 32];
-    __shared__ u32 s_long[64], s_nlong;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int p = i * kThreads + tid;
-        if (i * kThreads < n) {
-            const u32 m = __ballot_sync(0xffffffffu, p + 1 < n && a[p] < a[p + 1]);
-            if ((tid & 31) == 0) {
-                s_wrong[p >> 5] = m;
-            }
-        }
     }
     if (tid == 0) {
         s_nlong = 0;
     }
     __syncthreads();
-    bool ok = true;
-    for (int s = tid; s < nsub; s += kThreads) {
-        const int lo = first_of(s), hi = first_of(s + 1);
-        if (hi - lo < 2) {
-            continue;
-        }
-        // bits lo .. hi - 2
-        const int w0 = lo >> 5, w1 = (hi - 2) >> 5;
-        bool      wrong = false;
-        for (int w = w0; w <= w1; ++w) {
-            u32 m = s_wrong[w];
-            m &= w == w0 ? 0xffffffffu << (lo & 31) : 0xffffffffu;
-            m &= w == w1 ? 0xffffffffu >> (31 - ((hi - 2) & 31)) : 0xffffffffu;
-            wrong |= m != 0;
-        }
-        if (!wrong) {
-            continue;
-        }
-        if (hi - lo > 12) {
-            const u32 slot = atomicAdd(&s_nlong, 1u);
-            if (slot < 64u && hi - lo <= 512) {
-                s_long[slot] = (u32)s;
-            }
-            else {
-                ok = false;
-            }
-            continue;
-        }
-        for (int i = lo + 1; i < hi; ++i) {
-            const float x = a[i];
-            int         j = i - 1;
-            while (j >= lo && a[j] < x) {
-                a[j + 1] = a[j];
-                --j;
-            }
-            a[j + 1] = x;
+    // The 32 lanes of a warp take their keys from 32 places far apart: neighbours lie in the same sub-bucket.
+    const int seg = ((n + 31) / 32) | 1;
+#pragma unroll 1
+    for (int j = tid >> 5; j < seg; j += kWarps) {
+        const int p = lane * seg + j;
+        if (p < n) {
+            const u32 s = sp_sub_bucket(excl, a[p], maxv, start, n);
+            smem_add(&sub[s >> 1], 1u << (16 * (s & 1u)));
         }
     }
-    ok = __syncthreads_and(ok) != 0;
-    // A long sub-bucket holds few distinct values (a run of equal ones with a penalised column's beside it): a warp takes
-    // the largest value left, writes it as often as it occurs, and goes on.
-    const int lane = tid & 31;
-    for (u32 w = (u32)(tid >> 5); ok && w < s_nlong; w += kWarps) {
-        const int lo = first_of((int)s_long[w]), m = first_of((int)s_long[w] + 1) - lo;
-        u32       k[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            k[i] = i * 32 + lane < m ? fkey(a[lo + i * 32 + lane]) : 0u;
+    __syncthreads();
+    sp_sub_prefix(sub, words);
+#pragma unroll 1
+    for (int j = tid >> 5; j < seg; j += kWarps) {
+        const int p = lane * seg + j;
+        if (p < n) {
+            const float v   = a[p];
+            const u32   s   = sp_sub_bucket(excl, v, maxv, start, n);
+            const u32   old = atomicAdd(&sub[s >> 1], 1u << (16 * (s & 1u)));
+            tmp[(old >> (16 * (s & 1u))) & 0xffffu] = v;
         }
-        __syncwarp();
-        u32 below = 0xffffffffu;
-        for (int at_pos = 0; at_pos < m;) {
-            u32 top = 0;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                top = k[i] < below && k[i] > top ? k[i] : top;
+    }
+    __syncthreads();
+    // (the counters now hold where their sub-bucket ends)
+    auto end_of = [&](u32 s) { return (int)((sub[s >> 1] >> (16 * (s & 1u))) & 0xffffu); };
+#pragma unroll 1
+    for (int p = tid; p < n; p += kThreads) {
+        const float v  = tmp[p];
+        const u32   s  = sp_sub_bucket(excl, v, maxv, start, n);
+        const int   lo = s > 0 ? end_of(s - 1u) : 0, hi = end_of(s);
+        if (hi - lo > kSpShort) {
+            if (p == lo) {
+                list[atomicAdd(&s_nlong, 1u)] = (u32)lo | ((u32)(hi - lo) << 16);  // (at most n / 25 of them)
             }
-            top     = __reduce_max_sync(0xffffffffu, top);
-            u32 cnt = 0;
+            continue;
+        }
+        int to = lo;
+#pragma unroll 1
+        for (int j = lo; j < hi; j += 4) {
+            float x[4];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                cnt += k[i] == top ? 1u : 0u;
+            for (int q = 0; q < 4; ++q) {
+                x[q] = j + q < hi ? tmp[j + q] : -INFINITY;
             }
-            cnt = __reduce_add_sync(0xffffffffu, cnt);
-            if (cnt == 0) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                to += (x[q] > v ? 1 : 0) | (x[q] == v && j + q < p ? 1 : 0);
+            }
+        }
+        a[to] = v;
+    }
+    __syncthreads();
+    // A long sub-bucket holds few distinct values (16-bit logits: a run of equal ones, a penalised column's beside it): a warp
+    // takes the largest value left, writes it as often as it occurs, and goes on.
+    bool ok = true;
+#pragma unroll 1
+    for (u32 w = (u32)(tid >> 5); w < s_nlong; w += kWarps) {
+        const int lo = (int)(list[w] & 0xffffu), m = (int)(list[w] >> 16);
+        u32       below = 0xffffffffu;
+        int       pos = 0;
+        for (int d = 0; d < 256 && pos < m; ++d) {
+            u32 top = 0, c = 0;
+            for (int i = lane; i < m; i += 32) {
+                const u32 k = fkey(tmp[lo + i]);
+                c           = k >= below || k < top ? c : (k > top ? 1u : c + 1u);
+                top         = k < below && k > top ? k : top;
+            }
+            below = __reduce_max_sync(0xffffffffu, top);
+            c     = __reduce_add_sync(0xffffffffu, top == below ? c : 0u);
+            if (c == 0) {
                 break;
             }
-            for (int i = lane; i < (int)cnt; i += 32) {
-                a[lo + at_pos + i] = fkey_inv(top);
+            for (int i = lane; i < (int)c; i += 32) {
+                a[lo + pos + i] = fkey_inv(below);
             }
-            at_pos += (int)cnt;
-            below = top;
+            pos += (int)c;
         }
+        ok = ok && pos >= m;
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
+// All of an owner's keys: at once while they fill at most half of the area (its other half is tmp), else stretches of whole bins
+// one after the other, with tmp in the words behind the counters (`sub` to the end of `hist`).  A bin that is larger than a
+// stretch holds few distinct values (16-bit logits); more than 32 of them are given up.
+static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* hist, u32 start, int n, float maxv, int cap)
+{
+    __shared__ u32 s_end, s_top, s_cnt, s_val[32], s_num[32];
+    FTB_ASSUME_SHARED(a);
+    FTB_ASSUME_SHARED(excl);
+    const int  tid = threadIdx.x, lane = tid & 31;
+    u32* const list = hist + kSpBins - kSpLists;
+    if (n <= cap / 2) {
+        return sp_sort_keys(a, a + cap / 2, sub, excl, list, start, n, maxv);
+    }
+    const int most = (cap / 4 + kSpBins - kSpLists) * 4 / 5 - 4;  // (a quarter of a word for the counters, one for the key)
+    bool      ok   = true;
+    for (int at = 0; at < n;) {
+        int cnt = n - at;
+        if (cnt > most) {
+            // the last bin that starts within the stretch starts the next one
+            __syncthreads();
+            if (tid == 0) {
+                s_end = 0;
+                s_cnt = start + (u32)n;
+            }
+            __syncthreads();
+            const u32 first = start + (u32)at;
+            u32       last = 0, next = 0xffffffffu;
+            for (int b = tid; b < kSpBins; b += kThreads) {
+                const u32 e = excl[b];
+                last        = e > first && e <= first + (u32)most && e > last ? e : last;
+                next        = e > first && e < next ? e : next;
+            }
+            atomicMax(&s_end, last);
+            atomicMin(&s_cnt, next);
+            __syncthreads();
+            const bool bin_alone = s_end == 0;
+            cnt                  = (int)((bin_alone ? s_cnt : s_end) - first);
+            if (bin_alone) {
+                u32 below = 0xffffffffu;
+                int left = cnt, d = 0;
+                for (; d < 32 && left > 0; ++d) {
+                    __syncthreads();
+                    if (tid == 0) {
+                        s_top = 0;
+                        s_cnt = 0;
+                    }
+                    __syncthreads();
+                    u32 top = 0;
+                    for (int i = tid; i < cnt; i += kThreads) {
+                        const u32 k = fkey(a[at + i]);
+                        top         = k < below && k > top ? k : top;
+                    }
+                    top = __reduce_max_sync(0xffffffffu, top);
+                    if (lane == 0) {
+                        atomicMax(&s_top, top);
+                    }
+                    __syncthreads();
+                    below = s_top;
+                    u32 c = 0;
+                    for (int i = tid; i < cnt; i += kThreads) {
+                        c += fkey(a[at + i]) == below ? 1u : 0u;
+                    }
+                    c = __reduce_add_sync(0xffffffffu, c);
+                    if (lane == 0) {
+                        atomicAdd(&s_cnt, c);
+                    }
+                    __syncthreads();
+                    if (tid == 0) {
+                        s_val[d] = below;
+                        s_num[d] = s_cnt;
+                    }
+                    left = s_cnt != 0 ? left - (int)s_cnt : -1;
+                }
+                __syncthreads();
+                if (left == 0) {
+                    for (int q = 0, pos = at; q < d; ++q) {
+                        const float v = fkey_inv(s_val[q]);
+                        const int   c = (int)s_num[q];
+                        for (int i = tid; i < c; i += kThreads) {
+                            a[pos + i] = v;
+                        }
+                        pos += c;
+                    }
+                }
+                ok = ok && left == 0;
+                at += cnt;
+                continue;
+            }
+        }
+        ok = sp_sort_keys(a + at, (float*)(sub + cnt / 4 + 2), sub, excl, list, start + (u32)at, cnt, maxv) && ok;
+        at += cnt;
     }
     __syncthreads();
     return ok;
@@ -646,7 +790,8 @@ __device__ __forceinline__ float sp_key_at(const SpKeys& K, u32 pos)
     }
     return __uint_as_float(dld_u32(cluster_addr(K.area + 4u * (pos - K.start[o]), (u32)o)));
 }
-__device__ __forceinline__ void sp_load8(const SpKeys& K, u32 c, int lane, float* x)
+// eight keys of chunk c for this lane; `own`: this CTA's rank (0 where the keys lie in this CTA)
+__device__ __forceinline__ void sp_load8(const SpKeys& K, u32 c, int lane, int own, float* x)
 {
     const u32 total = K.start[K.owners], p0 = c * 256u + (u32)lane * 8u;
     int       o = 0;
@@ -654,10 +799,19 @@ __device__ __forceinline__ void sp_load8(const SpKeys& K, u32 c, int lane, float
         ++o;
     }
     if (p0 + 8u <= K.start[o + 1]) {
-        const u32 base = cluster_addr(K.area + 4u * (p0 - K.start[o]), (u32)o);
+        const u32 at = K.area + 4u * (p0 - K.start[o]);
+        if (o == own) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            x[i] = __uint_as_float(dld_u32(base + 4u * (u32)i));
+            for (int i = 0; i < 8; ++i) {
+                x[i] = __uint_as_float(lds_u32(at + 4u * (u32)i));
+            }
+        }
+        else {
+            const u32 base = cluster_addr(at, (u32)o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                x[i] = __uint_as_float(dld_u32(base + 4u * (u32)i));
+            }
         }
     }
     else {
@@ -686,24 +840,43 @@ __device__ __forceinline__ float sp_rake(const float* x, int lane)
     return inc;
 }
 
-// Warp 0 of the leader: running prefix over the chunk aggregates, the crossing inside its chunk, the crossing's
-// probability and its rank among the equal ones.  Returns the verdict (see SpShared).
-static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float* agg, float rand_num, bool complete, u32* p_out,
-                                                    u32* j_out)
+// Warp 0 of the leader: running prefix over the chunk aggregates (`agg` 16-byte aligned, readable up to a multiple of eight),
+// the crossing inside its chunk and the crossing's probability.  Returns the verdict (see SpShared).
+static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float* agg, float rand_num, bool complete, int own, u32* p_out,
+                                                    u32* sel_out)
 {
     FTB_ASSUME_SHARED(agg);
     const int lane = threadIdx.x & 31;
     const u32 N    = K.start[K.owners];
     const int nch  = (int)((N + 255u) / 256u);
     // chunk by chunk, as the reference's prefix functor accumulates; stopped a little early (inside a chunk the partial
-    // sums differ from prefix + aggregate in the last bits only)
+    // sums differ from prefix + aggregate in the last bits only).  The terms are not negative: eight at a time, the eight
+    // before the stop once more one by one.
     const float stop = rand_num * (1.0f - 1e-4f);
     float       R    = 0.0f;
-    int         c1   = nch;
-    for (int c = 0; c < nch; ++c) {
-        const float R2 = R + agg[c];
+    int         c1   = 0;
+    float4      x0 = *(const float4*)agg, x1 = *(const float4*)(agg + 4);
+    while (c1 + 8 <= nch) {
+        const int    nx = c1 + 16 <= ((nch + 7) & ~7) ? c1 + 8 : 0;
+        const float4 y0 = *(const float4*)(agg + nx), y1 = *(const float4*)(agg + nx + 4);
+        float        R2 = R + x0.x;
+        R2 += x0.y;
+        R2 += x0.z;
+        R2 += x0.w;
+        R2 += x1.x;
+        R2 += x1.y;
+        R2 += x1.z;
+        R2 += x1.w;
         if (R2 >= stop) {
-            c1 = c;
+            break;
+        }
+        R  = R2;
+        x0 = y0, x1 = y1;
+        c1 += 8;
+    }
+    for (; c1 < nch; ++c1) {
+        const float R2 = R + agg[c1];
+        if (R2 >= stop) {
             break;
         }
         R = R2;
@@ -711,7 +884,7 @@ static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float
     int sel = -1;
     for (int c = c1; c < nch; ++c) {
         float x[8];
-        sp_load8(K, (u32)c, lane, x);
+        sp_load8(K, (u32)c, lane, own, x);
         const float inc = sp_rake(x, lane);
         const float ag  = __shfl_sync(0xffffffffu, inc, 31);
         const float ex  = __shfl_up_sync(0xffffffffu, inc, 1);
@@ -743,29 +916,16 @@ static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float
             return 2;
         }
         // the cumulative sum never reached the draw: the reference leaves the best token in place
-        *p_out = __float_as_uint(sp_key_at(K, 0));
-        *j_out = 0;
+        *p_out   = __float_as_uint(sp_key_at(K, 0));
+        *sel_out = 0;
         return 1;
     }
-    const float p = sp_key_at(K, (u32)sel);
-    if (!complete && p == sp_key_at(K, N - 1)) {
+    const float p = sp_key_at(K, (u32)sel), last = complete ? 0.0f : sp_key_at(K, N - 1);
+    if (!complete && p == last) {
         return 2;  // the lowest class may have members that were not collected
     }
-    // first position with this probability: 32 probes at a time
-    u32 lo = 0, hi = (u32)sel;  // the answer lies in [lo, hi]
-    while (lo < hi) {
-        const u32 span = hi - lo, step = (span + 31u) / 32u;
-        const u32 q    = lo + (u32)lane * step;
-        const bool eq  = q >= hi || sp_key_at(K, q) == p;
-        const u32 m    = __ballot_sync(0xffffffffu, eq);
-        const int f    = m != 0 ? __ffs(m) - 1 : 32;
-        const u32 nhi  = lo + (u32)f * step;
-        const u32 nlo  = f == 0 ? lo : lo + (u32)(f - 1) * step + 1u;
-        hi             = nhi < hi ? nhi : hi;
-        lo             = nlo < hi ? nlo : hi;
-    }
-    *p_out = __float_as_uint(p);
-    *j_out = (u32)sel - lo;
+    *p_out   = __float_as_uint(p);
+    *sel_out = (u32)sel;
     return 0;
 }
 
@@ -841,14 +1001,27 @@ __device__ __forceinline__ void sp_write_topp(const KParams& P, const RowOut& O,
     }
 }
 
+__device__ __forceinline__ SpMap sp_map(const SplitArgs& A, unsigned char* smem)
+{
+    SpMap M;
+    M.y        = (float*)smem;
+    M.area     = (u32*)(M.y + A.slice);
+    M.area_cap = A.area;
+    M.merged   = M.area + A.area;
+    M.sub      = M.merged + kSpBins;
+    M.hist     = M.sub + A.area / 4;
+    return M;
+}
+
 // One row on the cluster.  Every branch that skips a cluster barrier depends on values that all CTAs hold alike.
 // Returns (leader only) whether the row is decided.
-template<int DT, int LGN, bool WHOLE>
-__device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, const SpMap& M, SpShared& X, const RowOut& O, int mode,
-                                       bool want_lp)
+template<int DT, int LGN>
+__device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, unsigned char* smem, SpShared& X, const RowOut& O, int mode,
+                                    bool want_lp)
 {
+    FTB_ASSUME_SHARED(smem);
+    const SpMap      M = sp_map(A, smem);
     __shared__ float s_u, s_denom;
-    __shared__ u32   s_start[kSpMaxN + 1], s_base[kSpMaxN + 1], s_rbase[kSpMaxN];
     __shared__ u32   s_base1, s_cutbin;
     const int        tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     constexpr int    n = 1 << LGN, lgvt = 10 - LGN;
@@ -877,6 +1050,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
         X.first_max = 0xffffffffu;
         X.best_tie  = 0;
         X.n_cls     = 0;
+        X.larger    = 0;
         X.bad_order = 0;
         curandState_t st = (mode == 1 ? P.topk_states : P.topp_states)[r];
         s_u              = curand_uniform(&st);
@@ -998,6 +1172,10 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
             }
 #pragma unroll
             for (int q = 0; q < n; ++q) {
+                // (a nucleus is placed by bin: what the CTAs before this one have of the bin goes where its count stood)
+                if (mode == 2) {
+                    dst_u32(cluster_addr(a, (u32)q), sum);
+                }
                 sum += part[q];
             }
 #pragma unroll
@@ -1178,10 +1356,14 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
         sorted = sp_bucket_sort(sorted, excl, n_cand, (u64*)M.y, n_cand <= 128 ? sorted + 1024 : sorted,
                                 [&](u64 e) { return sp_bin(maxv - key_of(e)); });
         trace_mark(O.trace, 8);
-        Smem S;
-        S.cand = (u64*)M.area;
-        S.hist = (u32*)M.y;
-        S.val2 = (float*)(M.y + kNB);
+        __shared__ Smem s_S;
+        const Smem&     S = s_S;
+        if (tid == 0) {
+            s_S.cand = (u64*)M.area;
+            s_S.hist = (u32*)M.y;
+            s_S.val2 = (float*)(M.y + kNB);
+        }
+        __syncthreads();
         if (!softmax) {
             return topk_finish(P, S, O, sorted, n_cand, k, u, P.topk_ps[r], true, false);
         }
@@ -1216,7 +1398,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
         __syncthreads();
         for (int c = wid; c * 256 < n_cand; c += kWarps) {
             float x[8];
-            sp_load8(s_K1, (u32)c, lane, x);
+            sp_load8(s_K1, (u32)c, lane, 0, x);
             const float inc = sp_rake(x, lane);
             if (lane == 31) {
                 X.agg[c] = inc;
@@ -1225,7 +1407,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
         __syncthreads();
         if (wid == 0) {
             u32       p = 0, j = 0;
-            const u32 v = sp_find_crossing(s_K1, X.agg, rand_num, complete, &p, &j);
+            const u32 v = sp_find_crossing(s_K1, X.agg, rand_num, complete, 0, &p, &j);
             if (lane == 0) {
                 s_res[0] = v, s_res[1] = p, s_res[2] = j;
             }
@@ -1249,6 +1431,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
                 --j;
                 rk += sorted[j] < e ? 1u : 0u;
             }
+            rk += (u32)j;  // (those of a larger probability)
             for (j = i + 1; j < n_cand && (u32)(sorted[j] >> 32) == key; ++j) {
                 rk += sorted[j] < e ? 1u : 0u;
             }
@@ -1265,81 +1448,59 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     // ---- a large nucleus: sorted by several CTAs ----
     int owners = (int)((N + 1023u) / 1024u);
     owners     = owners < 1 ? 1 : (owners > n ? n : owners);
-    auto owner_of = [&](u32 e) { return (int)(((u64)e * (u32)owners) / N); };
-    {
-        // this CTA's counts become cursors into its own list, ordered by bin
-        u32 c[PER], mine = 0, ltot;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            c[i] = M.hist[tid * PER + i];
-            mine += c[i];
-        }
-        u32 run = block_excl_u32(mine, &ltot);
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            M.hist[tid * PER + i] = run;
-            run += c[i];
-        }
-        __syncthreads();
-        if (tid <= kSpMaxN) {
-            s_start[tid] = tid == 0 ? 0u : N;
-            s_base[tid]  = tid == 0 ? 0u : (complete ? ltot : M.hist[b_thr + 1]);
-        }
-        __syncthreads();
-        for (int b = tid + 1; b <= b_thr; b += kThreads) {
-            // the first bin of an owner: where its keys start in the whole row's order and in this CTA's list
-            const int o = owner_of(excl[b]), before = owner_of(excl[b - 1]);
-            for (int q = before + 1; q <= o && q <= kSpMaxN; ++q) {
-                s_start[q] = excl[b];
-                s_base[q]  = M.hist[b];
-            }
-        }
-        __syncthreads();
-    }
     __shared__ SpKeys s_K;
+    __shared__ u32    s_bound[kSpMaxN];  // position e of the row's order: the last owner q with e >= s_bound[q]
     const SpKeys&     K = s_K;
     if (tid == 0) {
         s_K.area   = smem_addr(M.area);
         s_K.owners = owners;
     }
     if (tid <= kSpMaxN) {
-        s_K.start[tid] = s_start[tid];
+        s_K.start[tid] = tid == 0 ? 0u : N;
     }
-    const bool fits = N > 0 && __syncthreads_and(tid >= kSpMaxN || s_start[tid + 1] - s_start[tid] <= (u32)M.area_cap - 64u);
+    if (tid < kSpMaxN) {
+        s_bound[tid] = tid < owners ? ((u32)tid * N + (u32)owners - 1u) / (u32)owners : 0xffffffffu;
+    }
+    __syncthreads();
+    u32 owner_bits = 0;  // of this thread's bins, four bits each
+    {
+        auto advance = [&](int o, u32 e) {
+            while (o + 1 < kSpMaxN && e >= s_bound[o + 1]) {
+                ++o;
+            }
+            return o;
+        };
+        int o = tid == 0 ? 0 : advance(0, excl[tid * PER - 1]);
+        for (int i = 0; i < PER; ++i) {
+            // the first bin of an owner: where its keys start in the row's order
+            const int before = o;
+            const u32 e      = excl[tid * PER + i];
+            o                = tid * PER + i <= b_thr ? advance(o, e) : o;
+            for (int q = before + 1; q <= o; ++q) {
+                s_K.start[q] = e;
+            }
+            owner_bits |= (u32)o << (4 * i);
+        }
+    }
+    __syncthreads();
+    const bool fits = N > 0 && __syncthreads_and(tid >= kSpMaxN || s_K.start[tid + 1] - s_K.start[tid] <= (u32)M.area_cap - 64u);
     if (!fits) {
         return sp_leave(O, 6);
     }
     trace_mark(O.trace, 10);
-    // a range of every owner's area for this CTA's keys, then the keys (values: ordered like the probabilities)
-    if (tid < owners) {
-        const u32 cnt = s_base[tid + 1] - s_base[tid];
-        s_rbase[tid]  = cnt != 0 ? datom_add(cluster_addr(smem_addr(&X.area_n), (u32)tid), cnt) : 0u;
+    // per bin the place of this CTA's first key of it: the bin's in its owner's area, after the keys of the CTAs before
+    for (int i = 0; i < PER; ++i) {
+        const int b = tid * PER + i, o = (int)((owner_bits >> (4 * i)) & 15u);
+        M.hist[b]   = cluster_addr(K.area + 4u * (excl[b] - s_K.start[o] + M.hist[b]), (u32)o);
     }
     __syncthreads();
-    u32 first[n];  // first position of every owner after the leader
-#pragma unroll
-    for (int q = 1; q < n; ++q) {
-        first[q] = q < owners ? s_start[q] : 0xffffffffu;
-    }
-    sp_sweep(y, ny, fmaxf(sp_floor_value(maxv, b_thr), lowest), [&](int, float v) {
-        const int b = sp_bin(maxv - v);
-        if (b <= b_thr) {
-            const u32 pos = atomicAdd(&M.hist[b], 1u), e = excl[b];
-            int       o = 0;
-#pragma unroll
-            for (int q = 1; q < n; ++q) {
-                o += e >= first[q] ? 1 : 0;
-            }
-            dst_u32(cluster_addr(K.area + 4u * (s_rbase[o] + pos - s_base[o]), (u32)o), __float_as_uint(v));
-        }
-    });
+    sp_scatter_keys(y, ny, lowest, maxv, (u32)b_thr, smem_addr(M.hist));
     cluster_sync();
     trace_mark(O.trace, 11);
     if (rank < owners) {
         float* const a   = (float*)M.area;
-        const int    cnt = (int)(s_start[rank + 1] - s_start[rank]);
-        bool         bad = !sp_sort_area<(WHOLE ? kSpAreaMax : kSpAreaMid) / kThreads>(a, M.sub, excl, M.hist, s_start[rank], cnt, maxv,
-                                                                                       M.area_cap);
+        const int    cnt = (int)(K.start[rank + 1] - K.start[rank]);
+        bool         bad = !sp_sort_area(a, M.sub, excl, M.hist, K.start[rank], cnt, maxv, M.area_cap);
         for (int i = tid; i < cnt; i += kThreads) {
             a[i] = sp_prob<DT>(a[i], maxv, denom);
         }
@@ -1354,7 +1515,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     }
     if (owners > 1) {
         cluster_sync();
-        if (rank > 0 && rank < owners && tid == 0 && s_start[rank + 1] > s_start[rank]
+        if (rank > 0 && rank < owners && tid == 0 && K.start[rank + 1] > K.start[rank]
             && sp_key_at(K, K.start[rank] - 1u) < ((const float*)M.area)[0]) {
             dst_u32(cluster_addr(smem_addr(&X.bad_order), 0), 1u);
         }
@@ -1362,10 +1523,10 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     trace_mark(O.trace, 12);
     if (rank < owners) {
         // aggregates of the chunks that start in this owner's range
-        const u32 c0 = (s_start[rank] + 255u) >> 8, c1 = (s_start[rank + 1] + 255u) >> 8;
+        const u32 c0 = (K.start[rank] + 255u) >> 8, c1 = (K.start[rank + 1] + 255u) >> 8;
         for (u32 c = c0 + (u32)wid; c < c1; c += kWarps) {
             float x[8];
-            sp_load8(K, c, lane, x);
+            sp_load8(K, c, lane, rank, x);
             const float inc = sp_rake(x, lane);
             if (lane == 31) {
                 dst_u32(cluster_addr(smem_addr(&X.agg[c]), 0), __float_as_uint(inc));
@@ -1382,7 +1543,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     if (rank == 0 && wid == 0) {
         u32 p = 0, j = 0, verdict = 2;
         if (!X.bad_order) {
-            verdict = sp_find_crossing(K, X.agg, rand_num, complete, &p, &j);
+            verdict = sp_find_crossing(K, X.agg, rand_num, complete, 0, &p, &j);
         }
         if (lane < n) {
             const u32 q = (u32)lane;
@@ -1405,24 +1566,34 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, con
     const float e_sel = p_sel * denom, e_lo = e_sel * (1.0f - slack) - tiny, pad = 1e-4f + 2e-6f * fabsf(maxv);
     const float y_lo  = e_lo > 1e-37f ? maxv + __logf(e_lo) * 1.00001f - pad : -INFINITY;
     const float y_hi  = maxv + __logf(fmaxf(e_sel * (1.0f + slack) + tiny, 1e-37f)) * 0.99999f + pad;
-    sp_sweep(y, ny, fmaxf(y_lo, lowest), [&](int i, float v) {
-        if (v <= y_hi && sp_prob<DT>(v, maxv, denom) == p_sel) {
+    const u32 larger = sp_sweep_band(y, ny, fmaxf(y_lo, lowest), y_hi, [&](int i, float v) {
+        const float p = sp_prob<DT>(v, maxv, denom);
+        if (p == p_sel) {
             const u32 pos = datom_add(cluster_addr(smem_addr(&X.n_cls), 0), 1u);
             if (pos < (u32)M.area_cap) {
                 dst_u32(cluster_addr(K.area + 4u * pos, 0), (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1))));
             }
         }
+        return p > p_sel ? 1u : 0u;
     });
+    {
+        // columns of a larger probability: the class's first position in the sorted order
+        const u32 w = __reduce_add_sync(0xffffffffu, larger);
+        if (lane == 0 && w != 0) {
+            dred_add(cluster_addr(smem_addr(&X.larger), 0), w);
+        }
+    }
     cluster_sync();
     if (rank != 0) {
         return true;
     }
-    const u32 n_cls = X.n_cls, j_sel = X.j_sel;
+    const u32 n_cls = X.n_cls, j_sel = X.j_sel - X.larger;
     trace_mark(O.trace, 15);
     if (n_cls > (u32)M.area_cap || j_sel >= n_cls) {
         return sp_leave(O, 8);
     }
-    const int id = n_cls == 1 ? (int)M.area[0] : select_jth_column(M.area, (int)n_cls, (int)j_sel, (u32*)M.y, P.vocab_padded);
+    const int id = n_cls <= 512 ? sp_jth_of_few(M.area, (int)n_cls, (int)j_sel) :
+                                  select_jth_column(M.area, (int)n_cls, (int)j_sel, (u32*)M.y, P.vocab_padded);
     if (tid == 0) {
         sp_write_topp<DT>(P, O, id, p_sel, verdict == 0, want_lp);
     }
@@ -1507,6 +1678,11 @@ static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, int ar
 // of 30 steps of fresh normal logits, 800 x 126959 bf16 with log-probabilities: 1.2 / 1.2 ms (sigma 2.5, p 0.95), 2.3 / 2.7
 // (sigma 2, p 0.95, temperature 1.2), 27 / 43 (sigma 1.5, p 0.95, temperature 1.2); 60 x 200000 fp32: 0.9 / 1.8, 9.4 / 10.2 and
 // 13.6 / 15.1 ms.
+//
+// Stack: the form that keeps every row holds the general row code's frames under its own.  Builds of it with 1904 and 1952
+// bytes a thread ended steps of 37 rows (two CTAs of a cluster on an SM) with an illegal address, one of them with nothing
+// but two prints that never ran added to a source that runs at 1808; 16 rows (one CTA on an SM) ran.  No access of the code
+// is behind it: what grows is kept in shared memory instead, and the frame stays at 1728.
 template<int DT, int LGN, bool WHOLE>
 __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
                                                                      const __grid_constant__ SplitArgs A)
@@ -1514,13 +1690,6 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SpShared                           s_X;
     __shared__ RowOut                             s_O;
-    SpMap                                         M;
-    M.y      = (float*)smem_raw;
-    M.area   = (u32*)(M.y + A.slice);
-    M.area_cap = A.area;
-    M.merged   = M.area + A.area;
-    M.sub      = M.merged + kSpBins;
-    M.hist     = M.sub + A.area / 4;
     const int  tid = threadIdx.x, rank = (int)cluster_rank();
     const bool want_lp = P.cum_log_probs != nullptr || P.out_log_probs != nullptr;
     const int  first = (int)blockIdx.x >> LGN, step = (int)gridDim.x >> LGN;
@@ -1575,7 +1744,7 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
         __syncthreads();
         bool decided = true;
         if (mode != 0 && !fin) {
-            decided = sp_row<DT, LGN, WHOLE>(P, A, M, s_X, s_O, mode, want_lp);
+            decided = sp_row<DT, LGN>(P, A, smem_raw, s_X, s_O, mode, want_lp);
             __syncthreads();
         }
         if (rank == 0 && tid == 0) {

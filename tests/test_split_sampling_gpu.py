@@ -100,6 +100,43 @@ def test_wide_nuclei_of_many_rows(dtype, V, B, cuda_device):
         np.testing.assert_array_equal(got[1][k], v, err_msg=k)
 
 
+@pytest.mark.parametrize("dtype,V,B,sigma,grid,log_probs", [
+    (F32, 20000, 5, 0.5, 0, False),     # a nucleus of most columns, several owners, sub-buckets of a key or two
+    (F32, 50257, 9, 2.5, 0, True),      # either side of what the leader takes alone
+    (F32, 50257, 66, 1.5, 0, False),    # four CTAs a row, owners at and above half of their area
+    (F32, 128256, 3, 1.2, 0, False),    # eight owners with more keys than half of their area: stretch by stretch
+    (BF16, 128256, 4, 1.5, 8, False),   # runs of thousands of equal keys: a bin that is larger than a stretch
+    (BF16, 128256, 20, 2.0, 0, True), (F16, 51200, 40, 1.8, 0, True), (F16, 40960, 12, 1.0, 16, True)])
+def test_nucleus_widths(dtype, V, B, sigma, grid, log_probs, cuda_device):
+    """Top-p rows of every width: candidates of the leader, keys of one to eight owners, their sort in all its forms."""
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    got = []
+    for general in (1, 0):
+        g = torch.Generator(device=cuda_device)
+        g.manual_seed(V + B)
+        p = np.resize(np.asarray([0.2, 0.5, 0.8, 0.9, 0.97], np.float32), B)
+        layer = DynamicDecodeLayer(V, V, dtype, cuda_device)
+        layer.setup(B, 1, {"runtime_top_p": p, "repetition_penalty": np.asarray([1.05], np.float32), "random_seed": np.arange(B).astype(np.uint64)})
+        st = {"output_ids": torch.randint(1, V, (44, B), generator=g, device=cuda_device, dtype=torch.int32),
+              "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+              "sequence_length": torch.full((B,), 40, dtype=torch.int32, device=cuda_device)}
+        if log_probs:
+            st |= {"cum_log_probs": torch.zeros(B, device=cuda_device), "output_log_probs": torch.zeros(8, B, device=cuda_device)}
+        lib.ftb200_set_single_pass(1 - general)
+        try:
+            for s in range(3):
+                x = torch.randn(B, V, generator=g, device=cuda_device) * sigma
+                x = (x * grid).round() / grid if grid else x
+                layer.forward(st, {"logits": x.to(dtype), "step": 40 + s, "max_input_length": 40, "ite": 0, "local_batch_size": B,
+                                   "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)})
+            torch.cuda.synchronize()
+        finally:
+            lib.ftb200_set_single_pass(1)
+        got.append({k: v.cpu().numpy() for k, v in st.items()} | {"curand": layer.topp.curand.cpu().numpy()})
+    for k, v in got[0].items():
+        np.testing.assert_array_equal(got[1][k], v, err_msg=k)
+
+
 def one_kind(general, kind, dtype, V, B, device):
     """Two steps of a call with top-k rows or top-p rows alone; what they wrote and the launches they took."""
     from fastertransformer_b200 import DynamicDecodeLayer, lib
