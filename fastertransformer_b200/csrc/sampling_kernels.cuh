@@ -1093,6 +1093,68 @@ static __device__ __noinline__ int resolve_topk_class(u64* cls, int m, int want,
         __syncthreads();
         return r;
     }
+    if (m <= 2 * kThreads) {
+        // both orders by counting: two passes of m reads that all lanes share, where two sorting networks of 64 to 512 entries
+        // take 21 to 45 barriers each (k = 1024 with its class, one row: 21 us before, 14 now)
+        auto key_of = [&](u32 col) { return ((u64)((col / bs1) & 7u) << 56) | ((u64)(bs1 - 1 - (int)(col % bs1)) << 40) | col; };
+        u64  key1[2];
+        u32  key2[2];
+        if (tid == 0) {
+            s_ans = -1;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int a = tid + q * kThreads;
+            key1[q]     = a < m ? key_of((u32)(cls[a] & 0xffffffffu)) : 0u;
+            if (a < m) {
+                cls[a] = key1[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            key2[q] = 0xffffffffu;
+            if (tid + q * kThreads < m) {
+                const u32 lane  = (u32)(key1[q] >> 56);
+                const u64 first = (u64)lane << 56, mine = key1[q] - first;
+                u32       r     = lane_base[lane];
+#pragma unroll 8
+                for (int j = 0; j < m; ++j) {
+                    r += cls[j] - first < mine ? 1u : 0u;
+                }
+                if (r < (u32)k) {
+                    const u32 i2 = lane * (u32)k + r;  // < 8 * 1024
+                    key2[q]      = (((u32)bs2 - 1u - (i2 % (u32)bs2)) << 16) | i2;
+                }
+            }
+        }
+        u32* const keys = (u32*)cls;  // (the second order's keys over the first's; in shared or, for a huge nucleus, global memory)
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (tid + q * kThreads < m) {
+                keys[tid + q * kThreads] = key2[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (key2[q] != 0xffffffffu) {
+                int at = 0;
+#pragma unroll 8
+                for (int j = 0; j < m; ++j) {
+                    at += keys[j] < key2[q] ? 1 : 0;
+                }
+                if (at == (want < m ? want : m - 1)) {
+                    s_ans = (int)(u32)key1[q];
+                }
+            }
+        }
+        __syncthreads();
+        const int r = s_ans;
+        __syncthreads();
+        return r;
+    }
     if (tid < 8) {
         s_lane_cnt[tid] = 0;
     }
@@ -1434,107 +1496,93 @@ static __device__ __noinline__ bool topk_finish(const KParams& P, const Smem& S,
                             float top_p, bool use_exp, bool want_lp, bool open_end = false)
 {
     __shared__ int   s_pick, s_lo, s_hi;
-    __shared__ float s_e, s_sum;
+    __shared__ float s_sum;
     __shared__ u32   s_lane_base[8];
     const int        tid   = threadIdx.x;
-    const int        k_eff = k < n ? k : n;
+    const int        k_eff = k < n ? k : n, k32 = (k_eff + 31) & ~31;  // (k <= 1024, the room for the values)
+    float* const     val = S.val2;
+    float* const     run = (float*)S.hist;  // [k32] running values; the bucket counts are not needed any more
+    FTB_ASSUME_SHARED(val);
+    FTB_ASSUME_SHARED(run);
     if (tid < 8) {
         s_lane_base[tid] = 0;
+    }
+    if (tid == 0) {
+        s_pick = k_eff - 1;
     }
     // e_i in parallel; the sum and the walk keep the reference's sequential order (:276-287)
     {
         const float s_max = k_eff > 0 ? fkey_inv(~(u32)(sorted[0] >> 32)) : 0.0f;
-        for (int i = tid; i < k_eff; i += kThreads) {
-            float y   = fkey_inv(~(u32)(sorted[i] >> 32));
-            S.val2[i] = use_exp ? __expf(y - s_max) : y;
+#pragma unroll 1
+        for (int i = tid; i < k32; i += kThreads) {
+            const float y = i < k_eff ? fkey_inv(~(u32)(sorted[i] >> 32)) : 0.0f;
+            val[i]        = i >= k_eff ? 0.0f : (use_exp ? __expf(y - s_max) : y);
         }
     }
     __syncthreads();
-    // The sum and the walk are chains of dependent adds in the reference's order (one thread).  The walk stores
-    // every running value instead of testing it; the first one that ends the reference's loop is then found by
-    // all threads.  Operands are fetched eight at a time so that the chains do not wait for shared memory.
-    float* run = (float*)S.hist;  // [k_eff] running values; the bucket counts are not needed any more
-    FTB_ASSUME_SHARED(run);
-    __shared__ int s_walked;
-    if (tid == 0) {
-        s_pick   = k_eff > 0 ? k_eff - 1 : -1;
-        s_walked = 0;
-        if (k_eff > 0) {
-            const float* val = S.val2;
-            FTB_ASSUME_SHARED(val);
-            // (sixteen terms a round, four per load, the next sixteen on their way: the chain is the adds alone.
-            // k = 1024: 14 us with a load per term, 8 us)
-            const int k16 = k_eff & ~15;
-            float     sum = 0.0f;
-            float4    v[4], w[4];
-            auto      fetch = [&](float4* to, int i) {
+    // The sum and the walk are chains of dependent adds in the reference's order (one thread), 32 terms a round: while sixteen
+    // are added the next sixteen are on their way.  (The zeros behind the last term change neither.)  The walk stores every
+    // running value instead of testing it; the first one that ends the reference's loop is then found by all threads: the
+    // terms are not negative, so the running value only falls, and once a round ends at or below zero the reference's loop
+    // has stopped inside it.
+    if (tid == 0 && k32 > 0) {
+        float  sum = 0.0f;
+        float4 v[4], w[4];
+        auto   fetch = [&](float4* to, int i) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    to[j] = *(const float4*)(val + i + 4 * j);
-                }
-            };
-            if (k16 > 0) {
-                fetch(v, 0);
+            for (int j = 0; j < 4; ++j) {
+                to[j] = *(const float4*)(val + i + 4 * j);
             }
-            for (int i = 0; i < k16; i += 16) {
-                fetch(w, i + 16 < k16 ? i + 16 : 0);
+        };
+        auto add16 = [&](const float4* x) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sum += v[j].x;
-                    sum += v[j].y;
-                    sum += v[j].z;
-                    sum += v[j].w;
-                    v[j] = w[j];
-                }
+            for (int j = 0; j < 4; ++j) {
+                sum += x[j].x;
+                sum += x[j].y;
+                sum += x[j].z;
+                sum += x[j].w;
             }
-            for (int i = k16; i < k_eff; ++i) {
-                sum += val[i];
-            }
-            float rand_num = u * top_p * sum;
-            int   walked   = 0;
-            if (k16 > 0) {
-                fetch(v, 0);
-            }
-            // the terms are not negative, so the running value only falls: once a group of sixteen ends at or below
-            // zero the reference's loop has stopped inside it
-            for (int i = 0; i < k16 && !(rand_num <= 0.0f); i += 16) {
-                fetch(w, i + 16 < k16 ? i + 16 : 0);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float4 r;
-                    r.x      = rand_num - v[j].x;
-                    r.y      = r.x - v[j].y;
-                    r.z      = r.y - v[j].z;
-                    r.w      = r.z - v[j].w;
-                    rand_num = r.w;
-                    *(float4*)(run + i + 4 * j) = r;
-                    v[j] = w[j];
-                }
-                walked = i + 16;
-            }
-            if (walked == k16) {
-                for (int i = k16; i < k_eff && !(rand_num <= 0.0f); ++i) {
-                    rand_num = rand_num - val[i];
-                    run[i]   = rand_num;
-                    walked   = i + 1;
-                }
-            }
-            s_walked = walked;
-            s_sum    = sum;
+        };
+        fetch(v, 0);
+#pragma unroll 1
+        for (int i = 0; i < k32; i += 32) {
+            fetch(w, i + 16);
+            add16(v);
+            fetch(v, i + 32 < k32 ? i + 32 : 0);
+            add16(w);
         }
+        float rand_num = u * top_p * sum;
+        auto  walk16   = [&](const float4* x, int i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float4 r;
+                r.x      = rand_num - x[j].x;
+                r.y      = r.x - x[j].y;
+                r.z      = r.y - x[j].z;
+                r.w      = r.z - x[j].w;
+                rand_num = r.w;
+                *(float4*)(run + i + 4 * j) = r;
+            }
+        };
+        int walked = 0;
+#pragma unroll 1
+        do {
+            fetch(w, walked + 16);
+            walk16(v, walked);
+            fetch(v, walked + 32 < k32 ? walked + 32 : 0);
+            walk16(w, walked + 16);
+            walked += 32;
+        } while (walked < k32 && !(rand_num <= 0.0f));
+        s_lo  = walked;
+        s_sum = sum;
     }
     __syncthreads();
-    for (int i = tid, nw = s_walked; i < nw; i += kThreads) {
-        if (run[i] <= 0.0f || i == k - 1) {
-            atomicMin(&s_pick, i);
-            break;  // later entries of this thread are larger
+    // the first running value at or below zero (it lies in the last round) ends the loop, else the last term does
+    if (k32 > 0 && tid < 32) {
+        const int i = s_lo - 32 + tid;
+        if (i < k_eff && run[i] <= 0.0f && (i == 0 || !(run[i - 1] <= 0.0f))) {
+            s_pick = i;
         }
-    }
-    __syncthreads();
-    if (tid == 0 && s_pick >= 0) {
-        s_e  = S.val2[s_pick];
-        s_lo = s_pick;
-        s_hi = s_pick + 1;
     }
     __syncthreads();
     trace_mark(O.trace, 21);
@@ -1554,10 +1602,16 @@ static __device__ __noinline__ bool topk_finish(const KParams& P, const Smem& S,
         __syncthreads();
         return false;
     }
+#pragma unroll 1
     for (int i = tid; i < n; i += kThreads) {
         if ((u32)(sorted[i] >> 32) == kv) {
-            atomicMin(&s_lo, i);
-            atomicMax(&s_hi, i + 1);
+            // (equal entries stand together)
+            if (i == 0 || (u32)(sorted[i - 1] >> 32) != kv) {
+                s_lo = i;
+            }
+            if (i == n - 1 || (u32)(sorted[i + 1] >> 32) != kv) {
+                s_hi = i + 1;
+            }
         }
     }
     __syncthreads();
@@ -1570,24 +1624,10 @@ static __device__ __noinline__ bool topk_finish(const KParams& P, const Smem& S,
     else {
         const u32 bs1 = P.max_top_k <= 16 ? 128 : 256;
         const u32 bs2 = P.max_top_k <= 32 ? 128 : 256;
-        {
-            // per-thread counts packed 8 x 8 bits (a thread sees at most kCap / kThreads entries), one atomic
-            // per lane value and warp
-            const int sh1   = bs1 == 128 ? 7 : 8;
-            u64       packd = 0;
-            for (int i = tid; i < lo; i += kThreads) {
-                const u32 c = (u32)(sorted[i] & 0xffffffffu);
-                packd += 1ull << (8 * ((c >> sh1) & 7u));
-            }
-            for (int l = 0; l < 8; ++l) {
-                u32 cnt = (u32)(packd >> (8 * l)) & 0xffu;
-                for (int m = 16; m > 0; m >>= 1) {
-                    cnt += __shfl_xor_sync(0xffffffffu, cnt, m);
-                }
-                if ((tid & 31) == 0 && cnt != 0) {
-                    atomicAdd(&s_lane_base[l], cnt);
-                }
-            }
+        const int sh1 = bs1 == 128 ? 7 : 8;
+#pragma unroll 1
+        for (int i = tid; i < lo; i += kThreads) {
+            smem_add(&s_lane_base[((u32)sorted[i] >> sh1) & 7u], 1u);
         }
         __syncthreads();
         col = resolve_topk_class(sorted + lo, hi - lo, pick - lo, k, (int)bs1, (int)bs2, s_lane_base);
@@ -1598,12 +1638,12 @@ static __device__ __noinline__ bool topk_finish(const KParams& P, const Smem& S,
         }
         *O.id_out = col;
         if (want_lp) {
-            float log_prob = logf(s_e);
+            float log_prob = logf(val[pick]);  // (added by itself: fused with the logarithm's product or not would depend on the caller)
             if (P.cum_log_probs != nullptr) {
-                P.cum_log_probs[O.r] += log_prob;
+                P.cum_log_probs[O.r] = __fadd_rn(P.cum_log_probs[O.r], log_prob);
             }
             if (P.out_log_probs != nullptr) {
-                P.out_log_probs[O.r] = log_prob - logf(s_sum);
+                P.out_log_probs[O.r] = __fsub_rn(log_prob, logf(s_sum));
             }
         }
         write_lengths(P, O, col);
@@ -3160,7 +3200,7 @@ __device__ __noinline__ int row_topp_classes(const KParams& P, const Smem& S, co
         if (want_lp) {
             const float lprob = logf(p_sel);
             if (P.cum_log_probs != nullptr) {
-                P.cum_log_probs[O.r] += lprob;
+                P.cum_log_probs[O.r] = __fadd_rn(P.cum_log_probs[O.r], lprob);
             }
             if (P.out_log_probs != nullptr) {
                 P.out_log_probs[O.r] = lprob;
@@ -3338,7 +3378,7 @@ __device__ __noinline__ void row_softmax(const KParams& P, const Smem& S, const 
                 if (want_lp) {
                     float lprob = logf(p_max);
                     if (P.cum_log_probs != nullptr) {
-                        P.cum_log_probs[O.r] += lprob;
+                        P.cum_log_probs[O.r] = __fadd_rn(P.cum_log_probs[O.r], lprob);
                     }
                     if (P.out_log_probs != nullptr) {
                         P.out_log_probs[O.r] = lprob;
@@ -3762,7 +3802,7 @@ __device__ __noinline__ void row_softmax(const KParams& P, const Smem& S, const 
                 if (want_lp) {
                     float lprob = logf(fkey_inv(~(u32)(e >> 32)));
                     if (P.cum_log_probs != nullptr) {
-                        P.cum_log_probs[O.r] += lprob;
+                        P.cum_log_probs[O.r] = __fadd_rn(P.cum_log_probs[O.r], lprob);
                     }
                     if (P.out_log_probs != nullptr) {
                         P.out_log_probs[O.r] = lprob;
@@ -3841,7 +3881,7 @@ __device__ __forceinline__ void finished_topp_row(const KParams& P, const RowOut
         if (want_lp) {
             float lprob = logf(p0);
             if (P.cum_log_probs != nullptr) {
-                P.cum_log_probs[r] += lprob;
+                P.cum_log_probs[r] = __fadd_rn(P.cum_log_probs[r], lprob);
             }
             if (P.out_log_probs != nullptr) {
                 P.out_log_probs[r] = lprob;

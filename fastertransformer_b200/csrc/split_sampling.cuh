@@ -991,7 +991,7 @@ __device__ __forceinline__ void sp_write_topp(const KParams& P, const RowOut& O,
         if (want_lp) {
             const float lprob = logf(prob);
             if (P.cum_log_probs != nullptr) {
-                P.cum_log_probs[O.r] += lprob;
+                P.cum_log_probs[O.r] = __fadd_rn(P.cum_log_probs[O.r], lprob);
             }
             if (P.out_log_probs != nullptr) {
                 P.out_log_probs[O.r] = lprob;
