@@ -155,10 +155,10 @@ struct SpMap {
 
 struct SpShared {
     float wsum[32];        // warp sums of the soft-max denominator, written by all CTAs
-    u32   max_key[kSpMaxN];
+    u32   max_key;         // of the row's largest value
     u32   area_n;          // entries received
     u32   first_max;       // smallest column that holds the maximum
-    u32   best_tie;        // largest tie key of the columns that hold the maximum
+    u64   best[kSpMaxN * kWarps];  // arg-max rows, a warp each: key of its largest value << 32 | the largest tie key of its columns
     u32   n_cls;           // columns of the crossing class
     u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
     u32   p_sel, j_sel;    // crossing: probability (bits), position in the sorted order
@@ -339,21 +339,38 @@ __device__ __noinline__ void sp_chain_sums(const float* y, int nchunk, float max
     FTB_ASSUME_SHARED(y);
     const int tid = threadIdx.x, vt = 1 << lgvt;
     for (int t = tid; t < vt; t += kThreads) {
-        float a = 0.0f;
-        int   m = 0;
-        for (; m + 8 <= nchunk; m += 8) {
-            float e[8];
+        // the exponentials of the next eight chunks are on their way while those of the last eight are added
+        float       a   = 0.0f, e[8];
+        const int   m8  = nchunk & ~7;
+        const float* yt = y + t;
+        auto        eight = [&](int m, float* to) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                e[i] = round_to_T<DT>(__expf(y[((m + i) << lgvt) + t] - maxv));
+                to[i] = round_to_T<DT>(__expf(yt[(m + i) << lgvt] - maxv));
             }
+        };
+        if (m8 > 0) {
+            eight(0, e);
+        }
+#pragma unroll 1
+        for (int m = 8; m < m8; m += 8) {
+            float f[8];
+            eight(m, f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                a += e[i];
+                e[i] = f[i];
+            }
+        }
+        if (m8 > 0) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 a += e[i];
             }
         }
-        for (; m < nchunk; ++m) {
-            a += round_to_T<DT>(__expf(y[(m << lgvt) + t] - maxv));
+#pragma unroll 1
+        for (int m = m8; m < nchunk; ++m) {
+            a += round_to_T<DT>(__expf(yt[m << lgvt] - maxv));
         }
         // (vt is a multiple of 32: whole warps take part)
 #pragma unroll
@@ -744,29 +761,24 @@ static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* 
     return ok;
 }
 
-// First bin whose inclusive count reaches `want` (kSpBins - 1 when the total stays below) with, for half, a
-// probability at its far edge that cannot round to the one at `p_floor`.
-template<bool MIND_P>
-static __device__ int sp_bin_reaching(const u32* excl, u32 total, u32 want, float p_below, float inv_denom)
+// Half: first bin whose inclusive count reaches `want` (kSpBins - 1 when the total stays below) with a probability at its far
+// edge that cannot round to the one at `p_below`.
+static __device__ int sp_bin_below(const u32* excl, u32 total, u32 want, float p_below, float inv_denom)
 {
     __shared__ int s_b;
     constexpr int  PER = kSpBins / kThreads;
     const int      tid = threadIdx.x;
     FTB_ASSUME_SHARED(excl);
-    __syncthreads();
     if (tid == 0) {
         s_b = kSpBins - 1;
     }
     __syncthreads();
     int found = kSpBins;
+#pragma unroll
     for (int i = PER - 1; i >= 0; --i) {
         const int b    = tid * PER + i;
         const u32 incl = b + 1 < kSpBins ? excl[b + 1] : total;
-        bool      ok   = incl >= want;
-        if (MIND_P) {
-            ok = ok && __expf(-sp_edge(b)) * inv_denom <= p_below;
-        }
-        found = ok ? b : found;
+        found          = (incl >= want) & (__expf(-sp_edge(b)) * inv_denom <= p_below) ? b : found;
     }
     if (found < kSpBins) {
         atomicMin(&s_b, found);
@@ -1022,7 +1034,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     FTB_ASSUME_SHARED(smem);
     const SpMap      M = sp_map(A, smem);
     __shared__ float s_u, s_denom;
-    __shared__ u32   s_base1, s_cutbin;
+    __shared__ u32   s_base1;
     const int        tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     constexpr int    n = 1 << LGN, lgvt = 10 - LGN;
     const int        rank = (int)cluster_rank(), r = O.r;
@@ -1048,15 +1060,20 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     if (tid == 0) {
         X.area_n    = 0;
         X.first_max = 0xffffffffu;
-        X.best_tie  = 0;
         X.n_cls     = 0;
         X.larger    = 0;
         X.bad_order = 0;
-        curandState_t st = (mode == 1 ? P.topk_states : P.topp_states)[r];
-        s_u              = curand_uniform(&st);
+        X.max_key   = 0;
     }
     __syncthreads();
     cluster_arrive();  // this CTA's counters may be written by the others
+    // the row's arguments, sent for before the row so that nobody waits for them
+    const u32     k_row = mode == 1 ? P.topk_ks[r] : 0u;
+    const float   p_row = mode == 1 ? P.topk_ps[r] : P.topp_ps[r];
+    curandState_t draw;
+    if (tid == 0) {
+        draw = (mode == 1 ? P.topk_states : P.topp_states)[r];
+    }
     Xf X0;
     X0.bias       = P.bias;
     X0.apply_temp = P.apply_temp;
@@ -1074,6 +1091,9 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
         hist1                  = sp_history_id(P, col, input_len, (n + rank) * kThreads + tid);
     }
     sp_load_slice<DT>(P, X0, rowp, y, rank, lgvt, nchunk);
+    if (tid == 0) {
+        s_u = curand_uniform(&draw);
+    }
     trace_mark(O.trace, 0);
     cluster_wait();
     if (specials) {
@@ -1099,17 +1119,54 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
         const float4 v = *(const float4*)(y + i);
         best           = fmaxf(best, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
     }
-    {
-        const u32 k = (u32)block_max_u64((u64)(best > neg_max ? fkey(best) : 0u));
-        if (tid < n) {
-            dst_u32(cluster_addr(smem_addr(&X.max_key[rank]), (u32)tid), k);
+    const u32 warp_key = __reduce_max_sync(0xffffffffu, best > neg_max ? fkey(best) : 0u);
+    if (mode == 1 && !want_lp && k_row <= 1u) {
+        // ---- arg-max: value, then the reference's tie order (CTA lane and thread descending, column ascending).  Every warp
+        // looks for its own maximum's columns, so that one exchange brings the value and the tie together ----
+        const u32 bs1 = P.max_top_k <= 16 ? 128 : 256;
+        const int sh1 = bs1 == 128 ? 7 : 8;
+        u32       tie = 0;
+        if (warp_key != 0) {
+            sp_sweep(y, ny, fkey_inv(warp_key), [&](int i, float x) {
+                if (fkey(x) != warp_key) {
+                    return;  // (a zero of the other sign)
+                }
+                const u32 v = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
+                const u32 c = (((v >> sh1) & 7u) << 29) | ((v & (bs1 - 1)) << 21) | (0x1fffffu - v);
+                tie         = c > tie ? c : tie;
+            });
+            tie = __reduce_max_sync(0xffffffffu, tie);
         }
+        if (lane == 0) {
+            dst_u64(cluster_addr(smem_addr(&X.best[rank * kWarps + wid]), 0), ((u64)warp_key << 32) | tie);
+        }
+        cluster_sync();
+        trace_mark(O.trace, 2);
+        if (rank != 0) {
+            return true;
+        }
+        u64 b = 0;
+        for (int i = lane; i < n * kWarps; i += 32) {
+            const u64 w = X.best[i];
+            b           = w > b ? w : b;
+        }
+        b = warp_max_u64(b);
+        if (b != 0 && !(fkey_inv((u32)(b >> 32)) < INFINITY)) {
+            return sp_leave(O, 1);
+        }
+        if (tid == 0) {
+            // (nothing can be selected: token 0)
+            const int id = b != 0 ? (int)(0x1fffffu - ((u32)b & 0x1fffffu)) : 0;
+            *O.id_out    = id;
+            write_lengths(P, O, id);
+        }
+        return true;
+    }
+    if (lane < n) {
+        dred_max(cluster_addr(smem_addr(&X.max_key), (u32)lane), warp_key);
     }
     cluster_sync();
-    u32 kmax = 0;
-    for (int q = 0; q < n; ++q) {
-        kmax = X.max_key[q] > kmax ? X.max_key[q] : kmax;
-    }
+    const u32 kmax = X.max_key;
     trace_mark(O.trace, 2);
     const float u = s_u;
     if (kmax == 0) {
@@ -1123,31 +1180,6 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     const float maxv = fkey_inv(kmax);
     if (!(maxv < INFINITY)) {
         return sp_leave(O, 1);
-    }
-
-    if (mode == 1 && !want_lp && P.topk_ks[r] <= 1u) {
-        // ---- arg-max: value, then the reference's tie order (CTA lane and thread descending, column ascending) ----
-        const u32 bs1 = P.max_top_k <= 16 ? 128 : 256;
-        const int sh1 = bs1 == 128 ? 7 : 8;
-        u32       tie = 0;
-        sp_sweep(y, ny, maxv, [&](int i, float x) {
-            if (fkey(x) != kmax) {
-                return;  // (a zero of the other sign)
-            }
-            const u32 v = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
-            const u32 c = (((v >> sh1) & 7u) << 29) | ((v & (bs1 - 1)) << 21) | (0x1fffffu - v);
-            tie         = c > tie ? c : tie;
-        });
-        if (tie != 0) {
-            dred_max(cluster_addr(smem_addr(&X.best_tie), 0), tie);
-        }
-        cluster_sync();
-        if (rank == 0 && tid == 0) {
-            const int id = (int)(0x1fffffu - (X.best_tie & 0x1fffffu));
-            *O.id_out    = id;
-            write_lengths(P, O, id);
-        }
-        return true;
     }
 
     // ---- counts per bin; for a soft-max row the ordered denominator ----
@@ -1200,99 +1232,144 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     if (softmax && !(denom > 0.0f && denom < INFINITY)) {
         return sp_leave(O, 2);
     }
-    constexpr int PER = kSpBins / kThreads;
-    u32           total;
-    float         mass = 0.0f;  // lower bound of this thread's bins' probability (top-p rows)
-    {
-        u32 c[PER], mine = 0;
-        const float scale = 0.99f / denom;
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const int b = tid * PER + i;
-            c[i]        = M.merged[b];
-            mine += c[i];
-            if (mode == 2 && c[i] != 0 && b + 1 < kSpBins) {
-                mass += (float)c[i] * __expf(-sp_edge(b + 1)) * scale;
-            }
-        }
-        u32 run = block_excl_u32(mine, &total);
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            M.merged[tid * PER + i] = run;
-            run += c[i];
-        }
-    }
-    __syncthreads();
     u32* const excl = M.merged;
-
-    trace_mark(O.trace, 6);
-    // ---- how far down the selection can reach: every column of bins 0 .. b_thr takes part ----
-    int         k = 1, b_thr;
-    float       rand_num = 0.0f;
-    if (mode == 1) {
-        k     = (int)P.topk_ks[r];
-        k     = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
-        b_thr = sp_bin_reaching<false>(excl, total, (u32)k, 0.0f, 0.0f);
-        if (want_lp) {
-            // equal probabilities may lie in different bins: a few more columns, so that the k-th is not in the last class
-            const u32 incl = b_thr + 1 < kSpBins ? excl[b_thr + 1] : total;
-            b_thr          = sp_bin_reaching<false>(excl, total, incl + 32u, 0.0f, 0.0f);
-        }
-    }
-    else {
-    const float top_p = P.topp_ps[r];
-    const float p_max = round_to_T<DT>(round_to_T<DT>(1.0f) / denom);
-    if (p_max >= top_p) {
-        // arg-max shortcut of topp_beam_topk_kernel (sampling_topp_kernels.cu:801-860): first column of the maximum
-        u32 col = 0xffffffffu;
-        sp_sweep(y, ny, maxv, [&](int i, float v) {
-            if (v == maxv) {
-                const u32 c = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
-                col         = c < col ? c : col;
+    if (mode == 2) {
+        const float p_max = round_to_T<DT>(round_to_T<DT>(1.0f) / denom);
+        if (p_max >= p_row) {
+            // arg-max shortcut of topp_beam_topk_kernel (sampling_topp_kernels.cu:801-860): first column of the maximum
+            u32 col = 0xffffffffu;
+            sp_sweep(y, ny, maxv, [&](int i, float v) {
+                if (v == maxv) {
+                    const u32 c = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
+                    col         = c < col ? c : col;
+                }
+            });
+            if (col != 0xffffffffu) {
+                dred_min(cluster_addr(smem_addr(&X.first_max), 0), col);
             }
-        });
-        if (col != 0xffffffffu) {
-            dred_min(cluster_addr(smem_addr(&X.first_max), 0), col);
+            cluster_sync();
+            if (rank == 0 && tid == 0) {
+                sp_write_topp<DT>(P, O, (int)X.first_max, p_max, true, want_lp);
+            }
+            return true;
         }
-        cluster_sync();
-        if (rank == 0 && tid == 0) {
-            sp_write_topp<DT>(P, O, (int)X.first_max, p_max, true, want_lp);
-        }
-        return true;
     }
-    rand_num = u * top_p;
+
+    // ---- first position of every bin in the row's order, and how far down the selection can reach: every column of bins
+    // 0 .. b_thr takes part.  A thread holds eight bins: who holds the wanted one says so, and nobody else looks ----
+    constexpr int    PER      = kSpBins / kThreads;
+    const int        k        = mode == 1 ? ((int)k_row < 1 ? 1 : ((int)k_row > kMaxTopK ? kMaxTopK : (int)k_row)) : 1;
+    const float      rand_num = mode == 2 ? u * p_row : 0.0f;
+    __shared__ uint4 s_wcnt[kWarps / 4];
+    __shared__ float4 s_wmass[kWarps / 4];
+    __shared__ u32   s_cutbin, s_thr;
+    u32              total, run, mine = 0, c[PER];
     {
-        // first bin down to which the lower bound of the mass covers the draw
-        __shared__ float s_mw[kWarps];
-        float            incl = mass;
+        const uint4 m0 = ((const uint4*)M.merged)[2 * tid], m1 = ((const uint4*)M.merged)[2 * tid + 1];
+        c[0] = m0.x, c[1] = m0.y, c[2] = m0.z, c[3] = m0.w, c[4] = m1.x, c[5] = m1.y, c[6] = m1.z, c[7] = m1.w;
+        float mass = 0.0f;  // lower bound of this thread's bins' probability (top-p rows)
+        if (mode == 2) {
+            const float scale = 0.99f / denom;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int b = tid * PER + i;
+                if (c[i] != 0 && b + 1 < kSpBins) {
+                    mass += (float)c[i] * __expf(-sp_edge(b + 1)) * scale;
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            mine += c[i];
+        }
+        u32   incl  = mine;
+        float mincl = mass;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const float t = __shfl_up_sync(0xffffffffu, incl, off);
-            incl += lane >= off ? t : 0.0f;
+            const u32   t = __shfl_up_sync(0xffffffffu, incl, off);
+            const float f = __shfl_up_sync(0xffffffffu, mincl, off);
+            incl += lane >= off ? t : 0u;
+            mincl += lane >= off ? f : 0.0f;
         }
         if (lane == 31) {
-            s_mw[wid] = incl;
+            ((u32*)s_wcnt)[wid]    = incl;
+            ((float*)s_wmass)[wid] = mincl;
         }
         if (tid == 0) {
             s_cutbin = kSpBins - 1;
+            s_thr    = kSpBins - 1;
         }
         __syncthreads();
-        float base = 0.0f;
-        for (int i = 0; i < wid; ++i) {
-            base += s_mw[i];
+        u32   base = 0;
+        float mbase = 0.0f;
+        total       = 0;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) {
+            const u32 w = ((const u32*)s_wcnt)[i];
+            base += i < wid ? w : 0u;
+            total += w;
+            mbase += i < wid ? ((const float*)s_wmass)[i] : 0.0f;
         }
-        if (base + incl >= rand_num) {
-            // (the bin inside the thread's eight is not looked for: the last of them is taken)
+        run = base + incl - mine;
+        uint4 e0, e1;
+        e0.x = run, e0.y = e0.x + c[0], e0.z = e0.y + c[1], e0.w = e0.z + c[2];
+        e1.x = e0.w + c[3], e1.y = e1.x + c[4], e1.z = e1.y + c[5], e1.w = e1.z + c[6];
+        ((uint4*)M.merged)[2 * tid]     = e0;
+        ((uint4*)M.merged)[2 * tid + 1] = e1;
+        if (mode == 2 && mbase + mincl >= rand_num) {
+            // first bins down to which the lower bound of the mass covers the draw (the bin inside the thread's eight is not
+            // looked for: the last of them is taken)
             atomicMin(&s_cutbin, (u32)(tid * PER + PER - 1));
         }
-        __syncthreads();
+    }
+    // the bin whose inclusive count reaches `want` first
+    auto reaching = [&](u32 want) {
+        if (run < want && run + mine >= want) {
+            u32 r = run;
+            int b = tid * PER;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                r += c[i];
+                b += r < want ? 1 : 0;
+            }
+            s_thr = (u32)b;
+        }
+    };
+    if (mode == 1) {
+        reaching((u32)k);
+    }
+    __syncthreads();
+    trace_mark(O.trace, 6);
+    int b_thr;
+    if (mode == 1) {
+        b_thr = (int)s_thr;
+        if (want_lp) {
+            // equal probabilities may lie in different bins: a few more columns, so that the k-th is not in the last class
+            const u32 incl = b_thr + 1 < kSpBins ? excl[b_thr + 1] : total;
+            __syncthreads();
+            if (tid == 0) {
+                s_thr = kSpBins - 1;
+            }
+            __syncthreads();
+            reaching(incl + 32u);
+            __syncthreads();
+            b_thr = (int)s_thr;
+        }
+    }
+    else {
         const int b_star = (int)s_cutbin;
         // at least 64 columns more: the scan reads 32 entries past the crossing, and the crossing must not fall into
         // the lowest collected class; half-precision probabilities are equal over several bins
-        const u32   have = b_star + 1 < kSpBins ? excl[b_star + 1] : total;
-        const float p_at = __expf(-sp_edge(b_star + 1)) / denom;
-        b_thr = sp_bin_reaching<DT == FTB200_F16>(excl, total, have + 64u, p_at * (1.0f - 1.0f / 512.0f) - 1.3e-7f, 1.0f / denom);
-    }
+        const u32 have = b_star + 1 < kSpBins ? excl[b_star + 1] : total;
+        if (DT == FTB200_F16) {
+            const float p_at = __expf(-sp_edge(b_star + 1)) / denom;
+            b_thr            = sp_bin_below(excl, total, have + 64u, p_at * (1.0f - 1.0f / 512.0f) - 1.3e-7f, 1.0f / denom);
+        }
+        else {
+            reaching(have + 64u);
+            __syncthreads();
+            b_thr = (int)s_thr;
+        }
     }
     const bool complete = b_thr == kSpBins - 1;
     const u32  N        = complete ? total : excl[b_thr + 1];
@@ -1365,7 +1442,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
         }
         __syncthreads();
         if (!softmax) {
-            return topk_finish(P, S, O, sorted, n_cand, k, u, P.topk_ps[r], true, false);
+            return topk_finish(P, S, O, sorted, n_cand, k, u, p_row, true, false);
         }
         // values -> probabilities; their order has to be that of the values
         float* const pr  = (float*)M.merged;
@@ -1384,7 +1461,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
             return sp_leave(O, 3);
         }
         if (mode == 1) {
-            return topk_finish(P, S, O, sorted, n_cand, k, u, P.topk_ps[r], false, true, !complete);
+            return topk_finish(P, S, O, sorted, n_cand, k, u, p_row, false, true, !complete);
         }
         __shared__ SpKeys s_K1;
         __shared__ u32    s_res[3];
