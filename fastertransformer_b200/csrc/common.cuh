@@ -113,6 +113,29 @@ __device__ __forceinline__ void sts_u16(u32 a, u32 v)
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
 }
 
+// A launch whose blocks may come up while the kernel in front of it in the stream drains; the kernel calls
+// wait_for_previous() before it touches memory, which returns when that one has ended.  Hides the launch of a short kernel
+// (steps follow each other in a stream: 1 to 2 us each).
+template<class... P, class... A>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    cudaLaunchConfig_t  cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim          = grid;
+    cfg.blockDim         = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream           = st;
+    cfg.attrs            = attr;
+    cfg.numAttrs         = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void wait_for_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Tells the compiler that a pointer loaded from a structure points into shared memory, so that it emits
 // ld.shared / st.shared instead of generic accesses (every pointer of the kernel's shared-memory map qualifies).
 #define FTB_ASSUME_SHARED(p) __builtin_assume(__isShared(p))

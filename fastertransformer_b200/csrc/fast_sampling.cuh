@@ -2170,6 +2170,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
 template<int DT, bool TOPP, int VP = 0>
 __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(const __grid_constant__ KParams P)
 {
+    asm volatile("griddepcontrol.launch_dependents;");  // (the kernel that serves the rows left here waits for this grid's end)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FHdr                               s_hdr[2];
     __shared__ __align__(16) u32                  s_pre[kFPreWords];

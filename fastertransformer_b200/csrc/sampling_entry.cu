@@ -37,10 +37,10 @@ extern template int fast_sampling_occupancy<FTB200_BF16, true>(size_t, int*);
 extern template int fast_sampling_launch<FTB200_F16, true>(const KParams&, int, size_t, cudaStream_t);
 extern template int fast_sampling_launch<FTB200_BF16, true>(const KParams&, int, size_t, cudaStream_t);
 template<int DT>
-int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_general, cudaStream_t st);
-extern template int split_sampling_launch<FTB200_F32>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
-extern template int split_sampling_launch<FTB200_F16>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
-extern template int split_sampling_launch<FTB200_BF16>(const KParams&, const SplitArgs&, size_t, cudaStream_t);
+int split_sampling_launch(const KParams& K, const SplitArgs& A, cudaStream_t st);
+extern template int split_sampling_launch<FTB200_F32>(const KParams&, const SplitArgs&, cudaStream_t);
+extern template int split_sampling_launch<FTB200_F16>(const KParams&, const SplitArgs&, cudaStream_t);
+extern template int split_sampling_launch<FTB200_BF16>(const KParams&, const SplitArgs&, cudaStream_t);
 template<int DT>
 int split_resident(int lgn, bool whole, size_t smem);
 extern template int split_resident<FTB200_F32>(int, bool, size_t);
@@ -109,7 +109,7 @@ static int resident_clusters(int dtype, int lgn, bool whole, size_t smem)
     }
 }
 
-constexpr size_t kWholeTwoPerSm = 103 * 1024, kTwoPerSm = 107 * 1024 + 512, kThreePerSm = 69 * 1024;
+constexpr size_t kRoomyTwoPerSm = 103 * 1024, kTwoPerSm = 107 * 1024 + 512, kThreePerSm = 69 * 1024;
 
 // Whether the split kernel (a row over a cluster of CTAs) serves a call, and in which form.  `single_pass`: the
 // single-pass kernels could serve it too.  The lines come from timing both at 17000 .. 250000 columns and 6 .. 1024
@@ -123,8 +123,7 @@ constexpr size_t kWholeTwoPerSm = 103 * 1024, kTwoPerSm = 107 * 1024 + 512, kThr
 // 32000 71 / 64), with four a third more may wait (64 x 51200 51 / 68, 80 x 51200 66 / 69, 96 x 41000 75 / 77, 112 x 51200
 // 75 / 71), with eight, whose rows take one CTA longest, two rounds of them and more above 110000 columns (64 x 80000 81 / 80,
 // 80 x 80000 100 / 83, 80 x 100000 123 / 111; 64 x 128256 99 / 113, 80 x 128256 117 / 114).
-static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool single_pass, size_t smem_general,
-                         SplitArgs* A, bool* whole)
+static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool single_pass, SplitArgs* A)
 {
     const int rows = p->local_batch_size, vocab = p->vocab_size, sms = sm_count();
     if (vocab < 1024) {
@@ -160,7 +159,7 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
             return false;
         }
     }
-    // The form that keeps every row is taken while its clusters are resident at once, with two CTAs on an SM where shared
+    // The roomy form is taken while its clusters are resident at once, with two CTAs on an SM where shared
     // memory allows (16 x 128256 bf16, one CTA on an SM: k = 50 60 us a step, 46 in the other form; 14 rows 39 / 45).  The
     // collection areas: a wide nucleus of a flat row takes half of the columns, so up to 5/8 of a slice is
     // provided for as far as that residency holds (a row beyond it costs milliseconds in the general code).
@@ -174,12 +173,11 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     };
     const int  ctas  = rows << lgn;
     const auto keeps = [&](int per_sm, size_t budget) {
-        A->area           = area_within(budget, kSpAreaMax);
-        const size_t smem = split_smem_bytes(A->slice, A->area);
-        return mixed || few ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, smem > smem_general ? smem : smem_general);
+        A->area = area_within(budget, kSpAreaMax);
+        return mixed || few ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, split_smem_bytes(A->slice, A->area));
     };
-    *whole = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kWholeTwoPerSm && smem_general <= kWholeTwoPerSm && keeps(2, kWholeTwoPerSm)));
-    if (!*whole) {
+    A->roomy = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kRoomyTwoPerSm && keeps(2, kRoomyTwoPerSm)));
+    if (!A->roomy) {
         A->area = area_within(least <= kThreePerSm ? kThreePerSm : (least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem), kSpAreaMid);
     }
     return true;
@@ -189,6 +187,7 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
 static bool wide_areas(int vocab, SplitArgs* A)
 {
     A->lgn   = 3;
+    A->roomy = 1;
     A->slice = ((vocab + 1023) / 1024) << 7;
     A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
     A->area  = kSpAreaMax;
@@ -388,6 +387,7 @@ static int plan_sampling(const ftb200_sampling_params* p, KParams& K, size_t& sm
     K.redo_rows      = nullptr;
     K.row_count_dev  = nullptr;
     K.row_flags      = nullptr;
+    K.early          = 0;
     K.scratch        = (u64*)((char*)p->workspace + 256 + redo_list_bytes(p->local_batch_size));
     K.scratch_stride = scratch_stride_for(p->vocab_size_padded);
     return FTB200_OK;
@@ -402,8 +402,9 @@ extern "C" int ftb200_set_row_trace(uint64_t* device_buf)
 // One fused step.  `fork` allows the second stream of the single-pass kernels (made on first use); without it
 // the same kernels run one after the other on the caller's stream and nothing is created.
 namespace ftb200 {
+// left_only: the rows that the split kernel of the same step has flagged, by the general kernel.
 int decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop = nullptr,
-                              bool* stop_done = nullptr);
+                              bool* stop_done = nullptr, bool left_only = false);
 int stop_criteria_launch(const ftb200_sampling_params* p, const StopArgs& T, cudaStream_t st);
 }
 
@@ -443,6 +444,18 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     for (u32 spin = 1;; ++spin) {
         const u64 v = *w;
         if ((u32)(v >> 32) == T.sequence) {
+            if ((u32)v == kRowsLeft) {
+                // rare: rows that the split kernel's tables could not hold, then the criteria over the whole call
+                T.sequence = ++s->sequence;
+                rc         = decode_step_sampling_impl(p, true, nullptr, nullptr, true);
+                if (rc == FTB200_OK) {
+                    rc = stop_criteria_launch(p, T, (cudaStream_t)p->stream);
+                }
+                if (rc != FTB200_OK) {
+                    return rc;
+                }
+                continue;
+            }
             *should_stop = (u32)v == (u32)p->batch_size ? 1 : 0;
             return FTB200_OK;
         }
@@ -461,9 +474,12 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     }
 }
 
-int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop, bool* stop_done)
+int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop, bool* stop_done,
+                                      bool left_only)
 {
-    reset_launch_count();
+    if (!left_only) {
+        reset_launch_count();
+    }
     KParams K;
     size_t  smem = 0;
     int     grid = 0;
@@ -482,18 +498,20 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
                              && p->vocab_size >= 16384 + 16 && (K.apply_rep ? p->step : 0) <= fast_max_history()
                              && (K.bad_words != nullptr ? K.bad_words_len : 0) <= fast_max_words();
     SplitArgs A{};
-    bool      whole = false;
-    if (g_fast_path && choose_split(p, K, single_pass, smem, &A, &whole)) {
-        A.redo_flags = whole ? nullptr : (int*)((char*)p->workspace + 256);
-        if (whole && stop != nullptr) {
+    if (left_only) {
+        K.row_flags = (int*)((char*)p->workspace + 256);  // (as the split kernel of this step has set them)
+    }
+    else if (g_fast_path && choose_split(p, K, single_pass, &A)) {
+        A.redo_flags = (int*)((char*)p->workspace + 256);
+        if (A.roomy && stop != nullptr && stop->limit != nullptr) {
             A.stop     = *stop;
             *stop_done = true;
         }
         const auto launch = [&](const SplitArgs& args) {
             switch (p->dtype) {
-                case FTB200_F32: return split_sampling_launch<FTB200_F32>(K, args, smem, st);
-                case FTB200_F16: return split_sampling_launch<FTB200_F16>(K, args, smem, st);
-                default: return split_sampling_launch<FTB200_BF16>(K, args, smem, st);
+                case FTB200_F32: return split_sampling_launch<FTB200_F32>(K, args, st);
+                case FTB200_F16: return split_sampling_launch<FTB200_F16>(K, args, st);
+                default: return split_sampling_launch<FTB200_BF16>(K, args, st);
             }
         };
         rc = launch(A);
@@ -501,21 +519,20 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
             return rc;
         }
         note_launch(1);
-        if (whole) {
-            return FTB200_OK;
+        if (A.stop.limit != nullptr) {
+            return FTB200_OK;  // (the host hears of rows that are left and asks for them)
         }
         // Areas below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row) leave the flat
         // rows' wide nuclei: those go over eight CTAs with areas as large as shared memory allows.  Where these are below half
         // a slice too (above 163000 columns) the general kernel's many CTAs serve the several rows left sooner.
         SplitArgs B = A;
-        if (wide_areas(p->vocab_size, &B) && smem <= kSpMaxSmem && K.topp_states != nullptr && A.area < A.slice / 2
-            && B.area >= B.slice / 2) {
+        if (wide_areas(p->vocab_size, &B) && K.topp_states != nullptr && A.area < A.slice / 2 && B.area >= B.slice / 2) {
             B.clusters = sm_count() / kSpMaxN < p->local_batch_size ? sm_count() / kSpMaxN : p->local_batch_size;
             rc         = launch(B);
-            if (rc == FTB200_OK) {
-                note_launch(1);
+            if (rc != FTB200_OK) {
+                return rc;
             }
-            return rc;
+            note_launch(1);
         }
         K.row_flags = A.redo_flags;
     }
@@ -587,6 +604,7 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
             K.ticket        = K.ticket + 2;
             K.row_order     = F.redo_rows;
             K.row_count_dev = F.redo_count;
+            K.early         = side == nullptr && (topp_only || K.topp_states == nullptr);  // (one kernel in front, in this stream)
             if (K.trace != nullptr) {
                 K.trace += (size_t)p->local_batch_size * 32;  // the general kernel's records follow the single-pass kernel's
             }

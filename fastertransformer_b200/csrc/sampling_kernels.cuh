@@ -1095,7 +1095,7 @@ static __device__ __noinline__ int resolve_topk_class(u64* cls, int m, int want,
     }
     if (m <= 2 * kThreads) {
         // both orders by counting: two passes of m reads that all lanes share, where two sorting networks of 64 to 512 entries
-        // take 21 to 45 barriers each (k = 1024 with its class, one row: 21 us before, 14 now)
+        // take 21 to 45 barriers each (m = 150, one row: 2 us for 5 us)
         auto key_of = [&](u32 col) { return ((u64)((col / bs1) & 7u) << 56) | ((u64)(bs1 - 1 - (int)(col % bs1)) << 40) | col; };
         u64  key1[2];
         u32  key2[2];
@@ -1643,7 +1643,7 @@ static __device__ __noinline__ bool topk_finish(const KParams& P, const Smem& S,
                 P.cum_log_probs[O.r] = __fadd_rn(P.cum_log_probs[O.r], log_prob);
             }
             if (P.out_log_probs != nullptr) {
-                P.out_log_probs[O.r] = __fsub_rn(log_prob, logf(s_sum));
+                P.out_log_probs[O.r] = log_prob - logf(s_sum);
             }
         }
         write_lengths(P, O, col);
@@ -4034,16 +4034,18 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
     if (threadIdx.x == 0) {
         map_general_smem(P, S, smem_raw);
     }
+    // (launched while the kernel whose rows it may get still runs, see sampling_launch: flags and list are there when that has ended)
+    wait_for_previous();
     u64* gscratch = P.scratch + (size_t)blockIdx.x * P.scratch_stride;
     // rows to serve: the whole local batch, or the list the single-pass kernel left behind
-    const int n_rows = P.row_count_dev != nullptr ? (int)*P.row_count_dev : P.local_batch;
+    const int n_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
     for (int next = blockIdx.x;; next += gridDim.x) {
         __syncthreads();
         int t;
         if (P.row_flags != nullptr) {
             // the rows the split kernel left (normally none): no ticket, every CTA looks through its share
             t = next;
-            if (t < n_rows && P.row_flags[P.row_order != nullptr ? P.row_order[t] : t] == 0) {
+            if (t < n_rows && __ldcg(P.row_flags + (P.row_order != nullptr ? P.row_order[t] : t)) == 0) {
                 continue;
             }
         }
@@ -4328,6 +4330,7 @@ template<int DT>
 __global__ void __launch_bounds__(kThreads, 4)
 vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nranks, int* overflow, int area)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float                              s_u;
     __shared__ u32                                s_n, s_bound, s_bad, s_short;
@@ -4464,7 +4467,7 @@ int vp_merge_launch(const KParams& K, const u64* gathered, int nranks, int* over
     constexpr int kMostSmem = kCap * 8 + kNB * 4 + 1024 * 4;
     static std::atomic<bool> ready[kDevicesKnown];
     FTB_CUDA_CHECK(opt_in_smem(vp_merge_kernel<DT>, kMostSmem, ready));
-    vp_merge_kernel<DT><<<grid, kThreads, smem, st>>>(K, gathered, nranks, overflow, area);
+    FTB_CUDA_CHECK(launch_early(vp_merge_kernel<DT>, dim3((unsigned)grid), dim3(kThreads), smem, st, K, gathered, nranks, overflow, area));
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
 }
@@ -4513,6 +4516,11 @@ int sampling_occupancy(size_t smem, int* per_sm)
 template<int DT>
 int sampling_launch(const KParams& K, int grid, size_t smem, cudaStream_t st)
 {
+    if (K.row_flags != nullptr || K.early) {
+        // behind the split kernel or one single-pass kernel: comes up while that one drains (normally it finds no row)
+        FTB_CUDA_CHECK(launch_early(decode_sampling_kernel<DT>, dim3((unsigned)grid), dim3(kThreads), smem, st, K));
+        return FTB200_OK;
+    }
     decode_sampling_kernel<DT><<<grid, kThreads, smem, st>>>(K);
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;

@@ -13,11 +13,14 @@ constexpr int kSpMaxN     = 8;                       // portable cluster size
 constexpr size_t kSpMaxSmem = 216 * 1024;
 constexpr int kSpMinSlice = (kNB * 4 + 1024 * 4) / 4;  // the draw's histogram and values lie over the slice
 
+// Low word of a result that says: rows are left, and nothing has been counted (more rows than any batch has).
+constexpr u32 kRowsLeft = 0xffffffffu;
+
 // Stop criteria of the step, for the launch forms that finish everything themselves.
 struct StopArgs {
     const int*      stop_words;      // [local_batch, 2, stop_words_len] or null
     int             stop_words_len;
-    const uint32_t* limit;           // [batch_size] or null: then nothing is counted
+    const uint32_t* limit;           // [batch_size] or null: then the criteria have a launch of their own
     uint8_t*        finished;        // [batch_size], the whole batch
     u32*            arrived;         // one word, zero between calls
     u64*            result;          // page-locked host word: sequence << 32 | finished rows
@@ -28,9 +31,10 @@ struct SplitArgs {
     int  lgn;         // log2 of the CTAs per row
     int  slice;       // floats of the slice area
     int  area;        // keys of the collection area
-    int* redo_flags;  // [local_batch]: 1 when the row is left to decode_sampling_kernel (null: the kernel serves it itself)
-    StopArgs stop;    // (only where redo_flags is null)
-    int  clusters;    // 0: one per row; else so many, which look for rows with redo_flags set and serve those
+    int  roomy;       // the form with 128 registers
+    int* redo_flags;  // [local_batch]: 1 when the row is left to another launch
+    StopArgs stop;    // (roomy form; without a limit nothing is done for the criteria)
+    int  clusters;    // 0: one per row; else so many, which look for rows with redo_flags set and serve those (roomy form)
 };
 
 __host__ __device__ inline size_t split_smem_bytes(int slice, int area)

@@ -156,7 +156,6 @@ struct SpMap {
 struct SpShared {
     float wsum[32];        // warp sums of the soft-max denominator, written by all CTAs
     u32   max_key;         // of the row's largest value
-    u32   area_n;          // entries received
     u32   first_max;       // smallest column that holds the maximum
     u64   best[kSpMaxN * kWarps];  // arg-max rows, a warp each: key of its largest value << 32 | the largest tie key of its columns
     u32   n_cls;           // columns of the crossing class
@@ -179,16 +178,18 @@ __device__ __forceinline__ u32 sp_add_bias(u32 x, u32 b)
     return __float_as_uint(__uint_as_float(x) + __uint_as_float(b));
 }
 
-// Loads this CTA's columns of row r and stores their values after temperature and bias.
+// Loads this CTA's columns of row r and stores their values after temperature and bias.  Returns the thread's largest.
 template<int DT>
-__device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, const char* rowp, float* y, int rank, int lgvt,
+__device__ __forceinline__ float sp_load_slice(const KParams& P, const Xf& X, const char* rowp, float* y, int rank, int lgvt,
                                               int nchunk)
 {
     constexpr int ES = DT == FTB200_F32 ? 4 : 2, EPV = 16 / ES, LGE = DT == FTB200_F32 ? 2 : 3;
     const int     tid = threadIdx.x, vt = 1 << lgvt, col0 = rank << lgvt, vocab = P.vocab;
+    float         best = -INFINITY;
     if (((size_t)rowp & 15) == 0 && lgvt >= LGE) {
-        // a chunk of 1024 columns starts on a 16-byte boundary: whole vectors, four in flight per thread
-        constexpr int U   = 4;
+        // a chunk of 1024 columns starts on a 16-byte boundary: whole vectors, eight in flight per thread (a slice of 16000
+        // half-precision columns in one round)
+        constexpr int U   = 8;
         const int     lgv = lgvt - LGE, nv = nchunk << lgv;
         const bool    bias = X.apply_temp && X.bias != nullptr, bias_vec = DT != FTB200_BF16 && bias && ((size_t)X.bias & 15) == 0;
         Xf            T    = X;  // (a bias that comes by the vector is added here)
@@ -235,6 +236,7 @@ __device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, con
 #pragma unroll
                 for (int e = 0; e < EPV; e += 4) {
                     dst[e / 4] = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+                    best       = fmaxf(best, fmaxf(fmaxf(f[e], f[e + 1]), fmaxf(f[e + 2], f[e + 3])));
                 }
             }
         }
@@ -258,10 +260,12 @@ __device__ __forceinline__ void sp_load_slice(const KParams& P, const Xf& X, con
                 const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
                 if (i < ny) {
                     y[i] = v < vocab ? temp_value<DT>(X, q[u], v) : -INFINITY;
+                    best = fmaxf(best, y[i]);
                 }
             }
         }
     }
+    return best;
 }
 
 // History ids of the row that this CTA looks after, kHistRegs per thread: loaded before the row itself so that they are
@@ -941,50 +945,6 @@ static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float
     return 0;
 }
 
-// The leader's candidates (~key << 32 | column) into order.  The bins of the row are already counted: an entry goes to
-// its bin's range of the sorted list, and its place inside the range is the number of smaller entries there, a handful
-// unless many columns are equal.  Three barriers, where a sorting network takes tens.  `bin_of` gives an entry's bin.
-// Returns the sorted list (the second half of the candidate area); `excl` is used up.
-template<class B>
-static __device__ __forceinline__ u64* sp_bucket_sort(u64* cand, u32* excl, int n, u64* tmp, u64* dst, B&& bin_of)
-{
-    FTB_ASSUME_SHARED(cand);
-    FTB_ASSUME_SHARED(tmp);
-    FTB_ASSUME_SHARED(dst);
-    const int tid = threadIdx.x;
-    if (n <= 128) {
-        for (int i = tid; i < n; i += kThreads) {
-            const u64 e  = cand[i];
-            int       rk = 0;
-#pragma unroll 8
-            for (int j = 0; j < n; ++j) {
-                rk += cand[j] < e ? 1 : 0;
-            }
-            dst[rk] = e;
-        }
-        __syncthreads();
-        return dst;
-    }
-    for (int i = tid; i < n; i += kThreads) {
-        const u64 e                            = cand[i];
-        tmp[atomicAdd(&excl[bin_of(e)], 1u)] = e;  // the cursor of bin b ends at the start of bin b + 1
-    }
-    __syncthreads();
-    for (int i = tid; i < n; i += kThreads) {
-        const u64 e  = tmp[i];
-        const int b  = bin_of(e);
-        const int lo = b > 0 ? (int)excl[b - 1] : 0, hi = (int)excl[b];
-        int       rk = lo;
-#pragma unroll 4
-        for (int j = lo; j < hi; ++j) {
-            rk += tmp[j] < e ? 1 : 0;
-        }
-        dst[rk] = e;
-    }
-    __syncthreads();
-    return dst;
-}
-
 // Note of why a row is left to decode_sampling_kernel (word 25 of its trace record).
 __device__ __forceinline__ bool sp_leave(const RowOut& O, int why)
 {
@@ -1034,7 +994,6 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     FTB_ASSUME_SHARED(smem);
     const SpMap      M = sp_map(A, smem);
     __shared__ float s_u, s_denom;
-    __shared__ u32   s_base1;
     const int        tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     constexpr int    n = 1 << LGN, lgvt = 10 - LGN;
     const int        rank = (int)cluster_rank(), r = O.r;
@@ -1058,7 +1017,6 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
         }
     }
     if (tid == 0) {
-        X.area_n    = 0;
         X.first_max = 0xffffffffu;
         X.n_cls     = 0;
         X.larger    = 0;
@@ -1090,7 +1048,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
         hist0                  = sp_history_id(P, col, input_len, rank * kThreads + tid);
         hist1                  = sp_history_id(P, col, input_len, (n + rank) * kThreads + tid);
     }
-    sp_load_slice<DT>(P, X0, rowp, y, rank, lgvt, nchunk);
+    float best = sp_load_slice<DT>(P, X0, rowp, y, rank, lgvt, nchunk);
     if (tid == 0) {
         s_u = curand_uniform(&draw);
     }
@@ -1114,13 +1072,17 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
 
     // ---- row maximum ----
     trace_mark(O.trace, 1);
-    float best = -INFINITY;
-    for (int i = 4 * tid; i < ny; i += 4 * kThreads) {
-        const float4 v = *(const float4*)(y + i);
-        best           = fmaxf(best, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+    const bool arg_max = mode == 1 && !want_lp && k_row <= 1u;
+    if (specials || arg_max) {
+        // (some values have changed since they came in; an arg-max row wants the maximum of what each warp walks over below)
+        best = -INFINITY;
+        for (int i = 4 * tid; i < ny; i += 4 * kThreads) {
+            const float4 v = *(const float4*)(y + i);
+            best           = fmaxf(best, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+        }
     }
     const u32 warp_key = __reduce_max_sync(0xffffffffu, best > neg_max ? fkey(best) : 0u);
-    if (mode == 1 && !want_lp && k_row <= 1u) {
+    if (arg_max) {
         // ---- arg-max: value, then the reference's tie order (CTA lane and thread descending, column ascending).  Every warp
         // looks for its own maximum's columns, so that one exchange brings the value and the tie together ----
         const u32 bs1 = P.max_top_k <= 16 ? 128 : 256;
@@ -1204,10 +1166,8 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
             }
 #pragma unroll
             for (int q = 0; q < n; ++q) {
-                // (a nucleus is placed by bin: what the CTAs before this one have of the bin goes where its count stood)
-                if (mode == 2) {
-                    dst_u32(cluster_addr(a, (u32)q), sum);
-                }
+                // (what is selected is placed by bin: what the CTAs before this one have of the bin goes where its count stood)
+                dst_u32(cluster_addr(a, (u32)q), sum);
                 sum += part[q];
             }
 #pragma unroll
@@ -1376,69 +1336,77 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     trace_mark(O.trace, 9);
 
     if (N <= (u32)kSpCandCap) {
-        // ---- few candidates: the leader gets them all and finishes the row alone ----
-        // (a thread meets few candidates: the first four are remembered, more make it walk again)
-        u32         mine = 0, tot;
-        u64         keep0 = 0, keep1 = 0, keep2 = 0, keep3 = 0;
-        const float thr  = fmaxf(sp_floor_value(maxv, b_thr), lowest);
-        auto        entry = [&](int i, float v) {
-            const u32 col = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
-            return ((u64)(~fkey(v)) << 32) | col;
-        };
-        sp_sweep(y, ny, thr, [&](int i, float v) {
-            if (sp_bin(maxv - v) <= b_thr) {
-                keep3 = keep2, keep2 = keep1, keep1 = keep0;
-                keep0 = entry(i, v);
-                ++mine;
+        // ---- few candidates: the leader gets them all, bin by bin, and finishes the row alone ----
+        {
+            const u32 base = cluster_addr(smem_addr(M.area), 0);
+            u32       e    = run;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                // the place of this CTA's first entry of a bin
+                const int b = tid * PER + i;
+                if (b <= b_thr) {
+                    M.hist[b] = base + 8u * (e + M.hist[b]);
+                }
+                e += c[i];
             }
-        });
-        u32 at = block_excl_u32(mine, &tot);
-        if (tid == 0) {
-            s_base1 = tot != 0 ? datom_add(cluster_addr(smem_addr(&X.area_n), 0), tot) : 0u;
         }
         __syncthreads();
-        if (mine != 0) {
-            const u32 dst = cluster_addr(smem_addr(M.area), 0) + 8u * (at + s_base1);
-            if (mine <= 4) {
-                dst_u64(dst, keep0);
-                if (mine > 1) {
-                    dst_u64(dst + 8, keep1);
-                }
-                if (mine > 2) {
-                    dst_u64(dst + 16, keep2);
-                }
-                if (mine > 3) {
-                    dst_u64(dst + 24, keep3);
-                }
+        const float thr = fmaxf(sp_floor_value(maxv, b_thr), lowest);
+        sp_sweep(y, ny, thr, [&](int i, float v) {
+            const int b = sp_bin(maxv - v);
+            if (b <= b_thr) {
+                const u32 col = (u32)(((i >> lgvt) << 10) | (rank << lgvt) | (i & ((1 << lgvt) - 1)));
+                dst_u64(atomicAdd(&M.hist[b], 8u), ((u64)(~fkey(v)) << 32) | col);
             }
-            else {
-                u32 w = 0;
-                sp_sweep(y, ny, thr, [&](int i, float v) {
-                    if (sp_bin(maxv - v) <= b_thr) {
-                        dst_u64(dst + 8u * w, entry(i, v));
-                        ++w;
-                    }
-                });
-            }
-        }
+        });
         cluster_sync();
         trace_mark(O.trace, 7);
         if (rank != 0) {
             return true;
         }
-        // (the leader's slice has been read for the last time: it is the sort's and the draw's scratch)
+        // An entry's place inside its bin is the number of smaller ones there, a handful unless many columns are equal.  (The
+        // leader's slice has been read for the last time: the sorted list goes there, and the draw's scratch where the
+        // entries came in.)
         const int n_cand = (int)N;
         auto      key_of = [&](u64 e) { return fkey_inv(~(u32)(e >> 32)); };
-        u64*      sorted = (u64*)M.area;
-        sorted = sp_bucket_sort(sorted, excl, n_cand, (u64*)M.y, n_cand <= 128 ? sorted + 1024 : sorted,
-                                [&](u64 e) { return sp_bin(maxv - key_of(e)); });
+        u64*      sorted = (u64*)M.y;
+        {
+            const u64* in = (const u64*)M.area;
+            FTB_ASSUME_SHARED(in);
+#pragma unroll 1
+            for (int i = tid; i < n_cand; i += kThreads) {
+                const u64 e  = in[i];
+                const int b  = sp_bin(maxv - key_of(e));
+                const int lo = (int)excl[b], hi = b + 1 < kSpBins ? (int)excl[b + 1] : n_cand;
+                int       rk = lo;
+                int       j  = lo;
+#pragma unroll 1
+                for (; j + 4 <= hi; j += 4) {
+                    u64 o[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        o[q] = in[j + q];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        rk += o[q] < e ? 1 : 0;
+                    }
+                }
+#pragma unroll 1
+                for (; j < hi; ++j) {
+                    rk += in[j] < e ? 1 : 0;
+                }
+                sorted[rk] = e;
+            }
+            __syncthreads();
+        }
         trace_mark(O.trace, 8);
         __shared__ Smem s_S;
         const Smem&     S = s_S;
         if (tid == 0) {
             s_S.cand = (u64*)M.area;
-            s_S.hist = (u32*)M.y;
-            s_S.val2 = (float*)(M.y + kNB);
+            s_S.hist = M.area;
+            s_S.val2 = (float*)(M.area + kNB);
         }
         __syncthreads();
         if (!softmax) {
@@ -1526,7 +1494,6 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     int owners = (int)((N + 1023u) / 1024u);
     owners     = owners < 1 ? 1 : (owners > n ? n : owners);
     __shared__ SpKeys s_K;
-    __shared__ u32    s_bound[kSpMaxN];  // position e of the row's order: the last owner q with e >= s_bound[q]
     const SpKeys&     K = s_K;
     if (tid == 0) {
         s_K.area   = smem_addr(M.area);
@@ -1535,28 +1502,27 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     if (tid <= kSpMaxN) {
         s_K.start[tid] = tid == 0 ? 0u : N;
     }
-    if (tid < kSpMaxN) {
-        s_bound[tid] = tid < owners ? ((u32)tid * N + (u32)owners - 1u) / (u32)owners : 0xffffffffu;
-    }
     __syncthreads();
+    // The owner of a bin follows from its first position (any rule will do that rises with it and is the same in all CTAs).
+    const float per_key  = (float)owners / (float)N;
+    auto        owner_of = [&](u32 e) {
+        const int o = (int)((float)e * per_key);
+        return o < owners ? o : owners - 1;
+    };
     u32 owner_bits = 0;  // of this thread's bins, four bits each
     {
-        auto advance = [&](int o, u32 e) {
-            while (o + 1 < kSpMaxN && e >= s_bound[o + 1]) {
-                ++o;
-            }
-            return o;
-        };
-        int o = tid == 0 ? 0 : advance(0, excl[tid * PER - 1]);
+        u32 e = run;
+        int before = tid == 0 ? 0 : owner_of(excl[tid * PER - 1]);
+#pragma unroll
         for (int i = 0; i < PER; ++i) {
             // the first bin of an owner: where its keys start in the row's order
-            const int before = o;
-            const u32 e      = excl[tid * PER + i];
-            o                = tid * PER + i <= b_thr ? advance(o, e) : o;
+            const int o = tid * PER + i <= b_thr ? owner_of(e) : before;
             for (int q = before + 1; q <= o; ++q) {
                 s_K.start[q] = e;
             }
             owner_bits |= (u32)o << (4 * i);
+            before = o;
+            e += c[i];
         }
     }
     __syncthreads();
@@ -1566,9 +1532,16 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     }
     trace_mark(O.trace, 10);
     // per bin the place of this CTA's first key of it: the bin's in its owner's area, after the keys of the CTAs before
-    for (int i = 0; i < PER; ++i) {
-        const int b = tid * PER + i, o = (int)((owner_bits >> (4 * i)) & 15u);
-        M.hist[b]   = cluster_addr(K.area + 4u * (excl[b] - s_K.start[o] + M.hist[b]), (u32)o);
+    {
+        u32 e = run;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int b = tid * PER + i, o = (int)((owner_bits >> (4 * i)) & 15u);
+            if (b <= b_thr) {
+                M.hist[b] = cluster_addr(K.area + 4u * (e - s_K.start[o] + M.hist[b]), (u32)o);
+            }
+            e += c[i];
+        }
     }
     __syncthreads();
     sp_scatter_keys(y, ny, lowest, maxv, (u32)b_thr, smem_addr(M.hist));
@@ -1678,14 +1651,15 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
 }
 
 // The step's stop criteria (stop words of row r, then - by the last row of the call - the length limit and the count of
-// finished rows over the batch), by the CTA that finished row r.  Same results as stop_criteria_kernel.
-static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const StopArgs& T, int r)
+// finished rows over the batch), by the CTA that finished row r.  Same results as stop_criteria_kernel.  With rows left to
+// another launch (their flags are set) nothing is counted: the host is told, and sends that launch and the criteria.
+static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const StopArgs& T, int r, const int* flags, bool decided)
 {
     __shared__ u32 s_last, s_sum;
     const int      tid = threadIdx.x;
     const size_t   row = (size_t)P.ite * P.local_batch + r;
     __syncthreads();
-    if (T.stop_words != nullptr) {
+    if (T.stop_words != nullptr && decided) {
         const int* base = T.stop_words + (size_t)r * 2 * T.stop_words_len;
         const int* offs = base + T.stop_words_len;
         for (int i = tid; i < T.stop_words_len; i += kThreads) {
@@ -1700,9 +1674,6 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
         }
         __syncthreads();
     }
-    if (T.limit == nullptr) {
-        return;
-    }
     if (tid == 0) {
         __threadfence();
         s_last = atomicAdd(T.arrived, 1u) == (u32)P.local_batch - 1u ? 1u : 0u;
@@ -1711,6 +1682,18 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
     }
     __syncthreads();
     if (s_last == 0) {
+        return;
+    }
+    bool left = false;
+    for (int i = tid; i < P.local_batch; i += kThreads) {
+        left |= __ldcg(flags + i) != 0;
+    }
+    if (__syncthreads_or(left)) {
+        if (tid == 0) {
+            *T.arrived = 0;
+            __threadfence_system();
+            *(volatile u64*)T.result = ((u64)T.sequence << 32) | kRowsLeft;
+        }
         return;
     }
     u32 mine = 0;
@@ -1731,37 +1714,21 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
     }
 }
 
-// A row that the tables of the split form cannot hold, by the leader CTA alone.
-template<int DT>
-static __device__ __noinline__ void sp_whole_row(const KParams& P, int r, int area, unsigned char* smem, u64* rec)
-{
-    __shared__ Smem s_S;
-    Smem&           S = s_S;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        map_general_smem(P, S, smem);
-    }
-    __syncthreads();
-    process_row<DT>(P, S, r, P.scratch + (size_t)area * P.scratch_stride, rec);
-}
-
-// WHOLE: the kernel finishes every row itself (rows its tables cannot hold go through the general row code in the
-// leader CTA) and, when asked to, the step's stop criteria: one launch per decode step.  Taken while all rows are
-// resident at once; with more rows the general code's shared memory would cost residency, and the rows it is needed
-// for are left to a second launch: decode_sampling_kernel, or - where the areas of the first launch are small - a few
-// clusters of this form with all the shared memory there is (A.clusters), because a nucleus of half of 127000 columns takes
-// 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of 127000 columns; above 163000
-// columns there is no such launch, 49000 columns end it) still ends in the general code, so a batch of flat rows takes what its widest nucleus takes.  Mean and slowest
-// of 30 steps of fresh normal logits, 800 x 126959 bf16 with log-probabilities: 1.2 / 1.2 ms (sigma 2.5, p 0.95), 2.3 / 2.7
-// (sigma 2, p 0.95, temperature 1.2), 27 / 43 (sigma 1.5, p 0.95, temperature 1.2); 60 x 200000 fp32: 0.9 / 1.8, 9.4 / 10.2 and
-// 13.6 / 15.1 ms.
+// ROOMY: 128 registers, two CTAs on an SM, and - when asked to - the step's stop criteria: one launch per decode step.
+// Taken while all rows are resident at once; with more rows 80 registers and three CTAs on an SM are worth more.  Either form
+// flags the rows that its tables cannot hold for a second launch: decode_sampling_kernel, or - where the areas of the first
+// launch are small - a few clusters of the roomy form with all the shared memory there is (A.clusters), because a nucleus of half
+// of 127000 columns takes 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of
+// 127000 columns; above 163000 columns there is no such launch, 49000 columns end it) still ends in the general code, so a batch of
+// flat rows takes what its widest nucleus takes.  Mean and slowest of 30 steps of fresh normal logits, 800 x 126959 bf16 with
+// log-probabilities: 1.2 / 1.2 ms (sigma 2.5, p 0.95), 2.3 / 2.7 (sigma 2, p 0.95, temperature 1.2), 27 / 43 (sigma 1.5, p 0.95,
+// temperature 1.2); 60 x 200000 fp32: 0.9 / 1.8, 9.4 / 10.2 and 13.6 / 15.1 ms.
 //
-// Stack: the form that keeps every row holds the general row code's frames under its own.  Builds of it with 1904 and 1952
-// bytes a thread ended steps of 37 rows (two CTAs of a cluster on an SM) with an illegal address, one of them with nothing
-// but two prints that never ran added to a source that runs at 1808; 16 rows (one CTA on an SM) ran.  No access of the code
-// is behind it: what grows is kept in shared memory instead, and the frame stays at 1728.
-template<int DT, int LGN, bool WHOLE>
-__global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
+// The general row code is not part of this kernel.  It was, in the roomy form, for the rows it leaves; its frames brought the
+// stack to 1.7 to 1.9 KB a thread, and builds that differed in nothing but such sizes ended steps of two CTAs on an SM with an
+// illegal address, or did not.  Without it the stack is 0.1 KB.
+template<int DT, int LGN, bool ROOMY>
+__global__ void __launch_bounds__(kThreads, ROOMY ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
                                                                      const __grid_constant__ SplitArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1770,7 +1737,11 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
     const int  tid = threadIdx.x, rank = (int)cluster_rank();
     const bool want_lp = P.cum_log_probs != nullptr || P.out_log_probs != nullptr;
     const int  first = (int)blockIdx.x >> LGN, step = (int)gridDim.x >> LGN;
-    const bool again = WHOLE && A.redo_flags != nullptr;
+    const bool again = ROOMY && A.clusters > 0;
+    // Launched while the kernel in front of it in the stream drains: nothing of memory is touched before that one has ended.
+    // What serves the rows left here may come up in the same way.
+    wait_for_previous();
+    asm volatile("griddepcontrol.launch_dependents;");
     __shared__ u32 s_flagged[kWarps];
     int            base = -kThreads, w = kWarps;  // of the flagged rows: place in the search for the next one
     u32            word = 0;
@@ -1837,20 +1808,13 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
                 }
                 topp_decay_row(P, r, *s_O.id_out);
             }
-            if (!WHOLE) {
-                A.redo_flags[r] = decided ? 0 : 1;
-            }
+            A.redo_flags[r] = decided ? 0 : 1;
             if (s_O.trace != nullptr) {
                 s_O.trace[3] = global_timer_ns();
             }
         }
-        if (WHOLE && rank == 0) {
-            if (!decided) {
-                sp_whole_row<DT>(P, r, again ? first : r, smem_raw, nullptr);
-            }
-            if (A.stop.stop_words != nullptr || A.stop.limit != nullptr) {
-                sp_stop_criteria(P, A.stop, r);
-            }
+        if (ROOMY && rank == 0 && A.stop.limit != nullptr) {
+            sp_stop_criteria(P, A.stop, r, A.redo_flags, decided);
         }
         if (again) {
             cluster_sync();  // (the next row starts with nobody inside this one)
@@ -1859,11 +1823,11 @@ __global__ void __launch_bounds__(kThreads, WHOLE ? 2 : 3) split_sampling_kernel
     cluster_sync();  // no CTA leaves while another may still reach into its shared memory
 }
 
-template<int DT, int LGN, bool WHOLE>
+template<int DT, int LGN, bool ROOMY>
 cudaError_t split_opt_in()
 {
     static std::atomic<bool> opted_in[kDevicesKnown];
-    return opt_in_smem(split_sampling_kernel<DT, LGN, WHOLE>, kSpMaxSmem, opted_in);
+    return opt_in_smem(split_sampling_kernel<DT, LGN, ROOMY>, kSpMaxSmem, opted_in);
 }
 
 static inline void split_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int lgn, int clusters, size_t smem,
@@ -1881,18 +1845,21 @@ static inline void split_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttrib
     cfg.numAttrs             = 1;
 }
 
-template<int DT, int LGN, bool WHOLE>
+template<int DT, int LGN, bool ROOMY>
 int split_sampling_launch_n(const KParams& K, const SplitArgs& A, size_t smem, cudaStream_t st)
 {
-    FTB_CUDA_CHECK((split_opt_in<DT, LGN, WHOLE>()));
+    FTB_CUDA_CHECK((split_opt_in<DT, LGN, ROOMY>()));
     cudaLaunchConfig_t  cfg{};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     split_launch_config(cfg, attr, LGN, A.clusters > 0 ? A.clusters : K.local_batch, smem, st);
-    FTB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_sampling_kernel<DT, LGN, WHOLE>, K, A));
+    attr[1].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs                                       = 2;
+    FTB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_sampling_kernel<DT, LGN, ROOMY>, K, A));
     return FTB200_OK;
 }
 
-template<int DT, int LGN, bool WHOLE>
+template<int DT, int LGN, bool ROOMY>
 int split_resident_n(size_t smem)
 {
     // asked once per device and kilobyte of shared memory (what a call needs moves in steps of the vocabulary)
@@ -1910,8 +1877,8 @@ int split_resident_n(size_t smem)
         cudaLaunchAttribute attr[1];
         int                 n = 0;
         split_launch_config(cfg, attr, LGN, 1, (size_t)kb * 1024, nullptr);
-        if (split_opt_in<DT, LGN, WHOLE>() != cudaSuccess
-            || cudaOccupancyMaxActiveClusters(&n, split_sampling_kernel<DT, LGN, WHOLE>, &cfg) != cudaSuccess) {
+        if (split_opt_in<DT, LGN, ROOMY>() != cudaSuccess
+            || cudaOccupancyMaxActiveClusters(&n, split_sampling_kernel<DT, LGN, ROOMY>, &cfg) != cudaSuccess) {
             (void)cudaGetLastError();
             return 0;
         }
@@ -1925,26 +1892,21 @@ int split_resident_n(size_t smem)
 
 // Clusters of 2^lgn CTAs with `smem` bytes of shared memory each that the current device holds at once.
 template<int DT>
-int split_resident(int lgn, bool whole, size_t smem)
+int split_resident(int lgn, bool roomy, size_t smem)
 {
-    if (whole) {
+    if (roomy) {
         return lgn == 2 ? split_resident_n<DT, 2, true>(smem) : split_resident_n<DT, 3, true>(smem);
     }
     return lgn == 1 ? split_resident_n<DT, 1, false>(smem) : (lgn == 2 ? split_resident_n<DT, 2, false>(smem) : split_resident_n<DT, 3, false>(smem));
 }
 
-// smem_general: shared memory of the general row code, for the form that keeps every row.
 template<int DT>
-int split_sampling_launch(const KParams& K, const SplitArgs& A, size_t smem_general, cudaStream_t st)
+int split_sampling_launch(const KParams& K, const SplitArgs& A, cudaStream_t st)
 {
     const size_t smem = split_smem_bytes(A.slice, A.area);
-    const size_t both = smem > smem_general ? smem : smem_general;
-    if (A.clusters > 0) {
-        return split_sampling_launch_n<DT, 3, true>(K, A, both, st);
-    }
-    if (A.redo_flags == nullptr) {
-        return A.lgn == 2 ? split_sampling_launch_n<DT, 2, true>(K, A, both, st) :
-                            split_sampling_launch_n<DT, 3, true>(K, A, both, st);
+    if (A.roomy) {
+        return A.lgn == 2 ? split_sampling_launch_n<DT, 2, true>(K, A, smem, st) :
+                            split_sampling_launch_n<DT, 3, true>(K, A, smem, st);
     }
     switch (A.lgn) {
         case 1: return split_sampling_launch_n<DT, 1, false>(K, A, smem, st);
