@@ -72,10 +72,12 @@ struct GatherTree {
     const int* virtual_lengths;
     int        max_input_without_prompt_length, max_prefix_length;
     int*       output_ids;
+    int        by_maps;  // the tables of tree_by_maps() fit
 };
 
 __global__ void __launch_bounds__(kDkThreads) gather_tree_kernel(GatherTree p)
 {
+    wait_for_previous();
     __shared__ int     s_ids[kStage], s_par[kStage];
     __shared__ int     s_parent[kMaxBeams];
     __shared__ uint8_t s_bad[kMaxBeams];
@@ -195,12 +197,216 @@ __global__ void __launch_bounds__(kDkThreads) gather_tree_kernel(GatherTree p)
     }
 }
 
+// ---- the tree in registers --------------------------------------------------------------------------------------
+// A level's parents are a map of at most eight values (the beams, and "no parent", which stays): eight nibbles of a word.
+constexpr u32 kMapIdentity = 0x76543210u;
+constexpr int kTreeBeams = 7, kTreeLevels = 4;  // beams of a map, levels of a thread, at most
+// first f, then g: two byte selections, with g spread to bytes and the result packed again
+__device__ __forceinline__ u32 map_then(u32 f, u32 g)
+{
+    auto spread = [](u32 x) {
+        x = (x | (x << 8)) & 0x00ff00ffu;
+        return (x | (x << 4)) & 0x0f0f0f0fu;
+    };
+    auto pack = [](u32 x) {
+        x = (x | (x >> 4)) & 0x00ff00ffu;
+        return (x | (x >> 8)) & 0xffffu;
+    };
+    const u32 lo = spread(g & 0xffffu), hi = spread(g >> 16);
+    return pack(__byte_perm(lo, hi, f & 0xffffu)) | (pack(__byte_perm(lo, hi, f >> 16)) << 16);
+}
+__device__ __forceinline__ int map_of(u32 m, int x)
+{
+    return (int)((m >> (4 * x)) & 15u);
+}
+
+// Up to KB beams that have prompts of one length, and up to LV levels for each thread.  Parents and tokens go into shared memory,
+// neighbouring lanes to neighbouring words (a level is 4 K bytes of a row of all entries, so the number of lines that a
+// warp's load touches is what it costs); a thread holds the maps of its levels (consecutive ones, from the top down); one scan
+// over their compositions says where each beam's chain enters them; the tokens found go to where the parents were, and from
+// there into the tree and its transposed copy, each element written once.  Returns false, with nothing written, for entries of
+// another form.
+template<int KB, int LV>
+__device__ __forceinline__ bool tree_by_maps(const GatherTree& p, unsigned char* smem)
+{
+    __shared__ int s_top_token[KB];  // position of a beam's first end token
+    __shared__ u32 s_warp[kChainThreads / 32], s_broken;
+    const int      b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, K = p.beam_width, T = p.max_time;
+    const size_t   BK = (size_t)p.batch_size * K, col0 = (size_t)b * K;
+    const int      L = (T + kChainThreads - 1) / kChainThreads, first = T - 1 - tid * L;  // the thread's highest level
+    int* const     s_tok = (int*)smem;       // [T][K]
+    int* const     s_par = s_tok + T * K;    // [T][K]; then the token of every position
+    FTB_ASSUME_SHARED(s_tok);
+    FTB_ASSUME_SHARED(s_par);
+    const int step = kChainThreads / K, col = tid % K, t0 = tid / K;
+    if (t0 < step) {
+        constexpr int U = 8;
+        for (int t = t0; t < T; t += U * step) {
+            int v[U], w[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool   in = t + u * step < T;
+                const size_t g  = BK * (size_t)(t + u * step) + col0 + col;
+                v[u]            = in ? __ldg(p.step_ids + g) : 0;
+                w[u]            = in && p.parent_ids != nullptr ? __ldg(p.parent_ids + g) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (t + u * step < T) {
+                    s_tok[(t + u * step) * K + col] = v[u];
+                    s_par[(t + u * step) * K + col] = w[u];
+                }
+            }
+        }
+    }
+    const int max_il = p.input_lengths == nullptr ? 0 : p.max_input_length;
+    const int prompt_len = p.prefix_lengths == nullptr ? 0 : p.prefix_lengths[b];
+    const int virt       = p.virtual_lengths == nullptr ? 0 : p.virtual_lengths[b];
+    const int len        = (p.input_lengths == nullptr ? 0 : p.input_lengths[col0]) - virt;
+    const int end        = p.end_tokens[b];
+    const int trimmed    = p.max_prefix_length + (p.max_input_length - p.max_input_without_prompt_length);
+    int       max_len    = -1;
+    bool      even       = true;
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+        if (k < K) {
+            max_len = max(max_len, p.max_sequence_lengths[col0 + k] + p.final_step);
+            even    = even && (p.input_lengths == nullptr ? 0 : p.input_lengths[col0 + k]) - virt == len;
+        }
+    }
+    const int top = min(T, max_len), shift = max_il - len + prompt_len;
+    // (then positions 0 .. top - 1 - shift are those of the prompt's and the generated levels, one after the other)
+    if (!(even && prompt_len >= 0 && prompt_len <= len && len <= max_il && top > max_il)) {
+        __syncthreads();  // (the tables are laid out anew)
+        return false;
+    }
+    if (tid < KB) {
+        s_top_token[tid] = INT_MAX;
+    }
+    if (tid == 0) {
+        s_broken = 0;
+    }
+    __syncthreads();
+
+    // ---- the maps, and the composition of those of the threads in front ----
+    auto skipped = [&](int level) { return level < prompt_len || (level >= len && level < max_il); };
+    u32  m[LV], all = kMapIdentity;
+#pragma unroll
+    for (int l = 0; l < LV; ++l) {
+        const int level = first - l;
+        m[l]            = kMapIdentity;
+        if (l < L && level >= 0 && level < top && (level == top - 1 || !skipped(level))) {
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+                if (k < K) {
+                    int v = s_par[level * K + k];
+                    v     = (unsigned)v < (unsigned)K ? v : v % K;
+                    v     = v < 0 ? K : v;
+                    m[l]  = (m[l] & ~(15u << (4 * k))) | ((u32)v << (4 * k));
+                }
+            }
+        }
+        all = map_then(all, m[l]);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 before = __shfl_up_sync(0xffffffffu, all, o);
+        all              = lane >= o ? map_then(before, all) : all;
+    }
+    u32 entry = __shfl_up_sync(0xffffffffu, all, 1);
+    entry     = lane == 0 ? kMapIdentity : entry;
+    if (lane == 31) {
+        s_warp[wid] = all;
+    }
+    __syncthreads();
+    if (wid == 0) {
+        u32 w = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const u32 before = __shfl_up_sync(0xffffffffu, w, o);
+            w                = lane >= o ? map_then(before, w) : w;
+        }
+        s_warp[lane] = w;
+    }
+    else if (wid == 1 && lane < K) {
+        // (one update of the lengths per entry: see gather_tree_kernel; all threads have read them)
+        p.max_sequence_lengths[col0 + lane] = p.max_sequence_lengths[col0 + lane] + p.final_step - trimmed;
+        if (p.response_input_lengths != nullptr) {
+            p.response_input_lengths[col0 + lane] = len - prompt_len;
+        }
+    }
+    __syncthreads();
+    entry = map_then(wid > 0 ? s_warp[wid - 1] : kMapIdentity, entry);
+
+    // ---- tokens along the chains; a chain that broke off gives the end token.  Positions behind the sequence: end tokens, or
+    // what the caller left ----
+    const int first_t = max_il == 0 ? 1 : max_il, fill = max(0, max_len - shift), fill_end = T - p.max_prefix_length;
+    const int out_len = T - trimmed, behind = top - shift;
+    auto      at      = [&](int t, int j) { return BK * (size_t)t + col0 + j; };
+    u32       broken  = 0;
+#pragma unroll
+    for (int l = 0; l < LV; ++l) {
+        const int level = first - l;
+        if (l < L && level >= 0 && level < top && !skipped(level)) {
+            const int t = level < max_il ? level - prompt_len : level - shift;
+#pragma unroll
+            for (int j = 0; j < KB; ++j) {
+                if (j < K) {
+                    const int from = map_of(entry, j), w = from == K ? end : s_tok[level * K + from];
+                    broken |= from == K ? 1u << j : 0u;
+                    if (t >= first_t && t < top && w == end) {
+                        atomicMin(&s_top_token[j], t);
+                    }
+                    s_par[t * K + j] = w;
+                }
+            }
+        }
+        entry = map_then(entry, m[l]);
+    }
+    if (broken != 0) {
+        atomicOr(&s_broken, broken);
+    }
+    if (t0 < step) {
+        for (int t = behind + t0; t < T; t += step) {
+            const int w        = t >= fill && t < fill_end ? end : p.beams[at(t, col)];
+            s_par[t * K + col] = w;
+            if (t >= first_t && t < top && w == end) {
+                atomicMin(&s_top_token[col], t);
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- nothing but end tokens after the first one ----
+    if (t0 < step) {
+        const int cut_from = (s_broken >> col) & 1u ? INT_MAX : s_top_token[col];
+        int*      out      = p.output_ids == nullptr ? nullptr : p.output_ids + (col0 + col) * (size_t)out_len;
+#pragma unroll 4
+        for (int t = t0; t < T; t += step) {
+            const bool over = t > cut_from && t < top;
+            const int  w    = over ? end : s_par[t * K + col];
+            if (t < behind || over || (t >= fill && t < fill_end)) {
+                p.beams[at(t, col)] = w;
+            }
+            if (out != nullptr && t < out_len) {
+                out[t] = w;
+            }
+        }
+    }
+    return true;
+}
+
 // The tree with the whole parent table of an entry in shared memory.  Bound by latency: 8 levels of ids and parents in
 // flight per thread, then the chains, then one pass that writes and one that cuts and transposes.
-// 64 entries x 4 beams x 2048 levels: 245 us with one thread per chain, 17 us this way.
+// 64 entries x 4 beams x 2048 levels: 245 us with one thread per chain, 14.8 us this way (parents 4.7, walks 3.5, tokens 4.5, end
+// tokens 1.2), 18.4 a call; 12.7 a call by maps in registers, which serve up to seven beams and 4096 levels.
 __global__ void __launch_bounds__(kChainThreads) gather_tree_chains_kernel(GatherTree p)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem[];
+    if (p.by_maps && tree_by_maps<kTreeBeams, kTreeLevels>(p, smem)) {
+        return;
+    }
     __shared__ int     s_start[kMaxBeams], s_from[kMaxBeams], s_first[kMaxBeams];
     __shared__ uint8_t s_bad[kMaxBeams];
     __shared__ int     s_maxlen, s_uneven;
@@ -378,6 +584,7 @@ __global__ void __launch_bounds__(kDkThreads) finalize_kernel(int* output_ids, i
                                                               const float* topk_log_probs, const int* num_beams,
                                                               int K, int max_seq_len)
 {
+    wait_for_previous();
     __shared__ float s_score[2 * kMaxBeams];
     __shared__ int   s_rank[kMaxBeams];
     const int        b = blockIdx.x, tid = threadIdx.x, n = max(0, min(num_beams[b], 2 * K));
@@ -444,6 +651,7 @@ struct InsertPath {
 
 __global__ void __launch_bounds__(kDkThreads) insert_unfinished_path_kernel(InsertPath p)
 {
+    wait_for_previous();
     __shared__ int   s_ids[kStage], s_par[kStage], s_out[kStage];
     __shared__ float s_lp[kStage], s_lpout[kStage];
     __shared__ int   s_prev[kMaxArchiveBeams], s_len[kMaxArchiveBeams];
@@ -529,6 +737,7 @@ __global__ void __launch_bounds__(kDkThreads) insert_unfinished_path_kernel(Inse
 // The archive with the whole parent table of an entry in shared memory (see walk_chains).
 __global__ void __launch_bounds__(kChainThreads) insert_chains_kernel(InsertPath p)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_start[kMaxArchiveBeams], s_from[kMaxArchiveBeams];
     __shared__ int s_top;
@@ -685,14 +894,18 @@ extern "C" int ftb200_gather_tree(const ftb200_gather_tree_params* a)
     p.max_prefix_length               = a->max_prefix_soft_prompt_length;
     p.output_ids                      = a->output_ids;
     // the parent table of an entry in shared memory where it fits (50000 level-beams), else tile by tile
-    const size_t smem = chain_smem_bytes(a->max_time, a->beam_width);
+    size_t       smem   = chain_smem_bytes(a->max_time, a->beam_width);
+    const size_t tables = (size_t)a->max_time * a->beam_width * 8;  // tokens and parents as they are
+    p.by_maps = a->beam_width <= kTreeBeams && a->max_time <= kTreeLevels * kChainThreads && tables <= kChainMaxSmem;
+    smem      = p.by_maps && tables > smem ? tables : smem;
     if (smem <= kChainMaxSmem) {
         static std::atomic<bool> opted_in[kDevicesKnown];
         FTB_CUDA_CHECK(opt_in_smem(gather_tree_chains_kernel, kChainMaxSmem, opted_in));
-        gather_tree_chains_kernel<<<a->batch_size, kChainThreads, smem, (cudaStream_t)a->stream>>>(p);
+        FTB_CUDA_CHECK(launch_early(gather_tree_chains_kernel, dim3((unsigned)a->batch_size), dim3(kChainThreads), smem,
+                                    (cudaStream_t)a->stream, p));
     }
     else {
-        gather_tree_kernel<<<a->batch_size, kDkThreads, 0, (cudaStream_t)a->stream>>>(p);
+        FTB_CUDA_CHECK(launch_early(gather_tree_kernel, dim3((unsigned)a->batch_size), dim3(kDkThreads), 0, (cudaStream_t)a->stream, p));
     }
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);
@@ -716,9 +929,9 @@ extern "C" int ftb200_finalize(int* output_ids, int* sequence_lengths, float* cu
         return FTB200_UNSUPPORTED;
     }
     // a CTA per beam (each ranks the entry's few scores for itself): the copies of an entry's beams run side by side
-    finalize_kernel<<<dim3(batch_size, beam_width < 64 ? beam_width : 64), kDkThreads, 0, (cudaStream_t)stream>>>(
-        output_ids, sequence_lengths, cum_log_probs, output_log_probs, topk_output_ids, topk_sequence_lengths, scores,
-        topk_cum_log_probs, topk_log_probs, num_beams, beam_width, max_seq_len);
+    FTB_CUDA_CHECK(launch_early(finalize_kernel, dim3(batch_size, beam_width < 64 ? beam_width : 64), dim3(kDkThreads), 0,
+                                (cudaStream_t)stream, output_ids, sequence_lengths, cum_log_probs, output_log_probs, topk_output_ids,
+                                topk_sequence_lengths, scores, topk_cum_log_probs, topk_log_probs, num_beams, beam_width, max_seq_len));
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);
     return FTB200_OK;
@@ -764,10 +977,11 @@ extern "C" int ftb200_insert_unfinished_path(const ftb200_beam_hyps* hyps, const
     if (smem <= kChainMaxSmem) {
         static std::atomic<bool> opted_in[kDevicesKnown];
         FTB_CUDA_CHECK(opt_in_smem(insert_chains_kernel, kChainMaxSmem, opted_in));
-        insert_chains_kernel<<<batch_size, kChainThreads, smem, (cudaStream_t)stream>>>(p);
+        FTB_CUDA_CHECK(launch_early(insert_chains_kernel, dim3((unsigned)batch_size), dim3(kChainThreads), smem, (cudaStream_t)stream, p));
     }
     else {
-        insert_unfinished_path_kernel<<<batch_size, kDkThreads, 0, (cudaStream_t)stream>>>(p);
+        FTB_CUDA_CHECK(launch_early(insert_unfinished_path_kernel, dim3((unsigned)batch_size), dim3(kDkThreads), 0,
+                                    (cudaStream_t)stream, p));
     }
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);

@@ -29,3 +29,20 @@ def test_gather_tree_chains(kw, uneven):
 def test_insert_unfinished_path_chains(kw):
     c = dc.insert_case(**kw)
     dc.same(dc.run_insert("ours", c), dc.run_insert("oracle", c), float_keys=("normed",))
+
+
+@pytest.mark.parametrize("kw", [
+    dict(seed=121, B=3, K=1, T=1023, M=7), dict(seed=122, B=4, K=4, T=1024, M=9, final_step=1),
+    dict(seed=123, B=4, K=4, T=1025, M=64, bad_parents=True), dict(seed=124, B=2, K=7, T=2047, M=30, bad_parents=True),
+    dict(seed=125, B=2, K=5, T=4096, M=100, prefix=True, with_response=True), dict(seed=126, B=2, K=4, T=4097, M=20),
+    dict(seed=127, B=5, K=7, T=37, M=36), dict(seed=128, B=3, K=8, T=300, M=12), dict(seed=129, B=3, K=6, T=4096, M=5),
+    dict(seed=130, B=6, K=3, T=40, M=12, virtual=True, prefix=True), dict(seed=131, B=2, K=2, T=2048, M=2047, final_step=1)])
+def test_gather_tree_by_maps(kw):
+    """The form that composes the levels' maps: one to four levels a thread and one more, the most beams a map holds and one
+    more, tables that just fit and just do not, broken parents, sequences that end inside the prompt or behind the time."""
+    c = dc.gather_tree_case(**kw)
+    dc.same(dc.run_gather_tree("ours", c), dc.run_gather_tree("oracle", c))
+    c["seq_lengths"] = c["seq_lengths"] + kw["T"] // 3  # (some now end behind max_time)
+    dc.same(dc.run_gather_tree("ours", c), dc.run_gather_tree("oracle", c))
+    c["seq_lengths"][:] = np.maximum(kw["M"] - 2, 1)
+    dc.same(dc.run_gather_tree("ours", c), dc.run_gather_tree("oracle", c))
