@@ -94,7 +94,7 @@ __device__ __forceinline__ float fast_exp(float d)
     return exp2f(d * kLog2e);  // __expf under the reference's fast-math build
 }
 
-__device__ __forceinline__ void add_one(MaxSum& a, float x)
+__device__ __forceinline__ void add_plain(MaxSum& a, float x)
 {
     if (x > a.m) {
         a.s = a.s * fast_exp(a.m - x) + 1.0f;
@@ -111,13 +111,12 @@ __device__ __forceinline__ MaxSum merge(const MaxSum& a, const MaxSum& b)
     return {m, a.s * fast_exp(a.m - m) + b.s * fast_exp(b.m - m)};
 }
 
-template<typename T>
-__device__ __forceinline__ void add_vec(MaxSum& a, const uint4& v)
+__device__ __forceinline__ void add_plain_vec(MaxSum& a, const uint4& v)
 {
-    constexpr int N = LpType<T>::kPerVec;
+    constexpr int N = LpType<float>::kPerVec;
     float         x[N];
-    LpType<T>::unpack(v, x);
-    const float vm = LpType<T>::maximum(v, x);
+    LpType<float>::unpack(v, x);
+    const float vm = LpType<float>::maximum(v, x);
     if (vm > a.m) {
         a.s *= fast_exp(a.m - vm);
         a.m = vm;
@@ -129,6 +128,112 @@ __device__ __forceinline__ void add_vec(MaxSum& a, const uint4& v)
     }
     a.s += t;
 }
+
+// ---- 16-bit rows ------------------------------------------------------------------------------------------------
+// Two logits per instruction where that exists (packed fp32 fused multiply-add and add): the exponent of a term is one fused
+// multiply-add, x * log2(e) - m2 with m2 = m * log2(e) as it was rounded, and what that rounding lost, m * log2(e) - m2, is the
+// same for all terms and comes off the logarithm at the end.  Half of the instructions of a subtract, a multiply, an exponential
+// and an add a logit: 512 x 32 x 50257 half 238 -> 232 us (256 -> 249 on a warmer card).  Every fourth exponential by a polynomial
+// on the multiply-add pipes instead of the special-function unit was slower (242, half of them 278).
+__device__ __forceinline__ u64 pack2(float a, float b)
+{
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& a, float& b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+    u64 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+    u64 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// The sum of the two halves of s, times 2^m2, is the sum of exp(x) so far.  A maximum so large (or so low: a row of the
+// type's lowest value) that m2 would not be finite has no m2: then s stands for s * exp(m).
+template<typename T>
+struct PairSum {
+    float m, m2;
+    u64   s;
+    static constexpr bool kWide = sizeof(T) == 2 && LpType<T>::kLowest < -1e30f;
+    __device__ static bool beyond(float m) { return kWide && !(fabsf(m) < 1e30f); }
+    __device__ void        start()
+    {
+        m = LpType<T>::kLowest, m2 = m * kLog2e, s = 0;
+    }
+    // the sum with `to` >= m as its maximum
+    __device__ void raise(float to)
+    {
+        const float to2 = to * kLog2e;
+        const float f   = beyond(m) || beyond(to) ? fast_exp(m - to) : exp2f(m2 - to2);
+        float       a, b;
+        unpack2(s, a, b);
+        s = pack2(a * f, b * f);
+        m = to, m2 = to2;
+    }
+    __device__ void add_one(float x)
+    {
+        if (x > m) {
+            raise(x);
+        }
+        s = add2(s, pack2(beyond(m) ? fast_exp(x - m) : exp2f(fmaf(x, kLog2e, -m2)), 0.0f));
+    }
+    __device__ void add_vec(const uint4& v)
+    {
+        float x[8];
+        LpType<T>::unpack(v, x);
+        const float vm = LpType<T>::maximum(v, x);
+        if (vm > m) {
+            raise(vm);
+        }
+        if (beyond(m)) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s = add2(s, pack2(fast_exp(x[i] - m), 0.0f));
+            }
+            return;
+        }
+        const u64 l = pack2(kLog2e, kLog2e), o = pack2(-m2, -m2);
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            float a, b;
+            unpack2(fma2(pack2(x[i], x[i + 1]), l, o), a, b);
+            s = add2(s, pack2(exp2f(a), exp2f(b)));
+        }
+    }
+    __device__ MaxSum total() const
+    {
+        float a, b;
+        unpack2(s, a, b);
+        // (2^-d for a d of a unit of m2's last place)
+        return {m, beyond(m) ? a + b : (a + b) * fmaf(fmaf(m, kLog2e, -m2), -0.69314718f, 1.0f)};
+    }
+};
+// fp32 rows: at the copy rate with the plain form
+struct PlainSum {
+    MaxSum          a;
+    __device__ void start() { a = {LpType<float>::kLowest, 0.0f}; }
+    __device__ void add_one(float x) { add_plain(a, x); }
+    __device__ void add_vec(const uint4& v) { add_plain_vec(a, v); }
+    __device__ MaxSum total() const { return a; }
+};
+template<typename T>
+struct RowSum {
+    using type = PairSum<T>;
+};
+template<>
+struct RowSum<float> {
+    using type = PlainSum;
+};
 
 // One CTA per (step, sequence) row at a time.  Rows past a sequence's length are skipped without a read.
 //
@@ -145,6 +250,7 @@ __global__ void __launch_bounds__(kLpThreads, kLpCtas) context_log_probs_kernel(
                                                                         size_t vocab_padded, int batch_first,
                                                                         long long rows)
 {
+    wait_for_previous();
     constexpr int N = LpType<T>::kPerVec;
     __shared__ MaxSum s_part[kLpThreads / 32];
     const int         tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -213,13 +319,14 @@ __global__ void __launch_bounds__(kLpThreads, kLpCtas) context_log_probs_kernel(
         const size_t row_idx = batch_first ? (size_t)b * max_len + step : (size_t)step * batch + b;
         const T*     row     = logits + row_idx * vocab_padded;
 
-        MaxSum acc{LpType<T>::kLowest, 0.0f};
+        typename RowSum<T>::type sum;
+        sum.start();
         // Scalars up to the first 16-byte boundary, 16-byte vectors, scalars after the last full vector.
         const int mis  = (int)((reinterpret_cast<uintptr_t>(row) & 15) / sizeof(T));
         const int head = min(vocab, mis ? N - mis : 0);
         const int nvec = (vocab - head) / N;
         if (tid < head) {
-            add_one(acc, LpType<T>::get(row + tid));
+            sum.add_one(LpType<T>::get(row + tid));
         }
         const uint4* vp = reinterpret_cast<const uint4*>(row + head);
         int          i  = tid;
@@ -231,16 +338,17 @@ __global__ void __launch_bounds__(kLpThreads, kLpCtas) context_log_probs_kernel(
             }
 #pragma unroll
             for (int u = 0; u < kLpLoads; ++u) {
-                add_vec<T>(acc, v[u]);
+                sum.add_vec(v[u]);
             }
         }
         for (; i < nvec; i += kLpThreads) {
-            add_vec<T>(acc, ld_nc_v4(vp + i));
+            sum.add_vec(ld_nc_v4(vp + i));
         }
         const int tail0 = head + nvec * N;
         if (tail0 + tid < vocab) {  // fewer than N <= 8 elements remain
-            add_one(acc, LpType<T>::get(row + tail0 + tid));
+            sum.add_one(LpType<T>::get(row + tail0 + tid));
         }
+        MaxSum acc = sum.total();
 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -273,6 +381,7 @@ __global__ void __launch_bounds__(kLpThreads) sum_log_probs_kernel(float* cum, c
                                                                     const int* lengths, int max_len, int batch,
                                                                     int batch_first)
 {
+    wait_for_previous();
     __shared__ float s_part[kLpThreads / 32];
     const int        b = blockIdx.x, tid = threadIdx.x;
     const int        n = min(lengths[b], max_len) - 1;
@@ -312,14 +421,13 @@ int launch_log_probs(float* cum, const void* logits, const int* ids, const int* 
     const long long rows = (long long)(max_len - 1) * (long long)batch;
     if (rows > 0) {
         const int grid = (int)std::min<long long>(rows, (long long)n_sm * kLpCtas);
-        context_log_probs_kernel<T><<<grid, kLpThreads, 0, st>>>(log_probs, (const T*)logits, ids, lengths,
-                                                                 (int)max_len, (int)batch, (int)vocab,
-                                                                 vocab_padded, batch_first, rows);
+        FTB_CUDA_CHECK(launch_early(context_log_probs_kernel<T>, dim3((unsigned)grid), dim3(kLpThreads), 0, st, log_probs,
+                                    (const T*)logits, ids, lengths, (int)max_len, (int)batch, (int)vocab, vocab_padded, batch_first, rows));
         FTB_CUDA_CHECK(cudaGetLastError());
         note_launch(1);
     }
-    sum_log_probs_kernel<<<(int)batch, kLpThreads, 0, st>>>(cum, log_probs, lengths, (int)max_len, (int)batch,
-                                                           batch_first);
+    FTB_CUDA_CHECK(launch_early(sum_log_probs_kernel, dim3((unsigned)batch), dim3(kLpThreads), 0, st, cum, log_probs, lengths, (int)max_len,
+                                (int)batch, batch_first));
     FTB_CUDA_CHECK(cudaGetLastError());
     note_launch(1);
     return FTB200_OK;
