@@ -210,6 +210,7 @@ static __device__ __noinline__ void mark_ancestry(const BeamK& P, int bb, u32* b
 template<int DT, bool TEMP, int PEN>
 __global__ void __launch_bounds__(kBeamThreads, 3) beam_rows_kernel(const __grid_constant__ BeamK P)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // layout: ring of row tiles | u64 collected[kBeamCollect] | u32 bits[flag_words] | u32 list[list_words(listed)] | chain tables
     const u32      ring = (u32)__cvta_generic_to_shared(smem_raw);
@@ -800,7 +801,7 @@ static int beam_rows_launch(const BeamK& K, size_t smem, cudaStream_t st)
 {
     static std::atomic<bool> opted[kDevicesKnown];
     FTB_CUDA_CHECK(opt_in_smem(beam_rows_kernel<DT, TEMP, PEN>, kBeamMaxSmem, opted));
-    beam_rows_kernel<DT, TEMP, PEN><<<K.local_batch * K.K, kBeamThreads, smem, st>>>(K);
+    FTB_CUDA_CHECK(launch_early(beam_rows_kernel<DT, TEMP, PEN>, dim3((unsigned)(K.local_batch * K.K)), dim3(kBeamThreads), smem, st, K));
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
 }

@@ -58,6 +58,7 @@ template<int DT, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 1)
 vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpArgs V)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned short s_max[NT], s_hot[NT * 4];
     __shared__ u32            s_n, s_nspec, s_nhot, s_thr, s_kv, s_m, s_cnt[3], s_lost, s_args[5];
@@ -670,10 +671,10 @@ int vp_select_launch(const KParams& K, const VpArgs& V, size_t smem, int sms, cu
     int             grid  = sms * per_sm;
     grid                  = grid < tasks ? grid : (int)tasks;
     if (per_sm == 1) {
-        vp_select_kernel<DT, 512><<<grid, 512, smem, st>>>(K, V);
+        FTB_CUDA_CHECK(launch_early(vp_select_kernel<DT, 512>, dim3((unsigned)grid), dim3(512), smem, st, K, V));
     }
     else {
-        vp_select_kernel<DT, 256><<<grid, 256, smem, st>>>(K, V);
+        FTB_CUDA_CHECK(launch_early(vp_select_kernel<DT, 256>, dim3((unsigned)grid), dim3(256), smem, st, K, V));
     }
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
