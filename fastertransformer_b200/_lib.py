@@ -56,7 +56,20 @@ def _load():
     return l
 
 
+def _load_step_module():
+    """lib/_ftb200_step.so (host/step_module.c), which calls the library that is loaded here."""
+    import importlib.util
+    path = os.path.join(_HERE, "lib", "_ftb200_step.so")
+    if not os.path.exists(path):
+        raise ImportError("_ftb200_step.so is not built (%s). Run `python -m fastertransformer_b200.build`." % path)
+    spec = importlib.util.spec_from_file_location("_ftb200_step", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 lib = _load()
+step_module = _load_step_module()
 
 
 def check(status):

@@ -73,7 +73,25 @@ def build(verbose=False, force=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_step_module()
     return LIB
+
+
+def build_step_module():
+    """Compile the native half of DynamicDecodeLayer.forward (host/step_module.c) into lib/_ftb200_step.so, next to the
+    library it calls (found through its rpath)."""
+    import sysconfig
+    out, src = os.path.join(OUT, "_ftb200_step.so"), os.path.join(HERE, "host", "step_module.c")
+    deps = [src, os.path.join(INC, "ftb200.h")]
+    if os.path.exists(out) and os.path.exists(LIB) and all(os.path.getmtime(out) >= os.path.getmtime(d) for d in deps):
+        return out
+    cmd = ["gcc", "-O2", "-std=c11", "-Wall", "-fPIC", "-shared", src, "-I" + sysconfig.get_paths()["include"], "-I" + INC, "-L" + OUT,
+           "-lftb200", "-Wl,-rpath,$ORIGIN", "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("building the step module failed")
+    return out
 
 
 def build_shim_driver():

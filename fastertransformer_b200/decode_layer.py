@@ -10,7 +10,7 @@ import ctypes as C
 import numpy as np
 import torch
 
-from ._lib import BeamHyps, BeamParams, SamplingParams, SetupParams, StopParams, check, lib
+from ._lib import BeamHyps, BeamParams, SamplingParams, SetupParams, StopParams, check, lib, step_module as _step
 
 # Page-locked words that a step which missed its deadline has still to write, with an event behind that step: the host
 # allocator would hand them out again when their layer goes.
@@ -26,6 +26,7 @@ def _keep_until_done(word, stream):
 
 _DT = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 TIMEOUT = 6  # FTB200_TIMEOUT
+_LIBRARY = lib  # what the step module calls
 CURAND_STATE_BYTES = 48  # sizeof(curandState_t), XORWOW
 
 
@@ -89,6 +90,9 @@ class _Pack:
 class DynamicDecodeLayer:
     """Drop-in for the sampling half of fastertransformer::DynamicDecodeLayer<T>."""
 
+    _launches = 0
+    _native = None  # the whole batch's slice in _ftb200_step, once a call has gone through forward()'s own code
+
     def __init__(self, vocab_size, vocab_size_padded, dtype=torch.float32, device="cuda:0", stream=None):
         self.vocab_size = int(vocab_size)
         self.vocab_size_padded = int(vocab_size_padded)
@@ -106,9 +110,30 @@ class DynamicDecodeLayer:
         self._count_dev = None
         self._count_host = None
         self._stop = None
-        self.launches = 0
 
     # ---- helpers -------------------------------------------------------------------------------
+    @property
+    def launches(self):
+        """Kernels launched so far."""
+        return self._launches + (0 if self._native is None else _step.launches(self._native))
+
+    @launches.setter
+    def launches(self, n):
+        self._launches = n - (0 if self._native is None else _step.launches(self._native))
+
+    def _drop_native(self):
+        if self._native is not None:
+            self._launches, self._native = self.launches, None
+
+    def _make_native(self, logits, B, lo, lbs, P):
+        """Later calls of this form go to the library through one native call (host/step_module.c)."""
+        if (lo, lbs, B) != (0, self.batch_size, self.batch_size) or logits.dim() != 2 or self.stream is not None or _raw_stream is None \
+                or self._home is None or self._home < 0 or self._stream != self._home or lib is not _LIBRARY:
+            return
+        g, S = self._g, self._stop
+        self._native = _step.make(C.addressof(P), 0 if S is None else C.addressof(S), logits.dtype, _raw_stream, self._device_index,
+                                  self._home, B, g["temp"], self.penalty_type != 2 and g["pen"], g["minlen"])
+
     def _stream_ptr(self):
         return C.c_void_p(self._raw_stream())
 
@@ -135,6 +160,7 @@ class DynamicDecodeLayer:
         else:
             with torch.cuda.stream(self.stream):
                 t = make(*args, **kw)
+        self._drop_native()  # (it holds the addresses of what there was)
         on = self._raw_stream()
         if self._home != on:
             self._home = on if self._home is None else -1  # (several streams: none of them is the home of all)
@@ -182,6 +208,7 @@ class DynamicDecodeLayer:
         if beam_width != 1:
             return  # the beam layers have no set-up (BaseBeamSearchLayer.cu:123-127)
         B, dev, st = int(batch_size), self.device, self._stream_ptr()
+        self._drop_native()
         self.batch_size = B
         self._gate = {}
         a = runtime_args
@@ -277,6 +304,14 @@ class DynamicDecodeLayer:
 
     # ---- forward (DynamicDecodeLayer.cc:191-474, sampling branch) ---------------------------------
     def forward(self, outputs, inputs):
+        if self._native is not None and self.stream is None and not self.time_kernels:
+            done = _step.step(self._native, outputs, inputs, self.deadline_ms)
+            if done is True or done is False:
+                return done
+            if done is not None:
+                self._failed(done)
+            for g in self._gate.values():
+                g["ptrs"] = None  # (the argument block is not as _fill() left it)
         logits = inputs["logits"]
         shape = logits.shape
         if len(shape) == 3 and shape[1] > 1:
@@ -309,6 +344,8 @@ class DynamicDecodeLayer:
         lim = inputs.get("sequence_limit_length")
         if (sw is None and lim is None) or self.time_kernels or P.finished is None:
             self._sample(P)
+            if self._native is None and P.finished is not None and not self.time_kernels:
+                self._make_native(logits, B, lo, lbs, P)
             return self._stop_criteria(outputs, inputs, B, step, lbs, lo)
         # sampling, stop criteria and the wait for should_stop in one call
         S = self._stop
@@ -327,11 +364,16 @@ class DynamicDecodeLayer:
         S.sequence_limit_length = None if lim is None else lim.data_ptr()
         rc = lib.ftb200_decode_step(g["params_ref"], self._stop_ref, self.deadline_ms, self._should_stop_ref)
         if rc:
-            if rc == TIMEOUT:
-                _keep_until_done(self._result, self._run_stream())
-            check(rc)
-        self.launches += lib.ftb200_last_launch_count()
+            self._failed(rc)
+        self._launches += lib.ftb200_last_launch_count()
+        if self._native is None:
+            self._make_native(logits, B, lo, lbs, P)
         return bool(self._should_stop.value)
+
+    def _failed(self, rc):
+        if rc == TIMEOUT:
+            _keep_until_done(self._result, self._run_stream())
+        check(rc)
 
     # ---- beam search branch (DynamicDecodeLayer.cc:286-386 -> OnlineBeamSearchLayer::forward) -------
     def _forward_beam(self, outputs, inputs):
@@ -359,7 +401,7 @@ class DynamicDecodeLayer:
                 _ptr(out_ids), _ptr(outputs["parent_ids"]), B, lbs, K,
                 C.c_void_p(bw.data_ptr() if shared else bw.data_ptr() + ite * lbs * 2 * Lw * 4), int(shared), Lw,
                 ite * lbs, Vp, step, st))
-            self.launches += 1
+            self._launches += 1
 
         sub = 1 if self.has_diff_runtime_args else lbs
         n_sub = lbs // sub
@@ -384,7 +426,7 @@ class DynamicDecodeLayer:
             rc = lib.ftb200_beam_search_step(ref)
             if rc:
                 check(rc)
-            self.launches += lib.ftb200_last_launch_count()
+            self._launches += lib.ftb200_last_launch_count()
         return self._stop_criteria(outputs, inputs, B, step, lbs, ite * lbs, beam=K)
 
     def _fill_beam(self, outputs, inputs, key, B, K, Vp, L, mil, ite, lbs, sub, n_sub, es):
@@ -457,7 +499,7 @@ class DynamicDecodeLayer:
             None if sw is None else C.c_void_p(sw.data_ptr() + lo * 2 * L * 4), L, _ptr(outputs["finished"]),
             _ptr(lim), lo * beam, lbs, B, beam, step, _ptr(self._count_dev),
             C.c_void_p(self._count_host.data_ptr()), st))
-        self.launches += 1
+        self._launches += 1
         if lim is None:
             return False
         stop = C.c_int(0)
@@ -553,4 +595,4 @@ class DynamicDecodeLayer:
             self.kernel_events.append((e0, e1))
         else:
             check(lib.ftb200_decode_step_sampling(self._g["params_ref"]))
-        self.launches += lib.ftb200_last_launch_count()
+        self._launches += lib.ftb200_last_launch_count()

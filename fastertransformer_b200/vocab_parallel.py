@@ -140,14 +140,14 @@ class VocabParallelSampler(DynamicDecodeLayer):
         vocab = max(0, min(self.shard_size, self.vocab_size - off))
         P = self._params(outputs, inputs, shard_logits, max(vocab, 1), self.shard_size, self._record_halves)
         check(lib.ftb200_vocab_parallel_local(C.byref(P), off, self.cap, C.c_void_p(records.data_ptr())))
-        self.launches += 1
+        self._launches += 1
 
     def merge(self, outputs, inputs, gathered, logits_like):
         P = self._params(outputs, inputs, logits_like, self.vocab_size, self.shard_size * self.n_shards,
                          self._record_halves)
         check(lib.ftb200_vocab_parallel_merge(C.byref(P), C.c_void_p(gathered.data_ptr()), self.n_shards, self.cap,
                                               C.c_void_p(self._overflow.data_ptr())))
-        self.launches += 1
+        self._launches += 1
 
     def _buffers(self, B):
         shape = (B, 2 + self.cap)
@@ -184,10 +184,10 @@ class VocabParallelSampler(DynamicDecodeLayer):
             gathered = self._buffers(shards[0].shape[0])[1]
             ptrs = (C.c_void_p * len(shards))(*[sh.data_ptr() for sh in shards])
             check(lib.ftb200_vocab_parallel_shards(C.byref(P), ptrs, len(shards), self.shard_size, self.cap, gathered.data_ptr()))
-            self.launches += lib.ftb200_last_launch_count()
+            self._launches += lib.ftb200_last_launch_count()
             check(lib.ftb200_vocab_parallel_merge(C.byref(P), gathered.data_ptr(), self.n_shards, self.cap,
                                                   self._overflow.data_ptr()))
-            self.launches += 1
+            self._launches += 1
         if self._topp_rows is not None:
             self._sample_top_p_rows(outputs, inputs, torch.stack([sh.index_select(0, self._topp_rows) for sh in shards]))
             return
@@ -207,7 +207,7 @@ class VocabParallelSampler(DynamicDecodeLayer):
         self._full_rows.view(B, self.n_shards, self.shard_size).index_copy_(0, self._topp_rows, parts.permute(1, 0, 2))
         P = self._params(outputs, inputs, self._full_rows, self.vocab_size, Vp, "top_p")
         check(lib.ftb200_decode_step_sampling(C.byref(P)))
-        self.launches += lib.ftb200_last_launch_count()
+        self._launches += lib.ftb200_last_launch_count()
 
     def _undecided_rows(self, outputs, inputs):
         """Row indices (device tensor) the merge of this step left undecided, or None.  Reads the overflow
@@ -241,7 +241,7 @@ class VocabParallelSampler(DynamicDecodeLayer):
             if P.bad_words and not P.bad_words_shared:
                 P.bad_words = P.bad_words + r * 2 * P.bad_words_len * 4
             check(lib.ftb200_decode_step_sampling(C.byref(P)))
-            self.launches += 1
+            self._launches += 1
             self.resolved_rows += 1
 
     def overflow_count(self):
