@@ -176,8 +176,17 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
         A->area = area_within(budget, kSpAreaMax);
         return mixed || few ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, split_smem_bytes(A->slice, A->area));
     };
-    A->roomy = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kRoomyTwoPerSm && keeps(2, kRoomyTwoPerSm)));
-    if (!A->roomy) {
+    A->roomy    = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kRoomyTwoPerSm && keeps(2, kRoomyTwoPerSm)));
+    A->criteria = A->roomy;
+    if (!A->roomy && lgn >= 2 && least > kThreePerSm) {
+        // shared memory holds two CTAs on an SM, or one, whatever the registers: the roomy form for more rows than are resident
+        // too (96 x 128256 bf16 with both kinds of rows: 74 us a step, 85 with 80 registers and the criteria apart).  The
+        // last row does the criteria wherever it runs.
+        A->roomy    = 1;
+        A->criteria = mixed;
+        A->area     = area_within(least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem, kSpAreaMax);
+    }
+    else if (!A->roomy) {
         A->area = area_within(least <= kThreePerSm ? kThreePerSm : (least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem), kSpAreaMid);
     }
     return true;
@@ -388,6 +397,7 @@ static int plan_sampling(const ftb200_sampling_params* p, KParams& K, size_t& sm
     K.row_count_dev  = nullptr;
     K.row_flags      = nullptr;
     K.early          = 0;
+    K.stop_words     = nullptr;
     K.scratch        = (u64*)((char*)p->workspace + 256 + redo_list_bytes(p->local_batch_size));
     K.scratch_stride = scratch_stride_for(p->vocab_size_padded);
     return FTB200_OK;
@@ -498,15 +508,8 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
                              && p->vocab_size >= 16384 + 16 && (K.apply_rep ? p->step : 0) <= fast_max_history()
                              && (K.bad_words != nullptr ? K.bad_words_len : 0) <= fast_max_words();
     SplitArgs A{};
-    if (left_only) {
-        K.row_flags = (int*)((char*)p->workspace + 256);  // (as the split kernel of this step has set them)
-    }
-    else if (g_fast_path && choose_split(p, K, single_pass, &A)) {
-        A.redo_flags = (int*)((char*)p->workspace + 256);
-        if (A.roomy && stop != nullptr && stop->limit != nullptr) {
-            A.stop     = *stop;
-            *stop_done = true;
-        }
+    if (g_fast_path && choose_split(p, K, single_pass, &A)) {
+        A.redo_flags      = (int*)((char*)p->workspace + 256);
         const auto launch = [&](const SplitArgs& args) {
             switch (p->dtype) {
                 case FTB200_F32: return split_sampling_launch<FTB200_F32>(K, args, st);
@@ -514,18 +517,29 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
                 default: return split_sampling_launch<FTB200_BF16>(K, args, st);
             }
         };
-        rc = launch(A);
-        if (rc != FTB200_OK) {
-            return rc;
-        }
-        note_launch(1);
-        if (A.stop.limit != nullptr) {
-            return FTB200_OK;  // (the host hears of rows that are left and asks for them)
+        if (!left_only) {
+            SplitArgs F = A;
+            if (A.criteria && stop != nullptr && (stop->limit != nullptr || stop->stop_words != nullptr)) {
+                F.stop     = *stop;
+                *stop_done = true;
+            }
+            rc = launch(F);
+            if (rc != FTB200_OK) {
+                return rc;
+            }
+            note_launch(1);
+            if (F.stop.limit != nullptr) {
+                return FTB200_OK;  // (the host hears of rows that are left and asks for them)
+            }
         }
         // Areas below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row) leave the flat
         // rows' wide nuclei: those go over eight CTAs with areas as large as shared memory allows.  Where these are below half
         // a slice too (above 163000 columns) the general kernel's many CTAs serve the several rows left sooner.
-        SplitArgs B = A;
+        const bool words = !left_only && stop_done != nullptr && *stop_done;  // (no limit: who serves a row sees to its stop words)
+        SplitArgs  B     = A;
+        if (words) {
+            B.stop = *stop;
+        }
         if (wide_areas(p->vocab_size, &B) && K.topp_states != nullptr && A.area < A.slice / 2 && B.area >= B.slice / 2) {
             B.clusters = sm_count() / kSpMaxN < p->local_batch_size ? sm_count() / kSpMaxN : p->local_batch_size;
             rc         = launch(B);
@@ -535,6 +549,9 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
             note_launch(1);
         }
         K.row_flags = A.redo_flags;
+        if (words) {
+            K.stop_words = stop->stop_words, K.stop_words_len = stop->stop_words_len, K.stop_finished = stop->finished;
+        }
     }
     if (K.row_flags == nullptr) {
         FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));

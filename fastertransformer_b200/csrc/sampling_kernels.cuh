@@ -4010,6 +4010,27 @@ __device__ void process_row(const KParams& P, const Smem& S, int r, u64* gscratc
     }
 }
 
+// Stop words of row r against the sequence that ends with the step's token (kernels/stop_criteria_kernels.cu:24-80), by all
+// threads of the CTA that has just written it.
+static __device__ __noinline__ void row_stop_words(const KParams& P, const int* words, int len, uint8_t* finished, int r)
+{
+    const size_t row  = (size_t)P.ite * P.local_batch + r;
+    const int*   base = words + (size_t)r * 2 * len;
+    const int*   offs = base + len;
+    __syncthreads();
+    for (int i = threadIdx.x; i < len; i += kThreads) {
+        if (offs[i] < 0) {
+            continue;
+        }
+        const int start = i > 0 ? offs[i - 1] : 0, size = offs[i] - start;
+        if (P.step + 1 >= size
+            && tail_matches(P.output_ids, nullptr, base, start, size, P.step - (size - 1), (size_t)P.batch_size, row, 0, 1)) {
+            finished[row] = 1;
+        }
+    }
+    __syncthreads();
+}
+
 // Shared-memory map of the general row code (the size is computed by the entry point).
 __device__ __forceinline__ void map_general_smem(const KParams& P, Smem& S, unsigned char* smem)
 {
@@ -4067,6 +4088,9 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
             rec[0] = (u64)r, rec[1] = (u64)blockIdx.x, rec[2] = global_timer_ns();
         }
         process_row<DT>(P, S, r, gscratch, rec);
+        if (P.stop_words != nullptr) {
+            row_stop_words(P, P.stop_words, P.stop_words_len, P.stop_finished, r);
+        }
         if (rec != nullptr && threadIdx.x == 0) {
             rec[3] = global_timer_ns();
         }

@@ -63,6 +63,9 @@ struct KParams {
     // Rows the split kernel leaves: decode_sampling_kernel launched with row_flags != null serves the rows r with
     // row_flags[r] != 0.
     const int* row_flags;
+    const int* stop_words;      // [local_batch, 2, stop_words_len] or null: stop words of the rows so served
+    int        stop_words_len;
+    uint8_t*   stop_finished;   // [batch_size]
     int        early;  // decode_sampling_kernel may come up before the kernel in front of it in the stream has ended
     u64*     trace;           // optional per-row timeline: {row, CTA, start ns, end ns} per ticket, else null
     u64*     scratch;         // per-CTA candidate overflow area

@@ -20,7 +20,7 @@ constexpr u32 kRowsLeft = 0xffffffffu;
 struct StopArgs {
     const int*      stop_words;      // [local_batch, 2, stop_words_len] or null
     int             stop_words_len;
-    const uint32_t* limit;           // [batch_size] or null: then the criteria have a launch of their own
+    const uint32_t* limit;           // [batch_size] or null: then nothing is counted
     uint8_t*        finished;        // [batch_size], the whole batch
     u32*            arrived;         // one word, zero between calls
     u64*            result;          // page-locked host word: sequence << 32 | finished rows
@@ -32,8 +32,9 @@ struct SplitArgs {
     int  slice;       // floats of the slice area
     int  area;        // keys of the collection area
     int  roomy;       // the form with 128 registers
+    int  criteria;    // whether the launch may do the step's stop criteria (roomy form)
     int* redo_flags;  // [local_batch]: 1 when the row is left to another launch
-    StopArgs stop;    // (roomy form; without a limit nothing is done for the criteria)
+    StopArgs stop;    // (roomy form; without a limit the rows' stop words alone)
     int  clusters;    // 0: one per row; else so many, which look for rows with redo_flags set and serve those (roomy form)
 };
 

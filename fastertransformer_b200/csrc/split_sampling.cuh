@@ -1657,22 +1657,12 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
 {
     __shared__ u32 s_last, s_sum;
     const int      tid = threadIdx.x;
-    const size_t   row = (size_t)P.ite * P.local_batch + r;
     __syncthreads();
     if (T.stop_words != nullptr && decided) {
-        const int* base = T.stop_words + (size_t)r * 2 * T.stop_words_len;
-        const int* offs = base + T.stop_words_len;
-        for (int i = tid; i < T.stop_words_len; i += kThreads) {
-            if (offs[i] < 0) {
-                continue;
-            }
-            const int start = i > 0 ? offs[i - 1] : 0, size = offs[i] - start;
-            if (P.step + 1 >= size
-                && tail_matches(P.output_ids, nullptr, base, start, size, P.step - (size - 1), (size_t)P.batch_size, row, 0, 1)) {
-                T.finished[row] = 1;
-            }
-        }
-        __syncthreads();
+        row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
+    }
+    if (T.limit == nullptr) {
+        return;
     }
     if (tid == 0) {
         __threadfence();
@@ -1813,7 +1803,7 @@ __global__ void __launch_bounds__(kThreads, ROOMY ? 2 : 3) split_sampling_kernel
                 s_O.trace[3] = global_timer_ns();
             }
         }
-        if (ROOMY && rank == 0 && A.stop.limit != nullptr) {
+        if (ROOMY && rank == 0 && (A.stop.limit != nullptr || A.stop.stop_words != nullptr)) {
             sp_stop_criteria(P, A.stop, r, A.redo_flags, decided);
         }
         if (again) {

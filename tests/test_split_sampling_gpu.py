@@ -205,3 +205,45 @@ def test_empty_word_in_front_of_a_list(general, cuda_device):
     finally:
         lib.ftb200_set_single_pass(1)
     assert st["output_ids"][2].tolist() == [4001] * B
+
+
+@pytest.mark.parametrize("limit", [True, False])
+@pytest.mark.parametrize("dtype,V,B", [(F32, 50257, 6), (BF16, 128256, 9), (BF16, 128256, 40), (F32, 200000, 3)])
+def test_stop_criteria_with_rows_left_to_another_launch(dtype, V, B, limit, cuda_device):
+    """Stop words, and the count behind a length limit, when some rows' nuclei leave the first launch's areas: who serves a
+    row sees to its words, and the host hears of the rows that are left."""
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    got = []
+    for general in (1, 0):
+        g = torch.Generator(device=cuda_device)
+        g.manual_seed(V + B)
+        layer = DynamicDecodeLayer(V, V, dtype, cuda_device)
+        layer.setup(B, 1, {"runtime_top_k": np.resize(np.asarray([0, 0, 5], np.uint32), B),
+                           "runtime_top_p": np.resize(np.asarray([0.99, 0.3, 0.9], np.float32), B),
+                           "random_seed": np.arange(B).astype(np.uint64)})
+        st = {"output_ids": torch.ones(12, B, dtype=torch.int32, device=cuda_device),
+              "finished": torch.arange(B, device=cuda_device) == B // 2,
+              "sequence_length": torch.full((B,), 8, dtype=torch.int32, device=cuda_device)}
+        stops = []
+        lib.ftb200_set_single_pass(1 - general)
+        try:
+            for s in range(3):
+                x = torch.randn(B, V, generator=g, device=cuda_device) * 0.5
+                x[B - 1, :] = 0.0
+                hot = torch.arange(B, device=cuda_device) % 3 != 0  # these stop by their second word; rows 0, 3, ... are flat
+                x[hot, 77] = 30.0
+                words = torch.tensor([[[5, 77, 0], [1, 2, -1]]] * B, dtype=torch.int32, device=cuda_device)
+                words[1::2, 0, 1] = 78 if s == 0 else 77
+                kw = {"sequence_limit_length": torch.full((B,), 10, dtype=torch.int32, device=cuda_device)} if limit else {}
+                stop = layer.forward(st, {"logits": x.to(dtype), "step": 8 + s, "max_input_length": 8, "ite": 0, "local_batch_size": B,
+                                          "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device),
+                                          "stop_words_list": words, **kw})
+                stops.append(bool(stop))
+                stops.append(st["finished"].cpu().numpy().copy())
+            torch.cuda.synchronize()
+        finally:
+            lib.ftb200_set_single_pass(1)
+        got.append({k: v.cpu().numpy() for k, v in st.items()} | {"stops": np.hstack([np.atleast_1d(v) for v in stops])})
+    for k, v in got[0].items():
+        np.testing.assert_array_equal(got[1][k], v, err_msg=k)
+    assert got[0]["stops"][1 + 0:1 + B].any() and not got[0]["stops"][1:1 + B].all()
