@@ -2019,54 +2019,78 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
                 }
                 at += __shfl_sync(0xffffffffu, incl, 31);
             }
+            const int k16 = (k + 15) & ~15;  // (zeros behind the last term change neither the sum nor the walk)
+            if (k + lane < k16) {
+                flat[k + lane] = 0.0f;
+            }
             __syncwarp();
             trace_mark(trace, 8);
+            // Dependent adds in the reference's order, by one lane: sixteen terms a round, eight on their way while eight are added.
+            // The walk leaves its running values where the terms were; they only fall, so the first one that ends the
+            // reference's loop lies in the last round and is found by the warp, as is the run that it belongs to (1024 x
+            // 128256 bf16 with both kinds of rows: 182 us a step, 200 with a walk tested term by term and a search run by run).
+            int walked = 0;
             if (lane == 0) {
-                // dependent adds in the reference's order; operands come from shared memory eight at a time
-                const int k8  = k & ~7;
-                float     sum = 0.0f;
-                for (int i = 0; i < k8; i += 8) {
-                    const float4 a = *(const float4*)(flat + i), b = *(const float4*)(flat + i + 4);
-                    sum += a.x, sum += a.y, sum += a.z, sum += a.w;
-                    sum += b.x, sum += b.y, sum += b.z, sum += b.w;
-                }
-                for (int i = k8; i < k; ++i) {
-                    sum += flat[i];
+                float  sum = 0.0f;
+                float4 v0 = *(const float4*)flat, v1 = *(const float4*)(flat + 4);
+#pragma unroll 1
+                for (int i = 0; i < k16; i += 16) {
+                    const float4 w0 = *(const float4*)(flat + i + 8), w1 = *(const float4*)(flat + i + 12);
+                    sum += v0.x, sum += v0.y, sum += v0.z, sum += v0.w;
+                    sum += v1.x, sum += v1.y, sum += v1.z, sum += v1.w;
+                    const int nx = i + 16 < k16 ? i + 16 : 0;
+                    v0 = *(const float4*)(flat + nx), v1 = *(const float4*)(flat + nx + 4);
+                    sum += w0.x, sum += w0.y, sum += w0.z, sum += w0.w;
+                    sum += w1.x, sum += w1.y, sum += w1.z, sum += w1.w;
                 }
                 float rand_num = H.u * H.top_p * sum;
-                int   pick     = k - 1;
-                for (int i = 0; i < k; i += 8) {
-                    float v[8];
+                auto  walk4    = [&](const float4& x, int i) {
+                    float4 r;
+                    r.x                  = rand_num - x.x;
+                    r.y                  = r.x - x.y;
+                    r.z                  = r.y - x.z;
+                    r.w                  = r.z - x.w;
+                    rand_num             = r.w;
+                    *(float4*)(flat + i) = r;
+                };
+#pragma unroll 1
+                do {
+                    const float4 w0 = *(const float4*)(flat + walked + 8), w1 = *(const float4*)(flat + walked + 12);
+                    walk4(v0, walked);
+                    walk4(v1, walked + 4);
+                    const int nx = walked + 16 < k16 ? walked + 16 : 0;
+                    v0 = *(const float4*)(flat + nx), v1 = *(const float4*)(flat + nx + 4);
+                    walk4(w0, walked + 8);
+                    walk4(w1, walked + 12);
+                    walked += 16;
+                } while (walked < k16 && !(rand_num <= 0.0f));
+            }
+            walked = __shfl_sync(0xffffffffu, walked, 0);
+            __syncwarp();
+            const int  i0   = walked - 16 + lane;
+            const bool ends = lane < 16 && i0 < k && flat[i0] <= 0.0f;
+            const u32  hit  = __ballot_sync(0xffffffffu, ends);
+            const int  pick = hit != 0 ? walked - 16 + __ffs(hit) - 1 : k - 1;
+            // value of the picked entry: the run that holds position `pick`
+            int acc = 0, prun = 0;
+            for (int p0 = 0; p0 < nruns; p0 += 32) {
+                const int p    = p0 + lane;
+                int       incl = p < nruns ? (int)fc[p] : 0;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        v[j] = i + j < k ? flat[i + j] : 0.0f;
-                    }
-                    bool found = false;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if (!found && i + j < k) {
-                            rand_num -= v[j];
-                            if (rand_num <= 0.0f || i + j == k - 1) {
-                                pick  = i + j;
-                                found = true;
-                            }
-                        }
-                    }
-                    if (found) {
-                        break;
-                    }
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                    incl += lane >= o ? t : 0;
                 }
+                const u32 beyond = __ballot_sync(0xffffffffu, acc + incl > pick);
+                if (beyond != 0) {
+                    prun = p0 + __ffs(beyond) - 1;
+                    break;
+                }
+                acc += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (lane == 0) {
                 s_pick_idx = pick;
-                // value of the picked entry: the run that holds position `pick`
-                int acc = 0, prun = 0;
-                for (int p = 0; p < nruns; ++p) {
-                    acc += (int)fc[p];
-                    if (acc > pick) {
-                        prun = p;
-                        break;
-                    }
-                }
-                s_vsel = fe[prun];
+                s_vsel     = fe[prun];
             }
         }
         if (lane == 0) {
