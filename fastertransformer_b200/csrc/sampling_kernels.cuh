@@ -4365,10 +4365,32 @@ vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nran
     S.hist  = (u32*)(S.val2 + 1024);
     S.flags = nullptr, S.hash = nullptr, S.spre = nullptr, S.sfin = nullptr, S.hitq = nullptr, S.nhit = nullptr;
     const int tid = threadIdx.x;
+    // A row's arguments are loaded while the row before it is worked on, all at once.
+    struct Args {
+        u32     k;
+        float   p;
+        int     end;
+        uint8_t skip_k, skip_p, fin;
+    };
+    auto args_of = [&](int r) {
+        Args a{0u, 1.0f, 0, 0, 0, 0};
+        if (r < P.local_batch) {
+            a.skip_k = P.topk_states == nullptr ? 1 : (P.topk_skip != nullptr ? P.topk_skip[r] : 0);
+            a.skip_p = P.topp_states == nullptr ? 1 : (P.topp_skip != nullptr ? P.topp_skip[r] : 0);
+            a.fin    = P.finished != nullptr ? P.finished[r] : 0;
+            a.end    = P.end_ids[r];
+            a.k      = P.topk_states != nullptr ? P.topk_ks[r] : 0u;
+            a.p      = P.topk_states != nullptr ? P.topk_ps[r] : 1.0f;
+        }
+        return a;
+    };
+    Args next = args_of((int)blockIdx.x);
     for (int r = blockIdx.x; r < P.local_batch; r += gridDim.x) {
         __syncthreads();
-        const bool by_topk = P.topk_states != nullptr && !(P.topk_skip != nullptr && P.topk_skip[r]);
-        const bool by_topp = !by_topk && P.topp_states != nullptr && !(P.topp_skip != nullptr && P.topp_skip[r]);
+        const Args a       = next;
+        next               = args_of(r + (int)gridDim.x);  // (no CTA writes another row's)
+        const bool by_topk = a.skip_k == 0;
+        const bool by_topp = !by_topk && a.skip_p == 0;
         if (by_topp) {
             vp_merge_topp_row<DT>(P, S, gathered, nranks, overflow, r);
             continue;
@@ -4378,10 +4400,10 @@ vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nran
         }
         RowOut O;
         O.r      = r;
-        O.end_id = P.end_ids[r];
+        O.end_id = a.end;
         O.id_out = P.output_ids + (size_t)P.step * P.batch_size + (size_t)P.ite * P.local_batch + r;
         O.trace  = nullptr;
-        const bool fin = P.finished != nullptr ? P.finished[r] != 0 : false;
+        const bool fin = a.fin != 0;
         __syncthreads();
         if (fin) {
             if (tid == 0) {
@@ -4389,9 +4411,9 @@ vp_merge_kernel(const __grid_constant__ KParams P, const u64* gathered, int nran
             }
             continue;
         }
-        int k = (int)P.topk_ks[r];
+        int k = (int)a.k;
         k     = k < 1 ? 1 : (k > kMaxTopK ? kMaxTopK : k);
-        const float top_p = P.topk_ps[r];
+        const float top_p = a.p;
         if (tid == kThreads - 1) {
             s_before_k = P.topk_states[r];
             s_u        = draw_uniform(P.topk_states, r);

@@ -353,16 +353,20 @@ vp_select_kernel(const __grid_constant__ KParams P, const __grid_constant__ VpAr
                 }
                 lo = __reduce_min_sync(0xffffffffu, lo);
                 hi = __reduce_max_sync(0xffffffffu, hi);
+                // two bits a round: three bounds counted at once, ten bits each (a bound above the least one: at most NT - 1 reach it)
+                // (one bit a round: 295.9 us for 2048 rows of 8 x 32000 bf16, 292.7 so and with the merge's arguments ahead)
                 while (lo < hi) {
-                    const u32 mid = (lo + hi + 1) >> 1;
-                    u32       c   = 0;
+                    const u32 q = (hi - lo + 3) >> 2, m1 = lo + q, m2 = m1 + q, m3 = m2 + q;
+                    u32       c = 0;
 #pragma unroll
                     for (int i = 0; i < NT / 32; ++i) {
-                        c += mine[i] >= mid ? 1u : 0u;
+                        c += (mine[i] >= m1 ? 1u : 0u) + (mine[i] >= m2 ? 1u << 10 : 0u) + (mine[i] >= m3 ? 1u << 20 : 0u);
                     }
-                    c  = __reduce_add_sync(0xffffffffu, c);
-                    lo = c >= (u32)T.k ? mid : lo;
-                    hi = c >= (u32)T.k ? hi : mid - 1;
+                    c            = __reduce_add_sync(0xffffffffu, c);
+                    const bool a1 = (c & 1023u) >= (u32)T.k, a2 = (c >> 10 & 1023u) >= (u32)T.k, a3 = c >> 20 >= (u32)T.k;
+                    const u32  up = a3 ? hi : (a2 ? m3 : (a1 ? m2 : m1)) - 1;
+                    lo            = a3 ? m3 : (a2 ? m2 : (a1 ? m1 : lo));
+                    hi            = up < hi ? up : hi;
                 }
                 if (lane == 0) {
                     s_thr = lo;

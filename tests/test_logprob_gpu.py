@@ -170,3 +170,28 @@ def test_ragged_lengths_of_many_sequences(batch, bf):
     live = valid_mask(lengths, max_len, bf)
     assert np.abs(lp - np.asarray(want_lp).ravel()[: lp.size])[live].max() < TOL
     assert np.abs(cum - want_cum).max() < TOL * max_len
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("vocab,vp", [(1, 8), (7, 8), (2049, 2056), (8195, 8195), (50257, 50257)])
+def test_extreme_values_of_16_bit_rows(dtype, vocab, vp):
+    """-infinity, the type's lowest value, its largest and values of very different size, at each remainder of the pairs."""
+    max_len, batch = 6, 4
+    g = torch.Generator().manual_seed(vocab)
+    x = torch.randn(max_len, batch, vp, generator=g) * 4
+    low = torch.finfo(dtype).min
+    x[1, :, ::2] = -float("inf")
+    x[2, :, 1::3] = low
+    x[3] = x[3] * 100
+    x[4, 0], x[4, 1, 0], x[4, 2] = low, torch.finfo(dtype).max, 0.0
+    for t in range(max_len):
+        x[t, :, vocab - 1] = 1.5  # (the token that is scored below)
+    x = x.to(dtype)
+    ids = torch.full((max_len, batch), vocab - 1, dtype=torch.int32)
+    lengths = torch.full((batch,), max_len, dtype=torch.int32)
+    cum, lp = run_ours(x.cuda(), ids.cuda(), lengths.cuda(), vocab, False)
+    want = torch.log_softmax(x[:max_len - 1, :, :vocab].double(), -1)[..., vocab - 1].numpy()
+    # fp32 sums of the exponentials (2^-24 relative per term of a tree) and a result rounded to fp32
+    tol = 1e-6 * 8 + np.abs(want) * 2.0 ** -22
+    assert (np.abs(lp.reshape(max_len - 1, batch) - want) <= tol).all()
+    assert (np.abs(cum - want.sum(0)) <= tol.sum(0) * 2).all()
