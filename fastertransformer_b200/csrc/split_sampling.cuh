@@ -11,10 +11,10 @@
 //
 // What bounds it: latency.  A row takes six to ten cluster barriers (0.5 us each) and about six sweeps over its shared
 // memory; a CTA-per-row kernel walks eight times as many columns with the same 256 threads.  Measured on B200, one row
-// alone on its SMs: arg-max of 32000 columns 5 us, k = 50 of 50257 fp32 17 us, a nucleus of 50257 fp32 22 us (the general
-// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 10 us (k = 1) to 60 us (25000-column nucleus).  Batch
-// of 64 x 50257 fp32 top-p: 52 us a step (61 with the nucleus scattered by list and sorted in one unrolled pass); 48 x 51200
-// half with bias and log-probs: 67 us (83 so); 24 steps of 16 x 128256 bf16: 1707 us (1923 so).
+// alone on its SMs: arg-max of 32000 columns 4 us, k = 50 of 50257 fp32 13 us, a nucleus of 50257 fp32 19 us (the general
+// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 5 us (k = 1) to 60 us (25000-column nucleus).  Batch
+// of 64 x 50257 fp32 top-p: 43 us a step; 48 x 51200 half with bias and log-probs: 52 us; 24 steps of 16 x 128256 bf16: 1200 to
+// 1370 us.  Before the nucleus was placed by bin, sorted by short loops and the general row code taken out: 60, 83, 1600 to 1930.
 //
 // Code size matters: a row runs through most of this code once, so a loop that is unrolled for the largest case waits for
 // its instructions in every case.
@@ -535,7 +535,7 @@ static __device__ __noinline__ void sp_scatter_keys(const float* y, int ny, floa
 //
 // The keys go to `tmp` by sub-bucket and come back in order: three short loops, because a row passes through this code once and
 // an unrolled form waits for its instructions.  900 keys: 6 us, 4850 keys: 19 us (before, keys held in registers by code
-// unrolled for 10240 of them: 20 to 26 us).  Returns false when a long sub-bucket of many values would have to be ordered.
+// unrolled for 10240 of them: 20 to 26 us).  Above half of the area it goes stretch by stretch: 30 us for 7500 keys.  Returns false when a long sub-bucket of many values would have to be ordered.
 constexpr int kSpShort = 24;   // keys of a sub-bucket that every thread orders for itself
 constexpr int kSpLists = 256;  // words for the list of longer ones
 
@@ -570,8 +570,16 @@ static __device__ __forceinline__ void sp_sub_prefix(u32* sub, int words)
 }
 
 // n <= 25 * kSpLists
-static __device__ __noinline__ bool sp_sort_keys(float* a, float* tmp, u32* sub, const u32* excl, u32* list, u32 start, int n, float maxv)
+// words behind the counters that sp_sort_keys needs for n keys (two bit maps)
+__device__ __forceinline__ int sp_sort_bits(int n)
 {
+    return 2 * (n / 32 + 2);
+}
+
+static __device__ __noinline__ bool sp_sort_keys(float* a, float* tmp, u32* sub, u32* bits, const u32* excl, u32* list, u32 start, int n,
+                                                 float maxv, bool ties)
+{
+    FTB_ASSUME_SHARED(bits);
     FTB_ASSUME_SHARED(a);
     FTB_ASSUME_SHARED(tmp);
     FTB_ASSUME_SHARED(sub);
@@ -583,60 +591,137 @@ static __device__ __noinline__ bool sp_sort_keys(float* a, float* tmp, u32* sub,
     for (int i = tid; i < words; i += kThreads) {
         sub[i] = 0;
     }
+    u32* const edge = bits;              // a bit where a sub-bucket starts
+    u32* const turn = bits + n / 32 + 2;  // a bit where a key differs from the one in front of it
+#pragma unroll 1
+    for (int i = tid; i < sp_sort_bits(n); i += kThreads) {
+        bits[i] = i == 0 ? 1u : 0u;
+    }
     if (tid == 0) {
         s_nlong = 0;
     }
     __syncthreads();
     // The 32 lanes of a warp take their keys from 32 places far apart: neighbours lie in the same sub-bucket.
     const int seg = ((n + 31) / 32) | 1;
+    // Four keys at a time: their loads and atomics are on their way together.
+    constexpr int kAtOnce = 4;
+    float         v[kAtOnce];
+    u32           s[kAtOnce];
+    auto          take = [&](int j) {
+        u32 in = 0;
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+            const int  p  = lane * seg + j + q * kWarps;
+            const bool ok = (j + q * kWarps < seg) & (p < n);
+            v[q]          = ok ? a[p] : maxv;
+            in |= ok ? 1u << q : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+            s[q] = sp_sub_bucket(excl, v[q], maxv, start, n);
+        }
+        return in;
+    };
 #pragma unroll 1
-    for (int j = tid >> 5; j < seg; j += kWarps) {
-        const int p = lane * seg + j;
-        if (p < n) {
-            const u32 s = sp_sub_bucket(excl, a[p], maxv, start, n);
-            smem_add(&sub[s >> 1], 1u << (16 * (s & 1u)));
+    for (int j = tid >> 5; j < seg; j += kAtOnce * kWarps) {
+        const u32 in = take(j);
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+            if (in >> q & 1u) {
+                smem_add(&sub[s[q] >> 1], 1u << (16 * (s[q] & 1u)));
+            }
         }
     }
     __syncthreads();
     sp_sub_prefix(sub, words);
 #pragma unroll 1
-    for (int j = tid >> 5; j < seg; j += kWarps) {
-        const int p = lane * seg + j;
-        if (p < n) {
-            const float v   = a[p];
-            const u32   s   = sp_sub_bucket(excl, v, maxv, start, n);
-            const u32   old = atomicAdd(&sub[s >> 1], 1u << (16 * (s & 1u)));
-            tmp[(old >> (16 * (s & 1u))) & 0xffffu] = v;
+    for (int j = tid >> 5; j < seg; j += kAtOnce * kWarps) {
+        const u32 in = take(j);
+        u32       old[kAtOnce];
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+            old[q] = in >> q & 1u ? atomicAdd(&sub[s[q] >> 1], 1u << (16 * (s[q] & 1u))) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+            if (in >> q & 1u) {
+                tmp[(old[q] >> (16 * (s[q] & 1u))) & 0xffffu] = v[q];
+            }
         }
     }
     __syncthreads();
-    // (the counters now hold where their sub-bucket ends)
-    auto end_of = [&](u32 s) { return (int)((sub[s >> 1] >> (16 * (s & 1u))) & 0xffffu); };
+    // The counters now hold where their sub-bucket ends.  16-bit logits fill most sub-buckets with equal keys, which stay where
+    // they are: two bit maps tell (the place of every key looked for among up to 24: 16.7 us for the slowest row's sort of 48 x
+    // 51200 half, 14.8 so).
 #pragma unroll 1
-    for (int p = tid; p < n; p += kThreads) {
-        const float v  = tmp[p];
-        const u32   s  = sp_sub_bucket(excl, v, maxv, start, n);
-        const int   lo = s > 0 ? end_of(s - 1u) : 0, hi = end_of(s);
-        if (hi - lo > kSpShort) {
-            if (p == lo) {
-                list[atomicAdd(&s_nlong, 1u)] = (u32)lo | ((u32)(hi - lo) << 16);  // (at most n / 25 of them)
+    for (int i = tid; i < words; i += kThreads) {
+        const u32 c = sub[i], e0 = c & 0xffffu, e1 = c >> 16;
+        atomicOr(&edge[e0 >> 5], 1u << (e0 & 31u));
+        atomicOr(&edge[e1 >> 5], 1u << (e1 & 31u));
+    }
+    if (ties) {
+#pragma unroll 1
+        for (int w = tid >> 5; w * 32 < n; w += kWarps) {
+            const int   p = w * 32 + lane;
+            const float x = tmp[p < n ? p : n - 1], y = tmp[p == 0 ? 0 : (p < n ? p - 1 : n - 1)];
+            const u32   t = __ballot_sync(0xffffffffu, x != y);
+            if (lane == 0) {
+                turn[w] = t;
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int w = tid >> 5; w * 32 < n; w += kWarps) {
+        const int p = w * 32 + lane;
+        if (p >= n) {
+            break;
+        }
+        const float x  = tmp[p];
+        const u64   up = (2ull << lane) - 1ull, down = (2ull << (32 + lane)) - 1ull;  // bits up to this key, from this word and the one before
+        const u32   e0 = w > 0 ? edge[w - 1] : 0u, e1 = edge[w], e2 = edge[w + 1];
+        const u32   t0 = w > 0 ? turn[w - 1] : 0u, t1 = turn[w], t2 = turn[w + 1];
+        const u64   eb = (((u64)e1 << 32) | e0) & down, ea = (((u64)e2 << 32) | e1) & ~up;
+        const u64   tb = (((u64)(t1 | e1) << 32) | (t0 | e0)) & down, ta = (((u64)(t2 | e2) << 32) | (t1 | e1)) & ~up;
+        const int   lo = w * 32 + 31 - __clzll((long long)eb), hi = w * 32 - 1 + __ffsll((long long)ea);
+        const bool  seen = eb != 0 && ea != 0;  // (both ends within the three words)
+        if (seen && (hi - lo == 1
+                     || (ties && __clzll((long long)tb) == __clzll((long long)eb) && __ffsll((long long)ta) == __ffsll((long long)ea)))) {
+            a[p] = x;
+            continue;
+        }
+        if (!seen || hi - lo > kSpShort) {
+            if (e1 >> lane & 1u) {
+                int to = w + 1;
+                u32 e  = e2;
+                if (ea != 0) {
+                    to = hi;
+                }
+                else {
+                    while (e == 0) {  // (position n has a bit)
+                        e = edge[++to];
+                    }
+                    to = to * 32 + __ffs(e) - 1;
+                }
+                list[atomicAdd(&s_nlong, 1u)] = (u32)p | ((u32)(to - p) << 16);  // (at most n / 25 of them)
             }
             continue;
         }
+        // the larger ones, and the equal ones in front
         int to = lo;
 #pragma unroll 1
         for (int j = lo; j < hi; j += 4) {
-            float x[4];
+            float y[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                x[q] = j + q < hi ? tmp[j + q] : -INFINITY;
+                y[q] = j + q < hi ? tmp[j + q] : -INFINITY;
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                to += (x[q] > v ? 1 : 0) | (x[q] == v && j + q < p ? 1 : 0);
+                to += (y[q] > x ? 1 : 0) | (y[q] == x && j + q < p ? 1 : 0);
             }
         }
-        a[to] = v;
+        a[to] = x;
     }
     __syncthreads();
     // A long sub-bucket holds few distinct values (16-bit logits: a run of equal ones, a penalised column's beside it): a warp
@@ -645,8 +730,19 @@ static __device__ __noinline__ bool sp_sort_keys(float* a, float* tmp, u32* sub,
 #pragma unroll 1
     for (u32 w = (u32)(tid >> 5); w < s_nlong; w += kWarps) {
         const int lo = (int)(list[w] & 0xffffu), m = (int)(list[w] >> 16);
-        u32       below = 0xffffffffu;
-        int       pos = 0;
+        // (all equal, as a rule)
+        const float first = tmp[lo];
+        bool        same  = true;
+        for (int i = lane; i < m; i += 32) {
+            same &= tmp[lo + i] == first;
+            a[lo + i] = first;
+        }
+        if (__all_sync(0xffffffffu, same)) {
+            continue;
+        }
+        __syncwarp();
+        u32 below = 0xffffffffu;
+        int pos   = 0;
         for (int d = 0; d < 256 && pos < m; ++d) {
             u32 top = 0, c = 0;
             for (int i = lane; i < m; i += 32) {
@@ -672,7 +768,8 @@ static __device__ __noinline__ bool sp_sort_keys(float* a, float* tmp, u32* sub,
 // All of an owner's keys: at once while they fill at most half of the area (its other half is tmp), else stretches of whole bins
 // one after the other, with tmp in the words behind the counters (`sub` to the end of `hist`).  A bin that is larger than a
 // stretch holds few distinct values (16-bit logits); more than 32 of them are given up.
-static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* hist, u32 start, int n, float maxv, int cap)
+static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* excl, u32* hist, u32 start, int n, float maxv, int cap,
+                                                 bool ties)
 {
     __shared__ u32 s_end, s_top, s_cnt, s_val[32], s_num[32];
     FTB_ASSUME_SHARED(a);
@@ -680,9 +777,10 @@ static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* 
     const int  tid = threadIdx.x, lane = tid & 31;
     u32* const list = hist + kSpBins - kSpLists;
     if (n <= cap / 2) {
-        return sp_sort_keys(a, a + cap / 2, sub, excl, list, start, n, maxv);
+        return sp_sort_keys(a, a + cap / 2, sub, hist, excl, list, start, n, maxv, ties);  // (the maps fit: n / 16 words)
     }
-    const int most = (cap / 4 + kSpBins - kSpLists) * 4 / 5 - 4;  // (a quarter of a word for the counters, one for the key)
+    // (a quarter of a word for the counters, a sixteenth for the maps, one for the key)
+    const int most = (cap / 4 + kSpBins - kSpLists - 16) * 16 / 21;
     bool      ok   = true;
     for (int at = 0; at < n;) {
         int cnt = n - at;
@@ -758,7 +856,8 @@ static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* 
                 continue;
             }
         }
-        ok = sp_sort_keys(a + at, (float*)(sub + cnt / 4 + 2), sub, excl, list, start + (u32)at, cnt, maxv) && ok;
+        ok = sp_sort_keys(a + at, (float*)(sub + cnt / 4 + 2 + sp_sort_bits(cnt)), sub, sub + cnt / 4 + 2, excl, list, start + (u32)at, cnt, maxv,
+                          ties) && ok;
         at += cnt;
     }
     __syncthreads();
@@ -798,24 +897,29 @@ struct SpKeys {
     int owners;
     u32 start[kSpMaxN + 1];  // first position of every owner, then the total
 };
-__device__ __forceinline__ float sp_key_at(const SpKeys& K, u32 pos)
+// owner of a position (loads that do not wait for one another: with a search the aggregates of a wide row's chunks took 4.5 us, 2.3
+// so)
+__device__ __forceinline__ int sp_key_owner(const SpKeys& K, u32 pos)
 {
     int o = 0;
-    while (o + 1 < K.owners && pos >= K.start[o + 1]) {
-        ++o;
+#pragma unroll
+    for (int q = 1; q < kSpMaxN; ++q) {
+        o += pos >= K.start[q] ? 1 : 0;
     }
+    return o < K.owners ? o : K.owners - 1;
+}
+__device__ __forceinline__ float sp_key_at(const SpKeys& K, u32 pos)
+{
+    const int o = sp_key_owner(K, pos);
     return __uint_as_float(dld_u32(cluster_addr(K.area + 4u * (pos - K.start[o]), (u32)o)));
 }
 // eight keys of chunk c for this lane; `own`: this CTA's rank (0 where the keys lie in this CTA)
 __device__ __forceinline__ void sp_load8(const SpKeys& K, u32 c, int lane, int own, float* x)
 {
     const u32 total = K.start[K.owners], p0 = c * 256u + (u32)lane * 8u;
-    int       o = 0;
-    while (o + 1 < K.owners && p0 >= K.start[o + 1]) {
-        ++o;
-    }
-    if (p0 + 8u <= K.start[o + 1]) {
-        const u32 at = K.area + 4u * (p0 - K.start[o]);
+    const int o     = sp_key_owner(K, p0);
+    const u32 end   = K.start[o + 1], at = K.area + 4u * (p0 - K.start[o]);
+    if (p0 + 8u <= end) {
         if (o == own) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -831,9 +935,17 @@ __device__ __forceinline__ void sp_load8(const SpKeys& K, u32 c, int lane, int o
         }
     }
     else {
+        u32 from[8];  // (all places first: their loads are on their way together)
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            x[i] = p0 + (u32)i < total ? sp_key_at(K, p0 + (u32)i) : 0.0f;
+            const u32 p = p0 + (u32)i < total ? p0 + (u32)i : total - 1u;
+            const int q = sp_key_owner(K, p);
+            from[i]     = cluster_addr(K.area + 4u * (p - K.start[q]), (u32)q);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float y = __uint_as_float(dld_u32(from[i]));
+            x[i]          = p0 + (u32)i < total ? y : 0.0f;
         }
     }
 }
@@ -1550,7 +1662,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     if (rank < owners) {
         float* const a   = (float*)M.area;
         const int    cnt = (int)(K.start[rank + 1] - K.start[rank]);
-        bool         bad = !sp_sort_area(a, M.sub, excl, M.hist, K.start[rank], cnt, maxv, M.area_cap);
+        bool         bad = !sp_sort_area(a, M.sub, excl, M.hist, K.start[rank], cnt, maxv, M.area_cap, DT != FTB200_F32);
         for (int i = tid; i < cnt; i += kThreads) {
             a[i] = sp_prob<DT>(a[i], maxv, denom);
         }
