@@ -242,27 +242,53 @@ __device__ __forceinline__ float sp_load_slice(const KParams& P, const Xf& X, co
         }
     }
     else {
-        // a row that starts between two 16-byte boundaries: one column per load, eight in flight
-        constexpr int U  = 8;
-        const int     ny = nchunk << lgvt;
-        for (int i0 = tid; i0 < ny; i0 += kThreads * U) {
-            u32 q[U];
+        // a row that starts between two 16-byte boundaries: one column per load, eight in flight, a bias beside them (246 x 114514 bf16
+        // with a bias that was sent for once a column had come: 226 us a step, 162 so)
+        constexpr int U    = 8;
+        const int     ny   = nchunk << lgvt;
+        Xf            T    = X;
+        T.bias             = nullptr;  // (it is added here)
+        auto walk = [&](auto with_bias) {
+            constexpr bool kBias = decltype(with_bias)::value;
+            for (int i0 = tid; i0 < ny; i0 += kThreads * U) {
+                u32 q[U], b[kBias ? U : 1];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
-                q[u]        = 0;
-                if (i < ny && v < vocab) {
-                    q[u] = DT == FTB200_F32 ? __ldg((const u32*)rowp + v) : (u32)__ldg((const unsigned short*)rowp + v);
+                for (int u = 0; u < U; ++u) {
+                    const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
+                    q[u]        = 0;
+                    if (i < ny && v < vocab) {
+                        q[u] = DT == FTB200_F32 ? __ldg((const u32*)rowp + v) : (u32)__ldg((const unsigned short*)rowp + v);
+                        if (kBias) {
+                            b[kBias ? u : 0] = DT == FTB200_F32 ? __ldg((const u32*)X.bias + v) : (u32)__ldg((const unsigned short*)X.bias + v);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
+                    if (i < ny) {
+                        if (!kBias) {
+                            y[i] = v < vocab ? temp_value<DT>(T, q[u], v) : -INFINITY;
+                        }
+                        else if (v >= vocab) {
+                            y[i] = -INFINITY;
+                        }
+                        else if (DT == FTB200_BF16) {
+                            y[i] = (__uint_as_float(q[u] << 16) + __uint_as_float(b[kBias ? u : 0] << 16)) * X.inv_t;
+                        }
+                        else {
+                            y[i] = temp_value<DT>(T, sp_add_bias<DT>(q[u], b[kBias ? u : 0]), v);
+                        }
+                        best = fmaxf(best, y[i]);
+                    }
                 }
             }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
-                if (i < ny) {
-                    y[i] = v < vocab ? temp_value<DT>(X, q[u], v) : -INFINITY;
-                    best = fmaxf(best, y[i]);
-                }
-            }
+        };
+        if (X.apply_temp && X.bias != nullptr) {
+            walk(std::true_type{});
+        }
+        else {
+            walk(std::false_type{});
         }
     }
     return best;

@@ -247,3 +247,33 @@ def test_stop_criteria_with_rows_left_to_another_launch(dtype, V, B, limit, cuda
     for k, v in got[0].items():
         np.testing.assert_array_equal(got[1][k], v, err_msg=k)
     assert got[0]["stops"][1 + 0:1 + B].any() and not got[0]["stops"][1:1 + B].all()
+
+
+@pytest.mark.parametrize("dtype,V,B", [(F32, 16385, 5), (F16, 50257, 6), (BF16, 32001, 7), (BF16, 114514, 3), (F16, 4096, 2)])
+def test_bias_beside_rows_off_a_boundary(dtype, V, B, cuda_device):
+    """An embedding bias, rows that start between two 16-byte boundaries (and one size that does not)."""
+    from fastertransformer_b200 import DynamicDecodeLayer, lib
+    got = []
+    for general in (1, 0):
+        g = torch.Generator(device=cuda_device)
+        g.manual_seed(V)
+        layer = DynamicDecodeLayer(V, V, dtype, cuda_device)
+        layer.setup(B, 1, {"runtime_top_k": np.resize(np.asarray([0, 40], np.uint32), B), "runtime_top_p": np.asarray([0.9], np.float32),
+                           "temperature": np.asarray([0.7], np.float32), "random_seed": np.arange(B).astype(np.uint64)})
+        st = {"output_ids": torch.ones(12, B, dtype=torch.int32, device=cuda_device),
+              "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+              "sequence_length": torch.full((B,), 8, dtype=torch.int32, device=cuda_device),
+              "cum_log_probs": torch.zeros(B, device=cuda_device), "output_log_probs": torch.zeros(8, B, device=cuda_device)}
+        bias = (torch.randn(V, generator=g, device=cuda_device) * 2).to(dtype)
+        lib.ftb200_set_single_pass(1 - general)
+        try:
+            for s in range(3):
+                x = torch.randn(B, V, generator=g, device=cuda_device) * 2
+                layer.forward(st, {"logits": x.to(dtype), "step": 8 + s, "max_input_length": 8, "ite": 0, "local_batch_size": B,
+                                   "embedding_bias": bias, "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)})
+            torch.cuda.synchronize()
+        finally:
+            lib.ftb200_set_single_pass(1)
+        got.append({k: v.cpu().numpy() for k, v in st.items()})
+    for k, v in got[0].items():
+        np.testing.assert_array_equal(got[1][k], v, err_msg=k)
