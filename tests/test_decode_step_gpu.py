@@ -163,3 +163,48 @@ def test_step_under_capture(dtype, kind, V, B, cuda_device):
     recorded, direct = run(V, True), run(V, False)
     for a, b in zip(recorded, direct):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("form", ["plain", "bias", "words", "limit", "log_probs", "all", "other_buffers"])
+def test_native_step_equals_the_python_code(form, cuda_device, monkeypatch):
+    """forward() through the step module and through the code beside it: every optional entry, and buffers that change from
+    step to step."""
+    from fastertransformer_b200 import DynamicDecodeLayer, decode_layer
+    V, B, got = 9000, 5, []
+    for native in (True, False):
+        with monkeypatch.context() as m:
+            if not native:
+                m.setattr(decode_layer, "_LIBRARY", object())
+            g = torch.Generator(device=cuda_device)
+            g.manual_seed(3)
+            layer = DynamicDecodeLayer(V, V, torch.float16, cuda_device)
+            layer.setup(B, 1, {"runtime_top_k": np.asarray([0, 1, 9, 0, 64], np.uint32), "runtime_top_p": np.asarray([0.8], np.float32),
+                               "repetition_penalty": np.asarray([1.1], np.float32), "random_seed": np.arange(B).astype(np.uint64)})
+            st = {"output_ids": torch.ones(14, B, dtype=torch.int32, device=cuda_device),
+                  "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+                  "sequence_length": torch.full((B,), 8, dtype=torch.int32, device=cuda_device)}
+            if form in ("log_probs", "all"):
+                st["cum_log_probs"] = torch.zeros(B, device=cuda_device)
+                st["output_log_probs"] = torch.zeros(6, B, device=cuda_device)
+            extra = {}
+            if form in ("bias", "all"):
+                extra["embedding_bias"] = torch.randn(V, generator=g, device=cuda_device).half()
+            if form in ("words", "all"):
+                extra["stop_words_list"] = torch.tensor([[[7, 1, 9], [1, 3, -1]]] * B, dtype=torch.int32, device=cuda_device)
+                extra["bad_words_list"] = torch.tensor([[5], [1]], dtype=torch.int32, device=cuda_device)
+            if form in ("limit", "all"):
+                extra["sequence_limit_length"] = torch.full((B,), 11, dtype=torch.int32, device=cuda_device)
+            if form == "all":
+                extra["input_lengths"] = torch.full((B,), 6, dtype=torch.int32, device=cuda_device)
+            stops = []
+            for s in range(4):
+                x = (torch.randn(B, V, generator=g, device=cuda_device) * 3).half()
+                if form == "other_buffers" and s == 2:
+                    st = {k: v.clone() for k, v in st.items()}
+                stops.append(bool(layer.forward(st, {"logits": x, "step": 8 + s, "max_input_length": 8, "ite": 0, "local_batch_size": B,
+                                                     "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device), **extra})))
+            torch.cuda.synchronize()
+            assert (layer._native is not None) == native
+            got.append({k: v.cpu().numpy() for k, v in st.items()} | {"stops": np.asarray(stops), "launches": np.asarray(layer.launches)})
+    for k, v in got[1].items():
+        np.testing.assert_array_equal(got[0][k], v, err_msg=k)
