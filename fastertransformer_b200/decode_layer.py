@@ -131,8 +131,8 @@ class DynamicDecodeLayer:
                 or self._home is None or self._home < 0 or self._stream != self._home or lib is not _LIBRARY:
             return
         g, S = self._g, self._stop
-        self._native = _step.make(C.addressof(P), 0 if S is None else C.addressof(S), logits.dtype, _raw_stream, self._device_index,
-                                  self._home, B, g["temp"], self.penalty_type != 2 and g["pen"], g["minlen"])
+        self._native = _step.make(C.addressof(P), 0 if S is None else C.addressof(S), logits.dtype, _DT[logits.dtype], _raw_stream,
+                                  self._device_index, self._home, B, g["temp"], self.penalty_type != 2 and g["pen"], g["minlen"])
 
     def _stream_ptr(self):
         return C.c_void_p(self._raw_stream())

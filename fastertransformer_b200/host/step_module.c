@@ -2,9 +2,10 @@
  *
  * DynamicDecodeLayer.forward() (decode_layer.py) fills the library's argument block from some twenty dict entries and tensor
  * addresses; in Python that is 4.3 us of a step whose kernel takes 5 (one greedy row of 32000 columns).  This module does the same for
- * the common form of a call - the whole batch, on the stream the layer's memory was allocated on, the logits type of the
- * call before - and answers None for every other one, which the Python code then serves.  Every address and scalar is
- * read from the caller's objects in every call; nothing of theirs is kept.  What is kept of the layer (its argument blocks, the
+ * the common form of a call - the whole batch, on the stream the layer's memory was allocated on, logits of the type the slice
+ * was made for - and answers None for every other one, which the Python code then serves.  Every address and scalar is
+ * read from the caller's objects in every call; nothing of theirs is kept.  What a call of another form may have left in the
+ * argument block, the logits type among it, is written over by the next one.  What is kept of the layer (its argument blocks, the
  * constants of its set-up) belongs to it, and it drops the slice when one of these changes. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -20,7 +21,7 @@ typedef struct {
     ftb200_stop_params*     stop;   /* null until a call has needed one */
     PyObject *              dtype, *current_stream, *device_index;
     unsigned long long      home; /* stream the layer's memory was allocated on */
-    int                     batch, temp, pen, min_length;
+    int                     type, batch, temp, pen, min_length; /* (type: FTB200_F32 .. FTB200_BF16, what dtype stands for) */
     long long               launches;
 } Slice;
 
@@ -167,6 +168,7 @@ static PyObject* step(PyObject* self, PyObject* const* args, Py_ssize_t nargs)
     }
 
     ftb200_sampling_params* P = S->params;
+    P->dtype                  = S->type;
     P->step                   = (int)pos;
     P->max_input_length       = (int)mil;
     P->logits                 = x;
@@ -227,9 +229,9 @@ static PyObject* make(PyObject* self, PyObject* args)
     (void)self;
     unsigned long long params, stop, home;
     PyObject *         dtype, *current_stream, *device_index;
-    int                batch, temp, pen, min_length;
-    if (!PyArg_ParseTuple(args, "KKOOOKippi", &params, &stop, &dtype, &current_stream, &device_index, &home, &batch, &temp, &pen,
-                          &min_length)) {
+    int                type, batch, temp, pen, min_length;
+    if (!PyArg_ParseTuple(args, "KKOiOOKippi", &params, &stop, &dtype, &type, &current_stream, &device_index, &home, &batch, &temp,
+                          &pen, &min_length)) {
         return NULL;
     }
     Slice* S = (Slice*)PyMem_Calloc(1, sizeof(Slice));
@@ -242,7 +244,7 @@ static PyObject* make(PyObject* self, PyObject* args)
     S->current_stream = Py_NewRef(current_stream);
     S->device_index   = Py_NewRef(device_index);
     S->home           = home;
-    S->batch = batch, S->temp = temp, S->pen = pen, S->min_length = min_length;
+    S->type = type, S->batch = batch, S->temp = temp, S->pen = pen, S->min_length = min_length;
     PyObject* c = PyCapsule_New(S, kCapsule, drop);
     if (c == NULL) {
         PyMem_Free(S);
@@ -260,7 +262,7 @@ static PyObject* launches(PyObject* self, PyObject* capsule)
 static PyMethodDef methods[] = {
     {"step", (PyCFunction)(void (*)(void))step, METH_FASTCALL, "step(slice, outputs, inputs, deadline_ms) -> bool | int | None"},
     {"make", make, METH_VARARGS,
-     "make(params, stop, dtype, current_stream, device_index, home, batch, temperature, penalty, min_length) -> slice"},
+     "make(params, stop, dtype, type, current_stream, device_index, home, batch, temperature, penalty, min_length) -> slice"},
     {"launches", launches, METH_O, "kernels that a slice's steps have launched"},
     {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ftb200_step", NULL, -1, methods, NULL, NULL, NULL, NULL};

@@ -208,3 +208,22 @@ def test_native_step_equals_the_python_code(form, cuda_device, monkeypatch):
             got.append({k: v.cpu().numpy() for k, v in st.items()} | {"stops": np.asarray(stops), "launches": np.asarray(layer.launches)})
     for k, v in got[1].items():
         np.testing.assert_array_equal(got[0][k], v, err_msg=k)
+
+
+@pytest.mark.parametrize("types", [(F16, BF16, F16), (F16, F32, F16, F16), (F32, BF16, F16, F32)])
+def test_logits_types_in_turn(types, cuda_device):
+    """One layer whose logits change their type from call to call, against the maxima of each call's logits."""
+    from fastertransformer_b200 import DynamicDecodeLayer
+    V, B = 9001, 5
+    layer = DynamicDecodeLayer(V, V, types[0], cuda_device)
+    layer.setup(B, 1, {"runtime_top_k": np.asarray([1], np.uint32)})
+    st = {"output_ids": torch.ones(MIL + 4, B, dtype=torch.int32, device=cuda_device),
+          "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+          "sequence_length": torch.full((B,), MIL, dtype=torch.int32, device=cuda_device)}
+    for s, dtype in enumerate(types):
+        x = torch.full((B, V), -8.0, device=cuda_device)
+        want = torch.tensor([(s + 1) * (977 + b) % (V - 1) for b in range(B)], device=cuda_device)
+        x[torch.arange(B), want] = 8.0  # (exact in every type)
+        layer.forward(st, {"logits": x.to(dtype), "step": MIL + s, "max_input_length": MIL,
+                           "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)})
+        assert torch.equal(st["output_ids"][MIL + s].long(), want), s
