@@ -131,7 +131,7 @@ class DynamicDecodeLayer:
                 or self._home is None or self._home < 0 or self._stream != self._home or lib is not _LIBRARY:
             return
         g, S = self._g, self._stop
-        self._native = _step.make(C.addressof(P), 0 if S is None else C.addressof(S), logits.dtype, _DT[logits.dtype], _raw_stream,
+        self._native = _step.make(C.addressof(P), 0 if S is None else C.addressof(S), S, logits.dtype, _DT[logits.dtype], _raw_stream,
                                   self._device_index, self._home, B, g["temp"], self.penalty_type != 2 and g["pen"], g["minlen"])
 
     def _stream_ptr(self):
@@ -310,8 +310,6 @@ class DynamicDecodeLayer:
                 return done
             if done is not None:
                 self._failed(done)
-            for g in self._gate.values():
-                g["ptrs"] = None  # (the argument block is not as _fill() left it)
         logits = inputs["logits"]
         shape = logits.shape
         if len(shape) == 3 and shape[1] > 1:

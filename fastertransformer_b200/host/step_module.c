@@ -4,9 +4,10 @@
  * addresses; in Python that is 4.3 us of a step whose kernel takes 5 (one greedy row of 32000 columns).  This module does the same for
  * the common form of a call - the whole batch, on the stream the layer's memory was allocated on, logits of the type the slice
  * was made for - and answers None for every other one, which the Python code then serves.  Every address and scalar is
- * read from the caller's objects in every call; nothing of theirs is kept.  What a call of another form may have left in the
- * argument block, the logits type among it, is written over by the next one.  What is kept of the layer (its argument blocks, the
- * constants of its set-up) belongs to it, and it drops the slice when one of these changes. */
+ * read from the caller's objects in every call; nothing of theirs is kept.  What is kept of the layer is a copy of the argument
+ * block that its Python code filled, which nothing but this module reads or writes, and the constants of its set-up; the layer
+ * drops the slice when it is set up again or allocates memory.  The criteria's block, whose counter all steps of a layer share, is
+ * the layer's own, and the slice holds on to it. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -17,9 +18,10 @@
 int ftb200_last_launch_count(void);
 
 typedef struct {
-    ftb200_sampling_params* params; /* the layer's block, with its own buffers filled in */
-    ftb200_stop_params*     stop;   /* null until a call has needed one */
-    PyObject *              dtype, *current_stream, *device_index;
+    ftb200_sampling_params  params;      /* with the layer's own buffers filled in */
+    ftb200_stop_params*     stop;        /* null until a call has needed one */
+    PyObject *              stop_object, /* the ctypes structure that `stop` lies in */
+                           *dtype, *current_stream, *device_index;
     unsigned long long      home; /* stream the layer's memory was allocated on */
     int                     type, batch, temp, pen, min_length; /* (type: FTB200_F32 .. FTB200_BF16, what dtype stands for) */
     long long               launches;
@@ -167,7 +169,7 @@ static PyObject* step(PyObject* self, PyObject* const* args, Py_ssize_t nargs)
         goto python;
     }
 
-    ftb200_sampling_params* P = S->params;
+    ftb200_sampling_params* P = &S->params;
     P->dtype                  = S->type;
     P->step                   = (int)pos;
     P->max_input_length       = (int)mil;
@@ -217,6 +219,7 @@ static void drop(PyObject* capsule)
 {
     Slice* S = (Slice*)PyCapsule_GetPointer(capsule, kCapsule);
     if (S != NULL) {
+        Py_XDECREF(S->stop_object);
         Py_XDECREF(S->dtype);
         Py_XDECREF(S->current_stream);
         Py_XDECREF(S->device_index);
@@ -228,18 +231,19 @@ static PyObject* make(PyObject* self, PyObject* args)
 {
     (void)self;
     unsigned long long params, stop, home;
-    PyObject *         dtype, *current_stream, *device_index;
+    PyObject *         stop_object, *dtype, *current_stream, *device_index;
     int                type, batch, temp, pen, min_length;
-    if (!PyArg_ParseTuple(args, "KKOiOOKippi", &params, &stop, &dtype, &type, &current_stream, &device_index, &home, &batch, &temp,
-                          &pen, &min_length)) {
+    if (!PyArg_ParseTuple(args, "KKOOiOOKippi", &params, &stop, &stop_object, &dtype, &type, &current_stream, &device_index, &home,
+                          &batch, &temp, &pen, &min_length)) {
         return NULL;
     }
     Slice* S = (Slice*)PyMem_Calloc(1, sizeof(Slice));
     if (S == NULL) {
         return PyErr_NoMemory();
     }
-    S->params         = (ftb200_sampling_params*)(uintptr_t)params;
+    S->params         = *(const ftb200_sampling_params*)(uintptr_t)params;
     S->stop           = (ftb200_stop_params*)(uintptr_t)stop;
+    S->stop_object    = Py_NewRef(stop_object);
     S->dtype          = Py_NewRef(dtype);
     S->current_stream = Py_NewRef(current_stream);
     S->device_index   = Py_NewRef(device_index);
@@ -262,7 +266,8 @@ static PyObject* launches(PyObject* self, PyObject* capsule)
 static PyMethodDef methods[] = {
     {"step", (PyCFunction)(void (*)(void))step, METH_FASTCALL, "step(slice, outputs, inputs, deadline_ms) -> bool | int | None"},
     {"make", make, METH_VARARGS,
-     "make(params, stop, dtype, type, current_stream, device_index, home, batch, temperature, penalty, min_length) -> slice"},
+     "make(params, stop, stop_object, dtype, type, current_stream, device_index, home, batch, temperature, penalty, min_length) -> "
+     "slice; params and stop are addresses, params is copied"},
     {"launches", launches, METH_O, "kernels that a slice's steps have launched"},
     {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ftb200_step", NULL, -1, methods, NULL, NULL, NULL, NULL};

@@ -78,3 +78,22 @@ def test_each_call_is_of_its_own_type(types_, layer):
         call(layer, x)
         assert layer._native is not None
     assert [(p.dtype, p.logits) for p in layer.recorded()] == [(decode_layer._DT[x.dtype], x.data_ptr()) for x in given]
+
+
+def test_block_of_a_slice_is_its_own(layer):
+    """A call of other sizes for the same rows makes the layer a new argument block: the old one's memory is not the
+    native step's any more."""
+    x, twice = torch.zeros(8, 104, dtype=torch.float16), torch.zeros(16, 104, dtype=torch.float16)
+    call(layer, x)
+    old = layer._gate[(0, 8)]["params"]
+    call(layer, twice, local_batch_size=8)
+    C.memset(C.byref(old), 0xff, C.sizeof(old))  # (as its next owner may; the test still holds on to it)
+    call(layer, x)
+    call(layer, twice, local_batch_size=8)
+    assert bytes(old) == b"\xff" * C.sizeof(old)
+    got = layer.recorded()
+    assert [(p.batch_size, p.local_batch_size, p.vocab_size, p.logits) for p in got] == [
+        (8, 8, 100, x.data_ptr()), (16, 8, 100, twice.data_ptr())] * 2
+    for p in got[2:]:
+        for name in ("row_order", "topk_ks", "topk_states", "workspace", "workspace_bytes", "max_top_k"):
+            assert getattr(p, name) == getattr(got[0], name), name
