@@ -132,7 +132,7 @@ __device__ __forceinline__ void add_plain_vec(MaxSum& a, const uint4& v)
 // ---- 16-bit rows ------------------------------------------------------------------------------------------------
 // Two logits per instruction where that exists (packed fp32 fused multiply-add and add): the exponent of a term is one fused
 // multiply-add, x * log2(e) - m2 with m2 = m * log2(e) as it was rounded, and what that rounding lost, m * log2(e) - m2, is the
-// same for all terms and comes off the logarithm at the end.  Half of the instructions of a subtract, a multiply, an exponential
+// same for all terms and comes off the sum at the end.  Half of the instructions of a subtract, a multiply, an exponential
 // and an add a logit: 512 x 32 x 50257 half 238 -> 232 us (256 -> 249 on a warmer card).  Every fourth exponential by a polynomial
 // on the multiply-add pipes instead of the special-function unit was slower (242, half of them 278).
 __device__ __forceinline__ u64 pack2(float a, float b)
@@ -158,14 +158,19 @@ __device__ __forceinline__ u64 add2(u64 a, u64 b)
     return r;
 }
 
-// The sum of the two halves of s, times 2^m2, is the sum of exp(x) so far.  A maximum so large (or so low: a row of the
-// type's lowest value) that m2 would not be finite has no m2: then s stands for s * exp(m).
+// The sum of the two halves of s, times 2^m2, is the sum of exp(x) so far.  That wants a small d = m * log2(e) - m2: the terms
+// are 2^d times what they stand for, and total() takes that off with two terms of the series.  d is half a unit of m2's last
+// place, up to 2^-8 for the largest half (of the third term 3e-9 is left); bf16 reaches further, and a thread whose columns are all
+// masked with -1e10 so far has it for its maximum, with a d of hundreds.  From kBeyond on a bf16 maximum has no m2: s stands
+// for s * exp(m), by exact differences.  Values of bf16 on both sides of the line are 32 and more apart, so that going from one
+// form to the other scales the sum by e^-32 at most, and 2^d, within 2^-11 of 1, is no part of it.
 template<typename T>
 struct PairSum {
     float m, m2;
     u64   s;
-    static constexpr bool kWide = sizeof(T) == 2 && LpType<T>::kLowest < -1e30f;
-    __device__ static bool beyond(float m) { return kWide && !(fabsf(m) < 1e30f); }
+    static constexpr bool  kWide   = sizeof(T) == 2 && LpType<T>::kLowest < -65504.0f;
+    static constexpr float kBeyond = 8192.0f;
+    __device__ static bool beyond(float m) { return kWide && !(fabsf(m) < kBeyond); }
     __device__ void        start()
     {
         m = LpType<T>::kLowest, m2 = m * kLog2e, s = 0;
@@ -214,8 +219,8 @@ struct PairSum {
     {
         float a, b;
         unpack2(s, a, b);
-        // (2^-d for a d of a unit of m2's last place)
-        return {m, beyond(m) ? a + b : (a + b) * fmaf(fmaf(m, kLog2e, -m2), -0.69314718f, 1.0f)};
+        const float d = fmaf(m, kLog2e, -m2);  // 2^-d = 1 - d ln 2 + (d ln 2)^2 / 2 - ...
+        return {m, beyond(m) ? a + b : (a + b) * fmaf(d, fmaf(d, 0.24022651f, -0.69314718f), 1.0f)};
     }
 };
 // fp32 rows: at the copy rate with the plain form

@@ -195,3 +195,28 @@ def test_extreme_values_of_16_bit_rows(dtype, vocab, vp):
     tol = 1e-6 * 8 + np.abs(want) * 2.0 ** -22
     assert (np.abs(lp.reshape(max_len - 1, batch) - want) <= tol).all()
     assert (np.abs(cum - want.sum(0)) <= tol.sum(0) * 2).all()
+
+
+@pytest.mark.parametrize("mask", [-1e4, -1e9, -1e10, -1e12, -1e20])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("vocab", [515, 8195, 50257])
+def test_masked_columns_and_large_maxima(vocab, dtype, mask):
+    """A thread's running maximum is the mask's value until it meets a column that is not masked, and rows whose maximum
+    itself is large: all but a few columns at the end masked, every second one, all of them."""
+    g = torch.Generator().manual_seed(vocab)
+    peaks = [0.0, -300.0, 3e3, 8160.0, 8192.0, -8192.0, 1e4, 6e4, 1e5, 3e5, 1e6, 1e7, -1e9, 1e10, 1e12]
+    max_len, batch = len(peaks) + 1, 4
+    limit = 65504.0 if dtype == torch.float16 else 3e38
+    x = torch.randn(max_len, batch, vocab, generator=g) * 4
+    x[:-1] += torch.tensor(peaks).clamp(-limit, limit)[:, None, None]
+    x[:, 0, : vocab - 7] = mask
+    x[:, 1, ::2] = mask
+    x[:, 2] = mask
+    x = x.clamp(-limit, limit).to(dtype)
+    best = x.float().argmax(-1).int()  # (scored: the differences that count are small)
+    ids = torch.cat([torch.zeros(1, batch, dtype=torch.int32), best[:-1]])
+    lengths = torch.full((batch,), max_len, dtype=torch.int32)
+    _, lp = run_ours(x.cuda(), ids.cuda(), lengths.cuda(), vocab, False)
+    want = torch.log_softmax(x[:-1].double(), -1).gather(2, best[:-1, :, None].long())[..., 0].numpy()
+    # the bound of the test above: fp32 sums, and a result rounded to fp32
+    assert (np.abs(lp.reshape(max_len - 1, batch) - want) <= 8e-6 + np.abs(want) * 2.0 ** -22).all()
