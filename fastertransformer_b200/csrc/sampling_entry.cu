@@ -447,6 +447,14 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     if (rc != FTB200_OK || T.limit == nullptr) {
         return rc;
     }
+    // Rare: rows that the split kernel's tables could not hold, then the criteria over the whole call.  The rows are found
+    // by their flags on the device, so that these launches do nothing new where none is left.
+    bool       left_sent = !done;
+    const auto send_left = [&] {
+        left_sent   = true;
+        const int e = decode_step_sampling_impl(p, true, nullptr, nullptr, true);
+        return e == FTB200_OK ? stop_criteria_launch(p, T, (cudaStream_t)p->stream) : e;
+    };
     // The last kernel of the step stores (sequence, count) into the page-locked word: no query of the stream, whose
     // answer comes several microseconds after the kernel's end.
     const volatile u64* w  = T.result;
@@ -454,20 +462,15 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     for (u32 spin = 1;; ++spin) {
         const u64 v = *w;
         if ((u32)(v >> 32) == T.sequence) {
-            if ((u32)v == kRowsLeft) {
-                // rare: rows that the split kernel's tables could not hold, then the criteria over the whole call
-                T.sequence = ++s->sequence;
-                rc         = decode_step_sampling_impl(p, true, nullptr, nullptr, true);
-                if (rc == FTB200_OK) {
-                    rc = stop_criteria_launch(p, T, (cudaStream_t)p->stream);
-                }
-                if (rc != FTB200_OK) {
-                    return rc;
-                }
-                continue;
-            }
             *should_stop = (u32)v == (u32)p->batch_size ? 1 : 0;
             return FTB200_OK;
+        }
+        if (v == rows_left(T.sequence) && !left_sent) {
+            rc = send_left();
+            if (rc != FTB200_OK) {
+                return rc;
+            }
+            continue;
         }
         if ((spin & 1023u) == 0) {
             const cudaError_t e = cudaStreamQuery((cudaStream_t)p->stream);
@@ -477,6 +480,10 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
             }
             const auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0);
             if (timeout_ms >= 0 && ms.count() > timeout_ms) {
+                // (nobody may be there to read that rows are left: behind the step in its stream, whether there are any or not)
+                if (!left_sent && (rc = send_left()) != FTB200_OK) {
+                    return rc;
+                }
                 set_error("ftb200_decode_step: the step did not end within the deadline");
                 return FTB200_TIMEOUT;
             }
@@ -503,12 +510,12 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
     cudaStream_t st = (cudaStream_t)p->stream;
     // 16-bit logits without a bias, log-probs or timeline: the single-pass kernel serves the rows first and
     // leaves a list of the rows it does not cover; decode_sampling_kernel then works that list off.
-    const bool single_pass = g_fast_path && p->dtype != FTB200_F32 && K.bias == nullptr && K.cum_log_probs == nullptr
+    const bool single_pass = (g_fast_path || left_only) && p->dtype != FTB200_F32 && K.bias == nullptr && K.cum_log_probs == nullptr
                              && K.out_log_probs == nullptr && p->vocab_size_padded <= (1 << 20)
                              && p->vocab_size >= 16384 + 16 && (K.apply_rep ? p->step : 0) <= fast_max_history()
                              && (K.bad_words != nullptr ? K.bad_words_len : 0) <= fast_max_words();
     SplitArgs A{};
-    if (g_fast_path && choose_split(p, K, single_pass, &A)) {
+    if ((g_fast_path || left_only) && choose_split(p, K, single_pass, &A)) {
         A.redo_flags      = (int*)((char*)p->workspace + 256);
         const auto launch = [&](const SplitArgs& args) {
             switch (p->dtype) {

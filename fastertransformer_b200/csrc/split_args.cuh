@@ -13,8 +13,9 @@ constexpr int kSpMaxN     = 8;                       // portable cluster size
 constexpr size_t kSpMaxSmem = 216 * 1024;
 constexpr int kSpMinSlice = (kNB * 4 + 1024 * 4) / 4;  // the draw's histogram and values lie over the slice
 
-// Low word of a result that says: rows are left, and nothing has been counted (more rows than any batch has).
-constexpr u32 kRowsLeft = 0xffffffffu;
+// What a launch that leaves rows stores in place of its result.  No result: its high word is not the step's sequence number, so
+// that a caller who waits for that number goes on waiting.
+__host__ __device__ inline u64 rows_left(u32 sequence) { return ((u64)~sequence << 32) | 0xffffffffu; }
 
 // Stop criteria of the step, for the launch forms that finish everything themselves.
 struct StopArgs {

@@ -1820,7 +1820,7 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
         if (tid == 0) {
             *T.arrived = 0;
             __threadfence_system();
-            *(volatile u64*)T.result = ((u64)T.sequence << 32) | kRowsLeft;
+            *(volatile u64*)T.result = rows_left(T.sequence);
         }
         return;
     }

@@ -262,10 +262,10 @@ int ftb200_wait_should_stop(const int* finished_count_host, int batch_size, int 
  *   result_host   one 64-bit word of page-locked host memory the device can reach (cudaHostAlloc, cudaHostRegister)
  *   sequence      counts the calls on this block (in/out); the word holds sequence << 32 | finished rows afterwards
  * A block serves one call at a time.  *should_stop = 1 when all batch_size rows are finished; FTB200_TIMEOUT after
- * timeout_ms (negative: no deadline): the step is then still on its way and writes *result_host when it ends.  With a
- * length limit, rows that the first launch cannot hold (a nucleus of most of the vocabulary, thousands of equal values around
- * the k-th) are asked for by the host once that launch has said so, in this call: with the deadline missed they stay
- * without a token, their generator untouched.
+ * timeout_ms (negative: no deadline): the step is then still on its way, ends by itself and writes *result_host when
+ * it does.  With a length limit, rows that the first launch cannot hold (a nucleus of most of the vocabulary, thousands of equal
+ * values around the k-th) are sent for within this call, once that launch has said so in *result_host - with ~sequence for the
+ * high word: wait for `sequence` there - or when the deadline is missed; an error of these launches is returned.
  * ------------------------------------------------------------------------------------------ */
 typedef struct ftb200_stop_params {
     const int*      stop_words;

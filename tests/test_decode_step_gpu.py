@@ -227,3 +227,54 @@ def test_logits_types_in_turn(types, cuda_device):
         layer.forward(st, {"logits": x.to(dtype), "step": MIL + s, "max_input_length": MIL,
                            "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)})
         assert torch.equal(st["output_ids"][MIL + s].long(), want), s
+
+
+@pytest.mark.parametrize("dtype,V,B", [(F32, 50257, 6), (BF16, 128256, 9), (BF16, 128256, 40), (F32, 200000, 3)])
+def test_deadline_runs_out_with_rows_left(dtype, V, B, cuda_device):
+    """Rows that the first launch cannot hold, in a step whose deadline passes before that launch has run: the step ends by
+    itself all the same - each row's token, generator and stop word, the limit, the count in the word."""
+    from fastertransformer_b200 import DynamicDecodeLayer
+    from fastertransformer_b200._lib import FtbError
+    rt = C.CDLL("libcudart.so.12")
+    HOSTFN = C.CFUNCTYPE(None, C.c_void_p)
+    hold = HOSTFN(lambda _: time.sleep(0.3))
+    rt.cudaLaunchHostFunc.argtypes = [C.c_void_p, HOSTFN, C.c_void_p]
+    got = []
+    for late in (False, True):
+        g = torch.Generator(device=cuda_device)
+        g.manual_seed(V + B)
+        layer = DynamicDecodeLayer(V, V, dtype, cuda_device)
+        layer.setup(B, 1, {"runtime_top_k": np.resize(np.asarray([0, 0, 5], np.uint32), B),
+                           "runtime_top_p": np.resize(np.asarray([0.99, 0.3, 0.9], np.float32), B),
+                           "random_seed": np.arange(B).astype(np.uint64)})
+        st = {"output_ids": torch.full((MIL + 4, B), -1, dtype=torch.int32, device=cuda_device),
+              "finished": torch.arange(B, device=cuda_device) == B - 1,
+              "sequence_length": torch.full((B,), MIL, dtype=torch.int32, device=cuda_device)}
+        limits = torch.full((B,), MIL + 3, dtype=torch.int32, device=cuda_device)
+        limits[0] = MIL + 1
+        words = torch.tensor([[[77], [1]]] * B, dtype=torch.int32, device=cuda_device)
+        stream = torch.cuda.Stream(device=cuda_device)
+        torch.cuda.synchronize()
+        for s in range(3):
+            x = torch.randn(B, V, generator=g, device=cuda_device) * 0.5  # (flat: the rows of p = 0.99 keep most of the columns)
+            x[1, 77] = 30.0
+            inputs = {"logits": x.to(dtype), "step": MIL + s, "max_input_length": MIL, "stop_words_list": words,
+                      "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device), "sequence_limit_length": limits}
+            torch.cuda.synchronize()
+            with torch.cuda.stream(stream):
+                if late and s == 1:
+                    layer.deadline_ms = 20
+                    assert rt.cudaLaunchHostFunc(C.c_void_p(stream.cuda_stream), hold, None) == 0
+                    with pytest.raises(FtbError, match="deadline"):
+                        layer.forward(st, inputs)
+                    layer.deadline_ms = 10000
+                    stream.synchronize()
+                else:
+                    layer.forward(st, inputs)
+            # the word holds (calls so far, finished rows), whatever the host has waited for
+            assert int(layer._result) == (s + 1) << 32 | int(st["finished"].sum()) and int(layer._arrived) == 0
+        torch.cuda.synchronize()
+        got.append({k: v.cpu() for k, v in st.items()} | {"topk": layer.topk.curand.cpu(), "topp": layer.topp.curand.cpu()})
+    for k in got[0]:
+        assert torch.equal(got[0][k], got[1][k]), k
+    assert int(got[0]["output_ids"][MIL + 1].min()) >= 0 and int(got[0]["finished"].sum()) >= 3
