@@ -1,6 +1,7 @@
 """ctypes binding of libftb200.so (include/ftb200.h)."""
 import ctypes as C
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libftb200.so")
@@ -56,12 +57,16 @@ def _load():
     return l
 
 
-def _load_step_module():
-    """lib/_ftb200_step.so (host/step_module.c), which calls the library that is loaded here."""
+# (the suffix names the interpreter: another one has a module of its own)
+STEP_MODULE_PATH = os.path.join(_HERE, "lib", "_ftb200_step" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def _load_step_module(path=STEP_MODULE_PATH):
+    """host/step_module.c, which calls the library that is loaded here.  None where it was not built (no C compiler or
+    Python headers): decode_layer.py does the module's work too, some 4 us a step slower."""
     import importlib.util
-    path = os.path.join(_HERE, "lib", "_ftb200_step.so")
     if not os.path.exists(path):
-        raise ImportError("_ftb200_step.so is not built (%s). Run `python -m fastertransformer_b200.build`." % path)
+        return None
     spec = importlib.util.spec_from_file_location("_ftb200_step", path)
     module = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(module)

@@ -8,8 +8,10 @@ same approximate exp / log / divide instructions.
 """
 import concurrent.futures
 import os
+import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -78,14 +80,17 @@ def build(verbose=False, force=False):
 
 
 def build_step_module():
-    """Compile the native half of DynamicDecodeLayer.forward (host/step_module.c) into lib/_ftb200_step.so, next to the
-    library it calls (found through its rpath)."""
-    import sysconfig
-    out, src = os.path.join(OUT, "_ftb200_step.so"), os.path.join(HERE, "host", "step_module.c")
+    """Compile the native half of DynamicDecodeLayer.forward (host/step_module.c) for this interpreter, next to the library it
+    calls (found through its rpath).  Without a C compiler or Python's headers there is none, and the package does without."""
+    include = sysconfig.get_paths()["include"]
+    out, src = os.path.join(OUT, "_ftb200_step" + sysconfig.get_config_var("EXT_SUFFIX")), os.path.join(HERE, "host", "step_module.c")
     deps = [src, os.path.join(INC, "ftb200.h")]
     if os.path.exists(out) and os.path.exists(LIB) and all(os.path.getmtime(out) >= os.path.getmtime(d) for d in deps):
         return out
-    cmd = ["gcc", "-O2", "-std=c11", "-Wall", "-fPIC", "-shared", src, "-I" + sysconfig.get_paths()["include"], "-I" + INC, "-L" + OUT,
+    if shutil.which("gcc") is None or not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write("no gcc, or no Python.h in %s: the step module is not built, decode_layer.py does its work\n" % include)
+        return None
+    cmd = ["gcc", "-O2", "-std=c11", "-Wall", "-fPIC", "-shared", src, "-I" + include, "-I" + INC, "-L" + OUT,
            "-lftb200", "-Wl,-rpath,$ORIGIN", "-o", out]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:

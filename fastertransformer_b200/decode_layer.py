@@ -128,7 +128,7 @@ class DynamicDecodeLayer:
     def _make_native(self, logits, B, lo, lbs, P):
         """Later calls of this form go to the library through one native call (host/step_module.c)."""
         if (lo, lbs, B) != (0, self.batch_size, self.batch_size) or logits.dim() != 2 or self.stream is not None or _raw_stream is None \
-                or self._home is None or self._home < 0 or self._stream != self._home or lib is not _LIBRARY:
+                or _step is None or self._home is None or self._home < 0 or self._stream != self._home or lib is not _LIBRARY:
             return
         g, S = self._g, self._stop
         self._native = _step.make(C.addressof(P), 0 if S is None else C.addressof(S), S, logits.dtype, _DT[logits.dtype], _raw_stream,

@@ -3,6 +3,7 @@ reaches the library is the call's own, whatever calls came before it."""
 import ctypes as C
 import os
 import subprocess
+import sys
 import sysconfig
 import types
 
@@ -97,3 +98,16 @@ def test_block_of_a_slice_is_its_own(layer):
     for p in got[2:]:
         for name in ("row_order", "topk_ks", "topk_states", "workspace", "workspace_bytes", "max_top_k"):
             assert getattr(p, name) == getattr(got[0], name), name
+
+
+def test_package_without_the_module(layer, monkeypatch):
+    """No step module was built (or only another interpreter's): the package imports, and the Python code takes every step."""
+    code = ("import os; real = os.path.exists; os.path.exists = lambda p: '_ftb200_step' not in str(p) and real(p)\n"
+            "import fastertransformer_b200._lib as l; assert l.step_module is None and l.STEP_MODULE_PATH.endswith(%r)"
+            % sysconfig.get_config_var("EXT_SUFFIX"))
+    subprocess.check_call([sys.executable, "-c", code], cwd=ROOT)
+    monkeypatch.setattr(decode_layer, "_step", None)
+    x = torch.zeros(8, 104, dtype=torch.float16)
+    for _ in range(2):
+        call(layer, x)
+    assert layer._native is None and layer.launches == 2 and [p.logits for p in layer.recorded()] == [x.data_ptr()] * 2
