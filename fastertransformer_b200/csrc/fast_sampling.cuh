@@ -1173,6 +1173,10 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         while (freem != 0) {
             const int q = tid * rpt + __ffs(freem) - 1;
             freem &= freem - 1;
+            if (j >= (u32)n_sp) {
+                s_fail = 1;  // two patterns took one position, which only an exponential out of order could bring about
+                break;
+            }
             run_pr[q] = __float_as_uint(fkey_inv(~(u32)(spec[j] >> 32)));
             run_st[q] = 1u;
             ++j;

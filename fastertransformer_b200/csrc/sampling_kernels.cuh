@@ -2887,7 +2887,11 @@ __device__ __noinline__ int row_topp_classes(const KParams& P, const Smem& S, co
         for (int i = 0; i < RPT; ++i) {
             if ((freem >> i) & 1u) {
                 const int r = tid * RPT + i;
-                run_pr[r]   = __float_as_uint(fkey_inv(~(u32)(spec[j] >> 32)));
+                if (j >= (u32)ns) {
+                    s_fail = 1;  // two patterns took one position, which only an exponential out of order could bring about
+                    break;
+                }
+                run_pr[r] = __float_as_uint(fkey_inv(~(u32)(spec[j] >> 32)));
                 run_st[r]   = 1u;
                 ++j;
             }
