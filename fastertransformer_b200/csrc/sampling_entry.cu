@@ -179,9 +179,14 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     A->roomy    = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kRoomyTwoPerSm && keeps(2, kRoomyTwoPerSm)));
     A->criteria = A->roomy;
     if (!A->roomy && lgn >= 2 && least > kThreePerSm) {
-        // shared memory holds two CTAs on an SM, or one, whatever the registers: the roomy form for more rows than are resident
-        // too (96 x 128256 bf16 with both kinds of rows: 74 us a step, 85 with 80 registers and the criteria apart).  The
-        // last row does the criteria wherever it runs.
+        // Shared memory holds two CTAs on an SM, or one, whatever the registers: the roomy form for more rows than are resident
+        // too.  us a step without a length limit, 128 / 80 registers: with both kinds of rows, bf16, 40 x 128256 40 / 47, 128 x
+        // 128256 77 / 93, 160 x 100000 86 / 109, 250 x 65000 71 / 85, 200 x 50257 65 / 78; fp32, 300 x 128256 178 / 214; nucleus
+        // rows, 64 x 128256 bf16 70 / 83, 160 x 65000 fp32 80 / 97, 300 x 50257 fp32 118 / 150; k = 50, fp32, 96 x 128256 59 / 71.
+        // The criteria in the launch (the last row does them wherever it runs) against a launch of their own, with a limit:
+        // both kinds of rows 47 / 54, 87 / 91, 102 / 101, 80 / 84, 76 / 79, 195 / 192 for those six.  One kind of rows alone has
+        // them apart: 78 / 85 at 64 x 128256 bf16, 87 / 95 at 160 x 65000 fp32, but 264 / 260 and (k = 50) 197 / 189 at 300 x
+        // 128256 fp32, and no line between the two has been drawn.
         A->roomy    = 1;
         A->criteria = mixed;
         A->area     = area_within(least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem, kSpAreaMax);

@@ -9,12 +9,13 @@
 // others, and the special columns (history, bans) are scattered evenly.  What is exchanged per row is small: a bit per
 // special column, one maximum and 1024 / 32 / n partial sums per CTA, a 2048-bin histogram, the candidates.
 //
-// What bounds it: latency.  A row takes six to ten cluster barriers (0.5 us each) and about six sweeps over its shared
-// memory; a CTA-per-row kernel walks eight times as many columns with the same 256 threads.  Measured on B200, one row
+// What bounds it: latency.  A row takes cluster barriers of 0.5 us each - three for an arg-max row, six where few candidates are
+// left, eight or ten for a nucleus that one or several CTAs sort, one more with special columns, the last one at its end -
+// and about six sweeps over its shared memory; a CTA-per-row kernel walks eight times as many columns with the same 256 threads.  Measured on B200, one row
 // alone on its SMs: arg-max of 32000 columns 4 us, k = 50 of 50257 fp32 13 us, a nucleus of 50257 fp32 19 us (the general
-// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 5 us (k = 1) to 60 us (25000-column nucleus).  Batch
-// of 64 x 50257 fp32 top-p: 43 us a step; 48 x 51200 half with bias and log-probs: 52 us; 24 steps of 16 x 128256 bf16: 1200 to
-// 1370 us.  Before the nucleus was placed by bin, sorted by short loops and the general row code taken out: 60, 83, 1600 to 1930.
+// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 5 us (k = 1) to 58 us (25000-column nucleus).  Batch
+// of 64 x 50257 fp32 top-p: 42 us a step; 48 x 51200 half with bias and log-probs: 52 us; 24 steps of 16 x 128256 bf16: 1240 to
+// 1420 us.  Before the nucleus was placed by bin, sorted by short loops and the general row code taken out: 60, 83, 1600 to 1930.
 //
 // Code size matters: a row runs through most of this code once, so a loop that is unrolled for the largest case waits for
 // its instructions in every case.
@@ -560,8 +561,10 @@ static __device__ __noinline__ void sp_scatter_keys(const float* y, int ny, floa
 // distribution is; inside it a key's place is the number of larger ones.
 //
 // The keys go to `tmp` by sub-bucket and come back in order: three short loops, because a row passes through this code once and
-// an unrolled form waits for its instructions.  900 keys: 6 us, 4850 keys: 19 us (before, keys held in registers by code
-// unrolled for 10240 of them: 20 to 26 us).  Above half of the area it goes stretch by stretch: 30 us for 7500 keys.  Returns false when a long sub-bucket of many values would have to be ordered.
+// an unrolled form waits for its instructions.  fp32 / bf16 logits, all steps of the sort: 900 keys 5.3 / 5.9 us, 3000 11.4 /
+// 13.1, 4700 17 / 20 (keys held in registers by code unrolled for 10240 of them: 20 to 26 us).  Above half of the area it
+// goes stretch by stretch: 5600 keys 24 / 27 us, 7500 33 / 38.  Returns false when a long sub-bucket of many values would
+// have to be ordered.
 constexpr int kSpShort = 24;   // keys of a sub-bucket that every thread orders for itself
 constexpr int kSpLists = 256;  // words for the list of longer ones
 
@@ -1843,8 +1846,8 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
 }
 
 // ROOMY: 128 registers, two CTAs on an SM, and - when asked to - the step's stop criteria: one launch per decode step.
-// Taken while all rows are resident at once; with more rows 80 registers and three CTAs on an SM are worth more.  Either form
-// flags the rows that its tables cannot hold for a second launch: decode_sampling_kernel, or - where the areas of the first
+// Taken while all rows are resident at once, and beyond that where shared memory holds no third CTA on an SM; elsewhere 80
+// registers and three CTAs on an SM are worth more (choose_split).  Either form flags the rows that its tables cannot hold for a second launch: decode_sampling_kernel, or - where the areas of the first
 // launch are small - a few clusters of the roomy form with all the shared memory there is (A.clusters), because a nucleus of half
 // of 127000 columns takes 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of
 // 127000 columns; above 163000 columns there is no such launch, 49000 columns end it) still ends in the general code, so a batch of
@@ -1854,7 +1857,8 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
 //
 // The general row code is not part of this kernel.  It was, in the roomy form, for the rows it leaves; its frames brought the
 // stack to 1.7 to 1.9 KB a thread, and builds that differed in nothing but such sizes ended steps of two CTAs on an SM with an
-// illegal address, or did not.  Without it the stack is 0.1 KB.
+// illegal address, or did not.  The cause is not known: its index arithmetic, the sizes of its tables and the pointers it
+// takes for shared have been read through since and stay inside.  Without it the stack is 24 to 48 bytes, 184 in the other form.
 template<int DT, int LGN, bool ROOMY>
 __global__ void __launch_bounds__(kThreads, ROOMY ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
                                                                      const __grid_constant__ SplitArgs A)
