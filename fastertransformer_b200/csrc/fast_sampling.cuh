@@ -46,6 +46,7 @@ struct FMap {
     u32*            sval;  // [hash_slots] gathered raw word, then the final value of that column (float bits)
     u32*            hist;  // [kFBins]   columns per value class above the threshold
     u32*            stage; // [kFStageBytes / 4] token history, word list and last tokens of the row, as fetched
+    u32*            lo;    // [kFBins]   top-p rows: columns per bit pattern below the threshold
     uint4*          wbuf;  // [kWarps * kFRing] vectors parked during a pass (static shared memory of the kernel)
     unsigned short* wj;    // [kWarps * kFRing]
 };
@@ -53,27 +54,42 @@ struct FMap {
 constexpr int kFMaxHist    = 1024;  // token-history entries the single-pass kernel stages at a time
 constexpr int kFMaxHistAll = 4094;  // and in all (the table of special columns: step + words + 2 <= 4096)
 constexpr int kFMaxWords   = 128;   // bad-word list length it stages
+constexpr int kFRow2Ring   = 16384; // top-p rows, second pass: pairs of 1024-column chunks on their way, four of them
 constexpr int kFStageBytes = 8192;  // >= (kFMaxHist + 2 * kFMaxWords + 4) * 4; later kFPSpecCap listed columns of a top-p row
+// Special columns that a row with this table has at most (see the plan of the table in sampling_entry.cu).
+__host__ __device__ inline int fast_max_records(int hash_slots)
+{
+    return hash_slots <= 2048 ? hash_slots / 2 : (hash_slots / 4 * 3 < 4096 ? hash_slots / 4 * 3 : 4096);
+}
 // bytes of the per-vector mask area: one byte per aligned vector, and room for what follows the pass
-__host__ __device__ inline size_t fast_mask_bytes(int vocab_padded, bool topp)
+__host__ __device__ inline size_t fast_mask_bytes(int hash_slots, int vocab_padded, bool topp)
 {
     const size_t need = ((size_t)vocab_padded / 8 + 16 + 15) / 16 * 16;
     size_t post = (size_t)kFSpecCap * 8 + (size_t)kFRunBytes;  // the top-k rows' kernel
     if (topp) {
-        post = (size_t)kFPRuns * 8 > (size_t)kFPClsCap * 4 ? (size_t)kFPRuns * 8 : (size_t)kFPClsCap * 4;
+        // The second pass: its ring, a bucket for every warp and 2048 columns, a record for every special column.  Then the runs and one
+        // more first position, or the class's columns.
+        const size_t pass2 = kFRow2Ring + ((size_t)(kThreads / 32) * (vocab_padded / 2048 + 1) + (size_t)fast_max_records(hash_slots) + 3) / 4 * 16;
+        post = (size_t)kFPRuns * 8 + 16;
+        post = post > pass2 ? post : pass2;
+        static_assert((size_t)kFPRuns * 8 >= (size_t)kFPClsCap * 4, "area too small");
     }
     return need > post ? need : post;
 }
 __host__ __device__ inline size_t fast_smem_bytes(int hash_slots, int vocab_padded, bool topp)
 {
-    const size_t sv = hash_slots > kFBins ? hash_slots : kFBins;  // the value area doubles as a class table
-    return (size_t)kFCap * 4 + fast_mask_bytes(vocab_padded, topp) + (size_t)hash_slots * 4 + sv * 4 + (size_t)kFBins * 4
-           + (topp ? (size_t)kFPSpecCap * 8 : (size_t)kFStageBytes);  // (the area is the last of the map)
+    const size_t sv = topp || hash_slots > kFBins ? hash_slots : kFBins;  // (top-k rows: the value area doubles as a class table)
+    return (size_t)kFCap * 4 + fast_mask_bytes(hash_slots, vocab_padded, topp) + (size_t)hash_slots * 4 + sv * 4 + (size_t)kFBins * 4
+           + (topp ? (size_t)kFPSpecCap * 8 + (size_t)kFBins * 4 : (size_t)kFStageBytes);
 }
 
 __device__ __forceinline__ void cp_async4(u32 saddr, const void* g)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async8(u32 saddr, const void* g)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(saddr), "l"(g) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all()
 {
@@ -594,223 +610,186 @@ static __device__ float f_block_sum(float v, float* s_w)
     return t;
 }
 
+// Exclusive prefix of one value per thread over the CTA; *total, where given, receives the sum.
+static __device__ u32 f_block_excl(u32 v, u32* s_w, u32* total)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    u32       incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const u32 t = __shfl_up_sync(0xffffffffu, incl, off);
+        incl += lane >= off ? t : 0u;
+    }
+    __syncthreads();  // (the previous call's sums have been read)
+    if (lane == 31) {
+        s_w[wid] = incl;
+    }
+    __syncthreads();
+    u32 base = 0, tot = 0;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+        const u32 w = s_w[i];
+        base += i < wid ? w : 0u;
+        tot += w;
+    }
+    if (total != nullptr) {
+        *total = tot;
+    }
+    return base + incl - v;
+}
+
 // ---- shared memory by 32-bit address (the hot loop of pass 2 keeps no generic pointer) ----
-// (not volatile and without a memory clobber: the compiler may move and batch these reads - they are used on
-//  tables that nobody writes while the loop around them runs)
-__device__ __forceinline__ u32 lds_u8(u32 addr)
+// Counter i of those at `base`, one more when i < n: the predicate is inside the instruction (no branch around it: a run of these
+// stays one basic block).
+__device__ __forceinline__ void reds_inc_below(u32 base, u32 i, u32 n)
 {
-    u32 v;
-    asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-// The same under a predicate inside the instruction (no branch around it: a run of these stays one basic block).
-__device__ __forceinline__ void reds_inc_if(u32 addr, u32 cond)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p red.shared.add.u32 [%0], 1;\n\t}" ::"r"(addr), "r"(cond));
-}
-// Counter update whose result nobody in the surrounding loop reads: no memory clobber, so the arithmetic of
-// neighbouring columns is free to move across it.
-__device__ __forceinline__ void reds_add_free(u32 addr, u32 v)
-{
-    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v));
-}
-__device__ __forceinline__ uint2 lds_v2(u32 addr)
-{
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ void cp_async8(u32 saddr, const void* g)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(saddr), "l"(g) : "memory");
-}
-__device__ __forceinline__ u32 atoms_add(u32 addr, u32 v)
-{
-    u32 old;
-    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
-    return old;
-}
-__device__ __forceinline__ void sts_u64(u32 addr, u64 v)
-{
-    asm volatile("st.shared.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %1, %2;\n\t@p red.shared.add.u32 [%0], 1;\n\t}" ::"r"(base + 4u * i), "r"(i), "r"(n));
 }
 __device__ __forceinline__ void sts_f32(u32 addr, float v)
 {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
-// flags of column `id` in the hash at shared address `hash` (0 when it has no entry)
-__device__ __forceinline__ u32 f_lookup_saddr(u32 hash, int shift, int mask, int id)
+__device__ __forceinline__ uint2 lds_v2(u32 addr)
+{
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_f4(u32 addr, float a, float b, float c, float d)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void lds_f4(u32 addr, float& a, float& b, float& c, float& d)
+{
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "r"(addr) : "memory");
+}
+// slot of column `id` in the hash at shared address `hash`, -1 when it has none
+__device__ __forceinline__ int f_hash_find_saddr(u32 hash, int shift, int mask, int id)
 {
     u32 h = hash_slot(id, shift);
     for (int probe = 0; probe <= mask; ++probe) {
         const u32 v = lds_u32(hash + 4u * h);
         if (v == kHashEmpty) {
-            return 0;
+            return -1;
         }
         if ((v >> 2) == (u32)id) {
-            return v & 3u;
+            return (int)h;
         }
         h = (h + 1) & mask;
     }
-    return 0;
+    return -1;
 }
 
 // Scalars of pass 2 (one argument block, by value: it travels in the parameter space of the call).
 struct FPass2 {
     const char* rowp;
-    int         nch, vocab, shift, mask, apply_rep, penalty_type;
-    float       maxv, inv_t, theta, cut_y, thr_y, neg_max;
+    int         nch, vocab, shift, mask;
+    float       maxv, inv_t;
     u32         thr_key, lo_n;
-    u32         emask, hash, hlo, spec, nspec, out;  // shared-memory addresses
+    u32         hash, value, list, ends, ring, hlo, buf, out;  // shared-memory addresses
     __half      inv_t_h;
 };
 
+// Special columns of a top-p row, filed for pass 2: a bucket per warp and pair of 1024-column chunks (the columns that the
+// warp holds in registers at a time), a record per column: its slot in the hash, whose value word is the column's final
+// value, and its place among the warp's 2 x 128 columns.
+__device__ __forceinline__ u32 f_bucket(int v, int npair)
+{
+    return (u32)(((v & 1023) >> 7) * npair + (v >> 11));
+}
+__device__ __forceinline__ u32 f_record(int slot, int v)
+{
+    return ((u32)slot << 8) | (u32)((v >> 10) & 1) << 7 | (u32)(v & 127);
+}
+
 // Pass 2 of a top-p row over the whole 1024-column chunks [0, nch) and the ragged rest up to `vocab`: thread t
-// adds the exponentials of its four "virtual threads" chunk by chunk; with COUNTING the ordinary columns whose bit
-// pattern lies in the lo_n patterns below the threshold are counted; special columns take their final value and
-// are listed when it falls between the cut and the threshold.  The four sums go to out[4t .. 4t+3].
-template<int DT, bool TEMP, bool COUNTING>
+// adds the exponentials of its four "virtual threads" chunk by chunk; with COUNT the columns whose bit
+// pattern lies in the lo_n patterns below the threshold are counted (what the special ones among them add has been taken off
+// beforehand).  The four sums go to out[4t .. 4t+3].
+//
+// Special columns: rare for a thread, but some lane of a warp has one in nearly every pair of chunks.  The warp's exponentials go
+// through 1 KB of shared memory then, and lanes with a record each put the special ones in their places: 2 + 2 wide accesses
+// instead of a divergent table walk that picks one of sixteen registers and puts it back with selects (a third of the
+// instructions of the pass).  Rows of 128256 bf16
+// with 550 special columns, wide nuclei: 55 us with the walk, 38 so; 51200 half, 150 special columns: 19.7 and 12.4.
+enum { kCountNone, kCountPositive, kCountAny };  // (positive: threshold and cut both at or above +0)
+template<int DT, bool TEMP, int COUNT>
 __device__ __noinline__ void f_pass2(const FPass2 A)
 {
-    const int    tid = threadIdx.x;
+    const int    tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const float  maxv = A.maxv, inv_t = A.inv_t;
     const __half inv_t_h = A.inv_t_h;
     const u32    thr_key = A.thr_key, lo_n = A.lo_n, hlo = A.hlo;
     float        a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    // final value of a special column (kernels/sampling_penalty_kernels.cu:367-424, :485-500; a dead one is -inf)
-    auto special = [&](float y, u32 fl) {
-        if (fl & kFlagDead) {
-            return -INFINITY;
+    const char*  base = A.rowp + (size_t)tid * 8;
+    const int    nch = A.nch, npair = (nch + 1) >> 1;
+    // (kCountPositive: the index below the threshold is a plain difference of the raw patterns; a negative value, or one at or
+    // above the threshold, wraps to a huge index)
+    const u32 below = COUNT == kCountPositive ? (thr_key & 0x7fffu) - 1u : thr_key - 1u;
+    const u32  buf = A.buf + 1024u * (u32)wid, own = buf + 16u * (u32)lane;
+    const u32  ends = A.ends + 4u * (u32)(wid * npair);
+    u32        at   = wid > 0 ? lds_u32(ends - 4u) : 0u;
+    // A thread's columns of three pairs of chunks are on their way while it works on a pair: eight bytes each into a place of its own,
+    // so that nobody waits for anybody; a place is filled again a pair after it was read.
+    const u32 ring = A.ring + 8u * (u32)tid;
+    auto      send = [&](int m) {
+        const u32 to = ring + (u32)(m & 6) * (kFRow2Ring / 8);
+        if (m < nch) {
+            cp_async8(to, base + (size_t)m * 2048);
         }
-        if ((fl & kFlagHist) && A.apply_rep) {
-            if (A.penalty_type == FTB200_PENALTY_MULTIPLICATIVE) {
-                y = y < 0.0f ? y * A.theta : y / A.theta;
-            }
-            else if (A.penalty_type == FTB200_PENALTY_ADDITIVE) {
-                y = y - A.theta;
-            }
-            if (DT == FTB200_F16) {
-                y = __half2float(__float2half_rn(y));
-            }
+        if (m + 1 < nch) {
+            cp_async8(to + kFRow2Ring / 8, base + (size_t)(m + 1) * 2048);
         }
-        return y;
+        cp_async_commit();
     };
-    auto patch = [&](float y, int v) {  // rare: column v is special
-        const float yy = special(y, f_lookup_saddr(A.hash, A.shift, A.mask, v));
-        if (yy >= A.cut_y && !(yy >= A.thr_y) && yy > A.neg_max) {  // (those at or above the threshold are listed already)
-            const u32 pos = atoms_add(A.nspec, 1u);
-            if (pos < (u32)kFPSpecCap) {
-                sts_u64(A.spec + 8u * pos, ((u64)(~fkey(yy)) << 32) | (u32)v);
-            }
+    auto       count = [&](const uint2& q) {
+        const u32 w[4] = {q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            reds_inc_below(hlo, below - (COUNT == kCountPositive ? w[e] : key16(w[e])), lo_n);
         }
-        return yy;
     };
-    // A batch of UN chunks is worked on in stages, every stage over all 4 * UN columns of the thread: values,
-    // final values of the special ones (rare), exponentials, the four running sums in chunk order, counts.  The
-    // columns of a stage are independent of one another, so a warp has many instructions to issue between two
-    // dependent ones.
-    constexpr int UN     = 4;  // (larger batches run slower: the loop body then no longer sits in the instruction cache)
-    const char*   base   = A.rowp + (size_t)tid * 8;
-    const u32     embase = A.emask + (u32)(tid >> 1);
-    const int     nch    = A.nch;
-    const int     nib    = 4 * (tid & 1);
-    // (threshold and cut both at or above +0: see the counting stage)
-    const bool    pos_cut = thr_key - lo_n >= 0x8000u && thr_key > 0x8000u;
-    const u32     thr_m1  = (thr_key & 0x7fffu) - 1u;
-    for (int m0 = 0; m0 < nch; m0 += UN) {
-        uint2 raw[UN];
-        u32   em[UN];
-        float y[UN][4];
+    send(0);
+    send(2);
+    send(4);
+    // (one copy of the loop body: with two pairs in it, their loads in registers, it took 25 us for a row of 128256 without counts, with
+    // four 49, waiting for its instructions)
+#pragma unroll 1
+    for (int m = 0; m < nch; m += 2) {
+        cp_async_wait<2>();
+        const u32   from = ring + (u32)(m & 6) * (kFRow2Ring / 8);
+        const uint2 ca = lds_v2(from), cb = lds_v2(from + kFRow2Ring / 8);
+        const u32   end = lds_u32(ends + 4u * (u32)(m >> 1));
+        send(m + 6);
+        float x[8];
+        const u32 w[4] = {ca.x, ca.y, cb.x, cb.y};
 #pragma unroll
-        for (int uu = 0; uu < UN; ++uu) {
-            const bool in = m0 + uu < nch;
-            raw[uu]       = in ? ld_nc_v2(base + (size_t)(m0 + uu) * 2048) : make_uint2(0u, 0u);
-            em[uu]        = in ? (lds_u8(embase + (u32)(m0 + uu) * 128u) >> nib) & 0xfu : 0u;
+        for (int e = 0; e < 8; ++e) {
+            // a column at or below -MAX adds exactly zero, as in the reference's loop
+            const float y = f_value<DT>((e & 1) ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu, TEMP, inv_t, inv_t_h);
+            x[e]          = f_round_T<DT>(__expf(y - maxv));
         }
-#pragma unroll
-        for (int uu = 0; uu < UN; ++uu) {
-            y[uu][0] = f_value<DT>(raw[uu].x & 0xffffu, TEMP, inv_t, inv_t_h);
-            y[uu][1] = f_value<DT>(raw[uu].x >> 16, TEMP, inv_t, inv_t_h);
-            y[uu][2] = f_value<DT>(raw[uu].y & 0xffffu, TEMP, inv_t, inv_t_h);
-            y[uu][3] = f_value<DT>(raw[uu].y >> 16, TEMP, inv_t, inv_t_h);
+        if (end != at) {
+            sts_f4(own, x[0], x[1], x[2], x[3]);
+            sts_f4(own + 512u, x[4], x[5], x[6], x[7]);
+            __syncwarp();
+            for (u32 i = at + (u32)lane; i < end; i += 32) {
+                const u32 r = lds_u32(A.list + 4u * i);
+                sts_f32(buf + 4u * (r & 255u), f_round_T<DT>(__expf(__uint_as_float(lds_u32(A.value + 4u * (r >> 8))) - maxv)));
+            }
+            __syncwarp();
+            lds_f4(own, x[0], x[1], x[2], x[3]);
+            lds_f4(own + 512u, x[4], x[5], x[6], x[7]);
+            at = end;
         }
-        {
-            // Special columns: rare for a thread, but some lane of a warp has one in nearly every batch.  One copy of
-            // the code for the whole batch (the column is picked and put back with selects): a copy per column
-            // made the loop body several times larger than the instruction cache likes.
-            u32 todo = 0;
-#pragma unroll
-            for (int uu = 0; uu < UN; ++uu) {
-                todo |= em[uu] << (4 * uu);
-            }
-            while (todo != 0) {
-                const int j = __ffs(todo) - 1;
-                todo &= todo - 1;
-                float yv = 0.0f;
-#pragma unroll
-                for (int a = 0; a < 4 * UN; ++a) {
-                    yv = j == a ? y[a >> 2][a & 3] : yv;
-                }
-                yv = patch(yv, (m0 + (j >> 2)) * 1024 + 4 * tid + (j & 3));
-#pragma unroll
-                for (int a = 0; a < 4 * UN; ++a) {
-                    y[a >> 2][a & 3] = j == a ? yv : y[a >> 2][a & 3];
-                }
-            }
+        a0 += x[0], a1 += x[1], a2 += x[2], a3 += x[3];
+        if (COUNT) {
+            count(ca);
         }
-#pragma unroll
-        for (int uu = 0; uu < UN; ++uu) {
-            // a column at or below -MAX adds exactly zero, as in the reference's loop; the chunks past the end of
-            // the row are left out below
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                y[uu][e] = f_round_T<DT>(__expf(y[uu][e] - maxv));
-            }
-        }
-#pragma unroll
-        for (int uu = 0; uu < UN; ++uu) {
-            if (m0 + uu < nch) {
-                a0 += y[uu][0], a1 += y[uu][1], a2 += y[uu][2], a3 += y[uu][3];
-            }
-        }
-        if (COUNTING) {
-            // Ordinary columns between the cut and the threshold, per bit pattern.  With the cut at or above +0 (the
-            // usual case) the index below the threshold is a plain difference of the raw patterns: a negative
-            // value, or one at or above the threshold, wraps to a huge index.
-            if (pos_cut) {
-#pragma unroll
-                for (int uu = 0; uu < UN; ++uu) {
-                    if (m0 + uu < nch) {
-                        const u32 i0 = thr_m1 - (raw[uu].x & 0xffffu), i1 = thr_m1 - (raw[uu].x >> 16);
-                        const u32 i2 = thr_m1 - (raw[uu].y & 0xffffu), i3 = thr_m1 - (raw[uu].y >> 16);
-                        const u32 ok = ~em[uu];
-                        reds_inc_if(hlo + 4u * (i0 < lo_n ? i0 : 0u), (i0 < lo_n ? 1u : 0u) & ok);
-                        reds_inc_if(hlo + 4u * (i1 < lo_n ? i1 : 0u), (i1 < lo_n ? 2u : 0u) & ok);
-                        reds_inc_if(hlo + 4u * (i2 < lo_n ? i2 : 0u), (i2 < lo_n ? 4u : 0u) & ok);
-                        reds_inc_if(hlo + 4u * (i3 < lo_n ? i3 : 0u), (i3 < lo_n ? 8u : 0u) & ok);
-                    }
-                }
-            }
-            else {
-#pragma unroll
-                for (int uu = 0; uu < UN; ++uu) {
-                    if (m0 + uu < nch) {
-                        const u32 i0 = thr_key - 1u - key16(raw[uu].x & 0xffffu), i1 = thr_key - 1u - key16(raw[uu].x >> 16);
-                        const u32 i2 = thr_key - 1u - key16(raw[uu].y & 0xffffu), i3 = thr_key - 1u - key16(raw[uu].y >> 16);
-                        if (i0 < lo_n && !(em[uu] & 1u)) {
-                            reds_add_free(hlo + 4u * i0, 1u);
-                        }
-                        if (i1 < lo_n && !(em[uu] & 2u)) {
-                            reds_add_free(hlo + 4u * i1, 1u);
-                        }
-                        if (i2 < lo_n && !(em[uu] & 4u)) {
-                            reds_add_free(hlo + 4u * i2, 1u);
-                        }
-                        if (i3 < lo_n && !(em[uu] & 8u)) {
-                            reds_add_free(hlo + 4u * i3, 1u);
-                        }
-                    }
-                }
+        if (m + 1 < nch) {
+            a0 += x[4], a1 += x[5], a2 += x[6], a3 += x[7];
+            if (COUNT) {
+                count(cb);
             }
         }
     }
@@ -820,27 +799,202 @@ __device__ __noinline__ void f_pass2(const FPass2 A)
         if (v0 < A.vocab) {
             const unsigned short* row16 = (const unsigned short*)A.rowp;
             for (int e = 0; e < 4 && v0 + e < A.vocab; ++e) {
-                const u32 r  = (u32)__ldg(row16 + v0 + e);
-                const u32 fl = f_lookup_saddr(A.hash, A.shift, A.mask, v0 + e);
-                float     yy = f_value<DT>(r, TEMP, inv_t, inv_t_h);
-                if (fl != 0) {
-                    yy = patch(yy, v0 + e);
-                }
+                const u32 r    = (u32)__ldg(row16 + v0 + e);
+                const int slot = f_hash_find_saddr(A.hash, A.shift, A.mask, v0 + e);
+                const float yy = slot >= 0 ? __uint_as_float(lds_u32(A.value + 4u * (u32)slot)) : f_value<DT>(r, TEMP, inv_t, inv_t_h);
                 const float ex = f_round_T<DT>(__expf(yy - maxv));
                 a0 += e == 0 ? ex : 0.0f, a1 += e == 1 ? ex : 0.0f, a2 += e == 2 ? ex : 0.0f, a3 += e == 3 ? ex : 0.0f;
-                if (COUNTING && fl == 0) {
-                    const u32 i0 = thr_key - 1u - key16(r);
-                    if (i0 < lo_n) {
-                        reds_add_free(hlo + 4u * i0, 1u);
-                    }
+                if (COUNT) {
+                    reds_inc_below(hlo, thr_key - 1u - key16(r), lo_n);
                 }
             }
         }
     }
-    sts_f32(A.out + 16u * (u32)tid, a0);
-    sts_f32(A.out + 16u * (u32)tid + 4u, a1);
-    sts_f32(A.out + 16u * (u32)tid + 8u, a2);
-    sts_f32(A.out + 16u * (u32)tid + 12u, a3);
+    __syncthreads();  // (the sums lie over the warps' exponentials)
+    sts_f4(A.out + 16u * (u32)tid, a0, a1, a2, a3);
+}
+
+// The runs of a nucleus for the replay of the reference's scan (shared-memory addresses): probability and first position of each,
+// run at the first position of every 256-entry chunk, aggregate of every chunk.
+struct FRuns {
+    u32 pr, st, at, agg;
+    u32 N;
+    int M, nch;
+};
+// The 8 consecutive probabilities of this lane in chunks c, c + 8, .. (U of them, worked on together: a chunk alone is a search
+// of dependent loads, a walk and two serial chains).
+template<int U>
+__device__ __forceinline__ void f_load8(const FRuns& R, int c, float (*x)[8])
+{
+    const u32 p0 = (u32)c * 256u + (threadIdx.x & 31u) * 8u;
+    int       at[U], hi[U], span = 0;
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+        const bool in = c + q * kWarps < R.nch;
+        at[q]         = in ? (int)lds_u32(R.at + 4u * (u32)(c + q * kWarps)) : R.M - 1;
+        hi[q]         = in ? (int)lds_u32(R.at + 4u * (u32)(c + q * kWarps) + 4u) : R.M - 1;
+        span |= hi[q] - at[q];
+    }
+    for (int s = span > 0 ? 1 << (31 - __clz(span)) : 0; s > 0; s >>= 1) {
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int t = at[q] + s;
+            if (t <= hi[q] && lds_u32(R.st + 4u * (u32)t) <= p0 + (u32)(q * kWarps) * 256u) {
+                at[q] = t;
+            }
+        }
+    }
+    // Three runs from the first on, looked up ahead (a walk from run to run is a dependent load and a branch per step, which some
+    // lane of the warp takes nearly every time); a lane that needs more walks.
+    float pr[U][3];
+    u32   nx[U][3];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int t = at[q] + i < R.M ? at[q] + i : R.M - 1;
+            pr[q][i]    = __uint_as_float(lds_u32(R.pr + 4u * (u32)t));
+            nx[q][i]    = lds_u32(R.st + 4u * (u32)t + 4u);  // (behind the last run stands N)
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+        const u32 p = p0 + (u32)(q * kWarps) * 256u;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const u32 pe = p + (u32)e;
+            x[q][e]      = pe < nx[q][0] ? pr[q][0] : (pe < nx[q][1] ? pr[q][1] : pr[q][2]);
+            x[q][e]      = pe < R.N ? x[q][e] : 0.0f;
+        }
+        if (p + 7u >= nx[q][2] && nx[q][2] < R.N) {
+            int   i = at[q] + 2;
+            float v = pr[q][2];
+            u32   n = nx[q][2];
+#pragma unroll
+            for (int e = 3; e < 8; ++e) {
+                const u32 pe = p + (u32)e;
+                if (pe >= n && i + 1 < R.M) {
+                    ++i;
+                    v = __uint_as_float(lds_u32(R.pr + 4u * (u32)i));
+                    n = lds_u32(R.st + 4u * (u32)i + 4u);
+                }
+                x[q][e] = pe >= nx[q][2] && pe < R.N ? v : x[q][e];
+            }
+        }
+    }
+}
+// Aggregate of every 256-value chunk in cub::BlockScan's raking order (32 segments of 8, Kogge-Stone across the segment totals);
+// the chunks are independent of the running prefix.  Four chunks a warp at a time.
+static __device__ __noinline__ void f_chunk_aggregates(const FRuns R)
+{
+    constexpr int U = 4;
+    const int     lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int c = threadIdx.x >> 5; c < R.nch; c += kWarps * U) {
+        float x[U][8], inc[U];
+        f_load8<U>(R, c, x);
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            inc[q] = x[q][0];
+#pragma unroll
+            for (int i = 1; i < 8; ++i) {
+                inc[q] = inc[q] + x[q][i];
+            }
+        }
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const float t = __shfl_up_sync(0xffffffffu, inc[q], off);
+                if (lane >= off) {
+                    inc[q] = inc[q] + t;
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (lane == 31 && c + q * kWarps < R.nch) {
+                sts_f32(R.agg + 4u * (u32)(c + q * kWarps), inc[q]);
+            }
+        }
+    }
+}
+
+// The listed columns of a top-p row, (~key(probability) << 32) | column, into ascending order.  `bins` [kWarps * kFRing * 4] and `by` [n_sp]
+// are scratch (the ring of the pass and the records of the second one); `first`: no entry's leading word is below it.
+static __device__ __noinline__ void f_sort_listed(u64* spec, int n_sp, u32* bins, u64* by, u32* s_wsum, u32 first)
+{
+    const int tid = threadIdx.x;
+    FTB_ASSUME_SHARED(spec);
+    FTB_ASSUME_SHARED(bins);
+    FTB_ASSUME_SHARED(by);
+    FTB_ASSUME_SHARED(s_wsum);
+    if (n_sp <= kThreads) {
+        // (distinct words: the place of each is the number of smaller ones; no network and none of its barriers)
+        const u64 mine = tid < n_sp ? spec[tid] : ~0ull;
+        int       at   = 0;
+        if ((tid & ~31) < n_sp) {
+#pragma unroll 4
+            for (int b = 0; b < n_sp; ++b) {
+                at += spec[b] < mine ? 1 : 0;
+            }
+        }
+        __syncthreads();
+        if (tid < n_sp) {
+            spec[at] = mine;
+        }
+    }
+    else {
+        // Many of them (a long history): by bins of the probability's leading bits, 128 an octave, then by counting inside a bin, which
+        // holds a few.  (A sorting network over
+        // 600 of them: 9 us, this form 3.)
+        constexpr int kBins = kWarps * kFRing * 4;
+        auto bin_of = [&](u64 e) {
+            const u32 k = (u32)(e >> 32), b = (k > first ? k - first : 0u) >> 16;
+            return b < (u32)kBins ? b : (u32)kBins - 1u;
+        };
+        for (int i = tid; i < kBins; i += kThreads) {
+            bins[i] = 0;
+        }
+        __syncthreads();
+        for (int i = tid; i < n_sp; i += kThreads) {
+            smem_add(&bins[bin_of(spec[i])], 1u);
+        }
+        __syncthreads();
+        {
+            constexpr int PER = kBins / kThreads;
+            u32           c[PER], mine = 0;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                c[i] = bins[tid * PER + i];
+                mine += c[i];
+            }
+            u32 run = f_block_excl(mine, s_wsum, nullptr);
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                bins[tid * PER + i] = run;
+                run += c[i];
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < n_sp; i += kThreads) {
+            const u64 e = spec[i];
+            by[atomicAdd(&bins[bin_of(e)], 1u)] = e;
+        }
+        __syncthreads();
+        // (a bin's counter now holds where it ends, the one in front of it where it starts)
+        for (int i = tid; i < n_sp; i += kThreads) {
+            const u64 e  = by[i];
+            const u32 b  = bin_of(e);
+            const int lo = b > 0 ? (int)bins[b - 1] : 0, hi = (int)bins[b];
+            int       at = lo;
+#pragma unroll 1
+            for (int j = lo; j < hi; ++j) {
+                at += by[j] < e ? 1 : 0;
+            }
+            spec[at] = e;
+        }
+    }
 }
 
 // Everything of a top-p row after the pass and the listed columns.  Returns true when the row is done.
@@ -848,13 +1002,13 @@ template<int DT>
 __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, const FHdr& H, const FGeo& G, const FTopp T, u64* spec,
                                u32* s_nspec, const u32* s_mass, float mass_tail, u32 smax_key, u64* trace)
 {
-    __shared__ float s_w[kWarps], s_den, s_R;
+    __shared__ float s_w[kWarps], s_den;
     __shared__ u32   s_cut, s_wsum[kWarps], s_ncls, s_fail;
-    __shared__ int   s_c1, s_sel, s_imin, s_imax, s_first;
+    __shared__ int   s_sel, s_imin, s_imax, s_first, s_after;
     const int        tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const bool       temp = P.apply_temp != 0;
     u32* const       hist = S.hist;
-    u32* const       hlo  = S.sval;
+    u32* const       hlo  = S.lo;
     u32* const       cand = S.cand;
     FTB_ASSUME_SHARED(hist);
     FTB_ASSUME_SHARED(hlo);
@@ -882,6 +1036,27 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         mhi += __expf(fkey_inv(~(u32)(spec[i] >> 32)) - maxv);
     }
     mhi = f_block_sum(mhi, s_w);
+    // records of the special columns: their buckets' first places, then (below) every one to its place
+    const int  nwhole = P.vocab >> 10, npair = (nwhole + 1) >> 1, nbucket = kWarps * npair;
+    u32* const ends    = S.emask + kFRow2Ring / 4;
+    u32* const records = ends + nbucket;
+    FTB_ASSUME_SHARED(records);
+    FTB_ASSUME_SHARED(ends);
+    {
+        const int per = (nbucket + kThreads - 1) / kThreads, b0 = tid * per, b1 = b0 + per < nbucket ? b0 + per : nbucket;
+        u32       mine = 0;
+#pragma unroll 1
+        for (int b = b0; b < b1; ++b) {
+            mine += ends[b];
+        }
+        u32 run = f_block_excl(mine, s_wsum, nullptr);
+#pragma unroll 1
+        for (int b = b0; b < b1; ++b) {
+            const u32 c = ends[b];
+            ends[b]     = run;
+            run += c;
+        }
+    }
     if (wid == 0) {
         // (warp 0: four mass bins per lane, a scan over the lanes; the sums are estimates, their order is free)
         static_assert(kFMassBins == 128, "four bins per lane");
@@ -927,12 +1102,27 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
             s_fail = 0;
         }
     }
-    for (int i = tid; i < kFBins; i += kThreads) {
-        hlo[i] = 0;  // (the raw values of the special columns are done with: the listed ones carry their final value)
-    }
     __syncthreads();
     const u32   cut_key = s_cut;
     const float cut_y   = cut_key < thr_key ? value_of(cut_key) : T.thr_y;
+    for (int i = tid; i < P.hash_slots; i += kThreads) {
+        const u32 w  = S.hash[i];
+        const int id = (int)(w >> 2);
+        if (w == kHashEmpty || id >= P.vocab) {
+            continue;
+        }
+        if (id < nwhole * 1024) {
+            records[atomicAdd(&ends[f_bucket(id, npair)], 1u)] = f_record(i, id);
+        }
+        const float y = __uint_as_float(S.sval[i]);
+        if (y >= cut_y && !(y >= T.thr_y) && y > neg_max) {  // (those at or above the threshold are listed already)
+            const u32 pos = atomicAdd(s_nspec, 1u);
+            if (pos < (u32)kFPSpecCap) {
+                spec[pos] = ((u64)(~fkey(y)) << 32) | (u32)id;
+            }
+        }
+    }
+    __syncthreads();
     trace_mark(trace, 6);
 
     // ---- pass 2 ----
@@ -940,22 +1130,20 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     FTB_ASSUME_SHARED(s_vt);
     {
         FPass2 A;
-        A.rowp = G.rowp, A.nch = P.vocab / 1024, A.vocab = P.vocab, A.shift = P.hash_shift, A.mask = P.hash_slots - 1;
-        A.apply_rep = P.apply_rep, A.penalty_type = P.penalty_type;
-        A.maxv = maxv, A.inv_t = H.inv_t, A.theta = H.theta, A.cut_y = cut_y, A.thr_y = T.thr_y, A.neg_max = neg_max;
-        A.thr_key = thr_key, A.lo_n = thr_key - cut_key, A.inv_t_h = H.inv_t_h;
-        A.emask = (u32)__cvta_generic_to_shared(S.emask), A.hash = (u32)__cvta_generic_to_shared(S.hash);
-        A.hlo = (u32)__cvta_generic_to_shared(hlo), A.spec = (u32)__cvta_generic_to_shared(spec);
-        A.nspec = (u32)__cvta_generic_to_shared(s_nspec), A.out = (u32)__cvta_generic_to_shared(s_vt);
-        // (the common case without temperature comes in two forms: with and without the per-pattern count)
+        A.rowp = G.rowp, A.nch = nwhole, A.vocab = P.vocab, A.shift = P.hash_shift, A.mask = P.hash_slots - 1;
+        A.maxv = maxv, A.inv_t = H.inv_t, A.thr_key = thr_key, A.lo_n = thr_key - cut_key, A.inv_t_h = H.inv_t_h;
+        A.hash = (u32)__cvta_generic_to_shared(S.hash), A.value = (u32)__cvta_generic_to_shared(S.sval);
+        A.list = (u32)__cvta_generic_to_shared(records), A.ends = (u32)__cvta_generic_to_shared(ends), A.ring = (u32)__cvta_generic_to_shared(S.emask);
+        A.hlo = (u32)__cvta_generic_to_shared(hlo), A.out = (u32)__cvta_generic_to_shared(s_vt), A.buf = A.out;
+        const bool positive = cut_key >= 0x8000u && thr_key > 0x8000u;
         if (temp) {
-            f_pass2<DT, true, true>(A);
+            positive ? f_pass2<DT, true, kCountPositive>(A) : f_pass2<DT, true, kCountAny>(A);
         }
-        else if (cut_key < thr_key) {
-            f_pass2<DT, false, true>(A);
+        else if (cut_key >= thr_key) {
+            f_pass2<DT, false, kCountNone>(A);
         }
         else {
-            f_pass2<DT, false, false>(A);
+            positive ? f_pass2<DT, false, kCountPositive>(A) : f_pass2<DT, false, kCountAny>(A);
         }
     }
     __syncthreads();
@@ -1050,24 +1238,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         spec[i]     = ((u64)(~fkey(prob_of(fkey_inv(~(u32)(e >> 32))))) << 32) | (e & 0xffffffffu);
     }
     __syncthreads();
-    if (n_sp <= kThreads) {
-        // (distinct words: the place of each is the number of smaller ones; no network and none of its barriers)
-        const u64 mine = tid < n_sp ? spec[tid] : ~0ull;
-        int       at   = 0;
-        if ((tid & ~31) < n_sp) {
-#pragma unroll 4
-            for (int b = 0; b < n_sp; ++b) {
-                at += spec[b] < mine ? 1 : 0;
-            }
-        }
-        __syncthreads();
-        if (tid < n_sp) {
-            spec[at] = mine;
-        }
-    }
-    else {
-        group_sort_u64<CtaSync, true>(spec, n_sp, tid, kThreads, CtaSync());
-    }
+    f_sort_listed(spec, n_sp, (u32*)S.wbuf, (u64*)S.emask, s_wsum, ~fkey(p_max));
     __syncthreads();
     u32* const run_pr = S.emask;            // [kFPRuns] probability of the run (float bits), descending
     u32* const run_st = run_pr + kFPRuns;   // [kFPRuns] length, then first position of the run
@@ -1231,6 +1402,9 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
                 at += c;
             }
         }
+        if (tid == 0) {
+            run_st[M] = N;
+        }
     }
     __syncthreads();
     trace_mark(trace, 8);
@@ -1256,6 +1430,8 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
         return lo;
     };
+    FRuns R;
+    R.pr = (u32)__cvta_generic_to_shared(run_pr), R.st = (u32)__cvta_generic_to_shared(run_st), R.at = (u32)__cvta_generic_to_shared(hlo), R.agg = (u32)__cvta_generic_to_shared(hlo + 1008), R.M = M, R.N = N, R.nch = nch;
     // run at the first position of every 256-entry chunk, and the chunk aggregates (the pattern counts below the
     // threshold are done with: both live where they were)
     int* const   run_at = (int*)hlo;              // [nch + 1]
@@ -1266,87 +1442,19 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         run_at[c] = c < nch ? run_of((u32)c * 256u) : M - 1;
     }
     __syncthreads();
-    auto load8 = [&](int c, float* x) {  // the 8 consecutive probabilities of this lane in chunk c
-        const u32 p0 = (u32)c * 256u + (u32)lane * 8u;
-        int       i  = 0;
-        if (p0 < N) {
-            int lo = run_at[c], hi = run_at[c + 1];
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (run_st[mid] <= p0) {
-                    lo = mid;
-                }
-                else {
-                    hi = mid - 1;
-                }
-            }
-            i = lo;
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const u32 p = p0 + (u32)e;
-            if (p < N) {
-                if (i + 1 < M && run_st[i + 1] <= p) {
-                    ++i;
-                }
-                x[e] = __uint_as_float(run_pr[i]);
-            }
-            else {
-                x[e] = 0.0f;
-            }
-        }
-    };
-    // aggregate of every 256-value chunk in cub::BlockScan's raking order (32 segments of 8, Kogge-Stone across
-    // the segment totals); the chunks are independent of the running prefix
-    for (int c = wid; c < nch; c += kWarps) {
-        float x[8];
-        load8(c, x);
-        float up = x[0];
-#pragma unroll
-        for (int i = 1; i < 8; ++i) {
-            up = up + x[i];
-        }
-        float inc = up;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const float t = __shfl_up_sync(0xffffffffu, inc, off);
-            if (lane >= off) {
-                inc = inc + t;
-            }
-        }
-        if (lane == 31) {
-            agg[c] = inc;
-        }
-    }
+    f_chunk_aggregates(R);
     __syncthreads();
-    // running prefix chunk by chunk, as the reference's prefix functor accumulates it; stop a little early
+    // running prefix chunk by chunk, as the reference's prefix functor accumulates it; stopped a little early
     // (partial sums inside a chunk differ from prefix + aggregate only in the last bits)
-    if (tid == 0) {
-        float       R    = 0.0f;
-        int         c1   = nch;
-        const float stop = rand_num * (1.0f - 1e-4f);
-        for (int c = 0; c < nch; ++c) {
-            const float R2 = R + agg[c];
-            if (R2 >= stop) {
-                c1 = c;
-                break;
-            }
-            R = R2;
-        }
-        s_c1 = c1;
-        s_R  = R;
-    }
-    __syncthreads();
-    if (s_c1 >= nch) {
-        return false;  // the draw lies beyond the counted range
-    }
     if (wid == 0) {
-        float R   = s_R;
+        float pre = 0.0f;
         int   sel = -2;
-        for (int c = s_c1; c < nch; ++c) {
-            float x[8];
-            load8(c, x);
-            float up = x[0];
+        int   c   = running_prefix(agg, nch, rand_num * (1.0f - 1e-4f), pre);  // (nch: the draw lies beyond the counted range)
+        for (; c < nch; ++c) {
+            float x1[1][8];
+            f_load8<1>(R, c, x1);
+            const float* x  = x1[0];
+            float        up = x[0];
 #pragma unroll
             for (int i = 1; i < 8; ++i) {
                 up = up + x[i];
@@ -1361,7 +1469,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
             }
             const float ag  = __shfl_sync(0xffffffffu, inc, 31);
             const float ex  = __shfl_up_sync(0xffffffffu, inc, 1);
-            float       o   = lane == 0 ? R : R + ex;
+            float       o   = lane == 0 ? pre : pre + ex;
             u32         cnt = 0;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -1384,7 +1492,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
                 }
                 break;
             }
-            R = R + ag;
+            pre = pre + ag;
         }
         if (lane == 0) {
             s_sel = sel;
@@ -1415,6 +1523,18 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
             }
         }
         s_first = (int)run_st[lo];
+        int hj = M;  // first run behind them
+        lo     = i_at;
+        while (lo < hj) {
+            const int mid = (lo + hj) >> 1;
+            if (fkey(__uint_as_float(run_pr[mid])) >= k_sel) {
+                lo = mid + 1;
+            }
+            else {
+                hj = mid;
+            }
+        }
+        s_after = (int)run_st[lo];
     }
     __syncthreads();
     // bit patterns that map to this probability (one pattern past the counted range is looked at too: a class
@@ -1427,7 +1547,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
     }
     __syncthreads();
-    const int J = sel - s_first;
+    const int J = sel - s_first, n_all = s_after - s_first;  // place in the class, and its columns
     if (s_imax >= npat) {
         return false;
     }
@@ -1444,6 +1564,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
             }
         }
     }
+    int J_far = J;  // its place among the columns that are listed
     if (imax >= 0) {
         const u32 k_hi = ktop - (u32)imin, k_lo = ktop - (u32)imax;
         if (k_lo >= thr_key) {
@@ -1459,8 +1580,18 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
             }
         }
         else {
-            // below the threshold: one filtered pass over the row lists the ordinary columns of the band
-            __syncthreads();
+            // below the threshold: the ordinary columns of the band come from the row once more, and only as far as the J-th of
+            // the class - from whichever end it is nearer to, so a quarter of the row on average.  First the row's last columns.
+            const int tail0 = nfull * 8;
+            if (tail0 + tid < P.vocab && tid < 8 && hash_lookup_raw(S.hash, P.hash_shift, P.hash_slots - 1, tail0 + tid) == 0) {
+                const u32 key = key16((u32)__ldg((const unsigned short*)G.rowp + tail0 + tid));
+                if (key >= k_lo && key <= k_hi) {
+                    const u32 pos = atomicAdd(&s_ncls, 1u);
+                    if (pos < (u32)kFPClsCap) {
+                        cls[pos] = (u32)(tail0 + tid);
+                    }
+                }
+            }
             __shared__ FSink s_band;
             if (tid == 0) {
                 FSink& K = s_band;
@@ -1469,28 +1600,35 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
                 K.wbuf = S.wbuf, K.wj = S.wj;
             }
             __syncthreads();
-            f_stream<DT, true, kFUnroll>((const uint4*)(G.rowp + (size_t)G.head * 2), nfull, G.head, k_lo, k_hi, s_band, &s_fail);
-            // row edges
-            const int tail0 = G.head + nfull * 8;
-            const int nedge = G.head + (P.vocab - tail0 > 0 ? P.vocab - tail0 : 0);
-            for (int i = tid; i < nedge; i += kThreads) {
-                const int v = i < G.head ? i : tail0 + (i - G.head);
-                if (v < P.vocab && hash_lookup_raw(S.hash, P.hash_shift, P.hash_slots - 1, v) == 0) {
-                    const u32 key = key16((u32)__ldg((const unsigned short*)G.rowp + v));
-                    if (key >= k_lo && key <= k_hi) {
-                        const u32 pos = atomicAdd(&s_ncls, 1u);
-                        if (pos < (u32)kFPClsCap) {
-                            cls[pos] = (u32)v;
-                        }
-                    }
+            const int  known = (int)s_ncls;  // columns from anywhere in the row, in front of the band's
+            __syncthreads();
+            const bool back  = n_all - 1 - J < J, whole = known > kThreads;
+            const u32  kcol  = tid < known && !whole ? cls[tid] : 0u;
+            const int  need  = back ? n_all - 1 - J : J;
+            constexpr int kPart = kThreads * kFUnroll;
+            const int  parts = (nfull + kPart - 1) / kPart;
+            for (int i = 0; i < parts; ++i) {
+                const int part = back ? parts - 1 - i : i, j0 = part * kPart, nv = nfull - j0 < kPart ? nfull - j0 : kPart;
+                f_stream<DT, true, kFUnroll>((const uint4*)G.rowp + j0, nv, j0 * 8, k_lo, k_hi, s_band, &s_fail);
+                // the class's columns on the near side of what has been read: listed ones and the band's
+                const int edge = back ? j0 * 8 : (j0 + nv) * 8;
+                const int near = __syncthreads_count(tid < known && (back ? (int)kcol >= edge : (int)kcol < edge));
+                const int found = (int)s_ncls - known + near;
+                __syncthreads();  // (the count has been read before it goes on)
+                if (!whole && found > need) {
+                    break;
                 }
+            }
+            if (back) {
+                // (counted from the end: the columns left out all lie in front)
+                J_far = (int)s_ncls - 1 - need;
             }
         }
     }
     __syncthreads();
     trace_mark(trace, 10);
     const int ncls = (int)s_ncls;
-    if (ncls > kFPClsCap || J < 0 || J >= ncls) {
+    if (ncls > kFPClsCap || J_far < 0 || J_far >= ncls) {
         return false;
     }
     // J-th smallest column of the class (the reference's stable sort leaves equal probabilities in column order)
@@ -1499,12 +1637,18 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     }
     __syncthreads();
     for (int a = tid; a < ncls; a += kThreads) {
-        const u32 ca = cls[a];
-        int       rk = 0;
-        for (int b = 0; b < ncls; ++b) {
+        const u32    ca   = cls[a];
+        int          rk   = 0;
+        const uint4* four = (const uint4*)cls;
+#pragma unroll 2
+        for (int b = 0; b < ncls >> 2; ++b) {
+            const uint4 o = four[b];
+            rk += (o.x < ca ? 1 : 0) + (o.y < ca ? 1 : 0) + (o.z < ca ? 1 : 0) + (o.w < ca ? 1 : 0);
+        }
+        for (int b = ncls & ~3; b < ncls; ++b) {
             rk += cls[b] < ca ? 1 : 0;
         }
-        if (rk == J) {
+        if (rk == J_far) {
             s_sel = (int)ca;
         }
     }
@@ -1607,6 +1751,9 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     }
     for (int i = tid; i < kFBins; i += kThreads) {
         hist[i] = 0;
+        if (TOPP) {
+            S.lo[i] = 0;
+        }
     }
     for (int i = tid; i < (nfull + 3) / 4; i += kThreads) {
         emask32[i] = 0;
@@ -1782,10 +1929,19 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     trace_mark(trace, 4);
     // ---- listed columns: special ones with their final value, and the row's edges ----
     // (~key(value) << 32) | column.  Top-k rows: [kFSpecCap] where the per-vector bytes were (they are done with);
-    // top-p rows: [kFPSpecCap] where the row's set-up data was (the bytes are needed once more)
+    // top-p rows: [kFPSpecCap] where the row's set-up data was (the bytes make room for the records of the second pass)
     u64* const    spec     = TOPP ? (u64*)S.stage : (u64*)S.emask;
     constexpr int spec_cap = TOPP ? kFPSpecCap : kFSpecCap;
     FTB_ASSUME_SHARED(spec);
+    const int  nwhole = P.vocab >> 10, npair = (nwhole + 1) >> 1, nbucket = kWarps * npair;
+    u32* const ends   = S.emask + kFRow2Ring / 4;  // top-p rows: records per bucket, then where the buckets end
+    if (TOPP) {
+        FTB_ASSUME_SHARED(ends);
+        for (int i = tid; i < nbucket; i += kThreads) {
+            ends[i] = 0;
+        }
+        __syncthreads();
+    }
     {
         Xf X;
         X.bias = nullptr, X.inv_t = H.inv_t, X.theta = H.theta, X.neg_max = neg_max, X.inv_t_h = H.inv_t_h;
@@ -1802,7 +1958,44 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
                 }
             }
         };
-        for (int i = tid; i < P.hash_slots; i += kThreads) {
+        if (TOPP) {
+            // Every special column's final value goes where its raw value was, the pass that sums the exponentials reads it
+            // there.  That pass counts columns by raw value, the special ones with them, so they are taken off here.  Raw values
+            // below the threshold come from the row (it has just been read), four on their way per thread.
+            u32* const lo = S.lo;
+            FTB_ASSUME_SHARED(lo);
+            for (int i0 = tid; i0 < P.hash_slots; i0 += 4 * kThreads) {
+                u32 w[4], raw[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int i = i0 + q * kThreads;
+                    w[q]        = i < P.hash_slots ? hash[i] : kHashEmpty;
+                    w[q]        = w[q] != kHashEmpty && (int)(w[q] >> 2) < P.vocab ? w[q] : kHashEmpty;
+                    raw[q]      = w[q] != kHashEmpty ? sval[i] : 0u;
+                    if (raw[q] == 0xffffffffu) {
+                        raw[q] = (u32)__ldg((const unsigned short*)G.rowp + (w[q] >> 2));
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (w[q] == kHashEmpty) {
+                        continue;
+                    }
+                    const int   id = (int)(w[q] >> 2);
+                    const float y  = special_value<DT>(X, temp_value<DT>(X, raw[q], id), w[q] & 3u);
+                    sval[i0 + q * kThreads] = __float_as_uint(y);
+                    push(id, y);
+                    const u32 down = thr_key - 1u - key16(raw[q]);
+                    if (down < (u32)kFBins) {
+                        smem_add(&lo[down], 0xffffffffu);
+                    }
+                    if (id < nwhole * 1024) {
+                        smem_add(&ends[f_bucket(id, npair)], 1u);
+                    }
+                }
+            }
+        }
+        for (int i = tid; !TOPP && i < P.hash_slots; i += kThreads) {
             const u32 w = hash[i];
             if (w == kHashEmpty) {
                 continue;
@@ -2210,10 +2403,11 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     S.wj   = s_wj;
     S.cand = (u32*)smem_raw;
     S.emask = S.cand + kFCap;
-    S.hash  = S.emask + fast_mask_bytes(P.vocab_padded, TOPP) / 4;
+    S.hash  = S.emask + fast_mask_bytes(P.hash_slots, P.vocab_padded, TOPP) / 4;
     S.sval  = S.hash + P.hash_slots;
-    S.hist  = S.sval + (P.hash_slots > kFBins ? P.hash_slots : kFBins);
+    S.hist  = S.sval + (TOPP || P.hash_slots > kFBins ? P.hash_slots : kFBins);
     S.stage = S.hist + kFBins;
+    S.lo    = S.stage + 2 * kFPSpecCap;  // (top-p rows' kernel alone)
     }
     const int tid = threadIdx.x;
     // thread 0 keeps the next row's ticket and number between the stages

@@ -81,6 +81,43 @@ static __device__ void trace_mark(u64* rec, int i)
     }
 }
 
+// Running prefix over the aggregates of a nucleus scan's chunks (`agg` 16-byte aligned, readable up to a multiple of eight, no
+// negative ones), one addition after the other: the first chunk at which it reaches `stop` (n: none), and in R the prefix in front of
+// that chunk.  Eight at a time with the next eight on their way, the eight before the stop once more one by one.
+__device__ __forceinline__ int running_prefix(const float* agg, int n, float stop, float& R)
+{
+    FTB_ASSUME_SHARED(agg);
+    int    c  = 0;
+    float4 x0 = *(const float4*)agg, x1 = *(const float4*)(agg + 4);
+    R         = 0.0f;
+    while (c + 8 <= n) {
+        const int    nx = c + 16 <= ((n + 7) & ~7) ? c + 8 : 0;
+        const float4 y0 = *(const float4*)(agg + nx), y1 = *(const float4*)(agg + nx + 4);
+        float        R2 = R + x0.x;
+        R2 += x0.y;
+        R2 += x0.z;
+        R2 += x0.w;
+        R2 += x1.x;
+        R2 += x1.y;
+        R2 += x1.z;
+        R2 += x1.w;
+        if (R2 >= stop) {
+            break;
+        }
+        R  = R2;
+        x0 = y0, x1 = y1;
+        c += 8;
+    }
+    for (; c < n; ++c) {
+        const float R2 = R + agg[c];
+        if (R2 >= stop) {
+            break;
+        }
+        R = R2;
+    }
+    return c;
+}
+
 __device__ __forceinline__ u32 hash_slot(int id, int shift)
 {
     return (u32)(id * 2654435761u) >> shift;

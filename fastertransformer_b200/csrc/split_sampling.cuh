@@ -1007,37 +1007,9 @@ static __device__ __noinline__ u32 sp_find_crossing(const SpKeys& K, const float
     const u32 N    = K.start[K.owners];
     const int nch  = (int)((N + 255u) / 256u);
     // chunk by chunk, as the reference's prefix functor accumulates; stopped a little early (inside a chunk the partial
-    // sums differ from prefix + aggregate in the last bits only).  The terms are not negative: eight at a time, the eight
-    // before the stop once more one by one.
-    const float stop = rand_num * (1.0f - 1e-4f);
-    float       R    = 0.0f;
-    int         c1   = 0;
-    float4      x0 = *(const float4*)agg, x1 = *(const float4*)(agg + 4);
-    while (c1 + 8 <= nch) {
-        const int    nx = c1 + 16 <= ((nch + 7) & ~7) ? c1 + 8 : 0;
-        const float4 y0 = *(const float4*)(agg + nx), y1 = *(const float4*)(agg + nx + 4);
-        float        R2 = R + x0.x;
-        R2 += x0.y;
-        R2 += x0.z;
-        R2 += x0.w;
-        R2 += x1.x;
-        R2 += x1.y;
-        R2 += x1.z;
-        R2 += x1.w;
-        if (R2 >= stop) {
-            break;
-        }
-        R  = R2;
-        x0 = y0, x1 = y1;
-        c1 += 8;
-    }
-    for (; c1 < nch; ++c1) {
-        const float R2 = R + agg[c1];
-        if (R2 >= stop) {
-            break;
-        }
-        R = R2;
-    }
+    // sums differ from prefix + aggregate in the last bits only)
+    float     R  = 0.0f;
+    const int c1 = running_prefix(agg, nch, rand_num * (1.0f - 1e-4f), R);
     int sel = -1;
     for (int c = c1; c < nch; ++c) {
         float x[8];
