@@ -447,7 +447,7 @@ static __device__ int f_resolve_small(const u32* cols, int m, int want, int k, i
 // that none of the dependent loads behind it (ticket -> row number -> per-row arguments and generator state) is
 // waited for.
 struct FHdr {
-    int    t;  // ticket; >= the number of rows when none is left
+    int    t;  // ticket; local_batch when no row is left
     int    r, mode, fin, end_id, k;
     float  top_p, u, inv_t, theta;
     __half inv_t_h;
@@ -509,10 +509,10 @@ static __device__ void f_prefetch_header(const KParams& P, int nr, u32* pre)
 }
 
 // Header of ticket nt / row nr from what f_prefetch_header brought in (thread 0 only, after its copies landed).
-static __device__ void f_compose_header(const KParams& P, int nt, int nr, const u32* pre, FHdr& H)
+static __device__ void f_compose_header(const KParams& P, int nt, int rows, int nr, const u32* pre, FHdr& H)
 {
-    H.t = nt;
-    if (nt >= P.local_batch) {
+    H.t = nt < rows ? nt : P.local_batch;
+    if (nt >= rows) {
         return;
     }
     auto byte_at = [&](int slot, const void* p) { return (pre[slot] >> (8 * ((size_t)p & 3))) & 0xffu; };
@@ -946,8 +946,8 @@ static __device__ __noinline__ void f_sort_listed(u64* spec, int n_sp, u32* bins
     }
     else {
         // Many of them (a long history): by bins of the probability's leading bits, 128 an octave, then by counting inside a bin, which
-        // holds a few.  (A sorting network over
-        // 600 of them: 9 us, this form 3.)
+        // holds a few.  (Rows with 550 listed columns, runs and
+    // order together: 14.2 us with a sorting network over them, 13.1 so.)
         constexpr int kBins = kWarps * kFRing * 4;
         auto bin_of = [&](u64 e) {
             const u32 k = (u32)(e >> 32), b = (k > first ? k - first : 0u) >> 16;
@@ -2388,10 +2388,88 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     return true;
 }
 
-template<int DT, bool TOPP, int VP = 0>
-__global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(const __grid_constant__ KParams P)
+// The step's stop criteria for a host that waits for them, by the CTA that has just ended row r: the row's stop words, and - by the
+// CTA of the call's last row, whichever of the two kernels serves it - the length limit and the count of finished rows.  With rows on
+// the list nothing is counted: the host is told, and sends the kernel that serves them and the criteria.  A step of 1024 x 128256
+// then ends with the store of its last row's CTA, where the join of two streams, the general kernel over an empty list and the
+// criteria's kernel followed one another.
+static __device__ __noinline__ void f_stop_criteria(const KParams& P, const StopArgs& T, int r, bool done)
 {
-    asm volatile("griddepcontrol.launch_dependents;");  // (the kernel that serves the rows left here waits for this grid's end)
+    __shared__ u32 s_last;
+    const int      tid = threadIdx.x;
+    if (T.stop_words != nullptr && done) {
+        row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicAdd(T.arrived, 1u) == (u32)P.local_batch - 1u ? 1u : 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last == 0) {
+        return;
+    }
+    count_finished(P, T, __ldcg(P.redo_count) != 0);
+}
+
+// In front of the single-pass kernels: the header of the workspace (tickets, counters) to zero, and, where a call has rows of both
+// layers, either kernel's rows in the given order.  (Idle CTAs of the top-p rows' kernel that took 860 of 1024 rows off the tickets only
+// to see that they are the other kernel's held their SMs for 9 us.)  The layers' skip flags alone decide; the flags of finished
+// rows change while the kernels run.
+constexpr int kFListThreads = 1024;
+enum { kFHeadRowsK = 5, kFHeadRowsP = 6 };  // words of the header: rows of the two lists
+static __global__ void __launch_bounds__(kFListThreads) fast_rows_kernel(const __grid_constant__ KParams P, int* list_k, int* list_p)
+{
+    __shared__ u32 s_k[kFListThreads / 32], s_p[kFListThreads / 32];
+    asm volatile("griddepcontrol.launch_dependents;");
+    wait_for_previous();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int       n_k = 0, n_p = 0;
+    for (int base = 0; list_k != nullptr && base < P.local_batch; base += kFListThreads) {
+        const int  t  = base + tid;
+        const bool in = t < P.local_batch;
+        const int  r  = in ? (P.row_order != nullptr ? P.row_order[t] : t) : 0;
+        const bool topp = in && P.topk_skip != nullptr && P.topk_skip[r] != 0 && !(P.topp_skip != nullptr && P.topp_skip[r] != 0);
+        const u32  bk = __ballot_sync(0xffffffffu, in && !topp), bp = __ballot_sync(0xffffffffu, topp), below = (1u << lane) - 1u;
+        __syncthreads();
+        if (lane == 0) {
+            s_k[wid] = __popc(bk), s_p[wid] = __popc(bp);
+        }
+        __syncthreads();
+        int at_k = n_k, at_p = n_p;
+        for (int w = 0; w < kFListThreads / 32; ++w) {
+            const int ck = (int)s_k[w], cp = (int)s_p[w];
+            at_k += w < wid ? ck : 0, at_p += w < wid ? cp : 0;
+            n_k += ck, n_p += cp;
+        }
+        if (topp) {
+            list_p[at_p + __popc(bp & below)] = r;
+        }
+        else if (in) {
+            list_k[at_k + __popc(bk & below)] = r;
+        }
+    }
+    if (tid < 64) {
+        P.ticket[tid] = tid == kFHeadRowsK ? (u32)n_k : (tid == kFHeadRowsP ? (u32)n_p : 0u);
+    }
+}
+
+// The two kernels of a step with both kinds of rows follow each other in one stream and run side by side: the top-p rows' kernel lets
+// the other one come up at once, and that one waits for it at its end, so that what follows in the stream finds both done.  (A second
+// stream, forked and joined with events, cost four calls of the host in front of the kernels and a wait behind them.)
+template<int DT, bool TOPP, int VP = 0>
+__global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(const __grid_constant__ KParams P, const __grid_constant__ StopArgs T)
+{
+    // (the top-k rows' kernel comes up beside the top-p rows' one, which has seen the end of the kernel in front: it need not wait for
+    // that, but nothing that its SM has kept from before may be read)
+    if (TOPP || VP != 0) {
+        wait_for_previous();
+    }
+    else {
+        __threadfence();
+    }
+    asm volatile("griddepcontrol.launch_dependents;");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FHdr                               s_hdr[2];
     __shared__ __align__(16) u32                  s_pre[kFPreWords];
@@ -2411,15 +2489,17 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     }
     const int tid = threadIdx.x;
     // thread 0 keeps the next row's ticket and number between the stages
-    int nt = 0, nr = 0;
+    __shared__ int s_rows;  // rows of this kernel
+    int            nt = 0, nr = 0;
     if (tid == 0) {
-        nt = (int)atomicAdd(P.ticket + (TOPP ? 3 : 0), 1u);
-        if (nt < P.local_batch) {
-            nr = P.row_order != nullptr ? P.row_order[nt] : nt;
+        s_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
+        nt     = (int)atomicAdd(P.ticket + (TOPP ? 3 : 0), 1u);
+        if (nt < s_rows) {
+            nr = P.row_order != nullptr ? __ldcg(P.row_order + nt) : nt;
             f_prefetch_header(P, nr, s_pre);
             cp_async_wait_all();
         }
-        f_compose_header(P, nt, nr, s_pre, s_hdr[0]);
+        f_compose_header(P, nt, s_rows, nr, s_pre, s_hdr[0]);
     }
     for (int cur = 0;; cur ^= 1) {
         __syncthreads();
@@ -2437,36 +2517,24 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
             nt = (int)atomicAdd(P.ticket + (TOPP ? 3 : 0), 1u);  // stage 0 of the next row's header
         }
         auto stage1 = [&]() {
-            if (tid == 0 && nt < P.local_batch) {
-                nr = P.row_order != nullptr ? P.row_order[nt] : nt;
+            if (tid == 0 && nt < s_rows) {
+                nr = P.row_order != nullptr ? __ldcg(P.row_order + nt) : nt;
             }
         };
         auto stage2 = [&]() {
-            if (tid == 0 && nt < P.local_batch) {
+            if (tid == 0 && nt < s_rows) {
                 f_prefetch_header(P, nr, s_pre);
             }
         };
         bool       done   = false;
         int* const id_out = P.output_ids + (size_t)P.step * P.batch_size + (size_t)P.ite * P.local_batch + r;
-        const bool topp_row = H.mode == 2 && !H.fin;
-        if (VP == 0 && topp_row != TOPP && !(TOPP && P.topk_states == nullptr)) {
-            // the other kernel's row (a call without a top-k layer launches the top-p rows' kernel alone, and that one
-            // then looks after every row)
-            stage1();
-            stage2();
-            __syncthreads();
-            if (tid == 0) {
-                cp_async_wait_all();
-                f_compose_header(P, nt, nr, s_pre, s_hdr[cur ^ 1]);
-            }
-            continue;
-        }
+        const bool topp_row = H.mode == 2;
         if (VP != 0 && !(H.mode == 1 && !H.fin)) {
             // vocabulary-parallel local pass: a top-p row is left to the general kernel (its statistics form), any
             // other row has nothing to send
             stage1();
             stage2();
-            if (!topp_row) {
+            if (!topp_row || H.fin) {
                 if (tid == 0) {
                     P.vp_out[(size_t)r * (P.vp_cap + 2)] = 0;
                 }
@@ -2550,8 +2618,14 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
             }
             // the next row's header: its arguments were sent for before this row's pass
             cp_async_wait_all();
-            f_compose_header(P, nt, nr, s_pre, s_hdr[cur ^ 1]);
+            f_compose_header(P, nt, s_rows, nr, s_pre, s_hdr[cur ^ 1]);
         }
+        if (VP == 0 && T.limit != nullptr) {
+            f_stop_criteria(P, T, r, done);
+        }
+    }
+    if (!TOPP && VP == 0) {
+        wait_for_previous();
     }
 }
 
@@ -2579,10 +2653,20 @@ int fast_sampling_occupancy(size_t smem, int* per_sm)
     return FTB200_OK;
 }
 
-template<int DT, bool TOPP, int VP = 0>
-int fast_sampling_launch(const KParams& K, int grid, size_t smem, cudaStream_t st)
+inline int fast_rows_launch(const KParams& K, int* list_k, int* list_p, cudaStream_t st)
 {
-    fast_sampling_kernel<DT, TOPP, VP><<<grid, kThreads, smem, st>>>(K);
+    FTB_CUDA_CHECK(launch_early(fast_rows_kernel, dim3(1), dim3(kFListThreads), 0, st, K, list_k, list_p));
+    return FTB200_OK;
+}
+
+template<int DT, bool TOPP, int VP = 0>
+int fast_sampling_launch(const KParams& K, const StopArgs& T, int grid, size_t smem, bool beside, cudaStream_t st)
+{
+    if (beside) {
+        FTB_CUDA_CHECK(launch_early(fast_sampling_kernel<DT, TOPP, VP>, dim3((unsigned)grid), dim3(kThreads), smem, st, K, T));
+        return FTB200_OK;
+    }
+    fast_sampling_kernel<DT, TOPP, VP><<<grid, kThreads, smem, st>>>(K, T);
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
 }

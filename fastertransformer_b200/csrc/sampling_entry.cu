@@ -1,7 +1,6 @@
 // extern "C" entry of the fused decode-sampling step: argument checks, shared-memory plan, launch.
 #include <atomic>
 #include <chrono>
-#include <mutex>
 
 #include "sampling_params.cuh"
 #include "spans.cuh"
@@ -23,19 +22,19 @@ extern template int sampling_launch<FTB200_BF16>(const KParams&, int, size_t, cu
 template<int DT, bool TOPP, int VP = 0>
 int fast_sampling_occupancy(size_t smem, int* per_sm);
 template<int DT, bool TOPP, int VP = 0>
-int fast_sampling_launch(const KParams& K, int grid, size_t smem, cudaStream_t st);
+int fast_sampling_launch(const KParams& K, const StopArgs& T, int grid, size_t smem, bool beside, cudaStream_t st);
 extern template int fast_sampling_occupancy<FTB200_F16, false, 1>(size_t, int*);
 extern template int fast_sampling_occupancy<FTB200_BF16, false, 1>(size_t, int*);
-extern template int fast_sampling_launch<FTB200_F16, false, 1>(const KParams&, int, size_t, cudaStream_t);
-extern template int fast_sampling_launch<FTB200_BF16, false, 1>(const KParams&, int, size_t, cudaStream_t);
+extern template int fast_sampling_launch<FTB200_F16, false, 1>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
+extern template int fast_sampling_launch<FTB200_BF16, false, 1>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
 extern template int fast_sampling_occupancy<FTB200_F16, false>(size_t, int*);
 extern template int fast_sampling_occupancy<FTB200_BF16, false>(size_t, int*);
-extern template int fast_sampling_launch<FTB200_F16, false>(const KParams&, int, size_t, cudaStream_t);
-extern template int fast_sampling_launch<FTB200_BF16, false>(const KParams&, int, size_t, cudaStream_t);
+extern template int fast_sampling_launch<FTB200_F16, false>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
+extern template int fast_sampling_launch<FTB200_BF16, false>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
 extern template int fast_sampling_occupancy<FTB200_F16, true>(size_t, int*);
 extern template int fast_sampling_occupancy<FTB200_BF16, true>(size_t, int*);
-extern template int fast_sampling_launch<FTB200_F16, true>(const KParams&, int, size_t, cudaStream_t);
-extern template int fast_sampling_launch<FTB200_BF16, true>(const KParams&, int, size_t, cudaStream_t);
+extern template int fast_sampling_launch<FTB200_F16, true>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
+extern template int fast_sampling_launch<FTB200_BF16, true>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
 template<int DT>
 int split_sampling_launch(const KParams& K, const SplitArgs& A, cudaStream_t st);
 extern template int split_sampling_launch<FTB200_F32>(const KParams&, const SplitArgs&, cudaStream_t);
@@ -47,6 +46,7 @@ extern template int split_resident<FTB200_F32>(int, bool, size_t);
 extern template int split_resident<FTB200_F16>(int, bool, size_t);
 extern template int split_resident<FTB200_BF16>(int, bool, size_t);
 size_t fast_smem_for(int hash_slots, int vocab_padded, bool topp);
+int    fast_rows_for(const KParams& K, int* list_k, int* list_p, cudaStream_t st);
 int    fast_max_history();
 int    fast_max_words();
 template<int DT>
@@ -209,35 +209,6 @@ static bool wide_areas(int vocab, SplitArgs* A)
         A->area -= 1024;
     }
     return split_smem_bytes(A->slice, A->area) <= kSpMaxSmem;
-}
-
-// Second stream of the single-pass step (one per device, made on first use) with the two events of its fork and join.
-struct SideStream {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t  fork = nullptr, join = nullptr;
-    std::mutex   use;  // held from the record of `fork` to the wait on `join`: two host threads on one device
-                       // share the stream and the events, and a wait takes the latest record of its event
-};
-static int side_stream(SideStream** out)
-{
-    constexpr int     kMaxDev = 64;
-    static SideStream g_side[kMaxDev];
-    static std::mutex g_mu;
-    int               dev = 0;
-    FTB_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev) {
-        set_error("ftb200_decode_step_sampling: device ordinal out of range");
-        return FTB200_UNSUPPORTED;
-    }
-    std::lock_guard<std::mutex> lock(g_mu);
-    SideStream& s = g_side[dev];
-    if (s.stream == nullptr) {
-        FTB_CUDA_CHECK(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
-        FTB_CUDA_CHECK(cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming));
-        FTB_CUDA_CHECK(cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming));
-    }
-    *out = &s;
-    return FTB200_OK;
 }
 
 }  // namespace ftb200
@@ -414,18 +385,18 @@ extern "C" int ftb200_set_row_trace(uint64_t* device_buf)
     return FTB200_OK;
 }
 
-// One fused step.  `fork` allows the second stream of the single-pass kernels (made on first use); without it
-// the same kernels run one after the other on the caller's stream and nothing is created.
+// One fused step.
 namespace ftb200 {
-// left_only: the rows that the split kernel of the same step has flagged, by the general kernel.
-int decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop = nullptr,
+// left_only: the rows that the split kernel of the same step has flagged, or the single-pass kernels have listed, by the general
+// kernel.
+int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop = nullptr,
                               bool* stop_done = nullptr, bool left_only = false);
 int stop_criteria_launch(const ftb200_sampling_params* p, const StopArgs& T, cudaStream_t st);
 }
 
 extern "C" int ftb200_decode_step_sampling(const ftb200_sampling_params* p)
 {
-    return decode_step_sampling_impl(p, true);
+    return decode_step_sampling_impl(p);
 }
 
 extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_params* s, int timeout_ms, int* should_stop)
@@ -444,7 +415,7 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     T.result         = (u64*)s->result_host;
     T.sequence       = ++s->sequence;
     bool done        = false;
-    int  rc          = decode_step_sampling_impl(p, true, &T, &done);
+    int  rc          = decode_step_sampling_impl(p, &T, &done);
     if (rc == FTB200_OK && !done) {
         rc = stop_criteria_launch(p, T, (cudaStream_t)p->stream);
     }
@@ -452,12 +423,12 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     if (rc != FTB200_OK || T.limit == nullptr) {
         return rc;
     }
-    // Rare: rows that the split kernel's tables could not hold, then the criteria over the whole call.  The rows are found
+    // Rare: rows that the tables of the first launches could not hold, then the criteria over the whole call.  The rows are found
     // by their flags on the device, so that these launches do nothing new where none is left.
     bool       left_sent = !done;
     const auto send_left = [&] {
         left_sent   = true;
-        const int e = decode_step_sampling_impl(p, true, nullptr, nullptr, true);
+        const int e = decode_step_sampling_impl(p, nullptr, nullptr, true);
         return e == FTB200_OK ? stop_criteria_launch(p, T, (cudaStream_t)p->stream) : e;
     };
     // The last kernel of the step stores (sequence, count) into the page-locked word: no query of the stream, whose
@@ -496,8 +467,7 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     }
 }
 
-int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop, bool* stop_done,
-                                      bool left_only)
+int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, bool* stop_done, bool left_only)
 {
     if (!left_only) {
         reset_launch_count();
@@ -565,9 +535,7 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
             K.stop_words = stop->stop_words, K.stop_words_len = stop->stop_words_len, K.stop_finished = stop->finished;
         }
     }
-    if (K.row_flags == nullptr) {
-        FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
-    }
+    const bool list_left = left_only && K.row_flags == nullptr;  // (the single-pass kernels of this step have put rows on their list)
     if (single_pass && K.row_flags == nullptr) {
         const size_t fsmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, false);
         const size_t psmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, true);
@@ -586,58 +554,65 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork
             KParams F    = K;
             F.redo_count = K.ticket + 1;
             F.redo_rows  = (int*)((char*)p->workspace + 256);
+            StopArgs S{};
+            if (!list_left && stop != nullptr && stop->limit != nullptr) {
+                S          = *stop;
+                S.arrived  = K.ticket + 4;
+                *stop_done = true;
+            }
             // The rows of the top-p layer have a kernel of their own (it wants more registers than the top-k rows'
-            // kernel can spare); the two run side by side, the top-p one on a second stream that forks from and
-            // joins the caller's.  Each walks the row list and skips the other's rows.
-            SideStream*                  side      = nullptr;
-            std::unique_lock<std::mutex> side_use;
-            const bool  topp_only = K.topp_states != nullptr && K.topk_states == nullptr;  // no fork, one launch
-            if (K.topp_states != nullptr) {
-                cudaStream_t pst = st;
-                if (fork && !topp_only) {
-                    rc = side_stream(&side);
-                    if (rc != FTB200_OK) {
-                        return rc;
-                    }
-                    side_use = std::unique_lock<std::mutex>(side->use);
-                    FTB_CUDA_CHECK(cudaEventRecord(side->fork, st));
-                    FTB_CUDA_CHECK(cudaStreamWaitEvent(side->stream, side->fork, 0));
-                    pst = side->stream;
+            // kernel can spare); the two run side by side.
+            const bool topp_only = K.topp_states != nullptr && K.topk_states == nullptr;  // one launch
+            const bool both      = K.topp_states != nullptr && K.topk_states != nullptr;
+            int* const list_k    = (int*)K.scratch;  // (the general kernel takes the scratch area once these have ended)
+            int* const list_p    = list_k + p->local_batch_size;
+            if (!list_left) {
+                rc = fast_rows_for(F, both ? list_k : nullptr, list_p, st);
+                if (rc != FTB200_OK) {
+                    return rc;
+                }
+                note_launch(1);
+            }
+            if (K.topp_states != nullptr && !list_left) {
+                if (both) {
+                    F.row_order = list_p, F.row_count_dev = K.ticket + 6;
                 }
                 int pgrid = sm_count() * pper;
                 pgrid     = pgrid < p->local_batch_size ? pgrid : p->local_batch_size;
-                rc = f16 ? fast_sampling_launch<FTB200_F16, true>(F, pgrid, psmem, pst) :
-                           fast_sampling_launch<FTB200_BF16, true>(F, pgrid, psmem, pst);
+                rc = f16 ? fast_sampling_launch<FTB200_F16, true>(F, S, pgrid, psmem, true, st) :
+                           fast_sampling_launch<FTB200_BF16, true>(F, S, pgrid, psmem, true, st);
                 if (rc != FTB200_OK) {
                     return rc;
                 }
                 note_launch(1);
-                if (side != nullptr) {
-                    FTB_CUDA_CHECK(cudaEventRecord(side->join, side->stream));
-                }
             }
-            if (!topp_only) {
+            if (!topp_only && !list_left) {
+                if (both) {
+                    F.row_order = list_k, F.row_count_dev = K.ticket + 5;
+                }
                 int fgrid = sm_count() * fper;
                 fgrid     = fgrid < p->local_batch_size ? fgrid : p->local_batch_size;
-                rc = f16 ? fast_sampling_launch<FTB200_F16, false>(F, fgrid, fsmem, st) :
-                           fast_sampling_launch<FTB200_BF16, false>(F, fgrid, fsmem, st);
+                rc = f16 ? fast_sampling_launch<FTB200_F16, false>(F, S, fgrid, fsmem, both, st) :
+                           fast_sampling_launch<FTB200_BF16, false>(F, S, fgrid, fsmem, both, st);
                 if (rc != FTB200_OK) {
                     return rc;
                 }
                 note_launch(1);
             }
-            if (side != nullptr) {
-                FTB_CUDA_CHECK(cudaStreamWaitEvent(st, side->join, 0));
-                side_use.unlock();
+            if (S.limit != nullptr) {
+                return FTB200_OK;  // (the host hears of rows that are left and asks for them)
             }
             K.ticket        = K.ticket + 2;
             K.row_order     = F.redo_rows;
             K.row_count_dev = F.redo_count;
-            K.early         = side == nullptr && (topp_only || K.topp_states == nullptr);  // (one kernel in front, in this stream)
+            K.early         = 1;
             if (K.trace != nullptr) {
                 K.trace += (size_t)p->local_batch_size * 32;  // the general kernel's records follow the single-pass kernel's
             }
         }
+    }
+    if (K.row_flags == nullptr && K.row_count_dev == nullptr) {
+        FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
     }
     switch (p->dtype) {
         case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, grid, smem, st); break;
@@ -748,8 +723,8 @@ static int vp_local(const ftb200_sampling_params* p, int vocab_offset, int cap, 
             F.redo_rows  = (int*)((char*)p->workspace + 256);
             int fgrid    = sm_count() * fper;
             fgrid        = fgrid < p->local_batch_size ? fgrid : p->local_batch_size;
-            rc = f16 ? fast_sampling_launch<FTB200_F16, false, 1>(F, fgrid, fsmem, st) :
-                       fast_sampling_launch<FTB200_BF16, false, 1>(F, fgrid, fsmem, st);
+            rc = f16 ? fast_sampling_launch<FTB200_F16, false, 1>(F, StopArgs{}, fgrid, fsmem, false, st) :
+                       fast_sampling_launch<FTB200_BF16, false, 1>(F, StopArgs{}, fgrid, fsmem, false, st);
             if (rc != FTB200_OK) {
                 return rc;
             }

@@ -6,6 +6,10 @@ size_t fast_smem_for(int hash_slots, int vocab_padded, bool topp)
 {
     return fast_smem_bytes(hash_slots, vocab_padded, topp);
 }
+int fast_rows_for(const KParams& K, int* list_k, int* list_p, cudaStream_t st)
+{
+    return fast_rows_launch(K, list_k, list_p, st);
+}
 int fast_max_history()
 {
     return kFMaxHistAll;
@@ -16,6 +20,6 @@ int fast_max_words()
 }
 template int fast_sampling_occupancy<FTB200_F16, false>(size_t, int*);
 template int fast_sampling_occupancy<FTB200_BF16, false>(size_t, int*);
-template int fast_sampling_launch<FTB200_F16, false>(const KParams&, int, size_t, cudaStream_t);
-template int fast_sampling_launch<FTB200_BF16, false>(const KParams&, int, size_t, cudaStream_t);
+template int fast_sampling_launch<FTB200_F16, false>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
+template int fast_sampling_launch<FTB200_BF16, false>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
 }  // namespace ftb200

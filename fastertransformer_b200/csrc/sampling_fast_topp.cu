@@ -5,6 +5,6 @@
 namespace ftb200 {
 template int fast_sampling_occupancy<FTB200_F16, true>(size_t, int*);
 template int fast_sampling_occupancy<FTB200_BF16, true>(size_t, int*);
-template int fast_sampling_launch<FTB200_F16, true>(const KParams&, int, size_t, cudaStream_t);
-template int fast_sampling_launch<FTB200_BF16, true>(const KParams&, int, size_t, cudaStream_t);
+template int fast_sampling_launch<FTB200_F16, true>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
+template int fast_sampling_launch<FTB200_BF16, true>(const KParams&, const StopArgs&, int, size_t, bool, cudaStream_t);
 }  // namespace ftb200

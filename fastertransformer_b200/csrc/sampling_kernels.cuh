@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "device_once.cuh"
+#include "split_args.cuh"
 #include "sampling_params.cuh"
 
 namespace ftb200 {
@@ -4070,6 +4071,48 @@ static __device__ __noinline__ void row_stop_words(const KParams& P, const int* 
         }
     }
     __syncthreads();
+}
+
+// The length limit and the count of finished rows over the batch, stored for a host that polls the word: by the CTA that has seen every
+// row of the call arrive.  `left` (of any thread): rows wait for another launch, the host is told instead.  The fence that lets
+// the host find all of the step behind the word takes 1.3 us; it runs beside the loads of the flags, and a second one only
+// follows where the limit has ended a row (8 x 32000, a word each way: 19.9 us a step with one after the other, 19.0 so).
+static __device__ __noinline__ void count_finished(const KParams& P, const StopArgs& T, bool left)
+{
+    __shared__ u32 s_sum, s_changed;
+    const int      tid = threadIdx.x;
+    constexpr int  kCount = kThreads - 32;  // (the last warp sees to the fences and the word)
+    if (tid == kCount) {
+        s_sum = 0, s_changed = 0;
+    }
+    u32  mine = 0;
+    bool changed = false;
+    left         = __syncthreads_or(left);
+    if (tid == kCount) {
+        __threadfence_system();
+    }
+    for (int i = tid; !left && tid < kCount && i < P.batch_size; i += kCount) {
+        const uint8_t old = __ldcg(T.finished + i), f = (uint8_t)(old | ((u32)P.step >= T.limit[i] ? 1 : 0));
+        if (f != old) {
+            T.finished[i] = f;
+            changed       = true;
+        }
+        mine += f ? 1u : 0u;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((tid & 31) == 0 && mine != 0) {
+        atomicAdd(&s_sum, mine);
+    }
+    if (changed) {
+        s_changed = 1;
+    }
+    __syncthreads();
+    if (tid == kCount) {
+        if (s_changed != 0) {
+            __threadfence_system();
+        }
+        *(volatile u64*)T.result = left ? rows_left(T.sequence) : ((u64)T.sequence << 32) | s_sum;
+    }
 }
 
 // Shared-memory map of the general row code (the size is computed by the entry point).

@@ -51,7 +51,7 @@ int static_scratch(void** out)
 
 namespace ftb200 {
 struct StopArgs;
-int decode_step_sampling_impl(const ftb200_sampling_params* p, bool fork, const StopArgs* stop, bool* stop_done, bool left_only);
+int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, bool* stop_done, bool left_only);
 }
 
 extern "C" size_t ftb200_static_scratch_bytes(void)
@@ -88,5 +88,5 @@ extern "C" int ftb200_decode_step_sampling_static(const ftb200_sampling_params* 
     ftb200_sampling_params q = *p;
     q.workspace              = scratch;
     q.workspace_bytes        = kStaticScratchBytes;
-    return ftb200::decode_step_sampling_impl(&q, false, nullptr, nullptr, false);
+    return ftb200::decode_step_sampling_impl(&q, nullptr, nullptr, false);
 }

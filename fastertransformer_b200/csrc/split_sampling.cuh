@@ -24,7 +24,6 @@
 // above the collection areas, thousands of equal values around the k-th) go to the general row code.
 #pragma once
 #include "sampling_kernels.cuh"
-#include "split_args.cuh"
 
 namespace ftb200 {
 
@@ -1768,7 +1767,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
 // another launch (their flags are set) nothing is counted: the host is told, and sends that launch and the criteria.
 static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const StopArgs& T, int r, const int* flags, bool decided)
 {
-    __shared__ u32 s_last, s_sum;
+    __shared__ u32 s_last;
     const int      tid = threadIdx.x;
     __syncthreads();
     if (T.stop_words != nullptr && decided) {
@@ -1780,7 +1779,6 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
     if (tid == 0) {
         __threadfence();
         s_last = atomicAdd(T.arrived, 1u) == (u32)P.local_batch - 1u ? 1u : 0u;
-        s_sum  = 0;
         __threadfence();
     }
     __syncthreads();
@@ -1791,30 +1789,10 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
     for (int i = tid; i < P.local_batch; i += kThreads) {
         left |= __ldcg(flags + i) != 0;
     }
-    if (__syncthreads_or(left)) {
-        if (tid == 0) {
-            *T.arrived = 0;
-            __threadfence_system();
-            *(volatile u64*)T.result = rows_left(T.sequence);
-        }
-        return;
-    }
-    u32 mine = 0;
-    for (int i = tid; i < P.batch_size; i += kThreads) {
-        const uint8_t f = (uint8_t)(__ldcg(T.finished + i) | ((u32)P.step >= T.limit[i] ? 1 : 0));
-        T.finished[i]   = f;
-        mine += f ? 1u : 0u;
-    }
-    mine = __reduce_add_sync(0xffffffffu, mine);
-    if ((tid & 31) == 0) {
-        atomicAdd(&s_sum, mine);
-    }
-    __syncthreads();
     if (tid == 0) {
         *T.arrived = 0;
-        __threadfence_system();
-        *(volatile u64*)T.result = ((u64)T.sequence << 32) | s_sum;
     }
+    count_finished(P, T, left);
 }
 
 // ROOMY: 128 registers, two CTAs on an SM, and - when asked to - the step's stop criteria: one launch per decode step.
