@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kBeamThreads) beam_merge_kernel(const __grid_c
     __shared__ float s_old_cum[kMaxBeam], s_y[kTop];
     __shared__ int   s_newseq[kMaxBeam], s_word[kTop];
     const int        tid = threadIdx.x, b = blockIdx.x, K = P.K, twoK = 2 * K, V = P.vocab_padded;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the rows' kernel has ended and its results are visible
+    wait_for_previous();  // the rows' kernel has ended and its results are visible
 
     const int    end_id  = P.end_ids[b];
     const int    ncand   = K * twoK;

@@ -131,6 +131,13 @@ inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, siz
     cfg.numAttrs         = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// The blocks of a launch behind this kernel that allows for it may come up from here on, where they would else come up when the last
+// block of this one has gone.  (Not worth saying everywhere: beam rows and merge, 64 x 4 x 32000, took 23.9 us so and 19.9 without; the
+// general kernel, the gather tree and the log-probabilities the same either way.)
+__device__ __forceinline__ void let_next_come_up()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+}
 __device__ __forceinline__ void wait_for_previous()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -2422,7 +2422,7 @@ enum { kFHeadRowsK = 5, kFHeadRowsP = 6 };  // words of the header: rows of the 
 static __global__ void __launch_bounds__(kFListThreads) fast_rows_kernel(const __grid_constant__ KParams P, int* list_k, int* list_p)
 {
     __shared__ u32 s_k[kFListThreads / 32], s_p[kFListThreads / 32];
-    asm volatile("griddepcontrol.launch_dependents;");
+    let_next_come_up();
     wait_for_previous();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     int       n_k = 0, n_p = 0;
@@ -2469,7 +2469,7 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     else {
         __threadfence();
     }
-    asm volatile("griddepcontrol.launch_dependents;");
+    let_next_come_up();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FHdr                               s_hdr[2];
     __shared__ __align__(16) u32                  s_pre[kFPreWords];
