@@ -59,7 +59,7 @@ constexpr int kFStageBytes = 8192;  // >= (kFMaxHist + 2 * kFMaxWords + 4) * 4; 
 // Special columns that a row with this table has at most (see the plan of the table in sampling_entry.cu).
 __host__ __device__ inline int fast_max_records(int hash_slots)
 {
-    return hash_slots <= 2048 ? hash_slots / 2 : (hash_slots / 4 * 3 < 4096 ? hash_slots / 4 * 3 : 4096);
+    return hash_slots < 2048 ? hash_slots / 2 : (hash_slots / 4 * 3 < 4096 ? hash_slots / 4 * 3 : 4096);
 }
 // bytes of the per-vector mask area: one byte per aligned vector, and room for what follows the pass
 __host__ __device__ inline size_t fast_mask_bytes(int hash_slots, int vocab_padded, bool topp)
@@ -1042,15 +1042,21 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     u32* const records = ends + nbucket;
     FTB_ASSUME_SHARED(records);
     FTB_ASSUME_SHARED(ends);
-    {
-        const int per = (nbucket + kThreads - 1) / kThreads, b0 = tid * per, b1 = b0 + per < nbucket ? b0 + per : nbucket;
+    if (wid == 1) {
+        const int per = (nbucket + 31) / 32, b0 = lane * per, b1 = b0 + per < nbucket ? b0 + per : nbucket;
         u32       mine = 0;
-#pragma unroll 1
+#pragma unroll 4
         for (int b = b0; b < b1; ++b) {
             mine += ends[b];
         }
-        u32 run = f_block_excl(mine, s_wsum, nullptr);
-#pragma unroll 1
+        u32 incl = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const u32 t = __shfl_up_sync(0xffffffffu, incl, off);
+            incl += lane >= off ? t : 0u;
+        }
+        u32 run = incl - mine;
+#pragma unroll 4
         for (int b = b0; b < b1; ++b) {
             const u32 c = ends[b];
             ends[b]     = run;
@@ -1213,7 +1219,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         if (tid == 0) {
             *id_out = id;
             if (P.seq_len != nullptr && P.finished != nullptr) {
-                P.seq_len[H.r]  = P.seq_len[H.r] + 1;
+                atomicAdd(P.seq_len + H.r, 1);
                 P.finished[H.r] = id == H.end_id ? 1 : 0;
             }
         }
@@ -1660,7 +1666,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     if (tid == 0) {
         *id_out = id;
         if (P.seq_len != nullptr && P.finished != nullptr) {
-            P.seq_len[H.r]  = P.seq_len[H.r] + 1;
+            atomicAdd(P.seq_len + H.r, 1);
             P.finished[H.r] = id == H.end_id ? 1 : 0;
         }
     }
@@ -1745,18 +1751,24 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     }
     u32* const emask32 = S.emask;
     FTB_ASSUME_SHARED(emask32);
-    for (int i = tid; i < P.hash_slots; i += kThreads) {
-        hash[i] = kHashEmpty;
-        sval[i] = 0xffffffffu;  // no raw value seen: the column lies below the threshold
-    }
-    for (int i = tid; i < kFBins; i += kThreads) {
-        hist[i] = 0;
-        if (TOPP) {
-            S.lo[i] = 0;
+    {
+        // (four words a store: every array starts on a 16-byte boundary and has a multiple of four words)
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u), ones = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        static_assert(kHashEmpty == 0xffffffffu && kFBins % (4 * kThreads) == 0, "clearing by four words");
+        for (int i = tid; i < P.hash_slots / 4; i += kThreads) {
+            ((uint4*)hash)[i] = ones;
+            ((uint4*)sval)[i] = ones;  // no raw value seen: the column lies below the threshold
         }
-    }
-    for (int i = tid; i < (nfull + 3) / 4; i += kThreads) {
-        emask32[i] = 0;
+#pragma unroll
+        for (int i = 0; i < kFBins / 4; i += kThreads) {
+            ((uint4*)hist)[i + tid] = zero;
+            if (TOPP) {
+                ((uint4*)S.lo)[i + tid] = zero;
+            }
+        }
+        for (int i = tid; i < (nfull + 15) / 16; i += kThreads) {
+            ((uint4*)emask32)[i] = zero;
+        }
     }
     if (tid < 8) {
         s_lane_base[tid] = 0;
@@ -2381,36 +2393,22 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         }
         P.output_ids[(size_t)P.step * P.batch_size + col] = idc;
         if (P.seq_len != nullptr && P.finished != nullptr) {
-            P.seq_len[r]  = P.seq_len[r] + 1;
+            atomicAdd(P.seq_len + r, 1);
             P.finished[r] = idc == H.end_id ? 1 : 0;
         }
     }
     return true;
 }
 
-// The step's stop criteria for a host that waits for them, by the CTA that has just ended row r: the row's stop words, and - by the
-// CTA of the call's last row, whichever of the two kernels serves it - the length limit and the count of finished rows.  With rows on
-// the list nothing is counted: the host is told, and sends the kernel that serves them and the criteria.  A step of 1024 x 128256
-// then ends with the store of its last row's CTA, where the join of two streams, the general kernel over an empty list and the
-// criteria's kernel followed one another.
-static __device__ __noinline__ void f_stop_criteria(const KParams& P, const StopArgs& T, int r, bool done)
+// The step's end for a host that waits for it, by every CTA that has served rows (stop words are seen to row by row): the one that
+// brings the call's count of rows to its end, in whichever of the two kernels, does the length limit and the count of finished
+// rows - unless rows are on the list: then the kernel behind does, which serves them.  A step of 1024 x 128256 then ends with its last
+// row, where the join of two streams, the general kernel over an empty list and the criteria's kernel followed one another.
+static __device__ __noinline__ void f_step_end(const KParams& P, const StopArgs& T, int served)
 {
-    __shared__ u32 s_last;
-    const int      tid = threadIdx.x;
-    if (T.stop_words != nullptr && done) {
-        row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
+    if (arrived_last(T.arrived, served, P.local_batch) && __ldcg(P.redo_count) == 0) {
+        count_finished(P, T, nullptr);
     }
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(T.arrived, 1u) == (u32)P.local_batch - 1u ? 1u : 0u;
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_last == 0) {
-        return;
-    }
-    count_finished(P, T, __ldcg(P.redo_count) != 0);
 }
 
 // In front of the single-pass kernels: the header of the workspace (tickets, counters) to zero, and, where a call has rows of both
@@ -2461,9 +2459,9 @@ static __global__ void __launch_bounds__(kFListThreads) fast_rows_kernel(const _
 template<int DT, bool TOPP, int VP = 0>
 __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(const __grid_constant__ KParams P, const __grid_constant__ StopArgs T)
 {
-    // (the top-k rows' kernel comes up beside the top-p rows' one, which has seen the end of the kernel in front: it need not wait for
-    // that, but nothing that its SM has kept from before may be read)
-    if (TOPP || VP != 0) {
+    // (with both kinds of rows the top-k rows' kernel comes up beside the top-p rows' one, which has seen the end of the kernel in
+    // front: it need not wait for that, but nothing that its SM has kept from before may be read)
+    if (TOPP || VP != 0 || P.row_count_dev == nullptr) {
         wait_for_previous();
     }
     else {
@@ -2489,9 +2487,10 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     }
     const int tid = threadIdx.x;
     // thread 0 keeps the next row's ticket and number between the stages
-    __shared__ int s_rows;  // rows of this kernel
+    __shared__ int s_rows, s_served;  // rows of this kernel, and of this CTA so far
     int            nt = 0, nr = 0;
     if (tid == 0) {
+        s_served = 0;
         s_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
         nt     = (int)atomicAdd(P.ticket + (TOPP ? 3 : 0), 1u);
         if (nt < s_rows) {
@@ -2621,10 +2620,18 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
             f_compose_header(P, nt, s_rows, nr, s_pre, s_hdr[cur ^ 1]);
         }
         if (VP == 0 && T.limit != nullptr) {
-            f_stop_criteria(P, T, r, done);
+            if (T.stop_words != nullptr && done) {
+                row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
+            }
+            if (tid == 0) {
+                ++s_served;
+            }
         }
     }
-    if (!TOPP && VP == 0) {
+    if (VP == 0 && T.limit != nullptr && s_served != 0) {
+        f_step_end(P, T, s_served);
+    }
+    if (!TOPP && VP == 0 && P.row_count_dev != nullptr) {
         wait_for_previous();
     }
 }

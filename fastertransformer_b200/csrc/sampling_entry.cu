@@ -12,13 +12,13 @@ namespace ftb200 {
 template<int DT>
 int sampling_occupancy(size_t smem, int* per_sm);
 template<int DT>
-int sampling_launch(const KParams& K, int grid, size_t smem, cudaStream_t st);
+int sampling_launch(const KParams& K, const StopArgs& T, int grid, size_t smem, cudaStream_t st);
 extern template int sampling_occupancy<FTB200_F32>(size_t, int*);
 extern template int sampling_occupancy<FTB200_F16>(size_t, int*);
 extern template int sampling_occupancy<FTB200_BF16>(size_t, int*);
-extern template int sampling_launch<FTB200_F32>(const KParams&, int, size_t, cudaStream_t);
-extern template int sampling_launch<FTB200_F16>(const KParams&, int, size_t, cudaStream_t);
-extern template int sampling_launch<FTB200_BF16>(const KParams&, int, size_t, cudaStream_t);
+extern template int sampling_launch<FTB200_F32>(const KParams&, const StopArgs&, int, size_t, cudaStream_t);
+extern template int sampling_launch<FTB200_F16>(const KParams&, const StopArgs&, int, size_t, cudaStream_t);
+extern template int sampling_launch<FTB200_BF16>(const KParams&, const StopArgs&, int, size_t, cudaStream_t);
 template<int DT, bool TOPP, int VP = 0>
 int fast_sampling_occupancy(size_t smem, int* per_sm);
 template<int DT, bool TOPP, int VP = 0>
@@ -194,6 +194,8 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     else if (!A->roomy) {
         A->area = area_within(least <= kThreePerSm ? kThreePerSm : (least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem), kSpAreaMid);
     }
+    // (a row's number then need not be looked up in the order before anything of the row can be sent for)
+    A->at_once = few || rows <= resident_clusters(p->dtype, lgn, A->roomy != 0, split_smem_bytes(A->slice, A->area));
     return true;
 }
 
@@ -387,10 +389,12 @@ extern "C" int ftb200_set_row_trace(uint64_t* device_buf)
 
 // One fused step.
 namespace ftb200 {
-// left_only: the rows that the split kernel of the same step has flagged, or the single-pass kernels have listed, by the general
-// kernel.
-int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop = nullptr,
-                              bool* stop_done = nullptr, bool left_only = false);
+// What of a step's end the sampling launches see to: nothing, all of it unless rows are left (the host hears of them and sends
+// what serves them), or all of it.
+enum StepEnd : int { kStepEndNone, kStepEndRowsLeft, kStepEndAll };
+// left_only: the rows that the split kernel of the same step has flagged, by the general kernel.
+int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop = nullptr, StepEnd* end = nullptr,
+                              bool left_only = false);
 int stop_criteria_launch(const ftb200_sampling_params* p, const StopArgs& T, cudaStream_t st);
 }
 
@@ -414,18 +418,18 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     T.arrived        = s->arrived_dev;
     T.result         = (u64*)s->result_host;
     T.sequence       = ++s->sequence;
-    bool done        = false;
-    int  rc          = decode_step_sampling_impl(p, &T, &done);
-    if (rc == FTB200_OK && !done) {
+    StepEnd end      = kStepEndNone;
+    int     rc       = decode_step_sampling_impl(p, &T, &end);
+    if (rc == FTB200_OK && end == kStepEndNone) {
         rc = stop_criteria_launch(p, T, (cudaStream_t)p->stream);
     }
     *should_stop = 0;
     if (rc != FTB200_OK || T.limit == nullptr) {
         return rc;
     }
-    // Rare: rows that the tables of the first launches could not hold, then the criteria over the whole call.  The rows are found
+    // Rare: rows that the split kernel's tables could not hold, then the criteria over the whole call.  The rows are found
     // by their flags on the device, so that these launches do nothing new where none is left.
-    bool       left_sent = !done;
+    bool       left_sent = end != kStepEndRowsLeft;
     const auto send_left = [&] {
         left_sent   = true;
         const int e = decode_step_sampling_impl(p, nullptr, nullptr, true);
@@ -467,7 +471,7 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     }
 }
 
-int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, bool* stop_done, bool left_only)
+int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, StepEnd* end, bool left_only)
 {
     if (!left_only) {
         reset_launch_count();
@@ -492,6 +496,9 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
     SplitArgs A{};
     if ((g_fast_path || left_only) && choose_split(p, K, single_pass, &A)) {
         A.redo_flags      = (int*)((char*)p->workspace + 256);
+        if (A.at_once) {
+            K.row_order = nullptr;
+        }
         const auto launch = [&](const SplitArgs& args) {
             switch (p->dtype) {
                 case FTB200_F32: return split_sampling_launch<FTB200_F32>(K, args, st);
@@ -502,8 +509,8 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
         if (!left_only) {
             SplitArgs F = A;
             if (A.criteria && stop != nullptr && (stop->limit != nullptr || stop->stop_words != nullptr)) {
-                F.stop     = *stop;
-                *stop_done = true;
+                F.stop = *stop;
+                *end   = kStepEndRowsLeft;
             }
             rc = launch(F);
             if (rc != FTB200_OK) {
@@ -517,7 +524,7 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
         // Areas below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row) leave the flat
         // rows' wide nuclei: those go over eight CTAs with areas as large as shared memory allows.  Where these are below half
         // a slice too (above 163000 columns) the general kernel's many CTAs serve the several rows left sooner.
-        const bool words = !left_only && stop_done != nullptr && *stop_done;  // (no limit: who serves a row sees to its stop words)
+        const bool words = !left_only && end != nullptr && *end != kStepEndNone;  // (no limit: who serves a row sees to its stop words)
         SplitArgs  B     = A;
         if (words) {
             B.stop = *stop;
@@ -535,7 +542,7 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
             K.stop_words = stop->stop_words, K.stop_words_len = stop->stop_words_len, K.stop_finished = stop->finished;
         }
     }
-    const bool list_left = left_only && K.row_flags == nullptr;  // (the single-pass kernels of this step have put rows on their list)
+    StopArgs S{};
     if (single_pass && K.row_flags == nullptr) {
         const size_t fsmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, false);
         const size_t psmem = fast_smem_for(K.hash_slots, p->vocab_size_padded, true);
@@ -554,11 +561,10 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
             KParams F    = K;
             F.redo_count = K.ticket + 1;
             F.redo_rows  = (int*)((char*)p->workspace + 256);
-            StopArgs S{};
-            if (!list_left && stop != nullptr && stop->limit != nullptr) {
-                S          = *stop;
-                S.arrived  = K.ticket + 4;
-                *stop_done = true;
+            if (stop != nullptr && stop->limit != nullptr) {
+                S         = *stop;
+                S.arrived = K.ticket + 4;
+                *end      = kStepEndAll;
             }
             // The rows of the top-p layer have a kernel of their own (it wants more registers than the top-k rows'
             // kernel can spare); the two run side by side.
@@ -566,14 +572,12 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
             const bool both      = K.topp_states != nullptr && K.topk_states != nullptr;
             int* const list_k    = (int*)K.scratch;  // (the general kernel takes the scratch area once these have ended)
             int* const list_p    = list_k + p->local_batch_size;
-            if (!list_left) {
-                rc = fast_rows_for(F, both ? list_k : nullptr, list_p, st);
-                if (rc != FTB200_OK) {
-                    return rc;
-                }
-                note_launch(1);
+            rc                   = fast_rows_for(F, both ? list_k : nullptr, list_p, st);
+            if (rc != FTB200_OK) {
+                return rc;
             }
-            if (K.topp_states != nullptr && !list_left) {
+            note_launch(1);
+            if (K.topp_states != nullptr) {
                 if (both) {
                     F.row_order = list_p, F.row_count_dev = K.ticket + 6;
                 }
@@ -586,21 +590,22 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
                 }
                 note_launch(1);
             }
-            if (!topp_only && !list_left) {
+            if (!topp_only) {
                 if (both) {
                     F.row_order = list_k, F.row_count_dev = K.ticket + 5;
                 }
                 int fgrid = sm_count() * fper;
                 fgrid     = fgrid < p->local_batch_size ? fgrid : p->local_batch_size;
-                rc = f16 ? fast_sampling_launch<FTB200_F16, false>(F, S, fgrid, fsmem, both, st) :
-                           fast_sampling_launch<FTB200_BF16, false>(F, S, fgrid, fsmem, both, st);
+                rc = f16 ? fast_sampling_launch<FTB200_F16, false>(F, S, fgrid, fsmem, true, st) :
+                           fast_sampling_launch<FTB200_BF16, false>(F, S, fgrid, fsmem, true, st);
                 if (rc != FTB200_OK) {
                     return rc;
                 }
                 note_launch(1);
             }
             if (S.limit != nullptr) {
-                return FTB200_OK;  // (the host hears of rows that are left and asks for them)
+                S.arrived    = K.ticket + 7;
+                K.stop_words = S.stop_words, K.stop_words_len = S.stop_words_len, K.stop_finished = S.finished;
             }
             K.ticket        = K.ticket + 2;
             K.row_order     = F.redo_rows;
@@ -615,9 +620,9 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
         FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
     }
     switch (p->dtype) {
-        case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, grid, smem, st); break;
-        case FTB200_F16: rc = sampling_launch<FTB200_F16>(K, grid, smem, st); break;
-        default: rc = sampling_launch<FTB200_BF16>(K, grid, smem, st); break;
+        case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, S, grid, smem, st); break;
+        case FTB200_F16: rc = sampling_launch<FTB200_F16>(K, S, grid, smem, st); break;
+        default: rc = sampling_launch<FTB200_BF16>(K, S, grid, smem, st); break;
     }
     if (rc == FTB200_OK) {
         note_launch(1);
@@ -735,9 +740,9 @@ static int vp_local(const ftb200_sampling_params* p, int vocab_offset, int cap, 
         }
     }
     switch (p->dtype) {
-        case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, grid, smem, st); break;
-        case FTB200_F16: rc = sampling_launch<FTB200_F16>(K, grid, smem, st); break;
-        default: rc = sampling_launch<FTB200_BF16>(K, grid, smem, st); break;
+        case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, StopArgs{}, grid, smem, st); break;
+        case FTB200_F16: rc = sampling_launch<FTB200_F16>(K, StopArgs{}, grid, smem, st); break;
+        default: rc = sampling_launch<FTB200_BF16>(K, StopArgs{}, grid, smem, st); break;
     }
     if (rc == FTB200_OK) {
         note_launch(1);

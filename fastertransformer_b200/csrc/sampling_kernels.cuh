@@ -1521,7 +1521,7 @@ __device__ __forceinline__ void write_lengths(const KParams& P, const RowOut& O,
 {
     // rows that were already finished never get here (sampling_topk_kernels.cu:307-310)
     if (P.seq_len != nullptr && P.finished != nullptr) {
-        P.seq_len[O.r]  = P.seq_len[O.r] + 1;
+        atomicAdd(P.seq_len + O.r, 1);  // (nobody waits for what was there)
         P.finished[O.r] = id == O.end_id ? 1 : 0;
     }
 }
@@ -4073,26 +4073,49 @@ static __device__ __noinline__ void row_stop_words(const KParams& P, const int* 
     __syncthreads();
 }
 
+// Whether the `n` rows that this CTA has served bring the count of arrived ones to `all` (called by all threads, once every result has
+// been written by them).
+static __device__ bool arrived_last(u32* arrived, int n, int all)
+{
+    __shared__ u32 s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(arrived, (u32)n) + (u32)n == (u32)all ? 1u : 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
 // The length limit and the count of finished rows over the batch, stored for a host that polls the word: by the CTA that has seen every
-// row of the call arrive.  `left` (of any thread): rows wait for another launch, the host is told instead.  The fence that lets
+// row of the call arrive.  `flags` [local_batch] or null: where one is set, rows wait for another launch, and the
+// host is told instead.  The fence that lets
 // the host find all of the step behind the word takes 1.3 us; it runs beside the loads of the flags, and a second one only
 // follows where the limit has ended a row (8 x 32000, a word each way: 19.9 us a step with one after the other, 19.0 so).
-static __device__ __noinline__ void count_finished(const KParams& P, const StopArgs& T, bool left)
+static __device__ __noinline__ void count_finished(const KParams& P, const StopArgs& T, const int* flags)
 {
     __shared__ u32 s_sum, s_changed;
     const int      tid = threadIdx.x;
     constexpr int  kCount = kThreads - 32;  // (the last warp sees to the fences and the word)
+    // a thread's first row: everything on its way at once
+    const bool    mine_one = tid < kCount && tid < P.batch_size;
+    const uint8_t old_one  = mine_one ? __ldcg(T.finished + tid) : (uint8_t)0;
+    const u32     lim_one  = mine_one ? T.limit[tid] : 0u;
+    bool          left     = false;
+    for (int i = tid; flags != nullptr && i < P.local_batch; i += kThreads) {
+        left |= __ldcg(flags + i) != 0;
+    }
     if (tid == kCount) {
         s_sum = 0, s_changed = 0;
+        __threadfence_system();
     }
     u32  mine = 0;
     bool changed = false;
     left         = __syncthreads_or(left);
-    if (tid == kCount) {
-        __threadfence_system();
-    }
     for (int i = tid; !left && tid < kCount && i < P.batch_size; i += kCount) {
-        const uint8_t old = __ldcg(T.finished + i), f = (uint8_t)(old | ((u32)P.step >= T.limit[i] ? 1 : 0));
+        const uint8_t old = i == tid ? old_one : __ldcg(T.finished + i);
+        const uint8_t f   = (uint8_t)(old | ((u32)P.step >= (i == tid ? lim_one : T.limit[i]) ? 1 : 0));
         if (f != old) {
             T.finished[i] = f;
             changed       = true;
@@ -4130,7 +4153,7 @@ __device__ __forceinline__ void map_general_smem(const KParams& P, Smem& S, unsi
 }
 
 template<int DT>
-__global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __grid_constant__ KParams P)
+__global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __grid_constant__ KParams P, const __grid_constant__ StopArgs T)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int                                s_row;
@@ -4144,6 +4167,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
     u64* gscratch = P.scratch + (size_t)blockIdx.x * P.scratch_stride;
     // rows to serve: the whole local batch, or the list the single-pass kernel left behind
     const int n_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
+    int       served = 0;
     for (int next = blockIdx.x;; next += gridDim.x) {
         __syncthreads();
         int t;
@@ -4178,6 +4202,11 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
         if (rec != nullptr && threadIdx.x == 0) {
             rec[3] = global_timer_ns();
         }
+        ++served;
+    }
+    // (a host waits, and the single-pass kernels have left rows: the step ends here)
+    if (T.limit != nullptr && served != 0 && arrived_last(T.arrived, served, n_rows)) {
+        count_finished(P, T, nullptr);
     }
 }
 
@@ -4644,14 +4673,14 @@ int sampling_occupancy(size_t smem, int* per_sm)
 }
 
 template<int DT>
-int sampling_launch(const KParams& K, int grid, size_t smem, cudaStream_t st)
+int sampling_launch(const KParams& K, const StopArgs& T, int grid, size_t smem, cudaStream_t st)
 {
     if (K.row_flags != nullptr || K.early) {
         // behind the split kernel or one single-pass kernel: comes up while that one drains (normally it finds no row)
-        FTB_CUDA_CHECK(launch_early(decode_sampling_kernel<DT>, dim3((unsigned)grid), dim3(kThreads), smem, st, K));
+        FTB_CUDA_CHECK(launch_early(decode_sampling_kernel<DT>, dim3((unsigned)grid), dim3(kThreads), smem, st, K, T));
         return FTB200_OK;
     }
-    decode_sampling_kernel<DT><<<grid, kThreads, smem, st>>>(K);
+    decode_sampling_kernel<DT><<<grid, kThreads, smem, st>>>(K, T);
     FTB_CUDA_CHECK(cudaGetLastError());
     return FTB200_OK;
 }

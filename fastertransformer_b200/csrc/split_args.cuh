@@ -34,6 +34,7 @@ struct SplitArgs {
     int  area;        // keys of the collection area
     int  roomy;       // the form with 128 registers
     int  criteria;    // whether the launch may do the step's stop criteria (roomy form)
+    int  at_once;     // all clusters are resident together: the rows' order does not matter
     int* redo_flags;  // [local_batch]: 1 when the row is left to another launch
     StopArgs stop;    // (roomy form; without a limit the rows' stop words alone)
     int  clusters;    // 0: one per row; else so many, which look for rows with redo_flags set and serve those (roomy form)

@@ -162,7 +162,8 @@ struct SpShared {
     u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
     u32   p_sel, j_sel;    // crossing: probability (bits), position in the sorted order
     u32   larger;          // columns of a larger probability than the crossing's
-    u32   bad_order;
+    u32    bad_order;
+    u32    state[6];       // counter and words of the row's generator after its draw (nothing else of it moves)
     alignas(16) float agg[(kSpMaxN * kSpAreaMax) / 256];
 };
 
@@ -1274,7 +1275,12 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     }
     float best = sp_load_slice<DT>(P, X0, rowp, y, rank, lgvt, nchunk);
     if (tid == 0) {
-        s_u = curand_uniform(&draw);
+        s_u        = curand_uniform(&draw);
+        X.state[0] = draw.d;  // (stored with the result)
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            X.state[1 + i] = draw.v[i];
+        }
     }
     trace_mark(O.trace, 0);
     cluster_wait();
@@ -1901,8 +1907,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
 // another launch (their flags are set) nothing is counted: the host is told, and sends that launch and the criteria.
 static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const StopArgs& T, int r, const int* flags, bool decided)
 {
-    __shared__ u32 s_last;
-    const int      tid = threadIdx.x;
+    const int tid = threadIdx.x;
     __syncthreads();
     if (T.stop_words != nullptr && decided) {
         row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
@@ -1910,23 +1915,13 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
     if (T.limit == nullptr) {
         return;
     }
-    if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(T.arrived, 1u) == (u32)P.local_batch - 1u ? 1u : 0u;
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_last == 0) {
+    if (!arrived_last(T.arrived, 1, P.local_batch)) {
         return;
-    }
-    bool left = false;
-    for (int i = tid; i < P.local_batch; i += kThreads) {
-        left |= __ldcg(flags + i) != 0;
     }
     if (tid == 0) {
         *T.arrived = 0;
     }
-    count_finished(P, T, left);
+    count_finished(P, T, flags);
 }
 
 // ROOMY: 128 registers, two CTAs on an SM, and - when asked to - the step's stop criteria: one launch per decode step.
@@ -2016,11 +2011,16 @@ __global__ void __launch_bounds__(kThreads, ROOMY ? 2 : 3) split_sampling_kernel
                 if (mode == 1 && fin) {
                     *s_O.id_out = s_O.end_id;  // no draw, length unchanged (sampling_topk_kernels.cu:249-252)
                 }
-                else if (mode != 0) {
-                    const float u = draw_uniform(mode == 1 ? P.topk_states : P.topp_states, r);
-                    if (fin) {
-                        finished_topp_row<DT>(P, s_O, u, want_lp);
+                else if (mode != 0 && !fin) {
+                    curandState_t& st = (mode == 1 ? P.topk_states : P.topp_states)[r];
+                    st.d              = s_X.state[0];
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) {
+                        st.v[i] = s_X.state[1 + i];
                     }
+                }
+                else if (mode != 0) {
+                    finished_topp_row<DT>(P, s_O, draw_uniform(P.topp_states, r), want_lp);
                 }
                 topp_decay_row(P, r, *s_O.id_out);
             }
