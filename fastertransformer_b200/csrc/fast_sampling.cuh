@@ -2102,8 +2102,8 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         return true;
     }
     if constexpr (TOPP) {
-        if (n_ord < 1 || G.head != 0) {
-            return false;  // (the second pass wants the row on a 16-byte boundary)
+        if (n_ord < 1) {
+            return false;
         }
         FTopp T;
         T.thr_key = thr_key, T.relmax = s_relmax, T.n_ord = n_ord, T.n_sp = n_sp;
@@ -2546,7 +2546,8 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
             //  under the threshold candidates: those rows go to the general kernel)
             const bool lowers = !P.apply_rep || (P.penalty_type == FTB200_PENALTY_MULTIPLICATIVE ? H.theta >= 1.0f :
                                                  P.penalty_type == FTB200_PENALTY_ADDITIVE ? H.theta >= 0.0f : true);
-            const bool ok = lowers && G.nfull >= 2048 && G.nfull <= 65535 && H.inv_t > 0.0f && H.inv_t < 3.0e38f
+            // (the second pass of a top-p row wants it on a 16-byte boundary)
+            const bool ok = lowers && (!TOPP || G.head == 0) && G.nfull >= 2048 && G.nfull <= 65535 && H.inv_t > 0.0f && H.inv_t < 3.0e38f
                             && (P.apply_rep ? P.step : 0) <= kFMaxHistAll
                             && (P.bad_words != nullptr ? P.bad_words_len : 0) <= kFMaxWords;
             if (ok) {

@@ -130,7 +130,16 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
         return false;  // (the denominator's chains are then not 1024)
     }
     const bool topk = K.topk_states != nullptr, topp = K.topp_states != nullptr, mixed = topk && topp;
-    if (single_pass && (double)rows * vocab > (mixed ? 16.5e6 : (topp ? 9e6 : (K.max_top_k > 256 ? 4.2e6 : 2.1e6)))) {
+    // Nucleus rows off a 16-byte boundary (an odd vocabulary) are none of the single-pass kernels': they would all end in the general
+    // one.  us a step, general kernel / split form, bf16: nucleus rows alone, 300 x 17001 205 / 89, 1000 x 30001 613 / 290, 1000 x 50257
+    // 866 / 479, 150 x 128257 564 / 192, 500 x 128257 1183 / 616, 200 x 250001 1216 / 774: always the split form; both kinds, 1000 x 17001
+    // 218 / 160, 400 x 50257 316 / 137, 800 x 50257 352 / 309, 1000 x 50257 367 / 380, 150 x 128257 503 / 122, 300 x 128257 555 / 284, 1000 x
+    // 128257 665 / 888.
+    const bool off = topp && (((size_t)p->logits | (size_t)p->vocab_size_padded * 2) & 15) != 0;
+    if (single_pass && off && mixed && (double)rows * vocab > 48e6) {
+        return false;
+    }
+    if (single_pass && !off && (double)rows * vocab > (mixed ? 16.5e6 : (topp ? 9e6 : (K.max_top_k > 256 ? 4.2e6 : 2.1e6)))) {
         return false;
     }
     // CTAs per row: eight while they are all resident (and for rows so long that a slice would not leave room for
@@ -152,7 +161,7 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     }
     A->lgn             = lgn;
     const size_t least = split_smem_bytes(A->slice, kSpAreaMin);
-    if (single_pass && topp && !topk) {
+    if (single_pass && !off && topp && !topk) {
         const int at_once = resident_clusters(p->dtype, lgn, false, lgn == 1 ? least : kTwoPerSm);
         const int most    = lgn == 1 ? at_once : (lgn == 2 ? at_once * 4 / 3 : (int)(2.0 * at_once * (vocab > 110000 ? vocab / 110000.0 : 1.0)));
         if (rows > most) {

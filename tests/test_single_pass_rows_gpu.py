@@ -78,3 +78,12 @@ def test_nucleus_rows(dtype, V, B, history, sigma, shift, temperature, cuda_devi
 def test_rows_of_both_layers(dtype, V, B, penalty, waits, cuda_device):
     kw = dict(kinds="both", history=30, sigma=2.0, penalty=penalty, waits=waits)
     same(steps(True, dtype, V, B, cuda_device, **kw), steps(False, dtype, V, B, cuda_device, **kw))
+
+
+@pytest.mark.parametrize("dtype,V,B,kinds", [
+    (BF16, 17001, 600, "topp"), (F16, 30003, 350, "topp"), (BF16, 128257, 75, "topp"),
+    (F16, 17001, 1000, "both"), (BF16, 50257, 954, "both"), (BF16, 50257, 956, "both")])  # (either side of the line for both kinds)
+@pytest.mark.parametrize("waits", [False, True])
+def test_rows_off_a_16_byte_boundary(dtype, V, B, kinds, waits, cuda_device):
+    kw = dict(kinds=kinds, history=30, sigma=2.5, waits=waits, n=1 if B * V > 40e6 else 2)
+    same(steps(True, dtype, V, B, cuda_device, **kw), steps(False, dtype, V, B, cuda_device, **kw))
