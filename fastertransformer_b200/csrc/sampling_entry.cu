@@ -215,7 +215,7 @@ static bool wide_areas(int vocab, SplitArgs* A)
     A->roomy = 1;
     A->slice = ((vocab + 1023) / 1024) << 7;
     A->slice = A->slice < kSpMinSlice ? kSpMinSlice : A->slice;
-    A->area  = kSpAreaMax;
+    A->area  = kSpAreaWide;
     while (A->area > kSpAreaMin && split_smem_bytes(A->slice, A->area) > kSpMaxSmem) {
         A->area -= 1024;
     }
@@ -530,15 +530,17 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
                 return FTB200_OK;  // (the host hears of rows that are left and asks for them)
             }
         }
-        // Areas below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row) leave the flat
-        // rows' wide nuclei: those go over eight CTAs with areas as large as shared memory allows.  Where these are below half
-        // a slice too (above 163000 columns) the general kernel's many CTAs serve the several rows left sooner.
+        // Flat rows' wide nuclei that the areas do not hold go over eight CTAs with areas as large as shared memory allows: where the host
+        // has heard of rows left and the areas are larger than the first launch's, and behind every step that does not wait where those
+        // are below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row).  Where the large ones are below
+        // half a slice too (above 245000 columns) the general kernel's many CTAs serve the several rows left sooner.
         const bool words = !left_only && end != nullptr && *end != kStepEndNone;  // (no limit: who serves a row sees to its stop words)
         SplitArgs  B     = A;
         if (words) {
             B.stop = *stop;
         }
-        if (wide_areas(p->vocab_size, &B) && K.topp_states != nullptr && A.area < A.slice / 2 && B.area >= B.slice / 2) {
+        if (wide_areas(p->vocab_size, &B) && K.topp_states != nullptr && (left_only ? A.area << A.lgn < B.area << B.lgn : A.area < A.slice / 2)
+            && B.area >= B.slice / 2) {
             B.clusters = sm_count() / kSpMaxN < p->local_batch_size ? sm_count() / kSpMaxN : p->local_batch_size;
             rc         = launch(B);
             if (rc != FTB200_OK) {

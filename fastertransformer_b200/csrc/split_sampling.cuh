@@ -164,7 +164,7 @@ struct SpShared {
     u32   larger;          // columns of a larger probability than the crossing's
     u32    bad_order;
     u32    state[6];       // counter and words of the row's generator after its draw (nothing else of it moves)
-    alignas(16) float agg[(kSpMaxN * kSpAreaMax) / 256];
+    alignas(16) float agg[(kSpMaxN * kSpAreaWide) / 256];
 };
 
 // Bias of a 32-bit word of logits in the logits type's arithmetic (half: two rounded sums; fp32: one).  bf16 sums stay
@@ -805,7 +805,7 @@ static __device__ __noinline__ bool sp_sort_area(float* a, u32* sub, const u32* 
     FTB_ASSUME_SHARED(excl);
     const int  tid = threadIdx.x, lane = tid & 31;
     u32* const list = hist + kSpBins - kSpLists;
-    if (n <= cap / 2) {
+    if (n <= cap / 2 && n <= 25 * kSpLists) {
         return sp_sort_keys(a, a + cap / 2, sub, hist, excl, list, start, n, maxv, ties);  // (the maps fit: n / 16 words)
     }
     // (a quarter of a word for the counters, a sixteenth for the maps, one for the key)
@@ -1928,11 +1928,11 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
 // Taken while all rows are resident at once, and beyond that where shared memory holds no third CTA on an SM; elsewhere 80
 // registers and three CTAs on an SM are worth more (choose_split).  Either form flags the rows that its tables cannot hold for a second launch: decode_sampling_kernel, or - where the areas of the first
 // launch are small - a few clusters of the roomy form with all the shared memory there is (A.clusters), because a nucleus of half
-// of 127000 columns takes 0.2 ms here and 5 to 9 ms in the general code.  A nucleus beyond those areas too (64 % of
-// 127000 columns; above 163000 columns there is no such launch, 49000 columns end it) still ends in the general code, so a batch of
-// flat rows takes what its widest nucleus takes.  Mean and slowest of 30 steps of fresh normal logits, 800 x 126959 bf16 with
-// log-probabilities: 1.2 / 1.2 ms (sigma 2.5, p 0.95), 2.3 / 2.7 (sigma 2, p 0.95, temperature 1.2), 27 / 43 (sigma 1.5, p 0.95,
-// temperature 1.2); 60 x 200000 fp32: 0.9 / 1.8, 9.4 / 10.2 and 13.6 / 15.1 ms.
+// of 127000 columns takes 0.2 ms here and 5 to 9 ms in the general code.  Those areas hold 16384 keys a CTA, all of 128000 columns, and
+// 60 % of 200000; what is wider still ends in the general code, so a batch of such rows takes what its widest nucleus takes.  Mean of
+// steps of fresh normal logits with areas of 10240 keys / so, ms: 100 x 127000 bf16 with log-probabilities 0.29 / 0.30 (sigma 2, p
+// 0.95, temperature 1.2), 7.9 / 0.42 (sigma 1.5), 11.5 / 0.67 (sigma 0.8, p 0.98, temperature 1.1); 800 x 126959 (sigma 1.5) 14.1 /
+// 2.7; 60 x 200000 fp32 8.5 / 0.30 (sigma 2), 13.4 / 11.2 (sigma 1.5); 20 x 60000 fp32 (sigma 0.8) 1.38 / 0.15.
 //
 // The general row code is not part of this kernel.  It was, in the roomy form, for the rows it leaves; its frames brought the
 // stack to 1.7 to 1.9 KB a thread, and builds that differed in nothing but such sizes ended steps of two CTAs on an SM with an

@@ -87,3 +87,14 @@ def test_rows_of_both_layers(dtype, V, B, penalty, waits, cuda_device):
 def test_rows_off_a_16_byte_boundary(dtype, V, B, kinds, waits, cuda_device):
     kw = dict(kinds=kinds, history=30, sigma=2.5, waits=waits, n=1 if B * V > 40e6 else 2)
     same(steps(True, dtype, V, B, cuda_device, **kw), steps(False, dtype, V, B, cuda_device, **kw))
+
+
+@pytest.mark.parametrize("dtype,V,B,sigma,temperature", [
+    (BF16, 126959, 60, 1.5, 1.2),           # nuclei of most columns: beyond the first launch's areas, within the second's
+    (torch.float32, 128256, 12, 0.6, 1.0),  # an owner's 14000 keys, stretch by stretch
+    (F16, 131072, 20, 0.5, 1.0),            # as many columns as the areas hold, and rows that go to the general kernel
+    (BF16, 240000, 24, 1.2, 1.0)])          # areas of half a slice
+def test_flat_rows(dtype, V, B, sigma, temperature, cuda_device):
+    """A step that waits and whose widest nuclei the first launch leaves."""
+    kw = dict(kinds="topp", history=20, sigma=sigma, temperature=temperature, waits=True)
+    same(steps(True, dtype, V, B, cuda_device, **kw), steps(False, dtype, V, B, cuda_device, **kw))
