@@ -157,14 +157,18 @@ struct SpShared {
     float wsum[32];        // warp sums of the soft-max denominator, written by all CTAs
     u32   max_key;         // of the row's largest value
     u32   first_max;       // smallest column that holds the maximum
-    u64   best[kSpMaxN * kWarps];  // arg-max rows, a warp each: key of its largest value << 32 | the largest tie key of its columns
     u32   n_cls;           // columns of the crossing class
     u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
     u32   p_sel, j_sel;    // crossing: probability (bits), position in the sorted order
     u32   larger;          // columns of a larger probability than the crossing's
     u32    bad_order;
     u32    state[6];       // counter and words of the row's generator after its draw (nothing else of it moves)
-    alignas(16) float agg[(kSpMaxN * kSpAreaWide) / 256];
+    // (static and dynamic shared memory have to leave room for two CTAs with kTwoPerSm, which is asked for in whole kilobytes: at most 5120
+    // bytes of static memory)
+    union {
+        u64               best[kSpMaxN * kWarps];  // arg-max rows, a warp each: key of its largest value << 32 | the largest tie key of its columns
+        alignas(16) float agg[(kSpMaxN * kSpAreaWide) / 256];  // nuclei: sums of 256 probabilities
+    };
 };
 
 // Bias of a 32-bit word of logits in the logits type's arithmetic (half: two rounded sums; fp32: one).  bf16 sums stay
