@@ -451,6 +451,7 @@ struct FHdr {
     int    r, mode, fin, end_id, k;
     float  top_p, u, inv_t, theta;
     __half inv_t_h;
+    u64*   trace;  // the row's record of the diagnostic timeline, or null
 };
 // landing zone of the next row's arguments (32-bit words; the two generator states sit on 16-byte boundaries)
 constexpr int kFPreWords = 48;
@@ -710,10 +711,10 @@ __device__ __forceinline__ u32 f_record(int slot, int v)
 // Special columns: rare for a thread, but some lane of a warp has one in nearly every pair of chunks.  The warp's exponentials go
 // through 1 KB of shared memory then, and lanes with a record each put the special ones in their places: 2 + 2 wide accesses
 // instead of a divergent table walk that picks one of sixteen registers and puts it back with selects (a third of the
-// instructions of the pass).  Rows of 128256 bf16
-// with 550 special columns, wide nuclei: 55 us with the walk, 38 so; 51200 half, 150 special columns: 19.7 and 12.4.
+// instructions of the pass).  Rows of 116848
+// bf16 with 640 special columns, two on an SM: 32.9 us with the walk, 18.6 so; 51200 half, 150 special columns: 19.7 and 7.9.
 enum { kCountNone, kCountPositive, kCountAny };  // (positive: threshold and cut both at or above +0)
-template<int DT, bool TEMP, int COUNT>
+template<int DT, int COUNT>
 __device__ __noinline__ void f_pass2(const FPass2 A)
 {
     const int    tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -766,7 +767,7 @@ __device__ __noinline__ void f_pass2(const FPass2 A)
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             // a column at or below -MAX adds exactly zero, as in the reference's loop
-            const float y = f_value<DT>((e & 1) ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu, TEMP, inv_t, inv_t_h);
+            const float y = f_value<DT>((e & 1) ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu, true, inv_t, inv_t_h);
             x[e]          = f_round_T<DT>(__expf(y - maxv));
         }
         if (end != at) {
@@ -801,7 +802,7 @@ __device__ __noinline__ void f_pass2(const FPass2 A)
             for (int e = 0; e < 4 && v0 + e < A.vocab; ++e) {
                 const u32 r    = (u32)__ldg(row16 + v0 + e);
                 const int slot = f_hash_find_saddr(A.hash, A.shift, A.mask, v0 + e);
-                const float yy = slot >= 0 ? __uint_as_float(lds_u32(A.value + 4u * (u32)slot)) : f_value<DT>(r, TEMP, inv_t, inv_t_h);
+                const float yy = slot >= 0 ? __uint_as_float(lds_u32(A.value + 4u * (u32)slot)) : f_value<DT>(r, true, inv_t, inv_t_h);
                 const float ex = f_round_T<DT>(__expf(yy - maxv));
                 a0 += e == 0 ? ex : 0.0f, a1 += e == 1 ? ex : 0.0f, a2 += e == 2 ? ex : 0.0f, a3 += e == 3 ? ex : 0.0f;
                 if (COUNT) {
@@ -885,7 +886,7 @@ __device__ __forceinline__ void f_load8(const FRuns& R, int c, float (*x)[8])
 }
 // Aggregate of every 256-value chunk in cub::BlockScan's raking order (32 segments of 8, Kogge-Stone across the segment totals);
 // the chunks are independent of the running prefix.  Four chunks a warp at a time.
-static __device__ __noinline__ void f_chunk_aggregates(const FRuns R)
+static __device__ __forceinline__ void f_chunk_aggregates(const FRuns R)
 {
     constexpr int U = 4;
     const int     lane = threadIdx.x & 31;
@@ -999,8 +1000,8 @@ static __device__ __noinline__ void f_sort_listed(u64* spec, int n_sp, u32* bins
 
 // Everything of a top-p row after the pass and the listed columns.  Returns true when the row is done.
 template<int DT>
-__device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, const FHdr& H, const FGeo& G, const FTopp T, u64* spec,
-                               u32* s_nspec, const u32* s_mass, float mass_tail, u32 smax_key, u64* trace)
+__device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, const FHdr& H, const FGeo& G, const FTopp& T, u64* spec,
+                               u32* s_nspec, const u32* s_mass, float mass_tail, u32 smax_key)
 {
     __shared__ float s_w[kWarps], s_den;
     __shared__ u32   s_cut, s_wsum[kWarps], s_ncls, s_fail;
@@ -1129,7 +1130,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
     }
     __syncthreads();
-    trace_mark(trace, 6);
+    trace_mark(H.trace, 6);
 
     // ---- pass 2 ----
     float* const s_vt = (float*)S.wbuf;  // [1024] per-virtual-thread sums (the ring of the pass is idle)
@@ -1142,18 +1143,19 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         A.list = (u32)__cvta_generic_to_shared(records), A.ends = (u32)__cvta_generic_to_shared(ends), A.ring = (u32)__cvta_generic_to_shared(S.emask);
         A.hlo = (u32)__cvta_generic_to_shared(hlo), A.out = (u32)__cvta_generic_to_shared(s_vt), A.buf = A.out;
         const bool positive = cut_key >= 0x8000u && thr_key > 0x8000u;
-        if (temp) {
-            positive ? f_pass2<DT, true, kCountPositive>(A) : f_pass2<DT, true, kCountAny>(A);
+        // (without a temperature the factor is one, and one multiplication a column: two more copies of the pass cost more)
+        if (cut_key >= thr_key) {
+            f_pass2<DT, kCountNone>(A);
         }
-        else if (cut_key >= thr_key) {
-            f_pass2<DT, false, kCountNone>(A);
+        else if (positive) {
+            f_pass2<DT, kCountPositive>(A);
         }
         else {
-            positive ? f_pass2<DT, false, kCountPositive>(A) : f_pass2<DT, false, kCountAny>(A);
+            f_pass2<DT, kCountAny>(A);
         }
     }
     __syncthreads();
-    trace_mark(trace, 7);
+    trace_mark(H.trace, 7);
     {
         // the reference's blockReduceSum (utils/reduce_kernel_utils.cuh:73-103) over the 1024 partial sums: a
         // butterfly inside every group of 32, then one over the 32 group results
@@ -1413,11 +1415,11 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
     }
     __syncthreads();
-    trace_mark(trace, 8);
-    if (trace != nullptr && tid == 0) {
-        trace[4 + 20] = (u64)(thr_key - cut_key);
-        trace[4 + 21] = (u64)N;
-        trace[4 + 22] = (u64)T.n_ord;
+    trace_mark(H.trace, 8);
+    if (H.trace != nullptr && tid == 0) {
+        H.trace[4 + 20] = (u64)(thr_key - cut_key);
+        H.trace[4 + 21] = (u64)N;
+        H.trace[4 + 22] = (u64)T.n_ord;
     }
     const int nch = (int)((N + 255u) / 256u);
     if (nch > 1000 || N == 0) {
@@ -1506,7 +1508,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
     }
     __syncthreads();
     const int sel = s_sel;
-    trace_mark(trace, 9);
+    trace_mark(H.trace, 9);
     if (sel < 0 || (u32)sel >= N) {
         return false;
     }
@@ -1632,7 +1634,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
     }
     __syncthreads();
-    trace_mark(trace, 10);
+    trace_mark(H.trace, 10);
     const int ncls = (int)s_ncls;
     if (ncls > kFPClsCap || J_far < 0 || J_far >= ncls) {
         return false;
@@ -1682,7 +1684,7 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
 // vocabulary: token ids become columns by subtracting P.vocab_offset, and instead of drawing the row hands every
 // column whose value reaches the shard's k-th value (whole tie class) to the exchange record, as topk_tail does.
 template<int DT, bool TOPP, int VP, class S1, class S2>
-__device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const FHdr& H, u64* trace, S1&& stage1, S2&& stage2)
+__device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const FHdr& H, S1&& stage1, S2&& stage2)
 {
     static_assert(!(TOPP && VP), "the record form serves top-k rows");
     const int id_shift = VP ? P.vocab_offset : 0;
@@ -1796,7 +1798,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     cp_async_wait_all();  // history, word list and last tokens have landed
     __syncthreads();
     stage1();
-    trace_mark(trace, 0);
+    trace_mark(H.trace, 0);
 
     // ---- threshold from the sample (warp 0) while the other warps file the special columns: token history,
     //      banned words, min-length mask (the rules of build_row; kernels/sampling_penalty_kernels.cu:385-410,
@@ -1928,7 +1930,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         }
     }
     __syncthreads();
-    trace_mark(trace, 1);
+    trace_mark(H.trace, 1);
     if (long_words || want_s > 96u || !(thr_y > neg_max) || thr_key == 0u) {
         return false;  // (uniform for the CTA)
     }
@@ -1936,9 +1938,9 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     // ---- the pass ----
     f_stream<DT, false, kFUnroll>(vp, nfull, G.head, thr_key, 0u, s_sink, &s_relmax);
     __syncthreads();
-    trace_mark(trace, 2);
-    trace_mark(trace, 3);
-    trace_mark(trace, 4);
+    trace_mark(H.trace, 2);
+    trace_mark(H.trace, 3);
+    trace_mark(H.trace, 4);
     // ---- listed columns: special ones with their final value, and the row's edges ----
     // (~key(value) << 32) | column.  Top-k rows: [kFSpecCap] where the per-vector bytes were (they are done with);
     // top-p rows: [kFPSpecCap] where the row's set-up data was (the bytes make room for the records of the second pass)
@@ -2033,7 +2035,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         }
     }
     __syncthreads();
-    trace_mark(trace, 5);
+    trace_mark(H.trace, 5);
     const int n_ord = (int)s_ncand, n_sp = (int)s_nspec;
     if (s_bad || n_ord > kFCap || n_sp > spec_cap || n_ord + n_sp < (TOPP ? 1 : k)) {
         return false;
@@ -2105,17 +2107,21 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         if (n_ord < 1) {
             return false;
         }
-        FTopp T;
-        T.thr_key = thr_key, T.relmax = s_relmax, T.n_ord = n_ord, T.n_sp = n_sp;
-        T.thr_y = thr_y, T.neg_max = neg_max;
+        __shared__ FTopp s_T;  // (read where they are used: every register is taken)
+        __shared__ FGeo  s_G;
         const float top_ord = f_value<DT>(key16_inv(thr_key + s_relmax), temp, H.inv_t, H.inv_t_h);
         const float top_sp  = s_vmaxkey != 0 ? fkey_inv(s_vmaxkey) : -INFINITY;
-        T.maxv              = fmaxf(top_ord, top_sp);
+        if (tid == 0) {
+            s_T.thr_key = thr_key, s_T.relmax = s_relmax, s_T.n_ord = n_ord, s_T.n_sp = n_sp;
+            s_T.thr_y = thr_y, s_T.neg_max = neg_max, s_T.maxv = fmaxf(top_ord, top_sp);
+            s_G       = G;
+        }
         float mass_tail     = 0.0f;
         for (int i = 0; i < kWarps; ++i) {
             mass_tail += s_mtail[i];
         }
-        return fast_topp_tail<DT>(P, S, H, G, T, spec, &s_nspec, s_mass, mass_tail, s_smaxkey, trace);
+        __syncthreads();
+        return fast_topp_tail<DT>(P, S, H, s_G, s_T, spec, &s_nspec, s_mass, mass_tail, s_smaxkey);
     }
 
     // ---- the draw (warp 0): runs of equal values from the top, then the reference's sequential sum and walk ----
@@ -2203,7 +2209,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         }
         const int nruns = nA + n_sp;
         __syncwarp();
-        trace_mark(trace, 7);
+        trace_mark(H.trace, 7);
         if (!over) {
             // the first k entries of the sorted sequence, as exponentials against the largest value: every run
             // writes its copies (the sequence the reference's thread 0 walks, sampling_topk_kernels.cu:276-287)
@@ -2233,7 +2239,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
                 flat[k + lane] = 0.0f;
             }
             __syncwarp();
-            trace_mark(trace, 8);
+            trace_mark(H.trace, 8);
             // Dependent adds in the reference's order, by one lane: sixteen terms a round, eight on their way while eight are added.
             // The walk leaves its running values where the terms were; they only fall, so the first one that ends the
             // reference's loop lies in the last round and is found by the warp, as is the run that it belongs to (1024 x
@@ -2307,7 +2313,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         }
     }
     __syncthreads();
-    trace_mark(trace, 9);
+    trace_mark(H.trace, 9);
     if (s_nruns < 0) {
         return false;
     }
@@ -2360,7 +2366,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         }
     }
     __syncthreads();
-    trace_mark(trace, 10);
+    trace_mark(H.trace, 10);
     const int m = (int)s_ncls;
     // number of candidates above the class = position of its first member in the sorted sequence
     int lo_cnt = 0;
@@ -2456,6 +2462,9 @@ static __global__ void __launch_bounds__(kFListThreads) fast_rows_kernel(const _
 // The two kernels of a step with both kinds of rows follow each other in one stream and run side by side: the top-p rows' kernel lets
 // the other one come up at once, and that one waits for it at its end, so that what follows in the stream finds both done.  (A second
 // stream, forked and joined with events, cost four calls of the host in front of the kernels and a wait behind them.)
+// Spilled registers cost the top-p rows' kernel more than anything else: two CTAs with 100 KB of shared memory each leave L1 too little for
+// 200 bytes a thread, and every access goes to L2.  With its scalars in shared memory and three copies of the second pass it spills
+// 12 to 20 bytes (196 before): 256 x 51200 half 61.0 -> 52.8 us a step, 1024 x 128256 bf16 of both kinds 174.9 -> 163.0.
 template<int DT, bool TOPP, int VP = 0>
 __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(const __grid_constant__ KParams P, const __grid_constant__ StopArgs T)
 {
@@ -2507,8 +2516,9 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
             break;
         }
         const int  r   = H.r;
-        u64* const rec = P.trace != nullptr ? P.trace + ((size_t)H.t + (TOPP ? 2 * (size_t)P.local_batch : 0)) * kTraceWords : nullptr;
         if (tid == 0) {
+            u64* const rec = P.trace != nullptr ? P.trace + ((size_t)H.t + (TOPP ? 2 * (size_t)P.local_batch : 0)) * kTraceWords : nullptr;
+            s_hdr[cur].trace = rec;
             if (rec != nullptr) {
                 rec[0] = (u64)r, rec[1] = (u64)blockIdx.x, rec[2] = global_timer_ns();
                 rec[4 + 25] = (u64)clock64();
@@ -2551,7 +2561,7 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
                             && (P.apply_rep ? P.step : 0) <= kFMaxHistAll
                             && (P.bad_words != nullptr ? P.bad_words_len : 0) <= kFMaxWords;
             if (ok) {
-                done = fast_row<DT, TOPP, VP>(P, S, H, rec, stage1, stage2);
+                done = fast_row<DT, TOPP, VP>(P, S, H, stage1, stage2);
                 if (VP == 0 && done && tid == 0) {
                     curandState_t* states = H.mode == 1 ? P.topk_states : P.topp_states;
                     curandState_t  st     = states[r];
@@ -2596,10 +2606,10 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
         }
         __syncthreads();
         if (tid == 0) {
-            if (rec != nullptr) {
-                rec[3] = global_timer_ns();
-                rec[4 + 26] = (u64)clock64();
-                rec[4 + 27] = done ? 1 : 0;
+            if (H.trace != nullptr) {
+                H.trace[3] = global_timer_ns();
+                H.trace[4 + 26] = (u64)clock64();
+                H.trace[4 + 27] = done ? 1 : 0;
             }
             if (!done) {
                 P.redo_rows[atomicAdd(P.redo_count, 1u)] = r;
