@@ -1589,11 +1589,12 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
         else {
             // below the threshold: the ordinary columns of the band come from the row once more, and only as far as the J-th of
-            // the class - from whichever end it is nearer to, so a quarter of the row on average.  First the row's last columns.
+            // the class - from whichever end it is nearer to, so a quarter of the row on average.  First the row's last columns (those
+            // at or above the threshold are listed columns).
             const int tail0 = nfull * 8;
             if (tail0 + tid < P.vocab && tid < 8 && hash_lookup_raw(S.hash, P.hash_shift, P.hash_slots - 1, tail0 + tid) == 0) {
                 const u32 key = key16((u32)__ldg((const unsigned short*)G.rowp + tail0 + tid));
-                if (key >= k_lo && key <= k_hi) {
+                if (key >= k_lo && key <= k_hi && key < thr_key) {
                     const u32 pos = atomicAdd(&s_ncls, 1u);
                     if (pos < (u32)kFPClsCap) {
                         cls[pos] = (u32)(tail0 + tid);
@@ -2030,7 +2031,12 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
         for (int i = tid; i < nedge; i += kThreads) {
             const int v = i < G.head ? i : tail0 + (i - G.head);
             if (v < P.vocab && hash_lookup_raw(hash, X.hash_shift, X.hash_mask, v) == 0) {
-                push(v, temp_value<DT>(X, (u32)__ldg((const unsigned short*)G.rowp + v), v));
+                // (top-p rows: on this side of the threshold by its raw value, as every column that is not special; the second pass counts
+                // the others, half values that a temperature rounds to the threshold's among them)
+                const u32 raw = (u32)__ldg((const unsigned short*)G.rowp + v);
+                if (!TOPP || key16(raw) >= thr_key) {
+                    push(v, temp_value<DT>(X, raw, v));
+                }
             }
         }
     }
