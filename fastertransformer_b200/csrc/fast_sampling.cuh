@@ -1202,9 +1202,12 @@ __device__ __forceinline__ bool fast_topp_tail(const KParams& P, const FMap& S, 
         }
         __syncthreads();
         const u32 kmaxv = fkey(maxv);
+        if (DT == FTB200_F16 && temp && kmaxv == fkey(T.thr_y)) {
+            return false;  // (a temperature rounds neighbouring half values to one: it may hold columns below the threshold)
+        }
         for (int i = tid; i < T.n_ord; i += kThreads) {
             const u32 e = cand[i];
-            if ((e >> 20) == T.relmax && fkey(value_of(thr_key + (e >> 20))) == kmaxv) {
+            if (fkey(value_of(thr_key + (e >> 20))) == kmaxv) {
                 atomicMin(&s_sel, (int)(e & 0xfffffu));
             }
         }

@@ -77,3 +77,19 @@ def test_class_on_both_sides_of_the_threshold(V, padded, B, temperature, penalis
         history[:2] = torch.randint(padded - 8, V, (2, B), generator=g, device=cuda_device, dtype=torch.int32)
         history[2:] = torch.randint(1, V, (2, B), generator=g, device=cuda_device, dtype=torch.int32)
     compare(x.to(F16), V, B, cuda_device, top_p=0.98, history=history, temperature=temperature)
+
+
+def test_maximum_of_two_values(cuda_device):
+    """Two half values that a temperature rounds to one: the first column of either is the row's best one."""
+    V, B = 17408, 560
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(5)
+    # neighbours of [16, 32), 1 / 64 apart; divided by 1.3 they lie 0.012 apart, where half values do so by 1 / 128 and 1 / 64
+    low = 24.0 + torch.arange(B, device=cuda_device) % 64 / 64.0
+    x = torch.randn(B, V, generator=g, device=cuda_device) * 0.5 + 7.0
+    x[:, 100], x[:, 9000] = low, low + 1 / 64.0
+    scale = torch.tensor(1.0, device=cuda_device) / (torch.tensor(1.3, device=cuda_device) + 1e-6)
+    y = (x.to(F16)[:, [100, 9000]] * scale.to(F16)).cpu()
+    assert 50 < int((y[:, 0] == y[:, 1]).sum()) < B
+    history = torch.zeros(4, B, dtype=torch.int32, device=cuda_device)
+    compare(x.to(F16), V, B, cuda_device, top_p=0.3, history=history, temperature=1.3)
