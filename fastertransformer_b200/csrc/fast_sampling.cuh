@@ -36,6 +36,7 @@ constexpr int kFPSpecCap = 2048;  // top-p: listed columns above the cut (a hist
 constexpr int kFPClsCap  = 2048;  // top-p: members of the class the scan stops in
 constexpr int kFSampleV  = 2;     // sampled vectors per thread (4096 columns per row)
 constexpr int kFUnroll   = 8;     // 16-byte loads in flight per thread
+constexpr int kFMaxRank  = 96;    // highest rank among the sampled columns that the threads' maxima are good for
 
 // Shared-memory map of the single-pass kernel (dynamic shared memory, offsets fixed per launch).
 struct FMap {
@@ -60,6 +61,18 @@ constexpr int kFStageBytes = 8192;  // >= (kFMaxHist + 2 * kFMaxWords + 4) * 4; 
 __host__ __device__ inline int fast_max_records(int hash_slots)
 {
     return hash_slots < 2048 ? hash_slots / 2 : (hash_slots / 4 * 3 < 4096 ? hash_slots / 4 * 3 : 4096);
+}
+// Columns that a top-k row's threshold should let through: 2k, at least k + 256 (the estimate from a few sampled maxima
+// scatters widely); for k = 1 a handful is enough.
+__host__ __device__ inline int fast_topk_target(int k)
+{
+    return k == 1 ? 64 : (2 * k > k + 256 ? 2 * k : k + 256);
+}
+// Rank among the 4096 sampled columns of the value that `target` of ncols reach; a row with a higher one than kFMaxRank is left.
+__host__ __device__ inline u32 fast_sample_rank(int target, int ncols)
+{
+    const u32 rank = (u32)(((long long)target * (kFSampleV * kThreads * 8) + ncols - 1) / ncols);
+    return rank < 3u ? 3u : rank;
 }
 // bytes of the per-vector mask area: one byte per aligned vector, and room for what follows the pass
 __host__ __device__ inline size_t fast_mask_bytes(int hash_slots, int vocab_padded, bool topp)
@@ -1813,10 +1826,8 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     // scatters widely); for k = 1 a handful is enough
     // (a top-p row of a smaller vocabulary aims lower: the estimate needs the wanted rank well inside the 256
     //  per-thread maxima of the sample, want_s <= 96 below)
-    const int tp_cap = (int)(((long long)ncols * 96) / (kFSampleV * kThreads * 8));
-    const int target = TOPP ? (tp_cap < 2048 ? tp_cap : 2048) : (k == 1 ? 64 : (2 * k > k + 256 ? 2 * k : k + 256));
-    u32       want_s = (u32)(((long long)target * (kFSampleV * kThreads * 8) + ncols - 1) / ncols);
-    want_s           = want_s < 3u ? 3u : want_s;
+    const int tp_cap = (int)(((long long)ncols * kFMaxRank) / (kFSampleV * kThreads * 8));
+    const u32 want_s = fast_sample_rank(TOPP ? (tp_cap < 2048 ? tp_cap : 2048) : fast_topk_target(k), ncols);
     bool words_ok    = true;
     if (wid == 0) {
         u32       kmx = 0;
@@ -1935,7 +1946,7 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     }
     __syncthreads();
     trace_mark(H.trace, 1);
-    if (long_words || want_s > 96u || !(thr_y > neg_max) || thr_key == 0u) {
+    if (long_words || want_s > (u32)kFMaxRank || !(thr_y > neg_max) || thr_key == 0u) {
         return false;  // (uniform for the CTA)
     }
 
@@ -2415,14 +2426,16 @@ __device__ __forceinline__ bool fast_row(const KParams& P, const FMap& S, const 
     return true;
 }
 
-// The step's end for a host that waits for it, by every CTA that has served rows (stop words are seen to row by row): the one that
-// brings the call's count of rows to its end, in whichever of the two kernels, does the length limit and the count of finished
-// rows - unless rows are on the list: then the kernel behind does, which serves them.  A step of 1024 x 128256 then ends with its last
-// row, where the join of two streams, the general kernel over an empty list and the criteria's kernel followed one another.
-static __device__ __noinline__ void f_step_end(const KParams& P, const StopArgs& T, int served)
+// The step's end for a host that waits for it, by every CTA of the two kernels (stop words are seen to row by row): the last one
+// does the length limit and the count of finished rows, or tells the host that rows are on the list.  A step of 1024 x 128256
+// then ends with its last row, where the join of two streams, the general kernel over an empty list and the criteria's kernel followed
+// one another.  CTAs without a row arrive too (those of the top-k rows' kernel may come up last, where the top-p rows' one held their
+// SMs), and nothing is queued behind: when the host hears of the end, nothing of the step is left that could read the workspace or
+// take its tickets.
+static __device__ __noinline__ void f_step_end(const KParams& P, const StopArgs& T)
 {
-    if (arrived_last(T.arrived, served, P.local_batch) && __ldcg(P.redo_count) == 0) {
-        count_finished(P, T, nullptr);
+    if (arrived_last(T.arrived, T.ctas)) {
+        count_finished(P, T, nullptr, __ldcg(P.redo_count) != 0);
     }
 }
 
@@ -2505,10 +2518,9 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     }
     const int tid = threadIdx.x;
     // thread 0 keeps the next row's ticket and number between the stages
-    __shared__ int s_rows, s_served;  // rows of this kernel, and of this CTA so far
+    __shared__ int s_rows;  // rows of this kernel
     int            nt = 0, nr = 0;
     if (tid == 0) {
-        s_served = 0;
         s_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
         nt     = (int)atomicAdd(P.ticket + (TOPP ? 3 : 0), 1u);
         if (nt < s_rows) {
@@ -2639,17 +2651,12 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
             cp_async_wait_all();
             f_compose_header(P, nt, s_rows, nr, s_pre, s_hdr[cur ^ 1]);
         }
-        if (VP == 0 && T.limit != nullptr) {
-            if (T.stop_words != nullptr && done) {
-                row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
-            }
-            if (tid == 0) {
-                ++s_served;
-            }
+        if (VP == 0 && T.limit != nullptr && T.stop_words != nullptr && done) {
+            row_stop_words(P, T.stop_words, T.stop_words_len, T.finished, r);
         }
     }
-    if (VP == 0 && T.limit != nullptr && s_served != 0) {
-        f_step_end(P, T, s_served);
+    if (VP == 0 && T.limit != nullptr && T.ctas != 0) {
+        f_step_end(P, T);
     }
     if (!TOPP && VP == 0 && P.row_count_dev != nullptr) {
         wait_for_previous();

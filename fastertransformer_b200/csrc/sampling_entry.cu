@@ -49,6 +49,7 @@ size_t fast_smem_for(int hash_slots, int vocab_padded, bool topp);
 int    fast_rows_for(const KParams& K, int* list_k, int* list_p, cudaStream_t st);
 int    fast_max_history();
 int    fast_max_words();
+bool   fast_leaves_k(int k, int vocab);
 template<int DT>
 int vp_select_launch(const KParams& K, const VpArgs& V, size_t smem, int sms, cudaStream_t st);
 extern template int vp_select_launch<FTB200_F16>(const KParams&, const VpArgs&, size_t, int, cudaStream_t);
@@ -401,8 +402,29 @@ namespace ftb200 {
 // What of a step's end the sampling launches see to: nothing, all of it unless rows are left (the host hears of them and sends
 // what serves them), or all of it.
 enum StepEnd : int { kStepEndNone, kStepEndRowsLeft, kStepEndAll };
+struct StepTail {
+    StepEnd  end = kStepEndNone;
+    // the general kernel over the single-pass kernels' list of rows, which ends the step then; grid 0: there is no such list
+    KParams  K;
+    StopArgs S;
+    int      grid = 0;
+    size_t   smem = 0;
+};
+static int general_launch(int dtype, const KParams& K, const StopArgs& S, int grid, size_t smem, cudaStream_t st)
+{
+    int rc;
+    switch (dtype) {
+        case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, S, grid, smem, st); break;
+        case FTB200_F16: rc = sampling_launch<FTB200_F16>(K, S, grid, smem, st); break;
+        default: rc = sampling_launch<FTB200_BF16>(K, S, grid, smem, st); break;
+    }
+    if (rc == FTB200_OK) {
+        note_launch(1);
+    }
+    return rc;
+}
 // left_only: the rows that the split kernel of the same step has flagged, by the general kernel.
-int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop = nullptr, StepEnd* end = nullptr,
+int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop = nullptr, StepTail* tail = nullptr,
                               bool left_only = false);
 int stop_criteria_launch(const ftb200_sampling_params* p, const StopArgs& T, cudaStream_t st);
 }
@@ -427,20 +449,24 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     T.arrived        = s->arrived_dev;
     T.result         = (u64*)s->result_host;
     T.sequence       = ++s->sequence;
-    StepEnd end      = kStepEndNone;
-    int     rc       = decode_step_sampling_impl(p, &T, &end);
-    if (rc == FTB200_OK && end == kStepEndNone) {
+    StepTail tail;
+    int      rc = decode_step_sampling_impl(p, &T, &tail);
+    if (rc == FTB200_OK && tail.end == kStepEndNone) {
         rc = stop_criteria_launch(p, T, (cudaStream_t)p->stream);
     }
     *should_stop = 0;
     if (rc != FTB200_OK || T.limit == nullptr) {
         return rc;
     }
-    // Rare: rows that the split kernel's tables could not hold, then the criteria over the whole call.  The rows are found
-    // by their flags on the device, so that these launches do nothing new where none is left.
-    bool       left_sent = end != kStepEndRowsLeft;
+    // Rare: rows that the single-pass kernels left, by the general kernel, which ends the step; or rows that the split kernel's
+    // tables could not hold, then the criteria over the whole call.  The rows are found by their list or their flags on the
+    // device, so that these launches do nothing new where none is left.
+    bool       left_sent = tail.end != kStepEndRowsLeft;
     const auto send_left = [&] {
-        left_sent   = true;
+        left_sent = true;
+        if (tail.grid != 0) {
+            return general_launch(p->dtype, tail.K, tail.S, tail.grid, tail.smem, (cudaStream_t)p->stream);
+        }
         const int e = decode_step_sampling_impl(p, nullptr, nullptr, true);
         return e == FTB200_OK ? stop_criteria_launch(p, T, (cudaStream_t)p->stream) : e;
     };
@@ -480,7 +506,7 @@ extern "C" int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_p
     }
 }
 
-int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, StepEnd* end, bool left_only)
+int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, StepTail* tail, bool left_only)
 {
     if (!left_only) {
         reset_launch_count();
@@ -518,8 +544,8 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
         if (!left_only) {
             SplitArgs F = A;
             if (A.criteria && stop != nullptr && (stop->limit != nullptr || stop->stop_words != nullptr)) {
-                F.stop = *stop;
-                *end   = kStepEndRowsLeft;
+                F.stop    = *stop;
+                tail->end = kStepEndRowsLeft;
             }
             rc = launch(F);
             if (rc != FTB200_OK) {
@@ -534,7 +560,7 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
         // has heard of rows left and the areas are larger than the first launch's, and behind every step that does not wait where those
         // are below half a slice (above 98000 columns; above 49000, 24000 with four, two CTAs a row).  Where the large ones are below
         // half a slice too (above 245000 columns) the general kernel's many CTAs serve the several rows left sooner.
-        const bool words = !left_only && end != nullptr && *end != kStepEndNone;  // (no limit: who serves a row sees to its stop words)
+        const bool words = !left_only && tail != nullptr && tail->end != kStepEndNone;  // (no limit: who serves a row sees to its stop words)
         SplitArgs  B     = A;
         if (words) {
             B.stop = *stop;
@@ -572,11 +598,6 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
             KParams F    = K;
             F.redo_count = K.ticket + 1;
             F.redo_rows  = (int*)((char*)p->workspace + 256);
-            if (stop != nullptr && stop->limit != nullptr) {
-                S         = *stop;
-                S.arrived = K.ticket + 4;
-                *end      = kStepEndAll;
-            }
             // The rows of the top-p layer have a kernel of their own (it wants more registers than the top-k rows'
             // kernel can spare); the two run side by side.
             const bool topp_only = K.topp_states != nullptr && K.topk_states == nullptr;  // one launch
@@ -588,12 +609,27 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
                 return rc;
             }
             note_launch(1);
+            const int rows  = p->local_batch_size;
+            const int pgrid = K.topp_states == nullptr ? 0 : (sm_count() * pper < rows ? sm_count() * pper : rows);
+            const int fgrid = topp_only ? 0 : (sm_count() * fper < rows ? sm_count() * fper : rows);
+            if (stop != nullptr && stop->limit != nullptr) {
+                // A host that waits goes on once the last CTA has counted, and may hand the workspace to another stream then, so nothing
+                // that reads it may be queued behind: the host hears of rows left and sends the general kernel.  That costs
+                // a round trip; where there are such rows in all likelihood - a k that the sample is too small for, nucleus rows off
+                // a 16-byte boundary - the general kernel is queued and ends the step.  us a step, queued always / so: 867 x 26268 half,
+                // k = 50 64.8 / 59.2; nucleus rows at temperature 1.2, nine left, 260.4 / 267.6; 785 x 36096 bf16 of both kinds, 204 of them
+                // with k = 1024, 123.4 / 120.7; 1024 x 128256 166.2 / 165.6.
+                const bool queue = (!topp_only && fast_leaves_k(K.max_top_k, p->vocab_size))
+                                   || (K.topp_states != nullptr && (((size_t)p->logits | (size_t)p->vocab_size_padded * 2) & 15) != 0);
+                S         = *stop;
+                S.arrived = K.ticket + 4;
+                S.ctas    = queue ? 0u : (u32)(pgrid + fgrid);
+                tail->end = queue ? kStepEndAll : kStepEndRowsLeft;
+            }
             if (K.topp_states != nullptr) {
                 if (both) {
                     F.row_order = list_p, F.row_count_dev = K.ticket + 6;
                 }
-                int pgrid = sm_count() * pper;
-                pgrid     = pgrid < p->local_batch_size ? pgrid : p->local_batch_size;
                 rc = f16 ? fast_sampling_launch<FTB200_F16, true>(F, S, pgrid, psmem, true, st) :
                            fast_sampling_launch<FTB200_BF16, true>(F, S, pgrid, psmem, true, st);
                 if (rc != FTB200_OK) {
@@ -605,8 +641,6 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
                 if (both) {
                     F.row_order = list_k, F.row_count_dev = K.ticket + 5;
                 }
-                int fgrid = sm_count() * fper;
-                fgrid     = fgrid < p->local_batch_size ? fgrid : p->local_batch_size;
                 rc = f16 ? fast_sampling_launch<FTB200_F16, false>(F, S, fgrid, fsmem, true, st) :
                            fast_sampling_launch<FTB200_BF16, false>(F, S, fgrid, fsmem, true, st);
                 if (rc != FTB200_OK) {
@@ -625,20 +659,16 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
             if (K.trace != nullptr) {
                 K.trace += (size_t)p->local_batch_size * 32;  // the general kernel's records follow the single-pass kernel's
             }
+            if (S.ctas != 0) {
+                tail->K = K, tail->S = S, tail->grid = grid, tail->smem = smem;
+                return FTB200_OK;
+            }
         }
     }
     if (K.row_flags == nullptr && K.row_count_dev == nullptr) {
         FTB_CUDA_CHECK(cudaMemsetAsync(K.ticket, 0, 256, st));
     }
-    switch (p->dtype) {
-        case FTB200_F32: rc = sampling_launch<FTB200_F32>(K, S, grid, smem, st); break;
-        case FTB200_F16: rc = sampling_launch<FTB200_F16>(K, S, grid, smem, st); break;
-        default: rc = sampling_launch<FTB200_BF16>(K, S, grid, smem, st); break;
-    }
-    if (rc == FTB200_OK) {
-        note_launch(1);
-    }
-    return rc;
+    return general_launch(p->dtype, K, S, grid, smem, st);
 }
 
 extern "C" int ftb200_set_single_pass(int on)

@@ -14,6 +14,10 @@ int fast_max_history()
 {
     return kFMaxHistAll;
 }
+bool fast_leaves_k(int k, int vocab)
+{
+    return fast_sample_rank(fast_topk_target(k), vocab & ~7) > (u32)kFMaxRank;
+}
 int fast_max_words()
 {
     return kFMaxWords;

@@ -4073,27 +4073,27 @@ static __device__ __noinline__ void row_stop_words(const KParams& P, const int* 
     __syncthreads();
 }
 
-// Whether the `n` rows that this CTA has served bring the count of arrived ones to `all` (called by all threads, once every result has
-// been written by them).
-static __device__ bool arrived_last(u32* arrived, int n, int all)
+// Whether this CTA's arrival (of a row, or of the CTA itself) is the last of `all` (called by all threads, once every result has been
+// written by them).
+static __device__ bool arrived_last(u32* arrived, u32 all)
 {
     __shared__ u32 s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicAdd(arrived, (u32)n) + (u32)n == (u32)all ? 1u : 0u;
+        s_last = atomicAdd(arrived, 1u) + 1u == all ? 1u : 0u;
         __threadfence();
     }
     __syncthreads();
     return s_last != 0;
 }
 
-// The length limit and the count of finished rows over the batch, stored for a host that polls the word: by the CTA that has seen every
-// row of the call arrive.  `flags` [local_batch] or null: where one is set, rows wait for another launch, and the
+// The length limit and the count of finished rows over the batch, stored for a host that polls the word: by the CTA that has seen
+// everything of the call arrive.  `left`, or one of `flags` [local_batch] (or null): rows wait for another launch, and the
 // host is told instead.  The fence that lets
 // the host find all of the step behind the word takes 1.3 us; it runs beside the loads of the flags, and a second one only
 // follows where the limit has ended a row (8 x 32000, a word each way: 19.9 us a step with one after the other, 19.0 so).
-static __device__ __noinline__ void count_finished(const KParams& P, const StopArgs& T, const int* flags)
+static __device__ __noinline__ void count_finished(const KParams& P, const StopArgs& T, const int* flags, bool left)
 {
     __shared__ u32 s_sum, s_changed;
     const int      tid = threadIdx.x;
@@ -4102,7 +4102,6 @@ static __device__ __noinline__ void count_finished(const KParams& P, const StopA
     const bool    mine_one = tid < kCount && tid < P.batch_size;
     const uint8_t old_one  = mine_one ? __ldcg(T.finished + tid) : (uint8_t)0;
     const u32     lim_one  = mine_one ? T.limit[tid] : 0u;
-    bool          left     = false;
     for (int i = tid; flags != nullptr && i < P.local_batch; i += kThreads) {
         left |= __ldcg(flags + i) != 0;
     }
@@ -4167,7 +4166,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
     u64* gscratch = P.scratch + (size_t)blockIdx.x * P.scratch_stride;
     // rows to serve: the whole local batch, or the list the single-pass kernel left behind
     const int n_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
-    int       served = 0;
     for (int next = blockIdx.x;; next += gridDim.x) {
         __syncthreads();
         int t;
@@ -4202,11 +4200,11 @@ __global__ void __launch_bounds__(kThreads, 2) decode_sampling_kernel(const __gr
         if (rec != nullptr && threadIdx.x == 0) {
             rec[3] = global_timer_ns();
         }
-        ++served;
     }
-    // (a host waits, and the single-pass kernels have left rows: the step ends here)
-    if (T.limit != nullptr && served != 0 && arrived_last(T.arrived, served, n_rows)) {
-        count_finished(P, T, nullptr);
+    // A host waits, and the step ends here: with rows that the single-pass kernels have left, and where they leave the end to this kernel.
+    // Every CTA arrives, also one without a row, so that none is left to read the workspace once the host goes on.
+    if (T.limit != nullptr && (n_rows != 0 || T.ctas == 0) && arrived_last(T.arrived, gridDim.x)) {
+        count_finished(P, T, nullptr, false);
     }
 }
 

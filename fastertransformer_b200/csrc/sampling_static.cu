@@ -51,8 +51,8 @@ int static_scratch(void** out)
 
 namespace ftb200 {
 struct StopArgs;
-enum StepEnd : int;
-int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, StepEnd* end, bool left_only);
+struct StepTail;
+int decode_step_sampling_impl(const ftb200_sampling_params* p, const StopArgs* stop, StepTail* tail, bool left_only);
 }
 
 extern "C" size_t ftb200_static_scratch_bytes(void)

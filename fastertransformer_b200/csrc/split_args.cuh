@@ -27,6 +27,7 @@ struct StopArgs {
     u32*            arrived;         // one word, zero between calls
     u64*            result;          // page-locked host word: sequence << 32 | finished rows
     u32             sequence;
+    u32             ctas;            // single-pass kernels: CTAs that arrive, all of them; 0: the general kernel behind ends the step
 };
 
 struct SplitArgs {

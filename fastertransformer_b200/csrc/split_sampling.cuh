@@ -1919,13 +1919,13 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
     if (T.limit == nullptr) {
         return;
     }
-    if (!arrived_last(T.arrived, 1, P.local_batch)) {
+    if (!arrived_last(T.arrived, (u32)P.local_batch)) {
         return;
     }
     if (tid == 0) {
         *T.arrived = 0;
     }
-    count_finished(P, T, flags);
+    count_finished(P, T, flags, false);
 }
 
 // ROOMY: 128 registers, two CTAs on an SM, and - when asked to - the step's stop criteria: one launch per decode step.

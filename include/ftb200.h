@@ -266,6 +266,8 @@ int ftb200_wait_should_stop(const int* finished_count_host, int batch_size, int 
  * it does.  With a length limit, rows that the first launch cannot hold (a nucleus of most of the vocabulary, thousands of equal
  * values around the k-th) are sent for within this call, once that launch has said so in *result_host - with ~sequence for the
  * high word: wait for `sequence` there - or when the deadline is missed; an error of these launches is returned.
+ * After FTB200_OK with a length limit nothing of the step is left that reads or writes the caller's memory: the workspace and the
+ * block may be used on another stream, or freed.  (Without one the call does not wait, and stream order applies.)
  * ------------------------------------------------------------------------------------------ */
 typedef struct ftb200_stop_params {
     const int*      stop_words;

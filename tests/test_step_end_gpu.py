@@ -1,0 +1,79 @@
+"""The end of a step that waits, single-pass kernels: once the call has returned, nothing of the step is queued that could still read its
+workspace, so that the caller may use it on another stream at once."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+F16, BF16 = torch.float16, torch.bfloat16
+
+
+def make(dtype, V, B, kinds, device, penalty=1.1):
+    from fastertransformer_b200 import DynamicDecodeLayer
+    args = {"random_seed": np.arange(B).astype(np.uint64), "repetition_penalty": np.resize(np.asarray(penalty, np.float32), B)}
+    if kinds != "topk":
+        args["runtime_top_p"] = np.asarray([0.9], np.float32)
+    if kinds != "topp":
+        args["runtime_top_k"] = np.resize(np.asarray({"both": [0, 40, 1], "wide": [0, 1024, 1], "topk": [40]}[kinds], np.uint32), B)
+    layer = DynamicDecodeLayer(V, V, dtype, device)
+    layer.setup(B, 1, args)
+    return layer
+
+
+def run(layer, x, ids, step, limit):
+    B, V = x.shape
+    device = x.device
+    st = {"output_ids": ids, "finished": torch.zeros(B, dtype=torch.bool, device=device),
+          "sequence_length": torch.full((B,), step, dtype=torch.int32, device=device)}
+    inputs = {"logits": x, "step": step, "max_input_length": step, "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=device)}
+    if limit:
+        inputs["sequence_limit_length"] = torch.full((B,), step + 9, dtype=torch.int32, device=device)
+    torch.cuda.synchronize()
+    assert not layer.forward(st, inputs)
+    return st
+
+
+@pytest.mark.parametrize("kinds,penalty,launches", [
+    ("topk", 1.1, 2), ("topp", 1.1, 2), ("both", 1.1, 3),  # the header's kernel, then the rows' kernels
+    ("topp", [1.1, 0.9], 3), ("both", [1.1, 1.1, 0.9, 0.9], 4),  # rows whose penalty raises values are left: sent for
+    ("wide", 1.1, 4)])  # k = 1024 of few columns is always left: the general kernel is queued and ends the step
+def test_nothing_behind_the_end(kinds, penalty, launches, cuda_device):
+    from fastertransformer_b200 import lib
+    V, B = 32768, 560
+    layer = make(BF16, V, B, kinds, cuda_device, penalty)
+    x = (torch.randn(B, V, device=cuda_device) * 2.5).to(BF16)
+    run(layer, x, torch.ones(12, B, dtype=torch.int32, device=cuda_device), 8, True)
+    assert lib.ftb200_last_launch_count() == launches
+
+
+@pytest.mark.parametrize("dtype,V,B,kinds,penalty", [
+    (BF16, 32768, 560, "both", 1.1), (BF16, 128256, 200, "both", 1.1), (F16, 17408, 1024, "topp", 1.1),
+    (F16, 32768, 560, "both", [1.1, 0.9, 1.1]), (BF16, 32768, 560, "wide", 1.1)])
+def test_workspace_is_free_at_the_end(dtype, V, B, kinds, penalty, cuda_device):
+    """Two streams take turns with one layer, ordered by nothing but the host's wait; the workspace is written over in between."""
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(V + B)
+    rounds = 12
+    xs = [(torch.randn(B, V, generator=g, device=cuda_device) * 2.5).to(dtype) for _ in range(4)]
+    history = torch.randint(1, V, (20, B), generator=g, device=cuda_device, dtype=torch.int32)
+    results = []
+    for turns in (False, True):
+        layer = make(dtype, V, B, kinds, cuda_device, penalty)
+        streams = [torch.cuda.Stream(cuda_device) for _ in range(2 if turns else 1)]
+        ids = [history.clone() for _ in range(rounds)]
+        states = [{"output_ids": i, "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+                   "sequence_length": torch.full((B,), 16, dtype=torch.int32, device=cuda_device)} for i in ids]
+        inputs = [{"logits": x, "step": 16, "max_input_length": 16,
+                   "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device),
+                   "sequence_limit_length": torch.full((B,), 99, dtype=torch.int32, device=cuda_device)} for x in xs]
+        torch.cuda.synchronize()
+        for i in range(rounds):
+            with torch.cuda.stream(streams[i % len(streams)]):
+                if turns and i > 0:
+                    layer._workspace[:4096].fill_(1)
+                assert not layer.forward(states[i], inputs[i % 4])
+        torch.cuda.synchronize()
+        results.append([s[k].cpu().numpy() for s in states for k in ("output_ids", "sequence_length", "finished")])
+    for want, got in zip(*results):
+        np.testing.assert_array_equal(got, want)
