@@ -159,7 +159,11 @@ struct SpShared {
     u32   first_max;       // smallest column that holds the maximum
     u32   n_cls;           // columns of the crossing class
     u32   verdict;         // 0 class found, 1 draw beyond the whole row (best token), 2 leave the row
-    u32   p_sel, j_sel;    // crossing: probability (bits), position in the sorted order
+    union {
+        u32   p_sel;       // crossing: probability (bits),
+        float per_y;       // (until it is looked for: raw value per unit of a final value, bfloat16 rows)
+    };
+    u32   j_sel;           // position in the sorted order
     u32   larger;          // columns of a larger probability than the crossing's
     u32    bad_order;
     u32    state[6];       // counter and words of the row's generator after its draw (nothing else of it moves)
@@ -931,18 +935,39 @@ __device__ __forceinline__ void sp_sort_few(float* k, int m)
     }
 }
 
+// bfloat16 values without a bias that fall into bin b, by the distance of its edges in bit patterns; `per_y` raw values make one final one.
+__device__ __forceinline__ u32 sp_bf16_patterns(float maxv, int b, float per_y)
+{
+    return (fkey((maxv - sp_edge(b)) * per_y) >> 16) - (fkey((maxv - sp_edge(b + 1)) * per_y) >> 16);
+}
+
 // One nucleus owner's keys (bins b_lo .. b_hi, bin by bin in `a`) into descending order, in place, where a bin holds few values: bfloat16
 // logits without a bias, 128 values an octave, and the penalised columns' beside them.  A thread takes a bin of up to eight keys, a
-// warp a larger one: most hold one value, the others are written value by value.  Nothing is counted, prefixed or moved
-// through a second copy, and a full area goes like a half full one.  Returns false when a bin has more than 32 values: sp_sort_area
-// orders those (the bins may be in any order within).  An owner's 3000 keys, 128256 columns: 11.2 us with sp_sort_area, 5.2
-// so.  fp32 and half rows have too many values in a bin: 11 to 42 us where sp_sort_area takes 7 to 11.
-static __device__ __noinline__ bool sp_sort_bins(float* a, const u32* excl, u32 start, int n, int b_lo, int b_hi)
+// warp a larger one: most hold one value; up to 32 keys are ordered by counting, more are written value by value, up to 32 of them.
+// Nothing is counted, prefixed or moved through a second copy, and a full area goes like a half full one.  Returns false where
+// sp_sort_area has to order the keys (the bins may be in any order within).  An owner's 3000 keys, 128256 columns: 11.2 us with
+// sp_sort_area, 5.2 so.  fp32 and half rows have too many values in a bin: 11 to 42 us where sp_sort_area takes 7 to 11.
+//
+// So have bfloat16 rows whose nucleus comes near zero (flat ones): there a bin of more than 32 keys can hold more than kSpFewPatterns
+// values, and the owner goes to sp_sort_area before a key has been looked at.  us a step, p 0.95, sp_sort_area always / without this
+// test, every bin value by value / with it at 32 / 16 / 8 / 4: 8 x 32000, sigma 1 50.0 / 75.8 / 55.1 / 51.5 / 49.3 / 48.8; 16 x 50264, sigma 1.5
+// 53.6 / 73.8 / 54.2 / 52.4 / 51.1 / 51.0; 32 x 128256, sigma 2 121.9 / 104.4 / 103.1 / 102.8 / 104.4 / 107.1, sigma 2.5 71.1 / 64.3 / 64.4 /
+// 64.5 / 64.2 / 64.3.
+constexpr u32 kSpFewPatterns = 8;
+static __device__ __noinline__ bool sp_sort_bins(float* a, const u32* excl, u32 start, int n, int b_lo, int b_hi, float maxv, float per_y)
 {
     FTB_ASSUME_SHARED(a);
     FTB_ASSUME_SHARED(excl);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     bool      ok   = true;
+#pragma unroll 1
+    for (int b = b_lo + (int)threadIdx.x; b <= b_hi; b += kThreads) {
+        const u32 c = (b < b_hi ? excl[b + 1] : start + (u32)n) - excl[b];
+        ok          = ok && (c <= 32u || sp_bf16_patterns(maxv, b, per_y) <= kSpFewPatterns);
+    }
+    if (!__syncthreads_and(ok)) {
+        return false;
+    }
     int       turn = 0;  // larger bins in front, the same in every warp
 #pragma unroll 1
     for (int b0 = b_lo; b0 <= b_hi; b0 += 32) {
@@ -968,6 +993,20 @@ static __device__ __noinline__ bool sp_sort_bins(float* a, const u32* excl, u32 
                 same &= k[i] == first;
             }
             if (__all_sync(0xffffffffu, same)) {
+                continue;
+            }
+            if (m <= 32) {
+                const u32 mine = lane < m ? fkey(k[lane]) : 0u;
+                int       to   = 0;
+#pragma unroll 4
+                for (int j = 0; j < m; ++j) {
+                    const u32 x = __shfl_sync(0xffffffffu, mine, j);
+                    to += x > mine || (x == mine && j < lane) ? 1 : 0;
+                }
+                __syncwarp();
+                if (lane < m) {
+                    k[to] = fkey_inv(mine);
+                }
                 continue;
             }
             // each value with its count, the largest first
@@ -1280,6 +1319,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     float best = sp_load_slice<DT>(P, X0, rowp, y, rank, lgvt, nchunk);
     if (tid == 0) {
         s_u        = curand_uniform(&draw);
+        X.per_y    = P.apply_temp ? P.temperature[r] + 1e-6f : 1.0f;
         X.state[0] = draw.d;  // (stored with the result)
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
@@ -1804,7 +1844,7 @@ __device__ __forceinline__ bool sp_row(const KParams& P, const SplitArgs& A, uns
     if (rank < owners) {
         float* const a   = (float*)M.area;
         const int    cnt = (int)(K.start[rank + 1] - K.start[rank]);
-        bool         bad = !(DT == FTB200_BF16 && P.bias == nullptr && sp_sort_bins(a, excl, K.start[rank], cnt, s_blo, s_bhi))
+        bool         bad = !(DT == FTB200_BF16 && P.bias == nullptr && sp_sort_bins(a, excl, K.start[rank], cnt, s_blo, s_bhi, maxv, X.per_y))
                    && !sp_sort_area(a, M.sub, excl, M.hist, K.start[rank], cnt, maxv, M.area_cap, DT != FTB200_F32);
 #pragma unroll 4
         for (int i = tid; i < cnt; i += kThreads) {
