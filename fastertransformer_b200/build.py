@@ -8,6 +8,7 @@ same approximate exp / log / divide instructions.
 """
 import concurrent.futures
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -25,6 +26,35 @@ FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "--use_fast_math", "-lineinfo",
     "--expt-relaxed-constexpr", "--expt-extended-lambda", "-Xcompiler", "-fPIC", "-I" + INC, "-I" + CSRC,
 ]
+
+# What the assembler has to report of a kernel: the least registers - a kernel whose body the compiler has taken for unreachable (a wrong
+# __builtin_assume) comes out with a few, builds and ends in an illegal address - and the most static shared memory, in bytes, that
+# leaves room for two CTAs of it on an SM with what choose_split asks for in whole kilobytes (kTwoPerSm).
+LIMITS = {"split_sampling_kernel": (64, 5120), "fast_sampling_kernel": (64, None), "decode_sampling_kernel": (96, None)}
+
+
+def check_kernels(log):
+    """Raises RuntimeError where a kernel in the output of `ptxas -v` is outside of LIMITS; returns how many of them it has seen."""
+    seen, kernel = 0, None
+    for line in log.splitlines():
+        m = re.search(r"Compiling entry function '(\w+)'", line)
+        if m:
+            kernel = m[1]
+        m = re.search(r"Used (\d+) registers", line)
+        if not m or kernel is None:
+            continue
+        shared = re.search(r"(\d+) bytes smem", line)
+        shared = int(shared[1]) if shared else 0
+        for name, (least, most) in LIMITS.items():
+            if name not in kernel:
+                continue
+            seen += 1
+            if int(m[1]) < least:
+                raise RuntimeError("%s: %s registers, at least %d expected" % (kernel, m[1], least))
+            if most is not None and shared > most:
+                raise RuntimeError("%s: %d bytes of static shared memory, at most %d leave room for two CTAs on an SM" % (kernel, shared, most))
+        kernel = None
+    return seen
 
 
 def _newest_header():
@@ -46,11 +76,14 @@ def _sources():
     return out
 
 
-def _compile(src, obj, verbose):
-    cmd = [NVCC] + FLAGS + ["-x", "cu", "-c", src, "-o", obj]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    r = subprocess.run(cmd, capture_output=True, text=True)
+def _compile(src, obj):
+    r = subprocess.run([NVCC, "-Xptxas=-v"] + FLAGS + ["-x", "cu", "-c", src, "-o", obj], capture_output=True, text=True)
+    if r.returncode == 0:
+        try:
+            check_kernels(r.stdout + r.stderr)
+        except RuntimeError:
+            os.remove(obj)
+            raise
     return src, r.returncode, r.stdout + r.stderr
 
 
@@ -65,7 +98,7 @@ def build(verbose=False, force=False):
             jobs.append((src, obj))
     if jobs:
         with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as ex:
-            for src, rc, log in ex.map(lambda j: _compile(j[0], j[1], verbose), jobs):
+            for src, rc, log in ex.map(lambda j: _compile(j[0], j[1]), jobs):
                 if verbose or rc != 0:
                     sys.stderr.write(log)
                 if rc != 0:

@@ -168,7 +168,7 @@ struct SpShared {
     u32    bad_order;
     u32    state[6];       // counter and words of the row's generator after its draw (nothing else of it moves)
     // (static and dynamic shared memory have to leave room for two CTAs with kTwoPerSm, which is asked for in whole kilobytes: at most 5120
-    // bytes of static memory)
+    // bytes of static memory, which build.py checks)
     union {
         u64               best[kSpMaxN * kWarps];  // arg-max rows, a warp each: key of its largest value << 32 | the largest tie key of its columns
         alignas(16) float agg[(kSpMaxN * kSpAreaWide) / 256];  // nuclei: sums of 256 probabilities
