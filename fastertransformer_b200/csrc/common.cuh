@@ -142,6 +142,16 @@ __device__ __forceinline__ void wait_for_previous()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+__device__ __forceinline__ void store_release(u32* p, u32 v)
+{
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ u32 load_acquire(const u32* p)
+{
+    u32 v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // Tells the compiler that a pointer loaded from a structure points into shared memory, so that it emits
 // ld.shared / st.shared instead of generic accesses (every pointer of the kernel's shared-memory map qualifies).

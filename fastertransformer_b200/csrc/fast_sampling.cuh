@@ -2476,8 +2476,12 @@ static __global__ void __launch_bounds__(kFListThreads) fast_rows_kernel(const _
             list_k[at_k + __popc(bk & below)] = r;
         }
     }
-    if (tid < 64) {
-        P.ticket[tid] = tid == kFHeadRowsK ? (u32)n_k : (tid == kFHeadRowsP ? (u32)n_p : 0u);
+    if (tid < 64 && tid != kFHeadRowsK) {
+        P.ticket[tid] = tid == kFHeadRowsP ? (u32)n_p : 0u;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        store_release(P.ticket + kFHeadRowsK, (u32)n_k);  // (what the top-k rows' kernel acquires: see there)
     }
 }
 
@@ -2490,13 +2494,13 @@ static __global__ void __launch_bounds__(kFListThreads) fast_rows_kernel(const _
 template<int DT, bool TOPP, int VP = 0>
 __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(const __grid_constant__ KParams P, const __grid_constant__ StopArgs T)
 {
-    // (with both kinds of rows the top-k rows' kernel comes up beside the top-p rows' one, which has seen the end of the kernel in
-    // front: it need not wait for that, but nothing that its SM has kept from before may be read)
-    if (TOPP || VP != 0 || P.row_count_dev == nullptr) {
+    // With both kinds of rows the top-k rows' kernel comes up beside the top-p rows' one, whose CTAs have all seen the end of the list
+    // kernel by then, and that one the end of what is in front of it: everything read here has been written before this grid
+    // starts.  That it is seen follows from the list kernel's release of the number of rows, its last store, which thread 0 acquires
+    // below before any thread reads memory.
+    const bool beside = !TOPP && VP == 0 && P.row_count_dev != nullptr;
+    if (!beside) {
         wait_for_previous();
-    }
-    else {
-        __threadfence();
     }
     let_next_come_up();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2521,7 +2525,7 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     __shared__ int s_rows;  // rows of this kernel
     int            nt = 0, nr = 0;
     if (tid == 0) {
-        s_rows = P.row_count_dev != nullptr ? (int)__ldcg(P.row_count_dev) : P.local_batch;
+        s_rows = P.row_count_dev != nullptr ? (int)load_acquire(P.row_count_dev) : P.local_batch;
         nt     = (int)atomicAdd(P.ticket + (TOPP ? 3 : 0), 1u);
         if (nt < s_rows) {
             nr = P.row_order != nullptr ? __ldcg(P.row_order + nt) : nt;
@@ -2658,7 +2662,7 @@ __global__ void __launch_bounds__(kThreads, TOPP ? 2 : 3) fast_sampling_kernel(c
     if (VP == 0 && T.limit != nullptr && T.ctas != 0) {
         f_step_end(P, T);
     }
-    if (!TOPP && VP == 0 && P.row_count_dev != nullptr) {
+    if (beside) {
         wait_for_previous();
     }
 }

@@ -77,3 +77,36 @@ def test_workspace_is_free_at_the_end(dtype, V, B, kinds, penalty, cuda_device):
         results.append([s[k].cpu().numpy() for s in states for k in ("output_ids", "sequence_length", "finished")])
     for want, got in zip(*results):
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("dtype,V,B,kinds", [(BF16, 32768, 560, "both"), (F16, 32768, 560, "wide"), (BF16, 17408, 1024, "topp")])
+def test_kernels_side_by_side_under_capture(dtype, V, B, kinds, cuda_device):
+    """The kernels that follow each other without a wait in between, recorded in a graph; the logits and everything else are written
+    right in front of each replay."""
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(V)
+    xs = [(torch.randn(B, V, generator=g, device=cuda_device) * 2.5).to(dtype) for _ in range(6)]
+    results = []
+    for capture in (False, True):
+        layer = make(dtype, V, B, kinds, cuda_device)
+        x, step = torch.zeros_like(xs[0]), 8
+        st = {"output_ids": torch.ones(step + 2, B, dtype=torch.int32, device=cuda_device),
+              "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+              "sequence_length": torch.full((B,), step, dtype=torch.int32, device=cuda_device)}
+        inputs = {"logits": x, "step": step, "max_input_length": step, "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device)}
+        call = lambda: layer.forward(st, inputs)
+        if capture:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                call()
+            call = graph.replay
+        got = []
+        for logits in xs:
+            x.copy_(logits)
+            st["output_ids"][:step] = torch.arange(B, device=cuda_device, dtype=torch.int32) % 997
+            call()
+            got.append(st["output_ids"].clone())
+        torch.cuda.synchronize()
+        results.append([t.cpu().numpy() for t in got] + [layer.topk.curand.cpu().numpy(), layer.topp.curand.cpu().numpy()])
+    for want, got in zip(*results):
+        np.testing.assert_array_equal(got, want)
