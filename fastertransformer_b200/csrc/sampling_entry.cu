@@ -2,6 +2,7 @@
 #include <atomic>
 #include <chrono>
 
+#include "device_once.cuh"
 #include "sampling_params.cuh"
 #include "spans.cuh"
 #include "split_args.cuh"
@@ -410,6 +411,14 @@ struct StepTail {
     int      grid = 0;
     size_t   smem = 0;
 };
+// Whether the general kernel has been launched on the current device.  Its first launch takes milliseconds (the kernel is loaded, and the
+// device's memory for stack frames grows to its): where nothing else asks for it in the first steps, one of them does.
+static std::atomic<bool>* general_known(int dtype)
+{
+    static std::atomic<bool> known[kDevicesKnown][3];
+    int                      dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevicesKnown ? &known[dev][dtype] : nullptr;
+}
 static int general_launch(int dtype, const KParams& K, const StopArgs& S, int grid, size_t smem, cudaStream_t st)
 {
     int rc;
@@ -419,6 +428,10 @@ static int general_launch(int dtype, const KParams& K, const StopArgs& S, int gr
         default: rc = sampling_launch<FTB200_BF16>(K, S, grid, smem, st); break;
     }
     if (rc == FTB200_OK) {
+        std::atomic<bool>* const known = general_known(dtype);
+        if (known != nullptr && !known->load(std::memory_order_relaxed)) {
+            known->store(true, std::memory_order_relaxed);
+        }
         note_launch(1);
     }
     return rc;
@@ -616,10 +629,12 @@ int ftb200::decode_step_sampling_impl(const ftb200_sampling_params* p, const Sto
                 // A host that waits goes on once the last CTA has counted, and may hand the workspace to another stream then, so nothing
                 // that reads it may be queued behind: the host hears of rows left and sends the general kernel.  That costs
                 // a round trip; where there are such rows in all likelihood - a k that the sample is too small for, nucleus rows off
-                // a 16-byte boundary - the general kernel is queued and ends the step.  us a step, queued always / so: 867 x 26268 half,
-                // k = 50 64.8 / 59.2; nucleus rows at temperature 1.2, nine left, 260.4 / 267.6; 785 x 36096 bf16 of both kinds, 204 of them
-                // with k = 1024, 123.4 / 120.7; 1024 x 128256 166.2 / 165.6.
-                const bool queue = (!topp_only && fast_leaves_k(K.max_top_k, p->vocab_size))
+                // a 16-byte boundary - the general kernel is queued and ends the step; so it does in the first such step on a
+                // device.  us a step, queued always / so: 867 x 26268 half, k = 50 64.8 / 59.2; nucleus rows at temperature 1.2, nine left,
+                // 260.4 / 267.6; 785 x 36096 bf16 of both kinds, 204 of them with k = 1024, 123.4 / 120.7; 1024 x 128256 166.2 / 165.6.
+                const std::atomic<bool>* const known = general_known(p->dtype);
+                const bool queue = (known != nullptr && !known->load(std::memory_order_relaxed))
+                                   || (!topp_only && fast_leaves_k(K.max_top_k, p->vocab_size))
                                    || (K.topp_states != nullptr && (((size_t)p->logits | (size_t)p->vocab_size_padded * 2) & 15) != 0);
                 S         = *stop;
                 S.arrived = K.ticket + 4;

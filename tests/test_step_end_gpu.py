@@ -43,7 +43,8 @@ def test_nothing_behind_the_end(kinds, penalty, launches, cuda_device):
     V, B = 32768, 560
     layer = make(BF16, V, B, kinds, cuda_device, penalty)
     x = (torch.randn(B, V, device=cuda_device) * 2.5).to(BF16)
-    run(layer, x, torch.ones(12, B, dtype=torch.int32, device=cuda_device), 8, True)
+    for _ in range(2):  # (the first such step on a device queues the general kernel, which loads it)
+        run(layer, x, torch.ones(12, B, dtype=torch.int32, device=cuda_device), 8, True)
     assert lib.ftb200_last_launch_count() == launches
 
 
