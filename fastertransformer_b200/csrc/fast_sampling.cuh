@@ -583,10 +583,10 @@ __device__ __forceinline__ FGeo f_geometry(const KParams& P, int r)
 // (kernels/sampling_topp_kernels.cu:1294-1345 soft-max, :801-860 arg-max shortcut, :877-1004 sorted scan):
 //   pass 2 (the row again, mostly from L2): the soft-max denominator in the reference's order - thread t owns
 //     the "virtual threads" 4t..4t+3 (column mod 1024) and adds four exponentials per 1024-column chunk, strictly
-//     in chunk order; special columns take their final value (the per-vector bytes say where they are).  The
-//     same pass counts the bit patterns between a provisional cut and the threshold and lists the special
-//     columns that fall there, so that the sorted probability sequence is known as (probability, count) runs
-//     down to the cut;
+//     in chunk order; special columns take their final value from records filed beforehand, by warp and pair of
+//     chunks.  The same pass counts the bit patterns between a provisional cut and the threshold (the special
+//     columns' have been taken off, and those of them that fall there are listed from the table), so that the
+//     sorted probability sequence is known as (probability, count) runs down to the cut;
 //   the block scan of topp_sampling is replayed over the runs (cub::BlockScan<float,256> raking order: 32
 //     segments of 8, Kogge-Stone over the segment totals, running prefix chunk by chunk);
 //   the class (bit patterns of equal probability) that holds the crossing gives the id: its J-th column in

@@ -136,7 +136,8 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
     // one.  us a step, general kernel / split form, bf16: nucleus rows alone, 300 x 17001 205 / 89, 1000 x 30001 613 / 290, 1000 x 50257
     // 866 / 479, 150 x 128257 564 / 192, 500 x 128257 1183 / 616, 200 x 250001 1216 / 774: always the split form; both kinds, 1000 x 17001
     // 218 / 160, 400 x 50257 316 / 137, 800 x 50257 352 / 309, 1000 x 50257 367 / 380, 150 x 128257 503 / 122, 300 x 128257 555 / 284, 1000 x
-    // 128257 665 / 888.
+    // 128257 665 / 888.  (The line is coarse: above it 600 x 100001 is even, 507 / 500, and 600 x 128257, 606 / 546, and 300 x 250001, 924 /
+    // 861, would be quicker in the split form; the two that are not have 1000 rows.)
     const bool off = topp && (((size_t)p->logits | (size_t)p->vocab_size_padded * 2) & 15) != 0;
     if (single_pass && off && mixed && (double)rows * vocab > 48e6) {
         return false;

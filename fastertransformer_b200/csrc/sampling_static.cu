@@ -10,7 +10,7 @@
 // kept small; shapes that need more are refused and have to be sent in slices (the `ite` /
 // `local_batch_size` fields of the argument block exist for exactly that).
 // The entry point itself allocates nothing and creates nothing: no cudaMalloc / cudaFree, no stream, no event
-// (the single-pass kernels of the step run one after the other on the caller's stream here).
+// (all kernels of the step are launched in the caller's stream; the two single-pass ones run side by side in it).
 #include <mutex>
 
 #include "common.cuh"

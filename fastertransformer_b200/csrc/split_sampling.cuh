@@ -13,9 +13,9 @@
 // left, eight or ten for a nucleus that one or several CTAs sort, one more with special columns, the last one at its end -
 // and about six sweeps over its shared memory; a CTA-per-row kernel walks eight times as many columns with the same 256 threads.  Measured on B200, one row
 // alone on its SMs: arg-max of 32000 columns 4 us, k = 50 of 50257 fp32 13 us, a nucleus of 50257 fp32 19 us (the general
-// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 5 us (k = 1) to 58 us (25000-column nucleus).  Batch
-// of 64 x 50257 fp32 top-p: 42 us a step; 48 x 51200 half with bias and log-probs: 52 us; 24 steps of 16 x 128256 bf16: 1240 to
-// 1420 us.  Before the nucleus was placed by bin, sorted by short loops and the general row code taken out: 60, 83, 1600 to 1930.
+// kernel: 180 to 1100 us), 128256 bf16 with 2500 tokens of history 5 us (k = 1) to 45 us (the widest nucleus of 96 rows).  Batch
+// of 64 x 50257 fp32 top-p: 42 us a step; 48 x 51200 half with bias and log-probs: 51 us; 24 steps of 16 x 128256 bf16: 1300 to
+// 1390 us.  Before the nucleus was placed by bin, sorted by short loops and the general row code taken out: 60, 83, 1600 to 1930.
 //
 // Code size matters: a row runs through most of this code once, so a loop that is unrolled for the largest case waits for
 // its instructions in every case.

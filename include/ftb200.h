@@ -289,8 +289,8 @@ int ftb200_decode_step(const ftb200_sampling_params* p, ftb200_stop_params* s, i
  * a fixed area of ftb200_static_scratch_bytes() (64 MiB) built into the library; every GPU that loads the
  * library holds it until the process exits.  `workspace` and `workspace_bytes` of the argument block are
  * ignored; everything else means what it means above and the results are the same.  No cudaMalloc, cudaFree
- * or other allocating call is made, and no stream or event is created: the kernels of the step run one
- * after the other on `stream`.
+ * or other allocating call is made, and no stream or event is created: the kernels of the step are launched on
+ * `stream`, in whose order they stand.
  *
  *   - A shape whose ftb200_sampling_workspace_bytes() exceeds the area is refused with
  *     FTB200_WORKSPACE_SMALL.  For local_batch_size up to twice the SM count the need is

@@ -111,3 +111,46 @@ def test_kernels_side_by_side_under_capture(dtype, V, B, kinds, cuda_device):
         results.append([t.cpu().numpy() for t in got] + [layer.topk.curand.cpu().numpy(), layer.topp.curand.cpu().numpy()])
     for want, got in zip(*results):
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("kinds,penalty", [("both", [1.1, 0.9, 1.1]), ("topp", 1.1), ("wide", 1.1)])
+def test_deadline_with_rows_on_the_list(kinds, penalty, cuda_device):
+    """A step that misses its deadline while the stream is held sends what serves the rows left, and ends by itself."""
+    import ctypes as C
+    import time
+
+    from fastertransformer_b200 import lib
+    rt = C.CDLL("libcudart.so.12")
+    HOSTFN = C.CFUNCTYPE(None, C.c_void_p)
+    hold = HOSTFN(lambda _: time.sleep(0.3))
+    rt.cudaLaunchHostFunc.argtypes = [C.c_void_p, HOSTFN, C.c_void_p]
+    V, B, step = 32768, 560, 8
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(1)
+    xs = [(torch.randn(B, V, generator=g, device=cuda_device) * 2.5).to(BF16) for _ in range(3)]
+    got = []
+    for late in (False, True):
+        layer = make(BF16, V, B, kinds, cuda_device, penalty)
+        st = {"output_ids": torch.ones(step + 4, B, dtype=torch.int32, device=cuda_device),
+              "finished": torch.zeros(B, dtype=torch.bool, device=cuda_device),
+              "sequence_length": torch.full((B,), step, dtype=torch.int32, device=cuda_device)}
+        inputs = {"max_input_length": step, "end_id": torch.full((B,), V - 1, dtype=torch.int32, device=cuda_device),
+                  "sequence_limit_length": torch.full((B,), step + 2, dtype=torch.int32, device=cuda_device)}
+        stream, stops = torch.cuda.Stream(device=cuda_device), []
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            for s in range(3):
+                if late and s == 1:
+                    P, stop = layer._gate[0, B]["params"], C.c_int(-7)
+                    P.step, P.logits = step + s, xs[s].data_ptr()
+                    assert rt.cudaLaunchHostFunc(C.c_void_p(stream.cuda_stream), hold, None) == 0
+                    assert lib.ftb200_decode_step(layer._gate[0, B]["params_ref"], layer._stop_ref, 20, C.byref(stop)) == 6
+                    stream.synchronize()
+                    stops.append(bool(st["finished"].all()))
+                    continue
+                stops.append(layer.forward(st, dict(inputs, logits=xs[s], step=step + s)))
+        torch.cuda.synchronize()
+        assert stops == [False, False, True]
+        got.append([v.cpu().numpy() for v in st.values()] + [layer.topk.curand.cpu().numpy(), layer.topp.curand.cpu().numpy()])
+    for want, have in zip(*got):
+        np.testing.assert_array_equal(have, want)
