@@ -112,6 +112,7 @@ static int resident_clusters(int dtype, int lgn, bool whole, size_t smem)
 }
 
 constexpr size_t kRoomyTwoPerSm = 103 * 1024, kTwoPerSm = 107 * 1024 + 512, kThreePerSm = 69 * 1024;
+constexpr size_t kOnePerSm = 190 * 1024;  // one CTA, in the largest split of an SM's memory but one: L1 keeps 60 KB
 
 // Whether the split kernel (a row over a cluster of CTAs) serves a call, and in which form.  `single_pass`: the
 // single-pass kernels could serve it too.  The lines come from timing both at 17000 .. 250000 columns and 6 .. 1024
@@ -183,9 +184,16 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
         }
         return area;
     };
+    // With one CTA on an SM there is room for areas of half a slice up to 245000 columns, and no step needs the second launch for wider ones,
+    // which costs 3 us where nothing is flagged (area of 10240 keys and that launch / so: 28 x 208295 fp32 of both kinds with
+    // log-probabilities 77.7 / 74.1 us; with areas that leave L1 28 KB 75.5).
+    const auto one_on_an_sm = [&] {
+        const int area = area_within(kOnePerSm, kSpAreaWide);
+        return area < A->slice / 2 ? area_within(kSpMaxSmem, kSpAreaWide) : area;
+    };
     const int  ctas  = rows << lgn;
     const auto keeps = [&](int per_sm, size_t budget) {
-        A->area = area_within(budget, kSpAreaMax);
+        A->area = per_sm == 1 ? one_on_an_sm() : area_within(budget, kSpAreaMax);
         return mixed || few ? ctas <= per_sm * sms : rows <= resident_clusters(p->dtype, lgn, true, split_smem_bytes(A->slice, A->area));
     };
     A->roomy    = lgn >= 2 && (keeps(1, kSpMaxSmem) || (least <= kRoomyTwoPerSm && keeps(2, kRoomyTwoPerSm)));
@@ -201,7 +209,7 @@ static bool choose_split(const ftb200_sampling_params* p, const KParams& K, bool
         // 128256 fp32, and no line between the two has been drawn.
         A->roomy    = 1;
         A->criteria = mixed;
-        A->area     = area_within(least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem, kSpAreaMax);
+        A->area     = least <= kTwoPerSm ? area_within(kTwoPerSm, kSpAreaMax) : one_on_an_sm();
     }
     else if (!A->roomy) {
         A->area = area_within(least <= kThreePerSm ? kThreePerSm : (least <= kTwoPerSm ? kTwoPerSm : kSpMaxSmem), kSpAreaMid);

@@ -7,8 +7,8 @@ namespace ftb200 {
 constexpr int kSpBins     = 2048;
 constexpr int kSpAreaMin  = 5120;                   // fp32 keys a CTA can receive of a nucleus: least,
 constexpr int kSpAreaMid  = 6144;                   // most where the kernel keeps to 80 registers,
-constexpr int kSpAreaMax  = 10240;                  // and most where it has 128 (multiples of 1024; the launch chooses)
-constexpr int kSpAreaWide = 16384;                  // of the second launch, over rows that those are too small for: all of 128000 columns
+constexpr int kSpAreaMax  = 10240;                  // and most where it has 128 and two CTAs are on an SM (multiples of 1024; the launch chooses)
+constexpr int kSpAreaWide = 16384;                  // with one CTA on an SM, the second launch over flagged rows too: all of 128000 columns
 constexpr int kSpCandCap  = kSpAreaMin / 2;         // 64-bit candidates the leader can receive
 constexpr int kSpMaxN     = 8;                       // portable cluster size
 constexpr size_t kSpMaxSmem = 216 * 1024;
