@@ -251,27 +251,36 @@ __device__ __forceinline__ float sp_load_slice(const KParams& P, const Xf& X, co
         }
     }
     else {
-        // a row that starts between two 16-byte boundaries: one column per load, eight in flight, a bias beside them (246 x 114514 bf16
-        // with a bias that was sent for once a column had come: 226 us a step, 162 so)
+        // A row that starts between two 16-byte boundaries: one column per load, a bias beside it (246 x 114514 bf16 with a bias that was
+        // sent for once a column had come: 226 us a step, 162 so).  The next eight columns are on their way while eight are worked on, and no
+        // load stands behind a branch: how many were in flight otherwise changed with the registers around the loop.  us a step, loads
+        // behind a branch, as two builds of the same loop had them / eight, sixteen at a time without one / so: 28 x 208295 fp32 of both kinds
+        // 64.5, 77.2 / 85.3, 75.1 / 63.1; 200 x 101001 fp32 145.8, 154.6 / 169.4, 156.5 / 142.2; 100 x 128257 bf16 118.5, 106.7 / 87.5, 88.0 /
+        // 87.6; 300 x 39775 half nucleus rows 313, 182.2 / 172.5, 174.7 / 162.7; 246 x 114515 bf16, k = 40, with a bias 240, 219.6 / 184.0, 183.5 /
+        // 180.3.  (Four columns ahead of four: 75.7, 155.7, 98.1, 176.3, 201.0.)
         constexpr int U    = 8;
         const int     ny   = nchunk << lgvt;
         Xf            T    = X;
         T.bias             = nullptr;  // (it is added here)
         auto walk = [&](auto with_bias) {
             constexpr bool kBias = decltype(with_bias)::value;
-            for (int i0 = tid; i0 < ny; i0 += kThreads * U) {
-                u32 q[U], b[kBias ? U : 1];
+            u32            q[U], b[kBias ? U : 1];
+            auto           send = [&](int i0, u32* qn, u32* bn) {
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
-                    q[u]        = 0;
-                    if (i < ny && v < vocab) {
-                        q[u] = DT == FTB200_F32 ? __ldg((const u32*)rowp + v) : (u32)__ldg((const unsigned short*)rowp + v);
-                        if (kBias) {
-                            b[kBias ? u : 0] = DT == FTB200_F32 ? __ldg((const u32*)X.bias + v) : (u32)__ldg((const unsigned short*)X.bias + v);
-                        }
+                    const int at = i < ny && v < vocab ? v : 0;  // (no branch around a load)
+                    qn[u]        = DT == FTB200_F32 ? __ldg((const u32*)rowp + at) : (u32)__ldg((const unsigned short*)rowp + at);
+                    if (kBias) {
+                        bn[u] = DT == FTB200_F32 ? __ldg((const u32*)X.bias + at) : (u32)__ldg((const unsigned short*)X.bias + at);
                     }
                 }
+            };
+            send(tid, q, b);
+#pragma unroll 1
+            for (int i0 = tid; i0 < ny; i0 += kThreads * U) {
+                u32 qn[U], bn[kBias ? U : 1];
+                send(i0 + kThreads * U, qn, bn);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int i = i0 + u * kThreads, v = ((i >> lgvt) << 10) + col0 + (i & (vt - 1));
@@ -289,6 +298,10 @@ __device__ __forceinline__ float sp_load_slice(const KParams& P, const Xf& X, co
                             y[i] = temp_value<DT>(T, sp_add_bias<DT>(q[u], b[kBias ? u : 0]), v);
                         }
                         best = fmaxf(best, y[i]);
+                    }
+                    q[u] = qn[u];
+                    if (kBias) {
+                        b[kBias ? u : 0] = bn[kBias ? u : 0];
                     }
                 }
             }
