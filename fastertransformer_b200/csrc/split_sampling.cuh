@@ -1994,7 +1994,7 @@ static __device__ __noinline__ void sp_stop_criteria(const KParams& P, const Sto
 // The general row code is not part of this kernel.  It was, in the roomy form, for the rows it leaves; its frames brought the
 // stack to 1.7 to 1.9 KB a thread, and builds that differed in nothing but such sizes ended steps of two CTAs on an SM with an
 // illegal address, or did not.  The cause is not known: its index arithmetic, the sizes of its tables and the pointers it
-// takes for shared have been read through since and stay inside.  Without it the stack is 24 to 48 bytes, 184 in the other form.
+// takes for shared have been read through since and stay inside.  Without it the stack is 16 bytes, 152 in the other form.
 template<int DT, int LGN, bool ROOMY>
 __global__ void __launch_bounds__(kThreads, ROOMY ? 2 : 3) split_sampling_kernel(const __grid_constant__ KParams P,
                                                                      const __grid_constant__ SplitArgs A)
